@@ -18,66 +18,154 @@
 // Products accumulate in fp32 on the FMA pipes, each output one accumulator over ascending k, so a
 // token's result does not depend on which other tokens chose the same expert.  Nothing here reads
 // a count back on the host: grids are sized for the worst case and surplus blocks leave at once.
-#include "mma_tiles.cuh"
+#include "common.cuh"
 
 constexpr int EXPERT_BM = 32;  // slots per row tile of the FMA products
 
 // ---- router ------------------------------------------------------------------------------------
-// Two kernels.  route_logits: a block stages ROUTE_TT tokens' rows in shared memory as fp32 and each
+// Two kernels.  route_logits: a block stages tokens' rows in shared memory as fp32 and each
 // of its eight warps streams one expert's router row once for all of them (a step of a few tokens
 // still spreads the router over E / 8 blocks).  route_pick: one warp per token takes the `top`
 // largest logits -- the choice is made on the logits, which order the experts as their sigmoids do
 // but do not collapse into ties where the sigmoid saturates; lowest index on an exact tie -- and
 // writes sigmoid(logit) as the weight.
+//
+// A block takes `tt` tokens x 8 * EPW experts, a warp EPW experts of all the block's tokens.  What bounds it with many
+// tokens: every product needs a token's value from shared memory, so with one expert per warp the reads of shared memory,
+// not the FMAs, set the time (2048 tokens x 64 experts x 2048: 87 us); four experts per warp use each value four times
+// (QQ us).  With few tokens there are too few blocks instead: then two tokens and 8 experts a block, so that a decode
+// step's router runs on tens of SMs.  The order of a product's additions does not depend on the choice: a token's
+// logits are the same bits in every batch.
 constexpr int ROUTE_TT = 8;
 
-template <typename T>
+template <typename T, int EPW>
 __global__ void __launch_bounds__(256)
 route_logits_kernel(const T* __restrict__ h, long h_stride, const float* __restrict__ router, int num_tokens, int E,
-                    int W, int tt, float* __restrict__ logits) {
+                    int W, int tt, int vec, float* __restrict__ logits) {
   extern __shared__ float route_rows[];  // [tt][W], tt <= ROUTE_TT tokens per block
   pdl_wait();
   pdl_launch_dependents();
   const int t0 = blockIdx.x * tt;
   const int nt = min(tt, num_tokens - t0);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < nt * W; i += 256) {
-    const int t = i / W, k = i - t * W;
-    route_rows[i] = to_f32(h[(long)(t0 + t) * h_stride + k]);
+  for (int t = 0; t < nt; ++t) {
+    const T* src = h + (long)(t0 + t) * h_stride;
+    if (vec) {
+      for (int i = threadIdx.x * 8; i < W; i += 256 * 8) {
+        float v[8];
+        load8(src + i, v);
+        store8(route_rows + t * W + i, v);
+      }
+    } else {
+      for (int i = threadIdx.x; i < W; i += 256) route_rows[t * W + i] = to_f32(src[i]);
+    }
   }
   __syncthreads();
-  const int e = blockIdx.y * 8 + warp;
-  if (e >= E) return;
-  const float* wr = router + (long)e * W;
-  float acc[ROUTE_TT];
+  const int e0 = (blockIdx.y * 8 + warp) * EPW;
+  if (e0 >= E) return;
+  const float* wr[EPW];
 #pragma unroll
-  for (int t = 0; t < ROUTE_TT; ++t) acc[t] = 0.f;
+  for (int x = 0; x < EPW; ++x) wr[x] = router + (long)min(e0 + x, E - 1) * W;
+  float acc[EPW][ROUTE_TT];
+#pragma unroll
+  for (int x = 0; x < EPW; ++x)
+#pragma unroll
+    for (int t = 0; t < ROUTE_TT; ++t) acc[x][t] = 0.f;
   if ((W & 3) == 0) {
 #pragma unroll 2
     for (int i = lane * 4; i < W; i += 128) {
-      const float4 w4 = *reinterpret_cast<const float4*>(wr + i);
+      float4 w4[EPW];
+#pragma unroll
+      for (int x = 0; x < EPW; ++x) w4[x] = *reinterpret_cast<const float4*>(wr[x] + i);
 #pragma unroll
       for (int t = 0; t < ROUTE_TT; ++t) {
         if (t < nt) {
           const float4 x4 = *reinterpret_cast<const float4*>(route_rows + t * W + i);
-          acc[t] = fmaf(x4.x, w4.x, fmaf(x4.y, w4.y, fmaf(x4.z, w4.z, fmaf(x4.w, w4.w, acc[t]))));
+#pragma unroll
+          for (int x = 0; x < EPW; ++x)
+            acc[x][t] = fmaf(x4.x, w4[x].x, fmaf(x4.y, w4[x].y, fmaf(x4.z, w4[x].z, fmaf(x4.w, w4[x].w, acc[x][t]))));
         }
       }
     }
   } else {
     for (int i = lane; i < W; i += 32) {
-      const float w1 = wr[i];
 #pragma unroll
-      for (int t = 0; t < ROUTE_TT; ++t)
-        if (t < nt) acc[t] = fmaf(route_rows[t * W + i], w1, acc[t]);
+      for (int x = 0; x < EPW; ++x) {
+        const float w1 = wr[x][i];
+#pragma unroll
+        for (int t = 0; t < ROUTE_TT; ++t)
+          if (t < nt) acc[x][t] = fmaf(route_rows[t * W + i], w1, acc[x][t]);
+      }
     }
   }
 #pragma unroll
-  for (int t = 0; t < ROUTE_TT; ++t) {
-    if (t < nt) {
-      const float v = warp_sum(acc[t]);
-      if (lane == 0) logits[(long)(t0 + t) * E + e] = v;
+  for (int x = 0; x < EPW; ++x)
+#pragma unroll
+    for (int t = 0; t < ROUTE_TT; ++t) {
+      if (t < nt) {
+        const float v = warp_sum(acc[x][t]);
+        if (lane == 0 && e0 + x < E) logits[(long)(t0 + t) * E + e0 + x] = v;
+      }
     }
+}
+
+// The same choice as route_pick_kernel for up to 32 * PICK_REGS outputs: a token's logits are read once, all loads in
+// flight together, and wait in registers (one warp per token; lane l holds outputs l, l + 32, ...).
+constexpr int PICK_REGS = 8;
+__global__ void route_pick_regs_kernel(const float* __restrict__ logits, int num_tokens, int E, int top, int mode,
+                                       float scale, int* __restrict__ chosen, float* __restrict__ weights) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= num_tokens) return;
+  const float* z = logits + (long)t * E;
+  float v[PICK_REGS];
+#pragma unroll
+  for (int r = 0; r < PICK_REGS; ++r) v[r] = lane + 32 * r < E ? z[lane + 32 * r] : -INFINITY;
+  uint32_t open = 0;  // outputs of this lane that exist and have not been taken
+#pragma unroll
+  for (int r = 0; r < PICK_REGS; ++r) open |= (lane + 32 * r < E ? 1u : 0u) << r;
+  float total = 0.f, first = 0.f;
+  float mine[PICK_REGS];  // lane k % 32 keeps the score of choice k
+#pragma unroll
+  for (int r = 0; r < PICK_REGS; ++r) mine[r] = 0.f;
+  for (int k = 0; k < top; ++k) {
+    float best = -INFINITY;
+    int at = 0x7fffffff;
+#pragma unroll
+    for (int r = 0; r < PICK_REGS; ++r)
+      if ((open >> r & 1u) && (v[r] > best || (v[r] == best && lane + 32 * r < at))) {
+        best = v[r];
+        at = lane + 32 * r;
+      }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oa = __shfl_xor_sync(0xffffffffu, at, o);
+      if (ob > best || (ob == best && oa < at)) {
+        best = ob;
+        at = oa;
+      }
+    }
+    if (at >= E) {  // nothing but NaN is left: the lowest open output
+      int low = open ? lane + 32 * (__ffs(open) - 1) : 0x7fffffff;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) low = min(low, __shfl_xor_sync(0xffffffffu, low, o));
+      at = low;
+    }
+    if (k == 0) first = best;  // the largest logit: the softmax's reference point
+    const float score = mode == 2 ? expf(best - first) : 1.f / (1.f + expf(-best));
+    if (lane == 0) chosen[(long)t * top + k] = at;
+    if ((at & 31) == lane) open &= ~(1u << (at >> 5));
+#pragma unroll
+    for (int r = 0; r < PICK_REGS; ++r)
+      if (k == lane + 32 * r) mine[r] = score;
+    total += score;
+  }
+#pragma unroll
+  for (int r = 0; r < PICK_REGS; ++r) {
+    const int k = lane + 32 * r;
+    if (k < top) weights[(long)t * top + k] = (mode ? mine[r] / total : mine[r]) * scale;
   }
 }
 
@@ -207,7 +295,7 @@ __global__ void route_pick_softmax_all_kernel(const float* __restrict__ logits, 
     }
 }
 
-// logits: fp32 scratch [num_tokens, E] (left with the chosen entries at -inf).
+// logits: fp32 scratch [num_tokens, E].
 // scale: a factor on all weights.  mode 3 takes correction (fp32 [E] or null), count and keep (groups) and renorm; the other modes ignore them.
 Q3_EXPORT int q3_route_top(int dtype, const void* h, long h_stride, const float* router, int num_tokens, int E, int W,
                            int top, int mode, float* logits, int* chosen, float* weights, const float* correction,
@@ -216,25 +304,31 @@ Q3_EXPORT int q3_route_top(int dtype, const void* h, long h_stride, const float*
   if (mode == 3 && count > 1 && (E % count || keep < 1 || keep > count || top > keep * (E / count)))
     return Q3_ERR_ARGUMENT;
   if (num_tokens == 0) return Q3_OK;
-  int tt = ROUTE_TT;  // fewer tokens per block when their rows would not fit in shared memory
-  while (tt > 1 && (size_t)tt * W * sizeof(float) > 128 * 1024) tt >>= 1;
+  const bool many = num_tokens > 64;
+  int tt = many ? ROUTE_TT : 2;
+  while (tt > 1 && (size_t)tt * W * sizeof(float) > 128 * 1024) tt >>= 1;  // fewer where their rows would not fit
   const size_t smem = (size_t)tt * W * sizeof(float);
-  if (smem > 200 * 1024 || (reinterpret_cast<uintptr_t>(router) & 15) || (E + 7) / 8 > 65535) return Q3_ERR_UNSUPPORTED;
-  const dim3 grid((num_tokens + tt - 1) / tt, (E + 7) / 8);
+  const int per_block = many ? 32 : 8;  // experts per block
+  if (smem > 200 * 1024 || (reinterpret_cast<uintptr_t>(router) & 15) || (E + per_block - 1) / per_block > 65535)
+    return Q3_ERR_UNSUPPORTED;
+  const dim3 grid((num_tokens + tt - 1) / tt, (E + per_block - 1) / per_block);
+  const int vec = W % 8 == 0 && h_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0;
   cudaError_t e;
+#define Q3_ROUTE(T_, EPW_)                                                                                            \
+  do {                                                                                                                \
+    if (smem > 48 * 1024)                                                                                             \
+      cudaFuncSetAttribute(route_logits_kernel<T_, EPW_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
+    e = launch_pdl(route_logits_kernel<T_, EPW_>, grid, dim3(256), smem, stream, (const T_*)h, h_stride, router,      \
+                   num_tokens, E, W, tt, vec, logits);                                                                \
+  } while (0)
   if (dtype == Q3_DTYPE_F32) {
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(route_logits_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    e = launch_pdl(route_logits_kernel<float>, grid, dim3(256), smem, stream, (const float*)h, h_stride, router,
-                   num_tokens, E, W, tt, logits);
+    if (many) Q3_ROUTE(float, 4); else Q3_ROUTE(float, 1);
   } else if (dtype == Q3_DTYPE_BF16) {
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(route_logits_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    e = launch_pdl(route_logits_kernel<bf16>, grid, dim3(256), smem, stream, (const bf16*)h, h_stride, router,
-                   num_tokens, E, W, tt, logits);
+    if (many) Q3_ROUTE(bf16, 4); else Q3_ROUTE(bf16, 1);
   } else {
     return Q3_ERR_ARGUMENT;
   }
+#undef Q3_ROUTE
   if (e != cudaSuccess) return Q3_ERR_LAUNCH;
   if (mode == 3) {
     const size_t pick = (size_t)4 * (E + (count > 1 ? count : 0)) * sizeof(float);
@@ -243,8 +337,12 @@ Q3_EXPORT int q3_route_top(int dtype, const void* h, long h_stride, const float*
                    (const float*)logits, num_tokens, E, top, correction, count, keep, renorm, scale, chosen, weights);
     return e == cudaSuccess ? Q3_OK : Q3_ERR_LAUNCH;
   }
-  e = launch_pdl(route_pick_kernel, dim3((num_tokens + 3) / 4), dim3(128), 0, stream, logits, num_tokens, E, top,
-                 mode, scale, chosen, weights);
+  if (E <= 32 * PICK_REGS)
+    e = launch_pdl(route_pick_regs_kernel, dim3((num_tokens + 3) / 4), dim3(128), 0, stream, (const float*)logits,
+                   num_tokens, E, top, mode, scale, chosen, weights);
+  else
+    e = launch_pdl(route_pick_kernel, dim3((num_tokens + 3) / 4), dim3(128), 0, stream, logits, num_tokens, E, top,
+                   mode, scale, chosen, weights);
   return e == cudaSuccess ? Q3_OK : Q3_ERR_LAUNCH;
 }
 
@@ -252,7 +350,7 @@ Q3_EXPORT int q3_route_top(int dtype, const void* h, long h_stride, const float*
 // One block, for a few hundred slots.  Slots of one expert keep their order (slot s before slot
 // s' > s), so the grouping is the same on every run.
 __global__ void group_slots_kernel(const int* __restrict__ chosen, int S, int E, int bm, int* __restrict__ offsets,
-                                   int* __restrict__ tile_offsets, int* __restrict__ order) {
+                                   int* __restrict__ tile_offsets, int* __restrict__ order, int* __restrict__ place) {
   extern __shared__ int sm[];  // counts[E], cursor[E]
   int* counts = sm;
   int* cursor = sm + E;
@@ -281,52 +379,90 @@ __global__ void group_slots_kernel(const int* __restrict__ chosen, int S, int E,
     int rank = 0;
     for (int r = 0; r < s; ++r) rank += chosen[r] == e;
     order[cursor[e] + rank] = s;
+    if (place) place[s] = cursor[e] + rank;
   }
 }
 
 // The same for many slots: placement by atomic cursor (the order inside an expert's group may then
-// differ from run to run; every slot's result is computed on its own, so the outputs do not).
-__global__ void group_slots_atomic_kernel(const int* __restrict__ chosen, int S, int E, int bm,
-                                          int* __restrict__ offsets, int* __restrict__ tile_offsets,
-                                          int* __restrict__ order) {
+// differ from run to run; every slot's result is computed on its own, so the outputs do not).  One block: what bounds it
+// is latency, so a thread's choices are loaded at once and stay in registers for both passes (up to GROUP_REGS each, the
+// rest is read again), and one warp adds the counts up (12,288 slots of 64 experts: QQ us; loads one after the other and
+// one thread's sum took 16).  place (may be null): the grouped position of every slot.
+constexpr int GROUP_THREADS = 1024, GROUP_REGS = 16;
+__global__ void __launch_bounds__(GROUP_THREADS)
+group_slots_atomic_kernel(const int* __restrict__ chosen, int S, int E, int bm, int* __restrict__ offsets,
+                          int* __restrict__ tile_offsets, int* __restrict__ order, int* __restrict__ place) {
   extern __shared__ int sm[];
   int* counts = sm;
   int* cursor = sm + E;
+  const int tid = threadIdx.x;
   pdl_wait();
   pdl_launch_dependents();
-  for (int e = threadIdx.x; e < E; e += blockDim.x) counts[e] = 0;
+  for (int e = tid; e < E; e += GROUP_THREADS) counts[e] = 0;
+  int mine[GROUP_REGS];
+#pragma unroll
+  for (int r = 0; r < GROUP_REGS; ++r) mine[r] = tid + r * GROUP_THREADS < S ? chosen[tid + r * GROUP_THREADS] : -1;
   __syncthreads();
-  for (int s = threadIdx.x; s < S; s += blockDim.x) atomicAdd(&counts[chosen[s]], 1);
+#pragma unroll
+  for (int r = 0; r < GROUP_REGS; ++r)
+    if (mine[r] >= 0) atomicAdd(&counts[mine[r]], 1);
+  for (int s = tid + GROUP_REGS * GROUP_THREADS; s < S; s += GROUP_THREADS) atomicAdd(&counts[chosen[s]], 1);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int at = 0, tiles = 0;
-    for (int e = 0; e < E; ++e) {
-      offsets[e] = at;
-      tile_offsets[e] = tiles;
-      cursor[e] = at;
-      at += counts[e];
-      tiles += (counts[e] + bm - 1) / bm;
+  if (tid < 32) {
+    int at = 0, tiles = 0;  // sums over the experts before this batch of 32
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + tid;
+      const int n = e < E ? counts[e] : 0, m = (n + bm - 1) / bm;
+      int n_sum = n, m_sum = m;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, n_sum, o), b = __shfl_up_sync(0xffffffffu, m_sum, o);
+        if (tid >= o) {
+          n_sum += a;
+          m_sum += b;
+        }
+      }
+      if (e < E) {
+        offsets[e] = cursor[e] = at + n_sum - n;
+        tile_offsets[e] = tiles + m_sum - m;
+      }
+      at += __shfl_sync(0xffffffffu, n_sum, 31);
+      tiles += __shfl_sync(0xffffffffu, m_sum, 31);
     }
-    offsets[E] = at;
-    tile_offsets[E] = tiles;
+    if (tid == 0) {
+      offsets[E] = at;
+      tile_offsets[E] = tiles;
+    }
   }
   __syncthreads();
-  for (int s = threadIdx.x; s < S; s += blockDim.x) order[atomicAdd(&cursor[chosen[s]], 1)] = s;
+#pragma unroll
+  for (int r = 0; r < GROUP_REGS; ++r)
+    if (mine[r] >= 0) {
+      const int s = tid + r * GROUP_THREADS, at = atomicAdd(&cursor[mine[r]], 1);
+      order[at] = s;
+      if (place) place[s] = at;
+    }
+  for (int s = tid + GROUP_REGS * GROUP_THREADS; s < S; s += GROUP_THREADS) {
+    const int at = atomicAdd(&cursor[chosen[s]], 1);
+    order[at] = s;
+    if (place) place[s] = at;
+  }
 }
 
-// bm: slots per row tile of the products that will use tile_offsets (EXPERT_BM for the FMA kernels).
+// bm: slots per row tile of the products that will use tile_offsets (EXPERT_BM for the FMA kernels).  place: int32 [S],
+// the position of every slot in the grouped order, or null.
 Q3_EXPORT int q3_group_slots(const int* chosen, int S, int E, int bm, int* offsets, int* tile_offsets, int* order,
-                             cudaStream_t stream) {
+                             int* place, cudaStream_t stream) {
   if (!chosen || !offsets || !tile_offsets || !order || E < 1 || S < 0 || bm < 1) return Q3_ERR_ARGUMENT;
   if (E > 8192) return Q3_ERR_UNSUPPORTED;
   const size_t smem = 2 * (size_t)E * sizeof(int);
   cudaError_t e;
   if (S <= 512)
     e = launch_pdl(group_slots_kernel, dim3(1), dim3(512), smem, stream, chosen, S, E, bm, offsets, tile_offsets,
-                   order);
+                   order, place);
   else
-    e = launch_pdl(group_slots_atomic_kernel, dim3(1), dim3(1024), smem, stream, chosen, S, E, bm, offsets,
-                   tile_offsets, order);
+    e = launch_pdl(group_slots_atomic_kernel, dim3(1), dim3(GROUP_THREADS), smem, stream, chosen, S, E, bm, offsets,
+                   tile_offsets, order, place);
   return e == cudaSuccess ? Q3_OK : Q3_ERR_LAUNCH;
 }
 
@@ -514,279 +650,75 @@ Q3_EXPORT int q3_expert_up(int dtype, const void* h, long h_stride, const void* 
   return e == cudaSuccess ? Q3_OK : Q3_ERR_LAUNCH;
 }
 
-// ---- the same products on the tensor cores (bfloat16, mma.sync m16n8k16) ---------------------------
-// A block owns BM slots of one expert and 64 output columns (of gate and of up for GATE_UP); four
-// warps, WM = BM / 32 of them along the slots.  The slots' rows are gathered (and, for GATE_UP with
-// the weight on the input, multiplied by it and rounded to bfloat16) into shared memory, the
-// expert's rows come by cp.async through a ring of three stages, 32 of the inner dimension at a
-// time, while the slots' rows of the step after next are already in registers.  K is a multiple of 8
-// and all rows are 16-byte aligned.
-template <bool GATE_UP, int BM>
-__global__ void __launch_bounds__(128)
-expert_gemm_tc_kernel(const bf16* __restrict__ A, long a_stride, const bf16* __restrict__ B, bf16* __restrict__ C,
-                      int N, int K, const int* __restrict__ offsets, const int* __restrict__ tile_offsets,
-                      const int* __restrict__ order, const float* __restrict__ weights, int E, int top,
-                      int scale_input, float limit, float alpha, float up_offset) {
-  constexpr int BN = 64, BK = 32, KS = BK + 8, NB = GATE_UP ? 2 : 1, STAGES = 3;
-  constexpr int WM = BM / 32, WN = 4 / WM, COLS = BN / WN, NTW = COLS / 8;
-  constexpr int A_CHUNKS = BM * (BK / 8) / 128;  // 16-byte chunks of the slots' rows per thread and step
-  extern __shared__ __align__(16) unsigned char expert_smem[];
-  typedef bf16 (*WTile)[BN][KS];
-  typedef bf16 (*ATile)[KS];
-  bf16* w_base = reinterpret_cast<bf16*>(expert_smem);             // [STAGES][NB][BN][KS]
-  bf16* a_base = w_base + STAGES * NB * BN * KS;                   // [2][BM][KS]
-  __shared__ int slot_of[BM];
-  __shared__ float scale_of[BM];
-  pdl_wait();
-  pdl_launch_dependents();
-  const int tile = blockIdx.y;
-  if (tile >= tile_offsets[E]) return;
-  const int e = expert_of_tile(tile_offsets, E, tile);
-  const int row0 = offsets[e] + (tile - tile_offsets[e]) * BM;
-  const int rows = min(BM, offsets[e + 1] - row0);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int r = tid; r < BM; r += 128) {
-    const int slot = r < rows ? order[row0 + r] : -1;
-    slot_of[r] = slot;
-    scale_of[r] = (slot >= 0 && GATE_UP && scale_input) ? weights[slot] : 1.f;
-  }
-  __syncthreads();
-  const int wm = warp / WN, wn = warp % WN;
-  const int n0 = blockIdx.x * BN;
-  const bf16* Be = B + (long)e * NB * N * K;
-  const int steps = (K + BK - 1) / BK;
-
-  // the expert's rows of step s into ring stage s % STAGES (one commit group per call, also when empty)
-  auto load_w = [&](int s) {
-    if (s < steps) {
-      WTile Ws = reinterpret_cast<WTile>(w_base + (s % STAGES) * NB * BN * KS);
-      const int k0 = s * BK;
-      for (int c = tid; c < NB * BN * (BK / 8); c += 128) {
-        const int b = c / (BN * (BK / 8)), y = c % (BN * (BK / 8));
-        const int r = y / (BK / 8), ch = y % (BK / 8);
-        const int gn = n0 + r, gk = k0 + ch * 8;
-        const bool in = gn < N && gk < K;
-        cp_async16(smem_u32(&Ws[b][r][ch * 8]), in ? Be + ((long)b * N + gn) * K + gk : Be, in ? 16 : 0);
-      }
-    }
-    cp_async_commit();
-  };
-  // the slots' rows of step s into registers (gathered, and scaled where the weight is on the input)
-  uint4 a_regs[A_CHUNKS];
-  auto fetch_a = [&](int s) {
-#pragma unroll
-    for (int i = 0; i < A_CHUNKS; ++i) {
-      const int c = tid + i * 128;
-      const int r = c / (BK / 8), ch = c % (BK / 8);
-      const int slot = slot_of[r], gk = s * BK + ch * 8;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (s < steps && slot >= 0 && gk < K) {
-        const long arow = slot / top;
-        v = *reinterpret_cast<const uint4*>(A + arow * a_stride + gk);
-        if (GATE_UP && scale_input) {
-          __nv_bfloat162* hv = reinterpret_cast<__nv_bfloat162*>(&v);
-          const float w = scale_of[r];
-#pragma unroll
-          for (int x = 0; x < 4; ++x) {
-            const float2 f = __bfloat1622float2(hv[x]);
-            hv[x] = __floats2bfloat162_rn(f.x * w, f.y * w);
-          }
-        }
-      }
-      a_regs[i] = v;
-    }
-  };
-  auto store_a = [&](int s) {
-    ATile As = reinterpret_cast<ATile>(a_base + (s & 1) * BM * KS);
-#pragma unroll
-    for (int i = 0; i < A_CHUNKS; ++i) {
-      const int c = tid + i * 128;
-      *reinterpret_cast<uint4*>(&As[c / (BK / 8)][(c % (BK / 8)) * 8]) = a_regs[i];
-    }
-  };
-
-  float acc[NB][2][NTW][4];
-#pragma unroll
-  for (int b = 0; b < NB; ++b)
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-      for (int nt = 0; nt < NTW; ++nt)
-#pragma unroll
-        for (int x = 0; x < 4; ++x) acc[b][mt][nt][x] = 0.f;
-  load_w(0);
-  load_w(1);
-  fetch_a(0);
-  store_a(0);
-  fetch_a(1);
-  for (int s = 0; s < steps; ++s) {
-    cp_async_wait<1>();  // the weights of step s have landed (those of s + 1 may still be on their way)
-    __syncthreads();     // ... for every thread; rows of step s are stored; step s - 1 has been used up
-    load_w(s + 2);       // into the stage step s - 1 used
-    store_a(s + 1);      // into the buffer step s - 1 used
-    fetch_a(s + 2);
-    WTile Ws = reinterpret_cast<WTile>(w_base + (s % STAGES) * NB * BN * KS);
-    ATile As = reinterpret_cast<ATile>(a_base + (s & 1) * BM * KS);
-#pragma unroll
-    for (int kk = 0; kk < BK; kk += 16) {
-      uint32_t a[2][4];
-#pragma unroll
-      for (int mt = 0; mt < 2; ++mt)
-        ldmatrix_x4(a[mt], smem_u32(&As[wm * 32 + mt * 16 + (lane & 15)][kk + (lane >> 4) * 8]));
-#pragma unroll
-      for (int b = 0; b < NB; ++b)
-#pragma unroll
-        for (int np = 0; np < NTW / 2; ++np) {
-          uint32_t bb[4];
-          ldmatrix_x4(bb, smem_u32(&Ws[b][wn * COLS + np * 16 + (lane >> 4) * 8 + (lane & 7)][kk + ((lane >> 3) & 1) * 8]));
-#pragma unroll
-          for (int mt = 0; mt < 2; ++mt) {
-            mma_bf16(acc[b][mt][2 * np], a[mt], bb[0], bb[1]);
-            mma_bf16(acc[b][mt][2 * np + 1], a[mt], bb[2], bb[3]);
-          }
-        }
-    }
-  }
-  cp_async_wait<0>();
-#pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int slot = slot_of[wm * 32 + mt * 16 + half * 8 + (lane >> 2)];
-      if (slot < 0) continue;
-#pragma unroll
-      for (int nt = 0; nt < NTW; ++nt)
-#pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          const int gn = n0 + wn * COLS + nt * 8 + 2 * (lane & 3) + x;
-          if (gn >= N) continue;
-          if (GATE_UP) {
-            const float g = fminf(to_f32(from_f32<bf16>(acc[0][mt][nt][2 * half + x])), limit);
-            const float u = fminf(fmaxf(to_f32(from_f32<bf16>(acc[NB - 1][mt][nt][2 * half + x])), -limit), limit);
-            C[(long)slot * N + gn] = from_f32<bf16>((g / (1.f + expf(-alpha * g))) * (u + up_offset));
-          } else if (scale_input) {
-            const float r = fmaxf(to_f32(from_f32<bf16>(acc[0][mt][nt][2 * half + x])), 0.f);
-            C[(long)slot * N + gn] = from_f32<bf16>(r * r);
-          } else {
-            C[(long)slot * N + gn] = from_f32<bf16>(acc[0][mt][nt][2 * half + x]);
-          }
-        }
-    }
-}
-
-template <bool GATE_UP, int BM>
-static constexpr size_t expert_tc_smem() {
-  return (size_t)(3 * (GATE_UP ? 2 : 1) * 64 * 40 + 2 * BM * 40) * sizeof(bf16);
-}
-
-// The two products as above for bfloat16 with rows of 16-byte multiples; bm (32 or 64) is the row
-// tile that group_slots was given.
-Q3_EXPORT int q3_expert_gate_up_tc(const void* h, long h_stride, const void* gate_up, void* mid, int S, int E, int F,
-                                   int W, int top, int bm, const int* offsets, const int* tile_offsets,
-                                   const int* order, const float* weights, int scale_input, float limit, float alpha,
-                                   float up_offset, cudaStream_t stream) {
-  if (!h || !gate_up || !mid || !offsets || !tile_offsets || !order || !weights) return Q3_ERR_ARGUMENT;
-  if (E < 1 || F < 1 || W < 1 || top < 1 || (bm != 32 && bm != 64)) return Q3_ERR_ARGUMENT;
-  if (W % 8 || h_stride % 8 || (reinterpret_cast<uintptr_t>(h) & 15) || (reinterpret_cast<uintptr_t>(gate_up) & 15))
-    return Q3_ERR_UNSUPPORTED;
-  if (S == 0) return Q3_OK;
-  const int tiles = S / bm + (E < S ? E : S);
-  if (tiles > 65535) return Q3_ERR_UNSUPPORTED;
-  const dim3 grid((F + 63) / 64, tiles);
-  auto kernel = bm == 64 ? expert_gemm_tc_kernel<true, 64> : expert_gemm_tc_kernel<true, 32>;
-  const size_t smem = bm == 64 ? expert_tc_smem<true, 64>() : expert_tc_smem<true, 32>();
-  return launch_pdl(kernel, grid, dim3(128), smem, stream, (const bf16*)h, h_stride, (const bf16*)gate_up, (bf16*)mid, F,
-                    W, offsets, tile_offsets, order, weights, E, top, scale_input, limit, alpha, up_offset) == cudaSuccess
-             ? Q3_OK
-             : Q3_ERR_LAUNCH;
-}
-
-Q3_EXPORT int q3_expert_down_tc(const void* mid, const void* down, void* y, int S, int E, int F, int W, int bm,
-                                const int* offsets, const int* tile_offsets, const int* order, cudaStream_t stream) {
-  if (!mid || !down || !y || !offsets || !tile_offsets || !order || E < 1 || F < 1 || W < 1) return Q3_ERR_ARGUMENT;
-  if (bm != 32 && bm != 64) return Q3_ERR_ARGUMENT;
-  if (F % 8 || (reinterpret_cast<uintptr_t>(mid) & 15) || (reinterpret_cast<uintptr_t>(down) & 15))
-    return Q3_ERR_UNSUPPORTED;
-  if (S == 0) return Q3_OK;
-  const int tiles = S / bm + (E < S ? E : S);
-  if (tiles > 65535) return Q3_ERR_UNSUPPORTED;
-  const dim3 grid((W + 63) / 64, tiles);
-  auto kernel = bm == 64 ? expert_gemm_tc_kernel<false, 64> : expert_gemm_tc_kernel<false, 32>;
-  const size_t smem = bm == 64 ? expert_tc_smem<false, 64>() : expert_tc_smem<false, 32>();
-  return launch_pdl(kernel, grid, dim3(128), smem, stream, (const bf16*)mid, (long)F, (const bf16*)down, (bf16*)y, W, F,
-                    offsets, tile_offsets, order, (const float*)nullptr, E, 1, 0, 0.f, 0.f, 0.f) == cudaSuccess
-             ? Q3_OK
-             : Q3_ERR_LAUNCH;
-}
-
-Q3_EXPORT int q3_expert_up_tc(const void* h, long h_stride, const void* up, void* mid, int S, int E, int F, int W,
-                              int top, int bm, const int* offsets, const int* tile_offsets, const int* order, int act,
-                              cudaStream_t stream) {
-  if (!h || !up || !mid || !offsets || !tile_offsets || !order || E < 1 || F < 1 || W < 1 || top < 1)
-    return Q3_ERR_ARGUMENT;
-  if (bm != 32 && bm != 64) return Q3_ERR_ARGUMENT;
-  if (W % 8 || h_stride % 8 || (reinterpret_cast<uintptr_t>(h) & 15) || (reinterpret_cast<uintptr_t>(up) & 15))
-    return Q3_ERR_UNSUPPORTED;
-  if (S == 0) return Q3_OK;
-  const int tiles = S / bm + (E < S ? E : S);
-  if (tiles > 65535) return Q3_ERR_UNSUPPORTED;
-  const dim3 grid((F + 63) / 64, tiles);
-  auto kernel = bm == 64 ? expert_gemm_tc_kernel<false, 64> : expert_gemm_tc_kernel<false, 32>;
-  const size_t smem = bm == 64 ? expert_tc_smem<false, 64>() : expert_tc_smem<false, 32>();
-  return launch_pdl(kernel, grid, dim3(128), smem, stream, (const bf16*)h, h_stride, (const bf16*)up, (bf16*)mid, F, W,
-                    offsets, tile_offsets, order, (const float*)nullptr, E, top, act, 0.f, 0.f, 0.f) == cudaSuccess
-             ? Q3_OK
-             : Q3_ERR_LAUNCH;
-}
-
 // ---- per-token sum ----------------------------------------------------------------------------------
-template <typename T>
+// VEC values of one token per thread (8: 16-byte accesses, rows of a multiple of 8; what bounds it is memory: 2048
+// tokens x 2048 of 6 slots took 105 us with one value per thread, QQ us with 8).  place: the row of y that holds a slot
+// (null: the slot's own number).
+template <typename T, int VEC>
 __global__ void combine_kernel(const T* __restrict__ y, const float* __restrict__ weights, const T* __restrict__ shared,
                                const T* __restrict__ shared_gate, long gate_stride, T* __restrict__ out, long total,
                                int W, int top, const int* __restrict__ chosen, int stored, const T* __restrict__ h,
-                               long h_stride) {
+                               long h_stride, const int* __restrict__ place) {
   pdl_wait();
   pdl_launch_dependents();
-  const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long idx = ((long)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   if (idx >= total) return;
   const long t = idx / W;
   const int i = (int)(idx - t * W);
-  float sum = 0.f;
+  auto load = [](const T* p, float (&v)[VEC]) {
+    if constexpr (VEC == 8) load8(p, v); else v[0] = to_f32(*p);
+  };
+  float sum[VEC];
+#pragma unroll
+  for (int x = 0; x < VEC; ++x) sum[x] = 0.f;
+#pragma unroll 4
   for (int k = 0; k < top; ++k) {
+    const long slot = t * top + k;
     // a choice beyond the stored experts stands for an expert that returns its input
-    const bool same = chosen && chosen[t * top + k] >= stored;
-    const float v = same ? to_f32(h[t * h_stride + i]) : to_f32(y[(t * top + k) * W + i]);
-    sum += weights ? v * weights[t * top + k] : v;
+    const bool same = chosen && chosen[slot] >= stored;
+    float v[VEC];
+    load(same ? h + t * h_stride + i : y + (place ? (long)place[slot] : slot) * W + i, v);
+    const float w = weights ? weights[slot] : 1.f;
+#pragma unroll
+    for (int x = 0; x < VEC; ++x) sum[x] += weights ? v[x] * w : v[x];
   }
   if (shared) {
-    const float v = to_f32(shared[idx]);
-    sum += shared_gate ? v / (1.f + expf(-to_f32(shared_gate[t * gate_stride]))) : v;
+    float v[VEC];
+    load(shared + idx, v);
+    const float gate = shared_gate ? 1.f + expf(-to_f32(shared_gate[t * gate_stride])) : 1.f;
+#pragma unroll
+    for (int x = 0; x < VEC; ++x) sum[x] += shared_gate ? v[x] / gate : v[x];
   }
-  out[idx] = from_f32<T>(sum);
+  if constexpr (VEC == 8) store8(out + idx, sum); else out[idx] = from_f32<T>(sum[0]);
 }
 
 // y: [T * top, W]; weights: fp32 [T * top] or null (the weight was applied to the input);
 // shared: [T, W] or null; shared_gate: one logit per token, gate_stride elements apart, or null: the
 // shared expert's result is multiplied by the logit's sigmoid; out: [T, W].  chosen (int32 [T * top], with
 // h [T, W] rows h_stride apart, or null): a slot whose choice is >= `stored` takes the token's row of h in
-// place of y.
+// place of y.  place (int32 [T * top] or null): the row of y of every slot.
 Q3_EXPORT int q3_expert_combine(int dtype, const void* y, const float* weights, const void* shared,
                                 const void* shared_gate, long gate_stride, void* out, int num_tokens, int W, int top,
-                                const int* chosen, int stored, const void* h, long h_stride, cudaStream_t stream) {
+                                const int* chosen, int stored, const void* h, long h_stride, const int* place,
+                                cudaStream_t stream) {
   if (!y || !out || W < 1 || top < 1 || (chosen && !h)) return Q3_ERR_ARGUMENT;
   const long total = (long)num_tokens * W;
   if (total == 0) return Q3_OK;
-  const unsigned blocks = (unsigned)((total + 255) / 256);
+  const bool vec = W % 8 == 0 && (!chosen || h_stride % 8 == 0) &&
+                   (((uintptr_t)y | (uintptr_t)shared | (uintptr_t)out | (chosen ? (uintptr_t)h : 0)) & 15) == 0;
+  const unsigned blocks = (unsigned)((total / (vec ? 8 : 1) + 255) / 256);
   cudaError_t e;
-  if (dtype == Q3_DTYPE_F32)
-    e = launch_pdl(combine_kernel<float>, dim3(blocks), dim3(256), 0, stream, (const float*)y, weights,
-                   (const float*)shared, (const float*)shared_gate, gate_stride, (float*)out, total, W, top, chosen,
-                   stored, (const float*)h, h_stride);
-  else if (dtype == Q3_DTYPE_BF16)
-    e = launch_pdl(combine_kernel<bf16>, dim3(blocks), dim3(256), 0, stream, (const bf16*)y, weights,
-                   (const bf16*)shared, (const bf16*)shared_gate, gate_stride, (bf16*)out, total, W, top, chosen,
-                   stored, (const bf16*)h, h_stride);
-  else
+#define Q3_COMBINE(T_, VEC_)                                                                                       \
+  e = launch_pdl(combine_kernel<T_, VEC_>, dim3(blocks), dim3(256), 0, stream, (const T_*)y, weights,              \
+                 (const T_*)shared, (const T_*)shared_gate, gate_stride, (T_*)out, total, W, top, chosen, stored,   \
+                 (const T_*)h, h_stride, place)
+  if (dtype == Q3_DTYPE_F32) {
+    if (vec) Q3_COMBINE(float, 8); else Q3_COMBINE(float, 1);
+  } else if (dtype == Q3_DTYPE_BF16) {
+    if (vec) Q3_COMBINE(bf16, 8); else Q3_COMBINE(bf16, 1);
+  } else {
     return Q3_ERR_ARGUMENT;
+  }
+#undef Q3_COMBINE
   return e == cudaSuccess ? Q3_OK : Q3_ERR_LAUNCH;
 }

@@ -611,16 +611,31 @@ Q3_EXPORT int q3_fused_post_norm(int dtype, const void* pending, int pending_par
 
 // ---- clamped gated unit: g = min(gate, limit), u = clamp(up, -limit, limit),
 //      out = g * sigmoid(alpha * g) * (u + up_offset); gu rows are [gate (F) | up (F)] ----
-template <typename T>
+// VEC values per thread (8 where rows and bases allow 16-byte accesses; memory-bound: 2048 rows of 2816, one value per
+// thread 21.8 us, eight QQ us).
+template <typename T, int VEC>
 __global__ void clamped_glu_kernel(const T* __restrict__ gu, T* __restrict__ out, long total, int F, float limit,
                                    float alpha, float up_offset) {
-  const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_wait();
+  pdl_launch_dependents();
+  const long idx = ((long)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   if (idx >= total) return;
   const long t = idx / F;
   const int i = (int)(idx - t * F);
-  const float g = fminf(to_f32(gu[t * 2 * F + i]), limit);
-  const float u = fminf(fmaxf(to_f32(gu[t * 2 * F + F + i]), -limit), limit);
-  out[idx] = from_f32<T>((g / (1.f + expf(-alpha * g))) * (u + up_offset));
+  float g[VEC], u[VEC];
+  if constexpr (VEC == 8) {
+    load8(gu + t * 2 * F + i, g);
+    load8(gu + t * 2 * F + F + i, u);
+  } else {
+    g[0] = to_f32(gu[t * 2 * F + i]);
+    u[0] = to_f32(gu[t * 2 * F + F + i]);
+  }
+#pragma unroll
+  for (int e = 0; e < VEC; ++e) {
+    const float a = fminf(g[e], limit), b = fminf(fmaxf(u[e], -limit), limit);
+    g[e] = (a / (1.f + expf(-alpha * a))) * (b + up_offset);
+  }
+  if constexpr (VEC == 8) store8(out + idx, g); else out[idx] = from_f32<T>(g[0]);
 }
 
 Q3_EXPORT int q3_clamped_glu(int dtype, const void* gu, void* out, int num_rows, int F, float limit, float alpha,
@@ -628,14 +643,21 @@ Q3_EXPORT int q3_clamped_glu(int dtype, const void* gu, void* out, int num_rows,
   if (!gu || !out || F < 1) return Q3_ERR_ARGUMENT;
   const long total = (long)num_rows * F;
   if (total == 0) return Q3_OK;
-  const unsigned blocks = (unsigned)((total + 255) / 256);
-  if (dtype == Q3_DTYPE_F32)
-    clamped_glu_kernel<float><<<blocks, 256, 0, stream>>>((const float*)gu, (float*)out, total, F, limit, alpha, up_offset);
-  else if (dtype == Q3_DTYPE_BF16)
-    clamped_glu_kernel<bf16><<<blocks, 256, 0, stream>>>((const bf16*)gu, (bf16*)out, total, F, limit, alpha, up_offset);
-  else
+  const bool vec = F % 8 == 0 && aligned16(gu) && aligned16(out);
+  const unsigned blocks = (unsigned)((total / (vec ? 8 : 1) + 255) / 256);
+  cudaError_t e;
+#define Q3_CLAMPED(T_, VEC_)                                                                                     \
+  e = launch_pdl(clamped_glu_kernel<T_, VEC_>, dim3(blocks), dim3(256), 0, stream, (const T_*)gu, (T_*)out, total, F, \
+                 limit, alpha, up_offset)
+  if (dtype == Q3_DTYPE_F32) {
+    if (vec) Q3_CLAMPED(float, 8); else Q3_CLAMPED(float, 1);
+  } else if (dtype == Q3_DTYPE_BF16) {
+    if (vec) Q3_CLAMPED(bf16, 8); else Q3_CLAMPED(bf16, 1);
+  } else {
     return Q3_ERR_ARGUMENT;
-  return q3_launch_status();
+  }
+#undef Q3_CLAMPED
+  return e == cudaSuccess ? Q3_OK : Q3_ERR_LAUNCH;
 }
 
 // ---- gated slice of a second embedding: out[t, i] = gelu_tanh(gate[t, i]) * table[ids[t], offset + i] ----

@@ -95,21 +95,21 @@ _SIGNATURES = {
     "experts": {
         "q3_route_top": [c_int, c_void_p, c_long, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                          c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p],
-        "q3_group_slots": [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
-        "q3_expert_gate_up_tc": [c_void_p, c_long, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
-                                 c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_float, c_float, c_float, c_void_p],
-        "q3_expert_down_tc": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                              c_void_p, c_void_p],
+        "q3_group_slots": [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
         "q3_expert_gate_up": [c_int, c_void_p, c_long, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p,
                               c_void_p, c_void_p, c_void_p, c_int, c_float, c_float, c_float, c_void_p],
         "q3_expert_down": [c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                            c_void_p, c_void_p],
         "q3_expert_combine": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_long, c_void_p, c_int, c_int, c_int,
-                              c_void_p, c_int, c_void_p, c_long, c_void_p],
+                              c_void_p, c_int, c_void_p, c_long, c_void_p, c_void_p],
         "q3_expert_up": [c_int, c_void_p, c_long, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p,
                          c_void_p, c_void_p, c_int, c_void_p],
-        "q3_expert_up_tc": [c_void_p, c_long, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
-                            c_void_p, c_void_p, c_int, c_void_p],
+    },
+    "experts_tcgen05": {
+        "q3_expert_gather": [c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
+                             c_void_p],
+        "q3_expert_tcgen05": [c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
+                              c_float, c_float, c_float, c_void_p, c_void_p],
     },
     "rope_kv": {
         "q3_qk_norm_rope_store": [c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float,
@@ -1074,52 +1074,81 @@ class CudaOps:
         # identity experts are grouped like the stored ones (behind them); the products then stop at the stored
         # experts' last tile
         EA = E + num_identity
-        plan = torch.empty(2 * (EA + 1) + S, dtype=torch.int32, device=dev)
-        offsets, tile_offsets, order = plan[: EA + 1], plan[EA + 1: 2 * (EA + 1)], plan[2 * (EA + 1):]
-        # bfloat16 with 16-byte rows: the products run on the tensor cores, in row tiles of 64 slots when
-        # an expert gets about that many, else of 32
-        tensor_cores = (self.experts_tc and h.dtype == torch.bfloat16 and W % 8 == 0 and F % 8 == 0
-                        and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0)
-        bm = 64 if tensor_cores and S >= 48 * E else 32
-        self._call("experts", "q3_group_slots", "group_slots", _ptr(chosen), S, EA, bm, _ptr(offsets),
-                   _ptr(tile_offsets), _ptr(order))
+        plan = torch.empty(2 * (EA + 1) + 2 * S, dtype=torch.int32, device=dev)
+        offsets, tile_offsets, order = plan[: EA + 1], plan[EA + 1: 2 * (EA + 1)], plan[2 * (EA + 1): 2 * (EA + 1) + S]
+        on_input = weight_on == "input"
+        # bfloat16 with 16-byte rows: the products run on the tensor cores (csrc/experts_tcgen05.cu).  Measured against
+        # mma.sync tiles of 32 and 64 slots that it replaced, gate_up + down of 64 experts of 1408 x 2048, top 6: 8 tokens
+        # 129 against 173 us, 128 tokens 200 / 303, 2048 tokens 298 / 1606; no size was slower.
+        if (self.experts_tc and h.dtype == torch.bfloat16 and W % 8 == 0 and F % 8 == 0 and h.stride(0) % 8 == 0
+                and h.data_ptr() % 16 == 0):
+            return self._routed_experts_tc(h, chosen, weights if on_input else None, None if on_input else weights, gate_up,
+                                           down, plan, EA, 2 if gated else 1, limit, alpha, up_offset, shared, shared_gate,
+                                           num_identity)
+        self._call("experts", "q3_group_slots", "group_slots", _ptr(chosen), S, EA, 32, _ptr(offsets),
+                   _ptr(tile_offsets), _ptr(order), None)
         mid = torch.empty((S, F), dtype=h.dtype, device=dev)
         y = torch.empty((S, W), dtype=h.dtype, device=dev)
         out = torch.empty((T, W), dtype=h.dtype, device=dev)
         code, e = _dtype_code(h.dtype), h.element_size()
-        on_input = weight_on == "input"
         if self.timing is not None:  # every chosen expert's weights once, or once per slot when slots are few
             n_up = 2 if gated else 1
             self._costs(min(S, E) * n_up * F * W * e + T * W * e + S * F * e, 2.0 * n_up * S * F * W,
                         f" {S}x{W}->{n_up}x{F}")
-        if not gated and tensor_cores:
-            self._call("experts", "q3_expert_up_tc", "expert_up_tc", _ptr(h), h.stride(0), _ptr(gate_up), _ptr(mid), S,
-                       E, F, W, top, bm, _ptr(offsets), _ptr(tile_offsets), _ptr(order), 1)
-        elif not gated:
+        if not gated:
             self._call("experts", "q3_expert_up", "expert_up", code, _ptr(h), h.stride(0), _ptr(gate_up), _ptr(mid), S,
                        E, F, W, top, _ptr(offsets), _ptr(tile_offsets), _ptr(order), 1)
-        elif tensor_cores:
-            self._call("experts", "q3_expert_gate_up_tc", "expert_gate_up_tc", _ptr(h), h.stride(0), _ptr(gate_up),
-                       _ptr(mid), S, E, F, W, top, bm, _ptr(offsets), _ptr(tile_offsets), _ptr(order), _ptr(weights),
-                       int(on_input), float(limit), float(alpha), float(up_offset))
         else:
             self._call("experts", "q3_expert_gate_up", "expert_gate_up", code, _ptr(h), h.stride(0), _ptr(gate_up),
                        _ptr(mid), S, E, F, W, top, _ptr(offsets), _ptr(tile_offsets), _ptr(order), _ptr(weights),
                        int(on_input), float(limit), float(alpha), float(up_offset))
         if self.timing is not None:
             self._costs(min(S, E) * F * W * e + S * (F + W) * e, 2.0 * S * F * W, f" {S}x{F}->{W}")
-        if tensor_cores:
-            self._call("experts", "q3_expert_down_tc", "expert_down_tc", _ptr(mid), _ptr(down), _ptr(y), S, E, F, W,
-                       bm, _ptr(offsets), _ptr(tile_offsets), _ptr(order))
-        else:
-            self._call("experts", "q3_expert_down", "expert_down", code, _ptr(mid), _ptr(down), _ptr(y), S, E, F, W,
-                       _ptr(offsets), _ptr(tile_offsets), _ptr(order))
+        self._call("experts", "q3_expert_down", "expert_down", code, _ptr(mid), _ptr(down), _ptr(y), S, E, F, W,
+                   _ptr(offsets), _ptr(tile_offsets), _ptr(order))
         if self.timing is not None:
             self._costs((S + T + (T if shared is not None else 0)) * W * e)
         self._call("experts", "q3_expert_combine", "expert_combine", code, _ptr(y),
                    None if on_input else _ptr(weights), _ptr(shared), _ptr(shared_gate),
                    shared_gate.stride(0) if shared_gate is not None else 0, _ptr(out), T, W, top,
-                   _ptr(chosen) if num_identity else None, E, _ptr(h) if num_identity else None, h.stride(0))
+                   _ptr(chosen) if num_identity else None, E, _ptr(h) if num_identity else None, h.stride(0), None)
+        return out
+
+    def _routed_experts_tc(self, h, chosen, in_weights, out_weights, gate_up, down, plan, EA, unit, limit, alpha,
+                           up_offset, shared, shared_gate, num_identity):
+        """:meth:`routed_experts` with the products on csrc/experts_tcgen05.cu: the slots' rows are laid side by side in
+        the grouped order, both products keep that order, the per-token sum looks a slot's row up."""
+        T, W = h.shape
+        E, F, top = gate_up.shape[0], down.shape[2], chosen.shape[1]
+        S = T * top
+        e = h.element_size()
+        offsets, tile_offsets = plan[: EA + 1], plan[EA + 1: 2 * (EA + 1)]
+        order, place = plan[2 * (EA + 1): 2 * (EA + 1) + S], plan[2 * (EA + 1) + S:]
+        self._call("experts", "q3_group_slots", "group_slots", _ptr(chosen), S, EA, 256, _ptr(offsets),
+                   _ptr(tile_offsets), _ptr(order), _ptr(place))
+        rows = torch.empty((S, W), dtype=h.dtype, device=h.device)  # the slots' inputs, later their outputs
+        mid = torch.empty((S, F), dtype=h.dtype, device=h.device)
+        out = torch.empty((T, W), dtype=h.dtype, device=h.device)
+        if self.timing is not None:
+            self._costs((T + S) * W * e)
+        self._call("experts_tcgen05", "q3_expert_gather", "expert_gather", _ptr(h), h.stride(0), _ptr(in_weights),
+                   _ptr(order), _ptr(offsets), S, E, W, top, _ptr(rows))
+        err = _ptr(self._error_word(h.device))
+        if self.timing is not None:
+            self._costs((min(S, E) * unit * F * W + S * (W + F)) * e, 2.0 * unit * S * F * W, f" {S}x{W}->{unit}x{F}")
+        self._call("experts_tcgen05", "q3_expert_tcgen05", "expert_gate_up_tc" if unit == 2 else "expert_up_tc",
+                   unit, _ptr(gate_up), _ptr(rows), _ptr(mid), S, E, F, W, _ptr(offsets), _ptr(tile_offsets), float(limit),
+                   float(alpha), float(up_offset), err)
+        if self.timing is not None:
+            self._costs((min(S, E) * F * W + S * (F + W)) * e, 2.0 * S * F * W, f" {S}x{F}->{W}")
+        self._call("experts_tcgen05", "q3_expert_tcgen05", "expert_down_tc", 0, _ptr(down), _ptr(mid), _ptr(rows), S, E,
+                   W, F, _ptr(offsets), _ptr(tile_offsets), 0.0, 0.0, 0.0, err)
+        if self.timing is not None:
+            self._costs((S + T + (T if shared is not None else 0)) * W * e)
+        self._call("experts", "q3_expert_combine", "expert_combine", _dtype_code(h.dtype), _ptr(rows), _ptr(out_weights),
+                   _ptr(shared), _ptr(shared_gate), shared_gate.stride(0) if shared_gate is not None else 0, _ptr(out), T, W,
+                   top, _ptr(chosen) if num_identity else None, E, _ptr(h) if num_identity else None, h.stride(0),
+                   _ptr(place))
         return out
 
     # ---- position encoding + cache write -----------------------------------------------

@@ -130,7 +130,7 @@ class RoutedExperts(Part):
         if self.ctx.dtype == torch.float32:
             groups.append("gemm_f32")
         else:
-            groups += ["gemm_small_m", "gemm_stream"]
+            groups += ["gemm_small_m", "gemm_stream", "experts_tcgen05"]
         return groups
 
     def forward(self, h: torch.Tensor, step: StepContext) -> torch.Tensor:

@@ -1,0 +1,109 @@
+"""The routed experts' products on the tcgen05 kernel (csrc/experts_tcgen05.cu) against their torch statement, at the
+sizes where its tiles can go wrong: experts with no slot, one, a multiple of 32 and one more or less, a full chunk of 256 and
+the first sizes that take two and three; widths that end inside a slice of K or inside a tile of features."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+COUNTS = [0, 1, 31, 32, 33, 0, 255, 256, 257, 512, 513, 2]
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from qwen3_runtime_b200.ops.cuda import CudaOps
+
+    return CudaOps()
+
+
+def _choices(counts, top, g):
+    """``chosen [T, top]`` in which expert e is chosen counts[e] times (padded with a further expert), in random order."""
+    slots = torch.cat([torch.full((n,), e, dtype=torch.int32) for e, n in enumerate(counts)])
+    pad = -slots.numel() % top
+    slots = torch.cat([slots, torch.full((pad,), len(counts), dtype=torch.int32)])
+    return slots[torch.randperm(slots.numel(), generator=g)].view(-1, top).contiguous().cuda()
+
+
+@pytest.mark.parametrize("width,size", [(64, 64), (72, 136), (320, 88), (128, 392)])
+@pytest.mark.parametrize("unit,weight_on,identity", [("clamped_glu", "input", 0), ("clamped_glu", "output", 2), ("relu2", "output", 0)])
+def test_products_against_their_statement(ops, width, size, unit, weight_on, identity):
+    from emulated_ops import TorchOps
+
+    g = torch.Generator().manual_seed(width + size)
+    top = 3
+    chosen = _choices(COUNTS, top, g)
+    T, stored = chosen.shape[0], len(COUNTS) + 1 - identity
+    weights = torch.rand((T, top), generator=g).cuda() + 0.25
+    rows = torch.randn((T, width + 16), generator=g).to(torch.bfloat16).cuda()
+    h = rows[:, 8: 8 + width]  # rows wider than the layer
+    gated = 2 if unit == "clamped_glu" else 1
+    first = (width ** -0.5 * torch.randn((stored, gated * size, width), generator=g)).to(torch.bfloat16).cuda()
+    down = (size ** -0.5 * torch.randn((stored, width, size), generator=g)).to(torch.bfloat16).cuda()
+    shared = torch.randn((T, width), generator=g).to(torch.bfloat16).cuda()
+    kw = dict(weight_on=weight_on, shared=shared, activation=unit)
+    if unit == "clamped_glu":
+        kw.update(limit=1.5, alpha=1.702, up_offset=1.0, num_identity=identity)
+    else:
+        kw.update(shared_gate=torch.randn((T, 3), generator=g).to(torch.bfloat16).cuda()[:, 1])
+    launched = []
+    call = ops._call
+
+    def spy(group, name, what, *args):
+        launched.append(name)
+        return call(group, name, what, *args)
+
+    ops._call = spy
+    try:
+        got = ops.routed_experts(h, chosen, weights, first, down, **kw).float()
+    finally:
+        del ops._call
+    assert launched.count("q3_expert_tcgen05") == 2
+    ops.raise_if_kernel_error()
+    want = TorchOps().routed_experts(h, chosen, weights, first, down, **kw).float()
+    ops.experts_tc = False
+    other = ops.routed_experts(h, chosen, weights, first, down, **kw).float()
+    ops.experts_tc = True
+    # the kernels and the statement round the same places; a product's sum in another order moves a bfloat16 rounding by one unit, 2^-8 of
+    # the value, in the expert's hidden row and once more in its output, and the sum over three experts once more
+    bound = 3 * 2.0 ** -8 * float(want.abs().max())
+    assert float((got - want).abs().max()) <= bound
+    assert float((got - other).abs().max()) <= bound
+
+
+def test_one_token_and_many_experts(ops):
+    """Fewer slots than experts, and more tiles than pairs of SMs."""
+    from emulated_ops import TorchOps
+
+    g = torch.Generator().manual_seed(5)
+    for T, E, width, size in ((1, 40, 64, 64), (700, 200, 256, 264)):
+        chosen = torch.stack([torch.randperm(E, generator=g)[:2] for _ in range(T)]).int().cuda()
+        weights = torch.rand((T, 2), generator=g).cuda()
+        h = torch.randn((T, width), generator=g).to(torch.bfloat16).cuda()
+        first = (width ** -0.5 * torch.randn((E, 2 * size, width), generator=g)).to(torch.bfloat16).cuda()
+        down = (size ** -0.5 * torch.randn((E, width, size), generator=g)).to(torch.bfloat16).cuda()
+        kw = dict(limit=7.0, alpha=1.702, up_offset=1.0, weight_on="input")
+        got = ops.routed_experts(h, chosen, weights, first, down, **kw).float()
+        ops.raise_if_kernel_error()
+        want = TorchOps().routed_experts(h, chosen, weights, first, down, **kw).float()
+        assert float((got - want).abs().max()) <= 3 * 2.0 ** -8 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("tokens,experts,mode", [(1, 5, "sigmoid"), (64, 33, "softmax_chosen"), (65, 64, "sigmoid"), (200, 7, "sigmoid"),
+                                                 (130, 256, "softmax_chosen"), (130, 257, "sigmoid")])
+def test_router_in_every_batch(ops, tokens, experts, mode):
+    """A token's choice and weights are the same bits whatever the batch (few and many tokens take other launch shapes,
+    up to 256 outputs another kernel for the choice), and agree with the statement."""
+    from emulated_ops import TorchOps
+
+    g = torch.Generator().manual_seed(tokens)
+    h = torch.randn((tokens, 136), generator=g).to(torch.bfloat16).cuda()
+    router = (0.1 * torch.randn((experts, 136), generator=g)).cuda()
+    chosen, weights = ops.route_top(h, router, 5, score=mode)
+    want_c, want_w = TorchOps().route_top(h, router, 5, score=mode)
+    assert torch.equal(chosen, want_c) and float((weights - want_w).abs().max()) < 1e-5
+    for rows in (slice(0, 1), slice(tokens // 2, tokens)):
+        c, w = ops.route_top(h[rows], router, 5, score=mode)
+        assert torch.equal(c, chosen[rows]) and torch.equal(w, weights[rows])
