@@ -30,15 +30,16 @@ constexpr int EXPERT_BM = 32;  // slots per row tile of the FMA products
 // but do not collapse into ties where the sigmoid saturates; lowest index on an exact tie -- and
 // writes sigmoid(logit) as the weight.
 //
-// A block takes `tt` tokens x 8 * EPW experts, a warp EPW experts of all the block's tokens.  What bounds it with many
-// tokens: every product needs a token's value from shared memory, so with one expert per warp the reads of shared memory,
-// not the FMAs, set the time (2048 tokens x 64 experts x 2048: 87 us); four experts per warp use each value four times
-// (QQ us).  With few tokens there are too few blocks instead: then two tokens and 8 experts a block, so that a decode
-// step's router runs on tens of SMs.  The order of a product's additions does not depend on the choice: a token's
-// logits are the same bits in every batch.
+// Two kernels with the same order of additions (a token's logits are the same bits in every batch): lane l adds the
+// products of k = 4 l .. 4 l + 3, then of those + 128, and so on; the lanes' sums are added by halving.
+//   few tokens: a block stages 2 tokens' rows in shared memory, a warp computes one expert's logits, so that a decode
+//   step's router runs on tens of SMs;
+//   many tokens: a warp keeps 8 tokens x 8 experts in registers and reads operands straight from L1 (a block 16 tokens x
+//   32 experts).  With one expert per warp the reads of the tokens' values, not the FMAs, set the time: 2048 tokens x 64
+//   experts x 2048 took 87 us, with four experts per warp 47, now QQ1 (FMAs alone: 7).
 constexpr int ROUTE_TT = 8;
 
-template <typename T, int EPW>
+template <typename T>
 __global__ void __launch_bounds__(256)
 route_logits_kernel(const T* __restrict__ h, long h_stride, const float* __restrict__ router, int num_tokens, int E,
                     int W, int tt, int vec, float* __restrict__ logits) {
@@ -61,51 +62,92 @@ route_logits_kernel(const T* __restrict__ h, long h_stride, const float* __restr
     }
   }
   __syncthreads();
-  const int e0 = (blockIdx.y * 8 + warp) * EPW;
-  if (e0 >= E) return;
-  const float* wr[EPW];
+  const int e = blockIdx.y * 8 + warp;
+  if (e >= E) return;
+  const float* wr = router + (long)e * W;
+  float acc[ROUTE_TT];
 #pragma unroll
-  for (int x = 0; x < EPW; ++x) wr[x] = router + (long)min(e0 + x, E - 1) * W;
-  float acc[EPW][ROUTE_TT];
-#pragma unroll
-  for (int x = 0; x < EPW; ++x)
-#pragma unroll
-    for (int t = 0; t < ROUTE_TT; ++t) acc[x][t] = 0.f;
+  for (int t = 0; t < ROUTE_TT; ++t) acc[t] = 0.f;
   if ((W & 3) == 0) {
 #pragma unroll 2
     for (int i = lane * 4; i < W; i += 128) {
-      float4 w4[EPW];
-#pragma unroll
-      for (int x = 0; x < EPW; ++x) w4[x] = *reinterpret_cast<const float4*>(wr[x] + i);
+      const float4 w4 = *reinterpret_cast<const float4*>(wr + i);
 #pragma unroll
       for (int t = 0; t < ROUTE_TT; ++t) {
         if (t < nt) {
           const float4 x4 = *reinterpret_cast<const float4*>(route_rows + t * W + i);
-#pragma unroll
-          for (int x = 0; x < EPW; ++x)
-            acc[x][t] = fmaf(x4.x, w4[x].x, fmaf(x4.y, w4[x].y, fmaf(x4.z, w4[x].z, fmaf(x4.w, w4[x].w, acc[x][t]))));
+          acc[t] = fmaf(x4.x, w4.x, fmaf(x4.y, w4.y, fmaf(x4.z, w4.z, fmaf(x4.w, w4.w, acc[t]))));
         }
       }
     }
   } else {
     for (int i = lane; i < W; i += 32) {
+      const float w1 = wr[i];
 #pragma unroll
-      for (int x = 0; x < EPW; ++x) {
-        const float w1 = wr[x][i];
-#pragma unroll
-        for (int t = 0; t < ROUTE_TT; ++t)
-          if (t < nt) acc[x][t] = fmaf(route_rows[t * W + i], w1, acc[x][t]);
-      }
+      for (int t = 0; t < ROUTE_TT; ++t)
+        if (t < nt) acc[t] = fmaf(route_rows[t * W + i], w1, acc[t]);
     }
   }
 #pragma unroll
-  for (int x = 0; x < EPW; ++x)
+  for (int t = 0; t < ROUTE_TT; ++t) {
+    if (t < nt) {
+      const float v = warp_sum(acc[t]);
+      if (lane == 0) logits[(long)(t0 + t) * E + e] = v;
+    }
+  }
+}
+
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const bf16* p) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+constexpr int ROUTE_EPW = 8;               // experts per warp
+constexpr int ROUTE_WT = 2, ROUTE_WE = 4;  // warps of a block along tokens and along experts
+
+template <typename T>
+__global__ void __launch_bounds__(256, 2)
+route_logits_tile_kernel(const T* __restrict__ h, long h_stride, const float* __restrict__ router, int num_tokens, int E,
+                         int W, float* __restrict__ logits) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t0 = (blockIdx.x * ROUTE_WT + warp / ROUTE_WE) * ROUTE_TT;
+  const int e0 = (blockIdx.y * ROUTE_WE + warp % ROUTE_WE) * ROUTE_EPW;
+  if (t0 >= num_tokens || e0 >= E) return;
+  // tokens and experts past the end are read as the last one and not stored
+  const T* x[ROUTE_TT];
+  const float* w[ROUTE_EPW];
+#pragma unroll
+  for (int t = 0; t < ROUTE_TT; ++t) x[t] = h + (long)min(t0 + t, num_tokens - 1) * h_stride + lane * 4;
+#pragma unroll
+  for (int e = 0; e < ROUTE_EPW; ++e) w[e] = router + (long)min(e0 + e, E - 1) * W + lane * 4;
+  float acc[ROUTE_TT][ROUTE_EPW];
+#pragma unroll
+  for (int t = 0; t < ROUTE_TT; ++t)
+#pragma unroll
+    for (int e = 0; e < ROUTE_EPW; ++e) acc[t][e] = 0.f;
+  for (int i = 0; i < W - lane * 4; i += 128) {
+    float4 w4[ROUTE_EPW];
+#pragma unroll
+    for (int e = 0; e < ROUTE_EPW; ++e) w4[e] = load4(w[e] + i);
 #pragma unroll
     for (int t = 0; t < ROUTE_TT; ++t) {
-      if (t < nt) {
-        const float v = warp_sum(acc[x][t]);
-        if (lane == 0 && e0 + x < E) logits[(long)(t0 + t) * E + e0 + x] = v;
-      }
+      const float4 x4 = load4(x[t] + i);
+#pragma unroll
+      for (int e = 0; e < ROUTE_EPW; ++e)
+        acc[t][e] = fmaf(x4.x, w4[e].x, fmaf(x4.y, w4[e].y, fmaf(x4.z, w4[e].z, fmaf(x4.w, w4[e].w, acc[t][e]))));
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < ROUTE_TT; ++t)
+#pragma unroll
+    for (int e = 0; e < ROUTE_EPW; ++e) {
+      const float v = warp_sum(acc[t][e]);
+      if (lane == 0 && t0 + t < num_tokens && e0 + e < E) logits[(long)(t0 + t) * E + e0 + e] = v;
     }
 }
 
@@ -304,31 +346,41 @@ Q3_EXPORT int q3_route_top(int dtype, const void* h, long h_stride, const float*
   if (mode == 3 && count > 1 && (E % count || keep < 1 || keep > count || top > keep * (E / count)))
     return Q3_ERR_ARGUMENT;
   if (num_tokens == 0) return Q3_OK;
-  const bool many = num_tokens > 64;
-  int tt = many ? ROUTE_TT : 2;
-  while (tt > 1 && (size_t)tt * W * sizeof(float) > 128 * 1024) tt >>= 1;  // fewer where their rows would not fit
-  const size_t smem = (size_t)tt * W * sizeof(float);
-  const int per_block = many ? 32 : 8;  // experts per block
-  if (smem > 200 * 1024 || (reinterpret_cast<uintptr_t>(router) & 15) || (E + per_block - 1) / per_block > 65535)
-    return Q3_ERR_UNSUPPORTED;
-  const dim3 grid((num_tokens + tt - 1) / tt, (E + per_block - 1) / per_block);
-  const int vec = W % 8 == 0 && h_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0;
+  if (reinterpret_cast<uintptr_t>(router) & 15) return Q3_ERR_UNSUPPORTED;
+  if (dtype != Q3_DTYPE_F32 && dtype != Q3_DTYPE_BF16) return Q3_ERR_ARGUMENT;
+  const size_t elem = dtype == Q3_DTYPE_F32 ? 4 : 2;
+  // both kernels give the same bits; the tile kernel needs about 64 tokens to fill the SMs
+  const bool tile = num_tokens > 64 && W % 4 == 0 && h_stride % 4 == 0 &&
+                    (reinterpret_cast<uintptr_t>(h) & (4 * elem - 1)) == 0;
+  const int te = ROUTE_WE * ROUTE_EPW;
   cudaError_t e;
-#define Q3_ROUTE(T_, EPW_)                                                                                            \
-  do {                                                                                                                \
-    if (smem > 48 * 1024)                                                                                             \
-      cudaFuncSetAttribute(route_logits_kernel<T_, EPW_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
-    e = launch_pdl(route_logits_kernel<T_, EPW_>, grid, dim3(256), smem, stream, (const T_*)h, h_stride, router,      \
-                   num_tokens, E, W, tt, vec, logits);                                                                \
-  } while (0)
-  if (dtype == Q3_DTYPE_F32) {
-    if (many) Q3_ROUTE(float, 4); else Q3_ROUTE(float, 1);
-  } else if (dtype == Q3_DTYPE_BF16) {
-    if (many) Q3_ROUTE(bf16, 4); else Q3_ROUTE(bf16, 1);
+  if (tile && (E + te - 1) / te <= 65535) {
+    const dim3 grid((num_tokens + ROUTE_WT * ROUTE_TT - 1) / (ROUTE_WT * ROUTE_TT), (E + te - 1) / te);
+    if (dtype == Q3_DTYPE_F32)
+      e = launch_pdl(route_logits_tile_kernel<float>, grid, dim3(256), 0, stream, (const float*)h, h_stride, router,
+                     num_tokens, E, W, logits);
+    else
+      e = launch_pdl(route_logits_tile_kernel<bf16>, grid, dim3(256), 0, stream, (const bf16*)h, h_stride, router,
+                     num_tokens, E, W, logits);
   } else {
-    return Q3_ERR_ARGUMENT;
+    int tt = num_tokens > 64 ? ROUTE_TT : 2;
+    while (tt > 1 && (size_t)tt * W * sizeof(float) > 128 * 1024) tt >>= 1;  // fewer where their rows would not fit
+    const size_t smem = (size_t)tt * W * sizeof(float);
+    if (smem > 200 * 1024 || (E + 7) / 8 > 65535) return Q3_ERR_UNSUPPORTED;
+    const dim3 grid((num_tokens + tt - 1) / tt, (E + 7) / 8);
+    const int vec = W % 8 == 0 && h_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0;
+    if (dtype == Q3_DTYPE_F32) {
+      if (smem > 48 * 1024)
+        cudaFuncSetAttribute(route_logits_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      e = launch_pdl(route_logits_kernel<float>, grid, dim3(256), smem, stream, (const float*)h, h_stride, router,
+                     num_tokens, E, W, tt, vec, logits);
+    } else {
+      if (smem > 48 * 1024)
+        cudaFuncSetAttribute(route_logits_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      e = launch_pdl(route_logits_kernel<bf16>, grid, dim3(256), smem, stream, (const bf16*)h, h_stride, router,
+                     num_tokens, E, W, tt, vec, logits);
+    }
   }
-#undef Q3_ROUTE
   if (e != cudaSuccess) return Q3_ERR_LAUNCH;
   if (mode == 3) {
     const size_t pick = (size_t)4 * (E + (count > 1 ? count : 0)) * sizeof(float);
@@ -383,36 +435,55 @@ __global__ void group_slots_kernel(const int* __restrict__ chosen, int S, int E,
   }
 }
 
-// The same for many slots: placement by atomic cursor (the order inside an expert's group may then
-// differ from run to run; every slot's result is computed on its own, so the outputs do not).  One block: what bounds it
-// is latency, so a thread's choices are loaded at once and stay in registers for both passes (up to GROUP_REGS each, the
-// rest is read again), and one warp adds the counts up (12,288 slots of 64 experts: QQ us; loads one after the other and
-// one thread's sum took 16).  place (may be null): the grouped position of every slot.
-constexpr int GROUP_THREADS = 1024, GROUP_REGS = 16;
+// The same for many slots, in two kernels of a block per 1024 slots (the order inside an expert's group may differ from
+// run to run; every slot's result is computed on its own, so the outputs do not).  count_slots: a slot's rank among its
+// block's slots of the same expert and the block's counts; place_slots: every block adds up the counts of the blocks
+// before it and of all blocks.  What bounds this is the latency of the atomics on a few counters; one block for all
+// slots took 13 us for 12,288 slots of 64 experts, these two 8.
+constexpr int GROUP_THREADS = 1024;
 __global__ void __launch_bounds__(GROUP_THREADS)
-group_slots_atomic_kernel(const int* __restrict__ chosen, int S, int E, int bm, int* __restrict__ offsets,
-                          int* __restrict__ tile_offsets, int* __restrict__ order, int* __restrict__ place) {
+count_slots_kernel(const int* __restrict__ chosen, int S, int E, int* __restrict__ ranks, int* __restrict__ counts) {
   extern __shared__ int sm[];
-  int* counts = sm;
-  int* cursor = sm + E;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, s = blockIdx.x * GROUP_THREADS + tid;
+  for (int e = tid; e < E; e += GROUP_THREADS) sm[e] = 0;
   pdl_wait();
   pdl_launch_dependents();
-  for (int e = tid; e < E; e += GROUP_THREADS) counts[e] = 0;
-  int mine[GROUP_REGS];
-#pragma unroll
-  for (int r = 0; r < GROUP_REGS; ++r) mine[r] = tid + r * GROUP_THREADS < S ? chosen[tid + r * GROUP_THREADS] : -1;
+  const int e = s < S ? chosen[s] : -1;
   __syncthreads();
-#pragma unroll
-  for (int r = 0; r < GROUP_REGS; ++r)
-    if (mine[r] >= 0) atomicAdd(&counts[mine[r]], 1);
-  for (int s = tid + GROUP_REGS * GROUP_THREADS; s < S; s += GROUP_THREADS) atomicAdd(&counts[chosen[s]], 1);
+  if (e >= 0) ranks[s] = atomicAdd(&sm[e], 1);
+  __syncthreads();
+  for (int x = tid; x < E; x += GROUP_THREADS) counts[(long)blockIdx.x * E + x] = sm[x];
+}
+
+__global__ void __launch_bounds__(GROUP_THREADS)
+place_slots_kernel(const int* __restrict__ chosen, int S, int E, int bm, const int* __restrict__ ranks,
+                   const int* __restrict__ counts, int* __restrict__ offsets, int* __restrict__ tile_offsets,
+                   int* __restrict__ order, int* __restrict__ place) {
+  extern __shared__ int sm[];
+  int* total = sm;       // slots per expert; then the expert's first slot
+  int* before = sm + E;  // slots of the expert in earlier blocks
+  const int tid = threadIdx.x, s = blockIdx.x * GROUP_THREADS + tid;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int e = s < S ? chosen[s] : -1;
+  const int rank = s < S ? ranks[s] : 0;
+  for (int x = tid; x < E; x += GROUP_THREADS) {
+    int sum = 0, mine = 0;
+#pragma unroll 8
+    for (int b = 0; b < (int)gridDim.x; ++b) {
+      const int c = counts[(long)b * E + x];
+      if (b < (int)blockIdx.x) mine += c;
+      sum += c;
+    }
+    total[x] = sum;
+    before[x] = mine;
+  }
   __syncthreads();
   if (tid < 32) {
     int at = 0, tiles = 0;  // sums over the experts before this batch of 32
     for (int e0 = 0; e0 < E; e0 += 32) {
-      const int e = e0 + tid;
-      const int n = e < E ? counts[e] : 0, m = (n + bm - 1) / bm;
+      const int x = e0 + tid;
+      const int n = x < E ? total[x] : 0, m = (n + bm - 1) / bm;
       int n_sum = n, m_sum = m;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -422,47 +493,53 @@ group_slots_atomic_kernel(const int* __restrict__ chosen, int S, int E, int bm, 
           m_sum += b;
         }
       }
-      if (e < E) {
-        offsets[e] = cursor[e] = at + n_sum - n;
-        tile_offsets[e] = tiles + m_sum - m;
+      if (x < E) {
+        total[x] = at + n_sum - n;
+        if (blockIdx.x == 0) {
+          offsets[x] = at + n_sum - n;
+          tile_offsets[x] = tiles + m_sum - m;
+        }
       }
       at += __shfl_sync(0xffffffffu, n_sum, 31);
       tiles += __shfl_sync(0xffffffffu, m_sum, 31);
     }
-    if (tid == 0) {
+    if (tid == 0 && blockIdx.x == 0) {
       offsets[E] = at;
       tile_offsets[E] = tiles;
     }
   }
   __syncthreads();
-#pragma unroll
-  for (int r = 0; r < GROUP_REGS; ++r)
-    if (mine[r] >= 0) {
-      const int s = tid + r * GROUP_THREADS, at = atomicAdd(&cursor[mine[r]], 1);
-      order[at] = s;
-      if (place) place[s] = at;
-    }
-  for (int s = tid + GROUP_REGS * GROUP_THREADS; s < S; s += GROUP_THREADS) {
-    const int at = atomicAdd(&cursor[chosen[s]], 1);
+  if (e >= 0) {
+    const int at = total[e] + before[e] + rank;
     order[at] = s;
     if (place) place[s] = at;
   }
 }
 
 // bm: slots per row tile of the products that will use tile_offsets (EXPERT_BM for the FMA kernels).  place: int32 [S],
-// the position of every slot in the grouped order, or null.
+// the position of every slot in the grouped order, or null.  scratch: int32 [S + ceil(S / 1024) * E], used for more than
+// 512 slots.
 Q3_EXPORT int q3_group_slots(const int* chosen, int S, int E, int bm, int* offsets, int* tile_offsets, int* order,
-                             int* place, cudaStream_t stream) {
+                             int* place, int* scratch, cudaStream_t stream) {
   if (!chosen || !offsets || !tile_offsets || !order || E < 1 || S < 0 || bm < 1) return Q3_ERR_ARGUMENT;
   if (E > 8192) return Q3_ERR_UNSUPPORTED;
   const size_t smem = 2 * (size_t)E * sizeof(int);
   cudaError_t e;
-  if (S <= 512)
+  if (S <= 512) {
+    if (smem > 48 * 1024)
+      cudaFuncSetAttribute(group_slots_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     e = launch_pdl(group_slots_kernel, dim3(1), dim3(512), smem, stream, chosen, S, E, bm, offsets, tile_offsets,
                    order, place);
-  else
-    e = launch_pdl(group_slots_atomic_kernel, dim3(1), dim3(GROUP_THREADS), smem, stream, chosen, S, E, bm, offsets,
-                   tile_offsets, order, place);
+  } else {
+    if (!scratch) return Q3_ERR_ARGUMENT;
+    if (smem > 48 * 1024)
+      cudaFuncSetAttribute(place_slots_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const dim3 grid((S + GROUP_THREADS - 1) / GROUP_THREADS);
+    e = launch_pdl(count_slots_kernel, grid, dim3(GROUP_THREADS), smem / 2, stream, chosen, S, E, scratch, scratch + S);
+    if (e == cudaSuccess)
+      e = launch_pdl(place_slots_kernel, grid, dim3(GROUP_THREADS), smem, stream, chosen, S, E, bm,
+                     (const int*)scratch, (const int*)(scratch + S), offsets, tile_offsets, order, place);
+  }
   return e == cudaSuccess ? Q3_OK : Q3_ERR_LAUNCH;
 }
 

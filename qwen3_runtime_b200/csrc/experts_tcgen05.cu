@@ -1,6 +1,6 @@
 // The routed experts' products for prompt portions, in bfloat16 on the 5th-generation tensor cores.
 //
-//   gather      xs[r] = h[token(order[r])] (times the slot's weight where it multiplies the expert's input,
+//   gather      xs[place(slot)] = h[token(slot)] (times the slot's weight where it multiplies the expert's input,
 //               rounded to bfloat16): the slots' rows side by side, grouped by expert
 //   gate_up     mid[r] = glu(W_gate_e xs[r], W_up_e xs[r])   (or relu(W_up_e xs[r])^2 without a gate)
 //   down        y[r] = W_down_e mid[r]
@@ -64,6 +64,18 @@ __device__ __forceinline__ Tile tile_at(int tile, int ftiles, const int* __restr
   return t;
 }
 
+// First rows of a CTA's two boxes of 64 weight rows of a tile.
+template <int UNIT>
+__device__ __forceinline__ void weight_rows(const Tile& t, int N, int rank, int& w0, int& w1) {
+  if (UNIT == UNIT_GLU) {
+    w0 = t.expert * 2 * N + t.f * 128 + 64 * rank;
+    w1 = w0 + N;
+  } else {
+    w0 = t.expert * N + t.f * 256 + 128 * rank;
+    w1 = w0 + 64;
+  }
+}
+
 template <int UNIT>
 __global__ void __launch_bounds__(THREADS, 1)
 expert_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
@@ -124,15 +136,8 @@ expert_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
         const Tile t = tile_at(tile, ftiles, offsets, tile_offsets, E);
-        const int f0 = t.f * TILE_F;
-        int w0, w1;  // first rows of this CTA's two boxes of 64 weight rows
-        if (UNIT == UNIT_GLU) {
-          w0 = t.expert * 2 * N + f0 + 64 * (int)rank;
-          w1 = w0 + N;
-        } else {
-          w0 = t.expert * N + f0 + 128 * (int)rank;
-          w1 = w0 + 64;
-        }
+        int w0, w1;
+        weight_rows<UNIT>(t, N, rank, w0, w1);
         const int half = t.n / 2, boxes = (half + B_BOX_ROWS - 1) / B_BOX_ROWS;
         const int x0 = t.row0 + (int)rank * half;
         const uint32_t bytes = A_BYTES + boxes * B_BOX_BYTES;
@@ -268,29 +273,36 @@ expert_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
   if (threadIdx.x == 0 && abort_flag && error_word) atomicExch(error_word, 1);
 }
 
-// One block per slot of the grouped order; 16 bytes per thread and turn.
+// One block per token: its row is read once and written to the places of its slots; 16 bytes per thread and turn.
+// Slots whose choice is no stored expert have no row.
 __global__ void gather_slots_kernel(const bf16* __restrict__ h, long h_stride, const float* __restrict__ weights,
-                                    const int* __restrict__ order, const int* __restrict__ offsets, int E, int W, int top,
+                                    const int* __restrict__ chosen, const int* __restrict__ place, int E, int W, int top,
                                     bf16* __restrict__ xs) {
   pdl_wait();
   pdl_launch_dependents();
-  const int r = blockIdx.x;
-  if (r >= offsets[E]) return;  // choices that stand for no stored expert come last
-  const int slot = order[r];
-  const bf16* src = h + (long)(slot / top) * h_stride;
-  bf16* dst = xs + (long)r * W;
-  if (weights) {
-    const float w = weights[slot];
-    for (int i = threadIdx.x * 8; i < W; i += blockDim.x * 8) {
-      float v[8];
-      load8(src + i, v);
+  const long t = blockIdx.x;
+  const bf16* src = h + t * h_stride;
+  for (int i = threadIdx.x * 8; i < W; i += blockDim.x * 8) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(src + i);
+    const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&raw);
+    for (int k = 0; k < top; ++k) {
+      const long slot = t * top + k;
+      if (chosen[slot] >= E) continue;
+      bf16* dst = xs + (long)place[slot] * W + i;
+      if (weights) {
+        const float w = weights[slot];
+        float v[8];
 #pragma unroll
-      for (int x = 0; x < 8; ++x) v[x] *= w;
-      store8(dst + i, v);
+        for (int x = 0; x < 4; ++x) {
+          const float2 f = __bfloat1622float2(pairs[x]);
+          v[2 * x] = f.x * w;
+          v[2 * x + 1] = f.y * w;
+        }
+        store8(dst, v);
+      } else {
+        *reinterpret_cast<uint4*>(dst) = raw;
+      }
     }
-  } else {
-    for (int i = threadIdx.x * 8; i < W; i += blockDim.x * 8)
-      *reinterpret_cast<uint4*>(dst + i) = *reinterpret_cast<const uint4*>(src + i);
   }
 }
 
@@ -341,15 +353,16 @@ int launch(const void* w, long w_rows, const void* x, void* out, int S, int E, i
 
 }  // namespace
 
-// xs [S, W] bf16: row r is the token's row of slot order[r] (times weights[slot], fp32, if given).
-Q3_EXPORT int q3_expert_gather(const void* h, long h_stride, const float* weights, const int* order, const int* offsets,
-                               int S, int E, int W, int top, void* xs, cudaStream_t stream) {
-  if (!h || !order || !offsets || !xs || S < 0 || E < 1 || W < 1 || top < 1) return Q3_ERR_ARGUMENT;
+// xs [T * top, W] bf16: row place[slot] is the token's row of every slot with chosen[slot] < E (times weights[slot],
+// fp32, if given).
+Q3_EXPORT int q3_expert_gather(const void* h, long h_stride, const float* weights, const int* chosen, const int* place,
+                               int num_tokens, int E, int W, int top, void* xs, cudaStream_t stream) {
+  if (!h || !chosen || !place || !xs || num_tokens < 0 || E < 1 || W < 1 || top < 1) return Q3_ERR_ARGUMENT;
   if (W % 8 || h_stride % 8 || (((uintptr_t)h | (uintptr_t)xs) & 15)) return Q3_ERR_UNSUPPORTED;
-  if (S == 0) return Q3_OK;
+  if (num_tokens == 0) return Q3_OK;
   const int threads = W >= 2048 ? 256 : W >= 1024 ? 128 : 64;
-  return launch_pdl(gather_slots_kernel, dim3(S), dim3(threads), 0, stream, (const bf16*)h, h_stride, weights, order,
-                    offsets, E, W, top, (bf16*)xs) == cudaSuccess
+  return launch_pdl(gather_slots_kernel, dim3(num_tokens), dim3(threads), 0, stream, (const bf16*)h, h_stride, weights,
+                    chosen, place, E, W, top, (bf16*)xs) == cudaSuccess
              ? Q3_OK
              : Q3_ERR_LAUNCH;
 }

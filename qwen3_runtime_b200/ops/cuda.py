@@ -95,7 +95,7 @@ _SIGNATURES = {
     "experts": {
         "q3_route_top": [c_int, c_void_p, c_long, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                          c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p],
-        "q3_group_slots": [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
+        "q3_group_slots": [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
         "q3_expert_gate_up": [c_int, c_void_p, c_long, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p,
                               c_void_p, c_void_p, c_void_p, c_int, c_float, c_float, c_float, c_void_p],
         "q3_expert_down": [c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
@@ -219,7 +219,7 @@ _SIGNATURES = {
                                       c_int, c_float, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p],
     },
     "gemm_f32": {
-        "q3_gemm_f32": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
+        "q3_gemm_f32": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
     },
     "gemm_small_m": {
         "q3_gemm_small_m": [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
@@ -287,6 +287,7 @@ class CudaOps:
         self.tcgen05_pairs = True           # False: the tcgen05 product never pairs SMs (cta_group::1 only)
         self.fuse_decode_new_token = True   # False: always the separate q/k norm + rotation + store kernel
         self.latent_attention_tc = True     # False: attention over latent rows always on the general kernel
+        self.f32_tile = -1                  # which tile shape computes float32 products (-1: by their sizes; same bits)
         self.experts_tc = True              # False: the experts' products always on the FMA kernels
         self.chunk_tc = True                # False: attention under chunks or with turned values on the general kernel
         self.delta_chunks = True            # False: the delta rule's recurrence always token by token
@@ -1074,7 +1075,9 @@ class CudaOps:
         # identity experts are grouped like the stored ones (behind them); the products then stop at the stored
         # experts' last tile
         EA = E + num_identity
-        plan = torch.empty(2 * (EA + 1) + 2 * S, dtype=torch.int32, device=dev)
+        # offsets, tile offsets, order, places, and the grouping's scratch for many slots
+        scratch = S + -(-S // 1024) * EA if S > 512 else 0
+        plan = torch.empty(2 * (EA + 1) + 2 * S + scratch, dtype=torch.int32, device=dev)
         offsets, tile_offsets, order = plan[: EA + 1], plan[EA + 1: 2 * (EA + 1)], plan[2 * (EA + 1): 2 * (EA + 1) + S]
         on_input = weight_on == "input"
         # bfloat16 with 16-byte rows: the products run on the tensor cores (csrc/experts_tcgen05.cu).  Measured against
@@ -1085,8 +1088,9 @@ class CudaOps:
             return self._routed_experts_tc(h, chosen, weights if on_input else None, None if on_input else weights, gate_up,
                                            down, plan, EA, 2 if gated else 1, limit, alpha, up_offset, shared, shared_gate,
                                            num_identity)
+        self.launches += int(S > 512)  # two kernels
         self._call("experts", "q3_group_slots", "group_slots", _ptr(chosen), S, EA, 32, _ptr(offsets),
-                   _ptr(tile_offsets), _ptr(order), None)
+                   _ptr(tile_offsets), _ptr(order), None, _ptr(plan[2 * (EA + 1) + 2 * S:]) if scratch else None)
         mid = torch.empty((S, F), dtype=h.dtype, device=dev)
         y = torch.empty((S, W), dtype=h.dtype, device=dev)
         out = torch.empty((T, W), dtype=h.dtype, device=dev)
@@ -1123,16 +1127,18 @@ class CudaOps:
         S = T * top
         e = h.element_size()
         offsets, tile_offsets = plan[: EA + 1], plan[EA + 1: 2 * (EA + 1)]
-        order, place = plan[2 * (EA + 1): 2 * (EA + 1) + S], plan[2 * (EA + 1) + S:]
+        at = 2 * (EA + 1)
+        order, place, scratch = plan[at: at + S], plan[at + S: at + 2 * S], plan[at + 2 * S:]
+        self.launches += int(S > 512)  # two kernels
         self._call("experts", "q3_group_slots", "group_slots", _ptr(chosen), S, EA, 256, _ptr(offsets),
-                   _ptr(tile_offsets), _ptr(order), _ptr(place))
+                   _ptr(tile_offsets), _ptr(order), _ptr(place), _ptr(scratch) if S > 512 else None)
         rows = torch.empty((S, W), dtype=h.dtype, device=h.device)  # the slots' inputs, later their outputs
         mid = torch.empty((S, F), dtype=h.dtype, device=h.device)
         out = torch.empty((T, W), dtype=h.dtype, device=h.device)
         if self.timing is not None:
             self._costs((T + S) * W * e)
         self._call("experts_tcgen05", "q3_expert_gather", "expert_gather", _ptr(h), h.stride(0), _ptr(in_weights),
-                   _ptr(order), _ptr(offsets), S, E, W, top, _ptr(rows))
+                   _ptr(chosen), _ptr(place), T, E, W, top, _ptr(rows))
         err = _ptr(self._error_word(h.device))
         if self.timing is not None:
             self._costs((min(S, E) * unit * F * W + S * (W + F)) * e, 2.0 * unit * S * F * W, f" {S}x{W}->{unit}x{F}")
@@ -1737,7 +1743,7 @@ class CudaOps:
             if out is None:
                 out = torch.empty((M, N), dtype=torch.float32, device=x.device)
             self._call("gemm_f32", "q3_gemm_f32", "gemm_f32", _ptr(x), x.stride(0), _ptr(weight),
-                       weight.stride(0), _ptr(out), out.stride(0), M, N, K)
+                       weight.stride(0), _ptr(out), out.stride(0), M, N, K, self.f32_tile)
             return out
         if self._small_m_ok(x, weight):
             odt = out_dtype or x.dtype
