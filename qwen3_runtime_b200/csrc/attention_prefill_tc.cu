@@ -1,30 +1,40 @@
-// Causal attention of prompt portions over the paged cache on the 5th-generation tensor
-// cores: S = Q K^T and O += P V are tcgen05.mma with accumulators in tensor memory, Q, K and V
-// tiles arrive by TMA (128-byte swizzle) straight from the QKV buffer and the cache pages.
-// bfloat16, head_dim 128, group size a divisor of 128, page size 8/16/32/64, no window (a chunked mask,
-// turned values and sinks are options); the mma.sync kernels serve everything else.
+// Causal attention of prompt portions on the 5th-generation tensor cores: S = Q K^T and O += P V are tcgen05.mma
+// with accumulators in tensor memory; Q, K and V tiles arrive by TMA (128-byte swizzle).  bfloat16; three forms:
+//   PAGED    heads of 128 over the paged cache, straight from the QKV buffer and the pages (group size a divisor of 128,
+//            page size 8/16/32/64); options: a chunked mask, turned values, sinks;
+//   MAPS     differential attention: a head is two maps of 64 side by side in its 128 columns, over one value of 128;
+//            options: a chunked mask or a window;
+//   DENSE    keys of 192 = 128 of the head's own + 64 shared by the heads, values of 128, one key head per query head,
+//            from matrices that hold the keys and values of the step's sequences one after another (attention through
+//            a latent whose keys and values were expanded); options: a window, sinks.
+// The mma.sync kernels serve everything else.
 //
-// Work item: (sequence, kv head, two consecutive blocks of 128 rows, A and B); rows are the
-// (query token, head of the group) pairs in token-major order, so one 3-D TMA box
-// [128/G tokens, G heads, 64] is half a Q tile and the group's heads share every K/V tile.  Keys
-// come in tiles of 64 (64/page_size pages, one TMA box per page and half of D), and each tile
-// is used by both row blocks.  Per 64-key tile a row block's chain is long (TMEM load, exp2
-// on the special-function unit, shared-memory stores, fences, barrier round trips) and
-// leaves the tensor core and the exp2 unit idle most of the time; two blocks in flight hide
-// each other's chain.  Eleven warps:
-//   warp 0           : TMA producer (Q of both blocks once, then K and V tiles through 3-stage
-//                      rings; the lanes issue a tile's page boxes side by side);
+// Work item: (sequence, kv head, two row blocks A and B of 128 rows); rows are the (query token, head of the group) pairs in
+// token-major order, so one 3-D TMA box [128/G tokens, G heads, 64] is 64 columns of a Q tile and the group's heads share
+// every K/V tile.  PAGED and DENSE: A and B are consecutive blocks; MAPS: A and B are the two maps of the same rows.
+// Keys come in tiles of 64 (PAGED, MAPS: 64/page_size pages, one TMA box per page and 64 columns), and each tile is used
+// by both row blocks.  Per 64-key tile a row block's chain is long (TMEM load, exp2 on the special-function unit, TMEM
+// store, fences, barrier round trips) and leaves the tensor core and the exp2 unit idle most of the time; two blocks in
+// flight hide each other's chain.  Eleven warps:
+//   warp 0           : TMA producer (Q of both blocks once, then K and V tiles through rings of stages; the lanes issue a
+//                      tile's boxes side by side);
 //   warps 1 and 10,  : MMA issuers of block A and of block B.  Order per block: S_0, S_1, then
 //   one lane each      per tile j: P_j ready -> PV_j, S_(j+2).  S has two TMEM buffers per block,
 //                      so the tensor core works for one block while the other block's softmax
 //                      runs;
 //   warps 2..5, 6..9 : softmax of block A and of block B, one thread per row: reads S from
-//                      TMEM, masks, online softmax in fp32 (exp2, scale folded in), writes P
-//                      (bf16) to shared memory (two buffers per block) in the swizzled K-major
-//                      layout that the PV MMA reads; O stays in TMEM (the MMAs accumulate into
-//                      it) and is rescaled there only when a row's maximum has grown by more
-//                      than 2^8; finally stores O / l.
-// Tensor memory: all 512 columns, per block S0 [0,64), S1 [64,128), O [128,256).
+//                      TMEM, masks, online softmax in fp32 (exp2, scale folded in), writes P as bf16 over the first
+//                      32 columns of the S buffer that it came from, where the PV MMA reads it as its A operand; O stays
+//                      in TMEM (the MMAs accumulate into it) and is rescaled there only when a row's maximum has grown by
+//                      more than 2^8; finally stores O / l.  MAPS: block B's threads leave lambda O_B / l_B in shared
+//                      memory, block A's subtract it, divide by the root mean square and store.
+// Tensor memory: all 512 columns, per block S0 [0,64), S1 [64,128), O [128,256); P_j lies in S_j's columns.  S_(j+2) is
+// issued after PV_j by the same thread, and MMAs run in the order of issue, so it cannot overwrite P_j too early.
+// What bounds it: shared memory.  A QK step of 64 keys reads 6 KB per 32 cycles of MMA; with P in shared memory a tile and
+// block took about 900 cycles of its bandwidth against 512 of MMA and 512 of exp2, without it 640.  One layer of 2048 tokens,
+// 32 heads over 8: 49 us (57 with P in shared memory).  Forms: differential attention, 16 heads over 4, 2333 + 419 tokens: 61 us
+// (mma.sync: 247); latent, 16 heads, 2048 tokens, window 1024: 34 us and 26 us for the expansion (in the latent space on
+// mma.sync: 481).
 // V is the B operand of PV in MN-major form (rows = keys): descriptor with the halves of D
 // 8 KB apart (leading offset) and 8-key groups 1 KB apart (stride offset); 16 keys = 2 KB.
 // Keys past a block's last position are zeroed in shared memory before PV (stale or poisoned
@@ -34,17 +44,39 @@
 
 namespace {
 
-constexpr int D = 128;
+enum { PAGED = 0, MAPS = 1, DENSE = 2 };
+constexpr int D = 128;  // value size, and query/key size of PAGED and of both maps together
 constexpr int BLOCK_M = 128;
 constexpr int BLOCK_N = 64;
 constexpr int THREADS = 352;
-constexpr int Q_BYTES = BLOCK_M * D * 2;        // 32 KB: two halves of [128 rows][128 B]
-constexpr int KV_BYTES = BLOCK_N * D * 2;       // 16 KB: two halves of [64 rows][128 B]
-constexpr int P_BYTES = BLOCK_M * BLOCK_N * 2;  // 16 KB: [128 rows][128 B]
-constexpr int KV_STAGES = 3;                    // key tiles and value tiles in flight
-constexpr int SMEM_BYTES = 2 * Q_BYTES + 2 * KV_STAGES * KV_BYTES + 4 * P_BYTES + 1024;
+constexpr int HALF_Q = BLOCK_M * 128;           // 64 columns of a Q tile: [128 rows][128 B]
+constexpr int HALF_KV = BLOCK_N * 128;          // 64 columns of a K or V tile: [64 rows][128 B]
+constexpr int V_BYTES = 2 * HALF_KV;
 constexpr int TMEM_COLS = 512;                  // per row block: S0 [0,64), S1 [64,128), O [128,256)
 constexpr int TMEM_BLOCK = 256;
+
+template <int MODE>
+struct Sizes {
+  static constexpr int DK = MODE == DENSE ? 192 : 128;
+  static constexpr int Q_BYTES = DK / 64 * HALF_Q;
+  static constexpr int K_BYTES = DK / 64 * HALF_KV;
+  static constexpr int STAGES = MODE == DENSE ? 3 : 4;  // key tiles and value tiles in flight
+  static constexpr int SMEM = 2 * Q_BYTES + STAGES * (K_BYTES + V_BYTES) + 1024;
+};
+
+struct Params {
+  const int* block_table;
+  int max_pages;
+  const int *kv_lens, *cu_seqlens;
+  bf16* out;
+  int num_seqs, num_work, nq, nkv, ps;
+  float scale_log2;
+  int skip_single, chunk, window;
+  const float *turns, *sinks;
+  const int* kv_base;             // DENSE: key j of sequence s is row kv_base[s] + j
+  float lambda, eps, out_scale;   // MAPS
+  int* error_word;
+};
 
 // 2^x in one instruction (exp2f adds range fix-ups around the same instruction; results
 // below 2^-126 become zero here, which is what a probability that small is worth)
@@ -58,23 +90,24 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-enum { BAR_Q = 0, BAR_K_FULL = 1, BAR_K_EMPTY = BAR_K_FULL + KV_STAGES, BAR_V_FULL = BAR_K_EMPTY + KV_STAGES,
-       BAR_V_EMPTY = BAR_V_FULL + KV_STAGES, BAR_S_FULL = BAR_V_EMPTY + KV_STAGES,  // [block][buffer]
-       BAR_P_FULL = BAR_S_FULL + 4, BAR_PV_FULL = BAR_P_FULL + 2, NUM_BARS = BAR_PV_FULL + 2 };
-
+template <int MODE>
 __global__ void __launch_bounds__(THREADS, 1)
 prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                            const __grid_constant__ CUtensorMap tmap_v, const int* __restrict__ block_table,
-                            int max_pages, const int* __restrict__ kv_lens, const int* __restrict__ cu_seqlens,
-                            bf16* __restrict__ out, int num_seqs, int num_work, int nq, int nkv, int ps,
-                            float scale_log2, int skip_single, int chunk, const float* __restrict__ turns,
-                            const float* __restrict__ sinks, int* __restrict__ error_word) {
+                            const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_r,
+                            const __grid_constant__ Params p) {
+  typedef Sizes<MODE> Z;
+  constexpr int KV_STAGES = Z::STAGES, Q_BYTES = Z::Q_BYTES, K_BYTES = Z::K_BYTES, DK = Z::DK;
+  enum { BAR_Q = 0, BAR_K_FULL = 1, BAR_K_EMPTY = BAR_K_FULL + KV_STAGES, BAR_V_FULL = BAR_K_EMPTY + KV_STAGES,
+         BAR_V_EMPTY = BAR_V_FULL + KV_STAGES, BAR_S_FULL = BAR_V_EMPTY + KV_STAGES,  // [block][buffer]
+         BAR_P_FULL = BAR_S_FULL + 4, BAR_PV_FULL = BAR_P_FULL + 2, NUM_BARS = BAR_PV_FULL + 2 };
+  const int *block_table = p.block_table, *cu_seqlens = p.cu_seqlens;
+  const int max_pages = p.max_pages, nq = p.nq, nkv = p.nkv, ps = p.ps, chunk = p.chunk, window = p.window;
+  const float scale_log2 = p.scale_log2;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  unsigned char* q_s = base;                         // 2 blocks x [2 halves][128 rows][128 B]
-  unsigned char* k_s = q_s + 2 * Q_BYTES;            // KV_STAGES x [2 halves][64 rows][128 B]
-  unsigned char* v_s = k_s + KV_STAGES * KV_BYTES;   // KV_STAGES x [2 halves][64 rows][128 B]
-  unsigned char* p_s = v_s + KV_STAGES * KV_BYTES;   // 2 blocks x 2 buffers x [128 rows][128 B]
+  unsigned char* q_s = base;                         // 2 blocks x [DK / 64][128 rows][128 B]
+  unsigned char* k_s = q_s + 2 * Q_BYTES;            // KV_STAGES x [DK / 64][64 rows][128 B]
+  unsigned char* v_s = k_s + KV_STAGES * K_BYTES;    // KV_STAGES x [2 halves][64 rows][128 B]
   __shared__ __align__(8) unsigned long long bars[NUM_BARS];
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile int abort_flag;
@@ -91,11 +124,12 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
     abort_flag = 0;
     // heavy work (late rows of long prompts) first: walk the work list from its end
     int acc = 0, found = -1, rb = 0;
-    const int w = num_work - 1 - (int)(blockIdx.x / nkv);
-    for (int s = 0; s < num_seqs; ++s) {
+    const int w = p.num_work - 1 - (int)(blockIdx.x / nkv);
+    for (int s = 0; s < p.num_seqs; ++s) {
       const int ql = cu_seqlens[s + 1] - cu_seqlens[s];
-      if (ql <= 0 || (skip_single && ql == 1)) continue;
-      const int nb = ((ql * G + BLOCK_M - 1) / BLOCK_M + 1) / 2;  // pairs of row blocks
+      if (ql <= 0 || (p.skip_single && ql == 1)) continue;
+      int nb = (ql * G + BLOCK_M - 1) / BLOCK_M;  // row blocks
+      if (MODE != MAPS) nb = (nb + 1) / 2;        // pairs of them
       if (w < acc + nb) {
         found = s;
         rb = w - acc;
@@ -134,18 +168,19 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
   if (seq >= 0) {
     const int tok0 = cu_seqlens[seq];
     const int q_len = cu_seqlens[seq + 1] - tok0;
-    const int kv_len = kv_lens[seq];
+    const int kv_len = p.kv_lens[seq];
     const int rows = q_len * G;
     const int base_pos = kv_len - q_len;
     // row blocks A and B of this item; B may not exist (odd number of blocks)
     int row0[2], p_max[2], tiles[2];
-    // under a chunked mask the item's first visible key is that of its first row; tiles count from the tile it is in
-    const int p_first = base_pos + 2 * s_item[1] * BLOCK_M / G;
-    const int k_lo = chunk > 0 ? p_first / chunk * chunk : 0;
+    // under a chunked mask or a window the item's first visible key is that of its first row; tiles count from the tile
+    // it is in
+    const int p_first = base_pos + (MODE == MAPS ? 1 : 2) * s_item[1] * BLOCK_M / G;
+    const int k_lo = chunk > 0 ? p_first / chunk * chunk : (window > 0 ? max(0, p_first - window + 1) : 0);
     const int tile0 = k_lo / BLOCK_N;
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
-      row0[x] = (2 * s_item[1] + x) * BLOCK_M;
+      row0[x] = (MODE == MAPS ? s_item[1] : 2 * s_item[1] + x) * BLOCK_M;
       const bool live = row0[x] < rows;
       const int last_row = min(rows, row0[x] + BLOCK_M) - 1;
       p_max[x] = live ? base_pos + last_row / G : -1;
@@ -153,52 +188,72 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
     }
     const int num_tiles = max(tiles[0], tiles[1]);  // B lies after A, so this is B's count when B exists
     const int p_last = max(p_max[0], p_max[1]);
-    const int* bt = block_table + (long)seq * max_pages;
-    const int pages_per_tile = BLOCK_N / ps;
+    const int* bt = MODE == DENSE ? nullptr : block_table + (long)seq * max_pages;
+    const int pages_per_tile = MODE == DENSE ? 0 : BLOCK_N / ps;
 
     if (warp == 0) {  // ---- TMA producer: lane 0 waits and arms the barriers, the lanes share the loads ----
       if (lane == 0) {
-        mbar_expect_tx(bar(BAR_Q), tiles[1] ? 2 * Q_BYTES : Q_BYTES);
+        constexpr int BOXES = MODE == MAPS ? 1 : DK / 64;  // of a block; MAPS: map x is columns 64 x .. of the head
+        mbar_expect_tx(bar(BAR_Q), (tiles[1] ? 2 : 1) * BOXES * HALF_Q);
         for (int x = 0; x < 2; ++x) {
           if (!tiles[x]) continue;
-          const uint32_t dst = smem_addr(q_s) + x * Q_BYTES;
-          tma_load_3d(dst, &tmap_q, bar(BAR_Q), 0, kvh * G, tok0 + row0[x] / G);
-          tma_load_3d(dst + Q_BYTES / 2, &tmap_q, bar(BAR_Q), 64, kvh * G, tok0 + row0[x] / G);
+          for (int c = 0; c < BOXES; ++c) {
+            const bool turned = MODE == DENSE && c == 2;
+            tma_load_3d(smem_addr(q_s) + x * Q_BYTES + c * HALF_Q, turned ? &tmap_r : &tmap_q, bar(BAR_Q),
+                        turned ? 0 : 64 * (MODE == MAPS ? x : c), kvh * G, tok0 + row0[x] / G);
+          }
         }
       }
-      // a tile is 64 / ps pages x 2 halves of D: one box per lane (small boxes are slow to issue
-      // one after another from a single thread)
+      // PAGED, MAPS: a tile is 64 / ps pages x 2 halves of D, one box per lane (small boxes are slow to issue one after
+      // another from a single thread).  DENSE: five boxes of 64 rows (K: two of the head's own columns, one of the shared
+      // ones; V: two).
       const int my_page = lane >> 1, my_half = lane & 1;
+      const int row_base = MODE == DENSE ? p.kv_base[seq] : 0;
       int ok = 1;
       for (int j = 0; j < num_tiles && ok; ++j) {
         const int st = j % KV_STAGES;
         const uint32_t phase = (j / KV_STAGES) & 1;
-        // pages of this tile that exist in the block table (the rest of the tile is masked)
-        int page = -1;
-        if (my_page < pages_per_tile) {
-          const int pi = (tile0 + j) * pages_per_tile + my_page;
-          if (pi < max_pages && pi * ps <= p_last && (pi + 1) * ps > k_lo) page = bt[pi];
+        uint32_t k_bytes = K_BYTES, v_bytes = V_BYTES, off = 0;
+        int page = -1, y = 0;
+        if (MODE == DENSE) {
+          y = row_base + (tile0 + j) * BLOCK_N;
+        } else {
+          // pages of this tile that exist in the block table (the rest of the tile is masked)
+          if (my_page < pages_per_tile) {
+            const int pi = (tile0 + j) * pages_per_tile + my_page;
+            if (pi < max_pages && pi * ps <= p_last && (pi + 1) * ps > k_lo) page = bt[pi];
+          }
+          const uint32_t boxes = __popc(__ballot_sync(0xffffffffu, page >= 0));
+          k_bytes = v_bytes = boxes * (uint32_t)ps * 128u;
+          y = (page * nkv + kvh) * ps;
+          off = my_half * HALF_KV + my_page * ps * 128;
         }
-        const uint32_t boxes = __popc(__ballot_sync(0xffffffffu, page >= 0));
-        const uint32_t bytes = boxes * (uint32_t)ps * 128u;
-        const int y = (page * nkv + kvh) * ps;
-        const uint32_t off = st * KV_BYTES + my_half * (KV_BYTES / 2) + my_page * ps * 128;
         // keys
         if (lane == 0) {
           ok = mbar_wait(bar(BAR_K_EMPTY + st), phase ^ 1, &abort_flag);
-          if (ok) mbar_expect_tx(bar(BAR_K_FULL + st), bytes);
+          if (ok) mbar_expect_tx(bar(BAR_K_FULL + st), k_bytes);
         }
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) break;
-        if (page >= 0) tma_load_2d(smem_addr(k_s) + off, &tmap_k, bar(BAR_K_FULL + st), my_half * 64, y);
+        const uint32_t k_dst = smem_addr(k_s) + st * K_BYTES, v_dst = smem_addr(v_s) + st * V_BYTES;
+        if (MODE == DENSE) {
+          if (lane < 2) tma_load_2d(k_dst + lane * HALF_KV, &tmap_k, bar(BAR_K_FULL + st), kvh * D + lane * 64, y);
+          if (lane == 2) tma_load_2d(k_dst + 2 * HALF_KV, &tmap_v, bar(BAR_K_FULL + st), 0, y);
+        } else if (page >= 0) {
+          tma_load_2d(k_dst + off, &tmap_k, bar(BAR_K_FULL + st), my_half * 64, y);
+        }
         // values
         if (lane == 0) {
           ok = mbar_wait(bar(BAR_V_EMPTY + st), phase ^ 1, &abort_flag);
-          if (ok) mbar_expect_tx(bar(BAR_V_FULL + st), bytes);
+          if (ok) mbar_expect_tx(bar(BAR_V_FULL + st), v_bytes);
         }
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) break;
-        if (page >= 0) tma_load_2d(smem_addr(v_s) + off, &tmap_v, bar(BAR_V_FULL + st), my_half * 64, y);
+        if (MODE == DENSE) {  // the values lie beside the keys, behind those of all heads
+          if (lane < 2) tma_load_2d(v_dst + lane * HALF_KV, &tmap_k, bar(BAR_V_FULL + st), (nkv + kvh) * D + lane * 64, y);
+        } else if (page >= 0) {
+          tma_load_2d(v_dst + off, &tmap_v, bar(BAR_V_FULL + st), my_half * 64, y);
+        }
       }
     } else if (warp == 1 || warp == 10) {
       if (lane == 0) {  // ---- MMA issuers: warp 1 for block A, warp 10 for block B ------------------
@@ -210,7 +265,6 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
         const int my_tiles = tiles[x];
         constexpr uint32_t idesc_s = umma_idesc(BLOCK_M, BLOCK_N, 0);   // S = Q K^T: N = 64 keys
         constexpr uint32_t idesc_pv = umma_idesc(BLOCK_M, D, 1);        // PV: N = 128, V MN-major
-        const uint32_t p_addr = smem_addr(p_s) + 2 * x * P_BYTES;
         const uint32_t q_addr = smem_addr(q_s) + x * Q_BYTES;
         const uint32_t tmem_x = tmem + x * TMEM_BLOCK;
         // S_j into TMEM buffer j & 1, or just the hand-back of key tile j
@@ -222,12 +276,12 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
             return true;
           }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t k_addr = smem_addr(k_s) + st * KV_BYTES;
+          const uint32_t k_addr = smem_addr(k_s) + st * K_BYTES;
 #pragma unroll
-          for (int k = 0; k < D / 16; ++k) {
-            const uint32_t half = (k >> 2), sub = (k & 3) * 2;  // 4 steps of 32 bytes per 64-wide half
-            umma_bf16(tmem_x + sbuf * BLOCK_N, umma_desc(q_addr + half * (Q_BYTES / 2)) + sub,
-                 umma_desc(k_addr + half * (KV_BYTES / 2)) + sub, idesc_s, k > 0 ? 1u : 0u);
+          for (int k = 0; k < (MODE == MAPS ? 64 : DK) / 16; ++k) {
+            const uint32_t half = (k >> 2), sub = (k & 3) * 2;  // 4 steps of 32 bytes per 64 columns
+            umma_bf16(tmem_x + sbuf * BLOCK_N, umma_desc(q_addr + half * HALF_Q) + sub,
+                 umma_desc(k_addr + (MODE == MAPS ? x : half) * HALF_KV) + sub, idesc_s, k > 0 ? 1u : 0u);
           }
           umma_commit(bar(BAR_K_EMPTY + st));           // this block is done with the key tile
           umma_commit(bar(BAR_S_FULL + 2 * x + sbuf));  // S_j is in TMEM
@@ -245,17 +299,17 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
           if (!ok) break;
           if (j < my_tiles) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t v_addr = smem_addr(v_s) + st * KV_BYTES;
+            const uint32_t v_addr = smem_addr(v_s) + st * V_BYTES;
 #pragma unroll
-            for (int k = 0; k < BLOCK_N / 16; ++k)  // 16 keys: 32 bytes along P's rows, 2 KB down V's rows
-              umma_bf16(tmem_x + 2 * BLOCK_N, umma_desc(p_addr + pbuf * P_BYTES) + 2 * k,
-                   umma_desc_mn_major(v_addr + k * 2048, KV_BYTES / 2), idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < BLOCK_N / 16; ++k)  // 16 keys: 8 columns of P, 2 KB down V's rows
+              umma_bf16_tmem(tmem_x + 2 * BLOCK_N, tmem_x + pbuf * BLOCK_N + 8 * k,
+                   umma_desc_mn_major(v_addr + k * 2048, HALF_KV), idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
             umma_commit(bar(BAR_V_EMPTY + st));
             umma_commit(bar(BAR_PV_FULL + x));
           } else {
             mbar_arrive(bar(BAR_V_EMPTY + st));
           }
-          if (j + 2 < num_tiles) ok = keys(j + 2);  // its TMEM buffer (j & 1) was read before P_j was signalled
+          if (j + 2 < num_tiles) ok = keys(j + 2);  // its TMEM buffer held S_j and P_j: PV_j runs before it
         }
       }
     } else {  // ---- softmax: one thread per row; warps 2..5 block A, warps 6..9 block B ---------------
@@ -265,7 +319,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
       const int R = row0[x] + r;
       const bool row_ok = R < rows;
       const int pos = row_ok ? base_pos + R / G : -1;
-      const int lo = chunk > 0 && row_ok ? pos / chunk * chunk : 0;  // the row's first visible key
+      // the row's first visible key
+      const int lo = !row_ok ? 0 : (chunk > 0 ? pos / chunk * chunk : (window > 0 ? max(0, pos - window + 1) : 0));
       const int my_tiles = tiles[x];
       const uint32_t lane_base = tmem + x * TMEM_BLOCK + ((uint32_t)(quarter * 32) << 16);
       const uint32_t o_addr = lane_base + 2 * BLOCK_N;
@@ -295,7 +350,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
             if (key0 + 32 + c > pos) sb[c] = 0xff800000u;
           }
         }
-        if (key0 < lo) {  // keys of an earlier chunk
+        if (key0 < lo) {  // keys of an earlier chunk, or before the window
 #pragma unroll
           for (int c = 0; c < 32; ++c) {
             if (key0 + c < lo) sa[c] = 0xff800000u;
@@ -319,15 +374,14 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
         }
         const bool rescale = __any_sync(0xffffffffu, corr != 1.f) && j > 0;
         const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
-        // probabilities, rounded to bf16 as the MMA will see them, into the swizzled P tile; the
+        // probabilities, rounded to bf16 as the MMA will see them, over the scores in tensor memory; the
         // scaling and the row sum run on pairs of elements (packed fp32 instructions)
         float2 sums[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-        unsigned char* p_row = p_s + (2 * x + st) * P_BYTES + r * 128;  // buffer j & 1: PV_{j-1} may still read the other
+        uint32_t w[32];
         const float2 scale2 = make_float2(scale_log2, scale_log2);
         const float2 neg2 = make_float2(-m_use * scale_log2, -m_use * scale_log2);
 #pragma unroll
         for (int ch = 0; ch < 8; ++ch) {
-          uint32_t w[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int c = ch * 8 + 2 * e;
@@ -336,10 +390,10 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
             const float2 t2 = __ffma2_rn(s2, scale2, neg2);
             const float2 x2 = make_float2(ex2(t2.x), ex2(t2.y));
             sums[e] = __fadd2_rn(sums[e], x2);
-            w[e] = pack2(x2.x, x2.y);
+            w[ch * 4 + e] = pack2(x2.x, x2.y);
           }
-          *reinterpret_cast<uint4*>(p_row + ((ch ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
         }
+        tmem_store32(lane_base + st * BLOCK_N, w);
         {
           const float2 a = __fadd2_rn(sums[0], sums[1]), b = __fadd2_rn(sums[2], sums[3]);
           const float2 c = __fadd2_rn(a, b);
@@ -359,18 +413,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
               asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
               for (int c = 0; c < 32; ++c) ov[c] = __float_as_uint(__uint_as_float(ov[c]) * corr);
-              asm volatile(
-                  "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-                  "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-                  "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-                  ::"r"(o_addr + c0), "r"(ov[0]), "r"(ov[1]), "r"(ov[2]), "r"(ov[3]), "r"(ov[4]), "r"(ov[5]),
-                  "r"(ov[6]), "r"(ov[7]), "r"(ov[8]), "r"(ov[9]), "r"(ov[10]), "r"(ov[11]), "r"(ov[12]), "r"(ov[13]),
-                  "r"(ov[14]), "r"(ov[15]), "r"(ov[16]), "r"(ov[17]), "r"(ov[18]), "r"(ov[19]), "r"(ov[20]),
-                  "r"(ov[21]), "r"(ov[22]), "r"(ov[23]), "r"(ov[24]), "r"(ov[25]), "r"(ov[26]), "r"(ov[27]),
-                  "r"(ov[28]), "r"(ov[29]), "r"(ov[30]), "r"(ov[31])
-                  : "memory");
+              tmem_store32(o_addr + c0, ov);
             }
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
           }
         }
         // keys of this tile past the item's last position hold whatever the page held, keys before its first
@@ -381,22 +425,74 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
           if (!ok) break;
           const int vrow = r & 63, half = r >> 6;
           if (key0 + vrow > p_last || key0 + vrow < k_lo) {
-            uint4* dst = reinterpret_cast<uint4*>(v_s + vst * KV_BYTES + half * (KV_BYTES / 2) + vrow * 128);
+            uint4* dst = reinterpret_cast<uint4*>(v_s + vst * V_BYTES + half * HALF_KV + vrow * 128);
 #pragma unroll
             for (int ch = 0; ch < 8; ++ch) dst[ch] = make_uint4(0, 0, 0, 0);
           }
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // P (and zeroed V) visible to the MMA
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // zeroed V visible to the MMA
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         mbar_arrive(bar(BAR_P_FULL + x));
       }
       if (ok && my_tiles) ok = mbar_wait(bar(BAR_PV_FULL + x), (my_tiles - 1) & 1, &abort_flag);
-      if (ok && my_tiles) {
+      __syncwarp();
+      if constexpr (MODE == MAPS) {
+        // out = o / sqrt(mean(o^2) + eps) * out_scale, o = O_A / l_A - lambda O_B / l_B.  A row's 128 values pass from
+        // B's thread to A's through the Q tiles' shared memory (both blocks' products with Q are finished), 16 bytes at a
+        // time in places that differ between neighbouring rows.  All threads come here, also after an expired wait.
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const float inv = (x ? p.lambda : 1.f) / l_run;
+        float4* mine = reinterpret_cast<float4*>(q_s + r * 512);
+        asm volatile("bar.sync 2, 256;" ::: "memory");
+        if (x == 1) {
+#pragma unroll 1
+          for (int c0 = 0; c0 < D; c0 += 32) {
+            uint32_t ov[32];
+            tmem_load32(o_addr + c0, ov);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int c = 0; c < 32; c += 4)
+              mine[((c0 + c) >> 2) ^ (r & 31)] =
+                  make_float4(__uint_as_float(ov[c]) * inv, __uint_as_float(ov[c + 1]) * inv,
+                              __uint_as_float(ov[c + 2]) * inv, __uint_as_float(ov[c + 3]) * inv);
+          }
+        }
+        asm volatile("bar.sync 2, 256;" ::: "memory");
+        if (x == 0) {
+          float ss = 0.f;
+#pragma unroll 1
+          for (int c0 = 0; c0 < D; c0 += 32) {
+            uint32_t ov[32];
+            tmem_load32(o_addr + c0, ov);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int c = 0; c < 32; c += 4) {
+              float4* at = mine + (((c0 + c) >> 2) ^ (r & 31));
+              const float4 b = *at;
+              const float4 o = make_float4(__uint_as_float(ov[c]) * inv - b.x, __uint_as_float(ov[c + 1]) * inv - b.y,
+                                           __uint_as_float(ov[c + 2]) * inv - b.z, __uint_as_float(ov[c + 3]) * inv - b.w);
+              ss += o.x * o.x + o.y * o.y + o.z * o.z + o.w * o.w;
+              *at = o;
+            }
+          }
+          const float rstd = rsqrtf(ss / (float)D + p.eps) * p.out_scale;
+          if (ok && row_ok) {
+            bf16* dst = p.out + ((long)(tok0 + R / G) * nq + kvh * G + R % G) * D;
+#pragma unroll 4
+            for (int c = 0; c < D; c += 8) {
+              const float4 a = mine[(c >> 2) ^ (r & 31)], b = mine[((c >> 2) + 1) ^ (r & 31)];
+              const float v8[8] = {a.x * rstd, a.y * rstd, a.z * rstd, a.w * rstd, b.x * rstd, b.y * rstd, b.z * rstd, b.w * rstd};
+              store8(dst + c, v8);
+            }
+          }
+        }
+      } else if (ok && my_tiles) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // a head's sink: one more term in the denominator, in the units of the row's reference point
-        if (sinks && row_ok) l_run += exp2f(sinks[kvh * G + R % G] * LOG2_E - m_ref * scale_log2);
+        if (p.sinks && row_ok) l_run += exp2f(p.sinks[kvh * G + R % G] * LOG2_E - m_ref * scale_log2);
         const float inv = 1.f / l_run;
-        bf16* dst = row_ok ? out + ((long)(tok0 + R / G) * nq + kvh * G + R % G) * D : nullptr;
+        const float* turns = MODE == PAGED ? p.turns : nullptr;
+        bf16* dst = row_ok ? p.out + ((long)(tok0 + R / G) * nq + kvh * G + R % G) * D : nullptr;
         if (turns) {  // turned values: the sum is turned back, element c with element c + D / 2
           const float* cs = row_ok ? turns + (long)(tok0 + R / G) * D : nullptr;  // cos (D / 2), sin (D / 2)
 #pragma unroll 1
@@ -448,7 +544,40 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
   }
-  if (tid == 0 && abort_flag && error_word) atomicExch(error_word, 2);
+  if (tid == 0 && abort_flag && p.error_word) atomicExch(p.error_word, 2);
+}
+
+template <int MODE>
+int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tr, const Params& p,
+           cudaStream_t stream) {
+  static bool configured_on[Q3_MAX_DEVICES];
+  bool& configured = configured_on[q3_current_device()];
+  if (!configured) {
+    if (cudaFuncSetAttribute(prefill_attention_tc_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             Sizes<MODE>::SMEM) != cudaSuccess)
+      return Q3_ERR_LAUNCH;
+    configured = true;
+  }
+  prefill_attention_tc_kernel<MODE><<<dim3((unsigned)p.num_work * p.nkv), THREADS, Sizes<MODE>::SMEM, stream>>>(tq, tk, tv, tr, p);
+  return q3_launch_status();
+}
+
+// Q as [tokens][heads][columns]: boxes of 128 / G tokens x G heads x 64 columns
+bool q_map(CUtensorMap* map, const void* q, int cols, int nq, long num_tokens, long q_stride, int G) {
+  Q3EncodeTiledFn fn = q3_encode_tiled();
+  if (!fn) return false;
+  const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)nq, (cuuint64_t)num_tokens};
+  const cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)q_stride * 2};
+  const cuuint32_t box[3] = {64, (cuuint32_t)G, (cuuint32_t)(BLOCK_M / G)};
+  const cuuint32_t es[3] = {1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(q), dims, strides, box, es,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+bool paged_ok(const void* q, int q_stride, const void* kpages, const void* vpages, int nq, int nkv, int ps) {
+  return BLOCK_M % (nq / nkv) == 0 && (ps == 8 || ps == 16 || ps == 32 || ps == 64) && q_stride % 8 == 0 && nkv <= 65535 &&
+         (((uintptr_t)q | (uintptr_t)kpages | (uintptr_t)vpages) & 15) == 0;
 }
 
 }  // namespace
@@ -470,40 +599,68 @@ Q3_EXPORT int q3_paged_attention_prefill_tc(const void* q, int q_stride, int num
   if (chunk < 0 || ((uintptr_t)turns & 15)) return Q3_ERR_ARGUMENT;
   if (!q || !kpages || !vpages || !block_table || !kv_lens || !cu_seqlens || !out) return Q3_ERR_ARGUMENT;
   if (nq < 1 || nkv < 1 || nq % nkv) return Q3_ERR_ARGUMENT;
-  const int G = nq / nkv;
-  if (head_dim != D || BLOCK_M % G || (ps != 8 && ps != 16 && ps != 32 && ps != 64) || q_stride % 8 ||
-      nkv > 65535 || (((uintptr_t)q | (uintptr_t)kpages | (uintptr_t)vpages) & 15))
-    return Q3_ERR_UNSUPPORTED;
+  if (head_dim != D || !paged_ok(q, q_stride, kpages, vpages, nq, nkv, ps)) return Q3_ERR_UNSUPPORTED;
   if (num_work == 0) return Q3_OK;
-  Q3EncodeTiledFn fn = q3_encode_tiled();
-  if (!fn) return Q3_ERR_LAUNCH;
   CUtensorMap tq, tk, tv;
-  {
-    const cuuint64_t dims[3] = {(cuuint64_t)D, (cuuint64_t)nq, (cuuint64_t)num_tokens};
-    const cuuint64_t strides[2] = {(cuuint64_t)D * 2, (cuuint64_t)q_stride * 2};
-    const cuuint32_t box[3] = {64, (cuuint32_t)G, (cuuint32_t)(BLOCK_M / G)};
-    const cuuint32_t es[3] = {1, 1, 1};
-    if (fn(&tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(q), dims, strides, box, es,
-           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return Q3_ERR_LAUNCH;
-  }
   // pages as a matrix [rows of all pages and kv heads][D], read in boxes of one page x 64 dims
-  if (!q3_bf16_map(&tk, kpages, num_rows_kv, D, D, ps, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) ||
+  if (!q_map(&tq, q, D, nq, num_tokens, q_stride, nq / nkv) ||
+      !q3_bf16_map(&tk, kpages, num_rows_kv, D, D, ps, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) ||
       !q3_bf16_map(&tv, vpages, num_rows_kv, D, D, ps, CU_TENSOR_MAP_L2_PROMOTION_L2_128B))
     return Q3_ERR_LAUNCH;
-  static bool configured_on[Q3_MAX_DEVICES];
-  bool& configured = configured_on[q3_current_device()];
-  if (!configured) {
-    if (cudaFuncSetAttribute(prefill_attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) !=
-        cudaSuccess)
-      return Q3_ERR_LAUNCH;
-    configured = true;
-  }
-  dim3 grid((unsigned)num_work * nkv);
-  prefill_attention_tc_kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(tq, tk, tv, block_table, max_pages, kv_lens,
-                                                                    cu_seqlens, (bf16*)out, num_seqs, num_work, nq,
-                                                                    nkv, ps, scale * 1.4426950408889634f,
-                                                                    skip_single, chunk, turns, sinks, error_word);
-  return q3_launch_status();
+  const Params p = {block_table, max_pages, kv_lens, cu_seqlens, (bf16*)out, num_seqs, num_work, nq, nkv, ps,
+                    scale * LOG2_E, skip_single, chunk, 0, turns, sinks, nullptr, 0.f, 0.f, 0.f, error_word};
+  return launch<PAGED>(tq, tk, tv, tq, p, stream);
+}
+
+// Differential attention of every sequence of the step: query head h is [map 1 (64) | map 2 (64)] at column h * 128, key
+// pages hold both maps side by side, value pages the values of 128; out [num_tokens, nq, 128]: (a1 - lambda a2) divided by
+// its root mean square (eps inside the root), times out_scale.  num_work = sum over sequences of ceil(q_len * (nq / nkv) /
+// 128).  window or chunk > 0: the mask (not both).
+Q3_EXPORT int q3_diff_attention_prefill_tc(const void* q, int q_stride, int num_tokens, const void* kpages,
+                                           const void* vpages, long num_rows_kv, const int* block_table, int max_pages,
+                                           const int* kv_lens, const int* cu_seqlens, void* out, int num_seqs, int num_work,
+                                           int nq, int nkv, int ps, float scale, int window, int chunk, float lambda,
+                                           float eps, float out_scale, int* error_word, cudaStream_t stream) {
+  if (chunk < 0 || window < 0 || (chunk && window)) return Q3_ERR_ARGUMENT;
+  if (!q || !kpages || !vpages || !block_table || !kv_lens || !cu_seqlens || !out) return Q3_ERR_ARGUMENT;
+  if (nq < 1 || nkv < 1 || nq % nkv) return Q3_ERR_ARGUMENT;
+  if (!paged_ok(q, q_stride, kpages, vpages, nq, nkv, ps) || ((uintptr_t)out & 15)) return Q3_ERR_UNSUPPORTED;
+  if (num_work == 0) return Q3_OK;
+  CUtensorMap tq, tk, tv;
+  if (!q_map(&tq, q, D, nq, num_tokens, q_stride, nq / nkv) ||
+      !q3_bf16_map(&tk, kpages, num_rows_kv, D, D, ps, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) ||
+      !q3_bf16_map(&tv, vpages, num_rows_kv, D, D, ps, CU_TENSOR_MAP_L2_PROMOTION_L2_128B))
+    return Q3_ERR_LAUNCH;
+  const Params p = {block_table, max_pages, kv_lens, cu_seqlens, (bf16*)out, num_seqs, num_work, nq, nkv, ps,
+                    scale * LOG2_E, 0, chunk, window, nullptr, nullptr, nullptr, lambda, eps, out_scale, error_word};
+  return launch<MAPS>(tq, tk, tv, tq, p, stream);
+}
+
+// Attention over expanded keys and values: q [num_tokens, heads, q_cols] with row stride q_stride, of which the first 128
+// columns of a head are read; q_turned [num_tokens, heads, 64] dense: a head's part for the keys' shared columns; kv
+// [rows, 2 * heads * 128]: the heads' own 128 key columns, then the heads' values; shared [rows, *] with row stride
+// shared_stride: the 64 key columns that all heads share; key j of sequence s is row kv_base[s] + j (tiles of 64 keys are
+// read from multiples of 64 on, the first one that holds the sequence's first visible key).  out [num_tokens, heads, 128].
+// num_work = sum over sequences of ceil(ceil(q_len / 128) / 2).
+Q3_EXPORT int q3_dense_attention_prefill_tc(const void* q, int q_cols, int q_stride, const void* q_turned, int num_tokens,
+                                            const void* kv, const void* shared, long rows, long shared_stride,
+                                            const int* kv_base, const int* kv_lens, const int* cu_seqlens, void* out,
+                                            int num_seqs, int num_work, int heads, float scale, int window,
+                                            const float* sinks, int* error_word, cudaStream_t stream) {
+  if (!q || !q_turned || !kv || !shared || !kv_base || !kv_lens || !cu_seqlens || !out || heads < 1 || window < 0 || rows < 1 ||
+      q_cols < D)
+    return Q3_ERR_ARGUMENT;
+  if (q_cols % 8 || q_stride % 8 || shared_stride % 8 ||
+      (((uintptr_t)q | (uintptr_t)q_turned | (uintptr_t)kv | (uintptr_t)shared | (uintptr_t)out) & 15))
+    return Q3_ERR_UNSUPPORTED;
+  if (num_work == 0) return Q3_OK;
+  const long cols = 2L * heads * D;
+  CUtensorMap tq, tk, tv, tr;
+  if (!q_map(&tq, q, q_cols, heads, num_tokens, q_stride, 1) || !q_map(&tr, q_turned, 64, heads, num_tokens, 64L * heads, 1) ||
+      !q3_bf16_map(&tk, kv, rows, cols, cols, BLOCK_N, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) ||
+      !q3_bf16_map(&tv, shared, rows, 64, shared_stride, BLOCK_N, CU_TENSOR_MAP_L2_PROMOTION_L2_128B))
+    return Q3_ERR_LAUNCH;
+  const Params p = {nullptr, 0, kv_lens, cu_seqlens, (bf16*)out, num_seqs, num_work, heads, heads, BLOCK_N,
+                    scale * LOG2_E, 0, 0, window, nullptr, sinks, kv_base, 0.f, 0.f, 0.f, error_word};
+  return launch<DENSE>(tq, tk, tv, tr, p, stream);
 }

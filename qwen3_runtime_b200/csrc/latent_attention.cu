@@ -180,6 +180,52 @@ Q3_EXPORT int q3_rotate_heads(int dtype, const void* x, long xs_t, long xs_h, vo
   return q3_launch_status();
 }
 
+// ---- the cached rows of a step's sequences, side by side ------------------------------------------
+// Sequence s keeps its rows from key first_s on, first_s = the multiple of 64 at or before the first key that its first
+// new token sees; row kv_base[s] + j of `rows` is key j.  One warp per row, 16 bytes a lane and turn.
+__global__ void __launch_bounds__(256)
+latent_gather_kernel(const uint4* __restrict__ pages, int chunks, const int* __restrict__ block_table, int max_pages,
+                     const int* __restrict__ kv_lens, const int* __restrict__ cu_seqlens, int num_seqs, int ps, int window,
+                     uint4* __restrict__ rows, int* __restrict__ kv_base, int num_rows) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int r = blockIdx.x * 8 + warp;
+  int at = 0, seq = -1, key = 0;
+  for (int s = 0; s < num_seqs; ++s) {
+    const int kv = kv_lens[s], n = cu_seqlens[s + 1] - cu_seqlens[s];
+    const int first = window > 0 ? max(0, kv - n - window + 1) / 64 * 64 : 0;
+    if (r == 0 && lane == 0) kv_base[s] = at - first;
+    if (seq < 0 && r < at + kv - first) {
+      seq = s;
+      key = first + r - at;
+      if (r != 0) break;
+    }
+    at += kv - first;
+  }
+  if (r >= num_rows || seq < 0) return;
+  const int page = block_table[(long)seq * max_pages + key / ps];
+  uint4* dst = rows + (long)r * chunks;
+  const uint4* src = pages + ((long)page * ps + key % ps) * chunks;
+  for (int c = lane; c < chunks; c += 32) dst[c] = page >= 0 ? src[c] : make_uint4(0, 0, 0, 0);
+}
+
+// pages: [*, ps, width] bf16 of rows of a multiple of 16 bytes; rows: [num_rows, width]; num_rows = sum over the sequences
+// of kv_len - first (see above); kv_base: int32 [num_seqs].
+Q3_EXPORT int q3_latent_gather(const void* pages, int width, const int* block_table, int max_pages, const int* kv_lens,
+                               const int* cu_seqlens, int num_seqs, int ps, int window, void* rows, int* kv_base, int num_rows,
+                               cudaStream_t stream) {
+  if (!pages || !block_table || !kv_lens || !cu_seqlens || !rows || !kv_base || ps < 1 || num_seqs < 1 || num_rows < 1 ||
+      window < 0)
+    return Q3_ERR_ARGUMENT;
+  if (width % 8 || (((uintptr_t)pages | (uintptr_t)rows) & 15)) return Q3_ERR_UNSUPPORTED;
+  return launch_pdl(latent_gather_kernel, dim3((num_rows + 7) / 8), dim3(256), 0, stream, (const uint4*)pages, width / 8,
+                    block_table, max_pages, kv_lens, cu_seqlens, num_seqs, ps, window, (uint4*)rows, kv_base,
+                    num_rows) == cudaSuccess
+             ? Q3_OK
+             : Q3_ERR_LAUNCH;
+}
+
 // ---- attention over latent rows, any sizes -------------------------------------------------------
 // One block per (token, group of up to WARPS heads); one warp per head.  The query at absolute
 // position p sees rows lo..p of its sequence (lo = p - window + 1 with a window, else 0).  Rows are

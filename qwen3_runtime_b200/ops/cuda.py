@@ -79,6 +79,8 @@ _SIGNATURES = {
                                       c_int, c_void_p, c_int, c_float, c_void_p],
         "q3_rotate_heads": [c_int, c_void_p, c_long, c_long, c_void_p, c_long, c_long, c_void_p, c_void_p, c_int,
                             c_int, c_int, c_int, c_int, c_float, c_void_p],
+        "q3_latent_gather": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p,
+                             c_int, c_void_p],
         "q3_latent_attention": [c_int, c_void_p, c_long, c_long, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p,
                                 c_void_p, c_void_p, c_void_p, c_long, c_long, c_int, c_int, c_int, c_float, c_int,
                                 c_void_p],
@@ -209,6 +211,12 @@ _SIGNATURES = {
         "q3_paged_attention_prefill_tc": [c_void_p, c_int, c_int, c_void_p, c_void_p, ctypes.c_long, c_void_p, c_int,
                                           c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                           c_float, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
+        "q3_diff_attention_prefill_tc": [c_void_p, c_int, c_int, c_void_p, c_void_p, c_long, c_void_p, c_int, c_void_p,
+                                         c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int,
+                                         c_float, c_float, c_float, c_void_p, c_void_p],
+        "q3_dense_attention_prefill_tc": [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_long, c_long,
+                                          c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int,
+                                          c_void_p, c_void_p, c_void_p],
     },
     "attention_chunk": {
         "q3_chunk_attention_prefill": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
@@ -291,6 +299,8 @@ class CudaOps:
         self.experts_tc = True              # False: the experts' products always on the FMA kernels
         self.chunk_tc = True                # False: attention under chunks or with turned values on the general kernel
         self.delta_chunks = True            # False: the delta rule's recurrence always token by token
+        self.latent_expand = True           # False: prompts never expand the latent's keys and values
+        self.differential_tcgen05 = True    # False: differential attention never on the tcgen05 kernel
         self.differential_tc = True         # False: differential attention always on the general kernel
         self._tickets: torch.Tensor | None = None
         self._argmax_tickets: torch.Tensor | None = None
@@ -1006,6 +1016,58 @@ class CudaOps:
                    float(scale), int(window or 0))
         return out
 
+    # (query, key) pairs per cached row from which a step's prompts expand the keys and values (see latent_expand_rows)
+    LATENT_EXPAND_PAIRS = 32
+
+    def latent_expand_rows(self, step, *, dim, rot_dim, value_dim, kv_rank, window, dtype) -> int:
+        """How many cached rows :meth:`latent_attention_expanded` would expand for this step, or 0 where attention in the
+        latent space is the better one (or the only one).  A pair costs 2 x (kv_rank + rot_dim + kv_rank) flops in the
+        latent space (1088 products) against 320 with keys of 192 and values of 128, on a kernel that also runs at three
+        times the rate; expanding a row costs 2 x kv_rank x 256 flops per head once, however many queries see it."""
+        if not (self.latent_expand and step is not None and dtype == torch.bfloat16 and not step.decode_only
+                and not step.captured_width and (dim, rot_dim, value_dim) == (128, 64, 128) and kv_rank % 8 == 0):
+            return 0
+        rows = pairs = 0
+        cu = step.host_cu_seqlens
+        for b, kv in enumerate(step.host_kv_lens):
+            n = cu[b + 1] - cu[b]
+            rows += kv - (max(0, kv - n - window + 1) // 64 * 64 if window else 0)
+            full = min(n, max(0, kv - window)) if window else 0  # tokens that see a whole window
+            pairs += full * window if full else 0
+            pairs += (n - full) * (kv - n) + (n - full) * (n - full + 1) // 2
+        return rows if pairs >= self.LATENT_EXPAND_PAIRS * rows else 0
+
+    def latent_attention_expanded(self, q, q_turned, expand, rows, *, pages, kv_rank, block_table, sink, out, page_size, scale,
+                                  window, step):
+        """Attention of a step's prompts over cached rows ``[latent (kv_rank) | turned key part (64)]`` with keys and
+        values expanded: ``expand`` ``[2 * H * 128, kv_rank]`` makes the heads' key columns, then the heads' values, of the
+        ``rows`` rows the step's tokens see (:meth:`latent_expand_rows`); ``q`` ``[T, H, >= 128]`` (the first 128 columns of
+        a head), ``q_turned`` dense ``[T, H, 64]``, ``out`` dense ``[T, H, 128]``."""
+        T, H, _ = q.shape
+        width = pages.shape[-1]
+        qs = self._head_strides(q, "latent_attention_expanded")
+        if not (pages.is_contiguous() and out.is_contiguous() and q_turned.is_contiguous()
+                and q_turned.shape == (T, H, 64) and out.shape == (T, H, 128)):
+            raise KernelError("latent_attention_expanded: dense pages, turned queries [T, H, 64] and output [T, H, 128]")
+        dev = out.device
+        seen = torch.empty((rows, width), dtype=out.dtype, device=dev)
+        base = torch.empty(step.num_seqs, dtype=torch.int32, device=dev)
+        if self.timing is not None:
+            self._costs(2 * rows * width * out.element_size())
+        self._call("latent_attention", "q3_latent_gather", "latent_gather", _ptr(pages), width, _ptr(block_table),
+                   block_table.shape[1], _ptr(step.kv_lens), _ptr(step.cu_seqlens), step.num_seqs, page_size,
+                   int(window or 0), _ptr(seen), _ptr(base), rows)
+        kv = self.linear(seen[:, :kv_rank], expand)
+        cu = step.host_cu_seqlens
+        work = sum(-(-(-(-(cu[b + 1] - cu[b]) // 128)) // 2) for b in range(step.num_seqs) if cu[b + 1] > cu[b])
+        if self.timing is not None:
+            self._costs((rows * (2 * H * 128 + 64) + T * H * 320) * out.element_size())
+        self._call("attention_prefill_tc", "q3_dense_attention_prefill_tc", "latent_attention_expanded", _ptr(q), qs[1], qs[0],
+                   _ptr(q_turned), T, _ptr(kv), seen.data_ptr() + 2 * kv_rank, rows, width, _ptr(base), _ptr(step.kv_lens),
+                   _ptr(step.cu_seqlens), _ptr(out), step.num_seqs, work, H, float(scale), int(window or 0), _ptr(sink),
+                   _ptr(self._error_word(dev)))
+        return out
+
     # ---- routed experts (csrc/experts.cu) --------------------------------------------------------
     def route_top(self, h, router, top, renormalize=False, score="sigmoid", correction=None, groups=None, scale=1.0):
         """``(chosen int32 [T, top], weights float32 [T, top])``: the float32 router product, the
@@ -1533,6 +1595,19 @@ class CudaOps:
                            _ptr(step.kv_lens), _ptr(step.cu_seqlens), _ptr(out), out.stride(0), _ptr(mid),
                            step.num_seqs, num_heads, num_kv_heads, map_dim, value_dim, page_size, float(scale),
                            int(window or 0), int(chunk or 0), splits, float(lam), float(eps), float(out_scale))
+                return out
+            if (self.differential_tcgen05 and map_dim == 64 and value_dim == 128 and 128 % group == 0
+                    and page_size in (8, 16, 32, 64) and out.stride(0) == num_heads * value_dim
+                    and not (window and chunk) and all(t.data_ptr() % 16 == 0 for t in (out, k_pages, v_pages))):
+                # both maps as the two row blocks of the tcgen05 kernel.  Against the mma.sync kernel below: 16 heads over 4,
+                # 2333 + 419 tokens 61 against 247 us
+                cu = step.host_cu_seqlens
+                work = sum(-(-(cu[b + 1] - cu[b]) * group // 128) for b in range(step.num_seqs) if cu[b + 1] > cu[b])
+                self._call("attention_prefill_tc", "q3_diff_attention_prefill_tc", "differential_attention_tc", _ptr(q),
+                           q_stride, T, _ptr(k_pages), _ptr(v_pages), k_pages.shape[0] * num_kv_heads * page_size,
+                           _ptr(block_table), block_table.shape[1], _ptr(step.kv_lens), _ptr(step.cu_seqlens), _ptr(out),
+                           step.num_seqs, work, num_heads, num_kv_heads, page_size, float(scale), int(window or 0),
+                           int(chunk or 0), float(lam), float(eps), float(out_scale), _ptr(self._error_word(out.device)))
                 return out
             if map_dim in (32, 64, 128) and value_dim in (64, 128):
                 cu = step.host_cu_seqlens

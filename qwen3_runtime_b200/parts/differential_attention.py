@@ -70,7 +70,8 @@ class DifferentialAttention(Part):
 
     def kernel_groups(self):
         groups = ["rope_kv", "attention_generic"]
-        groups += ["gemm_f32"] if self.ctx.dtype == torch.float32 else ["gemm_small_m", "gemm_stream", "attention_diff"]
+        groups += ["gemm_f32"] if self.ctx.dtype == torch.float32 else ["gemm_small_m", "gemm_stream", "attention_diff",
+                                                                             "attention_prefill_tc"]
         return groups
 
     def cache_spec(self):

@@ -60,7 +60,7 @@ class LatentAttention(Part):
         self.pairing = getattr(self.position, "pairing", "interleaved")
         self.magnitude = float(getattr(self.position, "magnitude", 1.0))
         self.starts: list[int] = []
-        self.down_weight = self.uq_weight = self.uk_t = self.uv = self.o_weight = None
+        self.down_weight = self.uq_weight = self.uk_t = self.uv = self.expand = self.o_weight = None
         self.q_norm_weight = self.kv_norm_weight = self.sink = None
 
     def param_specs(self):
@@ -99,9 +99,16 @@ class LatentAttention(Part):
         self.uk_t = tensors["uk"].reshape(H, self.dim, self.kv_rank).transpose(1, 2).contiguous()
         self.uv = tensors["uv"].reshape(H, self.vdim, self.kv_rank).contiguous()
         self.o_weight = tensors["o"].contiguous()
+        # keys and values of all heads from a latent, for prompts (ops.latent_expand_rows)
+        self.expand = torch.cat([tensors["uk"], tensors["uv"]], dim=0).contiguous() if self._expands() else None
         self.q_norm_weight = tensors.get("dq.norm")
         self.kv_norm_weight = tensors["dkv.norm"]
         self.sink = tensors.get("sink")
+
+    def _expands(self) -> bool:
+        """Whether a prompt's attention can run on expanded keys and values (bfloat16, the sizes of that kernel)."""
+        return (self.ctx.dtype == torch.bfloat16 and (self.dim, self.rot_dim, self.vdim) == (128, 64, 128)
+                and self.kv_rank % 8 == 0 and hasattr(self.ops, "latent_expand_rows"))
 
     def kernel_groups(self):
         groups = ["latent_attention", "head_gemm", *self.position.kernel_groups()]
@@ -111,6 +118,8 @@ class LatentAttention(Part):
             groups += ["gemm_small_m", "gemm_stream"]
             if self.row_width % 16 == 0 and self.kv_rank % 16 == 0 and self.kv_rank <= 512:
                 groups.append("latent_attention_tc")
+            if self._expands():
+                groups.append("attention_prefill_tc")
         return groups
 
     def cache_spec(self):
@@ -145,17 +154,28 @@ class LatentAttention(Part):
                 positions=step.positions, token_seq=step.token_seq, block_table=block_table,
                 pages=cache.latent_pages, page_size=cache.page_size, write=cache.writes, q_out=None, **turn)
             q = down[:, : H * (self.dim + self.rot_dim)].view(T, H, self.dim + self.rot_dim)
-        q_lat = torch.empty((T, H, self.row_width), dtype=h.dtype, device=h.device)
-        ops.head_linear(q[:, :, : self.dim], self.uk_t, q_lat[:, :, : self.kv_rank])
-        ops.rotate_heads(q[:, :, self.dim:], q_lat[:, :, self.kv_rank:], positions=step.positions, inv_freq=inv_freq,
-                         **turn)
-        attended = torch.empty((T, H, self.kv_rank), dtype=h.dtype, device=h.device)
-        ops.latent_attention(
-            q_lat, pages=cache.latent_pages, value_dim=self.kv_rank, block_table=block_table,
-            token_seq=step.token_seq, positions=step.positions, sink=self.sink, out=attended,
-            page_size=cache.page_size, scale=self.scale, window=self.window, step=step)
         ctx_out = torch.empty((T, H, self.vdim), dtype=h.dtype, device=h.device)
-        ops.head_linear(attended, self.uv, ctx_out)
+        seen = 0
+        if self.expand is not None:
+            seen = ops.latent_expand_rows(step, dim=self.dim, rot_dim=self.rot_dim, value_dim=self.vdim, kv_rank=self.kv_rank,
+                                          window=self.window, dtype=h.dtype)
+        if seen:
+            q_turned = torch.empty((T, H, self.rot_dim), dtype=h.dtype, device=h.device)
+            ops.rotate_heads(q[:, :, self.dim:], q_turned, positions=step.positions, inv_freq=inv_freq, **turn)
+            ops.latent_attention_expanded(
+                q, q_turned, self.expand, seen, pages=cache.latent_pages, kv_rank=self.kv_rank, block_table=block_table,
+                sink=self.sink, out=ctx_out, page_size=cache.page_size, scale=self.scale, window=self.window, step=step)
+        else:
+            q_lat = torch.empty((T, H, self.row_width), dtype=h.dtype, device=h.device)
+            ops.head_linear(q[:, :, : self.dim], self.uk_t, q_lat[:, :, : self.kv_rank])
+            ops.rotate_heads(q[:, :, self.dim:], q_lat[:, :, self.kv_rank:], positions=step.positions, inv_freq=inv_freq,
+                             **turn)
+            attended = torch.empty((T, H, self.kv_rank), dtype=h.dtype, device=h.device)
+            ops.latent_attention(
+                q_lat, pages=cache.latent_pages, value_dim=self.kv_rank, block_table=block_table,
+                token_seq=step.token_seq, positions=step.positions, sink=self.sink, out=attended,
+                page_size=cache.page_size, scale=self.scale, window=self.window, step=step)
+            ops.head_linear(attended, self.uv, ctx_out)
         if self.gate:
             g0 = self.starts[2]
             ops.sigmoid_mul(ctx_out.view(T, H * self.vdim), down[:, g0: g0 + H * self.vdim])

@@ -1,0 +1,165 @@
+"""The forms of the tcgen05 prompt kernel beside plain heads (csrc/attention_prefill_tc.cu): both maps of differential
+attention as its two row blocks, and attention through a latent on expanded keys and values; against the other kernels of
+the same parts, over group sizes, page sizes, masks, portions behind a context, one-token portions and ragged ends."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from qwen3_runtime_b200.ops.cuda import CudaOps
+
+    return CudaOps()
+
+
+def _layer(ops, spec, page, slots, pages, seed):
+    """A mixer with random tensors, and what it needs for steps of its own."""
+    from qwen3_runtime_b200.cache.layout import CacheLayout
+    from qwen3_runtime_b200.cache.manager import CacheManager
+    from qwen3_runtime_b200.cache.storage import CacheStorage
+    from qwen3_runtime_b200.engine.batch import BatchBuilder
+    from qwen3_runtime_b200.parts.base import BuildContext, build_part
+
+    part = build_part("mixer", spec, BuildContext(dtype=torch.bfloat16, device=torch.device(DEV), ops=ops))
+    g = torch.Generator().manual_seed(seed)
+    tensors = {}
+    for name, ps in part.param_specs().items():
+        t = torch.randn(ps.shape, generator=g)
+        if ps.kind == "vector":
+            t = 0.1 * t if name[:2] in ("lq", "lk") else 1.0 + 0.1 * t
+            tensors[name] = t.cuda()
+        else:
+            tensors[name] = (t * ps.shape[-1] ** -0.5).bfloat16().cuda()
+    part.load(tensors)
+    layout = CacheLayout({0: part.cache_spec()})
+    cache = CacheManager(layout.group_specs, page, pages, slots)
+    storage = CacheStorage(layout, page, cache.num_pages, slots, torch.bfloat16, DEV)
+    return part, cache, storage, BatchBuilder(cache, DEV, vocab_size=10, max_positions=1 << 20)
+
+
+def _steps(ops, spec, page, portions, variants, seed=0):
+    """Runs ``portions`` (a list of steps, each a list of tokens per request; 0: the request sits the step out) once per
+    variant (a function that prepares ``ops``); pages that nothing was written to hold NaN.  The variants' outputs."""
+    from qwen3_runtime_b200.engine.batch import StepEntry
+
+    results = []
+    for prepare in variants:
+        total = [sum(s[i] for s in portions) for i in range(len(portions[0]))]
+        part, cache, storage, builder = _layer(ops, spec, page, len(total), sum(-(-n // page) for n in total) + 3, seed)
+        for t in storage.tensors:
+            for x in t if isinstance(t, tuple) else (t,):
+                x.fill_(float("nan"))
+        handles = [cache.open(i) for i in range(len(total))]
+        g = torch.Generator().manual_seed(seed + 1)
+        out = []
+        for step_tokens in portions:
+            entries = []
+            for rc, n in zip(handles, step_tokens):
+                if n:
+                    cache.reserve(rc, n)
+                    entries.append(StepEntry(rc, [0] * n, []))
+            step = builder.build(entries, scratch_page=storage.scratch_page, scratch_slot=storage.scratch_slot)
+            h = torch.randn((step.num_tokens, int(spec["hidden_size"])), generator=g).bfloat16().cuda()
+            restore = prepare(ops)
+            try:
+                out.append(part.forward(h, step, storage.view(0)).float())
+            finally:
+                restore()
+            ops.raise_if_kernel_error()
+            for e in entries:
+                cache.commit(e.cache, len(e.tokens))
+        results.append(out)
+    return results
+
+
+def _set(**values):
+    def prepare(ops):
+        before = {k: getattr(ops, k) for k in values}
+        for k, v in values.items():
+            setattr(ops, k, v)
+
+        def restore():
+            for k, v in before.items():
+                setattr(ops, k, v)
+
+        return restore
+
+    return prepare
+
+
+def _close(got, want, factor):
+    for a, b in zip(got, want):
+        assert bool(torch.isfinite(a).all())
+        # factor roundings of bfloat16 (2^-9 of the value) that the two ways do not share, on the output's largest value
+        assert float((a - b).abs().max()) <= factor * 2.0 ** -9 * float(b.abs().max())
+        assert float((a - b).norm()) <= 0.5 * factor * 2.0 ** -9 * float(b.norm())
+
+
+RAGGED = [[3, 200, 0, 1, 65], [129, 1, 300, 70, 64], [1, 31, 33, 256, 2]]
+
+
+@pytest.mark.parametrize("heads,kv_heads,page", [(4, 4, 16), (4, 2, 8), (8, 2, 32), (16, 2, 64), (16, 1, 16)])
+@pytest.mark.parametrize("mask", [dict(), dict(chunk=100), dict(chunk=64), dict(window=1), dict(window=90)])
+def test_both_maps_as_row_blocks(ops, heads, kv_heads, page, mask):
+    from qwen3_runtime_b200.config import PartSpec
+
+    spec = PartSpec("differential_attention", dict(hidden_size=128, num_heads=heads, num_kv_heads=kv_heads, dim=64, vdim=128,
+                                                   scale=0.3, diff=0.4, eps=1e-5, **mask))
+    launched = []
+    call = ops._call
+
+    def spy(group, name, what, *args):
+        launched.append(name)
+        return call(group, name, what, *args)
+
+    ops._call = spy
+    try:
+        got, want = _steps(ops, spec, page, RAGGED, [_set(), _set(differential_tc=False)])
+    finally:
+        del ops._call
+    assert launched.count("q3_diff_attention_prefill_tc") == len(RAGGED) and "q3_paged_attention_diff" in launched
+    # probabilities are rounded to bfloat16 here and not in the general kernel, and the subtraction of the two maps lifts
+    # that rounding by up to (1 + lambda) / |1 - lambda| (about 4 for lambda near 0.4 .. 0.6)
+    _close(got, want, 12)
+
+
+@pytest.mark.parametrize("heads,q_rank,gate,pairing,page", [(2, 64, None, "interleaved", 16), (3, 0, "sigmoid", "half", 8),
+                                                          (16, 96, None, "interleaved", 64)])
+@pytest.mark.parametrize("window", [None, 1, 64, 90, 300])
+@pytest.mark.parametrize("kv_rank", [64, 512])
+def test_expanded_keys_and_values(ops, heads, q_rank, gate, pairing, page, window, kv_rank):
+    from qwen3_runtime_b200.config import PartSpec
+
+    position = (PartSpec("rope_interleaved", dict(rotary_dim=64, theta=1e4)) if pairing == "interleaved" else
+                PartSpec("rotary_scaled", dict(rotary_dim=64, theta=1e4, pairing="half",
+                                               scaling=dict(kind="ramp", factor=8.0, original=512.0, fast=32.0, slow=1.0))))
+    spec = PartSpec("latent_attention", dict(hidden_size=128, num_heads=heads, dim=128, rot_dim=64, vdim=128, q_rank=q_rank,
+                                             kv_rank=kv_rank, eps=1e-5, scale=192 ** -0.5, window=window, sink=True, gate=gate,
+                                             position=position))
+    got, want = _steps(ops, spec, page, RAGGED, [_set(LATENT_EXPAND_PAIRS=0), _set(latent_expand=False)])
+    # queries, keys, values and the attended rows are rounded to bfloat16 at other places: four roundings on each side
+    _close(got, want, 12)
+
+
+def test_which_steps_expand(ops):
+    from types import SimpleNamespace
+
+    def rows(spans, window, **kw):
+        cu = [0]
+        for _c, n in spans:
+            cu.append(cu[-1] + n)
+        step = SimpleNamespace(decode_only=kw.get("decode", False), captured_width=0, host_cu_seqlens=cu,
+                               host_kv_lens=[c + n for c, n in spans])
+        return ops.latent_expand_rows(step, dim=128, rot_dim=64, value_dim=128, kv_rank=512, window=window, dtype=torch.bfloat16)
+
+    assert rows([(0, 2048)], None) == 2048 and rows([(0, 63)], None) == 63 and rows([(0, 62)], None) == 0
+    assert rows([(8000, 8)], None) == 0 and rows([(8000, 8)], 1024) == 0
+    assert rows([(1000, 512)], 100) == 512 + 1000 - 901 // 64 * 64
+    assert rows([(5, 1), (9, 1)], None, decode=True) == 0
