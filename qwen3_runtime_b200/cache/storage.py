@@ -92,13 +92,19 @@ class CacheStorage:
         """Fixed-size state starts from zero when a request starts or restarts."""
         if not slots:
             return
-        idx = None
+        # runs of neighbouring slots, so that no index has to be copied to the device (a copy from pageable memory waits
+        # for the device: the step's launches would start only then)
+        runs: list[list[int]] = []
+        for slot in sorted(set(slots)):
+            if runs and runs[-1][1] == slot:
+                runs[-1][1] = slot + 1
+            else:
+                runs.append([slot, slot + 1])
         for g, t in zip(self.layout.groups, self.tensors):
             if g.spec.paged:
                 continue
-            if idx is None:
-                idx = torch.tensor(slots, dtype=torch.long, device=t.device)
-            t.index_fill_(1, idx, 0)
+            for a, b in runs:
+                t[:, a:b].zero_()
 
     def poison_pages(self, paged_index: int, pages: list[int], value: float = float("nan")) -> None:
         """Overwrite pages (tests: a page that is used again must not leak old contents)."""

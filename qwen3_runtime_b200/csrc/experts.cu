@@ -34,9 +34,9 @@ constexpr int EXPERT_BM = 32;  // slots per row tile of the FMA products
 // products of k = 4 l .. 4 l + 3, then of those + 128, and so on; the lanes' sums are added by halving.
 //   few tokens: a block stages 2 tokens' rows in shared memory, a warp computes one expert's logits, so that a decode
 //   step's router runs on tens of SMs;
-//   many tokens: a warp keeps 8 tokens x 8 experts in registers and reads operands straight from L1 (a block 16 tokens x
+//   many tokens: a warp keeps 8 tokens x 8 experts in registers and reads operands straight from L1 (a block 8 tokens x
 //   32 experts).  With one expert per warp the reads of the tokens' values, not the FMAs, set the time: 2048 tokens x 64
-//   experts x 2048 took 87 us, with four experts per warp 47, now QQ1 (FMAs alone: 7).
+//   experts x 2048 took 87 us, with four experts per warp 47, now 27 (FMAs alone: 7).
 constexpr int ROUTE_TT = 8;
 
 template <typename T>
@@ -106,25 +106,23 @@ __device__ __forceinline__ float4 load4(const bf16* p) {
 }
 
 constexpr int ROUTE_EPW = 8;               // experts per warp
-constexpr int ROUTE_WT = 2, ROUTE_WE = 4;  // warps of a block along tokens and along experts
+constexpr int ROUTE_WT = 1, ROUTE_WE = 4;  // warps of a block along tokens and along experts
 
 template <typename T>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(32 * ROUTE_WT * ROUTE_WE, 3)
 route_logits_tile_kernel(const T* __restrict__ h, long h_stride, const float* __restrict__ router, int num_tokens, int E,
                          int W, float* __restrict__ logits) {
   pdl_wait();
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t0 = (blockIdx.x * ROUTE_WT + warp / ROUTE_WE) * ROUTE_TT;
-  const int e0 = (blockIdx.y * ROUTE_WE + warp % ROUTE_WE) * ROUTE_EPW;
+  int t0 = (blockIdx.x * ROUTE_WT + warp / ROUTE_WE) * ROUTE_TT;
+  int e0 = (blockIdx.y * ROUTE_WE + warp % ROUTE_WE) * ROUTE_EPW;
   if (t0 >= num_tokens || e0 >= E) return;
-  // tokens and experts past the end are read as the last one and not stored
-  const T* x[ROUTE_TT];
-  const float* w[ROUTE_EPW];
-#pragma unroll
-  for (int t = 0; t < ROUTE_TT; ++t) x[t] = h + (long)min(t0 + t, num_tokens - 1) * h_stride + lane * 4;
-#pragma unroll
-  for (int e = 0; e < ROUTE_EPW; ++e) w[e] = router + (long)min(e0 + e, E - 1) * W + lane * 4;
+  // a last group that would pass the end starts earlier: its first logits are computed twice, with the same bits
+  t0 = min(t0, num_tokens - ROUTE_TT);
+  e0 = min(e0, E - ROUTE_EPW);
+  const T* x = h + (long)t0 * h_stride + lane * 4;
+  const float* w = router + (long)e0 * W + lane * 4;
   float acc[ROUTE_TT][ROUTE_EPW];
 #pragma unroll
   for (int t = 0; t < ROUTE_TT; ++t)
@@ -133,10 +131,10 @@ route_logits_tile_kernel(const T* __restrict__ h, long h_stride, const float* __
   for (int i = 0; i < W - lane * 4; i += 128) {
     float4 w4[ROUTE_EPW];
 #pragma unroll
-    for (int e = 0; e < ROUTE_EPW; ++e) w4[e] = load4(w[e] + i);
+    for (int e = 0; e < ROUTE_EPW; ++e) w4[e] = load4(w + (long)e * W + i);
 #pragma unroll
     for (int t = 0; t < ROUTE_TT; ++t) {
-      const float4 x4 = load4(x[t] + i);
+      const float4 x4 = load4(x + t * h_stride + i);
 #pragma unroll
       for (int e = 0; e < ROUTE_EPW; ++e)
         acc[t][e] = fmaf(x4.x, w4[e].x, fmaf(x4.y, w4[e].y, fmaf(x4.z, w4[e].z, fmaf(x4.w, w4[e].w, acc[t][e]))));
@@ -147,7 +145,7 @@ route_logits_tile_kernel(const T* __restrict__ h, long h_stride, const float* __
 #pragma unroll
     for (int e = 0; e < ROUTE_EPW; ++e) {
       const float v = warp_sum(acc[t][e]);
-      if (lane == 0 && t0 + t < num_tokens && e0 + e < E) logits[(long)(t0 + t) * E + e0 + e] = v;
+      if (lane == 0) logits[(long)(t0 + t) * E + e0 + e] = v;
     }
 }
 
@@ -350,17 +348,17 @@ Q3_EXPORT int q3_route_top(int dtype, const void* h, long h_stride, const float*
   if (dtype != Q3_DTYPE_F32 && dtype != Q3_DTYPE_BF16) return Q3_ERR_ARGUMENT;
   const size_t elem = dtype == Q3_DTYPE_F32 ? 4 : 2;
   // both kernels give the same bits; the tile kernel needs about 64 tokens to fill the SMs
-  const bool tile = num_tokens > 64 && W % 4 == 0 && h_stride % 4 == 0 &&
+  const bool tile = num_tokens > 64 && E >= ROUTE_EPW && W % 4 == 0 && h_stride % 4 == 0 &&
                     (reinterpret_cast<uintptr_t>(h) & (4 * elem - 1)) == 0;
   const int te = ROUTE_WE * ROUTE_EPW;
   cudaError_t e;
   if (tile && (E + te - 1) / te <= 65535) {
     const dim3 grid((num_tokens + ROUTE_WT * ROUTE_TT - 1) / (ROUTE_WT * ROUTE_TT), (E + te - 1) / te);
     if (dtype == Q3_DTYPE_F32)
-      e = launch_pdl(route_logits_tile_kernel<float>, grid, dim3(256), 0, stream, (const float*)h, h_stride, router,
+      e = launch_pdl(route_logits_tile_kernel<float>, grid, dim3(32 * ROUTE_WT * ROUTE_WE), 0, stream, (const float*)h, h_stride, router,
                      num_tokens, E, W, logits);
     else
-      e = launch_pdl(route_logits_tile_kernel<bf16>, grid, dim3(256), 0, stream, (const bf16*)h, h_stride, router,
+      e = launch_pdl(route_logits_tile_kernel<bf16>, grid, dim3(32 * ROUTE_WT * ROUTE_WE), 0, stream, (const bf16*)h, h_stride, router,
                      num_tokens, E, W, logits);
   } else {
     int tt = num_tokens > 64 ? ROUTE_TT : 2;
@@ -729,7 +727,7 @@ Q3_EXPORT int q3_expert_up(int dtype, const void* h, long h_stride, const void* 
 
 // ---- per-token sum ----------------------------------------------------------------------------------
 // VEC values of one token per thread (8: 16-byte accesses, rows of a multiple of 8; what bounds it is memory: 2048
-// tokens x 2048 of 6 slots took 105 us with one value per thread, QQ us with 8).  place: the row of y that holds a slot
+// tokens x 2048 of 6 slots took 105 us with one value per thread, 18 us with 8).  place: the row of y that holds a slot
 // (null: the slot's own number).
 template <typename T, int VEC>
 __global__ void combine_kernel(const T* __restrict__ y, const float* __restrict__ weights, const T* __restrict__ shared,

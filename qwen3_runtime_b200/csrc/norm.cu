@@ -612,7 +612,7 @@ Q3_EXPORT int q3_fused_post_norm(int dtype, const void* pending, int pending_par
 // ---- clamped gated unit: g = min(gate, limit), u = clamp(up, -limit, limit),
 //      out = g * sigmoid(alpha * g) * (u + up_offset); gu rows are [gate (F) | up (F)] ----
 // VEC values per thread (8 where rows and bases allow 16-byte accesses; memory-bound: 2048 rows of 2816, one value per
-// thread 21.8 us, eight QQ us).
+// thread 21.8 us, eight 10 us).
 template <typename T, int VEC>
 __global__ void clamped_glu_kernel(const T* __restrict__ gu, T* __restrict__ out, long total, int F, float limit,
                                    float alpha, float up_offset) {

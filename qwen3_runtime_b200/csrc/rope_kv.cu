@@ -349,7 +349,7 @@ __global__ void qk_norm_store_vec_kernel(T* __restrict__ proj, long row_stride, 
                                          const T* __restrict__ v_first, long v_first_stride, float v_share,
                                          const int* __restrict__ positions, const int* __restrict__ token_seq,
                                          const int* __restrict__ block_table, int max_pages, T* __restrict__ kpages,
-                                         T* __restrict__ vpages, int ps, int shift, int write_kv) {
+                                         T* __restrict__ vpages, int ps, int shift, int write_kv, int maps) {
   pdl_wait();
   pdl_launch_dependents();
   const int t = blockIdx.x;
@@ -377,13 +377,13 @@ __global__ void qk_norm_store_vec_kernel(T* __restrict__ proj, long row_stride, 
   float ss = 0.f;
 #pragma unroll
   for (int e = 0; e < 8; ++e) ss += a[e] * a[e];
-  for (int o = lanes >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  for (int o = (lanes / maps) >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
   if (mine) {
     const float* w = is_q ? q_w : k_w;
     if (w) {
-      const float rstd = rsqrtf(ss / (float)D + eps);
+      const float rstd = rsqrtf(ss / (float)(D / maps) + eps);
       float wv[8];
-      load8(w + c, wv);
+      load8(w + c % (D / maps), wv);
 #pragma unroll
       for (int e = 0; e < 8; ++e) a[e] = (a[e] * rstd) * wv[e];
     }
@@ -420,7 +420,7 @@ static int launch_qk_norm_store_vec(void* proj, long row_stride, int nq, int nkv
                                     int v_start, const float* q_w, const float* k_w, float eps, const float* q_scale,
                                     const void* v_first, long v_first_stride, float v_share, const int* positions,
                                     const int* token_seq, const int* block_table, int max_pages, void* kpages,
-                                    void* vpages, int ps, int num_tokens, int write_kv, cudaStream_t stream) {
+                                    void* vpages, int ps, int num_tokens, int write_kv, int maps, cudaStream_t stream) {
   int shift = 0;
   while ((8 << shift) < D) ++shift;
   const long threads = (long)(write_kv ? nq + nkv + nv : nq) << shift;
@@ -428,7 +428,7 @@ static int launch_qk_norm_store_vec(void* proj, long row_stride, int nq, int nkv
   if (grid.y > 65535) return Q3_ERR_UNSUPPORTED;
   return launch_pdl(qk_norm_store_vec_kernel<T>, grid, dim3(128), 0, stream, (T*)proj, row_stride, nq, nkv, nv, D, Dv,
                     k_start, v_start, q_w, k_w, eps, q_scale, (const T*)v_first, v_first_stride, v_share, positions,
-                    token_seq, block_table, max_pages, (T*)kpages, (T*)vpages, ps, shift, write_kv) == cudaSuccess
+                    token_seq, block_table, max_pages, (T*)kpages, (T*)vpages, ps, shift, write_kv, maps) == cudaSuccess
              ? Q3_OK
              : Q3_ERR_LAUNCH;
 }
@@ -446,17 +446,21 @@ Q3_EXPORT int q3_qk_norm_store(int dtype, void* proj, long row_stride, int nq, i
   if (v_first && v_first_stride < (long)nv * Dv) return Q3_ERR_ARGUMENT;
   if (write_kv && (!token_seq || !block_table || !kpages || !vpages || max_pages < 1)) return Q3_ERR_ARGUMENT;
   if (num_tokens == 0) return Q3_OK;
-  if (maps == 1 && !inv_freq && D % 8 == 0 && Dv % 8 == 0 && D <= 256 && row_stride % 8 == 0 && k_start % 8 == 0 &&
+  // several maps: their lanes are neighbours and a power of two each (2752 tokens x 24 heads of two maps of 64: 12 us, one
+  // warp a head 40)
+  const int map_lanes = D / maps / 8;
+  const bool even_maps = maps == 1 || (D % (8 * maps) == 0 && (map_lanes & (map_lanes - 1)) == 0 && (maps & (maps - 1)) == 0);
+  if (even_maps && !inv_freq && D % 8 == 0 && Dv % 8 == 0 && D <= 256 && row_stride % 8 == 0 && k_start % 8 == 0 &&
       v_start % 8 == 0 && v_first_stride % 8 == 0 && rk_aligned16(proj) && rk_aligned16(kpages) && rk_aligned16(vpages) &&
       rk_aligned16(q_w) && rk_aligned16(k_w) && rk_aligned16(v_first)) {
     if (dtype == Q3_DTYPE_F32)
       return launch_qk_norm_store_vec<float>(proj, row_stride, nq, nkv, nv, D, Dv, k_start, v_start, q_w, k_w, eps, q_scale,
                                              v_first, v_first_stride, v_share, positions, token_seq, block_table, max_pages,
-                                             kpages, vpages, ps, num_tokens, write_kv, stream);
+                                             kpages, vpages, ps, num_tokens, write_kv, maps, stream);
     if (dtype == Q3_DTYPE_BF16)
       return launch_qk_norm_store_vec<bf16>(proj, row_stride, nq, nkv, nv, D, Dv, k_start, v_start, q_w, k_w, eps, q_scale,
                                             v_first, v_first_stride, v_share, positions, token_seq, block_table, max_pages,
-                                            kpages, vpages, ps, num_tokens, write_kv, stream);
+                                            kpages, vpages, ps, num_tokens, write_kv, maps, stream);
     return Q3_ERR_ARGUMENT;
   }
   constexpr int WARPS = 4;

@@ -169,6 +169,10 @@ _SIGNATURES = {
                                   c_void_p, c_float, c_void_p, c_void_p, c_int, c_void_p, c_float, c_float, c_void_p,
                                   c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                                   c_int, c_void_p, c_void_p],
+        "q3_decayed_segment_scan": [c_int, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long,
+                                  c_void_p, c_float, c_void_p, c_void_p, c_int, c_void_p, c_float, c_float, c_void_p,
+                                  c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
+                                  c_int, c_void_p, c_int, c_int, c_void_p, c_void_p],
         "q3_head_norm_gate": [c_int, c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p, c_long, c_void_p, c_long,
                               c_float, c_int, c_int, c_int, c_int, c_void_p],
         "q3_stabilised_gates": [c_int, c_void_p, c_void_p, c_long, c_void_p, c_void_p, c_float, c_void_p, c_void_p,
@@ -299,6 +303,7 @@ class CudaOps:
         self.experts_tc = True              # False: the experts' products always on the FMA kernels
         self.chunk_tc = True                # False: attention under chunks or with turned values on the general kernel
         self.delta_chunks = True            # False: the delta rule's recurrence always token by token
+        self.scan_segments = True           # False: the decayed state scan always token by token
         self.latent_expand = True           # False: prompts never expand the latent's keys and values
         self.differential_tcgen05 = True    # False: differential attention never on the tcgen05 kernel
         self.differential_tc = True         # False: differential attention always on the general kernel
@@ -713,13 +718,28 @@ class CudaOps:
             e = q.element_size()
             self._costs(2 * num_seqs * H * D * Dv * 4 + T * H * ((3 if z is not None else 2) * D + Dv) * e
                         + T * H * Dv * 4, 6.0 * T * H * D * Dv)
-        self._call("linear_state", "q3_decayed_state_scan", "decayed_state_scan", _dtype_code(q.dtype), _ptr(q),
-                   q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(z), z.stride(0) if z is not None else 0,
-                   _ptr(decay_bias), 1.0 / float(tau), _ptr(head_decay), _ptr(inv_freq), pairs, _ptr(positions),
-                   float(q_scale), float(k_scale), _ptr(state), _ptr(cu_seqlens), _ptr(state_slots), _ptr(out),
-                   int(num_seqs), H, D, Dv, modes[decay_mode], _ptr(token_decay), _ptr(token_k_scale),
-                   int(bool(ones_column)), _ptr(bonus))
+        args = (_dtype_code(q.dtype), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(z),
+                z.stride(0) if z is not None else 0, _ptr(decay_bias), 1.0 / float(tau), _ptr(head_decay), _ptr(inv_freq),
+                pairs, _ptr(positions), float(q_scale), float(k_scale), _ptr(state), _ptr(cu_seqlens), _ptr(state_slots),
+                _ptr(out), int(num_seqs), H, D, Dv, modes[decay_mode], _ptr(token_decay), _ptr(token_k_scale),
+                int(bool(ones_column)), _ptr(bonus))
+        seg = self._scan_segment(T, int(num_seqs), H, D, Dv)
+        if seg:
+            segments = T // seg + int(num_seqs)  # at least the sum of ceil(tokens / seg)
+            scratch = torch.empty(segments * H * D * (Dv + 1), dtype=torch.float32, device=q.device)
+            self.launches += 2 * int(segments > num_seqs)
+            self._call("linear_state", "q3_decayed_segment_scan", "decayed_state_scan", *args, seg, segments, _ptr(scratch))
+            return out
+        self._call("linear_state", "q3_decayed_state_scan", "decayed_state_scan", *args)
         return out
+
+    def _scan_segment(self, T, num_seqs, H, D, Dv) -> int:
+        """Tokens per segment of a decayed state scan, or 0 for the scan without segments: steps of many tokens per sequence
+        with keys of up to 128.  A multiple of 16, at least 32, for about two blocks per SM."""
+        if not self.scan_segments or D > 128 or T < max(64, 8 * num_seqs):
+            return 0
+        blocks = H * -(-Dv // (128 if D <= 64 else 64))
+        return max(32, 16 * -(-T // (16 * max(1, 2 * self.SM_COUNT // blocks))))
 
     def stabilised_gates(self, zi, zf, *, i_bias, f_bias, cap, m_state, cu_seqlens, state_slots, num_seqs):
         """The gates of a matrix memory with exponential gates and a running maximum m per (sequence, head)
