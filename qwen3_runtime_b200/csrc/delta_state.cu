@@ -382,8 +382,9 @@ Q3_EXPORT int q3_delta_scan(int dtype, const float* qn, const float* kn, const v
 // [DP][32] (G k | G q, transposed), [16][DP] the decayed-to-the-end keys, [DP] G_last, W and B [16][16].  Chunks of
 // sequence b start at place cu_seqlens[b] / 16 + b; tokens beyond a portion's end are k = q = 0, g = 1, beta = 0.
 // delta_chunk_scan: one block per (16 value columns, head, sequence); the state's columns stay in registers (and, for
-// the products with it, in shared memory), the next chunk's record is on its way while one is worked on.
+// the products with it, in shared memory), the next chunks' records are on their way while one is worked on.
 #define DC_C 16
+#define DC_STAGES 3  // records in shared memory: with two a chunk waited for its record (2048 tokens: the mixer 423 us, with three 407)
 #define DC_REC(DP) ((DP) * 49 + 2 * DC_C * DC_C)
 
 template <int DP>
@@ -507,8 +508,9 @@ delta_chunk_scan_kernel(const float* __restrict__ records, const T* __restrict__
                         const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots, float* __restrict__ out,
                         int H, int D, int Dv) {
   constexpr int VT = 16, REC = DC_REC(DP), RD = DP / 64, PS = 20;  // PS: row pitch of the partial sums
+  constexpr int STAGES = DC_STAGES;
   extern __shared__ __align__(16) float dc_smem[];
-  float* Ss = dc_smem + 2 * REC;       // [DP][VT]
+  float* Ss = dc_smem + STAGES * REC;  // [DP][VT]
   float* part = Ss + DP * VT;          // [8][32][PS]
   float* ys = part + 8 * 32 * PS;      // [16][VT]
   float* us = ys + DC_C * VT;          // [16][VT]
@@ -521,12 +523,15 @@ delta_chunk_scan_kernel(const float* __restrict__ records, const T* __restrict__
   const int chunks = (t1 - t0 + DC_C - 1) / DC_C;
   const float* rec0 = records + ((long)(t0 / DC_C + b) * H + h) * REC;
   auto load = [&](int c) {
-    const float* src = rec0 + (long)c * H * REC;
-    float* dst = dc_smem + (c & 1) * REC;
-    for (int x = tid * 4; x < REC; x += 1024) ds_copy16(dst + x, src + x);
-    asm volatile("cp.async.commit_group;\n" ::);
+    if (c < chunks) {
+      const float* src = rec0 + (long)c * H * REC;
+      float* dst = dc_smem + (c % STAGES) * REC;
+      for (int x = tid * 4; x < REC; x += 1024) ds_copy16(dst + x, src + x);
+    }
+    asm volatile("cp.async.commit_group;\n" ::);  // also when empty: one group per call
   };
-  load(0);
+#pragma unroll
+  for (int c = 0; c < STAGES - 1; ++c) load(c);
   // this thread's rows and columns of the state
   const int d0 = (tid >> 2) * RD, c0 = (tid & 3) * 4;
   float* Sg = state + ((long)state_slots[b] * H + h) * (long)D * Dv;
@@ -547,14 +552,12 @@ delta_chunk_scan_kernel(const float* __restrict__ records, const T* __restrict__
   float v_next = value(0);
   const int rt = (lane >> 2) * 4, ct = (lane & 3) * 4;
   for (int c = 0; c < chunks; ++c) {
-    asm volatile("cp.async.wait_group 0;\n" ::);
-    __syncthreads();  // the record and the state in shared memory are complete; nobody reads the other record
-    const float* rec = dc_smem + (c & 1) * REC;
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2));
+    __syncthreads();  // the record and the state in shared memory are complete; nobody reads the last record any more
+    const float* rec = dc_smem + (c % STAGES) * REC;
+    load(c + STAGES - 1);
     const float v = v_next;
-    if (c + 1 < chunks) {
-      load(c + 1);
-      v_next = value(c + 1);
-    }
+    if (c + 1 < chunks) v_next = value(c + 1);
     {  // [G k; G q] S, an eighth of the channels a warp, 4 x 4 sums a thread
       float acc[4][4];
 #pragma unroll
@@ -652,7 +655,7 @@ static int launch_delta_chunks(cudaStream_t stream, int num_tokens, int num_seqs
   if (launch_pdl(delta_chunk_rows_kernel<DP>, dim3(places, H), dim3(256), 0, stream, qn, kn, g, beta, cu_seqlens, num_seqs,
                  records, G, H, D) != cudaSuccess)
     return Q3_ERR_LAUNCH;
-  constexpr size_t smem = sizeof(float) * (2 * DC_REC(DP) + DP * 16 + 8 * 32 * 20 + 2 * DC_C * 16);
+  constexpr size_t smem = sizeof(float) * (DC_STAGES * DC_REC(DP) + DP * 16 + 8 * 32 * 20 + 2 * DC_C * 16);
   auto kernel = delta_chunk_scan_kernel<T, DP>;
   static bool configured_on[Q3_MAX_DEVICES];
   bool& configured = configured_on[q3_current_device()];

@@ -33,9 +33,12 @@
 // into segments of `seg` tokens: (1) every segment but a sequence's last works out the state it would leave behind if it
 // began with zeros, and the product of its decays; (2) the segments' first states follow one from another,
 // S <- diag(product) S + left behind; (3) every segment runs from its first state and writes its outputs, a sequence's last
-// one the slot.  All decays are at most one, so nothing grows, and every sum is fp32 as before.  A thread holds 4 x 4
-// elements of the state, so that a token's three rows and its values are read once for 16 updates, and the sums over the
-// row groups are folded: a lane gives half of its columns away at each step.  16 heads of 64 x 128, 2048 tokens: 160 us (54 + 15 + 91).
+// one the slot.  All decays are at most one, so nothing grows, and every sum is fp32 as before.  The rotations, decays and
+// scales of a token's rows are worked out by a kernel of their own (16 us), not in both passes and every column tile.  A
+// thread holds 4 x 8 elements of the state, so that a token's three rows and its values are read once for 32 updates, as
+// pairs of columns for the packed instructions (the issue slots bound the passes), and the sums over the row groups are
+// folded: a lane gives half of its columns away at each step.  16 heads of 64 x 128, 2048 tokens, the whole mixer: 565 us
+// with the scan above, 231 with 4 x 4 elements and rows worked out in the passes, 200 so.
 //
 // head_norm_gate: y[t, h, :] = o / sqrt(mean(o^2) + eps) * w * silu(g[t, h, :]) * out_scale, one warp
 // per (token, head); w may be absent.
@@ -281,20 +284,62 @@ struct ScanArgs {
   int seg;          // tokens per segment
   float* ends;      // [segments, H, D, Dv]: what a segment leaves behind, then the segments' first states
   float* products;  // [segments, H, D]
+  float* rows;      // [T, H, 3, DP], DP = 64 or 128
 };
 
-// DP: key rows (64 or 128), in DP / 4 row groups; CG column groups of 4.  Block: (segment, column tile, head).
+// A token's rows of a head as the scans read them, fp32 [T, H, 3, DP]: keys (turned, scaled), decays, queries (turned,
+// scaled); zero (and one) beyond D.  Worked out once: both scans and every column tile read the same rows.
+template <typename T, int DP>
+__global__ void __launch_bounds__(256)
+segment_rows_kernel(const __grid_constant__ ScanArgs a, long total) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const long x = (long)blockIdx.x * 256 + threadIdx.x;
+  if (x >= total) return;
+  const int i = x % DP;
+  const long th = x / DP, t = th / a.H;
+  const int h = (int)(th - t * a.H);
+  const T *q = (const T*)a.q + t * a.q_stride + h * a.D, *k = (const T*)a.k + t * a.k_stride + h * a.D;
+  float qv = 0.f, kv = 0.f, av = 1.f;
+  if (i < a.D) {
+    qv = to_f32(q[i]);
+    kv = to_f32(k[i]);
+    if (i < 2 * a.rot_pairs) {
+      const bool front = i < a.rot_pairs;
+      const int pair = front ? i : i - a.rot_pairs, other = front ? i + a.rot_pairs : pair;
+      float sn, cs;
+      sincosf((float)a.positions[t] * a.inv_freq[pair], &sn, &cs);
+      const float qp = to_f32(q[other]), kp = to_f32(k[other]);
+      qv = front ? qv * cs - qp * sn : qv * cs + qp * sn;
+      kv = front ? kv * cs - kp * sn : kv * cs + kp * sn;
+    }
+    qv *= a.q_scale;
+    kv *= a.k_scale;
+    if (a.tok_kscale) kv *= a.tok_kscale[t * a.H + h];
+    if (a.z) {
+      const float zz = to_f32(((const T*)a.z)[t * a.z_stride + h * a.D + i]) + (a.z_bias ? a.z_bias[h * a.D + i] : 0.f);
+      av = a.decay_mode == 1 ? expf(-expf(zz)) : expf((fminf(zz, 0.f) - log1pf(expf(-fabsf(zz)))) * a.inv_tau);
+    } else {
+      av = a.tok_decay ? a.tok_decay[t * a.H + h] : a.head_decay[h];
+    }
+  }
+  float* dst = a.rows + th * 3 * DP + i;
+  dst[0] = kv;
+  dst[DP] = av;
+  dst[2 * DP] = qv;
+}
+
+// DP: key rows (64 or 128), in DP / 4 row groups; CG column groups of 8: a thread holds 4 x 8 elements of the state.
+// Block: (segment, column tile, head).
 template <typename T, int DP, int CG, bool OUT, bool BONUS>
 __global__ void __launch_bounds__(DP / 4 * CG, 2)
 segment_scan_kernel(const __grid_constant__ ScanArgs a) {
-  constexpr int RG = DP / 4, THREADS = RG * CG, VT = 4 * CG, CT = SCAN_CT;
-  constexpr int EPT = CT * DP / THREADS, VPT = CT * VT / THREADS;
-  static_assert(EPT * THREADS == CT * DP && VPT * THREADS == CT * VT && (RG == 16 || RG == 32), "whole turns");
+  constexpr int RG = DP / 4, THREADS = RG * CG, VT = 8 * CG, CT = SCAN_CT;
+  constexpr int ROW = (OUT ? 3 : 2) * DP, VPT = CT * VT / THREADS;  // a token's k, a (and q) rows
+  static_assert(VPT * THREADS == CT * VT && (RG == 16 || RG == 32), "whole turns");
   extern __shared__ __align__(16) float scan_smem[];
-  float* qs = scan_smem;              // [2][CT][DP]
-  float* ks = qs + 2 * CT * DP;
-  float* as = ks + 2 * CT * DP;
-  float* vs = as + 2 * CT * DP;       // [2][CT][VT]
+  float* rs = scan_smem;              // [2][CT][ROW]
+  float* vs = rs + 2 * CT * ROW;      // [2][CT][VT]
   float* os = vs + 2 * CT * VT;       // [CT][VT]
   __shared__ int s_seq, s_first, s_count;
   const int tid = threadIdx.x;
@@ -325,16 +370,18 @@ segment_scan_kernel(const __grid_constant__ ScanArgs a) {
   if (!OUT && last) return;
   const int t0 = a.cu_seqlens[seq] + mine * a.seg, t1 = min(a.cu_seqlens[seq + 1], t0 + a.seg);
   const long slot = a.state_slots[seq];
-  const int rg = tid % RG, cg = tid / RG, i0 = rg * 4, c0 = cg * 4;
+  const int rg = tid % RG, cg = tid / RG, i0 = rg * 4, c0 = cg * 8;
   const long tile = ((long)blockIdx.x * H + h) * D;
   float* Sg = a.state + (slot * H + h) * (long)D * Dv;
-  float S[4][4];
+  float2 S[4][4];  // [row][pair of columns]
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      const int i = i0 + r, j = j0 + c0 + c;
-      S[r][c] = !OUT || i >= D || j >= Dv ? 0.f : (s_count > 1 ? a.ends[(tile + i) * Dv + j] : Sg[(long)i * Dv + j]);
+      const int i = i0 + r, j = j0 + c0 + 2 * c;
+      const float* src = s_count > 1 ? a.ends + (tile + i) * Dv : Sg + (long)i * Dv;
+      S[r][c].x = !OUT || i >= D || j >= Dv ? 0.f : src[j];
+      S[r][c].y = !OUT || i >= D || j + 1 >= Dv ? 0.f : src[j + 1];
     }
   float U[4], P[4];
 #pragma unroll
@@ -342,25 +389,18 @@ segment_scan_kernel(const __grid_constant__ ScanArgs a) {
     U[r] = (BONUS && i0 + r < D) ? a.bonus[h * D + i0 + r] : 0.f;
     P[r] = 1.f;
   }
-  const float decay_h = a.head_decay ? a.head_decay[h] : 1.f;
   const int Dvin = Dv - a.ones_col;
-  const T *q = (const T*)a.q, *k = (const T*)a.k, *v = (const T*)a.v, *z = (const T*)a.z;
-  T qr[EPT], kr[EPT], zr[EPT], qo[EPT], ko[EPT], vr[VPT];
-  auto fetch = [&](int t_at) {
-#pragma unroll
-    for (int m = 0; m < EPT; ++m) {
-      const int x = tid + m * THREADS, c = x / DP, i = x - c * DP;
-      const long t = t_at + c;
-      const bool live = t < t1 && i < D;
-      if (OUT) qr[m] = live ? q[t * a.q_stride + h * D + i] : from_f32<T>(0.f);
-      kr[m] = live ? k[t * a.k_stride + h * D + i] : from_f32<T>(0.f);
-      zr[m] = (live && z) ? z[t * a.z_stride + h * D + i] : from_f32<T>(0.f);
-      if (live && i < 2 * a.rot_pairs) {
-        const int other = i < a.rot_pairs ? i + a.rot_pairs : i - a.rot_pairs;
-        if (OUT) qo[m] = q[t * a.q_stride + h * D + other];
-        ko[m] = k[t * a.k_stride + h * D + other];
-      }
+  const T* v = (const T*)a.v;
+  T vr[VPT];
+  // a chunk's rows into buffer `to` (its values into registers): in flight while the chunk before is worked on
+  auto fetch = [&](int t_at, int to) {
+    const int n = min(CT, t1 - t_at);
+    for (int x = tid * 4; x < n * ROW; x += THREADS * 4) {
+      const int c = x / ROW;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(rs + to * CT * ROW + x)),
+                   "l"(a.rows + ((long)(t_at + c) * H + h) * 3 * DP + (x - c * ROW)) : "memory");
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
 #pragma unroll
     for (int m = 0; m < VPT; ++m) {
       const int x = tid + m * THREADS, c = x / VT, j = j0 + x % VT;
@@ -368,80 +408,63 @@ segment_scan_kernel(const __grid_constant__ ScanArgs a) {
       vr[m] = t < t1 && j < Dvin ? v[t * a.v_stride + h * Dvin + j] : from_f32<T>(t < t1 && j < Dv ? 1.f : 0.f);
     }
   };
-  auto stage = [&](int t_at, int buf) {
+  auto stage = [&](int to) {
 #pragma unroll
-    for (int m = 0; m < EPT; ++m) {
-      const int x = tid + m * THREADS, c = x / DP, i = x - c * DP;
-      const long t = t_at + c;
-      float qv = 0.f, kv = 0.f, av = 1.f;
-      if (t < t1 && i < D) {
-        qv = OUT ? to_f32(qr[m]) : 0.f;
-        kv = to_f32(kr[m]);
-        if (i < 2 * a.rot_pairs) {
-          const bool front = i < a.rot_pairs;
-          float sn, cs;
-          sincosf((float)a.positions[t] * a.inv_freq[front ? i : i - a.rot_pairs], &sn, &cs);
-          const float qp = OUT ? to_f32(qo[m]) : 0.f, kp = to_f32(ko[m]);
-          qv = front ? qv * cs - qp * sn : qv * cs + qp * sn;
-          kv = front ? kv * cs - kp * sn : kv * cs + kp * sn;
-        }
-        qv *= a.q_scale;
-        kv *= a.k_scale;
-        if (a.tok_kscale) kv *= a.tok_kscale[t * H + h];
-        if (z) {
-          const float zz = to_f32(zr[m]) + (a.z_bias ? a.z_bias[h * D + i] : 0.f);
-          av = a.decay_mode == 1 ? expf(-expf(zz)) : expf((fminf(zz, 0.f) - log1pf(expf(-fabsf(zz)))) * a.inv_tau);
-        } else {
-          av = a.tok_decay ? a.tok_decay[t * H + h] : decay_h;
-        }
-      }
-      if (OUT) qs[(buf * CT + c) * DP + i] = qv;
-      ks[(buf * CT + c) * DP + i] = kv;
-      as[(buf * CT + c) * DP + i] = av;
-    }
-#pragma unroll
-    for (int m = 0; m < VPT; ++m) vs[buf * CT * VT + tid + m * THREADS] = to_f32(vr[m]);
+    for (int m = 0; m < VPT; ++m) vs[to * CT * VT + tid + m * THREADS] = to_f32(vr[m]);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
   };
-  fetch(t0);
-  stage(t0, 0);
+  fetch(t0, 0);
+  stage(0);
   __syncthreads();
   int buf = 0;
   for (int t = t0; t < t1; t += CT, buf ^= 1) {
     const int n = min(CT, t1 - t);
     const bool more = t + CT < t1;
-    if (more) fetch(t + CT);
+    if (more) fetch(t + CT, buf ^ 1);
 #pragma unroll 2
     for (int c = 0; c < n; ++c) {
-      const float4 a4 = *reinterpret_cast<const float4*>(as + (buf * CT + c) * DP + i0);
-      const float4 k4 = *reinterpret_cast<const float4*>(ks + (buf * CT + c) * DP + i0);
-      const float4 v4 = *reinterpret_cast<const float4*>(vs + (buf * CT + c) * VT + c0);
-      const float aa[4] = {a4.x, a4.y, a4.z, a4.w}, kk[4] = {k4.x, k4.y, k4.z, k4.w}, vv[4] = {v4.x, v4.y, v4.z, v4.w};
-      float qq[4] = {0.f, 0.f, 0.f, 0.f}, acc[4] = {0.f, 0.f, 0.f, 0.f};
+      const float* row = rs + (buf * CT + c) * ROW + i0;
+      const float4 k4 = *reinterpret_cast<const float4*>(row);
+      const float4 a4 = *reinterpret_cast<const float4*>(row + DP);
+      const float4 va = *reinterpret_cast<const float4*>(vs + (buf * CT + c) * VT + c0);
+      const float4 vb = *reinterpret_cast<const float4*>(vs + (buf * CT + c) * VT + c0 + 4);
+      const float2 vv[4] = {make_float2(va.x, va.y), make_float2(va.z, va.w), make_float2(vb.x, vb.y), make_float2(vb.z, vb.w)};
+      const float aa[4] = {a4.x, a4.y, a4.z, a4.w}, kk[4] = {k4.x, k4.y, k4.z, k4.w};
+      float qq[4] = {0.f, 0.f, 0.f, 0.f};
+      float2 acc[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
       if (OUT) {
-        const float4 q4 = *reinterpret_cast<const float4*>(qs + (buf * CT + c) * DP + i0);
+        const float4 q4 = *reinterpret_cast<const float4*>(row + 2 * DP);
         qq[0] = q4.x; qq[1] = q4.y; qq[2] = q4.z; qq[3] = q4.w;
       }
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
-        if (!OUT) P[r] *= aa[r];
+        const float2 a2 = make_float2(aa[r], aa[r]), k2 = make_float2(kk[r], kk[r]), q2 = make_float2(qq[r], qq[r]);
+        const float2 u2 = make_float2(U[r], U[r]);
+        if (!OUT && tid < 32) P[r] *= aa[r];  // (the first warp's rows are all rows)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float kv = kk[r] * vv[e];
-          if (OUT && BONUS) acc[e] = fmaf(fmaf(U[r], kv, S[r][e]), qq[r], acc[e]);
-          S[r][e] = fmaf(aa[r], S[r][e], kv);
-          if (OUT && !BONUS) acc[e] = fmaf(S[r][e], qq[r], acc[e]);
+          const float2 kv = __fmul2_rn(k2, vv[e]);
+          if (OUT && BONUS) acc[e] = __ffma2_rn(__ffma2_rn(u2, kv, S[r][e]), q2, acc[e]);
+          S[r][e] = __ffma2_rn(a2, S[r][e], kv);
+          if (OUT && !BONUS) acc[e] = __ffma2_rn(S[r][e], q2, acc[e]);
         }
       }
       if (OUT) {
-        // the sums over the row groups, lanes rg: after two steps a lane has one column's sum over four groups
-        const bool hi1 = rg & 1, hi2 = rg & 2;
-        float u = hi1 ? acc[0] : acc[2], w = hi1 ? acc[1] : acc[3];
-        float x0 = (hi1 ? acc[2] : acc[0]) + __shfl_xor_sync(0xffffffffu, u, 1);
-        float x1 = (hi1 ? acc[3] : acc[1]) + __shfl_xor_sync(0xffffffffu, w, 1);
-        float y = (hi2 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, hi2 ? x0 : x1, 2);
+        // the sums over the row groups, lanes rg: a lane gives half of its columns away in each of three steps and then
+        // has one column's sum over eight groups
+        const bool h1 = rg & 1, h2 = rg & 2, h4 = rg & 4;
+        const float av[8] = {acc[0].x, acc[0].y, acc[1].x, acc[1].y, acc[2].x, acc[2].y, acc[3].x, acc[3].y};
+        float x4[4], x2[2];
 #pragma unroll
-        for (int o = 4; o < RG; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-        if (rg < 4) os[c * VT + c0 + 2 * (rg & 1) + (rg >> 1)] = y;
+        for (int e = 0; e < 4; ++e)
+          x4[e] = (h1 ? av[e + 4] : av[e]) + __shfl_xor_sync(0xffffffffu, h1 ? av[e] : av[e + 4], 1);
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          x2[e] = (h2 ? x4[e + 2] : x4[e]) + __shfl_xor_sync(0xffffffffu, h2 ? x4[e] : x4[e + 2], 2);
+        float y = (h4 ? x2[1] : x2[0]) + __shfl_xor_sync(0xffffffffu, h4 ? x2[0] : x2[1], 4);
+#pragma unroll
+        for (int o = 8; o < RG; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+        if (rg < 8) os[c * VT + c0 + 4 * (rg & 1) + (rg & 2) + (rg >> 2)] = y;
       }
     }
     if (OUT) {
@@ -451,7 +474,7 @@ segment_scan_kernel(const __grid_constant__ ScanArgs a) {
         if (j < Dv) a.out[((long)(t + c) * H + h) * Dv + j] = os[x];
       }
     }
-    if (more) stage(t + CT, buf ^ 1);
+    if (more) stage(buf ^ 1);
     __syncthreads();
   }
   float* dst = OUT ? Sg : a.ends + tile * Dv;
@@ -459,8 +482,11 @@ segment_scan_kernel(const __grid_constant__ ScanArgs a) {
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
-        if (i0 + r < D && j0 + c0 + c < Dv) dst[(long)(i0 + r) * Dv + j0 + c0 + c] = S[r][c];
+      for (int c = 0; c < 4; ++c) {
+        const int i = i0 + r, j = j0 + c0 + 2 * c;
+        if (i < D && j < Dv) dst[(long)i * Dv + j] = S[r][c].x;
+        if (i < D && j + 1 < Dv) dst[(long)i * Dv + j + 1] = S[r][c].y;
+      }
   }
   if (!OUT && blockIdx.y == 0 && cg == 0) {
 #pragma unroll
@@ -482,17 +508,27 @@ segment_join_kernel(const __grid_constant__ ScanArgs a) {
   if (count < 2 || x >= D * Dv) return;
   const int i = x / Dv;
   float S = a.state[((long)a.state_slots[seq] * a.H + h) * D * Dv + x];
-  for (int m = 0; m < count; ++m) {
-    const long at = ((long)(first + m) * a.H + h) * D;
-    const float left = m < count - 1 ? a.ends[at * Dv + x] : 0.f;
-    a.ends[at * Dv + x] = S;
-    if (m < count - 1) S = fmaf(a.products[at + i], S, left);
+  constexpr int AHEAD = 6;  // segments whose numbers are read together: the chain is one multiply-add a segment
+  for (int m0 = 0; m0 < count; m0 += AHEAD) {
+    float left[AHEAD], product[AHEAD];
+#pragma unroll
+    for (int e = 0; e < AHEAD; ++e) {
+      const long at = ((long)(first + m0 + e) * a.H + h) * D;
+      const bool live = m0 + e < count - 1;
+      left[e] = live ? a.ends[at * Dv + x] : 0.f;
+      product[e] = live ? a.products[at + i] : 0.f;
+    }
+#pragma unroll
+    for (int e = 0; e < AHEAD; ++e) {
+      if (m0 + e < count) a.ends[((long)(first + m0 + e) * a.H + h) * D * Dv + x] = S;
+      S = fmaf(product[e], S, left[e]);
+    }
   }
 }
 
 template <typename T, int DP, int CG, bool BONUS>
-static cudaError_t launch_segments(const ScanArgs& a, int segments, cudaStream_t stream) {
-  constexpr size_t smem = (size_t)(6 * SCAN_CT * DP + 3 * SCAN_CT * 4 * CG) * sizeof(float);
+static cudaError_t launch_segments(const ScanArgs& a, int num_tokens, int segments, cudaStream_t stream) {
+  constexpr size_t smem = (size_t)(6 * SCAN_CT * DP + 3 * SCAN_CT * 8 * CG) * sizeof(float);
   static bool configured_on[Q3_MAX_DEVICES];
   bool& configured = configured_on[q3_current_device()];
   if (!configured) {
@@ -504,9 +540,11 @@ static cudaError_t launch_segments(const ScanArgs& a, int segments, cudaStream_t
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  const dim3 grid((unsigned)segments, (unsigned)((a.Dv + 4 * CG - 1) / (4 * CG)), (unsigned)a.H), block(DP / 4 * CG);
-  cudaError_t e = cudaSuccess;
-  if (segments > a.num_seqs) {  // else every sequence is one segment
+  const dim3 grid((unsigned)segments, (unsigned)((a.Dv + 8 * CG - 1) / (8 * CG)), (unsigned)a.H), block(DP / 4 * CG);
+  const long elements = (long)num_tokens * a.H * DP;
+  cudaError_t e = launch_pdl(segment_rows_kernel<T, DP>, dim3((unsigned)((elements + 255) / 256)), dim3(256), 0, stream, a,
+                             elements);
+  if (e == cudaSuccess && segments > a.num_seqs) {  // else every sequence is one segment
     e = launch_pdl(segment_scan_kernel<T, DP, CG, false, BONUS>, grid, block, smem, stream, a);
     if (e == cudaSuccess)
       e = launch_pdl(segment_join_kernel, dim3((unsigned)((a.D * a.Dv + 255) / 256), (unsigned)a.H, (unsigned)a.num_seqs),
@@ -517,33 +555,38 @@ static cudaError_t launch_segments(const ScanArgs& a, int segments, cudaStream_t
 }
 
 // The same arguments as q3_decayed_state_scan, key sizes up to 128: in segments of `seg` tokens.  segments: the number of
-// them, sum over the sequences of ceil(tokens / seg), or more; scratch: fp32 [segments * H * D * (Dv + 1)].
+// them, sum over the sequences of ceil(tokens / seg), or more; scratch: fp32, 16-byte aligned, [num_tokens * H * 3 * DP +
+// segments * H * D * (Dv + 1)] with DP = 64 (D <= 64) or 128.
 Q3_EXPORT int q3_decayed_segment_scan(int dtype, const void* q, long q_stride, const void* k, long k_stride, const void* v,
                                       long v_stride, const void* z, long z_stride, const float* z_bias, float inv_tau,
                                       const float* head_decay, const float* inv_freq, int rot_pairs, const int* positions,
                                       float q_scale, float k_scale, float* state, const int* cu_seqlens,
                                       const int* state_slots, float* out, int num_seqs, int H, int D, int Dv,
                                       int decay_mode, const float* tok_decay, const float* tok_kscale, int ones_col,
-                                      const float* bonus, int seg, int segments, float* scratch, cudaStream_t stream) {
-  if (!q || !k || !v || !state || !cu_seqlens || !state_slots || !out || !scratch || seg < 1 || segments < 1)
+                                      const float* bonus, int seg, int segments, float* scratch, int num_tokens,
+                                      cudaStream_t stream) {
+  if (!q || !k || !v || !state || !cu_seqlens || !state_slots || !out || !scratch || seg < 1 || segments < 1 ||
+      num_tokens < 0 || ((uintptr_t)scratch & 15))
     return Q3_ERR_ARGUMENT;
   if (!z && !head_decay && !tok_decay) return Q3_ERR_ARGUMENT;
   if (decay_mode < 0 || decay_mode > 1 || ones_col < 0 || ones_col > 1 || Dv - ones_col < 1) return Q3_ERR_ARGUMENT;
   if (rot_pairs < 0 || 2 * rot_pairs > D || (rot_pairs && (!inv_freq || !positions))) return Q3_ERR_ARGUMENT;
   if (H < 1 || D < 1 || Dv < 1 || H > 65535 || num_seqs > 65535) return Q3_ERR_ARGUMENT;
   if (D > 128 || (dtype != Q3_DTYPE_F32 && dtype != Q3_DTYPE_BF16)) return Q3_ERR_UNSUPPORTED;
-  if (num_seqs == 0) return Q3_OK;
+  if (num_seqs == 0 || num_tokens == 0) return Q3_OK;
+  const long rows = (long)num_tokens * H * 3 * (D <= 64 ? 64 : 128);
   const ScanArgs a = {q, k, v, z, q_stride, k_stride, v_stride, z_stride, z_bias, inv_tau, head_decay, inv_freq, rot_pairs,
                       positions, q_scale, k_scale, state, cu_seqlens, state_slots, out, num_seqs, H, D, Dv, decay_mode,
-                      tok_decay, tok_kscale, ones_col, bonus, seg, scratch, scratch + (long)segments * H * D * Dv};
+                      tok_decay, tok_kscale, ones_col, bonus, seg, scratch + rows, scratch + rows + (long)segments * H * D * Dv,
+                      scratch};
   cudaError_t e;
 #define Q3_SEGMENTS(T)                                                                       \
   if (D <= 64)                                                                               \
-    e = bonus ? launch_segments<T, 64, 32, true>(a, segments, stream)                        \
-              : launch_segments<T, 64, 32, false>(a, segments, stream);                      \
+    e = bonus ? launch_segments<T, 64, 16, true>(a, num_tokens, segments, stream)                        \
+              : launch_segments<T, 64, 16, false>(a, num_tokens, segments, stream);                      \
   else                                                                                       \
-    e = bonus ? launch_segments<T, 128, 16, true>(a, segments, stream)                       \
-              : launch_segments<T, 128, 16, false>(a, segments, stream)
+    e = bonus ? launch_segments<T, 128, 8, true>(a, num_tokens, segments, stream)                       \
+              : launch_segments<T, 128, 8, false>(a, num_tokens, segments, stream)
   if (dtype == Q3_DTYPE_F32) {
     Q3_SEGMENTS(float);
   } else {

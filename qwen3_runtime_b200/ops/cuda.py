@@ -172,7 +172,8 @@ _SIGNATURES = {
         "q3_decayed_segment_scan": [c_int, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long,
                                   c_void_p, c_float, c_void_p, c_void_p, c_int, c_void_p, c_float, c_float, c_void_p,
                                   c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                                  c_int, c_void_p, c_int, c_int, c_void_p, c_void_p],
+                                  c_int, c_void_p, c_int, c_int, c_void_p, c_int,
+                                    c_void_p],
         "q3_head_norm_gate": [c_int, c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p, c_long, c_void_p, c_long,
                               c_float, c_int, c_int, c_int, c_int, c_void_p],
         "q3_stabilised_gates": [c_int, c_void_p, c_void_p, c_long, c_void_p, c_void_p, c_float, c_void_p, c_void_p,
@@ -726,20 +727,22 @@ class CudaOps:
         seg = self._scan_segment(T, int(num_seqs), H, D, Dv)
         if seg:
             segments = T // seg + int(num_seqs)  # at least the sum of ceil(tokens / seg)
-            scratch = torch.empty(segments * H * D * (Dv + 1), dtype=torch.float32, device=q.device)
-            self.launches += 2 * int(segments > num_seqs)
-            self._call("linear_state", "q3_decayed_segment_scan", "decayed_state_scan", *args, seg, segments, _ptr(scratch))
+            scratch = torch.empty(T * H * 3 * (64 if D <= 64 else 128) + segments * H * D * (Dv + 1), dtype=torch.float32,
+                                  device=q.device)
+            self.launches += 1 + 2 * int(segments > num_seqs)
+            self._call("linear_state", "q3_decayed_segment_scan", "decayed_state_scan", *args, seg, segments, _ptr(scratch), T)
             return out
         self._call("linear_state", "q3_decayed_state_scan", "decayed_state_scan", *args)
         return out
 
     def _scan_segment(self, T, num_seqs, H, D, Dv) -> int:
         """Tokens per segment of a decayed state scan, or 0 for the scan without segments: steps of many tokens per sequence
-        with keys of up to 128.  A multiple of 16, at least 32, for about two blocks per SM."""
-        if not self.scan_segments or D > 128 or T < max(64, 8 * num_seqs):
+        with keys of up to 128, whose rows (fp32, three per token and head) stay under 1 GiB.  At least 32, for two blocks
+        per SM (fewer and longer ones leave SMs with one)."""
+        if not self.scan_segments or D > 128 or T < max(64, 8 * num_seqs) or T * H * (64 if D <= 64 else 128) * 12 > 1 << 30:
             return 0
         blocks = H * -(-Dv // (128 if D <= 64 else 64))
-        return max(32, 16 * -(-T // (16 * max(1, 2 * self.SM_COUNT // blocks))))
+        return max(32, -(-T // max(1, 2 * self.SM_COUNT // blocks - (num_seqs - 1))))
 
     def stabilised_gates(self, zi, zf, *, i_bias, f_bias, cap, m_state, cu_seqlens, state_slots, num_seqs):
         """The gates of a matrix memory with exponential gates and a running maximum m per (sequence, head)
