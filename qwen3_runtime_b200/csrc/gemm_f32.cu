@@ -8,9 +8,13 @@
 // What bounds it: with many rows the FMA pipes (62 TFLOP/s for products of three registers, measured alone), with few
 // the weights' bytes.  Rows of both operands stay k-contiguous in shared memory (no transposition: cp.async moves 16
 // bytes at a time through a ring of stages), a thread reads four k-values of a row with one 16-byte load and uses each TM
-// or TN times.  A thread's rows and columns are (BM / TM) and (BN / TN) apart, so that the eight lanes of a load touch
-// eight neighbouring rows, whose stride of BK + 4 floats spreads them over all banks.  Since K may not be cut, an output
-// too small for large tiles gets smaller ones (SHAPES).
+// or TN times.  A thread's rows and columns are (BM / TM) and (BN / TN) apart, so that a load touches neighbouring rows,
+// whose stride of BK + 4 floats spreads them over all banks.  A 16-byte load takes two cycles of shared memory if lanes
+// that differ in bit 0, or those that differ in bit 1, read the same address, and four otherwise (measured): columns come
+// from lane bits 0, 2, 3 and rows from bits 1, 4, so that both operands' loads are of the first kind (32 x 32 tiles 26 ->
+// 35 TFLOP/s, 32 x 64 40 -> 42).  Long slices of k in two or three stages beat short ones in four or more (64 x 64: 742 ->
+// 696 us at 300 x 2560 -> 19456), and tiles of 128 rows or columns are nowhere the fastest.  Since K may not be cut, an
+// output too small for large tiles gets smaller ones (SHAPES).
 #include "common.cuh"
 
 #include <stdint.h>
@@ -38,7 +42,9 @@ gemm_f32_kernel(const float* __restrict__ A, int lda, const float* __restrict__ 
   static_assert(TX % 8 == 0 && TY % 4 == 0, "a warp is 4 x 8 threads");
   extern __shared__ __align__(16) float smem[];  // [STAGES][BM + BN][LD]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tx = (lane & 7) + 8 * (warp % (TX / 8)), ty = (lane >> 3) + 4 * (warp / (TX / 8));
+  // columns from lane bits 0, 2, 3 and rows from bits 1, 4 (see above)
+  const int tx = ((lane & 1) | ((lane >> 1) & 6)) + 8 * (warp % (TX / 8));
+  const int ty = (((lane >> 1) & 1) | ((lane >> 3) & 2)) + 4 * (warp / (TX / 8));
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   const int steps = (K + BK - 1) / BK;
   // a thread copies the same columns of rows PER apart in every step
@@ -136,16 +142,16 @@ int launch_tile(const float* A, int lda, const float* W, int ldw, float* C, int 
 }
 
 // Time of a product on a tile shape, about ns per k-value: `first` where every SM has one tile at most, `more` for each
-// further one.  Fitted to the choice, not to the times: over 50 products of 1..1000 rows at the Qwen3-4B and 8B sizes the
-// shape chosen is 0.4 % slower than the best one on average and 5 % at most.  Measured (us; one shape of 128 x 128 with
-// single-float loads took 2045 for both products of 300 rows): 300 x 2560 -> 19456: 761, 300 x 9728 -> 2560: 463, 1000
-// rows 46 TFLOP/s, one row 114 and 101.
+// further one.  Fitted to the choice, not to the times: over 147 products of 1..1000 rows at the Qwen3-4B and 8B sizes and
+// one of 2048 -> 1024 the shape chosen is 0.1 % slower than the best one on average and 4 % at most.  Measured (us; one
+// shape of 128 x 128 with single-float loads took 2045 for both products of 300 rows): 300 x 2560 -> 19456: 700, 300 x 9728
+// -> 2560: 414, 1000 rows 48 TFLOP/s, one row 84 and 88.
 struct Shape {
   int bm, bn;
   float first, more;
 };
-constexpr Shape SHAPES[] = {{128, 128, 115.4f, 149.4f}, {64, 128, 65.9f, 45.5f}, {64, 64, 38.7f, 23.7f},
-                            {32, 64, 15.8f, 14.2f},     {32, 32, 17.7f, 13.8f},  {16, 16, 5.4f, 4.6f}};
+constexpr Shape SHAPES[] = {{16, 32, 3.91f, 4.4f}, {64, 64, 21.7f, 11.8f}, {32, 64, 13.0f, 6.7f},
+                            {32, 32, 6.6f, 6.5f}, {16, 64, 12.9f, 4.3f},  {16, 16, 0.f, 3.5f}};
 constexpr int NUM_SHAPES = sizeof(SHAPES) / sizeof(SHAPES[0]);
 
 }  // namespace
@@ -174,11 +180,11 @@ Q3_EXPORT int q3_gemm_f32(const float* A, int lda, const float* W, int ldw, floa
   }
   const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
   switch (tile) {
-    case 0: return launch_tile<128, 128, 16, 8, 8, 4>(A, lda, W, ldw, C, ldc, M, N, K, vec, stream);
-    case 1: return launch_tile<64, 128, 16, 8, 8, 4>(A, lda, W, ldw, C, ldc, M, N, K, vec, stream);
-    case 2: return launch_tile<64, 64, 16, 4, 8, 4>(A, lda, W, ldw, C, ldc, M, N, K, vec, stream);
-    case 3: return launch_tile<32, 64, 32, 4, 4, 4>(A, lda, W, ldw, C, ldc, M, N, K, vec, stream);
-    case 4: return launch_tile<32, 32, 32, 2, 4, 6>(A, lda, W, ldw, C, ldc, M, N, K, vec, stream);
+    case 0: return launch_tile<16, 32, 64, 2, 4, 4>(A, lda, W, ldw, C, ldc, M, N, K, vec, stream);
+    case 1: return launch_tile<64, 64, 32, 8, 4, 3>(A, lda, W, ldw, C, ldc, M, N, K, vec, stream);
+    case 2: return launch_tile<32, 64, 64, 4, 4, 2>(A, lda, W, ldw, C, ldc, M, N, K, vec, stream);
+    case 3: return launch_tile<32, 32, 64, 2, 4, 3>(A, lda, W, ldw, C, ldc, M, N, K, vec, stream);
+    case 4: return launch_tile<16, 64, 64, 4, 4, 3>(A, lda, W, ldw, C, ldc, M, N, K, vec, stream);
     default: return launch_tile<16, 16, 64, 2, 1, 7>(A, lda, W, ldw, C, ldc, M, N, K, vec, stream);
   }
 }
