@@ -381,6 +381,9 @@ Q3_EXPORT int q3_delta_scan(int dtype, const float* qn, const float* kn, const v
 // delta_chunk_rows: everything that does not depend on the state, a record of DC_REC floats per (chunk, head):
 // [DP][32] (G k | G q, transposed), [16][DP] the decayed-to-the-end keys, [DP] G_last, W and B [16][16].  Chunks of
 // sequence b start at place cu_seqlens[b] / 16 + b; tokens beyond a portion's end are k = q = 0, g = 1, beta = 0.
+// Its pair products run down j with the decays' products in registers, 16 lanes to a row, and 30 shuffles fold a row's
+// sums (five per sum before); the substitution for W, a chain of 120 multiply-adds in 16 lanes, runs beside the record's
+// writing, which is in whole rows of 128 bytes.  2048 tokens of 16 heads: 48 -> 39 us.
 // delta_chunk_scan: one block per (16 value columns, head, sequence); the state's columns stay in registers (and, for
 // the products with it, in shared memory), the next chunks' records are on their way while one is worked on.
 #define DC_C 16
@@ -416,86 +419,126 @@ delta_chunk_rows_kernel(const float* __restrict__ qn, const float* __restrict__ 
   const int n = s_n;
   const long t0 = s_t0;
   if (n <= 0) return;
-  for (int x = tid; x < DC_C * DP; x += 256) {
+  // (whole 16 bytes where rows are made of them)
+  const bool vec = D % 4 == 0 && (((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)g) & 15) == 0;
+#pragma unroll
+  for (int x = tid * 4; x < DC_C * DP; x += 1024) {
     const int c = x / DP, i = x - c * DP;
-    const bool live = c < n && i < D;
-    ks[c][i] = live ? kn[((t0 + c) * G + gh) * D + i] : 0.f;
-    qs[c][i] = live ? qn[((t0 + c) * G + gh) * D + i] : 0.f;
-    gs[c][i] = live ? g[((t0 + c) * H + h) * D + i] : 1.f;
+    const long gi = ((t0 + c) * G + gh) * D + i, hi = ((t0 + c) * H + h) * D + i;
+    float4 k4 = make_float4(0.f, 0.f, 0.f, 0.f), q4 = k4, g4 = make_float4(1.f, 1.f, 1.f, 1.f);
+    if (c < n && i < D) {
+      if (vec) {
+        k4 = *reinterpret_cast<const float4*>(kn + gi);
+        q4 = *reinterpret_cast<const float4*>(qn + gi);
+        g4 = *reinterpret_cast<const float4*>(g + hi);
+      } else {
+        const bool in1 = i + 1 < D, in2 = i + 2 < D, in3 = i + 3 < D;
+        k4 = make_float4(kn[gi], in1 ? kn[gi + 1] : 0.f, in2 ? kn[gi + 2] : 0.f, in3 ? kn[gi + 3] : 0.f);
+        q4 = make_float4(qn[gi], in1 ? qn[gi + 1] : 0.f, in2 ? qn[gi + 2] : 0.f, in3 ? qn[gi + 3] : 0.f);
+        g4 = make_float4(g[hi], in1 ? g[hi + 1] : 1.f, in2 ? g[hi + 2] : 1.f, in3 ? g[hi + 3] : 1.f);
+      }
+    }
+    *reinterpret_cast<float4*>(&ks[c][i]) = k4;
+    *reinterpret_cast<float4*>(&qs[c][i]) = q4;
+    *reinterpret_cast<float4*>(&gs[c][i]) = g4;
   }
   if (tid < DC_C) be[tid] = tid < n ? beta[(t0 + tid) * H + h] : 0.f;
   __syncthreads();
+  {  // rows i of A and B, i = warp in the even lanes and 15 - warp in the odd ones; 16 lanes share the channels
+    constexpr int E = DP / 64;
+    const int i = lane & 1 ? DC_C - 1 - warp : warp, cl = lane >> 1;
+    float v[2 * DC_C];  // A_ij, then B_ij, this lane's channels
+    float wk[4 * E], wq[4 * E], qi[4 * E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const float4 q4 = *reinterpret_cast<const float4*>(&qs[i][cl * 4 + 64 * e]);
+      qi[4 * e] = q4.x; qi[4 * e + 1] = q4.y; qi[4 * e + 2] = q4.z; qi[4 * e + 3] = q4.w;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) wk[4 * e + m] = wq[4 * e + m] = 0.f;  // until j comes down to i
+    }
+#pragma unroll
+    for (int j = DC_C - 1; j >= 0; --j) {
+      float a = 0.f, b = 0.f;
+      if (j <= DC_C - 1 - warp) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          const float4 k4 = *reinterpret_cast<const float4*>(&ks[j][cl * 4 + 64 * e]);
+          const float4 g4 = *reinterpret_cast<const float4*>(&gs[j][cl * 4 + 64 * e]);
+          const float kj[4] = {k4.x, k4.y, k4.z, k4.w}, gj[4] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+          for (int m = 0; m < 4; ++m) {
+            float &x = wk[4 * e + m], &y = wq[4 * e + m];
+            x = j == i ? kj[m] : x;
+            y = j == i ? qi[4 * e + m] : y;
+            a = fmaf(x, kj[m], a);
+            b = fmaf(y, kj[m], b);
+            x *= gj[m];
+            y *= gj[m];
+          }
+        }
+      }
+      v[j] = a;
+      v[DC_C + j] = b;
+    }
+    // the sums over the 16 lanes: a lane gives half of its values away at each step and has two of them in the end
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int half = DC_C >> s;
+      const bool up = (cl >> s) & 1;
+#pragma unroll
+      for (int x = 0; x < half; ++x) {
+        const float give = up ? v[x] : v[x + half];
+        v[x] = (up ? v[x + half] : v[x]) + __shfl_xor_sync(0xffffffffu, give, 2 << s);
+      }
+    }
+    const int j = 4 * (cl & 2) + (cl & 4) + 2 * ((cl >> 3) & 1);
+    float* dst = cl & 1 ? &bs[i][j] : &as[i][j];  // (A's diagonal is not used)
+    dst[0] = v[0];
+    dst[1] = v[1];
+  }
+  __syncthreads();
   float* rec = records + ((long)place * H + h) * DC_REC(DP);
-  if (tid < DP) {  // the keys and queries decayed from the chunk's start, a channel's 32 values side by side
-    float* dst = rec + tid * 32;
+  if (warp == 0) {  // a chain of 120 multiply-adds while the other warps write the rest of the record
+    if (tid < DC_C) {  // column tid of W by forward substitution
+      float x[DC_C];
+#pragma unroll
+      for (int i = 0; i < DC_C; ++i) {
+        float acc = i == tid ? 1.f : 0.f;
+#pragma unroll
+        for (int j = 0; j < i; ++j) acc = fmaf(-as[i][j], x[j], acc);
+        x[i] = be[i] * acc;
+        rec[49 * DP + i * DC_C + tid] = x[i];
+      }
+    }
+    return;
+  }
+  const int at = tid - 32;
+  for (int x = at; x < 8 * DP; x += 224) {  // the keys and queries decayed from the chunk's start, four tokens of a channel
+    const int d = x >> 3, c0 = (x & 3) * 4;
     float run = 1.f;
 #pragma unroll
-    for (int c = 0; c < DC_C; c += 4) {
-      float a[4], b[4];
+    for (int c = 0; c < DC_C - 4; ++c)
+      if (c < c0) run *= gs[c][d];
+    const float(*src)[DP] = x & 4 ? qs : ks;
+    float r[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        run *= gs[c + e][tid];
-        a[e] = run * ks[c + e][tid];
-        b[e] = run * qs[c + e][tid];
-      }
-      *reinterpret_cast<float4*>(dst + c) = make_float4(a[0], a[1], a[2], a[3]);
-      *reinterpret_cast<float4*>(dst + DC_C + c) = make_float4(b[0], b[1], b[2], b[3]);
+    for (int e = 0; e < 4; ++e) {
+      run *= gs[c0 + e][d];
+      r[e] = run * src[c0 + e][d];
     }
-    rec[48 * DP + tid] = run;
-  } else if (tid < 2 * DP) {  // the keys decayed to the chunk's end
-    const int i = tid - DP;
+    *reinterpret_cast<float4*>(rec + 4 * x) = make_float4(r[0], r[1], r[2], r[3]);
+    if ((x & 7) == 3) rec[48 * DP + d] = run;
+  }
+  if (at < DP) {  // the keys decayed to the chunk's end
     float run = 1.f;
 #pragma unroll
     for (int c = DC_C - 1; c >= 0; --c) {
-      rec[32 * DP + c * DP + i] = run * ks[c][i];
-      run *= gs[c][i];
+      rec[32 * DP + c * DP + at] = run * ks[c][at];
+      run *= gs[c][at];
     }
   }
-  constexpr int E = DP / 32;
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {  // rows i and 15 - i: every warp the same work
-    const int i = half ? DC_C - 1 - warp : warp;
-    float wk[E], wq[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      wk[e] = ks[i][lane + 32 * e];
-      wq[e] = qs[i][lane + 32 * e];
-    }
-    for (int j = i; j >= 0; --j) {
-      float a = 0.f, b = 0.f;
-#pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const float kj = ks[j][lane + 32 * e];
-        a = fmaf(wk[e], kj, a);
-        b = fmaf(wq[e], kj, b);
-        const float gj = gs[j][lane + 32 * e];
-        wk[e] *= gj;
-        wq[e] *= gj;
-      }
-      a = warp_sum(a);
-      b = warp_sum(b);
-      if (lane == 0) {
-        as[i][j] = a;  // (the diagonal is not used)
-        bs[i][j] = b;
-      }
-    }
-  }
-  __syncthreads();
-  if (tid < DC_C) {  // column tid of W by forward substitution
-    float x[DC_C];
-#pragma unroll
-    for (int i = 0; i < DC_C; ++i) {
-      float acc = i == tid ? 1.f : 0.f;
-#pragma unroll
-      for (int j = 0; j < i; ++j) acc = fmaf(-as[i][j], x[j], acc);
-      x[i] = be[i] * acc;
-      rec[49 * DP + i * DC_C + tid] = x[i];
-    }
-  } else if (tid >= 64 && tid < 64 + DC_C * 4) {
-    const int i = (tid - 64) >> 2, j0 = ((tid - 64) & 3) * 4;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) rec[49 * DP + DC_C * DC_C + i * DC_C + j0 + e] = j0 + e <= i ? bs[i][j0 + e] : 0.f;
-  }
+  for (int x = at; x < DC_C * DC_C; x += 224)
+    rec[49 * DP + DC_C * DC_C + x] = x % DC_C <= x / DC_C ? bs[x / DC_C][x % DC_C] : 0.f;
 }
 
 __device__ __forceinline__ void ds_copy16(float* dst, const float* src) {
@@ -532,25 +575,29 @@ delta_chunk_scan_kernel(const float* __restrict__ records, const T* __restrict__
   };
 #pragma unroll
   for (int c = 0; c < STAGES - 1; ++c) load(c);
-  // this thread's rows and columns of the state
-  const int d0 = (tid >> 2) * RD, c0 = (tid & 3) * 4;
+  // Lane bits 0 and 2 choose four columns, bits 1, 3 and 4 the rows: lanes that differ in bit 0 (or in bit 1) then read the
+  // same address, and a 16-byte load takes two cycles of shared memory instead of four.
+  const int c0 = ((lane & 1) | ((lane >> 1) & 2)) * 4, group = ((lane >> 1) & 1) | ((lane >> 2) & 6);
+  const int d0 = warp * 8 * RD + group;  // this thread's rows of the state: d0 + 8 r
   float* Sg = state + ((long)state_slots[b] * H + h) * (long)D * Dv;
   float S[RD][4];
 #pragma unroll
   for (int r = 0; r < RD; ++r) {
 #pragma unroll
     for (int e = 0; e < 4; ++e)
-      S[r][e] = d0 + r < D && col0 + c0 + e < Dv ? Sg[(long)(d0 + r) * Dv + col0 + c0 + e] : 0.f;
-    *reinterpret_cast<float4*>(Ss + (d0 + r) * VT + c0) = make_float4(S[r][0], S[r][1], S[r][2], S[r][3]);
+      S[r][e] = d0 + 8 * r < D && col0 + c0 + e < Dv ? Sg[(long)(d0 + 8 * r) * Dv + col0 + c0 + e] : 0.f;
+    *reinterpret_cast<float4*>(Ss + (d0 + 8 * r) * VT + c0) = make_float4(S[r][0], S[r][1], S[r][2], S[r][3]);
   }
-  const int row = tid >> 4, col = tid & 15;  // the chunk's token and the value column of the small products
+  // the chunk's token and the value column of the small products; a warp's tokens are four apart, whose partial sums lie in
+  // different banks
+  const int row = (warp & 3) + 8 * (warp >> 2) + 4 * (lane >> 4), col = tid & 15;
   const bool col_in = col0 + col < Dv;
   auto value = [&](int c) {
     const long t = t0 + c * DC_C + row;
     return col_in && t < t1 ? to_f32(vc[(t * H + h) * Dv + col0 + col]) : 0.f;
   };
   float v_next = value(0);
-  const int rt = (lane >> 2) * 4, ct = (lane & 3) * 4;
+  const int rt = group * 4, ct = c0;
   for (int c = 0; c < chunks; ++c) {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2));
     __syncthreads();  // the record and the state in shared memory are complete; nobody reads the last record any more
@@ -620,7 +667,7 @@ delta_chunk_scan_kernel(const float* __restrict__ records, const T* __restrict__
     const float* kend = rec + 32 * DP;
 #pragma unroll
     for (int r = 0; r < RD; ++r) {
-      const float gl = rec[48 * DP + d0 + r];
+      const float gl = rec[48 * DP + d0 + 8 * r];
 #pragma unroll
       for (int e = 0; e < 4; ++e) S[r][e] *= gl;
     }
@@ -629,7 +676,7 @@ delta_chunk_scan_kernel(const float* __restrict__ records, const T* __restrict__
       const float4 u4 = *reinterpret_cast<const float4*>(us + j * VT + c0);
 #pragma unroll
       for (int r = 0; r < RD; ++r) {
-        const float kk = kend[j * DP + d0 + r];
+        const float kk = kend[j * DP + d0 + 8 * r];
         S[r][0] = fmaf(kk, u4.x, S[r][0]);
         S[r][1] = fmaf(kk, u4.y, S[r][1]);
         S[r][2] = fmaf(kk, u4.z, S[r][2]);
@@ -638,13 +685,13 @@ delta_chunk_scan_kernel(const float* __restrict__ records, const T* __restrict__
     }
 #pragma unroll
     for (int r = 0; r < RD; ++r)
-      *reinterpret_cast<float4*>(Ss + (d0 + r) * VT + c0) = make_float4(S[r][0], S[r][1], S[r][2], S[r][3]);
+      *reinterpret_cast<float4*>(Ss + (d0 + 8 * r) * VT + c0) = make_float4(S[r][0], S[r][1], S[r][2], S[r][3]);
   }
 #pragma unroll
   for (int r = 0; r < RD; ++r)
 #pragma unroll
     for (int e = 0; e < 4; ++e)
-      if (d0 + r < D && col0 + c0 + e < Dv) Sg[(long)(d0 + r) * Dv + col0 + c0 + e] = S[r][e];
+      if (d0 + 8 * r < D && col0 + c0 + e < Dv) Sg[(long)(d0 + 8 * r) * Dv + col0 + c0 + e] = S[r][e];
 }
 
 template <typename T, int DP>
@@ -664,10 +711,11 @@ static int launch_delta_chunks(cudaStream_t stream, int num_tokens, int num_seqs
       return Q3_ERR_LAUNCH;
     configured = true;
   }
-  return launch_pdl(kernel, dim3((Dv + 15) / 16, H, num_seqs), dim3(256), smem, stream, (const float*)records, (const T*)vc,
-                    state, cu_seqlens, state_slots, out, H, D, Dv) == cudaSuccess
-             ? Q3_OK
-             : Q3_ERR_LAUNCH;
+  // Not as a dependent launch: its blocks would start between the last blocks of the kernel before, two of the longest
+  // sequence's on some SMs while others have none (2048 tokens: the scan 278 us instead of 225).
+  kernel<<<dim3((Dv + 15) / 16, H, num_seqs), dim3(256), smem, stream>>>(records, (const T*)vc, state, cu_seqlens,
+                                                                        state_slots, out, H, D, Dv);
+  return q3_launch_status();
 }
 
 // The same as q3_delta_scan for key sizes up to 128, in chunks; records: (num_tokens / 16 + num_seqs) * H * (49 * DP +
