@@ -28,7 +28,7 @@
 // of the double buffer afterwards.  A token's arithmetic does not depend on where the step's portion
 // starts or ends, so the result has the same bits however a prompt is cut.
 //
-// segment_scan: the same recurrence for prompts.  The scan above is a chain over a sequence's tokens, 0.21 us each, with
+// segment_scan: the same recurrence for prompts in bfloat16.  The scan above is a chain over a sequence's tokens, 0.21 us each, with
 // one block per (head, 16 columns): 2048 tokens of 16 heads took 430 us with the SMs mostly idle.  Here a sequence is cut
 // into segments of `seg` tokens: (1) every segment but a sequence's last works out the state it would leave behind if it
 // began with zeros, and the product of its decays; (2) the segments' first states follow one from another,
@@ -554,7 +554,7 @@ static cudaError_t launch_segments(const ScanArgs& a, int num_tokens, int segmen
   return e;
 }
 
-// The same arguments as q3_decayed_state_scan, key sizes up to 128: in segments of `seg` tokens.  segments: the number of
+// The same arguments as q3_decayed_state_scan, bfloat16, key sizes up to 128: in segments of `seg` tokens.  segments: the number of
 // them, sum over the sequences of ceil(tokens / seg), or more; scratch: fp32, 16-byte aligned, [num_tokens * H * 3 * DP +
 // segments * H * D * (Dv + 1)] with DP = 64 (D <= 64) or 128.
 Q3_EXPORT int q3_decayed_segment_scan(int dtype, const void* q, long q_stride, const void* k, long k_stride, const void* v,
@@ -572,7 +572,7 @@ Q3_EXPORT int q3_decayed_segment_scan(int dtype, const void* q, long q_stride, c
   if (decay_mode < 0 || decay_mode > 1 || ones_col < 0 || ones_col > 1 || Dv - ones_col < 1) return Q3_ERR_ARGUMENT;
   if (rot_pairs < 0 || 2 * rot_pairs > D || (rot_pairs && (!inv_freq || !positions))) return Q3_ERR_ARGUMENT;
   if (H < 1 || D < 1 || Dv < 1 || H > 65535 || num_seqs > 65535) return Q3_ERR_ARGUMENT;
-  if (D > 128 || (dtype != Q3_DTYPE_F32 && dtype != Q3_DTYPE_BF16)) return Q3_ERR_UNSUPPORTED;
+  if (D > 128 || dtype != Q3_DTYPE_BF16) return Q3_ERR_UNSUPPORTED;
   if (num_seqs == 0 || num_tokens == 0) return Q3_OK;
   const long rows = (long)num_tokens * H * 3 * (D <= 64 ? 64 : 128);
   const ScanArgs a = {q, k, v, z, q_stride, k_stride, v_stride, z_stride, z_bias, inv_tau, head_decay, inv_freq, rot_pairs,
@@ -580,19 +580,12 @@ Q3_EXPORT int q3_decayed_segment_scan(int dtype, const void* q, long q_stride, c
                       tok_decay, tok_kscale, ones_col, bonus, seg, scratch + rows, scratch + rows + (long)segments * H * D * Dv,
                       scratch};
   cudaError_t e;
-#define Q3_SEGMENTS(T)                                                                       \
-  if (D <= 64)                                                                               \
-    e = bonus ? launch_segments<T, 64, 16, true>(a, num_tokens, segments, stream)                        \
-              : launch_segments<T, 64, 16, false>(a, num_tokens, segments, stream);                      \
-  else                                                                                       \
-    e = bonus ? launch_segments<T, 128, 8, true>(a, num_tokens, segments, stream)                       \
-              : launch_segments<T, 128, 8, false>(a, num_tokens, segments, stream)
-  if (dtype == Q3_DTYPE_F32) {
-    Q3_SEGMENTS(float);
-  } else {
-    Q3_SEGMENTS(bf16);
-  }
-#undef Q3_SEGMENTS
+  if (D <= 64)
+    e = bonus ? launch_segments<bf16, 64, 16, true>(a, num_tokens, segments, stream)
+              : launch_segments<bf16, 64, 16, false>(a, num_tokens, segments, stream);
+  else
+    e = bonus ? launch_segments<bf16, 128, 8, true>(a, num_tokens, segments, stream)
+              : launch_segments<bf16, 128, 8, false>(a, num_tokens, segments, stream);
   return e == cudaSuccess ? Q3_OK : Q3_ERR_LAUNCH;
 }
 

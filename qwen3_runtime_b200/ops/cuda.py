@@ -724,7 +724,8 @@ class CudaOps:
                 pairs, _ptr(positions), float(q_scale), float(k_scale), _ptr(state), _ptr(cu_seqlens), _ptr(state_slots),
                 _ptr(out), int(num_seqs), H, D, Dv, modes[decay_mode], _ptr(token_decay), _ptr(token_k_scale),
                 int(bool(ones_column)), _ptr(bonus))
-        seg = self._scan_segment(T, int(num_seqs), H, D, Dv)
+        # (float32 stays token by token: the same bits however a prompt is cut)
+        seg = self._scan_segment(T, int(num_seqs), H, D, Dv) if q.dtype == torch.bfloat16 else 0
         if seg:
             segments = T // seg + int(num_seqs)  # at least the sum of ceil(tokens / seg)
             scratch = torch.empty(T * H * 3 * (64 if D <= 64 else 128) + segments * H * D * (Dv + 1), dtype=torch.float32,
@@ -1042,11 +1043,12 @@ class CudaOps:
     # (query, key) pairs per cached row from which a step's prompts expand the keys and values (see latent_expand_rows)
     LATENT_EXPAND_PAIRS = 32
 
-    def latent_expand_rows(self, step, *, dim, rot_dim, value_dim, kv_rank, window, dtype) -> int:
+    def latent_expand_rows(self, step, *, heads, dim, rot_dim, value_dim, kv_rank, window, dtype) -> int:
         """How many cached rows :meth:`latent_attention_expanded` would expand for this step, or 0 where attention in the
         latent space is the better one (or the only one).  A pair costs 2 x (kv_rank + rot_dim + kv_rank) flops in the
         latent space (1088 products) against 320 with keys of 192 and values of 128, on a kernel that also runs at three
-        times the rate; expanding a row costs 2 x kv_rank x 256 flops per head once, however many queries see it."""
+        times the rate; expanding a row costs 2 x kv_rank x 256 flops per head once, however many queries see it.  The
+        expanded rows (512 bytes per head) stay under 2 GiB."""
         if not (self.latent_expand and step is not None and dtype == torch.bfloat16 and not step.decode_only
                 and not step.captured_width and (dim, rot_dim, value_dim) == (128, 64, 128) and kv_rank % 8 == 0):
             return 0
@@ -1058,7 +1060,7 @@ class CudaOps:
             full = min(n, max(0, kv - window)) if window else 0  # tokens that see a whole window
             pairs += full * window if full else 0
             pairs += (n - full) * (kv - n) + (n - full) * (n - full + 1) // 2
-        return rows if pairs >= self.LATENT_EXPAND_PAIRS * rows else 0
+        return rows if pairs >= self.LATENT_EXPAND_PAIRS * rows and rows * heads * 512 <= 1 << 31 else 0
 
     def latent_attention_expanded(self, q, q_turned, expand, rows, *, pages, kv_rank, block_table, sink, out, page_size, scale,
                                   window, step):

@@ -157,7 +157,7 @@ class LatentAttention(Part):
         ctx_out = torch.empty((T, H, self.vdim), dtype=h.dtype, device=h.device)
         seen = 0
         if self.expand is not None:
-            seen = ops.latent_expand_rows(step, dim=self.dim, rot_dim=self.rot_dim, value_dim=self.vdim, kv_rank=self.kv_rank,
+            seen = ops.latent_expand_rows(step, heads=H, dim=self.dim, rot_dim=self.rot_dim, value_dim=self.vdim, kv_rank=self.kv_rank,
                                           window=self.window, dtype=h.dtype)
         if seen:
             q_turned = torch.empty((T, H, self.rot_dim), dtype=h.dtype, device=h.device)

@@ -157,7 +157,8 @@ def test_which_steps_expand(ops):
             cu.append(cu[-1] + n)
         step = SimpleNamespace(decode_only=kw.get("decode", False), captured_width=0, host_cu_seqlens=cu,
                                host_kv_lens=[c + n for c, n in spans])
-        return ops.latent_expand_rows(step, dim=128, rot_dim=64, value_dim=128, kv_rank=512, window=window, dtype=torch.bfloat16)
+        return ops.latent_expand_rows(step, heads=3, dim=128, rot_dim=64, value_dim=128, kv_rank=512, window=window,
+                                      dtype=torch.bfloat16)
 
     assert rows([(0, 2048)], None) == 2048 and rows([(0, 63)], None) == 63 and rows([(0, 62)], None) == 0
     assert rows([(8000, 8)], None) == 0 and rows([(8000, 8)], 1024) == 0

@@ -90,6 +90,7 @@ def test_segments_against_float64_and_the_chain(ops, dtype, D, Dv, form):
             assert (ops._scan_segment(T, B, H, D, Dv + ones) > 0) == segments
             got[segments] = ops.decayed_state_scan(q.cuda(), k.cuda(), v.cuda(), state=state[segments], **kw).cpu().double()
         ops.scan_segments = True
+        assert dtype == torch.bfloat16 or torch.equal(got[True], got[False])  # float32 stays token by token
         at = [x + n for x, n in zip(at, lens)]
         # float32 sums of up to a few hundred addends (and float32 exponentials) against float64
         bound = 3e-5 * max(1.0, float(want.abs().max()))
