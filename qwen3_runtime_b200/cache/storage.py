@@ -92,19 +92,20 @@ class CacheStorage:
         """Fixed-size state starts from zero when a request starts or restarts."""
         if not slots:
             return
-        # runs of neighbouring slots, so that no index has to be copied to the device (a copy from pageable memory waits
-        # for the device: the step's launches would start only then)
-        runs: list[list[int]] = []
-        for slot in sorted(set(slots)):
-            if runs and runs[-1][1] == slot:
-                runs[-1][1] = slot + 1
-            else:
-                runs.append([slot, slot + 1])
+        count = self.scratch_slot + 1
+        if min(slots) < -count or max(slots) >= count:
+            raise IndexError(f"state slots are 0..{count - 1}, got {sorted(slots)}")
+        order = sorted({slot % count for slot in slots})
+        index = None
         for g, t in zip(self.layout.groups, self.tensors):
             if g.spec.paged:
                 continue
-            for a, b in runs:
-                t[:, a:b].zero_()
+            if order[-1] - order[0] + 1 == len(order):  # neighbours, as a single request's one slot: no index at all
+                t[:, order[0]:order[-1] + 1].zero_()
+                continue
+            if index is None:  # from pinned memory: a copy from pageable memory would wait for the device
+                index = torch.tensor(order, dtype=torch.long, pin_memory=t.is_cuda).to(t.device, non_blocking=True)
+            t.index_fill_(1, index, 0)
 
     def poison_pages(self, paged_index: int, pages: list[int], value: float = float("nan")) -> None:
         """Overwrite pages (tests: a page that is used again must not leak old contents)."""
