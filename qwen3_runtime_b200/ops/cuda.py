@@ -1047,20 +1047,35 @@ class CudaOps:
         """How many cached rows :meth:`latent_attention_expanded` would expand for this step, or 0 where attention in the
         latent space is the better one (or the only one).  A pair costs 2 x (kv_rank + rot_dim + kv_rank) flops in the
         latent space (1088 products) against 320 with keys of 192 and values of 128, on a kernel that also runs at three
-        times the rate; expanding a row costs 2 x kv_rank x 256 flops per head once, however many queries see it.  The
+        times the rate; expanding a row costs 2 x kv_rank x 256 flops per head once, however many queries see it.  Measured,
+        whole layers of 16, 32 and 128 heads, us in the latent space / expanded: 64 tokens 61 / 54, 75 / 71, 126 / 112; 64
+        behind 16,000 1229 / 362, 1241 / 431, 2500 / 790; 2000 beside 15 single tokens behind 4096 (33 pairs a row) 968 / 472,
+        1658 / 881; 500 beside 31 behind 512 (9 pairs a row) 173 / 192, 269 / 333, 792 / 1061: from 32 on none was slower.  The
+        answer is for the whole step: what shares it decides in which of the two ways a prompt's attention is rounded.  The
         expanded rows (512 bytes per head) stay under 2 GiB."""
         if not (self.latent_expand and step is not None and dtype == torch.bfloat16 and not step.decode_only
                 and not step.captured_width and (dim, rot_dim, value_dim) == (128, 64, 128) and kv_rank % 8 == 0):
             return 0
-        rows = pairs = 0
-        cu = step.host_cu_seqlens
-        for b, kv in enumerate(step.host_kv_lens):
-            n = cu[b + 1] - cu[b]
-            rows += kv - (max(0, kv - n - window + 1) // 64 * 64 if window else 0)
-            full = min(n, max(0, kv - window)) if window else 0  # tokens that see a whole window
-            pairs += full * window if full else 0
-            pairs += (n - full) * (kv - n) + (n - full) * (n - full + 1) // 2
+        rows, pairs = self._visible_rows_and_pairs(step, window)
         return rows if pairs >= self.LATENT_EXPAND_PAIRS * rows and rows * heads * 512 <= 1 << 31 else 0
+
+    @staticmethod
+    def _visible_rows_and_pairs(step, window):
+        """Cached rows that the step's tokens see (from a multiple of 64 on) and (query, key) pairs, once per step and
+        window: the layers of a step share the answer."""
+        seen = getattr(step, "extras", {})
+        key = ("visible_rows_and_pairs", window)
+        if key not in seen:
+            rows = pairs = 0
+            cu = step.host_cu_seqlens
+            for b, kv in enumerate(step.host_kv_lens):
+                n = cu[b + 1] - cu[b]
+                rows += kv - (max(0, kv - n - window + 1) // 64 * 64 if window else 0)
+                full = min(n, max(0, kv - window)) if window else 0  # tokens that see a whole window
+                pairs += full * window if full else 0
+                pairs += (n - full) * (kv - n) + (n - full) * (n - full + 1) // 2
+            seen[key] = rows, pairs
+        return seen[key]
 
     def latent_attention_expanded(self, q, q_turned, expand, rows, *, pages, kv_rank, block_table, sink, out, page_size, scale,
                                   window, step):

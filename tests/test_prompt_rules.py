@@ -1,0 +1,57 @@
+"""The kernel table's host-side rules for steps with prompts (no kernel runs)."""
+
+from __future__ import annotations
+
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from qwen3_runtime_b200.ops.cuda import CudaOps
+
+
+def _table():
+    """A kernel table of a B200 whose rules can be asked without a device."""
+    ops = object.__new__(CudaOps)
+    ops.SM_COUNT = 148
+    ops.latent_expand = ops.scan_segments = ops.differential_tc = ops.differential_tcgen05 = True
+    return ops
+
+
+class _Counted(list):
+    reads = 0
+
+    def __iter__(self):
+        self.reads += 1
+        return super().__iter__()
+
+
+def _step(spans):
+    cu = [0]
+    for _context, new in spans:
+        cu.append(cu[-1] + new)
+    return SimpleNamespace(decode_only=False, captured_width=0, host_cu_seqlens=cu, extras={},
+                           host_kv_lens=_Counted(c + n for c, n in spans))
+
+
+@pytest.mark.parametrize("window", [None, 100, 4096])
+def test_a_steps_layers_share_what_expanding_would_cost(window):
+    """Eager steps wait for the host: one walk over the step's sequences per step and window, not one per layer."""
+    ops = _table()
+    spans = [(0, 300), (777, 40)] + [(4096, 1)] * 40
+    rows = pairs = 0
+    for c, n in spans:
+        first = max(0, c + 1 - window) // 64 * 64 if window else 0
+        rows += c + n - first
+        pairs += sum(min(p + 1, window) if window else p + 1 for p in range(c, c + n))
+    step = _step(spans)
+    kw = dict(dim=128, rot_dim=64, value_dim=128, kv_rank=512, window=window, dtype=torch.bfloat16)
+    ops.LATENT_EXPAND_PAIRS = pairs / rows * 0.999
+    assert [ops.latent_expand_rows(step, heads=h, **kw) for h in (4, 4, 8, 4)] == [rows] * 4
+    ops.LATENT_EXPAND_PAIRS = pairs / rows * 1.001 + 1e-9
+    assert ops.latent_expand_rows(step, heads=4, **kw) == 0
+    assert step.host_kv_lens.reads == 1
+    kw["window"] = 77
+    ops.latent_expand_rows(step, heads=4, **kw)
+    ops.latent_expand_rows(_step(spans), heads=4, **kw)
+    assert step.host_kv_lens.reads == 2
