@@ -97,10 +97,12 @@ class LatentAttention(Part):
         # per head [kv_rank, dim]: the product that moves a query into the latent space contracts
         # over dim, which is the stored matrix's row index
         self.uk_t = tensors["uk"].reshape(H, self.dim, self.kv_rank).transpose(1, 2).contiguous()
-        self.uv = tensors["uv"].reshape(H, self.vdim, self.kv_rank).contiguous()
+        uv = tensors["uv"]
+        if self._expands():  # keys, then values of all heads from a latent, for prompts (ops.latent_expand_rows)
+            self.expand = torch.cat([tensors["uk"], uv], dim=0)
+            uv = self.expand[H * self.dim:]
+        self.uv = uv.reshape(H, self.vdim, self.kv_rank).contiguous()
         self.o_weight = tensors["o"].contiguous()
-        # keys and values of all heads from a latent, for prompts (ops.latent_expand_rows)
-        self.expand = torch.cat([tensors["uk"], tensors["uv"]], dim=0).contiguous() if self._expands() else None
         self.q_norm_weight = tensors.get("dq.norm")
         self.kv_norm_weight = tensors["dkv.norm"]
         self.sink = tensors.get("sink")

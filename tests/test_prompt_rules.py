@@ -55,3 +55,20 @@ def test_a_steps_layers_share_what_expanding_would_cost(window):
     ops.latent_expand_rows(step, heads=4, **kw)
     ops.latent_expand_rows(_step(spans), heads=4, **kw)
     assert step.host_kv_lens.reads == 2
+
+
+def test_a_latent_layer_keeps_its_value_rows_once():
+    from qwen3_runtime_b200.config import PartSpec
+    from qwen3_runtime_b200.parts.base import BuildContext, build_part
+
+    spec = PartSpec("latent_attention", dict(hidden_size=64, num_heads=2, dim=128, rot_dim=64, vdim=128, q_rank=32, kv_rank=16,
+                                             eps=1e-5, scale=0.1, window=None, sink=False,
+                                             position=PartSpec("rope_interleaved", dict(rotary_dim=64, theta=1e4))))
+    part = build_part("mixer", spec, BuildContext(dtype=torch.bfloat16, device=torch.device("cpu"), ops=_table()))
+    g = torch.Generator().manual_seed(0)
+    tensors = {n: torch.randn(s.shape, generator=g).to(torch.float32 if s.kind == "vector" else torch.bfloat16)
+               for n, s in part.param_specs().items()}
+    part.load(dict(tensors))
+    assert torch.equal(part.expand, torch.cat([tensors["uk"], tensors["uv"]]))
+    assert torch.equal(part.uv.reshape(-1, 16), tensors["uv"]) and part.uv.is_contiguous()
+    assert part.uv.untyped_storage().data_ptr() == part.expand.untyped_storage().data_ptr()
