@@ -168,12 +168,12 @@ _SIGNATURES = {
         "q3_decayed_state_scan": [c_int, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long,
                                   c_void_p, c_float, c_void_p, c_void_p, c_int, c_void_p, c_float, c_float, c_void_p,
                                   c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                                  c_int, c_void_p, c_void_p],
+                                  c_int, c_void_p, c_int, c_void_p],
         "q3_decayed_segment_scan": [c_int, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long,
                                   c_void_p, c_float, c_void_p, c_void_p, c_int, c_void_p, c_float, c_float, c_void_p,
                                   c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                                  c_int, c_void_p, c_int, c_int, c_void_p, c_int,
-                                    c_void_p],
+                                  c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
+                                    c_int, c_void_p],
         "q3_head_norm_gate": [c_int, c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p, c_long, c_void_p, c_long,
                               c_float, c_int, c_int, c_int, c_int, c_void_p],
         "q3_stabilised_gates": [c_int, c_void_p, c_void_p, c_long, c_void_p, c_void_p, c_float, c_void_p, c_void_p,
@@ -682,7 +682,7 @@ class CudaOps:
     def decayed_state_scan(self, q, k, v, *, state, cu_seqlens, state_slots, num_seqs, decay_logits=None,
                            decay_bias=None, tau=1.0, head_decay=None, inv_freq=None, positions=None, q_scale=1.0,
                            k_scale=1.0, decay_mode="sigmoid_pow", token_decay=None, token_k_scale=None, bonus=None,
-                           ones_column=False):
+                           ones_column=False, host_cu_seqlens=None):
         """``S_t = diag(a_t) S_(t-1) + k_t v_t^T``, ``o_t = S_t^T q_t`` per (sequence, head) on the float32
         state ``[slots, H, D, Dv]`` of the sequences' slots; returns float32 ``o`` ``[T, H, Dv]``.
         ``q, k`` ``[T, H, D]``, ``v`` ``[T, H, Dv]`` (views of wider rows allowed).  The decay is
@@ -725,16 +725,23 @@ class CudaOps:
                 _ptr(out), int(num_seqs), H, D, Dv, modes[decay_mode], _ptr(token_decay), _ptr(token_k_scale),
                 int(bool(ones_column)), _ptr(bonus))
         # (float32 stays token by token: the same bits however a prompt is cut)
-        seg = self._scan_segment(T, int(num_seqs), H, D, Dv) if q.dtype == torch.bfloat16 else 0
+        lens = [b - a for a, b in zip(host_cu_seqlens, host_cu_seqlens[1:])] if host_cu_seqlens else None
+        seg, shortest = self._scan_cut(T, int(num_seqs), H, D, Dv, lens) if q.dtype == torch.bfloat16 else (0, 0)
         if seg:
-            segments = T // seg + int(num_seqs)  # at least the sum of ceil(tokens / seg)
+            segments = sum(-(-n // seg) for n in lens if n >= shortest) if lens else T // seg + int(num_seqs)
             scratch = torch.empty(T * H * 3 * (64 if D <= 64 else 128) + segments * H * D * (Dv + 1), dtype=torch.float32,
                                   device=q.device)
-            self.launches += 1 + 2 * int(segments > num_seqs)
-            self._call("linear_state", "q3_decayed_segment_scan", "decayed_state_scan", *args, seg, segments, _ptr(scratch), T)
-            return out
-        self._call("linear_state", "q3_decayed_state_scan", "decayed_state_scan", *args)
+            cut = int((max(lens) if lens else T) > seg)
+            self.launches += 1 + 2 * cut
+            self._call("linear_state", "q3_decayed_segment_scan", "decayed_state_scan", *args, seg, shortest, segments, cut,
+                       _ptr(scratch), T)
+            if not lens or min(lens) >= shortest:
+                return out
+        self._call("linear_state", "q3_decayed_state_scan", "decayed_state_scan", *args, (shortest - 1) if seg else 0x7fffffff)
         return out
+
+    def _scan_cut(self, T, num_seqs, H, D, Dv, lens=None):
+        return self._scan_segment(T, num_seqs, H, D, Dv), 1
 
     def _scan_segment(self, T, num_seqs, H, D, Dv) -> int:
         """Tokens per segment of a decayed state scan, or 0 for the scan without segments: steps of many tokens per sequence
@@ -1638,9 +1645,12 @@ class CudaOps:
                 return out
             if (self.differential_tcgen05 and map_dim == 64 and value_dim == 128 and 128 % group == 0
                     and page_size in (8, 16, 32, 64) and out.stride(0) == num_heads * value_dim
-                    and not (window and chunk) and all(t.data_ptr() % 16 == 0 for t in (out, k_pages, v_pages))):
+                    and not (window and chunk) and step.max_kv_len * group >= 128
+                    and all(t.data_ptr() % 16 == 0 for t in (out, k_pages, v_pages))):
                 # both maps as the two row blocks of the tcgen05 kernel.  Against the mma.sync kernel below: 16 heads over 4,
-                # 2333 + 419 tokens 61 against 247 us
+                # 2333 + 419 tokens 61 against 247 us.  A step whose longest sequence fills no block of 128 rows is over before
+                # the kernel's set-up pays (whole layers of 16 heads, mma.sync / tcgen05: over 4, 2 tokens 29.8 / 31.8 us and 33
+                # tokens faster here; over 16, 33 tokens 33.9 / 36.0, 64 tokens 35.9 / 35.8, 128 tokens faster here)
                 cu = step.host_cu_seqlens
                 work = sum(-(-(cu[b + 1] - cu[b]) * group // 128) for b in range(step.num_seqs) if cu[b + 1] > cu[b])
                 self._call("attention_prefill_tc", "q3_diff_attention_prefill_tc", "differential_attention_tc", _ptr(q),
@@ -1652,7 +1662,7 @@ class CudaOps:
             if map_dim in (32, 64, 128) and value_dim in (64, 128):
                 cu = step.host_cu_seqlens
                 work = sum(-(-(cu[b + 1] - cu[b]) * group // 128) for b in range(step.num_seqs) if cu[b + 1] > cu[b])
-                self._call("attention_diff", "q3_diff_attention_prefill", "differential_attention_tc", _ptr(q),
+                self._call("attention_diff", "q3_diff_attention_prefill", "differential_attention_mma", _ptr(q),
                            q_stride, _ptr(k_pages), _ptr(v_pages), _ptr(block_table), block_table.shape[1],
                            _ptr(step.kv_lens), _ptr(step.cu_seqlens), _ptr(out), out.stride(0), step.num_seqs, work,
                            num_heads, num_kv_heads, map_dim, value_dim, page_size, float(scale), int(window or 0),
