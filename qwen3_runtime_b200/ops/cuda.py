@@ -168,12 +168,12 @@ _SIGNATURES = {
         "q3_decayed_state_scan": [c_int, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long,
                                   c_void_p, c_float, c_void_p, c_void_p, c_int, c_void_p, c_float, c_float, c_void_p,
                                   c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                                  c_int, c_void_p, c_int, c_void_p],
+                                  c_int, c_void_p, c_void_p],
         "q3_decayed_segment_scan": [c_int, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long,
                                   c_void_p, c_float, c_void_p, c_void_p, c_int, c_void_p, c_float, c_float, c_void_p,
                                   c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                                  c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
-                                    c_int, c_void_p],
+                                  c_int, c_void_p, c_int, c_int, c_void_p, c_int,
+                                    c_void_p],
         "q3_head_norm_gate": [c_int, c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p, c_long, c_void_p, c_long,
                               c_float, c_int, c_int, c_int, c_int, c_void_p],
         "q3_stabilised_gates": [c_int, c_void_p, c_void_p, c_long, c_void_p, c_void_p, c_float, c_void_p, c_void_p,
@@ -682,7 +682,7 @@ class CudaOps:
     def decayed_state_scan(self, q, k, v, *, state, cu_seqlens, state_slots, num_seqs, decay_logits=None,
                            decay_bias=None, tau=1.0, head_decay=None, inv_freq=None, positions=None, q_scale=1.0,
                            k_scale=1.0, decay_mode="sigmoid_pow", token_decay=None, token_k_scale=None, bonus=None,
-                           ones_column=False, host_cu_seqlens=None):
+                           ones_column=False):
         """``S_t = diag(a_t) S_(t-1) + k_t v_t^T``, ``o_t = S_t^T q_t`` per (sequence, head) on the float32
         state ``[slots, H, D, Dv]`` of the sequences' slots; returns float32 ``o`` ``[T, H, Dv]``.
         ``q, k`` ``[T, H, D]``, ``v`` ``[T, H, Dv]`` (views of wider rows allowed).  The decay is
@@ -725,23 +725,16 @@ class CudaOps:
                 _ptr(out), int(num_seqs), H, D, Dv, modes[decay_mode], _ptr(token_decay), _ptr(token_k_scale),
                 int(bool(ones_column)), _ptr(bonus))
         # (float32 stays token by token: the same bits however a prompt is cut)
-        lens = [b - a for a, b in zip(host_cu_seqlens, host_cu_seqlens[1:])] if host_cu_seqlens else None
-        seg, shortest = self._scan_cut(T, int(num_seqs), H, D, Dv, lens) if q.dtype == torch.bfloat16 else (0, 0)
+        seg = self._scan_segment(T, int(num_seqs), H, D, Dv) if q.dtype == torch.bfloat16 else 0
         if seg:
-            segments = sum(-(-n // seg) for n in lens if n >= shortest) if lens else T // seg + int(num_seqs)
+            segments = T // seg + int(num_seqs)  # at least the sum of ceil(tokens / seg)
             scratch = torch.empty(T * H * 3 * (64 if D <= 64 else 128) + segments * H * D * (Dv + 1), dtype=torch.float32,
                                   device=q.device)
-            cut = int((max(lens) if lens else T) > seg)
-            self.launches += 1 + 2 * cut
-            self._call("linear_state", "q3_decayed_segment_scan", "decayed_state_scan", *args, seg, shortest, segments, cut,
-                       _ptr(scratch), T)
-            if not lens or min(lens) >= shortest:
-                return out
-        self._call("linear_state", "q3_decayed_state_scan", "decayed_state_scan", *args, (shortest - 1) if seg else 0x7fffffff)
+            self.launches += 1 + 2 * int(segments > num_seqs)
+            self._call("linear_state", "q3_decayed_segment_scan", "decayed_state_scan", *args, seg, segments, _ptr(scratch), T)
+            return out
+        self._call("linear_state", "q3_decayed_state_scan", "decayed_state_scan", *args)
         return out
-
-    def _scan_cut(self, T, num_seqs, H, D, Dv, lens=None):
-        return self._scan_segment(T, num_seqs, H, D, Dv), 1
 
     def _scan_segment(self, T, num_seqs, H, D, Dv) -> int:
         """Tokens per segment of a decayed state scan, or 0 for the scan without segments: steps of many tokens per sequence

@@ -130,6 +130,18 @@ def test_both_maps_as_row_blocks(ops, heads, kv_heads, page, mask):
     _close(got, want, 12)
 
 
+@pytest.mark.parametrize("heads,kv_heads,mask", [(4, 2, dict(chunk=100)), (16, 2, dict(window=90)), (4, 4, dict())])
+def test_the_mma_sync_kernel_at_the_same_sizes(ops, heads, kv_heads, mask):
+    """It takes the steps whose longest sequence fills no block of 128 rows."""
+    from qwen3_runtime_b200.config import PartSpec
+
+    spec = PartSpec("differential_attention", dict(hidden_size=128, num_heads=heads, num_kv_heads=kv_heads, dim=64, vdim=128,
+                                                   scale=0.3, diff=0.4, eps=1e-5, **mask))
+    for portions in (RAGGED, [[2, 3, 0, 1, 7], [1, 2, 3, 0, 0]]):
+        got, want = _steps(ops, spec, 16, portions, [_set(differential_tcgen05=False), _set(differential_tc=False)])
+        _close(got, want, 12)
+
+
 @pytest.mark.parametrize("heads,q_rank,gate,pairing,page", [(2, 64, None, "interleaved", 16), (3, 0, "sigmoid", "half", 8),
                                                           (16, 96, None, "interleaved", 64)])
 @pytest.mark.parametrize("window", [None, 1, 64, 90, 300])

@@ -72,3 +72,27 @@ def test_a_latent_layer_keeps_its_value_rows_once():
     assert torch.equal(part.expand, torch.cat([tensors["uk"], tensors["uv"]]))
     assert torch.equal(part.uv.reshape(-1, 16), tensors["uv"]) and part.uv.is_contiguous()
     assert part.uv.untyped_storage().data_ptr() == part.expand.untyped_storage().data_ptr()
+
+
+@pytest.mark.parametrize("heads,kv_heads,new,kernel", [
+    (16, 4, [2], "mma"), (16, 4, [31], "mma"), (16, 4, [32], "tc"), (16, 4, [2, 500], "tc"), (16, 16, [127, 40], "mma"),
+    (16, 16, [128], "tc"), (16, 1, [2, 7], "mma"), (16, 1, [8], "tc")])
+def test_which_kernel_differential_prompts_take(heads, kv_heads, new, kernel):
+    """A step whose longest sequence fills no block of 128 rows stays on the mma.sync kernel; the two have names of their own."""
+    ops = _table()
+    ops.timing = None
+    ops._error_word = lambda device: None
+    launched = []
+    ops._call = lambda group, name, what, *args: launched.append((name, what))
+    step = _step([(0, n) for n in new])
+    step.num_seqs, step.max_kv_len = len(new), max(new)
+    step.kv_lens = step.cu_seqlens = torch.zeros(len(new) + 1, dtype=torch.int32)
+    T = sum(new)
+    pages = torch.zeros((4, kv_heads, 16, 128), dtype=torch.bfloat16)
+    ops.differential_attention(
+        torch.zeros((T, heads * 128), dtype=torch.bfloat16), heads * 128, num_heads=heads, num_kv_heads=kv_heads, map_dim=64,
+        value_dim=128, k_pages=pages, v_pages=pages, block_table=torch.zeros((len(new), 2), dtype=torch.int32),
+        token_seq=step.kv_lens, positions=step.kv_lens, out=torch.zeros((T, heads * 128), dtype=torch.bfloat16), page_size=16,
+        scale=1.0, lam=0.5, eps=1e-6, out_scale=1.0, chunk=2048, step=step)
+    assert launched == [{"tc": ("q3_diff_attention_prefill_tc", "differential_attention_tc"),
+                         "mma": ("q3_diff_attention_prefill", "differential_attention_mma")}[kernel]]
