@@ -238,12 +238,23 @@ __global__ void route_pick_kernel(float* __restrict__ logits, int num_tokens, in
         at = oa;
       }
     }
+    if (at >= E) {  // nothing but NaN is left: the lowest output not chosen yet, one of the first k + 1
+      int low = 0x7fffffff;
+      for (int e = lane; e <= k && low > e; e += 32) {
+        bool open = true;
+        for (int c = 0; c < k; ++c) open = open && chosen[(long)t * top + c] != e;
+        if (open) low = e;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) low = min(low, __shfl_xor_sync(0xffffffffu, low, o));
+      at = low;
+    }
     if (k == 0) first = best;  // the largest logit: the softmax's reference point
     const float score = mode == 2 ? expf(best - first) : 1.f / (1.f + expf(-best));
     if (lane == 0) {
       chosen[(long)t * top + k] = at;
       weights[(long)t * top + k] = score;
-      z[at] = -INFINITY;  // taken
+      z[at] = NAN;  // taken: compares false with everything
     }
     total += score;
     __syncwarp();
