@@ -132,12 +132,19 @@ int launch_tile(const float* A, int lda, const float* W, int ldw, float* C, int 
       return Q3_ERR_LAUNCH;
     configured = true;
   }
-  const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM), block((BM / TM) * (BN / TN));
-  if (grid.y > 65535) return Q3_ERR_UNSUPPORTED;
-  if (vec)
-    gemm_f32_kernel<BM, BN, BK, TM, TN, STAGES, true><<<grid, block, smem, stream>>>(A, lda, W, ldw, C, ldc, M, N, K);
-  else
-    gemm_f32_kernel<BM, BN, BK, TM, TN, STAGES, false><<<grid, block, smem, stream>>>(A, lda, W, ldw, C, ldc, M, N, K);
+  const dim3 block((BM / TM) * (BN / TN));
+  constexpr int MOST = 65535 * BM;  // rows of one launch: a grid has at most 65535 blocks along y
+  for (int m0 = 0;; m0 += MOST) {
+    const int rows = M - m0 < MOST ? M - m0 : MOST;
+    const dim3 grid((N + BN - 1) / BN, (rows + BM - 1) / BM);
+    const float* a = A + (long)m0 * lda;
+    float* c = C + (long)m0 * ldc;
+    if (vec)
+      gemm_f32_kernel<BM, BN, BK, TM, TN, STAGES, true><<<grid, block, smem, stream>>>(a, lda, W, ldw, c, ldc, rows, N, K);
+    else
+      gemm_f32_kernel<BM, BN, BK, TM, TN, STAGES, false><<<grid, block, smem, stream>>>(a, lda, W, ldw, c, ldc, rows, N, K);
+    if (rows == M - m0) break;
+  }
   return q3_launch_status();
 }
 

@@ -36,3 +36,16 @@ def test_tile_shapes_give_the_same_bits(ops, M, N, K, pad):
     assert float((out[0].double() - want).abs().max()) <= bound
     for other in out[1:]:
         assert torch.equal(out[0], other)
+
+
+@pytest.mark.parametrize("tile,rows", [(5, 65535 * 16), (3, 65535 * 32), (-1, 65535 * 64)])
+def test_more_rows_than_a_grid_has_blocks(ops, tile, rows):
+    x = (torch.arange((rows + 3) * 4, device="cuda") % 251).float().view(-1, 4)
+    w = torch.tensor([[1.0, 2.0, 3.0, 4.0], [5.0, 0.0, 0.0, 1.0]], device="cuda")
+    ops.f32_tile = tile
+    try:
+        out = ops.linear(x, w)
+    finally:
+        ops.f32_tile = -1
+    for n in range(2):  # sums of small whole numbers are exact
+        assert torch.equal(out[:, n], (x * w[n]).sum(1))
