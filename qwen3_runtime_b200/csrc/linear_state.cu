@@ -37,8 +37,9 @@
 // scales of a token's rows are worked out by a kernel of their own (16 us), not in both passes and every column tile.  A
 // thread holds 4 x 8 elements of the state, so that a token's three rows and its values are read once for 32 updates, as
 // pairs of columns for the packed instructions (the issue slots bound the passes), and the sums over the row groups are
-// folded: a lane gives half of its columns away at each step.  16 heads of 64 x 128, 2048 tokens, the whole mixer: 565 us
-// with the scan above, 231 with 4 x 4 elements and rows worked out in the passes, 200 so.
+// folded: a lane gives half of its columns away at each step.  A block finds its sequence with one warp, 32 sequences at a
+// time (one thread walking 128 sequences cost every block of every pass 20 us).  When this is the faster one, and with
+// which `seg`, is worked out from the sequences' lengths (ops/cuda.py, decayed_scan_segment).
 //
 // head_norm_gate: y[t, h, :] = o / sqrt(mean(o^2) + eps) * w * silu(g[t, h, :]) * out_scale, one warp
 // per (token, head); w may be absent.
@@ -287,9 +288,13 @@ struct ScanArgs {
   float* rows;      // [T, H, 3, DP], DP = 64 or 128
 };
 
+__device__ __forceinline__ int segments_of(const ScanArgs& a, int b) {
+  return (a.cu_seqlens[b + 1] - a.cu_seqlens[b] + a.seg - 1) / a.seg;
+}
+
 // A token's rows of a head as the scans read them, fp32 [T, H, 3, DP]: keys (turned, scaled), decays, queries (turned,
 // scaled); zero (and one) beyond D.  Worked out once: both scans and every column tile read the same rows.
-template <typename T, int DP>
+template <int DP>
 __global__ void __launch_bounds__(256)
 segment_rows_kernel(const __grid_constant__ ScanArgs a, long total) {
   pdl_wait();
@@ -299,7 +304,7 @@ segment_rows_kernel(const __grid_constant__ ScanArgs a, long total) {
   const int i = x % DP;
   const long th = x / DP, t = th / a.H;
   const int h = (int)(th - t * a.H);
-  const T *q = (const T*)a.q + t * a.q_stride + h * a.D, *k = (const T*)a.k + t * a.k_stride + h * a.D;
+  const bf16 *q = (const bf16*)a.q + t * a.q_stride + h * a.D, *k = (const bf16*)a.k + t * a.k_stride + h * a.D;
   float qv = 0.f, kv = 0.f, av = 1.f;
   if (i < a.D) {
     qv = to_f32(q[i]);
@@ -317,7 +322,7 @@ segment_rows_kernel(const __grid_constant__ ScanArgs a, long total) {
     kv *= a.k_scale;
     if (a.tok_kscale) kv *= a.tok_kscale[t * a.H + h];
     if (a.z) {
-      const float zz = to_f32(((const T*)a.z)[t * a.z_stride + h * a.D + i]) + (a.z_bias ? a.z_bias[h * a.D + i] : 0.f);
+      const float zz = to_f32(((const bf16*)a.z)[t * a.z_stride + h * a.D + i]) + (a.z_bias ? a.z_bias[h * a.D + i] : 0.f);
       av = a.decay_mode == 1 ? expf(-expf(zz)) : expf((fminf(zz, 0.f) - log1pf(expf(-fabsf(zz)))) * a.inv_tau);
     } else {
       av = a.tok_decay ? a.tok_decay[t * a.H + h] : a.head_decay[h];
@@ -331,7 +336,7 @@ segment_rows_kernel(const __grid_constant__ ScanArgs a, long total) {
 
 // DP: key rows (64 or 128), in DP / 4 row groups; CG column groups of 8: a thread holds 4 x 8 elements of the state.
 // Block: (segment, column tile, head).
-template <typename T, int DP, int CG, bool OUT, bool BONUS>
+template <int DP, int CG, bool OUT, bool BONUS>
 __global__ void __launch_bounds__(DP / 4 * CG, 2)
 segment_scan_kernel(const __grid_constant__ ScanArgs a) {
   constexpr int RG = DP / 4, THREADS = RG * CG, VT = 8 * CG, CT = SCAN_CT;
@@ -346,21 +351,31 @@ segment_scan_kernel(const __grid_constant__ ScanArgs a) {
   const int H = a.H, D = a.D, Dv = a.Dv, h = blockIdx.z, j0 = blockIdx.y * VT;
   pdl_wait();
   pdl_launch_dependents();
-  if (tid == 0) {
+  if (tid < 32) {  // the sequence that this segment belongs to, 32 sequences at a time
     int at = 0, seq = -1, first = 0, count = 0;
-    for (int b = 0; b < a.num_seqs; ++b) {
-      const int n = (a.cu_seqlens[b + 1] - a.cu_seqlens[b] + a.seg - 1) / a.seg;
-      if ((int)blockIdx.x < at + n) {
-        seq = b;
-        first = at;
-        count = n;
+    for (int b0 = 0; b0 < a.num_seqs; b0 += 32) {
+      const int n = b0 + tid < a.num_seqs ? segments_of(a, b0 + tid) : 0;
+      int sum = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, sum, o);
+        if (tid >= o) sum += x;
+      }
+      const uint32_t beyond = __ballot_sync(0xffffffffu, at + sum > (int)blockIdx.x);
+      if (beyond) {
+        const int l = __ffs(beyond) - 1;
+        seq = b0 + l;
+        count = __shfl_sync(0xffffffffu, n, l);
+        first = at + __shfl_sync(0xffffffffu, sum, l) - count;
         break;
       }
-      at += n;
+      at += __shfl_sync(0xffffffffu, sum, 31);
     }
-    s_seq = seq;
-    s_first = first;
-    s_count = count;
+    if (tid == 0) {
+      s_seq = seq;
+      s_first = first;
+      s_count = count;
+    }
   }
   __syncthreads();
   const int seq = s_seq;
@@ -390,8 +405,8 @@ segment_scan_kernel(const __grid_constant__ ScanArgs a) {
     P[r] = 1.f;
   }
   const int Dvin = Dv - a.ones_col;
-  const T* v = (const T*)a.v;
-  T vr[VPT];
+  const bf16* v = (const bf16*)a.v;
+  bf16 vr[VPT];
   // a chunk's rows into buffer `to` (its values into registers): in flight while the chunk before is worked on
   auto fetch = [&](int t_at, int to) {
     const int n = min(CT, t1 - t_at);
@@ -405,7 +420,7 @@ segment_scan_kernel(const __grid_constant__ ScanArgs a) {
     for (int m = 0; m < VPT; ++m) {
       const int x = tid + m * THREADS, c = x / VT, j = j0 + x % VT;
       const long t = t_at + c;
-      vr[m] = t < t1 && j < Dvin ? v[t * a.v_stride + h * Dvin + j] : from_f32<T>(t < t1 && j < Dv ? 1.f : 0.f);
+      vr[m] = t < t1 && j < Dvin ? v[t * a.v_stride + h * Dvin + j] : from_f32<bf16>(t < t1 && j < Dv ? 1.f : 0.f);
     }
   };
   auto stage = [&](int to) {
@@ -502,10 +517,16 @@ segment_join_kernel(const __grid_constant__ ScanArgs a) {
   pdl_launch_dependents();
   const int h = blockIdx.y, seq = blockIdx.z, D = a.D, Dv = a.Dv;
   const int x = blockIdx.x * 256 + threadIdx.x;
-  int first = 0;
-  for (int b = 0; b < seq; ++b) first += (a.cu_seqlens[b + 1] - a.cu_seqlens[b] + a.seg - 1) / a.seg;
-  const int count = (a.cu_seqlens[seq + 1] - a.cu_seqlens[seq] + a.seg - 1) / a.seg;
-  if (count < 2 || x >= D * Dv) return;
+  const int count = segments_of(a, seq);
+  if (count < 2) return;
+  int first = 0;  // segments of the sequences before: a warp counts 32 of them at a time
+  for (int b0 = 0; b0 < seq; b0 += 32) {
+    int n = b0 + (int)(threadIdx.x & 31) < seq ? segments_of(a, b0 + (int)(threadIdx.x & 31)) : 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+    first += n;
+  }
+  if (x >= D * Dv) return;
   const int i = x / Dv;
   float S = a.state[((long)a.state_slots[seq] * a.H + h) * D * Dv + x];
   constexpr int AHEAD = 6;  // segments whose numbers are read together: the chain is one multiply-add a segment
@@ -526,45 +547,50 @@ segment_join_kernel(const __grid_constant__ ScanArgs a) {
   }
 }
 
-template <typename T, int DP, int CG, bool BONUS>
-static cudaError_t launch_segments(const ScanArgs& a, int num_tokens, int segments, cudaStream_t stream) {
+template <int DP, int CG, bool BONUS>
+static cudaError_t launch_segments(const ScanArgs& a, int num_tokens, int segments, bool cut, cudaStream_t stream) {
   constexpr size_t smem = (size_t)(6 * SCAN_CT * DP + 3 * SCAN_CT * 8 * CG) * sizeof(float);
   static bool configured_on[Q3_MAX_DEVICES];
   bool& configured = configured_on[q3_current_device()];
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(segment_scan_kernel<T, DP, CG, false, BONUS>,
+    cudaError_t e = cudaFuncSetAttribute(segment_scan_kernel<DP, CG, false, BONUS>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(segment_scan_kernel<T, DP, CG, true, BONUS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      e = cudaFuncSetAttribute(segment_scan_kernel<DP, CG, true, BONUS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)smem);
     if (e != cudaSuccess) return e;
     configured = true;
   }
   const dim3 grid((unsigned)segments, (unsigned)((a.Dv + 8 * CG - 1) / (8 * CG)), (unsigned)a.H), block(DP / 4 * CG);
   const long elements = (long)num_tokens * a.H * DP;
-  cudaError_t e = launch_pdl(segment_rows_kernel<T, DP>, dim3((unsigned)((elements + 255) / 256)), dim3(256), 0, stream, a,
+  cudaError_t e = launch_pdl(segment_rows_kernel<DP>, dim3((unsigned)((elements + 255) / 256)), dim3(256), 0, stream, a,
                              elements);
-  if (e == cudaSuccess && segments > a.num_seqs) {  // else every sequence is one segment
-    e = launch_pdl(segment_scan_kernel<T, DP, CG, false, BONUS>, grid, block, smem, stream, a);
+  if (e == cudaSuccess && cut) {
+    e = launch_pdl(segment_scan_kernel<DP, CG, false, BONUS>, grid, block, smem, stream, a);
     if (e == cudaSuccess)
       e = launch_pdl(segment_join_kernel, dim3((unsigned)((a.D * a.Dv + 255) / 256), (unsigned)a.H, (unsigned)a.num_seqs),
                      dim3(256), 0, stream, a);
   }
-  if (e == cudaSuccess) e = launch_pdl(segment_scan_kernel<T, DP, CG, true, BONUS>, grid, block, smem, stream, a);
-  return e;
+  if (e != cudaSuccess) return e;
+  if (cut) return launch_pdl(segment_scan_kernel<DP, CG, true, BONUS>, grid, block, smem, stream, a);
+  // Not as a dependent launch right behind the rows: its few blocks would start between those of the rows kernel, two on
+  // some SMs while others have none (one prompt of 64 tokens, 16 heads: 45 us instead of 30).
+  segment_scan_kernel<DP, CG, true, BONUS><<<grid, block, smem, stream>>>(a);
+  return cudaGetLastError();
 }
 
-// The same arguments as q3_decayed_state_scan, bfloat16, key sizes up to 128: in segments of `seg` tokens.  segments: the number of
-// them, sum over the sequences of ceil(tokens / seg), or more; scratch: fp32, 16-byte aligned, [num_tokens * H * 3 * DP +
-// segments * H * D * (Dv + 1)] with DP = 64 (D <= 64) or 128.
+// The same arguments as q3_decayed_state_scan, bfloat16, key sizes up to 128: in segments of `seg` tokens.  segments: the
+// number of them, sum over the sequences of ceil(tokens / seg), or more; cut: whether a sequence may have more than one;
+// scratch: fp32, 16-byte aligned, num_tokens * H * 3 * DP with DP = 64 (D <= 64) or 128, and if cut segments * H * D *
+// (Dv + 1) more.
 Q3_EXPORT int q3_decayed_segment_scan(int dtype, const void* q, long q_stride, const void* k, long k_stride, const void* v,
                                       long v_stride, const void* z, long z_stride, const float* z_bias, float inv_tau,
                                       const float* head_decay, const float* inv_freq, int rot_pairs, const int* positions,
                                       float q_scale, float k_scale, float* state, const int* cu_seqlens,
                                       const int* state_slots, float* out, int num_seqs, int H, int D, int Dv,
                                       int decay_mode, const float* tok_decay, const float* tok_kscale, int ones_col,
-                                      const float* bonus, int seg, int segments, float* scratch, int num_tokens,
-                                      cudaStream_t stream) {
+                                      const float* bonus, int seg, int segments, int cut, float* scratch,
+                                      int num_tokens, cudaStream_t stream) {
   if (!q || !k || !v || !state || !cu_seqlens || !state_slots || !out || !scratch || seg < 1 || segments < 1 ||
       num_tokens < 0 || ((uintptr_t)scratch & 15))
     return Q3_ERR_ARGUMENT;
@@ -581,11 +607,11 @@ Q3_EXPORT int q3_decayed_segment_scan(int dtype, const void* q, long q_stride, c
                       scratch};
   cudaError_t e;
   if (D <= 64)
-    e = bonus ? launch_segments<bf16, 64, 16, true>(a, num_tokens, segments, stream)
-              : launch_segments<bf16, 64, 16, false>(a, num_tokens, segments, stream);
+    e = bonus ? launch_segments<64, 16, true>(a, num_tokens, segments, cut, stream)
+              : launch_segments<64, 16, false>(a, num_tokens, segments, cut, stream);
   else
-    e = bonus ? launch_segments<bf16, 128, 8, true>(a, num_tokens, segments, stream)
-              : launch_segments<bf16, 128, 8, false>(a, num_tokens, segments, stream);
+    e = bonus ? launch_segments<128, 8, true>(a, num_tokens, segments, cut, stream)
+              : launch_segments<128, 8, false>(a, num_tokens, segments, cut, stream);
   return e == cudaSuccess ? Q3_OK : Q3_ERR_LAUNCH;
 }
 

@@ -10,6 +10,7 @@ kernel does not support; they never substitute another code path silently.
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 from ctypes import c_float, c_int, c_long, c_void_p
 
@@ -172,8 +173,8 @@ _SIGNATURES = {
         "q3_decayed_segment_scan": [c_int, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long,
                                   c_void_p, c_float, c_void_p, c_void_p, c_int, c_void_p, c_float, c_float, c_void_p,
                                   c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                                  c_int, c_void_p, c_int, c_int, c_void_p, c_int,
-                                    c_void_p],
+                                  c_int, c_void_p, c_int, c_int, c_int, c_void_p,
+                                    c_int, c_void_p],
         "q3_head_norm_gate": [c_int, c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p, c_long, c_void_p, c_long,
                               c_float, c_int, c_int, c_int, c_int, c_void_p],
         "q3_stabilised_gates": [c_int, c_void_p, c_void_p, c_long, c_void_p, c_void_p, c_float, c_void_p, c_void_p,
@@ -280,6 +281,78 @@ class _Span:
         self.ops._cost = (0, 0, "")
         self.ops.timing.append((self.what + tag, self.start, self.stop, nbytes, flops))
         return False
+
+
+# ---- decayed state scans of bfloat16 steps: token by token or in segments -------------------------
+SCAN_SCRATCH = 1 << 28  # floats a segment scan may ask for (1 GiB)
+
+# Times in us of the two scans (csrc/linear_state.cu) on a B200, by the padded key size: least squares over 52 compositions
+# of sequences (one token to 8,000, alone, in equal numbers and mixed, up to 128 of them) x 6 head counts and sizes x up to 10
+# segment lengths; 6 % off on average.  A pass of the segments takes the longer of one block's chain (`alone` per token)
+# and all blocks at two per SM (`shared` per token, `block` per block); rows and joining cost `row` and `join` more, and
+# without a cut the first pass's launch is saved (`whole`).  The scan token by token takes the longer of the longest sequence
+# (`chain_token`) and all of its blocks of 16 columns (`load` per token, `start` per block).
+SCAN_COSTS = {
+    64: dict(row=20.7e-6, out=(0.40, 0.244, 24.1), ends=(0.20, 0.155, 1.6), join=11.3, whole=10.0, chain=8.2,
+             chain_token=0.215, load=0.110, start=0.9),
+    128: dict(row=10.1e-6, out=(0.42, 0.43, 29.2), ends=(0.20, 0.135, 1.4), join=12.5, whole=10.0, chain=8.1,
+              chain_token=0.30, load=0.249, start=3.8),
+}
+
+
+def _scan_blocks(H, D, Dv):
+    """Blocks of one segment: (head, tile of value columns)."""
+    return H * -(-Dv // (128 if D <= 64 else 64))
+
+
+def _scan_scratch(T, H, D, Dv, segments, cut):
+    """Floats of a segment scan: a token's rows, and where sequences are cut the segments' states and decays."""
+    return T * H * 3 * (64 if D <= 64 else 128) + (segments * H * D * (Dv + 1) if cut else 0)
+
+
+def _segments(cu, seg):
+    """(number of segments, longest sequence)"""
+    lens = [b - a for a, b in zip(cu, cu[1:])]
+    return sum(-(-n // seg) for n in lens), max(lens)
+
+
+@functools.lru_cache(maxsize=256)
+def decayed_scan_segment(cu, H, D, Dv, sms) -> int:
+    """Tokens per segment of a bfloat16 step's decayed state scan, or 0 for the scan token by token, whichever the measured
+    costs make the fastest (segments where they win by 10 % at least).  A segment's length follows from the whole step: one
+    prompt is cut so that its blocks fill the SMs once at two each, many short prompts fill them as they are.  Layers of 16
+    heads of 64 x 128, us token by token / so: 64 tokens 22 / 22; 512 118 / 65; 2040 443 / 133; 2040 beside 31 single tokens 775 / 207,
+    beside 127 817 / 325; 8 prompts of 256 244 / 150; 32 of 64 234 / 112.  A step of one short prompt and single tokens is never
+    cut where its blocks leave most SMs idle (16 heads of 128 x 128, 128 tokens beside 8: 75 / 83)."""
+    lens = [b - a for a, b in zip(cu, cu[1:])]
+    T, longest = sum(lens), max(lens)
+    c = SCAN_COSTS[64 if D <= 64 else 128]
+    blocks = _scan_blocks(H, D, Dv)
+    if longest < 16 or (longest < 192 and T < 3 * longest and blocks <= 32):
+        return 0
+
+    def one_pass(tokens, count, last, alone, shared, block):
+        return max(alone * last + block, (shared * tokens + block * count) * blocks / (2 * sms) + 0.5 * alone * last)
+
+    chain = c["chain_token"] * longest
+    columns = H * -(-Dv // 16) / sms
+    best = 0.9 * (c["chain"] + max(chain, (c["load"] * T + c["start"] * len(lens)) * columns + 0.5 * chain))
+    found = 0
+    one_wave = min(512, max(32, -(-T // max(1, 2 * sms // blocks))))
+    for seg in sorted({32, 48, 64, 96, 128, 192, 256, 384, 512, one_wave, longest}):
+        if seg > longest:
+            break
+        count = sum(-(-n // seg) for n in lens)
+        more = sum(-(-n // seg) - 1 for n in lens if n)
+        if _scan_scratch(T, H, D, Dv, count, more > 0) > SCAN_SCRATCH:
+            continue
+        cost = c["row"] * T * H * (64 if D <= 64 else 128) + one_pass(T, count, min(seg, longest), *c["out"])
+        cost += c["join"] + one_pass(more * seg, more, seg, *c["ends"]) if more else -c["whole"]
+        if seg == one_wave:  # its blocks end together: what the model does not see
+            cost *= 0.92
+        if cost < best:
+            best, found = cost, seg
+    return found
 
 
 class CudaOps:
@@ -679,10 +752,12 @@ class CudaOps:
         return out
 
     # ---- decayed matrix state (csrc/linear_state.cu) and short convolution (csrc/short_conv.cu) ----
+    scan_takes_lengths = True  # decayed_state_scan chooses by the step's lengths where it is given them
+
     def decayed_state_scan(self, q, k, v, *, state, cu_seqlens, state_slots, num_seqs, decay_logits=None,
                            decay_bias=None, tau=1.0, head_decay=None, inv_freq=None, positions=None, q_scale=1.0,
                            k_scale=1.0, decay_mode="sigmoid_pow", token_decay=None, token_k_scale=None, bonus=None,
-                           ones_column=False):
+                           ones_column=False, host_cu_seqlens=None):
         """``S_t = diag(a_t) S_(t-1) + k_t v_t^T``, ``o_t = S_t^T q_t`` per (sequence, head) on the float32
         state ``[slots, H, D, Dv]`` of the sequences' slots; returns float32 ``o`` ``[T, H, Dv]``.
         ``q, k`` ``[T, H, D]``, ``v`` ``[T, H, Dv]`` (views of wider rows allowed).  The decay is
@@ -694,7 +769,8 @@ class CudaOps:
         factor on k.  ``ones_column``: the values get one more column whose value is 1 (state and ``o`` then
         have ``Dv + 1`` columns; the last one of ``o`` is q times the decayed sum of the keys).  ``bonus``
         (float32 ``[H * D]``): ``o_t = (S_(t-1) + diag(bonus) k_t v_t^T)^T q_t``, the state read before its
-        update."""
+        update.  ``host_cu_seqlens``: the numbers of ``cu_seqlens`` on the host, by which bfloat16 steps are run token by
+        token or in segments of a chosen length (:func:`decayed_scan_segment`)."""
         T, H, D = q.shape
         Dv = v.shape[2] + int(bool(ones_column))
         modes = {"sigmoid_pow": 0, "exp_neg_exp": 1}
@@ -725,25 +801,34 @@ class CudaOps:
                 _ptr(out), int(num_seqs), H, D, Dv, modes[decay_mode], _ptr(token_decay), _ptr(token_k_scale),
                 int(bool(ones_column)), _ptr(bonus))
         # (float32 stays token by token: the same bits however a prompt is cut)
-        seg = self._scan_segment(T, int(num_seqs), H, D, Dv) if q.dtype == torch.bfloat16 else 0
+        cu = tuple(host_cu_seqlens) if host_cu_seqlens else None
+        seg = self._scan_segment(T, int(num_seqs), H, D, Dv, cu) if q.dtype == torch.bfloat16 else 0
         if seg:
-            segments = T // seg + int(num_seqs)  # at least the sum of ceil(tokens / seg)
-            scratch = torch.empty(T * H * 3 * (64 if D <= 64 else 128) + segments * H * D * (Dv + 1), dtype=torch.float32,
-                                  device=q.device)
-            self.launches += 1 + 2 * int(segments > num_seqs)
-            self._call("linear_state", "q3_decayed_segment_scan", "decayed_state_scan", *args, seg, segments, _ptr(scratch), T)
-            return out
-        self._call("linear_state", "q3_decayed_state_scan", "decayed_state_scan", *args)
+            segments, longest = _segments(cu, seg) if cu else (T // seg + int(num_seqs), T)
+            try:
+                scratch = torch.empty(_scan_scratch(T, H, D, Dv, segments, longest > seg), dtype=torch.float32, device=q.device)
+            except torch.OutOfMemoryError:
+                seg = 0  # token by token needs none
+        if seg:
+            self.launches += 1 + 2 * int(longest > seg)
+            self._call("linear_state", "q3_decayed_segment_scan", "decayed_state_scan", *args, seg, segments, int(longest > seg),
+                       _ptr(scratch), T)
+        else:
+            self._call("linear_state", "q3_decayed_state_scan", "decayed_state_scan", *args)
         return out
 
-    def _scan_segment(self, T, num_seqs, H, D, Dv) -> int:
-        """Tokens per segment of a decayed state scan, or 0 for the scan without segments: steps of many tokens per sequence
-        with keys of up to 128, whose rows (fp32, three per token and head) stay under 1 GiB.  At least 32, for two blocks
-        per SM (fewer and longer ones leave SMs with one)."""
-        if not self.scan_segments or D > 128 or T < max(64, 8 * num_seqs) or T * H * (64 if D <= 64 else 128) * 12 > 1 << 30:
+    def _scan_segment(self, T, num_seqs, H, D, Dv, cu=None) -> int:
+        """Tokens per segment of a bfloat16 decayed state scan, or 0 for the scan token by token.  Without the host's
+        ``cu_seqlens`` the step may hold anything: steps of many tokens per sequence are then cut as one long sequence,
+        for two blocks per SM (a sequence shorter than a segment is one block and no worse off)."""
+        if not self.scan_segments or D > 128:
             return 0
-        blocks = H * -(-Dv // (128 if D <= 64 else 64))
-        return max(32, -(-T // max(1, 2 * self.SM_COUNT // blocks - (num_seqs - 1))))
+        if cu:
+            return decayed_scan_segment(cu, H, D, Dv, self.SM_COUNT)
+        seg = max(32, -(-T // max(1, 2 * self.SM_COUNT // _scan_blocks(H, D, Dv))))
+        if T < max(64, 8 * num_seqs) or _scan_scratch(T, H, D, Dv, T // seg + num_seqs, True) > SCAN_SCRATCH:
+            return 0
+        return seg
 
     def stabilised_gates(self, zi, zf, *, i_bias, f_bias, cap, m_state, cu_seqlens, state_slots, num_seqs):
         """The gates of a matrix memory with exponential gates and a running maximum m per (sequence, head)

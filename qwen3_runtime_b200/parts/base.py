@@ -211,3 +211,8 @@ class ResidualStream:
         stream.resid = resid
         stream.source_pair = source_pair
         return stream
+
+
+def scan_lengths(ops, step: StepContext) -> dict:
+    """The step's lengths as an argument of ``ops.decayed_state_scan``, for a kernel table that chooses its scan by them."""
+    return dict(host_cu_seqlens=step.host_cu_seqlens) if getattr(ops, "scan_takes_lengths", False) else {}

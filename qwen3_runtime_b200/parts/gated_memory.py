@@ -27,7 +27,7 @@ from __future__ import annotations
 import torch
 
 from ..cache.layout import StateLayerSpec
-from .base import BuildContext, ParamSpec, Part, StepContext, register_part
+from .base import BuildContext, ParamSpec, Part, StepContext, register_part, scan_lengths
 from .linear_state import _pad_rows, heads_view
 
 
@@ -85,7 +85,7 @@ class MatrixLstm(Part):
             m_state=maximum.state, cu_seqlens=step.cu_seqlens, state_slots=step.state_slots, num_seqs=step.num_seqs)
         o = ops.decayed_state_scan(q, k, v, state=memory.state, cu_seqlens=step.cu_seqlens,
                                    state_slots=step.state_slots, num_seqs=step.num_seqs, token_decay=decay,
-                                   token_k_scale=k_scale, ones_column=True, q_scale=D ** -0.5)
+                                   token_k_scale=k_scale, ones_column=True, q_scale=D ** -0.5, **scan_lengths(ops, step))
         ctx = torch.empty((h.shape[0], H * Dv), dtype=h.dtype, device=h.device)
         ops.head_norm_gate(o, g, ctx.unflatten(1, (H, Dv)), weight=self.norm_weight, eps=self.eps, gate_act="sigmoid",
                            per_head_weight=True, denominator=m_run)
@@ -147,7 +147,7 @@ class ShiftedWkv(Part):
         z = ops.linear(ops.tanh_rows(ops.linear(x[4], w["w1"])), w["w2"]).unflatten(1, (H, D))
         o = ops.decayed_state_scan(r, k, v, state=memory.state, cu_seqlens=step.cu_seqlens,
                                    state_slots=step.state_slots, num_seqs=step.num_seqs, decay_logits=z,
-                                   decay_bias=self.w0, decay_mode="exp_neg_exp", bonus=self.bonus)
+                                   decay_bias=self.w0, decay_mode="exp_neg_exp", bonus=self.bonus, **scan_lengths(ops, step))
         ctx = torch.empty((h.shape[0], H * D), dtype=h.dtype, device=h.device)
         ops.head_norm_gate(o, g, ctx.unflatten(1, (H, D)), weight=self.norm_weight, eps=self.eps, gate_act="silu",
                            per_head_weight=True)

@@ -24,7 +24,7 @@ import torch
 
 from ..cache.layout import StateLayerSpec
 from ..config.spec import PartSpec
-from .base import Addend, BuildContext, ParamSpec, Part, StepContext, build_part, register_part
+from .base import Addend, BuildContext, ParamSpec, Part, StepContext, build_part, register_part, scan_lengths
 
 
 def heads_view(rows: torch.Tensor, start: int, heads: int, size: int) -> torch.Tensor:
@@ -162,7 +162,7 @@ class GatedLinearAttention(_DecayedStateMixer):
         z = ops.linear(low, self.a2).unflatten(1, (H, D))
         o = ops.decayed_state_scan(q, k, v, state=cache.state, cu_seqlens=step.cu_seqlens, state_slots=step.state_slots,
                                    num_seqs=step.num_seqs, decay_logits=z, decay_bias=self.a2_bias, tau=self.tau,
-                                   q_scale=D ** -0.5)
+                                   q_scale=D ** -0.5, **scan_lengths(ops, step))
         ops.head_norm_gate(o, g, out.unflatten(1, (H, Dv)), weight=self.norm_weight, eps=self.eps, out_scale=out_scale)
 
 
@@ -192,7 +192,7 @@ class Retention(_DecayedStateMixer):
         inv = self.position.device_inverse_frequencies() if self.position.style == "rotary" else None
         o = ops.decayed_state_scan(q, k, v, state=cache.state, cu_seqlens=step.cu_seqlens, state_slots=step.state_slots,
                                    num_seqs=step.num_seqs, head_decay=self.decay_dev, inv_freq=inv,
-                                   positions=step.positions, k_scale=D ** -0.5)
+                                   positions=step.positions, k_scale=D ** -0.5, **scan_lengths(ops, step))
         ops.head_norm_gate(o, g, out.unflatten(1, (H, Dv)), weight=None, eps=self.eps, out_scale=out_scale)
 
 

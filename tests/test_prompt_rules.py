@@ -96,3 +96,38 @@ def test_which_kernel_differential_prompts_take(heads, kv_heads, new, kernel):
         scale=1.0, lam=0.5, eps=1e-6, out_scale=1.0, chunk=2048, step=step)
     assert launched == [{"tc": ("q3_diff_attention_prefill_tc", "differential_attention_tc"),
                          "mma": ("q3_diff_attention_prefill", "differential_attention_mma")}[kernel]]
+
+
+def _cu(lens):
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    return tuple(cu)
+
+
+def test_state_scans_are_cut_by_the_lengths_of_their_sequences():
+    from qwen3_runtime_b200.ops.cuda import decayed_scan_segment
+
+    def seg(lens, heads=16, dim=64, vdim=128):
+        return decayed_scan_segment(_cu(lens), heads, dim, vdim, 148)
+
+    # single tokens beside a long prompt do not lengthen its segments
+    for heads, most in ((16, 128), (32, 256), (64, 512)):
+        for singles in (0, 1, 7, 15, 17, 19, 31, 63, 127):
+            assert 32 <= seg([1] * (singles // 2) + [2040] + [1] * (singles - singles // 2), heads) <= most
+    # one short prompt, or one beside a few tokens: a chain of few tokens is over before segments are joined
+    assert seg([64]) == seg([128]) == seg([1, 64, 1, 1, 1]) == seg([128] + [1] * 8) == seg([1] * 4096) == seg([15] * 64) == 0
+    # many short prompts fill the SMs as they are: a segment each
+    assert seg([64] * 32) == 64 and seg([128] * 16) == 128 and seg([32] * 64) == 32
+    # one prompt's blocks fill the SMs once
+    assert seg([2048]) == 114 and seg([2040], 32) == 227 and seg([2040], 16, 128) == 227
+    assert seg([0, 0]) == 0 and seg([0, 700, 0]) == seg([700]) > 0
+    # scratch (rows, and the segments' states where sequences are cut) stays within 1 GiB
+    assert seg([8000] * 4, 64, 128, 128) == 0 and seg([4000], 64, 128, 128) > 0
+
+
+def test_a_scan_with_unknown_lengths_is_cut_as_one_sequence():
+    ops = _table()
+    assert ops._scan_segment(2048, 1, 16, 64, 128) == ops._scan_segment(2048, 32, 16, 64, 128) == 114
+    assert ops._scan_segment(2048, 300, 16, 64, 128) == ops._scan_segment(63, 1, 16, 64, 128) == 0
+    assert ops._scan_segment(2048, 1, 16, 136, 128) == 0

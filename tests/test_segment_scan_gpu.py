@@ -101,3 +101,68 @@ def test_segments_against_float64_and_the_chain(ops, dtype, D, Dv, form):
             have = state[segments].cpu().double()[slots.long()]
             assert float((have - final).abs().max()) <= 3e-5 * max(1.0, float(final.abs().max()))
             assert torch.equal(state[segments][3].cpu(), start[3]), "a slot of another request was touched"
+
+
+MIXED = [[1] * 20 + [300] + [1] * 20 + [0, 45, 33], [1] * 40 + [129, 0, 200, 64], [64] * 44, [16] * 44]
+
+
+@pytest.mark.parametrize("D,Dv", [(64, 128), (128, 72)])
+@pytest.mark.parametrize("seg", [None, 32, 48, 300])
+def test_steps_of_many_sequences(ops, D, Dv, seg):
+    """One-token sequences, empty ones and prompts in one step, more sequences than a warp looks at together; with the
+    segment length that the lengths give and with others."""
+    g = torch.Generator().manual_seed(D)
+    H, B = 5, len(MIXED[0])
+    slots = torch.randperm(B + 3, generator=g)[:B].int()
+    start = torch.randn((B + 3, H, D, Dv), generator=g)
+    state, chain = start.clone().cuda(), start.clone().cuda()
+    for lens in MIXED:
+        T = sum(lens)
+        cu = torch.tensor([0] + lens).cumsum(0)
+        q, k, z = (torch.randn((T, H, D), generator=g).bfloat16().cuda() for _ in range(3))
+        v = torch.randn((T, H, Dv), generator=g).bfloat16().cuda()
+        kw = dict(cu_seqlens=cu.int().cuda(), state_slots=slots.cuda(), num_seqs=B, q_scale=0.5, decay_logits=z,
+                  decay_bias=torch.zeros(H * D).cuda(), tau=3.0, host_cu_seqlens=cu.tolist())
+        ops.scan_segments = False
+        want = ops.decayed_state_scan(q, k, v, state=chain, **kw)
+        ops.scan_segments = True
+        if seg:
+            ops._scan_segment = lambda *args: seg
+        try:
+            got = ops.decayed_state_scan(q, k, v, state=state, **kw)
+        finally:
+            ops.__dict__.pop("_scan_segment", None)
+        # float32 sums of a few hundred addends in another order
+        assert float((got - want).abs().max()) <= 3e-5 * max(1.0, float(want.abs().max()))
+        assert float((state - chain).abs().max()) <= 3e-5 * max(1.0, float(chain.abs().max()))
+    untouched = [s for s in range(B + 3) if s not in slots.tolist()]
+    assert torch.equal(state[untouched].cpu(), start[untouched])
+
+
+def test_a_scan_without_room_for_its_scratch_runs_token_by_token(ops):
+    H, D, Dv, T = 16, 64, 128, 4096
+    q, k, z = (torch.randn((T, H, D), device="cuda").bfloat16() for _ in range(3))
+    v = torch.randn((T, H, Dv), device="cuda").bfloat16()
+    kw = dict(cu_seqlens=torch.tensor([0, T], dtype=torch.int32, device="cuda"), num_seqs=1, decay_logits=z, tau=3.0,
+              state_slots=torch.zeros(1, dtype=torch.int32, device="cuda"), host_cu_seqlens=[0, T])
+    state = torch.zeros((1, H, D, Dv), device="cuda")
+    launched = []
+    call = ops._call
+
+    def spy(group, name, what, *args):
+        launched.append(name)
+        return call(group, name, what, *args)
+
+    ops._call = spy
+    total = torch.cuda.get_device_properties(0).total_memory
+    try:
+        with_room = ops.decayed_state_scan(q, k, v, state=state.clone(), **kw)
+        del with_room
+        torch.cuda.empty_cache()
+        # the output (33 MB) fits, the segments' scratch (70 MB) does not
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (70 << 20)) / total)
+        ops.decayed_state_scan(q, k, v, state=state.clone(), **kw)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+        del ops._call
+    assert launched == ["q3_decayed_segment_scan", "q3_decayed_state_scan"]
