@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(RG * VT)
 delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const T* __restrict__ vc,
                   const float* __restrict__ g, const float* __restrict__ beta, float* __restrict__ state,
                   const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots, float* __restrict__ out, int G,
-                  int H, int D, int Dv) {
+                  int H, int D, int Dv, int longest) {
   constexpr int THREADS = RG * VT, DP = RG * R, CPW = 32 / RG;
   constexpr int EPT = DS_CT * DP / THREADS;
   constexpr int VPT = (DS_CT * VT + THREADS - 1) / THREADS;
@@ -248,7 +248,7 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
   const int h = blockIdx.y, seq = blockIdx.z, gh = h / (H / G);
   const int j = blockIdx.x * VT + col;
   const int t0 = cu_seqlens[seq], t1 = cu_seqlens[seq + 1];
-  if (t1 <= t0) return;
+  if (t1 <= t0 || t1 - t0 > longest) return;
   float* Sg = state + ((long)state_slots[seq] * H + h) * (long)D * Dv;
   float S[R];
 #pragma unroll
@@ -340,18 +340,19 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
 template <typename T, int RG, int R, int VT>
 static cudaError_t launch_delta_scan(cudaStream_t stream, int num_seqs, const float* qn, const float* kn, const void* vc,
                                      const float* g, const float* beta, float* state, const int* cu_seqlens,
-                                     const int* state_slots, float* out, int G, int H, int D, int Dv) {
+                                     const int* state_slots, float* out, int G, int H, int D, int Dv, int longest) {
   constexpr size_t smem = (size_t)(6 * DS_CT * RG * R + 2 * DS_CT * VT + 2 * DS_CT) * sizeof(float);
   auto kernel = delta_scan_kernel<T, RG, R, VT>;
   if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   return launch_pdl(kernel, dim3((Dv + VT - 1) / VT, H, num_seqs), dim3(RG * VT), smem, stream, qn, kn, (const T*)vc, g,
-                    beta, state, cu_seqlens, state_slots, out, G, H, D, Dv);
+                    beta, state, cu_seqlens, state_slots, out, G, H, D, Dv, longest);
 }
 
-// qn, kn, vc, g, beta: delta_prepare's rows; state fp32 [slots, H, D, Dv]; out fp32 [T, H, Dv].
+// qn, kn, vc, g, beta: delta_prepare's rows; state fp32 [slots, H, D, Dv]; out fp32 [T, H, Dv].  Sequences of more than
+// `longest` tokens are left alone.
 Q3_EXPORT int q3_delta_scan(int dtype, const float* qn, const float* kn, const void* vc, const float* g,
                             const float* beta, float* state, const int* cu_seqlens, const int* state_slots, float* out,
-                            int num_seqs, int G, int H, int D, int Dv, cudaStream_t stream) {
+                            int num_seqs, int G, int H, int D, int Dv, int longest, cudaStream_t stream) {
   if (!qn || !kn || !vc || !g || !beta || !state || !cu_seqlens || !state_slots || !out) return Q3_ERR_ARGUMENT;
   if (G < 1 || H < 1 || H % G || D < 1 || Dv < 1 || H > 65535 || num_seqs > 65535) return Q3_ERR_ARGUMENT;
   if (D > 256 || (dtype != Q3_DTYPE_F32 && dtype != Q3_DTYPE_BF16)) return Q3_ERR_UNSUPPORTED;
@@ -359,7 +360,7 @@ Q3_EXPORT int q3_delta_scan(int dtype, const float* qn, const float* kn, const v
   cudaError_t e;
 #define Q3_DELTA_SCAN(T, RG, R, VT)                                                                                  \
   e = launch_delta_scan<T, RG, R, VT>(stream, num_seqs, qn, kn, vc, g, beta, state, cu_seqlens, state_slots, out, G, H, \
-                                      D, Dv)
+                                      D, Dv, longest)
 #define Q3_DELTA_SIZES(T)                                                                                            \
   if (D <= 16) Q3_DELTA_SCAN(T, 4, 4, 16); else if (D <= 32) Q3_DELTA_SCAN(T, 8, 4, 16);                              \
   else if (D <= 64) Q3_DELTA_SCAN(T, 8, 8, 16); else if (D <= 128) Q3_DELTA_SCAN(T, 16, 8, 16);                       \
@@ -394,7 +395,7 @@ template <int DP>
 __global__ void __launch_bounds__(256)
 delta_chunk_rows_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ g,
                         const float* __restrict__ beta, const int* __restrict__ cu_seqlens, int num_seqs,
-                        float* __restrict__ records, int G, int H, int D) {
+                        float* __restrict__ records, int G, int H, int D, int shortest) {
   __shared__ __align__(16) float ks[DC_C][DP], qs[DC_C][DP], gs[DC_C][DP];
   __shared__ float as[DC_C][DC_C + 1], bs[DC_C][DC_C + 1], be[DC_C];
   __shared__ int s_t0, s_n;
@@ -408,7 +409,7 @@ delta_chunk_rows_kernel(const float* __restrict__ qn, const float* __restrict__ 
       const int c0 = cu_seqlens[b], c1 = cu_seqlens[b + 1], base = c0 / DC_C + b;
       if (place >= base && place < c1 / DC_C + b + 1) {
         t0 = c0 + (place - base) * DC_C;
-        n = c1 - t0;
+        n = c1 - c0 < shortest ? 0 : c1 - t0;
         break;
       }
     }
@@ -549,7 +550,7 @@ template <typename T, int DP>
 __global__ void __launch_bounds__(256)
 delta_chunk_scan_kernel(const float* __restrict__ records, const T* __restrict__ vc, float* __restrict__ state,
                         const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots, float* __restrict__ out,
-                        int H, int D, int Dv) {
+                        int num_seqs, int H, int D, int Dv, int shortest) {
   constexpr int VT = 16, REC = DC_REC(DP), RD = DP / 64, PS = 20;  // PS: row pitch of the partial sums
   constexpr int STAGES = DC_STAGES;
   extern __shared__ __align__(16) float dc_smem[];
@@ -560,7 +561,19 @@ delta_chunk_scan_kernel(const float* __restrict__ records, const T* __restrict__
   pdl_wait();
   pdl_launch_dependents();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int h = blockIdx.y, b = blockIdx.z, col0 = blockIdx.x * VT;
+  const int h = blockIdx.y, col0 = blockIdx.x * VT;
+  int b = blockIdx.z;
+  if (shortest > 1) {  // the blockIdx.z-th sequence of at least that many tokens
+    int before = 0;
+    b = -1;
+    for (int b0 = 0; b0 < num_seqs && b < 0; b0 += 32) {
+      const bool in = b0 + lane < num_seqs && cu_seqlens[b0 + lane + 1] - cu_seqlens[b0 + lane] >= shortest;
+      const uint32_t found = __ballot_sync(0xffffffffu, in);
+      if (before + __popc(found) > (int)blockIdx.z) b = b0 + (int)__fns(found, 0, (int)blockIdx.z - before + 1);
+      before += __popc(found);
+    }
+    if (b < 0) return;
+  }
   const int t0 = cu_seqlens[b], t1 = cu_seqlens[b + 1];
   if (t1 <= t0) return;
   const int chunks = (t1 - t0 + DC_C - 1) / DC_C;
@@ -695,12 +708,13 @@ delta_chunk_scan_kernel(const float* __restrict__ records, const T* __restrict__
 }
 
 template <typename T, int DP>
-static int launch_delta_chunks(cudaStream_t stream, int num_tokens, int num_seqs, const float* qn, const float* kn,
+static int launch_delta_chunks(cudaStream_t stream, int num_tokens, int num_seqs, int num_long, const float* qn, const float* kn,
                                const void* vc, const float* g, const float* beta, float* records, float* state,
                                const int* cu_seqlens, const int* state_slots, float* out, int G, int H, int D, int Dv) {
   const int places = num_tokens / DC_C + num_seqs;
+  const int shortest = num_long < num_seqs ? 2 : 1;
   if (launch_pdl(delta_chunk_rows_kernel<DP>, dim3(places, H), dim3(256), 0, stream, qn, kn, g, beta, cu_seqlens, num_seqs,
-                 records, G, H, D) != cudaSuccess)
+                 records, G, H, D, shortest) != cudaSuccess)
     return Q3_ERR_LAUNCH;
   constexpr size_t smem = sizeof(float) * (DC_STAGES * DC_REC(DP) + DP * 16 + 8 * 32 * 20 + 2 * DC_C * 16);
   auto kernel = delta_chunk_scan_kernel<T, DP>;
@@ -712,24 +726,27 @@ static int launch_delta_chunks(cudaStream_t stream, int num_tokens, int num_seqs
     configured = true;
   }
   // Not as a dependent launch: its blocks would start between the last blocks of the kernel before, two of the longest
-  // sequence's on some SMs while others have none (2048 tokens: the scan 278 us instead of 225).
-  kernel<<<dim3((Dv + 15) / 16, H, num_seqs), dim3(256), smem, stream>>>(records, (const T*)vc, state, cu_seqlens,
-                                                                        state_slots, out, H, D, Dv);
+  // sequence's on some SMs while others have none (2048 tokens: the scan 278 us instead of 225).  No block for a one-token
+  // sequence either where num_long says so: with more blocks than SMs the first ones are no longer dealt out one to an SM
+  // (128 long blocks and 512 others: six SMs got two long ones; 16 heads, 2000 tokens beside 4 single ones: 496 us, so 435).
+  kernel<<<dim3((Dv + 15) / 16, H, num_long), dim3(256), smem, stream>>>(records, (const T*)vc, state, cu_seqlens,
+                                                                        state_slots, out, num_seqs, H, D, Dv, shortest);
   return q3_launch_status();
 }
 
-// The same as q3_delta_scan for key sizes up to 128, in chunks; records: (num_tokens / 16 + num_seqs) * H * (49 * DP +
+// The same as q3_delta_scan for key sizes up to 128, in chunks.  num_long: num_seqs, or the number of sequences of two tokens
+// and more, which are then the only ones served; records: (num_tokens / 16 + num_seqs) * H * (49 * DP +
 // 512) floats with DP = 64 (D <= 64) or 128.
 Q3_EXPORT int q3_delta_chunk_scan(int dtype, const float* qn, const float* kn, const void* vc, const float* g,
                                   const float* beta, float* records, float* state, const int* cu_seqlens,
-                                  const int* state_slots, float* out, int num_tokens, int num_seqs, int G, int H, int D,
-                                  int Dv, cudaStream_t stream) {
+                                  const int* state_slots, float* out, int num_tokens, int num_seqs, int num_long, int G,
+                                  int H, int D, int Dv, cudaStream_t stream) {
   if (!qn || !kn || !vc || !g || !beta || !records || !state || !cu_seqlens || !state_slots || !out) return Q3_ERR_ARGUMENT;
-  if (G < 1 || H < 1 || H % G || D < 1 || Dv < 1 || H > 65535 || num_seqs > 65535) return Q3_ERR_ARGUMENT;
+  if (G < 1 || H < 1 || H % G || D < 1 || Dv < 1 || H > 65535 || num_seqs > 65535 || num_long > num_seqs) return Q3_ERR_ARGUMENT;
   if (D > 128 || (dtype != Q3_DTYPE_F32 && dtype != Q3_DTYPE_BF16) || !ds_aligned(records)) return Q3_ERR_UNSUPPORTED;
-  if (num_seqs == 0 || num_tokens == 0) return Q3_OK;
+  if (num_long < 1 || num_tokens == 0) return Q3_OK;
 #define Q3_DELTA_CHUNKS(T, DP)                                                                                       \
-  return launch_delta_chunks<T, DP>(stream, num_tokens, num_seqs, qn, kn, vc, g, beta, records, state, cu_seqlens,   \
+  return launch_delta_chunks<T, DP>(stream, num_tokens, num_seqs, num_long, qn, kn, vc, g, beta, records, state, cu_seqlens,   \
                                     state_slots, out, G, H, D, Dv)
   if (dtype == Q3_DTYPE_F32) {
     if (D <= 64) Q3_DELTA_CHUNKS(float, 64);

@@ -141,9 +141,9 @@ _SIGNATURES = {
         "q3_ring_update": [c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                            c_void_p],
         "q3_delta_scan": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                          c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                          c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "q3_delta_chunk_scan": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                                c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "q3_delta_step": [c_int, c_void_p, c_long, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                           c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_float, c_void_p,
                           c_void_p, c_float, c_void_p, c_long, c_int, c_int, c_int, c_int, c_int, c_void_p],
@@ -924,13 +924,14 @@ class CudaOps:
         return C, taps
 
     def delta_rule(self, x, z, b, *, heads, kv_heads, dim, value_dim, conv_weight, ring, dt_bias, neg_a, state, positions,
-                   token_seq, cu_seqlens, state_slots, num_seqs, q_scale):
+                   token_seq, cu_seqlens, state_slots, num_seqs, q_scale, host_cu_seqlens=None):
         """The gated delta rule over a step's tokens (csrc/delta_state.cu): ``x`` ``[T, q heads | k heads | v heads]``
         is convolved per channel (``conv_weight`` float32 ``[taps, C]``; past inputs in ``ring`` float32 ``[slots, taps,
         C]``, brought up to date) and passed through silu, q and k become unit vectors (q times ``q_scale``), the decay
         per head and key channel is ``exp(neg_a[h] * softplus(z + dt_bias))`` (``z`` float32 ``[T, H * D]``), the step
         ``sigmoid(b)`` (``[T, H]``).  ``S <- decay * S; u = step * (v - S^T k); S <- S + k u^T; o = S^T q`` on the
-        float32 ``state`` ``[slots, H, D, Dv]``.  Returns float32 ``o`` ``[T, H, Dv]``."""
+        float32 ``state`` ``[slots, H, D, Dv]``.  Returns float32 ``o`` ``[T, H, Dv]``.  ``host_cu_seqlens``: the numbers
+        of ``cu_seqlens`` on the host, by which one-token sequences are told from prompts."""
         T = x.shape[0]
         H, G, D, Dv = heads, kv_heads, dim, value_dim
         C, taps = self._delta_columns(x, conv_weight, ring, G, H, D, Dv, "delta_rule")
@@ -960,19 +961,34 @@ class CudaOps:
         if self.timing is not None:
             self._costs(2 * num_seqs * H * D * Dv * 4 + T * (8 * G * D + H * Dv * (e + 4) + 4 * H * D),
                         7.0 * T * H * D * Dv)
+        longest = 0x7fffffff  # of the sequences that go token by token
         if self.delta_chunks and D <= 128 and T >= max(32, 4 * num_seqs):
             # prompts: chunks of 16 tokens (csrc/delta_state.cu); what does not depend on the state first
+            num_long = self._delta_long(host_cu_seqlens, int(num_seqs), H, Dv)
             padded = 64 if D <= 64 else 128
             records = torch.empty((T // 16 + num_seqs) * H * (49 * padded + 512), dtype=torch.float32, device=dev)
             self.launches += 1
             self._call("delta_state", "q3_delta_chunk_scan", "delta_chunk_scan", _dtype_code(x.dtype), _ptr(qn), _ptr(kn),
                        _ptr(vc), _ptr(g), _ptr(beta), _ptr(records), _ptr(state), _ptr(cu_seqlens), _ptr(state_slots),
-                       _ptr(out), T, int(num_seqs), G, H, D, Dv)
-            return out
+                       _ptr(out), T, int(num_seqs), num_long, G, H, D, Dv)
+            if num_long == num_seqs:
+                return out
+            longest = 1
         self._call("delta_state", "q3_delta_scan", "delta_scan", _dtype_code(x.dtype), _ptr(qn), _ptr(kn), _ptr(vc),
                    _ptr(g), _ptr(beta), _ptr(state), _ptr(cu_seqlens), _ptr(state_slots), _ptr(out), int(num_seqs), G, H,
-                   D, Dv)
+                   D, Dv, longest)
         return out
+
+    def _delta_long(self, cu, num_seqs, H, Dv) -> int:
+        """How many sequences of a step with prompts run in chunks: all, or those of two tokens and more.  Single tokens stay
+        apart where the prompts' blocks would have an SM each, which is lost when other blocks are launched with them
+        (csrc/delta_state.cu), and the tokens are few: 16 heads, us together / apart: 2000 tokens beside 4 single ones 496 / 435,
+        beside 20 497 / 464, 1000 beside 40 290 / 298; 32 heads (two blocks an SM anyway) 2000 beside 4 675 / 699."""
+        lens = [b - a for a, b in zip(cu, cu[1:])] if cu else []
+        num_long = sum(n > 1 for n in lens)
+        if num_long and num_long * H * -(-Dv // 16) <= self.SM_COUNT and max(lens) >= 40 * (num_seqs - num_long):
+            return num_long
+        return num_seqs
 
     def delta_step_ok(self, dim: int, value_dim: int) -> bool:
         """Whether :meth:`delta_step` takes heads of these sizes."""

@@ -18,7 +18,7 @@ from __future__ import annotations
 import torch
 
 from ..cache.layout import StateLayerSpec
-from .base import BuildContext, ParamSpec, StepContext, register_part
+from .base import BuildContext, ParamSpec, StepContext, register_part, scan_lengths
 from .linear_state import BranchMixer, _pad_rows
 
 
@@ -109,7 +109,7 @@ class GatedDelta(BranchMixer):
             return
         z = ops.linear(low_a, self.a2, out_dtype=torch.float32)
         gate = ops.linear(low_g, self.g2)
-        o = ops.delta_rule(x, z, b, token_seq=step.token_seq, **shared)
+        o = ops.delta_rule(x, z, b, token_seq=step.token_seq, **shared, **scan_lengths(ops, step))
         ops.head_norm_gate(o, gate.unflatten(1, (H, Dv)), out.unflatten(1, (H, Dv)), weight=self.norm_weight,
                            eps=self.eps, out_scale=out_scale, gate_act="sigmoid")
 

@@ -131,3 +131,14 @@ def test_a_scan_with_unknown_lengths_is_cut_as_one_sequence():
     assert ops._scan_segment(2048, 1, 16, 64, 128) == ops._scan_segment(2048, 32, 16, 64, 128) == 114
     assert ops._scan_segment(2048, 300, 16, 64, 128) == ops._scan_segment(63, 1, 16, 64, 128) == 0
     assert ops._scan_segment(2048, 1, 16, 136, 128) == 0
+
+
+def test_single_tokens_beside_one_delta_prompt_stay_out_of_its_chunks():
+    ops = _table()
+
+    def long(lens, heads=16, vdim=128):
+        return ops._delta_long(list(_cu(lens)), len(lens), heads, vdim)
+
+    assert long([2000] + [1] * 4) == long([1] * 10 + [2000] + [1] * 10) == 1 and long([1, 700], 8) == 1
+    assert long([1000] + [1] * 40) == 41 and long([2000] + [1] * 4, 32) == 5 and long([1500, 548, 1]) == 3
+    assert long([1500, 548]) == 2 and long([2048]) == 1 and ops._delta_long(None, 7, 16, 128) == 7
