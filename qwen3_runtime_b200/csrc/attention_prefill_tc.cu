@@ -19,7 +19,7 @@
 //   warp 0           : TMA producer (Q of both blocks once, then K and V tiles through rings of stages; the lanes issue a
 //                      tile's boxes side by side);
 //   warps 1 and 10,  : MMA issuers of block A and of block B.  Order per block: S_0, S_1, then
-//   one lane each      per tile j: P_j ready -> PV_j, S_(j+2).  S has two TMEM buffers per block,
+//   one lane each      per tile j: P_j ready -> PV_j, PV_j done -> S_(j+2).  S has two TMEM buffers per block,
 //                      so the tensor core works for one block while the other block's softmax
 //                      runs;
 //   warps 2..5, 6..9 : softmax of block A and of block B, one thread per row: reads S from
@@ -29,12 +29,14 @@
 //                      more than 2^8; finally stores O / l.  MAPS: block B's threads leave lambda O_B / l_B in shared
 //                      memory, block A's subtract it, divide by the root mean square and store.
 // Tensor memory: all 512 columns, per block S0 [0,64), S1 [64,128), O [128,256); P_j lies in S_j's columns.  S_(j+2) is
-// issued after PV_j by the same thread, and MMAs run in the order of issue, so it cannot overwrite P_j too early.
-// What bounds it: shared memory.  A QK step of 64 keys reads 6 KB per 32 cycles of MMA; with P in shared memory a tile and
-// block took about 900 cycles of its bandwidth against 512 of MMA and 512 of exp2, without it 640.  One layer of 2048 tokens,
-// 32 heads over 8: 49 us (57 with P in shared memory).  Forms: differential attention, 16 heads over 4, 2333 + 419 tokens: 61 us
-// (mma.sync: 247); latent, 16 heads, 2048 tokens, window 1024: 34 us and 26 us for the expansion (in the latent space on
-// mma.sync: 481).
+// issued when PV_j is complete: PTX promises an order of MMAs in flight only where they have the same accumulator and
+// shape, which these two have not.  The wait costs nothing (2048 tokens, 32 heads over 8: 56.3 us with and without; 8192: 584 and
+// 583), since the softmax has S_(j+1) by then.
+// What bounds it: the chain of a tile and block (S ready, TMEM load, exp2, TMEM store, barrier round trips); the products are
+// busy about a third of the time.  P in tensor memory instead of shared memory took little off it: one layer of 2048 tokens, 32
+// heads over 8, 58.4 -> 56.3 us, 64 heads over 8 110.6 -> 107.5 (behind a cold L2).  Forms: differential attention, 16 heads over 4,
+// 2333 + 419 tokens: 61 us (mma.sync: 247); latent, 16 heads, 2048 tokens, window 1024: 34 us and 26 us for the expansion (in
+// the latent space on mma.sync: 481).
 // V is the B operand of PV in MN-major form (rows = keys): descriptor with the halves of D
 // 8 KB apart (leading offset) and 8-key groups 1 KB apart (stride offset); 16 keys = 2 KB.
 // Keys past a block's last position are zeroed in shared memory before PV (stale or poisoned
@@ -309,7 +311,9 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
           } else {
             mbar_arrive(bar(BAR_V_EMPTY + st));
           }
-          if (j + 2 < num_tiles) ok = keys(j + 2);  // its TMEM buffer held S_j and P_j: PV_j runs before it
+          // S_(j+2) goes where S_j and P_j were: PV_j must have read P_j
+          if (j + 2 < num_tiles)
+            ok = (j + 2 >= my_tiles || mbar_wait(bar(BAR_PV_FULL + x), j & 1, &abort_flag)) && keys(j + 2);
         }
       }
     } else {  // ---- softmax: one thread per row; warps 2..5 block A, warps 6..9 block B ---------------
