@@ -176,3 +176,35 @@ def test_which_steps_expand(ops):
     assert rows([(8000, 8)], None) == 0 and rows([(8000, 8)], 1024) == 0
     assert rows([(1000, 512)], 100) == 512 + 1000 - 901 // 64 * 64
     assert rows([(5, 1), (9, 1)], None, decode=True) == 0
+
+
+def test_a_step_without_room_for_expanded_rows_stays_in_the_latent_space(ops):
+    from qwen3_runtime_b200.config import PartSpec
+
+    spec = PartSpec("latent_attention", dict(hidden_size=128, num_heads=32, dim=128, rot_dim=64, vdim=128, q_rank=64, kv_rank=64,
+                                             eps=1e-5, scale=192 ** -0.5, window=None, sink=True, gate=None,
+                                             position=PartSpec("rope_interleaved", dict(rotary_dim=64, theta=1e4))))
+    launched = []
+    call = ops._call
+    total = torch.cuda.get_device_properties(0).total_memory
+
+    def spy(group, name, what, *args):
+        launched.append(name)
+        return call(group, name, what, *args)
+
+    def no_room(ops):
+        # queries (98 MB), output (66) and the latent space's queries and rows (98) fit; queries, output, turned queries (33)
+        # and expanded keys and values (131) do not
+        torch.cuda.empty_cache()
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (300 << 20)) / total)
+        ops._call = spy
+
+        def restore():
+            del ops._call
+            torch.cuda.set_per_process_memory_fraction(1.0)
+
+        return restore
+
+    got, want = _steps(ops, spec, 16, [[8000]], [no_room, _set(latent_expand=False)])
+    assert "q3_dense_attention_prefill_tc" not in launched and "q3_rotate_heads" in launched
+    assert torch.equal(got[0], want[0])
