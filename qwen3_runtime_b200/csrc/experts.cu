@@ -105,18 +105,18 @@ __device__ __forceinline__ float4 load4(const bf16* p) {
   return make_float4(a.x, a.y, b.x, b.y);
 }
 
-constexpr int ROUTE_EPW = 8;               // experts per warp
-constexpr int ROUTE_WT = 1, ROUTE_WE = 4;  // warps of a block along tokens and along experts
+constexpr int ROUTE_EPW = 8;  // experts per warp
 
-template <typename T>
-__global__ void __launch_bounds__(32 * ROUTE_WT * ROUTE_WE, 3)
+// WT, WE: warps of a block along tokens and along experts
+template <typename T, int WT, int WE>
+__global__ void __launch_bounds__(32 * WT * WE, 3)
 route_logits_tile_kernel(const T* __restrict__ h, long h_stride, const float* __restrict__ router, int num_tokens, int E,
                          int W, float* __restrict__ logits) {
   pdl_wait();
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int t0 = (blockIdx.x * ROUTE_WT + warp / ROUTE_WE) * ROUTE_TT;
-  int e0 = (blockIdx.y * ROUTE_WE + warp % ROUTE_WE) * ROUTE_EPW;
+  int t0 = (blockIdx.x * WT + warp / WE) * ROUTE_TT;
+  int e0 = (blockIdx.y * WE + warp % WE) * ROUTE_EPW;
   if (t0 >= num_tokens || e0 >= E) return;
   // a last group that would pass the end starts earlier: its first logits are computed twice, with the same bits
   t0 = min(t0, num_tokens - ROUTE_TT);
@@ -361,16 +361,20 @@ Q3_EXPORT int q3_route_top(int dtype, const void* h, long h_stride, const float*
   // both kernels give the same bits; the tile kernel needs about 64 tokens to fill the SMs
   const bool tile = num_tokens > 64 && E >= ROUTE_EPW && W % 4 == 0 && h_stride % 4 == 0 &&
                     (reinterpret_cast<uintptr_t>(h) & (4 * elem - 1)) == 0;
-  const int te = ROUTE_WE * ROUTE_EPW;
+  // a block's four warps all have experts: 8 experts x 1024, 4096 tokens 23 us, with three idle warps a block 30
+  const int we = E > 2 * ROUTE_EPW ? 4 : E > ROUTE_EPW ? 2 : 1;
+  const int te = we * ROUTE_EPW, tokens = 4 / we * ROUTE_TT;
   cudaError_t e;
   if (tile && (E + te - 1) / te <= 65535) {
-    const dim3 grid((num_tokens + ROUTE_WT * ROUTE_TT - 1) / (ROUTE_WT * ROUTE_TT), (E + te - 1) / te);
-    if (dtype == Q3_DTYPE_F32)
-      e = launch_pdl(route_logits_tile_kernel<float>, grid, dim3(32 * ROUTE_WT * ROUTE_WE), 0, stream, (const float*)h, h_stride, router,
-                     num_tokens, E, W, logits);
-    else
-      e = launch_pdl(route_logits_tile_kernel<bf16>, grid, dim3(32 * ROUTE_WT * ROUTE_WE), 0, stream, (const bf16*)h, h_stride, router,
-                     num_tokens, E, W, logits);
+    const dim3 grid((num_tokens + tokens - 1) / tokens, (E + te - 1) / te);
+#define Q3_ROUTE_TILE(T_, WT_, WE_)                                                                                      \
+  e = launch_pdl(route_logits_tile_kernel<T_, WT_, WE_>, grid, dim3(32 * WT_ * WE_), 0, stream, (const T_*)h, h_stride, \
+                 router, num_tokens, E, W, logits)
+#define Q3_ROUTE_TILES(T_)                                                                                               \
+  do { if (we == 4) Q3_ROUTE_TILE(T_, 1, 4); else if (we == 2) Q3_ROUTE_TILE(T_, 2, 2); else Q3_ROUTE_TILE(T_, 4, 1); } while (0)
+    if (dtype == Q3_DTYPE_F32) Q3_ROUTE_TILES(float); else Q3_ROUTE_TILES(bf16);
+#undef Q3_ROUTE_TILES
+#undef Q3_ROUTE_TILE
   } else {
     int tt = num_tokens > 64 ? ROUTE_TT : 2;
     while (tt > 1 && (size_t)tt * W * sizeof(float) > 128 * 1024) tt >>= 1;  // fewer where their rows would not fit

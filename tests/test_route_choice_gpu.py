@@ -16,8 +16,8 @@ def _order(row: list[float], top: int) -> list[int]:
     return sorted(range(len(row)), key=lambda e: (math.isnan(row[e]), 0.0 if math.isnan(row[e]) else -row[e], e))[:top]
 
 
-@pytest.mark.parametrize("outputs", [40, 256, 257, 300])
-@pytest.mark.parametrize("tokens", [3, 70])
+@pytest.mark.parametrize("outputs", [8, 12, 17, 40, 256, 257, 300])
+@pytest.mark.parametrize("tokens", [3, 70, 97])
 @pytest.mark.parametrize("mode", [dict(), dict(renormalize=True), dict(score="softmax_chosen")])
 def test_choice_with_infinities_and_nan(outputs, tokens, mode):
     from qwen3_runtime_b200.ops.cuda import CudaOps
