@@ -412,8 +412,8 @@ Q3_EXPORT int q3_route_top(int dtype, const void* h, long h_stride, const float*
 }
 
 // ---- slots grouped by expert ----------------------------------------------------------------------
-// One block, for a few hundred slots.  Slots of one expert keep their order (slot s before slot
-// s' > s), so the grouping is the same on every run.
+// One block, for a few slots and experts.  Slots of one expert keep their order (slot s before slot
+// s' > s).
 __global__ void group_slots_kernel(const int* __restrict__ chosen, int S, int E, int bm, int* __restrict__ offsets,
                                    int* __restrict__ tile_offsets, int* __restrict__ order, int* __restrict__ place) {
   extern __shared__ int sm[];  // counts[E], cursor[E]
@@ -443,7 +443,7 @@ __global__ void group_slots_kernel(const int* __restrict__ chosen, int S, int E,
     const int e = chosen[s];
     int rank = 0;
     for (int r = 0; r < s; ++r) rank += chosen[r] == e;
-    order[cursor[e] + rank] = s;
+    if (order) order[cursor[e] + rank] = s;
     if (place) place[s] = cursor[e] + rank;
   }
 }
@@ -524,27 +524,28 @@ place_slots_kernel(const int* __restrict__ chosen, int S, int E, int bm, const i
   __syncthreads();
   if (e >= 0) {
     const int at = total[e] + before[e] + rank;
-    order[at] = s;
+    if (order) order[at] = s;
     if (place) place[s] = at;
   }
 }
 
-// bm: slots per row tile of the products that will use tile_offsets (EXPERT_BM for the FMA kernels).  place: int32 [S],
-// the position of every slot in the grouped order, or null.  scratch: int32 [S + ceil(S / 1024) * E], used for more than
-// 512 slots.
+// bm: slots per row tile of the products that will use tile_offsets (EXPERT_BM for the FMA kernels).  order: int32 [S], the
+// slots in the grouped order, or null.  place: int32 [S],
+// the position of every slot in the grouped order, or null.  scratch: int32 [S + ceil(S / 1024) * E] for the two kernels, or
+// null for the one block (512 slots at most).
 Q3_EXPORT int q3_group_slots(const int* chosen, int S, int E, int bm, int* offsets, int* tile_offsets, int* order,
                              int* place, int* scratch, cudaStream_t stream) {
-  if (!chosen || !offsets || !tile_offsets || !order || E < 1 || S < 0 || bm < 1) return Q3_ERR_ARGUMENT;
+  if (!chosen || !offsets || !tile_offsets || E < 1 || S < 0 || bm < 1) return Q3_ERR_ARGUMENT;
   if (E > 8192) return Q3_ERR_UNSUPPORTED;
   const size_t smem = 2 * (size_t)E * sizeof(int);
   cudaError_t e;
-  if (S <= 512) {
+  if (!scratch) {
+    if (S > 512) return Q3_ERR_ARGUMENT;
     if (smem > 48 * 1024)
       cudaFuncSetAttribute(group_slots_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     e = launch_pdl(group_slots_kernel, dim3(1), dim3(512), smem, stream, chosen, S, E, bm, offsets, tile_offsets,
                    order, place);
   } else {
-    if (!scratch) return Q3_ERR_ARGUMENT;
     if (smem > 48 * 1024)
       cudaFuncSetAttribute(place_slots_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const dim3 grid((S + GROUP_THREADS - 1) / GROUP_THREADS);

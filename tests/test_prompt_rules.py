@@ -133,6 +133,12 @@ def test_a_scan_with_unknown_lengths_is_cut_as_one_sequence():
     assert ops._scan_segment(2048, 1, 16, 136, 128) == 0
 
 
+def test_which_grouping_needs_scratch():
+    need = CudaOps._group_scratch
+    assert need(48, 8) == need(256, 48) == need(1, 1) == 0
+    assert need(257, 8) == 257 + 8 and need(16, 49) == 16 + 49 and need(1025, 64) == 1025 + 2 * 64
+
+
 def test_single_tokens_beside_one_delta_prompt_stay_out_of_its_chunks():
     ops = _table()
 
