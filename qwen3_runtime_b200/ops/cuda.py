@@ -316,6 +316,17 @@ def _segments(cu, seg):
     return sum(-(-n // seg) for n in lens), max(lens)
 
 
+def _one_wave(lens, most):
+    """The shortest segments, of 32 tokens and more, of which sequences of these lengths have ``most`` at most (0: there are
+    more sequences than that)."""
+    if not lens or len(lens) > most:
+        return 0
+    seg = max(32, -(-sum(lens) // most))
+    while sum(-(-n // seg) for n in lens) > most:  # the next length at which a sequence has a segment less
+        seg = min(-(-n // (-(-n // seg) - 1)) for n in lens if n > seg)
+    return seg
+
+
 @functools.lru_cache(maxsize=256)
 def decayed_scan_segment(cu, H, D, Dv, sms) -> int:
     """Tokens per segment of a bfloat16 step's decayed state scan, or 0 for the scan token by token, whichever the measured
@@ -338,8 +349,8 @@ def decayed_scan_segment(cu, H, D, Dv, sms) -> int:
     columns = H * -(-Dv // 16) / sms
     best = 0.9 * (c["chain"] + max(chain, (c["load"] * T + c["start"] * len(lens)) * columns + 0.5 * chain))
     found = 0
-    one_wave = min(512, max(32, -(-T // max(1, 2 * sms // blocks))))
-    for seg in sorted({32, 48, 64, 96, 128, 192, 256, 384, 512, one_wave, longest}):
+    one_wave = _one_wave([n for n in lens if n >= 32], max(1, 2 * sms // blocks))
+    for seg in sorted({32, 48, 64, 96, 128, 192, 256, 384, 512, one_wave or longest, longest}):
         if seg > longest:
             break
         count = sum(-(-n // seg) for n in lens)
@@ -348,7 +359,7 @@ def decayed_scan_segment(cu, H, D, Dv, sms) -> int:
             continue
         cost = c["row"] * T * H * (64 if D <= 64 else 128) + one_pass(T, count, min(seg, longest), *c["out"])
         cost += c["join"] + one_pass(more * seg, more, seg, *c["ends"]) if more else -c["whole"]
-        if seg == one_wave:  # its blocks end together: what the model does not see
+        if seg == one_wave:  # its blocks end together, which the model does not see
             cost *= 0.92
         if cost < best:
             best, found = cost, seg

@@ -119,11 +119,27 @@ def test_state_scans_are_cut_by_the_lengths_of_their_sequences():
     assert seg([64]) == seg([128]) == seg([1, 64, 1, 1, 1]) == seg([128] + [1] * 8) == seg([1] * 4096) == seg([15] * 64) == 0
     # many short prompts fill the SMs as they are: a segment each
     assert seg([64] * 32) == 64 and seg([128] * 16) == 128 and seg([32] * 64) == 32
-    # one prompt's blocks fill the SMs once
-    assert seg([2048]) == 114 and seg([2040], 32) == 227 and seg([2040], 16, 128) == 227
+    # a few prompts' blocks fill the SMs once
+    assert seg([2048]) == 114 and seg([2040], 32) == 227 and seg([2040], 16, 128) == 227 and seg([1024, 1024], 32) == 256
+    assert seg([2000] * 4, 64) == 2000
     assert seg([0, 0]) == 0 and seg([0, 700, 0]) == seg([700]) > 0
     # scratch (rows, and the segments' states where sequences are cut) stays within 1 GiB
     assert seg([8000] * 4, 64, 128, 128) == 0 and seg([4000], 64, 128, 128) > 0
+
+
+def test_segments_that_fill_the_sms_once():
+    import random
+
+    from qwen3_runtime_b200.ops.cuda import _one_wave
+
+    rnd = random.Random(0)
+    for _ in range(500):
+        lens, most = [rnd.randint(32, 3000) for _ in range(rnd.randint(1, 20))], rnd.randint(1, 40)
+        seg = _one_wave(lens, most)
+        count = lambda seg: sum(-(-n // seg) for n in lens)  # noqa: E731
+        assert (seg == 0) == (len(lens) > most)
+        assert not seg or (count(seg) <= most and (seg == 32 or count(seg - 1) > most))
+    assert _one_wave([], 5) == 0
 
 
 def test_a_scan_with_unknown_lengths_is_cut_as_one_sequence():

@@ -139,13 +139,14 @@ def test_steps_of_many_sequences(ops, D, Dv, seg):
     assert torch.equal(state[untouched].cpu(), start[untouched])
 
 
-def test_a_scan_without_room_for_its_scratch_runs_token_by_token(ops):
-    H, D, Dv, T = 16, 64, 128, 4096
+def test_a_scan_without_room_for_its_scratch_runs_token_by_token(ops, monkeypatch):
+    from qwen3_runtime_b200.ops import cuda
+
+    H, D, Dv, T = 16, 64, 128, 1024
     q, k, z = (torch.randn((T, H, D), device="cuda").bfloat16() for _ in range(3))
     v = torch.randn((T, H, Dv), device="cuda").bfloat16()
     kw = dict(cu_seqlens=torch.tensor([0, T], dtype=torch.int32, device="cuda"), num_seqs=1, decay_logits=z, tau=3.0,
               state_slots=torch.zeros(1, dtype=torch.int32, device="cuda"), host_cu_seqlens=[0, T])
-    state = torch.zeros((1, H, D, Dv), device="cuda")
     launched = []
     call = ops._call
 
@@ -153,16 +154,12 @@ def test_a_scan_without_room_for_its_scratch_runs_token_by_token(ops):
         launched.append(name)
         return call(group, name, what, *args)
 
-    ops._call = spy
-    total = torch.cuda.get_device_properties(0).total_memory
-    try:
-        with_room = ops.decayed_state_scan(q, k, v, state=state.clone(), **kw)
-        del with_room
-        torch.cuda.empty_cache()
-        # the output (33 MB) fits, the segments' scratch (70 MB) does not
-        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (70 << 20)) / total)
-        ops.decayed_state_scan(q, k, v, state=state.clone(), **kw)
-    finally:
-        torch.cuda.set_per_process_memory_fraction(1.0)
-        del ops._call
+    monkeypatch.setattr(ops, "_call", spy)
+    out = []
+    for room in (True, False):
+        if not room:  # 2^45 floats: more than any device has
+            monkeypatch.setattr(ops, "_scan_segment", lambda *args: 64)
+            monkeypatch.setattr(cuda, "_scan_scratch", lambda *args: 1 << 45)
+        out.append(ops.decayed_state_scan(q, k, v, state=torch.zeros((1, H, D, Dv), device="cuda"), **kw))
     assert launched == ["q3_decayed_segment_scan", "q3_decayed_state_scan"]
+    assert float((out[0] - out[1]).abs().max()) <= 3e-5 * float(out[1].abs().max())
