@@ -155,9 +155,98 @@ def test_expanded_keys_and_values(ops, heads, q_rank, gate, pairing, page, windo
     spec = PartSpec("latent_attention", dict(hidden_size=128, num_heads=heads, dim=128, rot_dim=64, vdim=128, q_rank=q_rank,
                                              kv_rank=kv_rank, eps=1e-5, scale=192 ** -0.5, window=window, sink=True, gate=gate,
                                              position=position))
-    got, want = _steps(ops, spec, page, RAGGED, [_set(LATENT_EXPAND_PAIRS=0), _set(latent_expand=False)])
+    launched = []
+    call = ops._call
+
+    def spied(**values):
+        def prepare(ops):
+            launched.append([])
+            ops._call = lambda group, name, what, *args: (launched[-1].append(name), call(group, name, what, *args))[1]
+            undo = _set(**values)(ops)
+
+            def restore():
+                undo()
+                del ops._call
+
+            return restore
+
+        return prepare
+
+    got, want = _steps(ops, spec, page, RAGGED, [spied(LATENT_EXPAND_PAIRS=0), spied(latent_expand=False)])
+    for step, names in enumerate(launched):  # every step of the first variant expands, none of the second
+        expanded = step < len(RAGGED)
+        assert names.count("q3_latent_gather") == names.count("q3_dense_attention_prefill_tc") == int(expanded)
+        assert any(n in names for n in ("q3_latent_attention", "q3_latent_attention_tc")) != expanded
     # queries, keys, values and the attended rows are rounded to bfloat16 at other places: four roundings on each side
     _close(got, want, 12)
+
+
+@pytest.mark.parametrize("window", [None, 90])
+@pytest.mark.parametrize("expand", [True, False])
+def test_latent_attention_against_float64(ops, window, expand):
+    """Both ways beside the layer as it is defined, in float64 on the layer's own bfloat16 tensors and rows."""
+    from qwen3_runtime_b200.config import PartSpec
+    from qwen3_runtime_b200.engine.batch import StepEntry
+
+    H, rank, W = 3, 64, 128
+    spec = PartSpec("latent_attention", dict(hidden_size=W, num_heads=H, dim=128, rot_dim=64, vdim=128, q_rank=0, kv_rank=rank,
+                                             eps=1e-5, scale=192 ** -0.5, window=window, sink=True, gate=None,
+                                             position=PartSpec("rope_interleaved", dict(rotary_dim=64, theta=1e4))))
+    part, cache, storage, builder = _layer(ops, spec, 16, 3, 60, 3)
+    g = torch.Generator().manual_seed(3)  # the tensors that _layer drew
+    t = {}
+    for name, ps in part.param_specs().items():
+        x = torch.randn(ps.shape, generator=g)
+        t[name] = ((1.0 + 0.1 * x) if ps.kind == "vector" else (x * ps.shape[-1] ** -0.5).bfloat16()).double()
+    handles = [cache.open(i) for i in range(3)]
+    past = [torch.zeros((0, rank + 64), dtype=torch.float64) for _ in handles]
+    inv = (1e4 ** (-torch.arange(0, 64, 2).float() / 64)).double()
+
+    def turn(x, pos):  # interleaved pairs
+        a = pos.double()[:, None] * inv
+        c, s = (f(a).reshape(-1, *[1] * (x.dim() - 2), 32) for f in (torch.cos, torch.sin))
+        u, v = x[..., 0::2], x[..., 1::2]
+        return torch.stack([u * c - v * s, u * s + v * c], -1).flatten(-2)
+
+    for lens in ([5, 200, 64], [130, 1, 70]):
+        entries = []
+        for rc, n in zip(handles, lens):
+            cache.reserve(rc, n)
+            entries.append(StepEntry(rc, [0] * n, []))
+        step = builder.build(entries, scratch_page=storage.scratch_page, scratch_slot=storage.scratch_slot)
+        h = torch.randn((sum(lens), W), generator=g).bfloat16()
+        restore = (_set(LATENT_EXPAND_PAIRS=0) if expand else _set(latent_expand=False))(ops)
+        try:
+            out = part.forward(h.cuda(), step, storage.view(0)).cpu().double()
+        finally:
+            restore()
+        ops.raise_if_kernel_error()
+        at = 0
+        for b, n in enumerate(lens):
+            x = h[at:at + n].double()
+            pos = torch.arange(past[b].shape[0], past[b].shape[0] + n)
+            q = (x @ t["q"].T).view(n, H, 192)
+            q = torch.cat([q[..., :128], turn(q[..., 128:], pos)], -1)
+            c = x @ t["dkv"].T
+            row = torch.cat([c[:, :rank] / (c[:, :rank].pow(2).mean(-1, keepdim=True) + 1e-5).sqrt() * t["dkv.norm"],
+                             turn(c[:, rank:], pos)], -1)
+            past[b] = torch.cat([past[b], row])
+            k = torch.cat([(past[b][:, :rank] @ t["uk"].T).view(-1, H, 128), past[b][:, None, rank:].expand(-1, H, -1)], -1)
+            v = (past[b][:, :rank] @ t["uv"].T).view(-1, H, 128)
+            s = torch.einsum("qhd,khd->hqk", q, k) * 192 ** -0.5
+            key = torch.arange(past[b].shape[0])
+            hidden = key[None] > pos[:, None]
+            if window:
+                hidden |= key[None] <= pos[:, None] - window
+            s = s.masked_fill(hidden, float("-inf"))
+            p = torch.softmax(torch.cat([s, t["sink"].view(H, 1, 1).expand(H, n, 1)], -1), -1)[..., :-1]
+            want = torch.einsum("hqk,khd->qhd", p, v).reshape(n, -1) @ t["o"].T
+            got = out[at:at + n]
+            # five roundings to bfloat16 (2^-9 each) on the way: row, query, key and value, attended row, output
+            assert float((got - want).norm()) <= 5 * 2.0 ** -9 * 2 * float(want.norm()), (b, n)
+            at += n
+        for e in entries:
+            cache.commit(e.cache, len(e.tokens))
 
 
 def test_which_steps_expand(ops):
@@ -184,27 +273,15 @@ def test_a_step_without_room_for_expanded_rows_stays_in_the_latent_space(ops):
     spec = PartSpec("latent_attention", dict(hidden_size=128, num_heads=32, dim=128, rot_dim=64, vdim=128, q_rank=64, kv_rank=64,
                                              eps=1e-5, scale=192 ** -0.5, window=None, sink=True, gate=None,
                                              position=PartSpec("rope_interleaved", dict(rotary_dim=64, theta=1e4))))
-    launched = []
-    call = ops._call
-    total = torch.cuda.get_device_properties(0).total_memory
-
-    def spy(group, name, what, *args):
-        launched.append(name)
-        return call(group, name, what, *args)
+    asked = []
 
     def no_room(ops):
-        # queries (98 MB), output (66) and the latent space's queries and rows (98) fit; queries, output, turned queries (33)
-        # and expanded keys and values (131) do not
-        torch.cuda.empty_cache()
-        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (300 << 20)) / total)
-        ops._call = spy
+        def expanded(*args, **kw):
+            asked.append(kw["page_size"])
+            raise torch.OutOfMemoryError("no room for the expanded rows")
 
-        def restore():
-            del ops._call
-            torch.cuda.set_per_process_memory_fraction(1.0)
+        ops.latent_attention_expanded = expanded
+        return lambda: ops.__dict__.pop("latent_attention_expanded")
 
-        return restore
-
-    got, want = _steps(ops, spec, 16, [[8000]], [no_room, _set(latent_expand=False)])
-    assert "q3_dense_attention_prefill_tc" not in launched and "q3_rotate_heads" in launched
-    assert torch.equal(got[0], want[0])
+    got, want = _steps(ops, spec, 16, [[300, 64], [100, 0]], [no_room, _set(latent_expand=False)])
+    assert asked == [16, 16] and all(torch.equal(a, b) for a, b in zip(got, want))
