@@ -1,5 +1,6 @@
 // Routed experts: router scores and choice, grouping of (token, choice) slots by expert on the
-// device, the experts' two products over their own slots, and the per-token sum.
+// device, the experts' two products over their own slots on the FMA pipes (float32, and bfloat16 of sizes
+// that experts_tcgen05.cu refuses), and the per-token sum.
 //
 //   route_top      z = W_router h in fp32, the `top` largest z (the order of their sigmoids; lowest
 //                  index on a tie) with sigmoid(z) as weights (optionally divided by their sum), or
@@ -23,20 +24,18 @@
 constexpr int EXPERT_BM = 32;  // slots per row tile of the FMA products
 
 // ---- router ------------------------------------------------------------------------------------
-// Two kernels.  route_logits: a block stages tokens' rows in shared memory as fp32 and each
-// of its eight warps streams one expert's router row once for all of them (a step of a few tokens
-// still spreads the router over E / 8 blocks).  route_pick: one warp per token takes the `top`
-// largest logits -- the choice is made on the logits, which order the experts as their sigmoids do
-// but do not collapse into ties where the sigmoid saturates; lowest index on an exact tie -- and
-// writes sigmoid(logit) as the weight.
-//
-// Two kernels with the same order of additions (a token's logits are the same bits in every batch): lane l adds the
-// products of k = 4 l .. 4 l + 3, then of those + 128, and so on; the lanes' sums are added by halving.
-//   few tokens: a block stages 2 tokens' rows in shared memory, a warp computes one expert's logits, so that a decode
-//   step's router runs on tens of SMs;
-//   many tokens: a warp keeps 8 tokens x 8 experts in registers and reads operands straight from L1 (a block 8 tokens x
-//   32 experts).  With one expert per warp the reads of the tokens' values, not the FMAs, set the time: 2048 tokens x 64
-//   experts x 2048 took 87 us, with four experts per warp 47, now 27 (FMAs alone: 7).
+// Logits, then the choice.  Two kernels compute logits, with the same order of additions (a token's logits are the same bits
+// in every batch): lane l adds the products of k = 4 l .. 4 l + 3, then of those + 128, and so on; the lanes' sums are added by
+// halving.
+//   few tokens (route_logits): a block stages 2 tokens' rows in shared memory as fp32, each of its eight warps streams one
+//   expert's router row for them, so that a decode step's router runs on tens of SMs;
+//   many tokens (route_logits_tile): a warp keeps 8 tokens x 8 experts in registers and reads operands straight from L1.  With
+//   fewer experts a warp the reads of the tokens' values, not the FMAs, set the time: 2048 tokens x 64 experts x 2048 27 us,
+//   with four experts per warp 47 (FMAs alone: 7).
+// Three kernels choose, one warp per token: the `top` largest logits -- the choice is made on the logits, which order the
+// experts as their sigmoids do but do not collapse into ties where the sigmoid saturates; lowest index on an exact tie, NaN
+// after every number -- with logits in registers (route_pick_regs, up to 256 outputs) or in memory (route_pick), and the choice
+// on a softmax over all outputs (route_pick_softmax_all).
 constexpr int ROUTE_TT = 8;
 
 template <typename T>

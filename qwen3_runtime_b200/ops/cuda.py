@@ -1295,8 +1295,9 @@ class CudaOps:
         offsets, tile_offsets, order = plan[: EA + 1], plan[EA + 1: 2 * (EA + 1)], plan[2 * (EA + 1): 2 * (EA + 1) + S]
         on_input = weight_on == "input"
         # bfloat16 with 16-byte rows: the products run on the tensor cores (csrc/experts_tcgen05.cu).  Measured against
-        # mma.sync tiles of 32 and 64 slots that it replaced, gate_up + down of 64 experts of 1408 x 2048, top 6: 8 tokens
-        # 129 against 173 us, 128 tokens 200 / 303, 2048 tokens 298 / 1606; no size was slower.
+        # mma.sync tiles of 32 and 64 slots, gate_up + down of 64 experts of 1408 x 2048, top 6: 8 tokens 129 against 173 us,
+        # 128 tokens 200 / 303, 2048 tokens 298 / 1606.  Whole layers, 8 to 256 experts of 256 to 4096, both units, 18 sizes
+        # from 1 to 4096 tokens: none slower (1 token, 64 experts 86 / 126; 256 experts of 256, 64 tokens 118 / 120).
         if (self.experts_tc and h.dtype == torch.bfloat16 and W % 8 == 0 and F % 8 == 0 and h.stride(0) % 8 == 0
                 and h.data_ptr() % 16 == 0):
             return self._routed_experts_tc(h, chosen, weights if on_input else None, None if on_input else weights, gate_up,
