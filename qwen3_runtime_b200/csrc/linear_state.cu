@@ -36,10 +36,11 @@
 // one the slot.  All decays are at most one, so nothing grows, and every sum is fp32 as before.  The rotations, decays and
 // scales of a token's rows are worked out by a kernel of their own (16 us), not in both passes and every column tile.  A
 // thread holds 4 x 8 elements of the state, so that a token's three rows and its values are read once for 32 updates, as
-// pairs of columns for the packed instructions (the issue slots bound the passes), and the sums over the row groups are
-// folded: a lane gives half of its columns away at each step.  A block finds its sequence with one warp, 32 sequences at a
-// time (one thread walking 128 sequences cost every block of every pass 20 us).  When this is the faster one, and with
-// which `seg`, is worked out from the sequences' lengths (ops/cuda.py, decayed_scan_segment).
+// pairs of columns for the packed instructions, and the sums over the row groups are folded: a lane gives half of its
+// columns away at each step.  The passes are bound by a block's chain over its tokens at two blocks an SM (issue slots 40 and 50 %
+// busy; waits for arithmetic and shared memory).  A block finds its sequence with one warp, 32 sequences at a time (one thread
+// walking 128 sequences cost every block of every pass 20 us).  When this is the faster scan, and with which `seg`, is worked
+// out from the sequences' lengths (ops/cuda.py, decayed_scan_segment).
 //
 // head_norm_gate: y[t, h, :] = o / sqrt(mean(o^2) + eps) * w * silu(g[t, h, :]) * out_scale, one warp
 // per (token, head); w may be absent.
