@@ -286,9 +286,9 @@ class _Span:
 # ---- decayed state scans of bfloat16 steps: token by token or in segments -------------------------
 SCAN_SCRATCH = 1 << 28  # floats a segment scan may ask for (1 GiB)
 
-# Times in us of the two scans (csrc/linear_state.cu) on a B200, by the padded key size: least squares over 52 compositions
+# Times in us of the two scans (csrc/linear_state.cu) on a B200, by the padded key size: least squares over 48 compositions
 # of sequences (one token to 8,000, alone, in equal numbers and mixed, up to 128 of them) x 6 head counts and sizes x up to 10
-# segment lengths; 6 % off on average.  A pass of the segments takes the longer of one block's chain (`alone` per token)
+# segment lengths; 8 % off on average.  A pass of the segments takes the longer of one block's chain (`alone` per token)
 # and all blocks at two per SM (`shared` per token, `block` per block); rows and joining cost `row` and `join` more, and
 # without a cut the first pass's launch is saved (`whole`).  The scan token by token takes the longer of the longest sequence
 # (`chain_token`) and all of its blocks of 16 columns (`load` per token, `start` per block).
@@ -330,11 +330,12 @@ def _one_wave(lens, most):
 @functools.lru_cache(maxsize=256)
 def decayed_scan_segment(cu, H, D, Dv, sms) -> int:
     """Tokens per segment of a bfloat16 step's decayed state scan, or 0 for the scan token by token, whichever the measured
-    costs make the fastest (segments where they win by 10 % at least).  A segment's length follows from the whole step: one
-    prompt is cut so that its blocks fill the SMs once at two each, many short prompts fill them as they are.  Layers of 16
-    heads of 64 x 128, us token by token / so: 64 tokens 22 / 22; 512 118 / 65; 2040 443 / 133; 2040 beside 31 single tokens 775 / 207,
-    beside 127 817 / 325; 8 prompts of 256 244 / 150; 32 of 64 234 / 112.  A step of one short prompt and single tokens is never
-    cut where its blocks leave most SMs idle (16 heads of 128 x 128, 128 tokens beside 8: 75 / 83)."""
+    costs make the fastest (segments where they win by 5 % at least).  A segment's length follows from the whole step: a few
+    prompts are cut so that their blocks fill the SMs once at two each, many short prompts fill them as they are.  16 heads
+    of 64 x 128, us token by token / so: 64 tokens 22 / 22; 512 118 / 65; 2040 446 / 134; 2040 beside 31 single tokens 760 / 190,
+    beside 127 817 / 341; 8 prompts of 256 244 / 155; 32 of 64 246 / 114; over 150 compositions nothing was slower than token by
+    token.  A step of one short prompt and single tokens is never cut where its blocks leave most SMs idle (16 heads of
+    128 x 128, 128 tokens beside 8: 75 / 83)."""
     lens = [b - a for a, b in zip(cu, cu[1:])]
     T, longest = sum(lens), max(lens)
     c = SCAN_COSTS[64 if D <= 64 else 128]
@@ -347,7 +348,7 @@ def decayed_scan_segment(cu, H, D, Dv, sms) -> int:
 
     chain = c["chain_token"] * longest
     columns = H * -(-Dv // 16) / sms
-    best = 0.9 * (c["chain"] + max(chain, (c["load"] * T + c["start"] * len(lens)) * columns + 0.5 * chain))
+    best = 0.95 * (c["chain"] + max(chain, (c["load"] * T + c["start"] * len(lens)) * columns + 0.5 * chain))
     found = 0
     one_wave = _one_wave([n for n in lens if n >= 32], max(1, 2 * sms // blocks))
     for seg in sorted({32, 48, 64, 96, 128, 192, 256, 384, 512, one_wave or longest, longest}):
@@ -360,7 +361,7 @@ def decayed_scan_segment(cu, H, D, Dv, sms) -> int:
         cost = c["row"] * T * H * (64 if D <= 64 else 128) + one_pass(T, count, min(seg, longest), *c["out"])
         cost += c["join"] + one_pass(more * seg, more, seg, *c["ends"]) if more else -c["whole"]
         if seg == one_wave:  # its blocks end together, which the model does not see
-            cost *= 0.92
+            cost *= 0.88
         if cost < best:
             best, found = cost, seg
     return found
