@@ -18,6 +18,7 @@
 //   delta_step       all of it for steps in which every sequence brings one token, with the decay's and the
 //                    gate's second low-rank products and the heads' output norm and gate: one kernel
 #include "common.cuh"
+#include "mma_tiles.cuh"
 
 #define DELTA_MAX_TAPS 16
 #define UNIT_EPS 1e-6f
@@ -375,50 +376,133 @@ Q3_EXPORT int q3_delta_scan(int dtype, const float* qn, const float* kn, const v
 // With G_i the product of a chunk's decays up to token i and S the state before the chunk, the recurrence is, in
 // matrices whose rows are the chunk's tokens (the WY form of a product of rank-one updates):
 //   A_ij = sum_d k_i k_j prod_(j < m <= i) g_m  (j < i)        B_ij = sum_d q_i k_j prod_(j < m <= i) g_m  (j <= i)
-//   W = (I + diag(beta) A)^(-1) diag(beta)
-//   U = W (V - (G k) S)      O = (G q) S + B U      S <- G_last S + sum_j (prod_(m > j) g_m k_j) u_j^T
-// Only products of decays occur, never quotients, so strong decays lose nothing.  All of it is fp32 FMA.
+//   P = (I + diag(beta) A)^(-1) diag(beta) (G k)                U0 = (I + diag(beta) A)^(-1) diag(beta) V
+//   Q = G q - B P                                              O0 = B U0
+//   U = U0 - P S      O = O0 + Q S      S <- G_last S + sum_j (prod_(m > j) g_m k_j) u_j^T
+// P, Q, U0 and O0 do not depend on the state, so only two products are left in the chain from chunk to chunk.  A row of P
+// is beta_i k_i times a product of contractions and no longer than beta_i |k_i|.  Only products of decays occur, never
+// quotients, so strong decays lose nothing.  All of it is fp32 FMA.
 //
-// delta_chunk_rows: everything that does not depend on the state, a record of DC_REC floats per (chunk, head):
-// [DP][32] (G k | G q, transposed), [16][DP] the decayed-to-the-end keys, [DP] G_last, W and B [16][16].  Chunks of
-// sequence b start at place cu_seqlens[b] / 16 + b; tokens beyond a portion's end are k = q = 0, g = 1, beta = 0.
-// Its pair products run down j with the decays' products in registers, 16 lanes to a row, and 30 shuffles fold a row's
-// sums (five per sum before); the substitution for W, a chain of 120 multiply-adds in 16 lanes, runs beside the record's
-// writing, which is in whole rows of 128 bytes.  2048 tokens of 16 heads: 48 -> 39 us.
-// delta_chunk_scan: one block per (16 value columns, head, sequence); the state's columns stay in registers (and, for
-// the products with it, in shared memory), the next chunks' records are on their way while one is worked on.
+// Products of matrices run on mma.sync with every operand as the sum of three bfloat16 (24 bits: nothing is lost) and the six
+// products of parts that matter, the largest alone and added last; what a product adds to the state is summed from zero and
+// added to it in fp32, once per chunk.  Everything else is fp32 FMA.  Against float64 (700 + 300 tokens, 16 heads of 128,
+// mean decays of 0.95 / 0.9997 a token): outputs 1.2e-7 / 2.2e-7, state 1.0e-7 / 2.2e-7; with FMA throughout 1.3e-7 / 3.4e-7
+// and 1.0e-7 / 3.6e-7.
+//
+// delta_chunk_rows: everything that does not depend on the state.  A record of DC_REC words per (chunk, head), operands in
+// three parts in the order of the products' fragments: P, Q and the decayed-to-the-end keys [DP / 16][3][32 lanes][4], G_last
+// [DP] in fp32; U0 in rows of its own, O0 where the output will be.  Chunks of sequence b start at place cu_seqlens[b] / 16 + b;
+// tokens beyond a portion's end are k = q = 0, g = 1, beta = 0.
+// delta_chunk_scan: one block per (16 value columns, head, sequence); the state's columns stay in registers, the next chunks'
+// records are on their way while one is worked on.
+// 1500 + 548 tokens of 16 heads, rows and scan: 41 + 225 us with FMA, four barriers a chunk and W, B in the chain; 56 + 114 us
+// now.  (The scan on FMA without W and B in the chain 144 us, on mma.sync with both halves' work in all warps 159, with the
+// parts made in the scan instead of stored 125; the rows with substitutions for every column on FMA 68.)
 #define DC_C 16
-#define DC_STAGES 3  // records in shared memory: with two a chunk waited for its record (2048 tokens: the mixer 423 us, with three 407)
-#define DC_REC(DP) ((DP) * 49 + 2 * DC_C * DC_C)
+#define DC_REC(DP) ((DP) * 73)
 
-template <int DP>
-__global__ void __launch_bounds__(256)
-delta_chunk_rows_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ g,
-                        const float* __restrict__ beta, const int* __restrict__ cu_seqlens, int num_seqs,
-                        float* __restrict__ records, int G, int H, int D, int shortest) {
-  __shared__ __align__(16) float ks[DC_C][DP], qs[DC_C][DP], gs[DC_C][DP];
-  __shared__ float as[DC_C][DC_C + 1], bs[DC_C][DC_C + 1], be[DC_C];
-  __shared__ int s_t0, s_n;
+// (x, y) as the sum of three bfloat16 pairs
+__device__ __forceinline__ void ds_split(float x, float y, uint32_t (&p)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p[i]) : "f"(y), "f"(x));
+    x -= __uint_as_float(p[i] << 16);
+    y -= __uint_as_float(p[i] & 0xffff0000u);
+  }
+}
+
+__device__ __forceinline__ void ds_copy16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
+}
+
+// four words of each of the three parts: a left operand, or two tiles of a right one
+__device__ __forceinline__ void ds_parts(uint32_t (&p)[3][4], const uint32_t* from, int lane) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const uint4 w = *reinterpret_cast<const uint4*>(from + i * 128 + lane * 4);
+    p[i][0] = w.x;
+    p[i][1] = w.y;
+    p[i][2] = w.z;
+    p[i][3] = w.w;
+  }
+}
+__device__ __forceinline__ void ds_mma_zero(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// acc = a b over 16 channels (or tokens) for two tiles of eight rows (or channels), operands in three parts.  The largest
+// product stands alone and is added last, rounded to nearest; the tiles' chains run side by side.
+// EXACT: b is bfloat16 as it is.
+template <bool EXACT = false>
+__device__ __forceinline__ void ds_products(float (&acc)[2][4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][4]) {
+  float small[2][4], mid[2][4];
+  auto set = [&](float(&sum)[2][4], int i, int j) {
+#pragma unroll
+    for (int n = 0; n < 2; ++n) ds_mma_zero(sum[n], a[i], b[j][2 * n], b[j][2 * n + 1]);
+  };
+  auto add = [&](float(&sum)[2][4], int i, int j) {
+#pragma unroll
+    for (int n = 0; n < 2; ++n) mma_bf16(sum[n], a[i], b[j][2 * n], b[j][2 * n + 1]);
+  };
+  if constexpr (EXACT) {
+    set(small, 2, 0);
+    set(mid, 1, 0);
+    set(acc, 0, 0);
+  } else {
+    set(small, 2, 0);
+    set(mid, 0, 1);
+    set(acc, 0, 0);
+    add(small, 0, 2);
+    add(mid, 1, 0);
+    add(small, 1, 1);
+  }
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[n][j] += mid[n][j] + small[n][j];
+}
+
+// A block makes one record.  Loads; the pairs' sums A and B; then, side by side, the decayed keys and queries (warps 4 up, in
+// place) and the 16 x 16 matrices W = (I + diag(beta) A)^(-1) diag(beta) and B W by substitution, a lane per column (warps 0
+// and 1); then a warp makes 16 channels of P = W (G k) and Q = G q - (B W) (G k) and 16 value columns of U0 = W V and O0 =
+// (B W) V on the tensor cores, whose accumulators are the fragments that the scan reads.  What bounds it is the number of its
+// instructions (14 000 a block, issued in half of the cycles).
+template <typename T, int DP>
+__global__ void __launch_bounds__(256, 3)
+delta_chunk_rows_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const T* __restrict__ vc,
+                        const float* __restrict__ g, const float* __restrict__ beta, const int* __restrict__ cu_seqlens,
+                        int num_seqs, uint32_t* __restrict__ records, float* __restrict__ u0, float* __restrict__ out,
+                        int G, int H, int D, int Dv, int shortest) {
+  constexpr int PITCH = DP + 4;  // tokens two apart lie 8 banks apart
+  __shared__ __align__(16) float ks[DC_C][PITCH], qs[DC_C][PITCH], gs[DC_C][PITCH];  // later: keys to the end, G q, G k
+  __shared__ __align__(16) float at[DC_C][DC_C], bt[DC_C][DC_C];                      // A and B, transposed
+  __shared__ __align__(16) uint32_t tp[2][3 * 128];                                   // W and B W as left operands
+  __shared__ float be[DC_C];
   pdl_wait();
   pdl_launch_dependents();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gr = lane >> 2, t4 = lane & 3;
   const int place = blockIdx.x, h = blockIdx.y, gh = h / (H / G);
-  if (tid == 0) {
-    int n = 0, t0 = 0;
-    for (int b = 0; b < num_seqs; ++b) {
+  int n = 0;
+  long t0 = 0;
+  for (int b0 = 0; b0 < num_seqs; b0 += 32) {  // whose chunk this is, every warp for itself, 32 sequences at a time
+    const int b = b0 + lane;
+    int first = 0, left = 0;
+    bool found = false;
+    if (b < num_seqs) {
       const int c0 = cu_seqlens[b], c1 = cu_seqlens[b + 1], base = c0 / DC_C + b;
-      if (place >= base && place < c1 / DC_C + b + 1) {
-        t0 = c0 + (place - base) * DC_C;
-        n = c1 - c0 < shortest ? 0 : c1 - t0;
-        break;
-      }
+      found = place >= base && place < c1 / DC_C + b + 1;
+      first = c0 + (place - base) * DC_C;
+      left = c1 - c0 < shortest ? 0 : min(c1 - first, DC_C);
     }
-    s_t0 = t0;
-    s_n = n > DC_C ? DC_C : n;
+    const uint32_t who = __ballot_sync(0xffffffffu, found);
+    if (who) {
+      t0 = __shfl_sync(0xffffffffu, first, __ffs(who) - 1);
+      n = __shfl_sync(0xffffffffu, left, __ffs(who) - 1);
+      break;
+    }
   }
-  __syncthreads();
-  const int n = s_n;
-  const long t0 = s_t0;
   if (n <= 0) return;
   // (whole 16 bytes where rows are made of them)
   const bool vec = D % 4 == 0 && (((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)g) & 15) == 0;
@@ -426,141 +510,254 @@ delta_chunk_rows_kernel(const float* __restrict__ qn, const float* __restrict__ 
   for (int x = tid * 4; x < DC_C * DP; x += 1024) {
     const int c = x / DP, i = x - c * DP;
     const long gi = ((t0 + c) * G + gh) * D + i, hi = ((t0 + c) * H + h) * D + i;
-    float4 k4 = make_float4(0.f, 0.f, 0.f, 0.f), q4 = k4, g4 = make_float4(1.f, 1.f, 1.f, 1.f);
-    if (c < n && i < D) {
-      if (vec) {
-        k4 = *reinterpret_cast<const float4*>(kn + gi);
-        q4 = *reinterpret_cast<const float4*>(qn + gi);
-        g4 = *reinterpret_cast<const float4*>(g + hi);
-      } else {
-        const bool in1 = i + 1 < D, in2 = i + 2 < D, in3 = i + 3 < D;
-        k4 = make_float4(kn[gi], in1 ? kn[gi + 1] : 0.f, in2 ? kn[gi + 2] : 0.f, in3 ? kn[gi + 3] : 0.f);
-        q4 = make_float4(qn[gi], in1 ? qn[gi + 1] : 0.f, in2 ? qn[gi + 2] : 0.f, in3 ? qn[gi + 3] : 0.f);
-        g4 = make_float4(g[hi], in1 ? g[hi + 1] : 1.f, in2 ? g[hi + 2] : 1.f, in3 ? g[hi + 3] : 1.f);
+    const bool live = c < n && i < D;
+    if (live && vec) {
+      ds_copy16(&ks[c][i], kn + gi);
+      ds_copy16(&qs[c][i], qn + gi);
+      ds_copy16(&gs[c][i], g + hi);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const bool in = live && i + e < D;
+        ks[c][i + e] = in ? kn[gi + e] : 0.f;
+        qs[c][i + e] = in ? qn[gi + e] : 0.f;
+        gs[c][i + e] = in ? g[hi + e] : 1.f;
       }
     }
-    *reinterpret_cast<float4*>(&ks[c][i]) = k4;
-    *reinterpret_cast<float4*>(&qs[c][i]) = q4;
-    *reinterpret_cast<float4*>(&gs[c][i]) = g4;
   }
   if (tid < DC_C) be[tid] = tid < n ? beta[(t0 + tid) * H + h] : 0.f;
-  __syncthreads();
-  {  // rows i of A and B, i = warp in the even lanes and 15 - warp in the odd ones; 16 lanes share the channels
-    constexpr int E = DP / 64;
-    const int i = lane & 1 ? DC_C - 1 - warp : warp, cl = lane >> 1;
-    float v[2 * DC_C];  // A_ij, then B_ij, this lane's channels
-    float wk[4 * E], wq[4 * E], qi[4 * E];
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  // this lane's values of the first 128 columns: tokens 2 t4, 2 t4 + 1, 2 t4 + 8, 2 t4 + 9 of columns 16 warp + gr (+ 8)
+  T vr[2][4];
+  auto values = [&](int col) {
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const float4 q4 = *reinterpret_cast<const float4*>(&qs[i][cl * 4 + 64 * e]);
-      qi[4 * e] = q4.x; qi[4 * e + 1] = q4.y; qi[4 * e + 2] = q4.z; qi[4 * e + 3] = q4.w;
-#pragma unroll
-      for (int m = 0; m < 4; ++m) wk[4 * e + m] = wq[4 * e + m] = 0.f;  // until j comes down to i
+    for (int x = 0; x < 4; ++x) {
+      const int c = 2 * t4 + (x & 1) + 4 * (x & 2);
+      const T* src = vc + ((t0 + c) * H + h) * Dv + col;
+      vr[0][x] = c < n && col < Dv ? src[0] : from_f32<T>(0.f);
+      vr[1][x] = c < n && col + 8 < Dv ? src[8] : from_f32<T>(0.f);
     }
+  };
+  values(warp * 16 + gr);
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+  {  // rows 15 - warp and warp of A and B, 17 pairs of tokens for every warp; the lanes share the channels
+    constexpr int E = DP / 32;
+    float v[48];  // row 15 - warp: A_ij, then B_ij, by i - j; row warp: the same
+    auto row = [&](const float* from, float(&to)[E]) {
+      if constexpr (E == 4) {
+        const float4 x = *reinterpret_cast<const float4*>(from + lane * 4);
+        to[0] = x.x; to[1] = x.y; to[2] = x.z; to[3] = x.w;
+      } else {
+        const float2 x = *reinterpret_cast<const float2*>(from + lane * 2);
+        to[0] = x.x; to[1] = x.y;
+      }
+    };
+    auto pairs = [&](int i, int most, int at_a, int at_b) {
+      float wk[E], wq[E];
+      row(ks[i], wk);
+      row(qs[i], wq);
 #pragma unroll
-    for (int j = DC_C - 1; j >= 0; --j) {
-      float a = 0.f, b = 0.f;
-      if (j <= DC_C - 1 - warp) {
+      for (int r = 0; r < most; ++r) {
+        float a = 0.f, b = 0.f;
+        if (r <= i) {
+          float kj[E], gj[E];
+          row(ks[i - r], kj);
+          row(gs[i - r], gj);
 #pragma unroll
-        for (int e = 0; e < E; ++e) {
-          const float4 k4 = *reinterpret_cast<const float4*>(&ks[j][cl * 4 + 64 * e]);
-          const float4 g4 = *reinterpret_cast<const float4*>(&gs[j][cl * 4 + 64 * e]);
-          const float kj[4] = {k4.x, k4.y, k4.z, k4.w}, gj[4] = {g4.x, g4.y, g4.z, g4.w};
-#pragma unroll
-          for (int m = 0; m < 4; ++m) {
-            float &x = wk[4 * e + m], &y = wq[4 * e + m];
-            x = j == i ? kj[m] : x;
-            y = j == i ? qi[4 * e + m] : y;
-            a = fmaf(x, kj[m], a);
-            b = fmaf(y, kj[m], b);
-            x *= gj[m];
-            y *= gj[m];
+          for (int e = 0; e < E; ++e) {
+            a = fmaf(wk[e], kj[e], a);
+            b = fmaf(wq[e], kj[e], b);
+            wk[e] *= gj[e];
+            wq[e] *= gj[e];
           }
         }
+        v[at_a + r] = a;  // (A's diagonal is not used)
+        v[at_b + r] = b;
       }
-      v[j] = a;
-      v[DC_C + j] = b;
-    }
-    // the sums over the 16 lanes: a lane gives half of its values away at each step and has two of them in the end
+    };
+    pairs(DC_C - 1 - warp, 16, 0, 16);
+    pairs(warp, 8, 32, 40);
+    // the sums over the lanes: a lane gives half of its values away at each step and has three of them in the end
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
-      const int half = DC_C >> s;
-      const bool up = (cl >> s) & 1;
+      const int half = 24 >> s;
+      const bool up = (lane >> s) & 1;
 #pragma unroll
       for (int x = 0; x < half; ++x) {
         const float give = up ? v[x] : v[x + half];
-        v[x] = (up ? v[x + half] : v[x]) + __shfl_xor_sync(0xffffffffu, give, 2 << s);
+        v[x] = (up ? v[x + half] : v[x]) + __shfl_xor_sync(0xffffffffu, give, 1 << s);
       }
     }
-    const int j = 4 * (cl & 2) + (cl & 4) + 2 * ((cl >> 3) & 1);
-    float* dst = cl & 1 ? &bs[i][j] : &as[i][j];  // (A's diagonal is not used)
-    dst[0] = v[0];
-    dst[1] = v[1];
+#pragma unroll
+    for (int x = 0; x < 3; ++x) v[x] += __shfl_xor_sync(0xffffffffu, v[x], 16);
+    if (lane < 16) {
+      const int first = (lane & 1) * 24 + (lane & 2) * 6 + (lane & 4) / 4 * 6 + (lane & 8) / 8 * 3;
+#pragma unroll
+      for (int x = 0; x < 3; ++x) {
+        const int at_v = first + x;
+        const int i = at_v < 32 ? DC_C - 1 - warp : warp, r = at_v < 32 ? at_v & 15 : at_v & 7;
+        const bool is_b = at_v < 32 ? at_v >= 16 : at_v >= 40;
+        if (r <= i) (is_b ? bt : at)[i - r][i] = v[x];
+      }
+    }
   }
   __syncthreads();
-  float* rec = records + ((long)place * H + h) * DC_REC(DP);
-  if (warp == 0) {  // a chain of 120 multiply-adds while the other warps write the rest of the record
-    if (tid < DC_C) {  // column tid of W by forward substitution
-      float x[DC_C];
+  uint32_t* rec = records + ((long)place * H + h) * DC_REC(DP);
+  if (warp < 2) {  // column c of W (warp 0) or of B W (warp 1), in two lanes
+    const int c = lane & 15;
+    float x[DC_C], y[DC_C];
 #pragma unroll
-      for (int i = 0; i < DC_C; ++i) {
-        float acc = i == tid ? 1.f : 0.f;
+    for (int i = 0; i < DC_C; ++i) x[i] = i == c ? 1.f : 0.f, y[i] = 0.f;
 #pragma unroll
-        for (int j = 0; j < i; ++j) acc = fmaf(-as[i][j], x[j], acc);
-        x[i] = be[i] * acc;
-        rec[49 * DP + i * DC_C + tid] = x[i];
+    for (int j = 0; j < DC_C; ++j) {
+      x[j] *= be[j];
+#pragma unroll
+      for (int i4 = j / 4 * 4; i4 < DC_C; i4 += 4) {
+        const float4 a4 = *reinterpret_cast<const float4*>(&at[j][i4]);
+        const float4 b4 = *reinterpret_cast<const float4*>(&bt[j][i4]);
+        const float av[4] = {a4.x, a4.y, a4.z, a4.w}, bv[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+          if (i4 + m > j) x[i4 + m] = fmaf(-av[m], x[j], x[i4 + m]);
+          if (i4 + m >= j) y[i4 + m] = fmaf(bv[m], x[j], y[i4 + m]);
+        }
       }
     }
-    return;
-  }
-  const int at = tid - 32;
-  for (int x = at; x < 8 * DP; x += 224) {  // the keys and queries decayed from the chunk's start, four tokens of a channel
-    const int d = x >> 3, c0 = (x & 3) * 4;
-    float run = 1.f;
+    // a lane's rows are eight, and two lanes make pairs of columns: the even one those of even rows
+    const int half = lane >> 4;
+    const bool odd = c & 1;
 #pragma unroll
-    for (int c = 0; c < DC_C - 4; ++c)
-      if (c < c0) run *= gs[c][d];
-    const float(*src)[DP] = x & 4 ? qs : ks;
-    float r[4];
+    for (int m = 0; m < 4; ++m) {
+      float r[2];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      run *= gs[c0 + e][d];
-      r[e] = run * src[c0 + e][d];
+      for (int e = 0; e < 2; ++e)
+        r[e] = warp ? (half ? y[2 * m + e + 8] : y[2 * m + e]) : (half ? x[2 * m + e + 8] : x[2 * m + e]);
+      const float other = __shfl_xor_sync(0xffffffffu, odd ? r[0] : r[1], 1);
+      uint32_t p[3];
+      ds_split(odd ? other : r[0], odd ? r[1] : other, p);
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        tp[warp][i * 128 + ((2 * m + odd) * 4 + ((c & 7) >> 1)) * 4 + half + 2 * (c >> 3)] = p[i];
     }
-    *reinterpret_cast<float4*>(rec + 4 * x) = make_float4(r[0], r[1], r[2], r[3]);
-    if ((x & 7) == 3) rec[48 * DP + d] = run;
-  }
-  if (at < DP) {  // the keys decayed to the chunk's end
-    float run = 1.f;
+  } else if (tid >= 128 && tid - 128 < DP) {  // decays from the chunk's start and to its end
+    const int d = tid - 128;
+    float run = 1.f, gd[DC_C], kd[DC_C];
 #pragma unroll
-    for (int c = DC_C - 1; c >= 0; --c) {
-      rec[32 * DP + c * DP + at] = run * ks[c][at];
-      run *= gs[c][at];
+    for (int i = 0; i < DC_C; ++i) {
+      gd[i] = gs[i][d];
+      kd[i] = ks[i][d];
+      run *= gd[i];
+      gs[i][d] = run * kd[i];
+      qs[i][d] *= run;
+    }
+    rec[72 * DP + d] = __float_as_uint(run);
+    run = 1.f;
+#pragma unroll
+    for (int i = DC_C - 1; i >= 0; --i) {
+      ks[i][d] = run * kd[i];
+      run *= gd[i];
     }
   }
-  for (int x = at; x < DC_C * DC_C; x += 224)
-    rec[49 * DP + DC_C * DC_C + x] = x % DC_C <= x / DC_C ? bs[x / DC_C][x % DC_C] : 0.f;
+  __syncthreads();
+  uint32_t w3[3][4], bw3[3][4];
+  ds_parts(w3, tp[0], lane);
+  ds_parts(bw3, tp[1], lane);
+  // tokens 2 t4, 2 t4 + 1, 2 t4 + 8, 2 t4 + 9 of channels 16 warp + gr (+ 8), in parts
+  auto right = [&](const float(*from)[PITCH], uint32_t(&to)[3][4]) {
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const float* f = &from[2 * t4 + 8 * (x & 1)][warp * 16 + gr + 4 * (x & 2)];
+      uint32_t p[3];
+      ds_split(f[0], f[PITCH], p);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) to[m][x] = p[m];
+    }
+  };
+  auto store = [&](uint32_t* to, const uint32_t (&p)[3][4]) {
+#pragma unroll
+    for (int m = 0; m < 3; ++m)
+      *reinterpret_cast<uint4*>(to + m * 128 + lane * 4) = make_uint4(p[m][0], p[m][1], p[m][2], p[m][3]);
+  };
+  if (warp < DP / 16) {
+    uint32_t gk[3][4];
+    float acc[2][4];
+    // accumulators (rows gr, gr + 8; channels 2 t4, 2 t4 + 1 of two tiles) as two tiles of eight rows of the scan's right operand
+    auto record = [&](uint32_t* to) {
+      uint32_t r[3][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          uint32_t p[3];
+          ds_split(acc[x][2 * i], acc[x][2 * i + 1], p);
+#pragma unroll
+          for (int m = 0; m < 3; ++m) r[m][2 * i + x] = p[m];
+        }
+      store(to + warp * 384, r);
+    };
+    right(gs, gk);
+    ds_products(acc, w3, gk);
+    record(rec);
+    ds_products(acc, bw3, gk);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        const float2 q = *reinterpret_cast<const float2*>(&qs[gr + 8 * i][warp * 16 + 8 * x + 2 * t4]);
+        acc[x][2 * i] = q.x - acc[x][2 * i];
+        acc[x][2 * i + 1] = q.y - acc[x][2 * i + 1];
+      }
+    record(rec + 24 * DP);
+    right(ks, gk);
+    store(rec + 48 * DP + warp * 384, gk);
+  }
+  for (int col = warp * 16; col < Dv; col += 128) {
+    if (col >= 128) values(col + gr);
+    uint32_t v3[3][4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      uint32_t p[3];
+      ds_split(to_f32(vr[x >> 1][2 * (x & 1)]), to_f32(vr[x >> 1][2 * (x & 1) + 1]), p);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) v3[m][x] = p[m];
+    }
+    auto rows_out = [&](float* to, const uint32_t (&left)[3][4]) {
+      float acc[2][4];
+      ds_products<sizeof(T) == 2>(acc, left, v3);
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int c = gr + 4 * (j & 2), i = col + 8 * x + 2 * t4 + (j & 1);
+          if (c < n && i < Dv) to[((t0 + c) * H + h) * Dv + i] = acc[x][j];
+        }
+    };
+    rows_out(u0, w3);
+    rows_out(out, bw3);
+  }
 }
 
-__device__ __forceinline__ void ds_copy16(float* dst, const float* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
-}
-
-template <typename T, int DP>
-__global__ void __launch_bounds__(256)
-delta_chunk_scan_kernel(const float* __restrict__ records, const T* __restrict__ vc, float* __restrict__ state,
-                        const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots, float* __restrict__ out,
-                        int num_seqs, int H, int D, int Dv, int shortest) {
-  constexpr int VT = 16, REC = DC_REC(DP), RD = DP / 64, PS = 20;  // PS: row pitch of the partial sums
-  constexpr int STAGES = DC_STAGES;
-  extern __shared__ __align__(16) float dc_smem[];
-  float* Ss = dc_smem + STAGES * REC;  // [DP][VT]
-  float* part = Ss + DP * VT;          // [8][32][PS]
-  float* ys = part + 8 * 32 * PS;      // [16][VT]
-  float* us = ys + DC_C * VT;          // [16][VT]
+// The state is held transposed, as the accumulators of its update (rows: the 16 value columns; columns: a warp's 16
+// channels), which is also the layout of the left operand of the products with it.  Half of the warps are the chain: P S
+// (the warps' parts are added through shared memory), U, the update, two barriers a chunk.  The other half fetches the
+// records and makes O from the state's parts, which the chain leaves in shared memory, while the chain goes on.  What bounds
+// it is the chain's latency, 1.0 us a chunk (products 0.2, shared memory two thirds busy).  `out` holds O0.
+template <int DP>
+__global__ void __launch_bounds__(4 * DP, 2)
+delta_chunk_scan_kernel(const float* __restrict__ records, const float* __restrict__ u0, float* __restrict__ state,
+                        const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots, float* out, int num_seqs,
+                        int H, int D, int Dv, int shortest) {
+  constexpr int VT = 16, REC = DC_REC(DP), NT = 4 * DP, WARPS = DP / 16;
+  extern __shared__ __align__(16) uint32_t dc_smem[];                    // two records, then
+  float2* part = reinterpret_cast<float2*>(dc_smem + 2 * REC);           // [P, Q][WARPS][2 tiles][2 column halves][32]
+  uint32_t* ss = reinterpret_cast<uint32_t*>(part + 2 * WARPS * 128);    // the state's parts: [WARPS][3][32][4]
+  uint32_t* us = ss + WARPS * 384;                                       // U's: [3][32][4]
   pdl_wait();
   pdl_launch_dependents();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+  const bool chain = tid < NT / 2;
+  const int wtid = chain ? tid : tid - NT / 2, warp = wtid >> 5;
   const int h = blockIdx.y, col0 = blockIdx.x * VT;
   int b = blockIdx.z;
   if (shortest > 1) {  // the blockIdx.z-th sequence of at least that many tokens
@@ -577,177 +774,188 @@ delta_chunk_scan_kernel(const float* __restrict__ records, const T* __restrict__
   const int t0 = cu_seqlens[b], t1 = cu_seqlens[b + 1];
   if (t1 <= t0) return;
   const int chunks = (t1 - t0 + DC_C - 1) / DC_C;
-  const float* rec0 = records + ((long)(t0 / DC_C + b) * H + h) * REC;
-  auto load = [&](int c) {
-    if (c < chunks) {
-      const float* src = rec0 + (long)c * H * REC;
-      float* dst = dc_smem + (c % STAGES) * REC;
-      for (int x = tid * 4; x < REC; x += 1024) ds_copy16(dst + x, src + x);
+  // A thread's sums (the first four warps of a half): tile of eight rows, half of the columns, lane of the fragment: two tokens
+  // of a column.
+  const int o_col = col0 + ((wtid & 31) >> 2) + ((wtid >> 2) & 8), o_tok = ((wtid >> 3) & 8) + 2 * (wtid & 3);
+  const bool sums = wtid < 128 && o_col < Dv;
+  float x_next = 0.f, y_next = 0.f;
+  auto base_value = [&](const float* rows, int c) {
+    const int t = t0 + c * DC_C + o_tok;
+    const float* p = rows + ((long)t * H + h) * Dv + o_col;
+    x_next = sums && t < t1 ? p[0] : 0.f;
+    y_next = sums && t + 1 < t1 ? p[(long)H * Dv] : 0.f;
+  };
+  auto sum_parts = [&](const float2* from) {
+    float2 s = from[wtid];
+#pragma unroll
+    for (int w = 1; w < WARPS; ++w) {
+      const float2 p = from[w * 128 + wtid];
+      s.x += p.x;
+      s.y += p.y;
     }
-    asm volatile("cp.async.commit_group;\n" ::);  // also when empty: one group per call
+    return s;
   };
+  auto write_part = [&](float2* to, const float(&acc)[2][4]) {
 #pragma unroll
-  for (int c = 0; c < STAGES - 1; ++c) load(c);
-  // Lane bits 0 and 2 choose four columns, bits 1, 3 and 4 the rows: lanes that differ in bit 0 (or in bit 1) then read the
-  // same address, and a 16-byte load takes two cycles of shared memory instead of four.
-  const int c0 = ((lane & 1) | ((lane >> 1) & 2)) * 4, group = ((lane >> 1) & 1) | ((lane >> 2) & 6);
-  const int d0 = warp * 8 * RD + group;  // this thread's rows of the state: d0 + 8 r
-  float* Sg = state + ((long)state_slots[b] * H + h) * (long)D * Dv;
-  float S[RD][4];
-#pragma unroll
-  for (int r = 0; r < RD; ++r) {
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      S[r][e] = d0 + 8 * r < D && col0 + c0 + e < Dv ? Sg[(long)(d0 + 8 * r) * Dv + col0 + c0 + e] : 0.f;
-    *reinterpret_cast<float4*>(Ss + (d0 + 8 * r) * VT + c0) = make_float4(S[r][0], S[r][1], S[r][2], S[r][3]);
-  }
-  // the chunk's token and the value column of the small products; a warp's tokens are four apart, whose partial sums lie in
-  // different banks
-  const int row = (warp & 3) + 8 * (warp >> 2) + 4 * (lane >> 4), col = tid & 15;
-  const bool col_in = col0 + col < Dv;
-  auto value = [&](int c) {
-    const long t = t0 + c * DC_C + row;
-    return col_in && t < t1 ? to_f32(vc[(t * H + h) * Dv + col0 + col]) : 0.f;
+    for (int i = 0; i < 2; ++i) {
+      to[warp * 128 + i * 64 + lane] = make_float2(acc[i][0], acc[i][1]);
+      to[warp * 128 + i * 64 + 32 + lane] = make_float2(acc[i][2], acc[i][3]);
+    }
   };
-  float v_next = value(0);
-  const int rt = group * 4, ct = c0;
-  for (int c = 0; c < chunks; ++c) {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2));
-    __syncthreads();  // the record and the state in shared memory are complete; nobody reads the last record any more
-    const float* rec = dc_smem + (c % STAGES) * REC;
-    load(c + STAGES - 1);
-    const float v = v_next;
-    if (c + 1 < chunks) v_next = value(c + 1);
-    {  // [G k; G q] S, an eighth of the channels a warp, 4 x 4 sums a thread
-      float acc[4][4];
+  if (!chain) {
+    // P is needed a barrier before the rest of its record: its next one is asked for as soon as the last one has been read
+    const uint32_t* rec0 = reinterpret_cast<const uint32_t*>(records) + ((long)(t0 / DC_C + b) * H + h) * REC;
+    auto load = [&](int c, int what) {  // what: 1 for P, 2 for the rest
+      if (c < chunks) {
+        const uint32_t* src = rec0 + (long)c * H * REC + wtid * 4;
+        uint32_t* dst = dc_smem + (c & 1) * REC + wtid * 4;
+        if (what & 1) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+          for (int x = 0; x < 3; ++x) ds_copy16(dst + x * 2 * NT, src + x * 2 * NT);  // 24 DP words
+        }
+        if (what & 2) {
 #pragma unroll
-      for (int dd = 0; dd < DP / 8; ++dd) {
-        const int d = warp * (DP / 8) + dd;
-        const float4 a = *reinterpret_cast<const float4*>(rec + d * 32 + rt);
-        const float4 s = *reinterpret_cast<const float4*>(Ss + d * VT + ct);
-        const float av[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          acc[i][0] = fmaf(av[i], s.x, acc[i][0]);
-          acc[i][1] = fmaf(av[i], s.y, acc[i][1]);
-          acc[i][2] = fmaf(av[i], s.z, acc[i][2]);
-          acc[i][3] = fmaf(av[i], s.w, acc[i][3]);
+          for (int x = 3; x < 9; ++x) ds_copy16(dst + x * 2 * NT, src + x * 2 * NT);
+          if (wtid < DP / 4) ds_copy16(dst + 18 * NT, src + 18 * NT);
         }
       }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        *reinterpret_cast<float4*>(part + (warp * 32 + rt + i) * PS + ct) =
-            make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-    }
-    __syncthreads();
-    float pk = 0.f, o = 0.f;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) {
-      pk += part[(w * 32 + row) * PS + col];
-      o += part[(w * 32 + 16 + row) * PS + col];
-    }
-    ys[row * VT + col] = v - pk;
-    __syncthreads();
-    {
-      const float* W = rec + 49 * DP + row * DC_C;
-      float u = 0.f;
-#pragma unroll
-      for (int j = 0; j < DC_C; j += 4) {  // (W is zero beyond the diagonal)
-        const float4 w4 = *reinterpret_cast<const float4*>(W + j);
-        u = fmaf(w4.x, ys[j * VT + col], u);
-        u = fmaf(w4.y, ys[(j + 1) * VT + col], u);
-        u = fmaf(w4.z, ys[(j + 2) * VT + col], u);
-        u = fmaf(w4.w, ys[(j + 3) * VT + col], u);
-      }
-      us[row * VT + col] = u;
-    }
-    __syncthreads();
-    {
-      const float* B = rec + 49 * DP + DC_C * DC_C + row * DC_C;
-#pragma unroll
-      for (int j = 0; j < DC_C; j += 4) {
-        const float4 b4 = *reinterpret_cast<const float4*>(B + j);
-        o = fmaf(b4.x, us[j * VT + col], o);
-        o = fmaf(b4.y, us[(j + 1) * VT + col], o);
-        o = fmaf(b4.z, us[(j + 2) * VT + col], o);
-        o = fmaf(b4.w, us[(j + 3) * VT + col], o);
-      }
-      const long t = t0 + c * DC_C + row;
-      if (col_in && t < t1) out[(t * H + h) * Dv + col0 + col] = o;
-    }
-    const float* kend = rec + 32 * DP;
-#pragma unroll
-    for (int r = 0; r < RD; ++r) {
-      const float gl = rec[48 * DP + d0 + 8 * r];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) S[r][e] *= gl;
-    }
-#pragma unroll
-    for (int j = 0; j < DC_C; ++j) {
-      const float4 u4 = *reinterpret_cast<const float4*>(us + j * VT + c0);
-#pragma unroll
-      for (int r = 0; r < RD; ++r) {
-        const float kk = kend[j * DP + d0 + 8 * r];
-        S[r][0] = fmaf(kk, u4.x, S[r][0]);
-        S[r][1] = fmaf(kk, u4.y, S[r][1]);
-        S[r][2] = fmaf(kk, u4.z, S[r][2]);
-        S[r][3] = fmaf(kk, u4.w, S[r][3]);
+    };
+    load(0, 3);
+    load(1, 1);
+    asm volatile("cp.async.commit_group;\n" ::);
+    base_value(out, 0);
+    asm volatile("cp.async.wait_group 0;\n" ::);
+    asm volatile("bar.sync 2, %0;" ::"n"(NT) : "memory");  // the first record is there
+    for (int c = 0; c < chunks; ++c) {
+      asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");  // the state's parts are there; P and the last record have been read
+      asm volatile("cp.async.wait_group 0;\n" ::);
+      load(c + 1, 2);
+      load(c + 2, 1);
+      asm volatile("cp.async.commit_group;\n" ::);
+      uint32_t a[3][4], q[3][4];
+      ds_parts(a, ss + warp * 384, lane);
+      asm volatile("bar.sync 3, %0;" ::"n"(NT / 2) : "memory");  // everyone's copies of the group before have arrived
+      asm volatile("bar.arrive 2, %0;" ::"n"(NT) : "memory");  // the next P is there, the state's parts are read
+      ds_parts(q, dc_smem + (c & 1) * REC + 24 * DP + warp * 384, lane);
+      float acc[2][4];
+      ds_products(acc, a, q);
+      write_part(part + WARPS * 128, acc);
+      asm volatile("bar.sync 3, %0;" ::"n"(NT / 2) : "memory");
+      if (wtid < 128) {
+        const float2 s = sum_parts(part + WARPS * 128);
+        const int t = t0 + c * DC_C + o_tok;
+        float* p = out + ((long)t * H + h) * Dv + o_col;
+        if (sums && t < t1) p[0] = x_next + s.x;
+        if (sums && t + 1 < t1) p[(long)H * Dv] = y_next + s.y;
+        base_value(out, c + 1);
       }
     }
+    return;
+  }
+  float* Sg = state + ((long)state_slots[b] * H + h) * (long)D * Dv;
+  float S[2][4];  // channel 16 warp + 8 i + 2 t4 + (j & 1), value column g + 8 (j >> 1)
 #pragma unroll
-    for (int r = 0; r < RD; ++r)
-      *reinterpret_cast<float4*>(Ss + (d0 + 8 * r) * VT + c0) = make_float4(S[r][0], S[r][1], S[r][2], S[r][3]);
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int d = warp * 16 + 8 * i + 2 * t4 + (j & 1), col = col0 + g + 8 * (j >> 1);
+      S[i][j] = d < D && col < Dv ? Sg[(long)d * Dv + col] : 0.f;
+    }
+  base_value(u0, 0);
+  auto state_product = [&](const uint32_t* rec) {
+    uint32_t a[3][4], p[3][4];
+    ds_parts(p, rec + warp * 384, lane);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      uint32_t w[3];
+      ds_split(S[i >> 1][2 * (i & 1)], S[i >> 1][2 * (i & 1) + 1], w);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) a[m][i] = w[m];
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      *reinterpret_cast<uint4*>(ss + warp * 384 + i * 128 + lane * 4) = make_uint4(a[i][0], a[i][1], a[i][2], a[i][3]);
+    float acc[2][4];
+    ds_products(acc, a, p);
+    write_part(part, acc);
+  };
+  asm volatile("bar.sync 2, %0;" ::"n"(NT) : "memory");
+  state_product(dc_smem);
+  for (int c = 0; c < chunks; ++c) {
+    asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
+    if (wtid < 128) {
+      const float2 s = sum_parts(part);
+      uint32_t p[3];
+      ds_split(x_next - s.x, y_next - s.y, p);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) us[i * 128 + (wtid & 31) * 4 + (wtid >> 5)] = p[i];
+      base_value(u0, c + 1);
+    }
+    asm volatile("bar.sync 2, %0;" ::"n"(NT) : "memory");
+    const uint32_t* rec = dc_smem + (c & 1) * REC;
+    uint32_t a[3][4], k[3][4];
+    ds_parts(k, rec + 48 * DP + warp * 384, lane);
+    ds_parts(a, us, lane);
+    float acc[2][4];
+    ds_products(acc, a, k);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float2 gl = *reinterpret_cast<const float2*>(rec + 72 * DP + warp * 16 + 8 * i + 2 * t4);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) S[i][j] = fmaf(j & 1 ? gl.y : gl.x, S[i][j], acc[i][j]);
+    }
+    state_product(dc_smem + ((c + 1) & 1) * REC);  // (behind the last chunk: nobody reads what this makes)
   }
 #pragma unroll
-  for (int r = 0; r < RD; ++r)
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (d0 + 8 * r < D && col0 + c0 + e < Dv) Sg[(long)(d0 + 8 * r) * Dv + col0 + c0 + e] = S[r][e];
+    for (int j = 0; j < 4; ++j) {
+      const int d = warp * 16 + 8 * i + 2 * t4 + (j & 1), col = col0 + g + 8 * (j >> 1);
+      if (d < D && col < Dv) Sg[(long)d * Dv + col] = S[i][j];
+    }
 }
 
 template <typename T, int DP>
 static int launch_delta_chunks(cudaStream_t stream, int num_tokens, int num_seqs, int num_long, const float* qn, const float* kn,
-                               const void* vc, const float* g, const float* beta, float* records, float* state,
+                               const void* vc, const float* g, const float* beta, float* records, float* u0, float* state,
                                const int* cu_seqlens, const int* state_slots, float* out, int G, int H, int D, int Dv) {
   const int places = num_tokens / DC_C + num_seqs;
   const int shortest = num_long < num_seqs ? 2 : 1;
-  if (launch_pdl(delta_chunk_rows_kernel<DP>, dim3(places, H), dim3(256), 0, stream, qn, kn, g, beta, cu_seqlens, num_seqs,
-                 records, G, H, D, shortest) != cudaSuccess)
-    return Q3_ERR_LAUNCH;
-  constexpr size_t smem = sizeof(float) * (DC_STAGES * DC_REC(DP) + DP * 16 + 8 * 32 * 20 + 2 * DC_C * 16);
-  auto kernel = delta_chunk_scan_kernel<T, DP>;
+  constexpr size_t smem = sizeof(float) * (2 * DC_REC(DP) + DP * 32 + DP * 24 + 3 * 128);
+  auto rows = delta_chunk_rows_kernel<T, DP>;
+  auto scan = delta_chunk_scan_kernel<DP>;
   static bool configured_on[Q3_MAX_DEVICES];
   bool& configured = configured_on[q3_current_device()];
   if (!configured) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      return Q3_ERR_LAUNCH;
+    if (cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return Q3_ERR_LAUNCH;
     configured = true;
   }
+  if (launch_pdl(rows, dim3(places, H), dim3(256), 0, stream, qn, kn, (const T*)vc, g, beta, cu_seqlens, num_seqs,
+                 reinterpret_cast<uint32_t*>(records), u0, out, G, H, D, Dv, shortest) != cudaSuccess)
+    return Q3_ERR_LAUNCH;
   // Not as a dependent launch: its blocks would start between the last blocks of the kernel before, two of the longest
-  // sequence's on some SMs while others have none (2048 tokens: the scan 278 us instead of 225).  No block for a one-token
-  // sequence either where num_long says so: with more blocks than SMs the first ones are no longer dealt out one to an SM
-  // (128 long blocks and 512 others: six SMs got two long ones; 16 heads, 2000 tokens beside 4 single ones: 496 us, so 435).
-  kernel<<<dim3((Dv + 15) / 16, H, num_long), dim3(256), smem, stream>>>(records, (const T*)vc, state, cu_seqlens,
-                                                                        state_slots, out, num_seqs, H, D, Dv, shortest);
+  // sequence's on some SMs while others have none.  No block for a one-token sequence either where num_long says so: with
+  // more blocks than SMs the first ones are no longer dealt out one to an SM (128 long blocks and 512 others: six SMs got two
+  // long ones).
+  scan<<<dim3((Dv + 15) / 16, H, num_long), dim3(4 * DP), smem, stream>>>(records, u0, state, cu_seqlens, state_slots, out,
+                                                                      num_seqs, H, D, Dv, shortest);
   return q3_launch_status();
 }
 
 // The same as q3_delta_scan for key sizes up to 128, in chunks.  num_long: num_seqs, or the number of sequences of two tokens
-// and more, which are then the only ones served; records: (num_tokens / 16 + num_seqs) * H * (49 * DP +
-// 512) floats with DP = 64 (D <= 64) or 128.
+// and more, which are then the only ones served; records: (num_tokens / 16 + num_seqs) * H * 73 * DP
+// words with DP = 64 (D <= 64) or 128; u0: scratch of the output's size.
 Q3_EXPORT int q3_delta_chunk_scan(int dtype, const float* qn, const float* kn, const void* vc, const float* g,
-                                  const float* beta, float* records, float* state, const int* cu_seqlens,
-                                  const int* state_slots, float* out, int num_tokens, int num_seqs, int num_long, int G,
+                                  const float* beta, float* records, float* u0, float* state,
+                                  const int* cu_seqlens, const int* state_slots, float* out, int num_tokens, int num_seqs, int num_long, int G,
                                   int H, int D, int Dv, cudaStream_t stream) {
-  if (!qn || !kn || !vc || !g || !beta || !records || !state || !cu_seqlens || !state_slots || !out) return Q3_ERR_ARGUMENT;
+  if (!qn || !kn || !vc || !g || !beta || !records || !u0 || !state || !cu_seqlens || !state_slots || !out) return Q3_ERR_ARGUMENT;
   if (G < 1 || H < 1 || H % G || D < 1 || Dv < 1 || H > 65535 || num_seqs > 65535 || num_long > num_seqs) return Q3_ERR_ARGUMENT;
   if (D > 128 || (dtype != Q3_DTYPE_F32 && dtype != Q3_DTYPE_BF16) || !ds_aligned(records)) return Q3_ERR_UNSUPPORTED;
   if (num_long < 1 || num_tokens == 0) return Q3_OK;
 #define Q3_DELTA_CHUNKS(T, DP)                                                                                       \
-  return launch_delta_chunks<T, DP>(stream, num_tokens, num_seqs, num_long, qn, kn, vc, g, beta, records, state, cu_seqlens,   \
-                                    state_slots, out, G, H, D, Dv)
+  return launch_delta_chunks<T, DP>(stream, num_tokens, num_seqs, num_long, qn, kn, vc, g, beta, records, u0, state,   \
+                                    cu_seqlens, state_slots, out, G, H, D, Dv)
   if (dtype == Q3_DTYPE_F32) {
     if (D <= 64) Q3_DELTA_CHUNKS(float, 64);
     Q3_DELTA_CHUNKS(float, 128);

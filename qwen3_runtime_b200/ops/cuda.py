@@ -143,7 +143,8 @@ _SIGNATURES = {
         "q3_delta_scan": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                           c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "q3_delta_chunk_scan": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                                c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
+                                c_void_p],
         "q3_delta_step": [c_int, c_void_p, c_long, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                           c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_float, c_void_p,
                           c_void_p, c_float, c_void_p, c_long, c_int, c_int, c_int, c_int, c_int, c_void_p],
@@ -978,11 +979,12 @@ class CudaOps:
             # prompts: chunks of 16 tokens (csrc/delta_state.cu); what does not depend on the state first
             num_long = self._delta_long(host_cu_seqlens, int(num_seqs), H, Dv)
             padded = 64 if D <= 64 else 128
-            records = torch.empty((T // 16 + num_seqs) * H * (49 * padded + 512), dtype=torch.float32, device=dev)
+            records = torch.empty((T // 16 + num_seqs) * H * 73 * padded, dtype=torch.float32, device=dev)
+            u0 = torch.empty_like(out)
             self.launches += 1
             self._call("delta_state", "q3_delta_chunk_scan", "delta_chunk_scan", _dtype_code(x.dtype), _ptr(qn), _ptr(kn),
-                       _ptr(vc), _ptr(g), _ptr(beta), _ptr(records), _ptr(state), _ptr(cu_seqlens), _ptr(state_slots),
-                       _ptr(out), T, int(num_seqs), num_long, G, H, D, Dv)
+                       _ptr(vc), _ptr(g), _ptr(beta), _ptr(records), _ptr(u0), _ptr(state), _ptr(cu_seqlens),
+                       _ptr(state_slots), _ptr(out), T, int(num_seqs), num_long, G, H, D, Dv)
             if num_long == num_seqs:
                 return out
             longest = 1
@@ -994,8 +996,8 @@ class CudaOps:
     def _delta_long(self, cu, num_seqs, H, Dv) -> int:
         """How many sequences of a step with prompts run in chunks: all, or those of two tokens and more.  Single tokens stay
         apart where the prompts' blocks would have an SM each, which is lost when other blocks are launched with them
-        (csrc/delta_state.cu), and the tokens are few: 16 heads, us together / apart: 2000 tokens beside 4 single ones 496 / 435,
-        beside 20 497 / 464, 1000 beside 40 290 / 298; 32 heads (two blocks an SM anyway) 2000 beside 4 675 / 699."""
+        (csrc/delta_state.cu), and the tokens are few: 16 heads, us together / apart: 2000 tokens beside 4 single ones 300 / 233,
+        beside 20 306 / 261, 1000 beside 40 181 / 196; 32 heads (two blocks an SM anyway) 2000 beside 4 389 / 400."""
         lens = [b - a for a, b in zip(cu, cu[1:])] if cu else []
         num_long = sum(n > 1 for n in lens)
         if num_long and num_long * H * -(-Dv // 16) <= self.SM_COUNT and max(lens) >= 40 * (num_seqs - num_long):
