@@ -14,34 +14,39 @@
 // every K/V tile.  PAGED and DENSE: A and B are consecutive blocks; MAPS: A and B are the two maps of the same rows.
 // Keys come in tiles of 64 (PAGED, MAPS: 64/page_size pages, one TMA box per page and 64 columns), and each tile is used
 // by both row blocks.  Per 64-key tile a row block's chain is long (TMEM load, exp2 on the special-function unit, TMEM
-// store, fences, barrier round trips) and leaves the tensor core and the exp2 unit idle most of the time; two blocks in
-// flight hide each other's chain.  Eleven warps:
-//   warp 0           : TMA producer (Q of both blocks once, then K and V tiles through rings of stages; the lanes issue a
-//                      tile's boxes side by side);
-//   warps 1 and 10,  : MMA issuers of block A and of block B.  Order per block: S_0, S_1, then
-//   one lane each      per tile j: P_j ready -> PV_j, PV_j done -> S_(j+2).  S has two TMEM buffers per block,
-//                      so the tensor core works for one block while the other block's softmax
-//                      runs;
-//   warps 2..5, 6..9 : softmax of block A and of block B, one thread per row: reads S from
-//                      TMEM, masks, online softmax in fp32 (exp2, scale folded in), writes P as bf16 over the first
-//                      32 columns of the S buffer that it came from, where the PV MMA reads it as its A operand; O stays
-//                      in TMEM (the MMAs accumulate into it) and is rescaled there only when a row's maximum has grown by
-//                      more than 2^8; finally stores O / l.  MAPS: block B's threads leave lambda O_B / l_B in shared
-//                      memory, block A's subtract it, divide by the root mean square and store.
-// Tensor memory: all 512 columns, per block S0 [0,64), S1 [64,128), O [128,256); P_j lies in S_j's columns.  S_(j+2) is
-// issued when PV_j is complete: PTX promises an order of MMAs in flight only where they have the same accumulator and
-// shape, which these two have not.  The wait costs nothing (2048 tokens, 32 heads over 8: 56.3 us with and without; 8192: 584 and
-// 583), since the softmax has S_(j+1) by then.
-// What bounds it: the chain of a tile and block (S ready, TMEM load, exp2, TMEM store, barrier round trips); the products are
-// busy about a third of the time.  P in tensor memory instead of shared memory took little off it: one layer of 2048 tokens, 32
-// heads over 8, 58.4 -> 56.3 us, 64 heads over 8 110.6 -> 107.5 (behind a cold L2).  Forms: differential attention, 16 heads over 4,
-// 2333 + 419 tokens: 61 us (mma.sync: 247); latent, 16 heads, 2048 tokens, window 1024: 34 us and 26 us for the expansion (in
-// the latent space on mma.sync: 481).
+// store, fences, barrier round trips) and leaves the tensor core and the exp2 unit idle for much of the time; two blocks in
+// flight hide each other's chain.  Sixteen warps:
+//   warps 0..3       : TMA producers, keys and values, 64 columns each, through rings of stages (the fourth one brings Q of
+//                      both blocks first);
+//   warps 4..7, 8..11: softmax of block A and of block B, one thread per row: reads S_j from TMEM and gives its place back at
+//                      once, masks, online softmax in fp32 (exp2, scale folded in), writes P_j as bf16 into one of two
+//                      buffers in TMEM, where the PV MMA reads it as its A operand; O stays in TMEM (the MMAs accumulate
+//                      into it) and is rescaled there only when a row's maximum has grown by more than 2^8; finally stores
+//                      O / l.  MAPS: block B's threads leave lambda O_B / l_B in shared memory, block A's subtract it, divide
+//                      by the root mean square and store;
+//   warps 12, 13     : MMA issuers of S for block A and B: S_(j+1) as soon as S_j is in registers;
+//   warps 14, 15     : MMA issuers of PV for block A and B: PV_j when P_j is written.
+// Tensor memory: all 512 columns, per block S [0,64), P_0 and P_1 [64,128), O [128,256).
+// What bounds it: the softmax warps, and behind them the products (S with 64 columns is bound by its reads of shared memory,
+// 45 cycles per 16 k-values) and the keys' and values' way from L2 (32 KB a step and SM).  A step of both blocks takes 1650
+// cycles where the exp2 unit alone needs 1024.  What counted was code, not arithmetic: 32 heads over 8, 8192 tokens, one layer,
+// us (2048 tokens: 48 -> 44):
+//   554  one issuer per block (PV_j before S_(j+2): its waits, commits and products took longer than the softmax of a tile), one
+//        producer, S twice and P over S
+//   550  S issued before PV by warps of their own, four producers
+//   512  tiles that all rows see as a whole without the masks' branches; waits with their slow part out of line
+//   457  the reference point moved without a branch, the rescaling out of line
+// Not kept: 128 keys a step (830: the chain of a block twice as long), turns of the two blocks at the exponentials (482),
+// S_(j+1) loaded beside the exponentials of tile j with 192 registers a thread (585), waits that try again without looking at
+// the clock (512 -> 562).  Forms: differential attention, 16 heads over 4, 2333 + 419 tokens 60 -> 54 us (mma.sync: 247);
+// latent, 16 heads, 2048 tokens, window 1024: 34 -> 31 us and 26 us for the expansion (in the latent space on mma.sync: 481).
 // V is the B operand of PV in MN-major form (rows = keys): descriptor with the halves of D
 // 8 KB apart (leading offset) and 8-key groups 1 KB apart (stride offset); 16 keys = 2 KB.
 // Keys past a block's last position are zeroed in shared memory before PV (stale or poisoned
 // page contents must not meet a zero probability).  Every mbarrier wait is bounded; on expiry
 // the block raises its abort flag and the global error word, frees TMEM and returns.
+#include <type_traits>
+
 #include "async_tiles.cuh"
 
 namespace {
@@ -50,12 +55,12 @@ enum { PAGED = 0, MAPS = 1, DENSE = 2 };
 constexpr int D = 128;  // value size, and query/key size of PAGED and of both maps together
 constexpr int BLOCK_M = 128;
 constexpr int BLOCK_N = 64;
-constexpr int THREADS = 352;
+constexpr int THREADS = 512;
 constexpr int HALF_Q = BLOCK_M * 128;           // 64 columns of a Q tile: [128 rows][128 B]
 constexpr int HALF_KV = BLOCK_N * 128;          // 64 columns of a K or V tile: [64 rows][128 B]
 constexpr int V_BYTES = 2 * HALF_KV;
-constexpr int TMEM_COLS = 512;                  // per row block: S0 [0,64), S1 [64,128), O [128,256)
-constexpr int TMEM_BLOCK = 256;
+constexpr int TMEM_COLS = 512;                  // per row block: S [0,64), P [64,128) (two buffers), O [128,256)
+constexpr int TMEM_BLOCK = 256, TMEM_P = 64, TMEM_O = 128;
 
 template <int MODE>
 struct Sizes {
@@ -92,6 +97,66 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// The warps that copy and multiply run as a whole, and only the instruction itself is one lane's: an arrival and its wait, there
+// and back between two warps, take 511 cycles between single lanes and 247 between whole warps.
+__device__ __forceinline__ void mma_ss(bool leader, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"((uint32_t)leader)
+      : "memory");
+}
+__device__ __forceinline__ void mma_ts(bool leader, uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"((uint32_t)leader)
+      : "memory");
+}
+__device__ __forceinline__ void commit(bool leader, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+      ::"r"(bar), "r"((uint32_t)leader)
+      : "memory");
+}
+
+// A wait that is one instruction and a branch that is not taken where the barrier is complete, or becomes so while the
+// instruction holds the warp; the rest is out of line.  (Branches are what the softmax warps stumble over.)
+__device__ __noinline__ bool wait_on(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return mbar_wait(bar, parity, abort_flag);
+}
+__device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  if (__builtin_expect(mbar_try_wait(bar, parity), 1)) return true;
+  return wait_on(bar, parity, abort_flag);
+}
+// a row's D accumulators in tensor memory times `corr`; rare, and out of line for the same reason
+__device__ __noinline__ void rescale_rows(uint32_t o_addr, float corr) {
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+  for (int c0 = 0; c0 < D; c0 += 32) {
+    uint32_t ov[32];
+    tmem_load32(o_addr + c0, ov);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int c = 0; c < 32; ++c) ov[c] = __float_as_uint(__uint_as_float(ov[c]) * corr);
+    tmem_store32(o_addr + c0, ov);
+  }
+}
+__device__ __forceinline__ void arrive_if(bool yes, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}"
+      ::"r"(bar), "r"((uint32_t)yes)
+      : "memory");
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, 1)
 prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -100,8 +165,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
   typedef Sizes<MODE> Z;
   constexpr int KV_STAGES = Z::STAGES, Q_BYTES = Z::Q_BYTES, K_BYTES = Z::K_BYTES, DK = Z::DK;
   enum { BAR_Q = 0, BAR_K_FULL = 1, BAR_K_EMPTY = BAR_K_FULL + KV_STAGES, BAR_V_FULL = BAR_K_EMPTY + KV_STAGES,
-         BAR_V_EMPTY = BAR_V_FULL + KV_STAGES, BAR_S_FULL = BAR_V_EMPTY + KV_STAGES,  // [block][buffer]
-         BAR_P_FULL = BAR_S_FULL + 4, BAR_PV_FULL = BAR_P_FULL + 2, NUM_BARS = BAR_PV_FULL + 2 };
+         BAR_V_EMPTY = BAR_V_FULL + KV_STAGES, BAR_S_FULL = BAR_V_EMPTY + KV_STAGES,  // [block], like the rest
+         BAR_S_EMPTY = BAR_S_FULL + 2, BAR_P_FULL = BAR_S_EMPTY + 2, BAR_PV_FULL = BAR_P_FULL + 2, NUM_BARS = BAR_PV_FULL + 2 };
   const int *block_table = p.block_table, *cu_seqlens = p.cu_seqlens;
   const int max_pages = p.max_pages, nq = p.nq, nkv = p.nkv, ps = p.ps, chunk = p.chunk, window = p.window;
   const float scale_log2 = p.scale_log2;
@@ -143,19 +208,20 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
     s_item[1] = rb;
     mbar_init(bar(BAR_Q), 1);
     for (int i = 0; i < KV_STAGES; ++i) {
-      mbar_init(bar(BAR_K_FULL + i), 1);
+      mbar_init(bar(BAR_K_FULL + i), 2);   // two producers
       mbar_init(bar(BAR_K_EMPTY + i), 2);  // both issuers
-      mbar_init(bar(BAR_V_FULL + i), 1);
+      mbar_init(bar(BAR_V_FULL + i), 2);
       mbar_init(bar(BAR_V_EMPTY + i), 2);
     }
-    for (int i = 0; i < 4; ++i) mbar_init(bar(BAR_S_FULL + i), 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(BAR_P_FULL + i), 128);
+      mbar_init(bar(BAR_S_FULL + i), 1);
+      mbar_init(bar(BAR_S_EMPTY + i), 4);  // a block's softmax warps
+      mbar_init(bar(BAR_P_FULL + i), 4);
       mbar_init(bar(BAR_PV_FULL + i), 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {
+  if (warp == 12) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_s)),
                  "r"(TMEM_COLS)
                  : "memory");
@@ -193,8 +259,10 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
     const int* bt = MODE == DENSE ? nullptr : block_table + (long)seq * max_pages;
     const int pages_per_tile = MODE == DENSE ? 0 : BLOCK_N / ps;
 
-    if (warp == 0) {  // ---- TMA producer: lane 0 waits and arms the barriers, the lanes share the loads ----
-      if (lane == 0) {
+    if (warp < 4) {  // ---- TMA producers: keys and values, 64 columns each ----
+      const int part = warp;  // keys: 0, 1; values: 2, 3
+      const int half = part & 1;
+      if (part == 3 && lane == 0) {
         constexpr int BOXES = MODE == MAPS ? 1 : DK / 64;  // of a block; MAPS: map x is columns 64 x .. of the head
         mbar_expect_tx(bar(BAR_Q), (tiles[1] ? 2 : 1) * BOXES * HALF_Q);
         for (int x = 0; x < 2; ++x) {
@@ -206,118 +274,110 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
           }
         }
       }
-      // PAGED, MAPS: a tile is 64 / ps pages x 2 halves of D, one box per lane (small boxes are slow to issue one after
-      // another from a single thread).  DENSE: five boxes of 64 rows (K: two of the head's own columns, one of the shared
-      // ones; V: two).
-      const int my_page = lane >> 1, my_half = lane & 1;
+      // PAGED, MAPS: a tile is 64 / ps pages, one box per page; each lane holds a page of the next tile.  DENSE: boxes of 64
+      // rows (keys: two of the head's own columns, one of the shared ones; the values lie beside the keys, behind those of all
+      // heads).
       const int row_base = MODE == DENSE ? p.kv_base[seq] : 0;
-      int ok = 1;
-      for (int j = 0; j < num_tiles && ok; ++j) {
-        const int st = j % KV_STAGES;
-        const uint32_t phase = (j / KV_STAGES) & 1;
-        uint32_t k_bytes = K_BYTES, v_bytes = V_BYTES, off = 0;
-        int page = -1, y = 0;
+      const uint32_t full = bar(part < 2 ? BAR_K_FULL : BAR_V_FULL), empty = bar(part < 2 ? BAR_K_EMPTY : BAR_V_EMPTY);
+      const uint32_t stage_bytes = part < 2 ? K_BYTES : V_BYTES;
+      const uint32_t dst0 = smem_addr(part < 2 ? k_s : v_s) + half * HALF_KV;
+      const CUtensorMap* map = MODE == DENSE || part < 2 ? &tmap_k : &tmap_v;
+      auto page_of = [&](int j) -> int {  // pages of tile j that exist in the block table (the rest of the tile is masked)
+        const int pi = (tile0 + j) * pages_per_tile + lane;
+        const bool in = lane < pages_per_tile && j < num_tiles && pi < max_pages && pi * ps <= p_last && (pi + 1) * ps > k_lo;
+        return in ? bt[pi] : -1;
+      };
+      int next = MODE == DENSE ? 0 : page_of(0);
+      int st = 0;
+      uint32_t phase = 1;
+      for (int j = 0; j < num_tiles; ++j) {
+        const int page = next;
+        const uint32_t dst = dst0 + st * stage_bytes;
+        uint32_t bytes = HALF_KV + (MODE == DENSE && part == 1 ? HALF_KV : 0);
+        if (MODE != DENSE) {
+          bytes = __popc(__ballot_sync(0xffffffffu, page >= 0)) * (uint32_t)ps * 128u;
+          next = page_of(j + 1);
+        }
+        if (!__all_sync(0xffffffffu, mbar_wait(empty + 8 * st, phase, &abort_flag))) break;
+        if (lane == 0) mbar_expect_tx(full + 8 * st, bytes);
         if (MODE == DENSE) {
-          y = row_base + (tile0 + j) * BLOCK_N;
+          if (lane == 0) {
+            const int y = row_base + (tile0 + j) * BLOCK_N;
+            tma_load_2d(dst, map, full + 8 * st, (part < 2 ? kvh : nkv + kvh) * D + half * 64, y);
+            if (part == 1) tma_load_2d(dst + HALF_KV, &tmap_v, full + 8 * st, 0, y);
+          }
         } else {
-          // pages of this tile that exist in the block table (the rest of the tile is masked)
-          if (my_page < pages_per_tile) {
-            const int pi = (tile0 + j) * pages_per_tile + my_page;
-            if (pi < max_pages && pi * ps <= p_last && (pi + 1) * ps > k_lo) page = bt[pi];
+          for (int u = 0; u < pages_per_tile; ++u) {
+            const int pg = __shfl_sync(0xffffffffu, page, u);
+            if (lane == 0 && pg >= 0) tma_load_2d(dst + u * ps * 128, map, full + 8 * st, half * 64, (pg * nkv + kvh) * ps);
           }
-          const uint32_t boxes = __popc(__ballot_sync(0xffffffffu, page >= 0));
-          k_bytes = v_bytes = boxes * (uint32_t)ps * 128u;
-          y = (page * nkv + kvh) * ps;
-          off = my_half * HALF_KV + my_page * ps * 128;
         }
-        // keys
-        if (lane == 0) {
-          ok = mbar_wait(bar(BAR_K_EMPTY + st), phase ^ 1, &abort_flag);
-          if (ok) mbar_expect_tx(bar(BAR_K_FULL + st), k_bytes);
-        }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (!ok) break;
-        const uint32_t k_dst = smem_addr(k_s) + st * K_BYTES, v_dst = smem_addr(v_s) + st * V_BYTES;
-        if (MODE == DENSE) {
-          if (lane < 2) tma_load_2d(k_dst + lane * HALF_KV, &tmap_k, bar(BAR_K_FULL + st), kvh * D + lane * 64, y);
-          if (lane == 2) tma_load_2d(k_dst + 2 * HALF_KV, &tmap_v, bar(BAR_K_FULL + st), 0, y);
-        } else if (page >= 0) {
-          tma_load_2d(k_dst + off, &tmap_k, bar(BAR_K_FULL + st), my_half * 64, y);
-        }
-        // values
-        if (lane == 0) {
-          ok = mbar_wait(bar(BAR_V_EMPTY + st), phase ^ 1, &abort_flag);
-          if (ok) mbar_expect_tx(bar(BAR_V_FULL + st), v_bytes);
-        }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (!ok) break;
-        if (MODE == DENSE) {  // the values lie beside the keys, behind those of all heads
-          if (lane < 2) tma_load_2d(v_dst + lane * HALF_KV, &tmap_k, bar(BAR_V_FULL + st), (nkv + kvh) * D + lane * 64, y);
-        } else if (page >= 0) {
-          tma_load_2d(v_dst + off, &tmap_v, bar(BAR_V_FULL + st), my_half * 64, y);
-        }
+        if (++st == KV_STAGES) st = 0, phase ^= 1;
       }
-    } else if (warp == 1 || warp == 10) {
-      if (lane == 0) {  // ---- MMA issuers: warp 1 for block A, warp 10 for block B ------------------
-        // Issuing is work too (descriptors, a dozen instructions per tile and block, barrier round
-        // trips), so each block has its own issuing thread.  Both use every K and V tile: its
-        // "empty" barrier counts two arrivals, a commit from an issuer that multiplied with the
+    } else if (warp > 11) {
+      {  // ---- MMA issuers: warps 12 and 13 for S of block A and B, warps 14 and 15 for PV ---------
+        // Issuing is work too (descriptors, barrier round trips of a hundred cycles each, a queue in front of the tensor
+        // core): one thread that issued both products of a block needed longer for a tile than the softmax.  Both blocks use
+        // every K and V tile: its "empty" barrier counts two arrivals, a commit from an issuer that multiplied with the
         // tile and a plain arrival (after the tile's "full") from one that had no use for it.
-        const int x = warp == 1 ? 0 : 1;
+        const int x = warp & 1;
+        const bool leader = lane == 0;
         const int my_tiles = tiles[x];
-        constexpr uint32_t idesc_s = umma_idesc(BLOCK_M, BLOCK_N, 0);   // S = Q K^T: N = 64 keys
-        constexpr uint32_t idesc_pv = umma_idesc(BLOCK_M, D, 1);        // PV: N = 128, V MN-major
-        const uint32_t q_addr = smem_addr(q_s) + x * Q_BYTES;
         const uint32_t tmem_x = tmem + x * TMEM_BLOCK;
-        // S_j into TMEM buffer j & 1, or just the hand-back of key tile j
-        auto keys = [&](int j) -> bool {
-          const int st = j % KV_STAGES, sbuf = j & 1;
-          if (!mbar_wait(bar(BAR_K_FULL + st), (j / KV_STAGES) & 1, &abort_flag)) return false;
-          if (j >= my_tiles) {
-            mbar_arrive(bar(BAR_K_EMPTY + st));
-            return true;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t k_addr = smem_addr(k_s) + st * K_BYTES;
-#pragma unroll
-          for (int k = 0; k < (MODE == MAPS ? 64 : DK) / 16; ++k) {
-            const uint32_t half = (k >> 2), sub = (k & 3) * 2;  // 4 steps of 32 bytes per 64 columns
-            umma_bf16(tmem_x + sbuf * BLOCK_N, umma_desc(q_addr + half * HALF_Q) + sub,
-                 umma_desc(k_addr + (MODE == MAPS ? x : half) * HALF_KV) + sub, idesc_s, k > 0 ? 1u : 0u);
-          }
-          umma_commit(bar(BAR_K_EMPTY + st));           // this block is done with the key tile
-          umma_commit(bar(BAR_S_FULL + 2 * x + sbuf));  // S_j is in TMEM
-          return true;
-        };
-        bool ok = my_tiles == 0 || mbar_wait(bar(BAR_Q), 0, &abort_flag);
-        for (int j = 0; j < 2 && j < num_tiles && ok; ++j) ok = keys(j);
-        for (int j = 0; j < num_tiles && ok; ++j) {
-          const int st = j % KV_STAGES, pbuf = j & 1;
-          if (j < my_tiles) {
-            ok = mbar_wait(bar(BAR_P_FULL + x), j & 1, &abort_flag);  // P_j written, S_j and PV_{j-1} consumed
+        if (warp < 14) {
+          constexpr uint32_t idesc = umma_idesc(BLOCK_M, BLOCK_N, 0);   // S = Q K^T: N = 64 keys
+          const uint32_t q_addr = smem_addr(q_s) + x * Q_BYTES;
+          bool ok = my_tiles == 0 || mbar_wait(bar(BAR_Q), 0, &abort_flag);
+          int st = 0;
+          uint32_t phase = 0;
+          for (int j = 0; j < num_tiles && ok; ++j) {
+            // S_j as soon as the softmax has S_(j-1) in its registers
+            if (j > 0 && j < my_tiles) ok = mbar_wait(bar(BAR_S_EMPTY + x), (j - 1) & 1, &abort_flag);
+            if (ok) ok = mbar_wait(bar(BAR_K_FULL + st), phase, &abort_flag);
             if (!ok) break;
-          }
-          ok = mbar_wait(bar(BAR_V_FULL + st), (j / KV_STAGES) & 1, &abort_flag);
-          if (!ok) break;
-          if (j < my_tiles) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t v_addr = smem_addr(v_s) + st * V_BYTES;
+            if (j < my_tiles) {
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              const uint32_t k_addr = smem_addr(k_s) + st * K_BYTES;
 #pragma unroll
-            for (int k = 0; k < BLOCK_N / 16; ++k)  // 16 keys: 8 columns of P, 2 KB down V's rows
-              umma_bf16_tmem(tmem_x + 2 * BLOCK_N, tmem_x + pbuf * BLOCK_N + 8 * k,
-                   umma_desc_mn_major(v_addr + k * 2048, HALF_KV), idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
-            umma_commit(bar(BAR_V_EMPTY + st));
-            umma_commit(bar(BAR_PV_FULL + x));
-          } else {
-            mbar_arrive(bar(BAR_V_EMPTY + st));
+              for (int k = 0; k < (MODE == MAPS ? 64 : DK) / 16; ++k) {
+                const uint32_t half = (k >> 2), sub = (k & 3) * 2;  // 4 steps of 32 bytes per 64 columns
+                mma_ss(leader, tmem_x, umma_desc(q_addr + half * HALF_Q) + sub,
+                     umma_desc(k_addr + (MODE == MAPS ? x : half) * HALF_KV) + sub, idesc, k > 0 ? 1u : 0u);
+              }
+              commit(leader, bar(BAR_S_FULL + x));    // S_j is in TMEM
+              commit(leader, bar(BAR_K_EMPTY + st));  // this block is done with the key tile
+            } else {
+              if (leader) mbar_arrive(bar(BAR_K_EMPTY + st));
+            }
+            if (++st == KV_STAGES) st = 0, phase ^= 1;
           }
-          // S_(j+2) goes where S_j and P_j were: PV_j must have read P_j
-          if (j + 2 < num_tiles)
-            ok = (j + 2 >= my_tiles || mbar_wait(bar(BAR_PV_FULL + x), j & 1, &abort_flag)) && keys(j + 2);
+        } else {
+          constexpr uint32_t idesc = umma_idesc(BLOCK_M, D, 1);        // PV: N = 128, V MN-major
+          bool ok = true;
+          int st = 0;
+          uint32_t phase = 0;
+          for (int j = 0; j < num_tiles && ok; ++j) {
+            if (j < my_tiles) ok = mbar_wait(bar(BAR_P_FULL + x), j & 1, &abort_flag);  // P_j written, O at rest
+            if (ok) ok = mbar_wait(bar(BAR_V_FULL + st), phase, &abort_flag);
+            if (!ok) break;
+            if (j < my_tiles) {
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              const uint32_t v_addr = smem_addr(v_s) + st * V_BYTES;
+#pragma unroll
+              for (int k = 0; k < BLOCK_N / 16; ++k)  // 16 keys: 8 columns of P, 2 KB down V's rows
+                mma_ts(leader, tmem_x + TMEM_O, tmem_x + TMEM_P + (j & 1) * (BLOCK_N / 2) + 8 * k,
+                     umma_desc_mn_major(v_addr + k * 2048, HALF_KV), idesc, (j > 0 || k > 0) ? 1u : 0u);
+              commit(leader, bar(BAR_PV_FULL + x));
+              commit(leader, bar(BAR_V_EMPTY + st));
+            } else {
+              if (leader) mbar_arrive(bar(BAR_V_EMPTY + st));
+            }
+            if (++st == KV_STAGES) st = 0, phase ^= 1;
+          }
         }
       }
     } else {  // ---- softmax: one thread per row; warps 2..5 block A, warps 6..9 block B ---------------
-      const int x = (warp - 2) >> 2;
+      const int x = (warp - 4) >> 2;
       const int quarter = warp & 3;
       const int r = quarter * 32 + lane;  // row of the tile = TMEM lane
       const int R = row0[x] + r;
@@ -327,40 +387,37 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
       const int lo = !row_ok ? 0 : (chunk > 0 ? pos / chunk * chunk : (window > 0 ? max(0, pos - window + 1) : 0));
       const int my_tiles = tiles[x];
       const uint32_t lane_base = tmem + x * TMEM_BLOCK + ((uint32_t)(quarter * 32) << 16);
-      const uint32_t o_addr = lane_base + 2 * BLOCK_N;
+      const uint32_t o_addr = lane_base + TMEM_O;
       // O stays in TMEM and the MMAs accumulate into it.  The reference point of the exponentials
       // (m_ref) is only moved when a row's maximum exceeds it by more than 2^8 after scaling; then
       // O and l are rescaled.  Probabilities may therefore reach 2^8, which bf16 and fp32 hold easily,
       // and the final O / l is unchanged.
-      const float slack = 8.f / scale_log2;
+      const float slack = fminf(8.f / scale_log2, 1e38f);
       float m_ref = -INFINITY, l_run = 0.f;
-      bool ok = true;
-      for (int j = 0; j < my_tiles && ok; ++j) {
-        const int st = j & 1;             // S buffer and P buffer of this tile
-        const int vst = j % KV_STAGES;    // its value tile
-        ok = mbar_wait(bar(BAR_S_FULL + 2 * x + st), (j >> 1) & 1, &abort_flag);
-        if (!ok) break;
+      const float2 scale2 = make_float2(scale_log2, scale_log2);
+      // One tile.  EDGE: some row of the block does not see all of its keys, or some of them lie outside of what the item reads;
+      // the others have no branch but the rare one for a new reference point, so that loads, maxima and exponentials
+      // are scheduled as one run of instructions.
+      auto step = [&](int j, auto edge) -> bool {
+        constexpr bool EDGE = decltype(edge)::value;
+        const int key0 = (tile0 + j) * BLOCK_N;
+        if (!wait(bar(BAR_S_FULL + x), j & 1, &abort_flag)) return false;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         uint32_t sa[32], sb[32];
-        tmem_load32(lane_base + st * BLOCK_N, sa);
-        tmem_load32(lane_base + st * BLOCK_N + 32, sb);
+        tmem_load32(lane_base, sa);
+        tmem_load32(lane_base + 32, sb);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        const int key0 = (tile0 + j) * BLOCK_N;
-        float mx = -INFINITY;
-        if (key0 + BLOCK_N - 1 > pos) {  // the tile crosses this row's diagonal
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        arrive_if(lane == 0, bar(BAR_S_EMPTY + x));  // S_(j+1) may come
+        if constexpr (EDGE) {
 #pragma unroll
           for (int c = 0; c < 32; ++c) {
-            if (key0 + c > pos) sa[c] = 0xff800000u;       // -inf
-            if (key0 + 32 + c > pos) sb[c] = 0xff800000u;
+            if (key0 + c > pos || key0 + c < lo) sa[c] = 0xff800000u;  // -inf
+            if (key0 + 32 + c > pos || key0 + 32 + c < lo) sb[c] = 0xff800000u;
           }
         }
-        if (key0 < lo) {  // keys of an earlier chunk, or before the window
-#pragma unroll
-          for (int c = 0; c < 32; ++c) {
-            if (key0 + c < lo) sa[c] = 0xff800000u;
-            if (key0 + 32 + c < lo) sb[c] = 0xff800000u;
-          }
-        }
+        float mx;
         {  // eight independent running maxima: a single chain of 64 would expose its latency
           float part[8];
 #pragma unroll
@@ -371,74 +428,83 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
           mx = fmaxf(fmaxf(fmaxf(part[0], part[1]), fmaxf(part[2], part[3])),
                      fmaxf(fmaxf(part[4], part[5]), fmaxf(part[6], part[7])));
         }
-        float corr = 1.f;
-        if (mx > m_ref + slack || (m_ref == -INFINITY && mx > -INFINITY)) {
-          corr = m_ref == -INFINITY ? 0.f : exp2f((m_ref - mx) * scale_log2);
-          m_ref = mx;
-        }
-        const bool rescale = __any_sync(0xffffffffu, corr != 1.f) && j > 0;
+        const float m_old = m_ref;
+        m_ref = mx > m_ref + slack ? mx : m_ref;  // (also from -infinity)
+        const bool moved = __any_sync(0xffffffffu, m_ref != m_old);
         const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
-        // probabilities, rounded to bf16 as the MMA will see them, over the scores in tensor memory; the
-        // scaling and the row sum run on pairs of elements (packed fp32 instructions)
+        // probabilities, rounded to bf16 as the MMA will see them, into tensor memory; the scaling and the row sum run on
+        // pairs of elements (packed fp32 instructions)
         float2 sums[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
         uint32_t w[32];
-        const float2 scale2 = make_float2(scale_log2, scale_log2);
         const float2 neg2 = make_float2(-m_use * scale_log2, -m_use * scale_log2);
 #pragma unroll
         for (int ch = 0; ch < 8; ++ch) {
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int c = ch * 8 + 2 * e;
-            const float2 s2 = make_float2(__uint_as_float(c < 32 ? sa[c] : sb[c - 32]),
-                                          __uint_as_float(c + 1 < 32 ? sa[c + 1] : sb[c + 1 - 32]));
+            const float2 s2 = make_float2(__uint_as_float(c < 32 ? sa[c & 31] : sb[c & 31]),
+                                          __uint_as_float(c < 32 ? sa[(c + 1) & 31] : sb[(c + 1) & 31]));
             const float2 t2 = __ffma2_rn(s2, scale2, neg2);
             const float2 x2 = make_float2(ex2(t2.x), ex2(t2.y));
             sums[e] = __fadd2_rn(sums[e], x2);
             w[ch * 4 + e] = pack2(x2.x, x2.y);
           }
         }
-        tmem_store32(lane_base + st * BLOCK_N, w);
+        tmem_store32(lane_base + TMEM_P + (j & 1) * (BLOCK_N / 2), w);
         {
           const float2 a = __fadd2_rn(sums[0], sums[1]), b = __fadd2_rn(sums[2], sums[3]);
           const float2 c = __fadd2_rn(a, b);
+          const float corr = m_ref == m_old ? 1.f : exp2f((m_old - m_ref) * scale_log2);  // 0 from -infinity
           l_run = l_run * corr + (c.x + c.y);
         }
-        // PV_{j-1} must be finished before P_j is signalled: it keeps this barrier from running a
-        // phase ahead of the waiters, and O must be at rest if it has to be rescaled
-        if (j > 0) {
-          ok = mbar_wait(bar(BAR_PV_FULL + x), (j - 1) & 1, &abort_flag);
-          if (!ok) break;
-          if (rescale) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll 1
-            for (int c0 = 0; c0 < D; c0 += 32) {
-              uint32_t ov[32];
-              tmem_load32(o_addr + c0, ov);
-              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-              for (int c = 0; c < 32; ++c) ov[c] = __float_as_uint(__uint_as_float(ov[c]) * corr);
-              tmem_store32(o_addr + c0, ov);
-            }
+        // PV_(j-1) must be finished before P_j is signalled: it keeps this barrier from running a phase ahead of the waiters,
+        // P_(j+1) goes where P_(j-1) was, and O must be at rest if it has to be rescaled
+        if (!EDGE || j > 0) {
+          if (!wait(bar(BAR_PV_FULL + x), (j - 1) & 1, &abort_flag)) return false;
+          if (__builtin_expect(moved, 0)) {
+            rescale_rows(o_addr, m_ref == m_old ? 1.f : exp2f((m_old - m_ref) * scale_log2));
           }
         }
         // keys of this tile past the item's last position hold whatever the page held, keys before its first
         // visible one may not have been loaded at all: zero their value rows before PV reads them (both blocks
         // do, each before its own PV; keys between the blocks' last positions are real and only masked)
-        if (key0 + BLOCK_N - 1 > p_last || key0 < k_lo) {
-          ok = mbar_wait(bar(BAR_V_FULL + vst), (j / KV_STAGES) & 1, &abort_flag);
-          if (!ok) break;
-          const int vrow = r & 63, half = r >> 6;
-          if (key0 + vrow > p_last || key0 + vrow < k_lo) {
-            uint4* dst = reinterpret_cast<uint4*>(v_s + vst * V_BYTES + half * HALF_KV + vrow * 128);
+        if constexpr (EDGE) {
+          if (key0 + BLOCK_N - 1 > p_last || key0 < k_lo) {
+            const int vst = j % KV_STAGES;
+            if (!wait(bar(BAR_V_FULL + vst), (j / KV_STAGES) & 1, &abort_flag)) return false;
+            const int vrow = r & 63, half = r >> 6;
+            if (key0 + vrow > p_last || key0 + vrow < k_lo) {
+              uint4* dst = reinterpret_cast<uint4*>(v_s + vst * V_BYTES + half * HALF_KV + vrow * 128);
 #pragma unroll
-            for (int ch = 0; ch < 8; ++ch) dst[ch] = make_uint4(0, 0, 0, 0);
+              for (int ch = 0; ch < 8; ++ch) dst[ch] = make_uint4(0, 0, 0, 0);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // zeroed V visible to the MMA
           }
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // zeroed V visible to the MMA
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        mbar_arrive(bar(BAR_P_FULL + x));
+        __syncwarp();
+        arrive_if(lane == 0, bar(BAR_P_FULL + x));
+        return true;
+      };
+      // tiles that every row of the block sees as a whole: from the last row's first key on, up to the first row's position
+      const int row_first = row0[x], row_last = min(rows, row0[x] + BLOCK_M) - 1;
+      const int pos_first = base_pos + row_first / G, pos_last = base_pos + row_last / G;
+      const int lo_last = chunk > 0 ? pos_last / chunk * chunk : (window > 0 ? max(0, pos_last - window + 1) : 0);
+      int whole0 = 1, whole1 = 0;  // such tiles behind the first one
+      if (row0[x] + BLOCK_M <= rows) {  // (rows that are none see nothing)
+        whole0 = max(1, (max(lo_last, k_lo) + BLOCK_N - 1) / BLOCK_N - tile0);
+        whole1 = min(my_tiles, (pos_first + 1) / BLOCK_N - tile0);
       }
-      if (ok && my_tiles) ok = mbar_wait(bar(BAR_PV_FULL + x), (my_tiles - 1) & 1, &abort_flag);
+      bool ok = true;
+      for (int j = 0; j < my_tiles && ok; ++j) {
+        if (j < whole0 || j >= whole1) {
+          ok = step(j, std::true_type());
+        } else {
+          while (step(j, std::false_type()) && ++j < whole1) {}
+          ok = j-- == whole1;
+        }
+      }
+      if (ok && my_tiles) ok = wait(bar(BAR_PV_FULL + x), (my_tiles - 1) & 1, &abort_flag);
       __syncwarp();
       if constexpr (MODE == MAPS) {
         // out = o / sqrt(mean(o^2) + eps) * out_scale, o = O_A / l_A - lambda O_B / l_B.  A row's 128 values pass from
@@ -544,7 +610,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 1) {
+  if (warp == 12) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
   }
