@@ -1,5 +1,5 @@
 // C[M, N] = A[M, K] * W[N, K]^T in true fp32 on the FMA pipes: no tensor cores, no
-// TF32.  Every output element is one accumulator that takes its K products in
+// TF32 (large weights: gemm_f32_split.cuh, on the tensor cores in three bfloat16 parts).  Every output element is one accumulator that takes its K products in
 // ascending k order, so a row of C does not depend on M, on the tile shape chosen
 // for M, or on where the row sits in the batch.  This is the matrix product of the
 // engine's 32-bit path (the reference's fp32 path is torch on the CPU,
@@ -16,6 +16,7 @@
 // 696 us at 300 x 2560 -> 19456), and tiles of 128 rows or columns are nowhere the fastest.  Since K may not be cut, an
 // output too small for large tiles gets smaller ones (SHAPES).
 #include "common.cuh"
+#include "gemm_f32_split.cuh"
 
 #include <stdint.h>
 

@@ -1,0 +1,427 @@
+// C[M, N] = A[M, K] * W[N, K]^T of float32 matrices on the tensor cores, every operand as the sum of three bfloat16 (8 + 8 + 8
+// bits: nothing is lost) and the six products of parts that matter; the other three are below 2^-26 of a product.
+//
+// The accumulators of tcgen05.mma round towards zero at every step (products of 2560 values: 2.7e-6 off, 7e-6 if all are
+// positive; one chain of fp32 FMA 4.5e-7), so a chain is never longer than a slice of 64 k-values: its 20 small products first,
+// which cost no digits of the sum, then the 4 large ones; the slice's result is added to fp32 registers, rounded to nearest, in
+// ascending k.  K may be cut into segments, whose sums are added in order by a second kernel; how many depends on N and K
+// only.  So a row of C does not depend on M, on the tile chosen for M, or on where the row sits in the batch, and lies nearer to
+// the exact product than the FMA chain (split_matrix and the kernel below; K from 1024: see the dispatch).
+//
+// Weights are the 128 rows of an MMA, tokens its 16 to 160 columns.  Roles of a block (one per SM, persistent over items of
+// (128 weight rows, segment, token tile), token tiles of the same weights side by side):
+//   warp 0       TMA: the tokens' three parts (made beforehand by split_matrix) of a slice, one box of 64 columns per part
+//   warp 1       MMA issuer
+//   warps 2..9   weights: 16 bytes of float32 per lane from global memory, a slice ahead in registers, split and written in the
+//                128-byte swizzle; and sums: the accumulators of the slice before (two buffers in tensor memory) into
+//                registers, a row and half of the columns a thread; at the item's end they are stored
+// What bounds it: a slice takes 1900 cycles with few tokens, the weights' way (wait, split, write, the products' hand-over), and
+// 2700 with 160, with the sums' beside it; its 24 products take 900 to 1900 of them.  300 tokens: 19456 x 2560 704 us on the FMA
+// pipes, 236 here; 2560 x 9728 415 and 120.
+#include "async_tiles.cuh"
+
+namespace split {
+
+constexpr int ROWS = 128, SLICE = 64, MOST_TOKENS = 160, THREADS = 10 * 32;
+constexpr int AHEAD = 4;  // slices
+constexpr int W_PART = ROWS * 128, W_STAGE = 3 * W_PART;
+constexpr int smem_bytes(int tokens) { return 2 * (W_STAGE + 3 * tokens * 128) + 1024; }
+enum { BAR_W_FULL = 0, BAR_X_FULL = 2, BAR_EMPTY = 4, BAR_D_FULL = 6, BAR_D_EMPTY = 8, BAR_END = 10, NUM_BARS = 11 };
+
+// (x, y) as the sum of three pairs of bfloat16
+__device__ __forceinline__ void parts_of(float x, float y, uint32_t (&p)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p[i]) : "f"(y), "f"(x));
+    x -= __uint_as_float(p[i] << 16);
+    y -= __uint_as_float(p[i] & 0xffff0000u);
+  }
+}
+
+// x [M, K], rows ldx apart, as three dense bfloat16 matrices one behind the other; K a multiple of 8
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+split_matrix(const float* __restrict__ x, long ldx, uint4* __restrict__ to, int M, int K) {
+  const long at = (long)blockIdx.x * 256 + threadIdx.x, per_row = K / 8;
+  if (at >= M * per_row) return;
+  const long m = at / per_row;
+  const float* src = x + m * ldx + (at - m * per_row) * 8;
+  float v[8];
+  if (VEC) {
+    load8(src, v);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = src[i];
+  }
+  uint32_t p[4][3];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) parts_of(v[2 * i], v[2 * i + 1], p[i]);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) to[i * M * per_row + at] = make_uint4(p[0][i], p[1][i], p[2][i], p[3][i]);
+}
+
+struct Args {
+  const float *a, *w;  // the float32 operands
+  long lda, ldw;
+  float* out;          // [segments][M][ldc]
+  long ldc, plane;
+  int M, N, K, segments, slices_per_segment, tokens, token_tiles, items;
+  int* error_word;
+};
+
+__device__ __forceinline__ void tmem_load8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+}
+
+// Parts of infinities, and of what rounds up to one, have no sum: such results once more, as float32 gives them.  (Out of line:
+// eighty copies of it behind the sums took 15 us an item to be fetched and jumped over.)
+__device__ __noinline__ void as_float32(const Args& p, float* dst, int row, int t0, int tokens, int k0, int k1) {
+  for (int i = 0; i < tokens; ++i) {
+    const float y = dst[(long)i * p.ldc];
+    if (y == y) continue;
+    const float *a = p.a + (long)(t0 + i) * p.lda, *w = p.w + (long)row * p.ldw;
+    float sum = 0.f;
+    for (int k = k0; k < k1; ++k) sum = fmaf(a[k], w[k], sum);
+    dst[(long)i * p.ldc] = sum;
+  }
+}
+
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_f32_split_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ Args p) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const uint32_t x_part = (uint32_t)p.tokens * 128, x_stage = 3 * x_part;
+  unsigned char* w_s = base;                       // 2 x [3 parts][128 rows][128 B]
+  const uint32_t x_s = smem_addr(base + 2 * W_STAGE);  // 2 x [3 parts][tokens][128 B]
+  __shared__ __align__(8) unsigned long long bars[NUM_BARS];
+  __shared__ uint32_t tmem_base_s;
+  __shared__ volatile int abort_flag;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t bar0 = smem_addr(&bars[0]);
+  auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
+  if (tid == 0) {
+    abort_flag = 0;
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar(BAR_W_FULL + i), 8);   // the weights' warps
+      mbar_init(bar(BAR_X_FULL + i), 1);
+      mbar_init(bar(BAR_EMPTY + i), 1);
+      mbar_init(bar(BAR_D_FULL + i), 1);
+      mbar_init(bar(BAR_D_EMPTY + i), 8);  // the sums' warps
+    }
+    mbar_init(bar(BAR_END), 1);
+    mbar_init_fence();
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_addr(&tmem_base_s)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_base_s;
+  const int slices = (p.K + SLICE - 1) / SLICE;
+  struct Item {
+    int row0, token0, segment, first, count;  // slices first .. first + count - 1
+  };
+  auto item_at = [&](int i) {
+    Item it;
+    const int rest = i / p.token_tiles;
+    it.token0 = (i - rest * p.token_tiles) * p.tokens;
+    const int tile = rest / p.segments;
+    it.segment = rest - tile * p.segments;
+    it.row0 = tile * ROWS;
+    it.first = it.segment * p.slices_per_segment;
+    it.count = min(p.slices_per_segment, slices - it.first);
+    return it;
+  };
+
+  const int warp_u = __shfl_sync(0xffffffffu, warp, 0);
+  if (warp == 0) {  // ---- the tokens' parts ----
+    int s = 0;
+    bool ok = true;
+    for (int i = blockIdx.x; i < p.items && ok; i += gridDim.x) {
+      const Item it = item_at(i);
+      for (int c = 0; c < it.count && ok; ++c, ++s) {
+        const int st = s & 1;
+        ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_EMPTY + st), ((s >> 1) & 1) ^ 1, &abort_flag));
+        if (ok && lane == 0) {
+          mbar_expect_tx(bar(BAR_X_FULL + st), x_stage);
+          for (int q = 0; q < 3; ++q)
+            tma_load_3d(x_s + st * x_stage + q * x_part, &xmap, bar(BAR_X_FULL + st), (it.first + c) * SLICE, it.token0, q);
+        }
+      }
+    }
+    // after a wait that expired: the boxes in flight
+    if (!ok && lane == 0)
+      for (int b = max(0, s - 3); b < s - 1; ++b) mbar_wait_drain(bar(BAR_X_FULL + (b & 1)), (b >> 1) & 1);
+  } else if (warp_u == 1) {  // ---- products ----
+    // (one lane chosen by elect.sync, in a warp that runs as a whole: descriptors then stay in uniform registers, and an MMA is
+    // issued every 37 cycles; chosen by its number 60 to 78)
+    const bool leader = elect_one();
+    const uint32_t idesc = umma_idesc(ROWS, p.tokens);
+    const uint32_t w_addr = smem_addr(w_s), tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
+    int s = 0;
+    bool ok = true;
+    for (int i = blockIdx.x; i < p.items && ok; i += gridDim.x) {
+      const int count = item_at(i).count;
+      for (int c = 0; c < count; ++c, ++s) {
+        const int st = s & 1;
+        const uint32_t phase = (s >> 1) & 1;
+        // (the three at once: one after the other they would cost three times the wait's latency)
+        const bool d = mbar_try_wait(bar(BAR_D_EMPTY + st), phase ^ 1), w = mbar_try_wait(bar(BAR_W_FULL + st), phase),
+                   t = mbar_try_wait(bar(BAR_X_FULL + st), phase);
+        if (!__all_sync(0xffffffffu, d & w & t))
+          ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_D_EMPTY + st), phase ^ 1, &abort_flag) &&
+                                           mbar_wait(bar(BAR_W_FULL + st), phase, &abort_flag) &&
+                                           mbar_wait(bar(BAR_X_FULL + st), phase, &abort_flag));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint64_t wd = umma_desc(w_addr + st * W_STAGE), xd = umma_desc(x_s + st * x_stage);
+        const uint32_t acc = tmem_u + st * 256, xp = x_part >> 4;
+        if (leader) {
+          auto product = [&](int wq, int xq, bool first) {  // 16 k-values are 32 bytes: 2 descriptor units
+#pragma unroll
+            for (int k = 0; k < SLICE / 16; ++k)
+              umma_bf16(acc, wd + wq * (W_PART >> 4) + 2 * k, xd + xq * xp + 2 * k, idesc, first && k == 0 ? 0u : 1u);
+          };
+          product(2, 0, true);
+          product(0, 2, false);
+          product(1, 1, false);
+          product(1, 0, false);
+          product(0, 1, false);
+          product(0, 0, false);
+          umma_commit(bar(BAR_EMPTY + st));
+          umma_commit(bar(BAR_D_FULL + st));
+        }
+        __syncwarp();
+      }
+    }
+    if (leader) {  // nothing of this block's is in flight any more when the tensor memory is freed
+      umma_commit(bar(BAR_END));
+      mbar_wait_drain(bar(BAR_END), 0);
+    }
+    __syncwarp();
+  } else {  // ---- weights and sums ----
+    const int worker = warp - 2, quarter = warp & 3, cols = p.tokens / 2, col0 = (worker >> 2) * cols;
+    const uint32_t from = tmem + ((uint32_t)(quarter * 32) << 16) + col0;
+    const int r0 = worker * 16 + (lane >> 4), kl = (lane & 15) * 4;
+    unsigned char* const w_dst = w_s + r0 * 128 + (lane & 1) * 8;
+    float4 v[8];  // rows r0 + 2 i, k-values kl .. kl + 3 of the slice that is split next
+    const float* w_row = p.w;  // the first of those rows
+    int rows_left = 0;         // (rows from N on are read as that row, and not stored)
+    auto item_rows = [&](const Item& it) {
+      w_row = p.w + (long)min(it.row0 + r0, p.N - 1) * p.ldw + kl;
+      rows_left = p.N - it.row0 - r0;
+    };
+    auto load = [&](int slice) {
+      const float* src = w_row + slice * SLICE;
+      const bool in = slice * SLICE + kl < p.K;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        v[i] = in ? __ldg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (2 * i + 2 < rows_left) src += 2 * p.ldw;
+      }
+    };
+    // Into L2 ahead of the loads: a slice is 128 rows of two lines, one a thread.
+    auto ahead = [&](const Item& it, int slice) {
+      const int row = it.row0 + (tid - 64 >> 1), k = slice * SLICE + (tid & 1) * 32;
+      if (row < p.N && k < p.K) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w + (long)row * p.ldw + k));
+    };
+    float sum[MOST_TOKENS / 2];
+    auto add = [&](int s) -> bool {  // the accumulators of stage s
+      const int st = s & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait(bar(BAR_D_FULL + st), (s >> 1) & 1, &abort_flag))) return false;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int g = 0; g < MOST_TOKENS / 2; g += 16) {
+        if (g < cols) {
+          uint32_t r[2][8];
+          tmem_load8(from + st * 256 + g, r[0]);
+          if (g + 8 < cols) tmem_load8(from + st * 256 + g + 8, r[1]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int e = 0; e < 8; ++e) sum[g + e] += __uint_as_float(r[0][e]);
+          if (g + 8 < cols) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) sum[g + 8 + e] += __uint_as_float(r[1][e]);
+          }
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(BAR_D_EMPTY + st));
+      return true;
+    };
+    if ((int)blockIdx.x < p.items) {
+      const Item it = item_at(blockIdx.x);
+      item_rows(it);
+      load(it.first);
+      for (int c = 1; c < AHEAD && c < it.count; ++c) ahead(it, it.first + c);
+    }
+    int s = 0;
+    bool ok = true;
+    for (int x = blockIdx.x; x < p.items && ok; x += gridDim.x) {
+      const Item it = item_at(x);
+      const int after = x + (int)gridDim.x;
+      const Item nx = item_at(after < p.items ? after : x);
+#pragma unroll
+      for (int i = 0; i < MOST_TOKENS / 2; ++i) sum[i] = 0.f;
+      for (int c = 0; c < it.count && ok; ++c, ++s) {
+        const int st = s & 1;
+        ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_EMPTY + st), ((s >> 1) & 1) ^ 1, &abort_flag));
+        if (!ok) break;
+        unsigned char* dst = w_dst + st * W_STAGE;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          uint32_t lo[3], hi[3];
+          parts_of(v[i].x, v[i].y, lo);
+          parts_of(v[i].z, v[i].w, hi);
+          const int at = i * 256 + ((((lane & 15) >> 1) ^ ((r0 + 2 * i) & 7)) * 16);
+#pragma unroll
+          for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(dst + q * W_PART + at) = make_uint2(lo[q], hi[q]);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(BAR_W_FULL + st));
+        if (c + 1 < it.count) {
+          load(it.first + c + 1);
+        } else if (after < p.items) {
+          item_rows(nx);
+          load(nx.first);
+        }
+        if (c + AHEAD < it.count) ahead(it, it.first + c + AHEAD);
+        else if (after < p.items && c + AHEAD - it.count < nx.count) ahead(nx, nx.first + c + AHEAD - it.count);
+        if (c > 0) ok = add(s - 1);  // while this slice's products run
+      }
+      if (ok) ok = add(s - 1);
+      if (!ok) break;
+      const int row = it.row0 + quarter * 32 + lane, t0 = it.token0 + col0;
+      if (row < p.N) {
+        float* dst = p.out + it.segment * p.plane + (long)t0 * p.ldc + row;
+        bool none = false;
+#pragma unroll
+        for (int i = 0; i < MOST_TOKENS / 2; ++i) {
+          if (i < cols && t0 + i < p.M) {
+            dst[(long)i * p.ldc] = sum[i];
+            none |= sum[i] != sum[i];
+          }
+        }
+        if (none) as_float32(p, dst, row, t0, min(cols, p.M - t0), it.first * SLICE, min(p.K, (it.first + it.count) * SLICE));
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+  }
+  if (tid == 0 && abort_flag && p.error_word) atomicExch(p.error_word, 2);
+}
+
+// the segments' sums, in order
+__global__ void __launch_bounds__(256)
+add_segments(const float* __restrict__ planes, long plane, int segments, float* __restrict__ out, long ldc, int M, int N) {
+  const long at = ((long)blockIdx.x * 256 + threadIdx.x) * 4;
+  const long m = at / N, n = at - m * N;
+  if (m >= M) return;
+  float4 sum = *reinterpret_cast<const float4*>(planes + at);
+  for (int s = 1; s < segments; ++s) {
+    const float4 v = *reinterpret_cast<const float4*>(planes + s * plane + at);
+    sum.x += v.x;
+    sum.y += v.y;
+    sum.z += v.z;
+    sum.w += v.w;
+  }
+  float* dst = out + m * ldc + n;
+  dst[0] = sum.x;
+  dst[1] = sum.y;
+  dst[2] = sum.z;
+  dst[3] = sum.w;
+}
+
+// Segments of K for N features: the fewest slices one after another on 148 SMs at one token tile, against the sums that every
+// segment writes and a second kernel reads.  300 tokens / one, us, with 1, 2, 3, 4, 6, 8 segments (the choice behind the sizes):
+// 19456 x 2560 (2) 249/120, 236/105, 241/103, 253/101, 284/105, 300/107; 24576 x 4096 (3) 398/179, 425/154, 400/146, 431/161,
+// 464/159, 490/166; 4096 x 12288 (4) 286/241, 212/136, 232/101, 220/83, 230/105, 238/89; 2560 x 9728 (7: 120/52) 222/194,
+// 144/112, 124/81, 151/68, 134/54, 146/71.  Of N and K only, whatever the device: the bits depend on it.
+static inline int segments_of(int N, int K) {
+  const int tiles = (N + ROWS - 1) / ROWS, slices = (K + SLICE - 1) / SLICE;
+  int best = 1, best_cost = 0;
+  for (int n = 1; n <= 8 && (n == 1 || n <= slices / 8); ++n) {
+    const int cost = 25 * ((tiles * n + 147) / 148) * ((slices + n - 1) / n) + n * tiles;
+    if (n == 1 || cost < best_cost) best = n, best_cost = cost;
+  }
+  return best;
+}
+
+}  // namespace split
+
+// Segments the product's K is cut into; 0: not a product for this kernel.  The tokens must have no say in it, so the line is
+// where few tokens do not lose: weights of 20 M values (one token, us, here / FMA: 2560 x 9728 52 / 89, 4096 x 12288 83 / 112,
+// 19456 x 2560 105 / 85, 24576 x 4096 146 / 132, hence 157 / 174 and 229 / 244 for a feed-forward; 6144 x 2560 60 / 38).
+Q3_EXPORT int q3_gemm_f32_split_segments(int N, int K) {
+  return N < 256 || N % 4 || K < 1024 || K % 8 || (long)N * K < 20000000 ? 0 : split::segments_of(N, K);
+}
+
+// As q3_gemm_f32.  parts: scratch of 3 * M * K bfloat16; planes: scratch of segments * M * N floats where there is more than one
+// segment.  W: rows at 16-byte boundaries.  error_word: device int set to 2 if a wait inside the kernel expired.
+Q3_EXPORT int q3_gemm_f32_split(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int M, int N, int K,
+                                void* parts, float* planes, int* error_word, cudaStream_t stream) {
+  using namespace split;
+  const int segments = q3_gemm_f32_split_segments(N, K);
+  if (!A || !W || !C || !parts || !error_word || lda < K || ldw < K || ldc < N || segments < 1 || (segments > 1 && !planes))
+    return Q3_ERR_ARGUMENT;
+  if (ldw % 4 || ((uintptr_t)W & 15) || ((uintptr_t)parts & 15) || ((uintptr_t)planes & 15)) return Q3_ERR_UNSUPPORTED;
+  if (M == 0) return Q3_OK;
+  static int sms_on[Q3_MAX_DEVICES];
+  const int device = q3_current_device();
+  if (!sms_on[device]) {
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+        cudaFuncSetAttribute(gemm_f32_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(MOST_TOKENS)) !=
+            cudaSuccess)
+      return Q3_ERR_LAUNCH;
+    sms_on[device] = sms;
+  }
+  const int sms = sms_on[device];
+  const long work = (long)M * (K / 8);
+  const unsigned blocks = (unsigned)((work + 255) / 256);
+  if (lda % 4 == 0 && ((uintptr_t)A & 15) == 0)
+    split_matrix<true><<<blocks, 256, 0, stream>>>(A, lda, (uint4*)parts, M, K);
+  else
+    split_matrix<false><<<blocks, 256, 0, stream>>>(A, lda, (uint4*)parts, M, K);
+  // The token tile: rounds over the SMs times a slice's time, which is that of shared memory (a token's parts are read by 24
+  // products and written once, the weights' read and written) or of the weights' bytes.
+  const int tiles = (N + ROWS - 1) / ROWS;
+  int best = 0;
+  double best_cost = 0;
+  for (int n = (M + MOST_TOKENS - 1) / MOST_TOKENS, tries = 0; tries < 4; ++n, ++tries) {
+    const int t = ((M + n - 1) / n + 15) / 16 * 16;
+    const long items = (long)tiles * segments * ((M + t - 1) / t);
+    const double slice = 24 * (4096 + 32 * t) + W_STAGE + 384 * t;
+    const double cost = (double)((items + sms - 1) / sms) * (slice < 180000 ? 180000 : slice);
+    if (!best || cost < best_cost) best = t, best_cost = cost;
+  }
+  Args p = {A, W, lda, ldw, segments > 1 ? planes : C, segments > 1 ? N : ldc, (long)M * N, M, N, K, segments, 0, best, 0, 0, error_word};
+  const int slices = (K + SLICE - 1) / SLICE;
+  p.slices_per_segment = (slices + segments - 1) / segments;
+  p.token_tiles = (M + best - 1) / best;
+  p.items = tiles * segments * p.token_tiles;
+  CUtensorMap map;
+  Q3EncodeTiledFn encode = q3_encode_tiled();
+  if (!encode) return Q3_ERR_LAUNCH;
+  const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)M, 3};
+  const cuuint64_t strides[2] = {(cuuint64_t)K * 2, (cuuint64_t)M * K * 2};
+  const cuuint32_t box[3] = {SLICE, (cuuint32_t)best, 1}, es[3] = {1, 1, 1};
+  if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, parts, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return Q3_ERR_LAUNCH;
+  const int grid = p.items < sms ? p.items : sms;
+  gemm_f32_split_kernel<<<grid, THREADS, smem_bytes(best), stream>>>(map, p);
+  if (segments > 1)
+    add_segments<<<(unsigned)(((long)M * N / 4 + 255) / 256), 256, 0, stream>>>(planes, (long)M * N, segments, C, ldc, M, N);
+  return q3_launch_status();
+}

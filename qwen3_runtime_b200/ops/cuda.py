@@ -235,6 +235,9 @@ _SIGNATURES = {
     },
     "gemm_f32": {
         "q3_gemm_f32": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
+        "q3_gemm_f32_split_segments": [c_int, c_int],
+        "q3_gemm_f32_split": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
+                              c_void_p, c_void_p],
     },
     "gemm_small_m": {
         "q3_gemm_small_m": [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
@@ -386,6 +389,8 @@ class CudaOps:
         self.tcgen05_pairs = True           # False: the tcgen05 product never pairs SMs (cta_group::1 only)
         self.fuse_decode_new_token = True   # False: always the separate q/k norm + rotation + store kernel
         self.latent_attention_tc = True     # False: attention over latent rows always on the general kernel
+        self.f32_split = True               # False: float32 products on the FMA pipes whatever their sizes
+        self._segments_cache: dict[tuple[int, int], int] = {}
         self.f32_tile = -1                  # which tile shape computes float32 products (-1: by their sizes; same bits)
         self.experts_tc = True              # False: the experts' products always on the FMA kernels
         self.chunk_tc = True                # False: attention under chunks or with turned values on the general kernel
@@ -1953,7 +1958,8 @@ class CudaOps:
         return self.add_bias(self._product(x, weight, out, out_dtype, False), bias)
 
     def _product(self, x, weight, out=None, out_dtype=None, partial_sums=False):
-        """``x[M, K] @ weight[N, K]^T``.  float32: this engine's FMA kernel (no TF32).
+        """``x[M, K] @ weight[N, K]^T``.  float32: on the tensor cores with operands in three bfloat16 parts, which is
+        nearer to the exact product than a chain of fp32 FMA (:meth:`_f32_segments`), small sizes on the FMA pipes; no TF32.
         bfloat16, at most 16 tokens: one of this engine's two weight-streaming kernels
         (:meth:`_small_product`).  bfloat16, more tokens: the library product with fp32
         accumulation, as the reference's ``nn.Linear`` (qwen3_runtime/models/qwen3.py:76-77,
@@ -1983,6 +1989,19 @@ class CudaOps:
         if x.dtype == torch.float32:
             if out is None:
                 out = torch.empty((M, N), dtype=torch.float32, device=x.device)
+            segments = self._f32_segments(x, weight)
+            if segments and M:
+                # (in portions of rows, which bounds the scratch: a row's bits do not depend on its neighbours)
+                most = min(M, self.F32_SPLIT_ROWS)
+                parts = torch.empty(3 * most * K, dtype=torch.bfloat16, device=x.device)
+                planes = torch.empty((segments, most, N), dtype=torch.float32, device=x.device) if segments > 1 else None
+                for m in range(0, M, most):
+                    rows = min(most, M - m)
+                    self.launches += 1 + (segments > 1)
+                    self._call("gemm_f32", "q3_gemm_f32_split", "gemm_f32_split", _ptr(x[m:]), x.stride(0), _ptr(weight),
+                               weight.stride(0), _ptr(out[m:]), out.stride(0), rows, N, K, _ptr(parts), _ptr(planes),
+                               _ptr(self._error_word(x.device)))
+                return out
             self._call("gemm_f32", "q3_gemm_f32", "gemm_f32", _ptr(x), x.stride(0), _ptr(weight),
                        weight.stride(0), _ptr(out), out.stride(0), M, N, K, self.f32_tile)
             return out
@@ -1998,6 +2017,19 @@ class CudaOps:
             with self._timed("library_mm"):
                 return self._library_mm(x, weight, out, out_dtype)
         return self._library_mm(x, weight, out, out_dtype)
+
+    F32_SPLIT_ROWS = 4096
+
+    def _f32_segments(self, x, weight) -> int:
+        """Segments of K in the float32 product on the tensor cores (csrc/gemm_f32_split.cuh); 0: the FMA kernel computes it.
+        The choice must not depend on the tokens, so that a row's bits do not: the weight's sizes and rows only."""
+        N, K = weight.shape
+        if not self.f32_split or self.f32_tile >= 0 or weight.stride(0) % 4 or weight.data_ptr() % 16:
+            return 0
+        segments = self._segments_cache.get((N, K))
+        if segments is None:
+            segments = self._segments_cache[(N, K)] = int(self._get("gemm_f32", "q3_gemm_f32_split_segments")(N, K))
+        return segments
 
     @staticmethod
     def _library_mm(x, weight, out, out_dtype):

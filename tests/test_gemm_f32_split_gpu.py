@@ -1,0 +1,79 @@
+"""float32 products on the tensor cores in three bfloat16 parts: nearer to float64 than the FMA chain, a row's bits whatever the
+number of rows and the tile, sizes that end inside a tile, a slice or a segment, rows of wider matrices, infinities and NaN."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from qwen3_runtime_b200.ops.cuda import CudaOps
+
+    return CudaOps()
+
+
+def _matrices(M, N, K, pad=0, positive=False, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed + N + K)
+    w = torch.randn((N, K + pad), generator=g, device="cuda")[:, :K]
+    x = torch.randn((M, K + pad), generator=g, device="cuda")[:, :K]
+    return (x.abs(), w.abs()) if positive else (x, w)
+
+
+@pytest.mark.parametrize("N,K,pad", [(19456, 1032, 0), (2308, 9728, 4), (4100, 4936, 0), (260, 77000, 8), (19500, 1088, 1)])
+@pytest.mark.parametrize("positive", [False, True])
+def test_nearer_than_the_fma_chain_and_the_same_for_any_rows(ops, N, K, pad, positive):
+    x, w = _matrices(337, N, K, pad if pad % 4 == 0 else 0, positive)
+    if pad % 4:  # (rows of x without whole 16 bytes; the weights' rows decide who computes)
+        x = torch.cat([x, x[:, :pad]], dim=1)[:, :K]
+    assert ops._f32_segments(x, w) > 0
+    want = x.double() @ w.double().t()
+    got = ops.linear(x, w)
+    ops.raise_if_kernel_error()
+    ops.f32_split = False
+    try:
+        chain = ops.linear(x, w)
+    finally:
+        ops.f32_split = True
+    error = float((got.double() - want).norm() / want.norm())
+    assert error <= float((chain.double() - want).norm() / want.norm())
+    # slices of 64 values round towards zero at most 24 times, their sums to nearest: far below a chain's K roundings
+    assert error <= 2.0 ** -24 * (6 + (K / 64) ** 0.5)
+    for rows in (1, 2, 15, 16, 17, 33, 96, 159, 160, 161, 320, 321):
+        assert torch.equal(ops.linear(x[:rows], w), got[:rows]), rows
+
+
+def test_not_for_weights_it_would_slow_down(ops):
+    for N, K in ((2560, 4096), (6144, 2560), (100, 300000), (20000, 1000), (19456, 1028), (19457, 2560)):
+        w = torch.empty((N, K), device="cuda")
+        assert ops._f32_segments(w[:1], w) == 0, (N, K)
+    w = torch.empty((19456, 2561), device="cuda")[:, :2560]
+    assert ops._f32_segments(w[:1], w) == 0
+
+
+def test_infinities_as_float32_gives_them(ops):
+    x, w = _matrices(5, 19456, 1088)
+    x[1, 7], x[2, 8], x[2, 9] = float("inf"), float("inf"), float("-inf")
+    x[3, 1000] = float("nan")
+    w[11, 3] = float("-inf")
+    w[12, 1087], x[:, 1087] = 3.4e38, 0.5  # (rounds up to infinity in 16 bits; its products do not overflow)
+    got, want = ops.linear(x, w), x.double() @ w.double().t()
+    ops.raise_if_kernel_error()
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got[got.isinf()], want[got.isinf()].float())
+    assert torch.equal(got.isinf(), want.float().isinf())
+
+
+def test_many_rows_in_portions(ops):
+    x, w = _matrices(700, 2560, 9728)
+    want = ops.linear(x, w)
+    ops.F32_SPLIT_ROWS = 256
+    try:
+        got = torch.full((700, 2570), float("nan"), device="cuda")
+        ops.linear(x, w, out=got[:, :2560])
+    finally:
+        del ops.F32_SPLIT_ROWS
+    assert torch.equal(got[:, :2560], want) and bool(got[:, 2560:].isnan().all())
