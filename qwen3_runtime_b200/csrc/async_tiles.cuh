@@ -174,6 +174,16 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a_desc, uint
       ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// the same with the A operand in tensor memory: bf16 pairs, two k-values per 32-bit column, rows in the lanes
+__device__ __forceinline__ void umma_bf16_tmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t idesc,
+                                               uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // True in one lane of a warp that is here as a whole.  MMAs and commits in code guarded by it keep their descriptors in uniform
 // registers: 37 cycles for an MMA of 16 columns and 47 for one of 64, which is what they take to compute; 60 where lane 0
 // branches off by its number.

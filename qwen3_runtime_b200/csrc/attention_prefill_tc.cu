@@ -28,14 +28,15 @@
 //   warps 14, 15     : MMA issuers of PV for block A and B: PV_j when P_j is written.
 // Tensor memory: all 512 columns, per block S [0,64), P_0 and P_1 [64,128), O [128,256).
 // What bounds it: the softmax warps, and behind them the products (S with 64 columns is bound by its reads of shared memory,
-// 45 cycles per 16 k-values) and the keys' and values' way from L2 (32 KB a step and SM).  A step of both blocks takes 1650
+// 45 cycles per 16 k-values) and the keys' and values' way from L2 (32 KB a step and SM).  A step of both blocks takes 1520
 // cycles where the exp2 unit alone needs 1024.  What counted was code, not arithmetic: 32 heads over 8, 8192 tokens, one layer,
-// us (2048 tokens: 48 -> 44):
+// us (2048 tokens: 48 -> 43):
 //   554  one issuer per block (PV_j before S_(j+2): its waits, commits and products took longer than the softmax of a tile), one
 //        producer, S twice and P over S
 //   550  S issued before PV by warps of their own, four producers
 //   512  tiles that all rows see as a whole without the masks' branches; waits with their slow part out of line
 //   457  the reference point moved without a branch, the rescaling out of line
+//   440  the issuers' lane chosen by elect.sync (an MMA of 64 columns every 47 cycles instead of 60 to 78)
 // Not kept: 128 keys a step (830: the chain of a block twice as long), turns of the two blocks at the exponentials (482),
 // S_(j+1) loaded beside the exponentials of tile j with 192 registers a thread (585), waits that try again without looking at
 // the clock (512 -> 562).  Forms: differential attention, 16 heads over 4, 2333 + 419 tokens 60 -> 54 us (mma.sync: 247);
@@ -95,35 +96,6 @@ __device__ __forceinline__ float ex2(float x) {
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
-}
-
-// The warps that copy and multiply run as a whole, and only the instruction itself is one lane's: an arrival and its wait, there
-// and back between two warps, take 511 cycles between single lanes and 247 between whole warps.
-__device__ __forceinline__ void mma_ss(bool leader, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.ne.b32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"((uint32_t)leader)
-      : "memory");
-}
-__device__ __forceinline__ void mma_ts(bool leader, uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.ne.b32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"((uint32_t)leader)
-      : "memory");
-}
-__device__ __forceinline__ void commit(bool leader, uint32_t bar) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\t"
-      "setp.ne.b32 q, %1, 0;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
-      ::"r"(bar), "r"((uint32_t)leader)
-      : "memory");
 }
 
 // A wait that is one instruction and a branch that is not taken where the barrier is complete, or becomes so while the
@@ -315,65 +287,68 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
         if (++st == KV_STAGES) st = 0, phase ^= 1;
       }
     } else if (warp > 11) {
-      {  // ---- MMA issuers: warps 12 and 13 for S of block A and B, warps 14 and 15 for PV ---------
-        // Issuing is work too (descriptors, barrier round trips of a hundred cycles each, a queue in front of the tensor
-        // core): one thread that issued both products of a block needed longer for a tile than the softmax.  Both blocks use
-        // every K and V tile: its "empty" barrier counts two arrivals, a commit from an issuer that multiplied with the
-        // tile and a plain arrival (after the tile's "full") from one that had no use for it.
-        const int x = warp & 1;
-        const bool leader = lane == 0;
-        const int my_tiles = tiles[x];
-        const uint32_t tmem_x = tmem + x * TMEM_BLOCK;
-        if (warp < 14) {
-          constexpr uint32_t idesc = umma_idesc(BLOCK_M, BLOCK_N, 0);   // S = Q K^T: N = 64 keys
-          const uint32_t q_addr = smem_addr(q_s) + x * Q_BYTES;
-          bool ok = my_tiles == 0 || mbar_wait(bar(BAR_Q), 0, &abort_flag);
-          int st = 0;
-          uint32_t phase = 0;
-          for (int j = 0; j < num_tiles && ok; ++j) {
-            // S_j as soon as the softmax has S_(j-1) in its registers
-            if (j > 0 && j < my_tiles) ok = mbar_wait(bar(BAR_S_EMPTY + x), (j - 1) & 1, &abort_flag);
-            if (ok) ok = mbar_wait(bar(BAR_K_FULL + st), phase, &abort_flag);
-            if (!ok) break;
-            if (j < my_tiles) {
-              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // ---- MMA issuers: warps 12 and 13 for S of block A and B, warps 14 and 15 for PV ---------
+      // Issuing is work too (descriptors, barrier round trips of a hundred cycles each, a queue in front of the tensor
+      // core): one thread that issued both products of a block needed longer for a tile than the softmax.  The warps run as
+      // a whole (an arrival and its wait, there and back, take 511 cycles between single lanes and 247 between warps).  Both
+      // blocks use every K and V tile: its "empty" barrier counts two arrivals, a commit from an issuer that multiplied with
+      // the tile and a plain arrival (after the tile's "full") from one that had no use for it.
+      const int role = __shfl_sync(0xffffffffu, warp, 0), x = role & 1;
+      const int mine = __shfl_sync(0xffffffffu, tiles[x], 0), all = __shfl_sync(0xffffffffu, num_tiles, 0);
+      const uint32_t tmem_x = __shfl_sync(0xffffffffu, tmem, 0) + x * TMEM_BLOCK;
+      const bool leader = elect_one();
+      auto wait_all = [&](int b, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar(b), parity, &abort_flag)); };
+      int st = 0;
+      uint32_t phase = 0;
+      if (role < 14) {
+        constexpr uint32_t idesc = umma_idesc(BLOCK_M, BLOCK_N, 0);  // S = Q K^T: N = 64 keys
+        const uint32_t q_addr = smem_addr(q_s) + x * Q_BYTES;
+        bool ok = mine == 0 || wait_all(BAR_Q, 0);
+        for (int j = 0; j < all && ok; ++j) {
+          // S_j as soon as the softmax has S_(j-1) in its registers
+          ok = (j == 0 || j >= mine || wait_all(BAR_S_EMPTY + x, (j - 1) & 1)) && wait_all(BAR_K_FULL + st, phase);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          if (leader) {
+            if (j < mine) {
               const uint32_t k_addr = smem_addr(k_s) + st * K_BYTES;
 #pragma unroll
               for (int k = 0; k < (MODE == MAPS ? 64 : DK) / 16; ++k) {
                 const uint32_t half = (k >> 2), sub = (k & 3) * 2;  // 4 steps of 32 bytes per 64 columns
-                mma_ss(leader, tmem_x, umma_desc(q_addr + half * HALF_Q) + sub,
+                umma_bf16(tmem_x, umma_desc(q_addr + half * HALF_Q) + sub,
                      umma_desc(k_addr + (MODE == MAPS ? x : half) * HALF_KV) + sub, idesc, k > 0 ? 1u : 0u);
               }
-              commit(leader, bar(BAR_S_FULL + x));    // S_j is in TMEM
-              commit(leader, bar(BAR_K_EMPTY + st));  // this block is done with the key tile
+              umma_commit(bar(BAR_S_FULL + x));    // S_j is in TMEM
+              umma_commit(bar(BAR_K_EMPTY + st));  // this block is done with the key tile
             } else {
-              if (leader) mbar_arrive(bar(BAR_K_EMPTY + st));
+              mbar_arrive(bar(BAR_K_EMPTY + st));
             }
-            if (++st == KV_STAGES) st = 0, phase ^= 1;
           }
-        } else {
-          constexpr uint32_t idesc = umma_idesc(BLOCK_M, D, 1);        // PV: N = 128, V MN-major
-          bool ok = true;
-          int st = 0;
-          uint32_t phase = 0;
-          for (int j = 0; j < num_tiles && ok; ++j) {
-            if (j < my_tiles) ok = mbar_wait(bar(BAR_P_FULL + x), j & 1, &abort_flag);  // P_j written, O at rest
-            if (ok) ok = mbar_wait(bar(BAR_V_FULL + st), phase, &abort_flag);
-            if (!ok) break;
-            if (j < my_tiles) {
-              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (++st == KV_STAGES) st = 0, phase ^= 1;
+        }
+      } else {
+        constexpr uint32_t idesc = umma_idesc(BLOCK_M, D, 1);  // PV: N = 128, V MN-major
+        bool ok = true;
+        for (int j = 0; j < all && ok; ++j) {
+          ok = (j >= mine || wait_all(BAR_P_FULL + x, j & 1)) && wait_all(BAR_V_FULL + st, phase);  // P_j written, O at rest
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          if (leader) {
+            if (j < mine) {
               const uint32_t v_addr = smem_addr(v_s) + st * V_BYTES;
 #pragma unroll
               for (int k = 0; k < BLOCK_N / 16; ++k)  // 16 keys: 8 columns of P, 2 KB down V's rows
-                mma_ts(leader, tmem_x + TMEM_O, tmem_x + TMEM_P + (j & 1) * (BLOCK_N / 2) + 8 * k,
+                umma_bf16_tmem(tmem_x + TMEM_O, tmem_x + TMEM_P + (j & 1) * (BLOCK_N / 2) + 8 * k,
                      umma_desc_mn_major(v_addr + k * 2048, HALF_KV), idesc, (j > 0 || k > 0) ? 1u : 0u);
-              commit(leader, bar(BAR_PV_FULL + x));
-              commit(leader, bar(BAR_V_EMPTY + st));
+              umma_commit(bar(BAR_PV_FULL + x));
+              umma_commit(bar(BAR_V_EMPTY + st));
             } else {
-              if (leader) mbar_arrive(bar(BAR_V_EMPTY + st));
+              mbar_arrive(bar(BAR_V_EMPTY + st));
             }
-            if (++st == KV_STAGES) st = 0, phase ^= 1;
           }
+          __syncwarp();
+          if (++st == KV_STAGES) st = 0, phase ^= 1;
         }
       }
     } else {  // ---- softmax: one thread per row; warps 2..5 block A, warps 6..9 block B ---------------
