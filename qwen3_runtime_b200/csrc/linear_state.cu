@@ -28,23 +28,20 @@
 // of the double buffer afterwards.  A token's arithmetic does not depend on where the step's portion
 // starts or ends, so the result has the same bits however a prompt is cut.
 //
-// segment_scan: the same recurrence for prompts in bfloat16.  The scan above is a chain over a sequence's tokens, 0.21 us each, with
+// Segments: the same recurrence for prompts in bfloat16.  The scan above is a chain over a sequence's tokens, 0.21 us each, with
 // one block per (head, 16 columns): 2048 tokens of 16 heads took 430 us with the SMs mostly idle.  Here a sequence is cut
 // into segments of `seg` tokens: (1) every segment but a sequence's last works out the state it would leave behind if it
 // began with zeros, and the product of its decays; (2) the segments' first states follow one from another,
 // S <- diag(product) S + left behind; (3) every segment runs from its first state and writes its outputs, a sequence's last
-// one the slot.  All decays are at most one, so nothing grows, and every sum is fp32 as before.  The rotations, decays and
-// scales of a token's rows are worked out by a kernel of their own (16 us), not in both passes and every column tile.  A
-// thread holds 4 x 8 elements of the state, so that a token's three rows and its values are read once for 32 updates, as
-// pairs of columns for the packed instructions, and the sums over the row groups are folded: a lane gives half of its
-// columns away at each step.  The passes are bound by a block's chain over its tokens at two blocks an SM (issue slots 40 and 50 %
-// busy; waits for arithmetic and shared memory).  A block finds its sequence with one warp, 32 sequences at a time (one thread
-// walking 128 sequences cost every block of every pass 20 us).  When this is the faster scan, and with which `seg`, is worked
-// out from the sequences' lengths (ops/cuda.py, decayed_scan_segment).
+// one the slot.  All decays are at most one, so nothing grows, and every sum is fp32 as before.  Within a segment 16 tokens are
+// one step of matrix products (below): token by token the two passes and the rows took 133 us for 2048 tokens of 16 heads of
+// 64 x 128 and 229 for 128 x 128, in chunks 83 and 134.  When this is the faster scan, and with which `seg`, is worked out from
+// the sequences' lengths (ops/cuda.py, decayed_scan_segment, chunk_segment).
 //
 // head_norm_gate: y[t, h, :] = o / sqrt(mean(o^2) + eps) * w * silu(g[t, h, :]) * out_scale, one warp
 // per (token, head); w may be absent.
 #include "common.cuh"
+#include "split_mma.cuh"
 
 #define SCAN_CT 16  // tokens per chunk
 
@@ -286,229 +283,57 @@ struct ScanArgs {
   int seg;          // tokens per segment
   float* ends;      // [segments, H, D, Dv]: what a segment leaves behind, then the segments' first states
   float* products;  // [segments, H, D]
-  float* rows;      // [T, H, 3, DP], DP = 64 or 128
 };
 
 __device__ __forceinline__ int segments_of(const ScanArgs& a, int b) {
   return (a.cu_seqlens[b + 1] - a.cu_seqlens[b] + a.seg - 1) / a.seg;
 }
 
-// A token's rows of a head as the scans read them, fp32 [T, H, 3, DP]: keys (turned, scaled), decays, queries (turned,
-// scaled); zero (and one) beyond D.  Worked out once: both scans and every column tile read the same rows.
-template <int DP>
-__global__ void __launch_bounds__(256)
-segment_rows_kernel(const __grid_constant__ ScanArgs a, long total) {
-  pdl_wait();
-  pdl_launch_dependents();
-  const long x = (long)blockIdx.x * 256 + threadIdx.x;
-  if (x >= total) return;
-  const int i = x % DP;
-  const long th = x / DP, t = th / a.H;
-  const int h = (int)(th - t * a.H);
-  const bf16 *q = (const bf16*)a.q + t * a.q_stride + h * a.D, *k = (const bf16*)a.k + t * a.k_stride + h * a.D;
-  float qv = 0.f, kv = 0.f, av = 1.f;
-  if (i < a.D) {
-    qv = to_f32(q[i]);
-    kv = to_f32(k[i]);
-    if (i < 2 * a.rot_pairs) {
-      const bool front = i < a.rot_pairs;
-      const int pair = front ? i : i - a.rot_pairs, other = front ? i + a.rot_pairs : pair;
-      float sn, cs;
-      sincosf((float)a.positions[t] * a.inv_freq[pair], &sn, &cs);
-      const float qp = to_f32(q[other]), kp = to_f32(k[other]);
-      qv = front ? qv * cs - qp * sn : qv * cs + qp * sn;
-      kv = front ? kv * cs - kp * sn : kv * cs + kp * sn;
-    }
-    qv *= a.q_scale;
-    kv *= a.k_scale;
-    if (a.tok_kscale) kv *= a.tok_kscale[t * a.H + h];
-    if (a.z) {
-      const float zz = to_f32(((const bf16*)a.z)[t * a.z_stride + h * a.D + i]) + (a.z_bias ? a.z_bias[h * a.D + i] : 0.f);
-      av = a.decay_mode == 1 ? expf(-expf(zz)) : expf((fminf(zz, 0.f) - log1pf(expf(-fabsf(zz)))) * a.inv_tau);
-    } else {
-      av = a.tok_decay ? a.tok_decay[t * a.H + h] : a.head_decay[h];
-    }
+// Channel i < D of a token's key (turned, scaled), decay and query (turned, scaled) of a head, from its raw values.
+__device__ __forceinline__ void scan_element(const ScanArgs& a, long t, int h, int i, float& kv, float& av, float& qv, float zz) {
+  if (i < 2 * a.rot_pairs) {
+    const bf16 *q = (const bf16*)a.q + t * a.q_stride + h * a.D, *k = (const bf16*)a.k + t * a.k_stride + h * a.D;
+    const bool front = i < a.rot_pairs;
+    const int pair = front ? i : i - a.rot_pairs, other = front ? i + a.rot_pairs : pair;
+    float sn, cs;
+    sincosf((float)a.positions[t] * a.inv_freq[pair], &sn, &cs);
+    const float qp = to_f32(q[other]), kp = to_f32(k[other]);
+    qv = front ? qv * cs - qp * sn : qv * cs + qp * sn;
+    kv = front ? kv * cs - kp * sn : kv * cs + kp * sn;
   }
-  float* dst = a.rows + th * 3 * DP + i;
-  dst[0] = kv;
-  dst[DP] = av;
-  dst[2 * DP] = qv;
+  qv *= a.q_scale;
+  kv *= a.k_scale;
+  if (a.tok_kscale) kv *= a.tok_kscale[t * a.H + h];
+  if (a.z) {
+    av = a.decay_mode == 1 ? expf(-expf(zz)) : expf((fminf(zz, 0.f) - log1pf(expf(-fabsf(zz)))) * a.inv_tau);
+  } else {
+    av = a.tok_decay ? a.tok_decay[t * a.H + h] : a.head_decay[h];
+  }
 }
 
-// DP: key rows (64 or 128), in DP / 4 row groups; CG column groups of 8: a thread holds 4 x 8 elements of the state.
-// Block: (segment, column tile, head).
-template <int DP, int CG, bool OUT, bool BONUS>
-__global__ void __launch_bounds__(DP / 4 * CG, 2)
-segment_scan_kernel(const __grid_constant__ ScanArgs a) {
-  constexpr int RG = DP / 4, THREADS = RG * CG, VT = 8 * CG, CT = SCAN_CT;
-  constexpr int ROW = (OUT ? 3 : 2) * DP, VPT = CT * VT / THREADS;  // a token's k, a (and q) rows
-  static_assert(VPT * THREADS == CT * VT && (RG == 16 || RG == 32), "whole turns");
-  extern __shared__ __align__(16) float scan_smem[];
-  float* rs = scan_smem;              // [2][CT][ROW]
-  float* vs = rs + 2 * CT * ROW;      // [2][CT][VT]
-  float* os = vs + 2 * CT * VT;       // [CT][VT]
-  __shared__ int s_seq, s_first, s_count;
-  const int tid = threadIdx.x;
-  const int H = a.H, D = a.D, Dv = a.Dv, h = blockIdx.z, j0 = blockIdx.y * VT;
-  pdl_wait();
-  pdl_launch_dependents();
-  if (tid < 32) {  // the sequence that this segment belongs to, 32 sequences at a time
-    int at = 0, seq = -1, first = 0, count = 0;
-    for (int b0 = 0; b0 < a.num_seqs; b0 += 32) {
-      const int n = b0 + tid < a.num_seqs ? segments_of(a, b0 + tid) : 0;
-      int sum = n;
+// The sequence that this block's segment (blockIdx.x) belongs to (-1: none), the number of that sequence's first segment and
+// how many it has.  Every warp for itself, 32 sequences at a time.
+__device__ __forceinline__ int segment_owner(const ScanArgs& a, int& first, int& count) {
+  const int lane = threadIdx.x & 31;
+  int at = 0;
+  for (int b0 = 0; b0 < a.num_seqs; b0 += 32) {
+    const int n = b0 + lane < a.num_seqs ? segments_of(a, b0 + lane) : 0;
+    int sum = n;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int x = __shfl_up_sync(0xffffffffu, sum, o);
-        if (tid >= o) sum += x;
-      }
-      const uint32_t beyond = __ballot_sync(0xffffffffu, at + sum > (int)blockIdx.x);
-      if (beyond) {
-        const int l = __ffs(beyond) - 1;
-        seq = b0 + l;
-        count = __shfl_sync(0xffffffffu, n, l);
-        first = at + __shfl_sync(0xffffffffu, sum, l) - count;
-        break;
-      }
-      at += __shfl_sync(0xffffffffu, sum, 31);
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += x;
     }
-    if (tid == 0) {
-      s_seq = seq;
-      s_first = first;
-      s_count = count;
+    const uint32_t beyond = __ballot_sync(0xffffffffu, at + sum > (int)blockIdx.x);
+    if (beyond) {
+      const int l = __ffs(beyond) - 1;
+      count = __shfl_sync(0xffffffffu, n, l);
+      first = at + __shfl_sync(0xffffffffu, sum, l) - count;
+      return b0 + l;
     }
+    at += __shfl_sync(0xffffffffu, sum, 31);
   }
-  __syncthreads();
-  const int seq = s_seq;
-  if (seq < 0) return;
-  const int mine = blockIdx.x - s_first;  // the segment's number in its sequence
-  const bool last = mine == s_count - 1;
-  if (!OUT && last) return;
-  const int t0 = a.cu_seqlens[seq] + mine * a.seg, t1 = min(a.cu_seqlens[seq + 1], t0 + a.seg);
-  const long slot = a.state_slots[seq];
-  const int rg = tid % RG, cg = tid / RG, i0 = rg * 4, c0 = cg * 8;
-  const long tile = ((long)blockIdx.x * H + h) * D;
-  float* Sg = a.state + (slot * H + h) * (long)D * Dv;
-  float2 S[4][4];  // [row][pair of columns]
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int i = i0 + r, j = j0 + c0 + 2 * c;
-      const float* src = s_count > 1 ? a.ends + (tile + i) * Dv : Sg + (long)i * Dv;
-      S[r][c].x = !OUT || i >= D || j >= Dv ? 0.f : src[j];
-      S[r][c].y = !OUT || i >= D || j + 1 >= Dv ? 0.f : src[j + 1];
-    }
-  float U[4], P[4];
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    U[r] = (BONUS && i0 + r < D) ? a.bonus[h * D + i0 + r] : 0.f;
-    P[r] = 1.f;
-  }
-  const int Dvin = Dv - a.ones_col;
-  const bf16* v = (const bf16*)a.v;
-  bf16 vr[VPT];
-  // a chunk's rows into buffer `to` (its values into registers): in flight while the chunk before is worked on
-  auto fetch = [&](int t_at, int to) {
-    const int n = min(CT, t1 - t_at);
-    for (int x = tid * 4; x < n * ROW; x += THREADS * 4) {
-      const int c = x / ROW;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(rs + to * CT * ROW + x)),
-                   "l"(a.rows + ((long)(t_at + c) * H + h) * 3 * DP + (x - c * ROW)) : "memory");
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-#pragma unroll
-    for (int m = 0; m < VPT; ++m) {
-      const int x = tid + m * THREADS, c = x / VT, j = j0 + x % VT;
-      const long t = t_at + c;
-      vr[m] = t < t1 && j < Dvin ? v[t * a.v_stride + h * Dvin + j] : from_f32<bf16>(t < t1 && j < Dv ? 1.f : 0.f);
-    }
-  };
-  auto stage = [&](int to) {
-#pragma unroll
-    for (int m = 0; m < VPT; ++m) vs[to * CT * VT + tid + m * THREADS] = to_f32(vr[m]);
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-  };
-  fetch(t0, 0);
-  stage(0);
-  __syncthreads();
-  int buf = 0;
-  for (int t = t0; t < t1; t += CT, buf ^= 1) {
-    const int n = min(CT, t1 - t);
-    const bool more = t + CT < t1;
-    if (more) fetch(t + CT, buf ^ 1);
-#pragma unroll 2
-    for (int c = 0; c < n; ++c) {
-      const float* row = rs + (buf * CT + c) * ROW + i0;
-      const float4 k4 = *reinterpret_cast<const float4*>(row);
-      const float4 a4 = *reinterpret_cast<const float4*>(row + DP);
-      const float4 va = *reinterpret_cast<const float4*>(vs + (buf * CT + c) * VT + c0);
-      const float4 vb = *reinterpret_cast<const float4*>(vs + (buf * CT + c) * VT + c0 + 4);
-      const float2 vv[4] = {make_float2(va.x, va.y), make_float2(va.z, va.w), make_float2(vb.x, vb.y), make_float2(vb.z, vb.w)};
-      const float aa[4] = {a4.x, a4.y, a4.z, a4.w}, kk[4] = {k4.x, k4.y, k4.z, k4.w};
-      float qq[4] = {0.f, 0.f, 0.f, 0.f};
-      float2 acc[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-      if (OUT) {
-        const float4 q4 = *reinterpret_cast<const float4*>(row + 2 * DP);
-        qq[0] = q4.x; qq[1] = q4.y; qq[2] = q4.z; qq[3] = q4.w;
-      }
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const float2 a2 = make_float2(aa[r], aa[r]), k2 = make_float2(kk[r], kk[r]), q2 = make_float2(qq[r], qq[r]);
-        const float2 u2 = make_float2(U[r], U[r]);
-        if (!OUT && tid < 32) P[r] *= aa[r];  // (the first warp's rows are all rows)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 kv = __fmul2_rn(k2, vv[e]);
-          if (OUT && BONUS) acc[e] = __ffma2_rn(__ffma2_rn(u2, kv, S[r][e]), q2, acc[e]);
-          S[r][e] = __ffma2_rn(a2, S[r][e], kv);
-          if (OUT && !BONUS) acc[e] = __ffma2_rn(S[r][e], q2, acc[e]);
-        }
-      }
-      if (OUT) {
-        // the sums over the row groups, lanes rg: a lane gives half of its columns away in each of three steps and then
-        // has one column's sum over eight groups
-        const bool h1 = rg & 1, h2 = rg & 2, h4 = rg & 4;
-        const float av[8] = {acc[0].x, acc[0].y, acc[1].x, acc[1].y, acc[2].x, acc[2].y, acc[3].x, acc[3].y};
-        float x4[4], x2[2];
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          x4[e] = (h1 ? av[e + 4] : av[e]) + __shfl_xor_sync(0xffffffffu, h1 ? av[e] : av[e + 4], 1);
-#pragma unroll
-        for (int e = 0; e < 2; ++e)
-          x2[e] = (h2 ? x4[e + 2] : x4[e]) + __shfl_xor_sync(0xffffffffu, h2 ? x4[e] : x4[e + 2], 2);
-        float y = (h4 ? x2[1] : x2[0]) + __shfl_xor_sync(0xffffffffu, h4 ? x2[0] : x2[1], 4);
-#pragma unroll
-        for (int o = 8; o < RG; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-        if (rg < 8) os[c * VT + c0 + 4 * (rg & 1) + (rg & 2) + (rg >> 2)] = y;
-      }
-    }
-    if (OUT) {
-      __syncthreads();
-      for (int x = tid; x < n * VT; x += THREADS) {
-        const int c = x / VT, j = j0 + x % VT;
-        if (j < Dv) a.out[((long)(t + c) * H + h) * Dv + j] = os[x];
-      }
-    }
-    if (more) stage(buf ^ 1);
-    __syncthreads();
-  }
-  float* dst = OUT ? Sg : a.ends + tile * Dv;
-  if (!OUT || last) {
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int i = i0 + r, j = j0 + c0 + 2 * c;
-        if (i < D && j < Dv) dst[(long)i * Dv + j] = S[r][c].x;
-        if (i < D && j + 1 < Dv) dst[(long)i * Dv + j + 1] = S[r][c].y;
-      }
-  }
-  if (!OUT && blockIdx.y == 0 && cg == 0) {
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-      if (i0 + r < D) a.products[tile + i0 + r] = P[r];
-  }
+  return -1;
 }
 
 // Step 2: one thread per element of the state; what the segments left behind becomes their first states.
@@ -548,42 +373,442 @@ segment_join_kernel(const __grid_constant__ ScanArgs a) {
   }
 }
 
-template <int DP, int CG, bool BONUS>
-static cudaError_t launch_segments(const ScanArgs& a, int num_tokens, int segments, bool cut, cudaStream_t stream) {
-  constexpr size_t smem = (size_t)(6 * SCAN_CT * DP + 3 * SCAN_CT * 8 * CG) * sizeof(float);
+// ---- a segment in chunks of 16 tokens ------------------------------------------------------------------
+// With G_i the product of a chunk's decays up to token i and S the state before the chunk, in matrices whose rows are the
+// chunk's tokens:
+//   B_ij = sum_d q_i k_j prod_(j < m <= i) a_m  (j <= i)      O = B V + (G q) S
+//   S <- G_last S + sum_j (prod_(m > j) a_m k_j) v_j^T
+// (with a bonus u, which reads the state before its update: prod_(j < m < i), G_(i - 1), and B_ii = sum_d q_i u k_i).  Only
+// products of decays occur, never quotients, and nothing in the state's chain but one multiply-add per chunk depends on the chunk
+// before.  The products run on mma.sync, fp32 operands in three bfloat16 parts (split_mma.cuh), values as they are; what is added
+// to the state is summed from zero.
+//
+// scan_chunk_rows, a block per (chunk, head): a record of SC_REC words, namely B, G q and the keys decayed to the chunk's end as
+// parts in the order of the scan's fragments, [3][32 lanes][4] for every 16 channels, G_last [DP], whether values are not finite;
+// behind it the values in that order, 128 words for 16 columns.  Chunks of sequence b start at place cu_seqlens[b] / 16 + b; tokens
+// beyond a portion's end are k = q = v = 0, a = 1.  Bound by instructions (2.5 a cycle; the decays' exponentials, the pairs'
+// sums): 38 us for 2048 tokens of 16 heads of 64 x 128, 30 with the loads' addresses worked out once and 8 blocks an SM.
+// scan_chunk_states, a block per (segment, 32 value columns, head): the state transposed in registers as in delta_state.cu, a
+// warp 16 channels; the warps' parts of (G q) S meet in shared memory, one barrier a chunk, and are added a chunk later.  The same
+// prompt, us: 20 + 59 with values and B V read and written beside the records, 13 + 29 so (two stages, so that 4 blocks fit an
+// SM; 11 + 35 with three).  What is left waits for shared memory and the MMAs' results.
+#define SC_C 16
+#define SC_TILES 2  // of 16 value columns, in a block
+#define SC_STAGES 2
+#define SC_REC(DP) (388 + (DP) * 49)  // a record before its values
+#define SC_VALUES(Dv) (((Dv) + 16 * SC_TILES - 1) / (16 * SC_TILES) * SC_TILES * 128)
+
+__device__ __forceinline__ void sc_copy16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
+}
+
+template <int DP>
+__global__ void __launch_bounds__(2 * DP, 512 / DP)
+scan_chunk_rows_kernel(const __grid_constant__ ScanArgs a, uint32_t* __restrict__ records) {
+  constexpr int PITCH = DP + 4, WARPS = DP / 16, NT = 2 * DP, E = DP / 32;
+  __shared__ __align__(16) float ks[SC_C][PITCH], qs[SC_C][PITCH], gs[SC_C][PITCH];  // later: keys to the end, G q
+  __shared__ __align__(16) float bs[SC_C][SC_C + 4];                                  // B
+  pdl_wait();
+  pdl_launch_dependents();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gr = lane >> 2, t4 = lane & 3;
+  const int place = blockIdx.x, h = blockIdx.y, H = a.H, Dv = a.Dv, Dvin = Dv - a.ones_col;
+  int n = 0;
+  long t0 = 0;
+  for (int b0 = 0; b0 < a.num_seqs; b0 += 32) {  // whose chunk this is, every warp for itself, 32 sequences at a time
+    const int b = b0 + lane;
+    int first = 0, left = 0;
+    bool found = false;
+    if (b < a.num_seqs) {
+      const int c0 = a.cu_seqlens[b], c1 = a.cu_seqlens[b + 1], base = c0 / SC_C + b;
+      found = place >= base && place < c1 / SC_C + b + 1;
+      first = c0 + (place - base) * SC_C;
+      left = min(c1 - first, SC_C);
+    }
+    const uint32_t who = __ballot_sync(0xffffffffu, found);
+    if (who) {
+      t0 = __shfl_sync(0xffffffffu, first, __ffs(who) - 1);
+      n = __shfl_sync(0xffffffffu, left, __ffs(who) - 1);
+      break;
+    }
+  }
+  if (n <= 0) return;
+  {  // a thread one channel of every other token; all of its loads in flight together
+    const int i = tid % DP, c0 = tid / DP;
+    const long t = t0 + c0;
+    const bf16 *q = (const bf16*)a.q + t * a.q_stride + h * a.D + i, *k = (const bf16*)a.k + t * a.k_stride + h * a.D + i;
+    const bf16* z = (const bf16*)a.z + t * a.z_stride + h * a.D + i;
+    const bool channel = i < a.D, logits = a.z && channel;
+    float qv[8], kv[8], zv[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const bool live = channel && c0 + 2 * e < n;
+      qv[e] = live ? to_f32(*q) : 0.f;
+      kv[e] = live ? to_f32(*k) : 0.f;
+      zv[e] = live && logits ? to_f32(*z) : 0.f;
+      q += 2 * a.q_stride, k += 2 * a.k_stride, z += 2 * a.z_stride;
+    }
+    const float zb = logits && a.z_bias ? a.z_bias[h * a.D + i] : 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int c = c0 + 2 * e;
+      float av = 1.f;
+      if (channel && c < n) scan_element(a, t + 2 * e, h, i, kv[e], av, qv[e], zv[e] + zb);
+      ks[c][i] = kv[e];
+      gs[c][i] = av;
+      qs[c][i] = qv[e];
+    }
+  }
+  float bonus[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) bonus[e] = a.bonus && lane + 32 * e < a.D ? a.bonus[h * a.D + lane + 32 * e] : 0.f;
+  __syncthreads();
+  for (int w = warp; w < 8; w += WARPS) {  // rows 15 - w and w of B, 17 pairs of tokens; the lanes share the channels
+    float v[24];  // row 15 - w by i - j, then row w
+    auto pairs = [&](int i, int most, int at) {
+      float wq[E], b = 0.f;
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        wq[e] = qs[i][lane + 32 * e];
+        b = fmaf(wq[e], a.bonus ? bonus[e] * ks[i][lane + 32 * e] : ks[i][lane + 32 * e], b);
+        if (!a.bonus) wq[e] *= gs[i][lane + 32 * e];
+      }
+      v[at] = b;
+#pragma unroll
+      for (int r = 1; r < most; ++r) {
+        b = 0.f;
+        if (r <= i) {
+#pragma unroll
+          for (int e = 0; e < E; ++e) {
+            b = fmaf(wq[e], ks[i - r][lane + 32 * e], b);
+            wq[e] *= gs[i - r][lane + 32 * e];
+          }
+        }
+        v[at + r] = b;
+      }
+    };
+    pairs(SC_C - 1 - w, 16, 0);
+    pairs(w, 8, 16);
+    // the sums over the lanes: a lane gives half of its values away in each of three steps and has three of them in the end
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+      const int half = 12 >> s;
+      const bool up = (lane >> s) & 1;
+#pragma unroll
+      for (int x = 0; x < half; ++x) {
+        const float give = up ? v[x] : v[x + half];
+        v[x] = (up ? v[x + half] : v[x]) + __shfl_xor_sync(0xffffffffu, give, 1 << s);
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+      v[x] += __shfl_xor_sync(0xffffffffu, v[x], 8);
+      v[x] += __shfl_xor_sync(0xffffffffu, v[x], 16);
+    }
+    if (lane < 8) {
+      const int first = (lane & 1) * 12 + (lane & 2) * 3 + (lane & 4) / 4 * 3;
+#pragma unroll
+      for (int x = 0; x < 3; ++x) {
+        const int at = first + x, i = at < 16 ? SC_C - 1 - w : w, r = at & (at < 16 ? 15 : 7);
+        if (r <= i) bs[i][i - r] = v[x];
+      }
+    }
+  }
+  for (int x = tid; x < SC_C * SC_C; x += NT)
+    if (x % SC_C > x / SC_C) bs[x / SC_C][x % SC_C] = 0.f;
+  __syncthreads();
+  uint32_t* rec = records + ((long)place * H + h) * (SC_REC(DP) + SC_VALUES(Dv));
+  if (tid < DP) {  // decays from the chunk's start and to its end
+    float run = 1.f, gd[SC_C];
+#pragma unroll
+    for (int i = 0; i < SC_C; ++i) {
+      gd[i] = gs[i][tid];
+      const float before = run;
+      run *= gd[i];
+      qs[i][tid] *= a.bonus ? before : run;
+    }
+    rec[384 + 48 * DP + tid] = __float_as_uint(run);
+    run = 1.f;
+#pragma unroll
+    for (int i = SC_C - 1; i >= 0; --i) {
+      ks[i][tid] *= run;
+      run *= gd[i];
+    }
+  }
+  __syncthreads();
+  auto store = [&](uint32_t* to, const uint32_t (&w)[3][4]) {
+#pragma unroll
+    for (int m = 0; m < 3; ++m)
+      *reinterpret_cast<uint4*>(to + m * 128 + lane * 4) = make_uint4(w[m][0], w[m][1], w[m][2], w[m][3]);
+  };
+  uint32_t w3[3][4];
+  auto put = [&](int x, float lo, float hi) {
+    uint32_t p[3];
+    ds_split(lo, hi, p);
+#pragma unroll
+    for (int m = 0; m < 3; ++m) w3[m][x] = p[m];
+  };
+  if (warp == 0) {  // of tokens gr (+ 8), the weights of tokens 2 t4, 2 t4 + 1 (+ 8)
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const float2 f = *reinterpret_cast<const float2*>(&bs[gr + 4 * (x & 2)][2 * t4 + 8 * (x & 1)]);
+      put(x, f.x, f.y);
+    }
+    store(rec, w3);
+  }
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {  // tokens gr (+ 8) of channels 2 t4, 2 t4 + 1 (+ 8)
+    const float2 f = *reinterpret_cast<const float2*>(&qs[gr + 4 * (x & 2)][warp * 16 + 2 * t4 + 8 * (x & 1)]);
+    put(x, f.x, f.y);
+  }
+  store(rec + 384 + warp * 384, w3);
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {  // tokens 2 t4, 2 t4 + 1 (+ 8) of channels gr (+ 8)
+    const float* f = &ks[2 * t4 + 8 * (x & 1)][warp * 16 + gr + 4 * (x & 2)];
+    put(x, f[0], f[PITCH]);
+  }
+  store(rec + 384 + 24 * DP + warp * 384, w3);
+  const bf16 *v = (const bf16*)a.v + t0 * a.v_stride + h * Dvin, one = from_f32<bf16>(1.f), none = from_f32<bf16>(0.f);
+  int odd = 0;  // values that are not finite
+  for (int w = warp; w < SC_VALUES(Dv) / 128; w += WARPS) {  // transposed: columns gr (+ 8), tokens 2 t4, 2 t4 + 1 (+ 8)
+    uint32_t word[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const int c = 2 * t4 + 4 * (x & 2), j = 16 * w + gr + 8 * (x & 1);
+      const bf16 beyond = j < Dv ? one : none;
+      __nv_bfloat162 pair;
+      pair.x = c >= n ? none : j < Dvin ? v[c * a.v_stride + j] : beyond;
+      pair.y = c + 1 >= n ? none : j < Dvin ? v[(c + 1) * a.v_stride + j] : beyond;
+      word[x] = *reinterpret_cast<uint32_t*>(&pair);
+    }
+    *reinterpret_cast<uint4*>(rec + SC_REC(DP) + w * 128 + lane * 4) = make_uint4(word[0], word[1], word[2], word[3]);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) odd |= (word[x] & 0x7f80u) == 0x7f80u || (word[x] & 0x7f800000u) == 0x7f800000u;
+  }
+  odd = __syncthreads_or(odd);
+  if (tid == 0) rec[384 + 49 * DP] = odd;
+}
+
+// The chunk's own share of a thread's outputs, as ds_products orders them, where values are not finite: a weight of zero is no
+// reason to touch an earlier token's output.  rec: the weights' parts; v: the column tile's values.
+__device__ __noinline__ void own_tokens(float* own, const uint32_t* rec, const uint32_t* v, int lane) {
+  for (int x = 0; x < 8; ++x) {
+    const int t = 8 * (x >> 2) + 2 * (lane & 3) + (x & 1), col = (lane >> 2) + 4 * (x & 2);
+    float sum = 0.f;
+    for (int j = 0; j <= t; ++j) {
+      const int at = (((t & 7) * 4 + ((j & 7) >> 1)) << 2) + 2 * (t >> 3) + (j >> 3), shift = j & 1 ? 0 : 16;
+      float w = 0.f;
+      for (int m = 2; m >= 0; --m) w += __uint_as_float((rec[m * 128 + at] << shift) & 0xffff0000u);
+      const uint32_t pair = v[(((col & 7) * 4 + ((j & 7) >> 1)) << 2) + 2 * (j >> 3) + (col >> 3)];
+      sum = fmaf(w, __uint_as_float((pair << shift) & 0xffff0000u), sum);
+    }
+    own[x] = sum;
+  }
+}
+
+template <int DP, bool OUT>
+__global__ void __launch_bounds__(2 * DP, DP == 64 ? 4 : 2)
+scan_chunk_states_kernel(const __grid_constant__ ScanArgs a, const uint32_t* __restrict__ records) {
+  constexpr int NC = SC_TILES, VT = 16 * NC, NT = 2 * DP, WARPS = DP / 16, PITCH = VT + 4, N = SC_C * VT / NT;
+  constexpr int SKIP = OUT ? 0 : 384 + 24 * DP, HEAD = SC_REC(DP) - SKIP, REC = HEAD + NC * 128;  // what is read of a record
+  constexpr int Q0 = 384, K0 = 384 + 24 * DP - SKIP, GL = K0 + 24 * DP;
+  extern __shared__ __align__(16) uint32_t sc_smem[];                 // the records' ring, then
+  float* part = reinterpret_cast<float*>(sc_smem + SC_STAGES * REC);  // [2][WARPS][SC_C][PITCH]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gr = lane >> 2, t4 = lane & 3;
+  const int col0 = blockIdx.y * VT, h = blockIdx.z;
+  const int H = a.H, D = a.D, Dv = a.Dv;
+  int first, count;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int b = segment_owner(a, first, count);
+  if (b < 0) return;
+  const int mine = blockIdx.x - first;  // the segment's number in its sequence
+  const bool last = mine == count - 1;
+  if (!OUT && last) return;
+  const int seq0 = a.cu_seqlens[b], t0 = seq0 + mine * a.seg, t1 = min(a.cu_seqlens[b + 1], t0 + a.seg);
+  const int chunks = (t1 - t0 + SC_C - 1) / SC_C;
+  const long rec_size = SC_REC(DP) + SC_VALUES(Dv);
+  const uint32_t* rec0 = records + ((long)(seq0 / SC_C + b + mine * (a.seg / SC_C)) * H + h) * rec_size;
+  auto load = [&](int c) {
+    if (c < chunks) {
+      const uint32_t* src = rec0 + (long)c * H * rec_size;
+      uint32_t* dst = sc_smem + (c % SC_STAGES) * REC;
+#pragma unroll
+      for (int x = 0; x < (REC / 4 + NT - 1) / NT; ++x) {
+        const int at = (tid + x * NT) * 4;
+        if (at < REC) sc_copy16(dst + at, src + (at < HEAD ? SKIP + at : SC_REC(DP) + blockIdx.y * NC * 128 + at - HEAD));
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::);  // also when empty: one group per call
+  };
+#pragma unroll
+  for (int c = 0; c < SC_STAGES - 1; ++c) load(c);
+  const long tile = ((long)blockIdx.x * H + h) * D;
+  float* Sg = a.state + ((long)a.state_slots[b] * H + h) * (long)D * Dv;
+  const float* from = count > 1 ? a.ends + tile * Dv : Sg;
+  float S[NC][2][4], P[2][2];  // channel 16 warp + 8 i + 2 t4 + (j & 1), value column 16 w + gr + 8 (j >> 1)
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    P[i][0] = P[i][1] = 1.f;
+#pragma unroll
+    for (int w = 0; w < NC; ++w)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int d = warp * 16 + 8 * i + 2 * t4 + (j & 1), col = col0 + 16 * w + gr + 8 * (j >> 1);
+        S[w][i][j] = OUT && d < D && col < Dv ? from[(long)d * Dv + col] : 0.f;
+      }
+  }
+  const int o_tok = tid / (VT / N), o_col = tid % (VT / N) * N;  // this thread's outputs: N columns of a token
+  const bool whole = Dv % N == 0;
+  auto finish = [&](int c) {  // chunk c's outputs
+    const float* from = part + ((c & 1) * WARPS * SC_C + o_tok) * PITCH + o_col;
+    float sum[N];
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w)
+#pragma unroll
+      for (int x = 0; x < N; x += 2) {
+        const float2 f = *reinterpret_cast<const float2*>(from + w * SC_C * PITCH + x);
+        sum[x] = w ? sum[x] + f.x : f.x;
+        sum[x + 1] = w ? sum[x + 1] + f.y : f.y;
+      }
+    const int t = t0 + c * SC_C + o_tok, col = col0 + o_col;
+    if (t >= t1) return;
+    float* p = a.out + ((long)t * H + h) * Dv + col;
+    if (whole && col < Dv) {
+      if constexpr (N == 4) *reinterpret_cast<float4*>(p) = make_float4(sum[0], sum[1], sum[2], sum[3]);
+      else *reinterpret_cast<float2*>(p) = make_float2(sum[0], sum[1]);
+    } else {
+#pragma unroll
+      for (int x = 0; x < N; ++x)
+        if (col + x < Dv) p[x] = sum[x];
+    }
+  };
+  for (int c = 0; c < chunks; ++c) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(SC_STAGES - 2));
+    __syncthreads();  // the record is there, the last one read; the parts of chunk c - 1 are there, those of c - 2 read
+    load(c + SC_STAGES - 1);
+    const uint32_t* rec = sc_smem + (c % SC_STAGES) * REC;
+    uint32_t v3[NC][3][4], r[3][4];
+#pragma unroll
+    for (int w = 0; w < NC; ++w) {
+      const uint4 word = *reinterpret_cast<const uint4*>(rec + HEAD + w * 128 + lane * 4);
+      v3[w][0][0] = word.x, v3[w][0][1] = word.y, v3[w][0][2] = word.z, v3[w][0][3] = word.w;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) v3[w][1][x] = v3[w][2][x] = 0u;
+    }
+    if (OUT) {
+      ds_parts(r, rec + Q0 + warp * 384, lane);
+#pragma unroll
+      for (int w = 0; w < NC; ++w) {
+        uint32_t s3[3][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint32_t p[3];
+          ds_split(S[w][i >> 1][2 * (i & 1)], S[w][i >> 1][2 * (i & 1) + 1], p);
+#pragma unroll
+          for (int m = 0; m < 3; ++m) s3[m][i] = p[m];
+        }
+        float acc[2][4];
+        ds_products(acc, s3, r);
+        if (warp == w) {  // this warp's share has the chunk's own tokens too
+          uint32_t b3[3][4];
+          float own[2][4];
+          if (rec[GL + DP]) {
+            own_tokens(&own[0][0], rec, rec + HEAD + w * 128, lane);
+          } else {
+            ds_parts(b3, rec, lane);
+            ds_products<false, true>(own, v3[w], b3);
+          }
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] += own[i][j];
+        }
+        float* to = part + (((c & 1) * WARPS + warp) * SC_C + 2 * t4) * PITCH + 16 * w + gr;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) to[(8 * i + (j & 1)) * PITCH + 8 * (j >> 1)] = acc[i][j];
+      }
+    }
+    ds_parts(r, rec + K0 + warp * 384, lane);
+    float2 gl[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      gl[i] = *reinterpret_cast<const float2*>(rec + GL + warp * 16 + 8 * i + 2 * t4);
+      P[i][0] *= gl[i].x;
+      P[i][1] *= gl[i].y;
+    }
+#pragma unroll
+    for (int w = 0; w < NC; ++w) {
+      float acc[2][4];
+      ds_products<false, true>(acc, v3[w], r);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) S[w][i][j] = fmaf(j & 1 ? gl[i].y : gl[i].x, S[w][i][j], acc[i][j]);
+    }
+    if (OUT && c > 0) finish(c - 1);
+  }
+  if (OUT) {
+    __syncthreads();
+    finish(chunks - 1);
+  }
+  float* dst = OUT ? Sg : a.ends + tile * Dv;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int d0 = warp * 16 + 8 * i + 2 * t4;
+    if (!OUT || last) {
+#pragma unroll
+      for (int w = 0; w < NC; ++w)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int d = d0 + (j & 1), col = col0 + 16 * w + gr + 8 * (j >> 1);
+          if (d < D && col < Dv) dst[(long)d * Dv + col] = S[w][i][j];
+        }
+    }
+    if (!OUT && blockIdx.y == 0 && gr == 0) {
+      if (d0 < D) a.products[tile + d0] = P[i][0];
+      if (d0 + 1 < D) a.products[tile + d0 + 1] = P[i][1];
+    }
+  }
+}
+
+template <int DP>
+static cudaError_t launch_segments(const ScanArgs& a, int num_tokens, int segments, bool cut, uint32_t* records,
+                                   cudaStream_t stream) {
+  constexpr size_t ends_smem = sizeof(uint32_t) * SC_STAGES * (25 * DP + 4 + SC_TILES * 128);
+  constexpr size_t smem = sizeof(uint32_t) * (SC_STAGES * (SC_REC(DP) + SC_TILES * 128) + 2 * DP / 16 * SC_C * (16 * SC_TILES + 4));
+  auto ends = scan_chunk_states_kernel<DP, false>, scan = scan_chunk_states_kernel<DP, true>;
   static bool configured_on[Q3_MAX_DEVICES];
   bool& configured = configured_on[q3_current_device()];
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(segment_scan_kernel<DP, CG, false, BONUS>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(segment_scan_kernel<DP, CG, true, BONUS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(ends, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ends_smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  const dim3 grid((unsigned)segments, (unsigned)((a.Dv + 8 * CG - 1) / (8 * CG)), (unsigned)a.H), block(DP / 4 * CG);
-  const long elements = (long)num_tokens * a.H * DP;
-  cudaError_t e = launch_pdl(segment_rows_kernel<DP>, dim3((unsigned)((elements + 255) / 256)), dim3(256), 0, stream, a,
-                             elements);
-  if (e == cudaSuccess && cut) {
-    e = launch_pdl(segment_scan_kernel<DP, CG, false, BONUS>, grid, block, smem, stream, a);
+  const dim3 grid((unsigned)segments, (unsigned)((a.Dv + 16 * SC_TILES - 1) / (16 * SC_TILES)), (unsigned)a.H), block(2 * DP);
+  cudaError_t e = launch_pdl(scan_chunk_rows_kernel<DP>, dim3((unsigned)(num_tokens / SC_C + a.num_seqs), (unsigned)a.H),
+                             dim3(2 * DP), 0, stream, a, records);
+  if (e != cudaSuccess) return e;
+  // Neither pass is a dependent launch: its blocks would start between those of the kernel before and crowd some SMs while others
+  // stay empty (a prompt of 2048 tokens, 16 heads of 64 x 128, segments of 1024: the second pass 101 us).
+  if (cut) {
+    ends<<<grid, block, ends_smem, stream>>>(a, records);
+    e = cudaGetLastError();
     if (e == cudaSuccess)
       e = launch_pdl(segment_join_kernel, dim3((unsigned)((a.D * a.Dv + 255) / 256), (unsigned)a.H, (unsigned)a.num_seqs),
                      dim3(256), 0, stream, a);
+    if (e != cudaSuccess) return e;
   }
-  if (e != cudaSuccess) return e;
-  if (cut) return launch_pdl(segment_scan_kernel<DP, CG, true, BONUS>, grid, block, smem, stream, a);
-  // Not as a dependent launch right behind the rows: its few blocks would start between those of the rows kernel, two on
-  // some SMs while others have none (one prompt of 64 tokens, 16 heads: 45 us instead of 30).
-  segment_scan_kernel<DP, CG, true, BONUS><<<grid, block, smem, stream>>>(a);
+  scan<<<grid, block, smem, stream>>>(a, records);
   return cudaGetLastError();
 }
 
-// The same arguments as q3_decayed_state_scan, bfloat16, key sizes up to 128: in segments of `seg` tokens.  segments: the
-// number of them, sum over the sequences of ceil(tokens / seg), or more; cut: whether a sequence may have more than one;
-// scratch: fp32, 16-byte aligned, num_tokens * H * 3 * DP with DP = 64 (D <= 64) or 128, and if cut segments * H * D *
-// (Dv + 1) more.
+// The same arguments as q3_decayed_state_scan, bfloat16, key sizes up to 128: in segments of `seg` tokens, a multiple of 16.
+// segments: the number of them, sum over the sequences of ceil(tokens / seg), or more; cut: whether a sequence may have more than
+// one; scratch: 32-bit words, 16-byte aligned, (num_tokens / 16 + num_seqs) * H * (388 + 49 * DP + 256 * ceil(Dv / 32)) with
+// DP = 64 (D <= 64) or 128, and if cut segments * H * D * (Dv + 1) more.
 Q3_EXPORT int q3_decayed_segment_scan(int dtype, const void* q, long q_stride, const void* k, long k_stride, const void* v,
                                       long v_stride, const void* z, long z_stride, const float* z_bias, float inv_tau,
                                       const float* head_decay, const float* inv_freq, int rot_pairs, const int* positions,
@@ -592,7 +817,7 @@ Q3_EXPORT int q3_decayed_segment_scan(int dtype, const void* q, long q_stride, c
                                       int decay_mode, const float* tok_decay, const float* tok_kscale, int ones_col,
                                       const float* bonus, int seg, int segments, int cut, float* scratch,
                                       int num_tokens, cudaStream_t stream) {
-  if (!q || !k || !v || !state || !cu_seqlens || !state_slots || !out || !scratch || seg < 1 || segments < 1 ||
+  if (!q || !k || !v || !state || !cu_seqlens || !state_slots || !out || !scratch || seg < 1 || seg % SC_C || segments < 1 ||
       num_tokens < 0 || ((uintptr_t)scratch & 15))
     return Q3_ERR_ARGUMENT;
   if (!z && !head_decay && !tok_decay) return Q3_ERR_ARGUMENT;
@@ -601,18 +826,14 @@ Q3_EXPORT int q3_decayed_segment_scan(int dtype, const void* q, long q_stride, c
   if (H < 1 || D < 1 || Dv < 1 || H > 65535 || num_seqs > 65535) return Q3_ERR_ARGUMENT;
   if (D > 128 || dtype != Q3_DTYPE_BF16) return Q3_ERR_UNSUPPORTED;
   if (num_seqs == 0 || num_tokens == 0) return Q3_OK;
-  const long rows = (long)num_tokens * H * 3 * (D <= 64 ? 64 : 128);
+  const int DP = D <= 64 ? 64 : 128;
+  float* ends = scratch + ((long)num_tokens / SC_C + num_seqs) * H * (SC_REC(DP) + SC_VALUES(Dv));
+  uint32_t* records = reinterpret_cast<uint32_t*>(scratch);
   const ScanArgs a = {q, k, v, z, q_stride, k_stride, v_stride, z_stride, z_bias, inv_tau, head_decay, inv_freq, rot_pairs,
                       positions, q_scale, k_scale, state, cu_seqlens, state_slots, out, num_seqs, H, D, Dv, decay_mode,
-                      tok_decay, tok_kscale, ones_col, bonus, seg, scratch + rows, scratch + rows + (long)segments * H * D * Dv,
-                      scratch};
-  cudaError_t e;
-  if (D <= 64)
-    e = bonus ? launch_segments<64, 16, true>(a, num_tokens, segments, cut, stream)
-              : launch_segments<64, 16, false>(a, num_tokens, segments, cut, stream);
-  else
-    e = bonus ? launch_segments<128, 8, true>(a, num_tokens, segments, cut, stream)
-              : launch_segments<128, 8, false>(a, num_tokens, segments, cut, stream);
+                      tok_decay, tok_kscale, ones_col, bonus, seg, ends, ends + (long)segments * H * D * Dv};
+  const cudaError_t e = DP == 64 ? launch_segments<64>(a, num_tokens, segments, cut, records, stream)
+                                 : launch_segments<128>(a, num_tokens, segments, cut, records, stream);
   return e == cudaSuccess ? Q3_OK : Q3_ERR_LAUNCH;
 }
 

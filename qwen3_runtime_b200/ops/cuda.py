@@ -290,8 +290,9 @@ class _Span:
 # ---- decayed state scans of bfloat16 steps: token by token or in segments -------------------------
 SCAN_SCRATCH = 1 << 28  # floats a segment scan may ask for (1 GiB)
 
-# Times in us of the two scans (csrc/linear_state.cu) on a B200, by the padded key size: least squares over 48 compositions
-# of sequences (one token to 8,000, alone, in equal numbers and mixed, up to 128 of them) x 6 head counts and sizes x up to 10
+# Times in us of the scan token by token and of segments run token by token, by the padded key size: what cutting has to win by.
+# (Segments are run in chunks now, which takes 0.55 to 0.75 of these times, see CHUNK_COSTS.)  Least squares over 48 compositions of
+# sequences (one token to 8,000, alone, in equal numbers and mixed, up to 128 of them) x 6 head counts and sizes x up to 10
 # segment lengths; 8 % off on average.  A pass of the segments takes the longer of one block's chain (`alone` per token)
 # and all blocks at two per SM (`shared` per token, `block` per block); rows and joining cost `row` and `join` more, and
 # without a cut the first pass's launch is saved (`whole`).  The scan token by token takes the longer of the longest sequence
@@ -304,14 +305,26 @@ SCAN_COSTS = {
 }
 
 
+# Times in us of the segments in chunks of 16 tokens (csrc/linear_state.cu) on a B200, by the padded key size: least squares over
+# 19 compositions x 5 head counts and sizes x up to 11 segment lengths, 5 % off on average; the length that they choose is 1.2 %
+# slower than the best on average, 13 % at worst.  `row` per (chunk, head); a pass takes the chain of one segment (`alone` per chunk)
+# and all blocks' work (`shared` per chunk, `block` per block, on an SM); joining costs `join` and `state` per million values.
+CHUNK_COSTS = {
+    64: dict(row=0.0103, out=(0.70, 0.292, 0.76), ends=(0.35, 0.152, 0.0), join=5.4, state=3.6),
+    128: dict(row=0.0186, out=(0.64, 0.710, 1.40), ends=(0.48, 0.258, 0.0), join=3.9, state=3.6),
+}
+
+
 def _scan_blocks(H, D, Dv):
     """Blocks of one segment: (head, tile of value columns)."""
     return H * -(-Dv // (128 if D <= 64 else 64))
 
 
-def _scan_scratch(T, H, D, Dv, segments, cut):
-    """Floats of a segment scan: a token's rows, and where sequences are cut the segments' states and decays."""
-    return T * H * 3 * (64 if D <= 64 else 128) + (segments * H * D * (Dv + 1) if cut else 0)
+def _scan_scratch(T, num_seqs, H, D, Dv, segments, cut):
+    """Floats of a segment scan: the records of its chunks of 16 tokens, and where sequences are cut the segments' states and
+    decays."""
+    record = 388 + 49 * (64 if D <= 64 else 128) + 256 * -(-Dv // 32)
+    return (T // 16 + num_seqs) * H * record + (segments * H * D * (Dv + 1) if cut else 0)
 
 
 def _segments(cu, seg):
@@ -360,13 +373,42 @@ def decayed_scan_segment(cu, H, D, Dv, sms) -> int:
             break
         count = sum(-(-n // seg) for n in lens)
         more = sum(-(-n // seg) - 1 for n in lens if n)
-        if _scan_scratch(T, H, D, Dv, count, more > 0) > SCAN_SCRATCH:
+        if _scan_scratch(T, len(lens), H, D, Dv, count, more > 0) > SCAN_SCRATCH:
             continue
         cost = c["row"] * T * H * (64 if D <= 64 else 128) + one_pass(T, count, min(seg, longest), *c["out"])
         cost += c["join"] + one_pass(more * seg, more, seg, *c["ends"]) if more else -c["whole"]
         if seg == one_wave:  # its blocks end together, which the model does not see
             cost *= 0.88
         if cost < best:
+            best, found = cost, seg
+    return found
+
+
+@functools.lru_cache(maxsize=256)
+def chunk_segment(cu, H, D, Dv, sms, seg) -> int:
+    """Tokens per segment, a multiple of 16, of a step that is to be cut (``seg`` of :func:`decayed_scan_segment`: one of the lengths
+    looked at), whichever the measured costs make the fastest.  16 heads of 64 x 128, us in segments of 32 / 128 / 256 / 512 tokens /
+    uncut: 2048 tokens 112 / 85 / 83 / 91 / 136; 8 prompts of 256 112 / 89 / 65; 4 heads, 2048 52 / 42 / 48 / 67 / 118."""
+    lens = [b - a for a, b in zip(cu, cu[1:])]
+    T, longest = sum(lens), max(lens)
+    c = CHUNK_COSTS[64 if D <= 64 else 128]
+    blocks = H * -(-Dv // 32) / sms
+    chunks = sum(-(-n // 16) for n in lens)
+
+    def one_pass(chunks, count, last, alone, shared, block):
+        return alone * last + (shared * chunks + block * count) * blocks
+
+    best, found = None, seg
+    for seg in sorted({-(-n // 16) * 16 for n in (32, 64, 96, 128, 192, 256, 512, 1024, seg, longest) if n <= longest}):
+        count = sum(-(-n // seg) for n in lens)
+        more = sum(-(-n // seg) - 1 for n in lens if n)
+        if _scan_scratch(T, len(lens), H, D, Dv, count, more > 0) > SCAN_SCRATCH:
+            continue
+        cost = c["row"] * chunks * H + one_pass(chunks, count, min(seg, longest) / 16, *c["out"])
+        if more:
+            cost += c["join"] + c["state"] * 1e-6 * count * H * D * Dv
+            cost += one_pass(more * seg / 16, more, seg / 16, *c["ends"])
+        if best is None or cost < best:
             best, found = cost, seg
     return found
 
@@ -822,9 +864,11 @@ class CudaOps:
         cu = tuple(host_cu_seqlens) if host_cu_seqlens else None
         seg = self._scan_segment(T, int(num_seqs), H, D, Dv, cu) if q.dtype == torch.bfloat16 else 0
         if seg:
+            seg = -(-seg // 16) * 16  # whole chunks
             segments, longest = _segments(cu, seg) if cu else (T // seg + int(num_seqs), T)
             try:
-                scratch = torch.empty(_scan_scratch(T, H, D, Dv, segments, longest > seg), dtype=torch.float32, device=q.device)
+                scratch = torch.empty(_scan_scratch(T, int(num_seqs), H, D, Dv, segments, longest > seg), dtype=torch.float32,
+                                      device=q.device)
             except torch.OutOfMemoryError:
                 seg = 0  # token by token needs none
         if seg:
@@ -842,9 +886,10 @@ class CudaOps:
         if not self.scan_segments or D > 128:
             return 0
         if cu:
-            return decayed_scan_segment(cu, H, D, Dv, self.SM_COUNT)
+            seg = decayed_scan_segment(cu, H, D, Dv, self.SM_COUNT)
+            return chunk_segment(cu, H, D, Dv, self.SM_COUNT, seg) if seg else 0
         seg = max(32, -(-T // max(1, 2 * self.SM_COUNT // _scan_blocks(H, D, Dv))))
-        if T < max(64, 8 * num_seqs) or _scan_scratch(T, H, D, Dv, T // seg + num_seqs, True) > SCAN_SCRATCH:
+        if T < max(64, 8 * num_seqs) or _scan_scratch(T, num_seqs, H, D, Dv, T // seg + num_seqs, True) > SCAN_SCRATCH:
             return 0
         return seg
 

@@ -164,3 +164,19 @@ def test_single_tokens_beside_one_delta_prompt_stay_out_of_its_chunks():
     assert long([2000] + [1] * 4) == long([1] * 10 + [2000] + [1] * 10) == 1 and long([1, 700], 8) == 1
     assert long([1000] + [1] * 40) == 41 and long([2000] + [1] * 4, 32) == 5 and long([1500, 548, 1]) == 3
     assert long([1500, 548]) == 2 and long([2048]) == 1 and ops._delta_long(None, 7, 16, 128) == 7
+
+
+def test_segments_are_whole_chunks_of_a_measured_length():
+    from qwen3_runtime_b200.ops.cuda import SCAN_SCRATCH, _scan_scratch, _segments, chunk_segment
+
+    for lens in ([2048], [2040] + [1] * 31, [256] * 8, [64] * 32, [17] * 100, [1000, 33, 0, 700], [4000] * 4):
+        for heads, dim, vdim in ((4, 64, 128), (16, 64, 128), (16, 128, 128), (64, 128, 128)):
+            for seg in (32, 114, 2000):
+                got = chunk_segment(_cu(lens), heads, dim, vdim, 148, seg)
+                assert got == seg or (got % 16 == 0 and 16 <= got < max(lens) + 16)
+                count, longest = _segments(_cu(lens), got)
+                if got != seg:
+                    assert _scan_scratch(sum(lens), len(lens), heads, dim, vdim, count, longest > got) <= SCAN_SCRATCH
+    # many blocks need no cut, few heads short segments
+    assert chunk_segment(_cu([256] * 8), 16, 64, 128, 148, 128) == 256 and chunk_segment(_cu([64] * 32), 16, 64, 128, 148, 64) == 64
+    assert chunk_segment(_cu([2048]), 4, 64, 128, 148, 32) < chunk_segment(_cu([2048]), 16, 64, 128, 148, 114) <= 512
