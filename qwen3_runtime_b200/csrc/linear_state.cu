@@ -395,7 +395,7 @@ segment_join_kernel(const __grid_constant__ ScanArgs a) {
 #define SC_C 16
 #define SC_TILES 2  // of 16 value columns, in a block
 #define SC_STAGES 2
-#define SC_REC(DP) (388 + (DP) * 49)  // a record before its values
+#define SC_REC(DP) (416 + (DP) * 49)  // a record before its values, whole lines of 128 bytes
 #define SC_VALUES(Dv) (((Dv) + 16 * SC_TILES - 1) / (16 * SC_TILES) * SC_TILES * 128)
 
 __device__ __forceinline__ void sc_copy16(void* dst, const void* src) {
@@ -588,21 +588,19 @@ scan_chunk_rows_kernel(const __grid_constant__ ScanArgs a, uint32_t* __restrict_
   if (tid == 0) rec[384 + 49 * DP] = odd;
 }
 
-// The chunk's own share of a thread's outputs, as ds_products orders them, where values are not finite: a weight of zero is no
-// reason to touch an earlier token's output.  rec: the weights' parts; v: the column tile's values.
-__device__ __noinline__ void own_tokens(float* own, const uint32_t* rec, const uint32_t* v, int lane) {
-  for (int x = 0; x < 8; ++x) {
-    const int t = 8 * (x >> 2) + 2 * (lane & 3) + (x & 1), col = (lane >> 2) + 4 * (x & 2);
-    float sum = 0.f;
-    for (int j = 0; j <= t; ++j) {
-      const int at = (((t & 7) * 4 + ((j & 7) >> 1)) << 2) + 2 * (t >> 3) + (j >> 3), shift = j & 1 ? 0 : 16;
-      float w = 0.f;
-      for (int m = 2; m >= 0; --m) w += __uint_as_float((rec[m * 128 + at] << shift) & 0xffff0000u);
-      const uint32_t pair = v[(((col & 7) * 4 + ((j & 7) >> 1)) << 2) + 2 * (j >> 3) + (col >> 3)];
-      sum = fmaf(w, __uint_as_float((pair << shift) & 0xffff0000u), sum);
-    }
-    own[x] = sum;
+// The chunk's own share of an output (element x of a thread's eight, as ds_products orders them) where values are not finite: a
+// weight of zero is no reason to touch an earlier token's output.  rec: the weights' parts; v: the column tile's values.
+__device__ __noinline__ float own_token(const uint32_t* rec, const uint32_t* v, int x) {
+  const int lane = threadIdx.x & 31, t = 8 * (x >> 2) + 2 * (lane & 3) + (x & 1), col = (lane >> 2) + 4 * (x & 2);
+  float sum = 0.f;
+  for (int j = 0; j <= t; ++j) {
+    const int at = (((t & 7) * 4 + ((j & 7) >> 1)) << 2) + 2 * (t >> 3) + (j >> 3), shift = j & 1 ? 0 : 16;
+    float w = 0.f;
+    for (int m = 2; m >= 0; --m) w += __uint_as_float((rec[m * 128 + at] << shift) & 0xffff0000u);
+    const uint32_t pair = v[(((col & 7) * 4 + ((j & 7) >> 1)) << 2) + 2 * (j >> 3) + (col >> 3)];
+    sum = fmaf(w, __uint_as_float((pair << shift) & 0xffff0000u), sum);
   }
+  return sum;
 }
 
 template <int DP, bool OUT>
@@ -712,11 +710,11 @@ scan_chunk_states_kernel(const __grid_constant__ ScanArgs a, const uint32_t* __r
         if (warp == w) {  // this warp's share has the chunk's own tokens too
           uint32_t b3[3][4];
           float own[2][4];
+          ds_parts(b3, rec, lane);
+          ds_products<false, true>(own, v3[w], b3);
           if (rec[GL + DP]) {
-            own_tokens(&own[0][0], rec, rec + HEAD + w * 128, lane);
-          } else {
-            ds_parts(b3, rec, lane);
-            ds_products<false, true>(own, v3[w], b3);
+#pragma unroll
+            for (int x = 0; x < 8; ++x) own[x >> 2][x & 3] = own_token(rec, rec + HEAD + w * 128, x);
           }
 #pragma unroll
           for (int i = 0; i < 2; ++i)
@@ -776,7 +774,7 @@ scan_chunk_states_kernel(const __grid_constant__ ScanArgs a, const uint32_t* __r
 template <int DP>
 static cudaError_t launch_segments(const ScanArgs& a, int num_tokens, int segments, bool cut, uint32_t* records,
                                    cudaStream_t stream) {
-  constexpr size_t ends_smem = sizeof(uint32_t) * SC_STAGES * (25 * DP + 4 + SC_TILES * 128);
+  constexpr size_t ends_smem = sizeof(uint32_t) * SC_STAGES * (25 * DP + 32 + SC_TILES * 128);
   constexpr size_t smem = sizeof(uint32_t) * (SC_STAGES * (SC_REC(DP) + SC_TILES * 128) + 2 * DP / 16 * SC_C * (16 * SC_TILES + 4));
   auto ends = scan_chunk_states_kernel<DP, false>, scan = scan_chunk_states_kernel<DP, true>;
   static bool configured_on[Q3_MAX_DEVICES];
@@ -807,7 +805,7 @@ static cudaError_t launch_segments(const ScanArgs& a, int num_tokens, int segmen
 
 // The same arguments as q3_decayed_state_scan, bfloat16, key sizes up to 128: in segments of `seg` tokens, a multiple of 16.
 // segments: the number of them, sum over the sequences of ceil(tokens / seg), or more; cut: whether a sequence may have more than
-// one; scratch: 32-bit words, 16-byte aligned, (num_tokens / 16 + num_seqs) * H * (388 + 49 * DP + 256 * ceil(Dv / 32)) with
+// one; scratch: 32-bit words, 16-byte aligned, (num_tokens / 16 + num_seqs) * H * (416 + 49 * DP + 256 * ceil(Dv / 32)) with
 // DP = 64 (D <= 64) or 128, and if cut segments * H * D * (Dv + 1) more.
 Q3_EXPORT int q3_decayed_segment_scan(int dtype, const void* q, long q_stride, const void* k, long k_stride, const void* v,
                                       long v_stride, const void* z, long z_stride, const float* z_bias, float inv_tau,

@@ -323,7 +323,7 @@ def _scan_blocks(H, D, Dv):
 def _scan_scratch(T, num_seqs, H, D, Dv, segments, cut):
     """Floats of a segment scan: the records of its chunks of 16 tokens, and where sequences are cut the segments' states and
     decays."""
-    record = 388 + 49 * (64 if D <= 64 else 128) + 256 * -(-Dv // 32)
+    record = 416 + 49 * (64 if D <= 64 else 128) + 256 * -(-Dv // 32)
     return (T // 16 + num_seqs) * H * record + (segments * H * D * (Dv + 1) if cut else 0)
 
 
