@@ -170,6 +170,10 @@ _loaded: dict[str, ctypes.CDLL] = {}
 _lock = threading.Lock()
 
 
+def is_loaded(group: str) -> bool:
+    return group in _loaded
+
+
 def load_group(group: str) -> ctypes.CDLL:
     with _lock:
         lib = _loaded.get(group)

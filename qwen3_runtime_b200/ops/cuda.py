@@ -471,11 +471,12 @@ class CudaOps:
         self.timing: list | None = None
         self._cost = (0, 0, "")
         if groups:
-            build.compile_groups([g for g in groups])
+            build.compile_groups([g for g in groups if not build.is_loaded(g)])
 
     def prepare(self, groups: list[str]) -> None:
         """Compile (in parallel) the kernel groups a model is going to use."""
-        build.compile_groups([g for g in groups if g in _SIGNATURES])
+        # (what this process has loaded stays loaded, so its sources need not be read and hashed for every table: 0.5 ms and more)
+        build.compile_groups([g for g in groups if g in _SIGNATURES and not build.is_loaded(g)])
 
     # ---- plumbing -------------------------------------------------------------------
     def _get(self, group: str, name: str):
