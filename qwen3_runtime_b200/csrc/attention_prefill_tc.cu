@@ -386,10 +386,19 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
         __syncwarp();
         arrive_if(lane == 0, bar(BAR_S_EMPTY + x));  // S_(j+1) may come
         if constexpr (EDGE) {
+          if (key0 + BLOCK_N - 1 > pos) {  // the tile crosses this row's diagonal
 #pragma unroll
-          for (int c = 0; c < 32; ++c) {
-            if (key0 + c > pos || key0 + c < lo) sa[c] = 0xff800000u;  // -inf
-            if (key0 + 32 + c > pos || key0 + 32 + c < lo) sb[c] = 0xff800000u;
+            for (int c = 0; c < 32; ++c) {
+              if (key0 + c > pos) sa[c] = 0xff800000u;  // -inf
+              if (key0 + 32 + c > pos) sb[c] = 0xff800000u;
+            }
+          }
+          if (key0 < lo) {  // keys of an earlier chunk, or before the window
+#pragma unroll
+            for (int c = 0; c < 32; ++c) {
+              if (key0 + c < lo) sa[c] = 0xff800000u;
+              if (key0 + 32 + c < lo) sb[c] = 0xff800000u;
+            }
           }
         }
         float mx;
@@ -465,11 +474,10 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
       const int row_first = row0[x], row_last = min(rows, row0[x] + BLOCK_M) - 1;
       const int pos_first = base_pos + row_first / G, pos_last = base_pos + row_last / G;
       const int lo_last = chunk > 0 ? pos_last / chunk * chunk : (window > 0 ? max(0, pos_last - window + 1) : 0);
-      int whole0 = 1, whole1 = 0;  // such tiles behind the first one
-      if (row0[x] + BLOCK_M <= rows) {  // (rows that are none see nothing)
-        whole0 = max(1, (max(lo_last, k_lo) + BLOCK_N - 1) / BLOCK_N - tile0);
-        whole1 = min(my_tiles, (pos_first + 1) / BLOCK_N - tile0);
-      }
+      // (What rows that are none see in a last block has no say: nothing of theirs is stored.  A last block that goes through tiles with
+      // masks only is the longest of its sequence: 32 heads over 8, 500 tokens behind 3000, 76 us; so 64.)
+      const int whole0 = max(1, (max(lo_last, k_lo) + BLOCK_N - 1) / BLOCK_N - tile0);
+      const int whole1 = min(my_tiles, (pos_first + 1) / BLOCK_N - tile0);  // such tiles behind the first one
       bool ok = true;
       for (int j = 0; j < my_tiles && ok; ++j) {
         if (j < whole0 || j >= whole1) {
