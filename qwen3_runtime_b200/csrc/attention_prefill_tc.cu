@@ -138,7 +138,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
   constexpr int KV_STAGES = Z::STAGES, Q_BYTES = Z::Q_BYTES, K_BYTES = Z::K_BYTES, DK = Z::DK;
   enum { BAR_Q = 0, BAR_K_FULL = 1, BAR_K_EMPTY = BAR_K_FULL + KV_STAGES, BAR_V_FULL = BAR_K_EMPTY + KV_STAGES,
          BAR_V_EMPTY = BAR_V_FULL + KV_STAGES, BAR_S_FULL = BAR_V_EMPTY + KV_STAGES,  // [block], like the rest
-         BAR_S_EMPTY = BAR_S_FULL + 2, BAR_P_FULL = BAR_S_EMPTY + 2, BAR_PV_FULL = BAR_P_FULL + 2, NUM_BARS = BAR_PV_FULL + 2 };
+         BAR_S_EMPTY = BAR_S_FULL + 2, BAR_P_FULL = BAR_S_EMPTY + 2, BAR_PV_FULL = BAR_P_FULL + 2,
+         BAR_END = BAR_PV_FULL + 2, NUM_BARS = BAR_END + 4 };
   const int *block_table = p.block_table, *cu_seqlens = p.cu_seqlens;
   const int max_pages = p.max_pages, nq = p.nq, nkv = p.nkv, ps = p.ps, chunk = p.chunk, window = p.window;
   const float scale_log2 = p.scale_log2;
@@ -191,6 +192,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
       mbar_init(bar(BAR_P_FULL + i), 4);
       mbar_init(bar(BAR_PV_FULL + i), 1);
     }
+    for (int i = 0; i < 4; ++i) mbar_init(bar(BAR_END + i), 1);  // the issuers
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 12) {
@@ -260,7 +262,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
         return in ? bt[pi] : -1;
       };
       int next = MODE == DENSE ? 0 : page_of(0);
-      int st = 0;
+      int st = 0, issued = 0;
       uint32_t phase = 1;
       for (int j = 0; j < num_tiles; ++j) {
         const int page = next;
@@ -272,6 +274,9 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
         }
         if (!__all_sync(0xffffffffu, mbar_wait(empty + 8 * st, phase, &abort_flag))) break;
         if (lane == 0) mbar_expect_tx(full + 8 * st, bytes);
+#ifdef Q3_TEST_WITHHOLD_A_BOX  // (a test build leaves one half of the keys' boxes out: the stage never fills, a wait runs out)
+        if (part != 1)
+#endif
         if (MODE == DENSE) {
           if (lane == 0) {
             const int y = row_base + (tile0 + j) * BLOCK_N;
@@ -285,6 +290,13 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
           }
         }
         if (++st == KV_STAGES) st = 0, phase ^= 1;
+        ++issued;
+      }
+      // The last boxes may still be in flight when the others have given up.  (Then a stage that the other producer did not come to
+      // any more is waited for until the limit.)
+      if (lane == 0) {
+        if (part == 3) mbar_wait_drain(bar(BAR_Q), 0);
+        for (int j = max(0, issued - KV_STAGES); j < issued; ++j) mbar_wait_drain(full + 8 * (j % KV_STAGES), (j / KV_STAGES) & 1);
       }
     } else if (warp > 11) {
       // ---- MMA issuers: warps 12 and 13 for S of block A and B, warps 14 and 15 for PV ---------
@@ -318,8 +330,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
                 umma_bf16(tmem_x, umma_desc(q_addr + half * HALF_Q) + sub,
                      umma_desc(k_addr + (MODE == MAPS ? x : half) * HALF_KV) + sub, idesc, k > 0 ? 1u : 0u);
               }
-              umma_commit(bar(BAR_S_FULL + x));    // S_j is in TMEM
               umma_commit(bar(BAR_K_EMPTY + st));  // this block is done with the key tile
+              umma_commit(bar(BAR_S_FULL + x));    // S_j is in TMEM
             } else {
               mbar_arrive(bar(BAR_K_EMPTY + st));
             }
@@ -341,8 +353,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
               for (int k = 0; k < BLOCK_N / 16; ++k)  // 16 keys: 8 columns of P, 2 KB down V's rows
                 umma_bf16_tmem(tmem_x + TMEM_O, tmem_x + TMEM_P + (j & 1) * (BLOCK_N / 2) + 8 * k,
                      umma_desc_mn_major(v_addr + k * 2048, HALF_KV), idesc, (j > 0 || k > 0) ? 1u : 0u);
-              umma_commit(bar(BAR_PV_FULL + x));
               umma_commit(bar(BAR_V_EMPTY + st));
+              umma_commit(bar(BAR_PV_FULL + x));
             } else {
               mbar_arrive(bar(BAR_V_EMPTY + st));
             }
@@ -351,7 +363,12 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
           if (++st == KV_STAGES) st = 0, phase ^= 1;
         }
       }
-    } else {  // ---- softmax: one thread per row; warps 2..5 block A, warps 6..9 block B ---------------
+      if (leader) {  // nothing of this issuer's is in flight any more when the tensor memory is freed
+        umma_commit(bar(BAR_END + role - 12));
+        mbar_wait_drain(bar(BAR_END + role - 12), 0);
+      }
+      __syncwarp();
+    } else {  // ---- softmax: one thread per row; warps 4..7 block A, warps 8..11 block B -------------
       const int x = (warp - 4) >> 2;
       const int quarter = warp & 3;
       const int r = quarter * 32 + lane;  // row of the tile = TMEM lane

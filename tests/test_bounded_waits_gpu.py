@@ -1,0 +1,66 @@
+"""Waits that run out: second builds of kernels, under other names and with short limits (about 1 ms for a wait, 10 ms for the wait
+on what is still in flight), leave boxes out, so that a stage's barrier is a flag that nothing sets.  The kernel must come back by
+itself with its error word set, and the context must stay usable."""
+
+from __future__ import annotations
+
+import ctypes
+import math
+
+import pytest
+import torch
+
+import test_kernels_gpu as tk
+
+pytestmark = pytest.mark.gpu
+
+DEFINES = ("-DQ3_WAIT_LIMIT_CYCLES=2000000ll", "-DQ3_DRAIN_LIMIT_CYCLES=20000000ll", "-DQ3_TEST_WITHHOLD_A_BOX")
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from qwen3_runtime_b200.ops.cuda import CudaOps
+
+    return CudaOps()
+
+
+def _build(group, name):
+    from qwen3_runtime_b200.ops import build
+    from qwen3_runtime_b200.ops.cuda import _SIGNATURES
+
+    fn = getattr(ctypes.CDLL(str(build.compile_group(group, variant="_withheld_box", defines=DEFINES))), name)
+    fn.argtypes, fn.restype = _SIGNATURES[group][name], ctypes.c_int
+    return fn
+
+
+def _expires(fn, *args):
+    """Run fn(..., error word, stream); the error word afterwards."""
+    word = torch.zeros(1, dtype=torch.int32, device="cuda")
+    start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    start.record()
+    code = fn(*args, word.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    stop.record()
+    assert code == 0
+    torch.cuda.synchronize()  # returns: every wait in the kernel is bounded
+    assert start.elapsed_time(stop) < 2000.0
+    return int(word.item())
+
+
+@pytest.mark.parametrize("context,tokens", [(0, 20), (700, 100)])
+def test_prompt_attention(ops, context, tokens):
+    nq, nkv, ps, lens, qlens = 8, 2, 16, [context + tokens], [tokens]
+    pr = tk.attention_problem(nq, nkv, 128, ps, lens, qlens, torch.bfloat16, 11)
+    step = tk.step_for(lens, qlens)
+    out = torch.zeros((tokens, nq * 128), dtype=torch.bfloat16, device="cuda")
+    work = -(-(-(-tokens * nq // nkv // 128)) // 2)
+    scale = 1 / math.sqrt(128)
+    assert _expires(_build("attention_prefill_tc", "q3_paged_attention_prefill_tc"), pr["q"].data_ptr(), pr["q"].stride(0), tokens,
+                    pr["k"].data_ptr(), pr["v"].data_ptr(), pr["k"].numel() // 128, pr["bt"].data_ptr(), pr["bt"].shape[1],
+                    step.kv_lens.data_ptr(), step.cu_seqlens.data_ptr(), out.data_ptr(), 1, work, nq, nkv, 128, ps, scale, 0, 0,
+                    None, None) == 2
+    # the ordinary build of the same kernel gives the right result
+    ops.paged_attention(pr["q"], pr["q"].stride(0), num_heads=nq, num_kv_heads=nkv, head_dim=128, k_pages=pr["k"],
+                        v_pages=pr["v"], block_table=pr["bt"], token_seq=pr["seq"], positions=pr["pos"], out=out,
+                        page_size=ps, scale=scale, window=None, step=step)
+    ops.raise_if_kernel_error()
+    tk.close(out, tk.run_attention(tk.REF, pr, nq, nkv, 128, ps, torch.bfloat16), torch.bfloat16, "after", bf16_tol=1e-2)
