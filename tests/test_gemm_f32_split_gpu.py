@@ -77,3 +77,37 @@ def test_many_rows_in_portions(ops):
     finally:
         del ops.F32_SPLIT_ROWS
     assert torch.equal(got[:, :2560], want) and bool(got[:, 2560:].isnan().all())
+
+
+def _times(ops, calls, n=15):
+    """Median device time of each call, in turn, behind a cold L2."""
+    cold = torch.empty(1 << 26, device="cuda")
+    events = [[(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(n)] for _ in calls]
+    for call in calls:
+        call()
+    for i in range(n):
+        for call, pairs in zip(calls, events):
+            cold.add_(1.0)
+            pairs[i][0].record()
+            call()
+            pairs[i][1].record()
+    torch.cuda.synchronize()
+    return [sorted(a.elapsed_time(b) for a, b in pairs)[n // 2] for pairs in events]
+
+
+def test_values_that_are_no_numbers_cost_little_and_stay_with_their_row(ops):
+    x, w = _matrices(300, 19456, 2560)
+    y, last, v = torch.full_like(x, float("nan")), x.clone(), w.clone()
+    last[7, 2559], last[8, 0] = float("nan"), float("inf")
+    v[3, 1000] = float("nan")
+    finite, one, every, weight = _times(ops, [lambda: ops.linear(x, w), lambda: ops.linear(last, w), lambda: ops.linear(y, w),
+                                              lambda: ops.linear(x, v)], 5)
+    assert max(one, every, weight) <= 8 * finite, (finite, one, every, weight)
+    want = ops.linear(x, w)
+    got = ops.linear(last, w)
+    keep = [i for i in range(300) if i not in (7, 8)]
+    assert got[7].isnan().all() and got[8].isinf().all() and torch.equal(got[keep], want[keep])
+    got = ops.linear(x, v)
+    assert got[:, 3].isnan().all() and torch.equal(got[:, 4:], want[:, 4:]) and torch.equal(got[:, :3], want[:, :3])
+    assert ops.linear(y, w).isnan().all()
+    ops.raise_if_kernel_error()
