@@ -175,19 +175,22 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_con
     bool ok = true;
     for (int i = blockIdx.x; i < p.items && ok; i += gridDim.x) {
       const Item it = item_at(i);
-      for (int c = 0; c < it.count && ok; ++c, ++s) {
+      for (int c = 0; c < it.count; ++c, ++s) {
         const int st = s & 1;
         ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_EMPTY + st), ((s >> 1) & 1) ^ 1, &abort_flag));
-        if (ok && lane == 0) {
+        if (!ok) break;
+        if (lane == 0) {
           mbar_expect_tx(bar(BAR_X_FULL + st), x_stage);
+#ifndef Q3_TEST_WITHHOLD_A_BOX  // (a test build leaves the tokens' boxes out: the stage never fills, a wait runs out)
           for (int q = 0; q < 3; ++q)
             tma_load_3d(x_s + st * x_stage + q * x_part, &xmap, bar(BAR_X_FULL + st), (it.first + c) * SLICE, it.token0, q);
+#endif
         }
       }
     }
-    // after a wait that expired: the boxes in flight
-    if (!ok && lane == 0)
-      for (int b = max(0, s - 3); b < s - 1; ++b) mbar_wait_drain(bar(BAR_X_FULL + (b & 1)), (b >> 1) & 1);
+    // the last boxes may still be in flight when the others have given up
+    if (lane == 0)
+      for (int b = max(0, s - 2); b < s; ++b) mbar_wait_drain(bar(BAR_X_FULL + (b & 1)), (b >> 1) & 1);
   } else if (warp_u == 1) {  // ---- products ----
     // (one lane chosen by elect.sync, in a warp that runs as a whole: descriptors then stay in uniform registers, and an MMA is
     // issued every 37 cycles; chosen by its number 60 to 78)

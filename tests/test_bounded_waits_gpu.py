@@ -64,3 +64,21 @@ def test_prompt_attention(ops, context, tokens):
                         page_size=ps, scale=scale, window=None, step=step)
     ops.raise_if_kernel_error()
     tk.close(out, tk.run_attention(tk.REF, pr, nq, nkv, 128, ps, torch.bfloat16), torch.bfloat16, "after", bf16_tol=1e-2)
+
+
+@pytest.mark.parametrize("rows", [1, 33, 300])
+def test_float32_product(ops, rows):
+    N, K = 19456, 1088
+    w = torch.randn((N, K), device="cuda")
+    x = torch.randn((rows, K), device="cuda")
+    segments = ops._f32_segments(x, w)
+    assert segments > 0
+    parts = torch.zeros(3 * rows * K, dtype=torch.bfloat16, device="cuda")
+    planes = torch.zeros((segments, rows, N), device="cuda")
+    out = torch.zeros((rows, N), device="cuda")
+    assert _expires(_build("gemm_f32", "q3_gemm_f32_split"), x.data_ptr(), K, w.data_ptr(), K, out.data_ptr(), N, rows, N, K,
+                    parts.data_ptr(), planes.data_ptr()) == 2
+    # the ordinary build of the same kernel gives the right result
+    got, want = ops.linear(x, w).double(), x.double() @ w.double().t()
+    ops.raise_if_kernel_error()
+    assert float((got - want).norm() / want.norm()) < 1e-6
