@@ -15,18 +15,27 @@
 //   warps 2..9   weights: 16 bytes of float32 per lane from global memory, a slice ahead in registers, split and written in the
 //                128-byte swizzle; and sums: the accumulators of the slice before (two buffers in tensor memory) into
 //                registers, a row and half of the columns a thread; at the item's end they are stored
-// What bounds it: a slice takes 1900 cycles with few tokens, the weights' way (wait, split, write, the products' hand-over), and
-// 2700 with 160, with the sums' beside it; its 24 products take 900 to 1900 of them.  300 tokens: 19456 x 2560 704 us on the FMA
-// pipes, 236 here; 2560 x 9728 415 and 120.
+// Up to 32 tokens (kernel of its own, the same sums): where few products follow, the weights' loads a slice ahead, 2600 cycles under
+// load, were what a slice waited for.
+//   warp 10      TMA: the weights' slices as they are, up to eight ahead in what shared memory the few tokens leave
+//   warps 2..9   read them from there; an item has 48 to 128 rows, whichever fills the rounds over the SMs
+// What bounds it: with 160 tokens a slice takes 2700 cycles, its 24 products 1900 of them, the sums and the weights' way (wait,
+// split, write, hand-over) the rest; with up to 32 tokens and 128 rows 1800, the weights' way, which is 4.5 TB/s.  us, on the FMA
+// pipes / here: 300 tokens 19456 x 2560 701 / 218, 2560 x 9728 412 / 112; one token 19456 x 2560 82 / 73 (105 without that kernel),
+// 24576 x 4096 129 / 105 (145), 151936 x 2560 383 / 345 (495), 4096 x 12288 111 / 64 (82).
 #include "async_tiles.cuh"
 
 namespace split {
 
-constexpr int ROWS = 128, SLICE = 64, MOST_TOKENS = 160, THREADS = 10 * 32;
+constexpr int ROWS = 128, SLICE = 64, MOST_TOKENS = 160, FEW_TOKENS = 32;
 constexpr int AHEAD = 4;  // slices
 constexpr int W_PART = ROWS * 128, W_STAGE = 3 * W_PART;
-constexpr int smem_bytes(int tokens) { return 2 * (W_STAGE + 3 * tokens * 128) + 1024; }
-enum { BAR_W_FULL = 0, BAR_X_FULL = 2, BAR_EMPTY = 4, BAR_D_FULL = 6, BAR_D_EMPTY = 8, BAR_END = 10, NUM_BARS = 11 };
+constexpr int MOST_RAW = 8;  // few tokens: slices of weights as they are, on their way
+constexpr int threads(int most) { return (most == FEW_TOKENS ? 11 : 10) * 32; }
+constexpr int smem_bytes(int rows, int tokens, int raw) { return 768 * (rows + tokens) + raw * rows * SLICE * 4 + 1024; }
+constexpr int MOST_SMEM = 231936;
+enum { BAR_W_FULL = 0, BAR_X_FULL = 2, BAR_EMPTY = 4, BAR_D_FULL = 6, BAR_D_EMPTY = 8, BAR_END = 10, BAR_RAW_FULL = 11,
+       BAR_RAW_EMPTY = BAR_RAW_FULL + MOST_RAW, NUM_BARS = BAR_RAW_EMPTY + MOST_RAW };
 
 // (x, y) as the sum of three pairs of bfloat16
 __device__ __forceinline__ void parts_of(float x, float y, uint32_t (&p)[3]) {
@@ -66,9 +75,15 @@ struct Args {
   float* out;          // [segments][M][ldc]
   long ldc, plane;
   int M, N, K, segments, slices_per_segment, tokens, token_tiles, items;
+  int rows, raw;  // weight rows of an item: 128, with few tokens a multiple of 16 up to it; slots of the weights' ring
   int* error_word;
 };
 
+__device__ __forceinline__ float4 load_shared4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ void tmem_load8(uint32_t taddr, uint32_t (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
@@ -120,13 +135,20 @@ __device__ __noinline__ void as_float32(const Args& p, float* out, bool open, in
   }
 }
 
-__global__ void __launch_bounds__(THREADS, 1)
-gemm_f32_split_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ Args p) {
+// MOST: tokens that there are registers for.  FEW_TOKENS: the weights come by TMA (warp 10) into a ring of their own.
+template <int MOST>
+__global__ void __launch_bounds__(threads(MOST), 1)
+gemm_f32_split_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
+                      const __grid_constant__ Args p) {
+  constexpr bool FEW = MOST == FEW_TOKENS;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const uint32_t x_part = (uint32_t)p.tokens * 128, x_stage = 3 * x_part;
-  unsigned char* w_s = base;                       // 2 x [3 parts][128 rows][128 B]
-  const uint32_t x_s = smem_addr(base + 2 * W_STAGE);  // 2 x [3 parts][tokens][128 B]
+  // (an MMA reads 128 rows: behind the item's own it finds what follows in shared memory, and makes rows that are not stored)
+  const uint32_t w_part = FEW ? (uint32_t)p.rows * 128 : W_PART, w_stage = 3 * w_part, raw_stage = (uint32_t)p.rows * SLICE * 4;
+  unsigned char* w_s = base;                       // 2 x [3 parts][rows][128 B]
+  const uint32_t x_s = smem_addr(base) + 2 * w_stage;  // 2 x [3 parts][tokens][128 B]
+  const uint32_t raw_s = x_s + 2 * x_stage;            // FEW: p.raw x [rows][256 B]
   __shared__ __align__(8) unsigned long long bars[NUM_BARS];
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile int abort_flag;
@@ -143,6 +165,10 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_con
       mbar_init(bar(BAR_D_EMPTY + i), 8);  // the sums' warps
     }
     mbar_init(bar(BAR_END), 1);
+    for (int i = 0; FEW && i < p.raw; ++i) {
+      mbar_init(bar(BAR_RAW_FULL + i), 1);
+      mbar_init(bar(BAR_RAW_EMPTY + i), 8);  // the weights' warps
+    }
     mbar_init_fence();
   }
   if (warp == 1) {
@@ -163,7 +189,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_con
     it.token0 = (i - rest * p.token_tiles) * p.tokens;
     const int tile = rest / p.segments;
     it.segment = rest - tile * p.segments;
-    it.row0 = tile * ROWS;
+    it.row0 = tile * p.rows;
     it.first = it.segment * p.slices_per_segment;
     it.count = min(p.slices_per_segment, slices - it.first);
     return it;
@@ -191,6 +217,24 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_con
     // the last boxes may still be in flight when the others have given up
     if (lane == 0)
       for (int b = max(0, s - 2); b < s; ++b) mbar_wait_drain(bar(BAR_X_FULL + (b & 1)), (b >> 1) & 1);
+  } else if (FEW && warp_u == 10) {  // ---- few tokens: the weights ----
+    int s = 0, st = 0;
+    uint32_t phase = 1;
+    bool ok = true;
+    for (int i = blockIdx.x; i < p.items && ok; i += gridDim.x) {
+      const Item it = item_at(i);
+      for (int c = 0; c < it.count; ++c, ++s) {
+        ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_RAW_EMPTY + st), phase, &abort_flag));
+        if (!ok) break;
+        if (lane == 0) {
+          mbar_expect_tx(bar(BAR_RAW_FULL + st), raw_stage);
+          tma_load_2d(raw_s + st * raw_stage, &wmap, bar(BAR_RAW_FULL + st), (it.first + c) * SLICE, it.row0);
+        }
+        if (++st == p.raw) st = 0, phase ^= 1;
+      }
+    }
+    if (lane == 0)
+      for (int b = max(0, s - p.raw); b < s; ++b) mbar_wait_drain(bar(BAR_RAW_FULL + b % p.raw), (b / p.raw) & 1);
   } else if (warp_u == 1) {  // ---- products ----
     // (one lane chosen by elect.sync, in a warp that runs as a whole: descriptors then stay in uniform registers, and an MMA is
     // issued every 37 cycles; chosen by its number 60 to 78)
@@ -213,13 +257,13 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_con
                                            mbar_wait(bar(BAR_X_FULL + st), phase, &abort_flag));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint64_t wd = umma_desc(w_addr + st * W_STAGE), xd = umma_desc(x_s + st * x_stage);
+        const uint64_t wd = umma_desc(w_addr + st * w_stage), xd = umma_desc(x_s + st * x_stage);
         const uint32_t acc = tmem_u + st * 256, xp = x_part >> 4;
         if (leader) {
           auto product = [&](int wq, int xq, bool first) {  // 16 k-values are 32 bytes: 2 descriptor units
 #pragma unroll
             for (int k = 0; k < SLICE / 16; ++k)
-              umma_bf16(acc, wd + wq * (W_PART >> 4) + 2 * k, xd + xq * xp + 2 * k, idesc, first && k == 0 ? 0u : 1u);
+              umma_bf16(acc, wd + wq * (w_part >> 4) + 2 * k, xd + xq * xp + 2 * k, idesc, first && k == 0 ? 0u : 1u);
           };
           product(2, 0, true);
           product(0, 2, false);
@@ -241,9 +285,12 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_con
   } else {  // ---- weights and sums ----
     const int worker = warp - 2, quarter = warp & 3, cols = p.tokens / 2, col0 = (worker >> 2) * cols;
     const uint32_t from = tmem + ((uint32_t)(quarter * 32) << 16) + col0;
-    const int r0 = worker * 16 + (lane >> 4), kl = (lane & 15) * 4;
+    // the 16 threads of a row are neighbours; a thread's rows are r0 + STEP i
+    constexpr int STEP = FEW ? 16 : 2;
+    const int r0 = (FEW ? worker * 2 : worker * 16) + (lane >> 4), kl = (lane & 15) * 4;
     unsigned char* const w_dst = w_s + r0 * 128 + (lane & 1) * 8;
-    float4 v[8];  // rows r0 + 2 i, k-values kl .. kl + 3 of the slice that is split next
+    const uint32_t raw = raw_s + r0 * 256 + (lane & 15) * 16;
+    float4 v[8];  // rows r0 + STEP i, k-values kl .. kl + 3 of the slice that is split next
     const float* w_row = p.w;  // the first of those rows
     int rows_left = 0;         // (rows from N on are read as that row, and not stored)
     auto item_rows = [&](const Item& it) {
@@ -264,13 +311,22 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_con
       const int row = it.row0 + (tid - 64 >> 1), k = slice * SLICE + (tid & 1) * 32;
       if (row < p.N && k < p.K) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w + (long)row * p.ldw + k));
     };
-    float sum[MOST_TOKENS / 2];
+    int raw_st = 0;  // FEW: the ring's slot that is read next
+    uint32_t raw_phase = 0;
+    auto load_raw = [&]() -> bool {
+      if (!__all_sync(0xffffffffu, mbar_wait(bar(BAR_RAW_FULL + raw_st), raw_phase, &abort_flag))) return false;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i * 16 < p.rows) v[i] = load_shared4(raw + raw_st * raw_stage + i * 16 * 256);
+      return true;
+    };
+    float sum[MOST / 2];
     auto add = [&](int s) -> bool {  // the accumulators of stage s
       const int st = s & 1;
       if (!__all_sync(0xffffffffu, mbar_wait(bar(BAR_D_FULL + st), (s >> 1) & 1, &abort_flag))) return false;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-      for (int g = 0; g < MOST_TOKENS / 2; g += 16) {
+      for (int g = 0; g < MOST / 2; g += 16) {
         if (g < cols) {
           uint32_t r[2][8];
           tmem_load8(from + st * 256 + g, r[0]);
@@ -289,45 +345,55 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_con
       if (lane == 0) mbar_arrive(bar(BAR_D_EMPTY + st));
       return true;
     };
-    if ((int)blockIdx.x < p.items) {
+    bool ok = true;
+    if (FEW) {
+      ok = load_raw();
+    } else {
       const Item it = item_at(blockIdx.x);
       item_rows(it);
       load(it.first);
       for (int c = 1; c < AHEAD && c < it.count; ++c) ahead(it, it.first + c);
     }
     int s = 0;
-    bool ok = true;
     for (int x = blockIdx.x; x < p.items && ok; x += gridDim.x) {
       const Item it = item_at(x);
       const int after = x + (int)gridDim.x;
       const Item nx = item_at(after < p.items ? after : x);
 #pragma unroll
-      for (int i = 0; i < MOST_TOKENS / 2; ++i) sum[i] = 0.f;
+      for (int i = 0; i < MOST / 2; ++i) sum[i] = 0.f;
       for (int c = 0; c < it.count && ok; ++c, ++s) {
         const int st = s & 1;
         ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_EMPTY + st), ((s >> 1) & 1) ^ 1, &abort_flag));
         if (!ok) break;
-        unsigned char* dst = w_dst + st * W_STAGE;
+        unsigned char* dst = w_dst + st * w_stage;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
+          if (FEW && i * 16 >= p.rows) break;  // (rows beyond stay as they are: a result depends on its own row only)
           uint32_t lo[3], hi[3];
           parts_of(v[i].x, v[i].y, lo);
           parts_of(v[i].z, v[i].w, hi);
-          const int at = i * 256 + ((((lane & 15) >> 1) ^ ((r0 + 2 * i) & 7)) * 16);
+          const int at = i * STEP * 128 + ((((lane & 15) >> 1) ^ ((r0 + STEP * i) & 7)) * 16);
 #pragma unroll
-          for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(dst + q * W_PART + at) = make_uint2(lo[q], hi[q]);
+          for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(dst + q * w_part + at) = make_uint2(lo[q], hi[q]);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(BAR_W_FULL + st));
-        if (c + 1 < it.count) {
-          load(it.first + c + 1);
-        } else if (after < p.items) {
-          item_rows(nx);
-          load(nx.first);
+        if (FEW) {
+          // (given back behind the stores of what they became: an arrival does not wait for loads that are still on their way)
+          if (lane == 0) mbar_arrive(bar(BAR_RAW_EMPTY + raw_st));
+          if (++raw_st == p.raw) raw_st = 0, raw_phase ^= 1;
+          if ((c + 1 < it.count || after < p.items) && !(ok = load_raw())) break;
+        } else {
+          if (c + 1 < it.count) {
+            load(it.first + c + 1);
+          } else if (after < p.items) {
+            item_rows(nx);
+            load(nx.first);
+          }
+          if (c + AHEAD < it.count) ahead(it, it.first + c + AHEAD);
+          else if (after < p.items && c + AHEAD - it.count < nx.count) ahead(nx, nx.first + c + AHEAD - it.count);
         }
-        if (c + AHEAD < it.count) ahead(it, it.first + c + AHEAD);
-        else if (after < p.items && c + AHEAD - it.count < nx.count) ahead(nx, nx.first + c + AHEAD - it.count);
         if (c > 0) ok = add(s - 1);  // while this slice's products run
       }
       if (ok) ok = add(s - 1);
@@ -335,9 +401,9 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_con
       const int row0 = it.row0 + quarter * 32, t0 = it.token0 + col0;
       float* out = p.out + it.segment * p.plane + (long)t0 * p.ldc + row0;
       bool none = false;
-      if (row0 + lane < p.N) {
+      if (quarter * 32 + lane < p.rows && row0 + lane < p.N) {
 #pragma unroll
-        for (int i = 0; i < MOST_TOKENS / 2; ++i) {
+        for (int i = 0; i < MOST / 2; ++i) {
           if (i < cols && t0 + i < p.M) {
             out[(long)i * p.ldc + lane] = sum[i];
             none |= sum[i] != sum[i];
@@ -379,10 +445,10 @@ add_segments(const float* __restrict__ planes, long plane, int segments, float* 
 }
 
 // Segments of K for N features: the fewest slices one after another on 148 SMs at one token tile, against the sums that every
-// segment writes and a second kernel reads.  300 tokens / one, us, with 1, 2, 3, 4, 6, 8 segments (the choice behind the sizes):
-// 19456 x 2560 (2) 249/120, 236/105, 241/103, 253/101, 284/105, 300/107; 24576 x 4096 (3) 398/179, 425/154, 400/146, 431/161,
-// 464/159, 490/166; 4096 x 12288 (4) 286/241, 212/136, 232/101, 220/83, 230/105, 238/89; 2560 x 9728 (7: 120/52) 222/194,
-// 144/112, 124/81, 151/68, 134/54, 146/71.  Of N and K only, whatever the device: the bits depend on it.
+// segment writes and a second kernel reads.  300 tokens, us when this was chosen, with 1, 2, 3, 4, 6, 8 segments (the choice behind
+// the sizes): 19456 x 2560 (2) 249, 236, 241, 253, 284, 300; 24576 x 4096 (3) 398, 425, 400, 431, 464, 490; 4096 x 12288 (4) 286,
+// 212, 232, 220, 230, 238; 2560 x 9728 (7: 120) 222, 144, 124, 151, 134, 146.  Of N and K only, whatever the device: the bits
+// depend on it.
 static inline int segments_of(int N, int K) {
   const int tiles = (N + ROWS - 1) / ROWS, slices = (K + SLICE - 1) / SLICE;
   int best = 1, best_cost = 0;
@@ -396,8 +462,8 @@ static inline int segments_of(int N, int K) {
 }  // namespace split
 
 // Segments the product's K is cut into; 0: not a product for this kernel.  The tokens must have no say in it, so the line is
-// where few tokens do not lose: weights of 20 M values (one token, us, here / FMA: 2560 x 9728 52 / 89, 4096 x 12288 83 / 112,
-// 19456 x 2560 105 / 85, 24576 x 4096 146 / 132, hence 157 / 174 and 229 / 244 for a feed-forward; 6144 x 2560 60 / 38).
+// where few tokens do not lose: weights of 20 M values (one token, us, here / FMA: 8192 x 2560 38 / 41, 7680 x 2688 38 / 43,
+// 12288 x 2048 44 / 43, 5120 x 5120 44 / 64, 2560 x 9728 42 / 88).
 Q3_EXPORT int q3_gemm_f32_split_segments(int N, int K) {
   return N < 256 || N % 4 || K < 1024 || K % 8 || (long)N * K < 20000000 ? 0 : split::segments_of(N, K);
 }
@@ -417,8 +483,10 @@ Q3_EXPORT int q3_gemm_f32_split(const float* A, int lda, const float* W, int ldw
   if (!sms_on[device]) {
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
-        cudaFuncSetAttribute(gemm_f32_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(MOST_TOKENS)) !=
-            cudaSuccess)
+        cudaFuncSetAttribute(gemm_f32_split_kernel<MOST_TOKENS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             smem_bytes(ROWS, MOST_TOKENS, 0)) != cudaSuccess ||
+        cudaFuncSetAttribute(gemm_f32_split_kernel<FEW_TOKENS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             MOST_SMEM) != cudaSuccess)
       return Q3_ERR_LAUNCH;
     sms_on[device] = sms;
   }
@@ -431,22 +499,33 @@ Q3_EXPORT int q3_gemm_f32_split(const float* A, int lda, const float* W, int ldw
     split_matrix<false><<<blocks, 256, 0, stream>>>(A, lda, (uint4*)parts, M, K);
   // The token tile: rounds over the SMs times a slice's time, which is that of shared memory (a token's parts are read by 24
   // products and written once, the weights' read and written) or of the weights' bytes.
-  const int tiles = (N + ROWS - 1) / ROWS;
-  int best = 0;
+  int best = 0, rows = ROWS;
   double best_cost = 0;
-  for (int n = (M + MOST_TOKENS - 1) / MOST_TOKENS, tries = 0; tries < 4; ++n, ++tries) {
+  if (M <= FEW_TOKENS) {
+    // One token tile, and the rows of an item whichever make the rounds times a slice's cycles (its products', or its weights' way)
+    // the fewest.  One token, us with 128 / 112 / 96 / 80 rows: 19456 x 2560 79 / 75 / 73 / 87, 24576 x 4096 106 / 118 / 130 / 142,
+    // 8192 x 2560 40 / 38 / 54 / 52, 151936 x 2560 345 / 372 / 386 / 429.
+    best = M <= 16 ? 16 : 32;
+    for (int r = ROWS; r >= 48; r -= 16) {
+      const long items = (long)((N + r - 1) / r) * segments;
+      const double cost = (double)((items + sms - 1) / sms) * (600 + 15 * r / 2 < 1040 ? 1040 : 600 + 15 * r / 2);
+      if (r == ROWS || cost < best_cost) rows = r, best_cost = cost;
+    }
+  }
+  const int tiles = (N + rows - 1) / rows;
+  for (int n = (M + MOST_TOKENS - 1) / MOST_TOKENS, tries = 0; M > FEW_TOKENS && tries < 4; ++n, ++tries) {
     const int t = ((M + n - 1) / n + 15) / 16 * 16;
     const long items = (long)tiles * segments * ((M + t - 1) / t);
     const double slice = 24 * (4096 + 32 * t) + W_STAGE + 384 * t;
     const double cost = (double)((items + sms - 1) / sms) * (slice < 180000 ? 180000 : slice);
     if (!best || cost < best_cost) best = t, best_cost = cost;
   }
-  Args p = {A, W, lda, ldw, segments > 1 ? planes : C, segments > 1 ? N : ldc, (long)M * N, M, N, K, segments, 0, best, 0, 0, error_word};
+  Args p = {A, W, lda, ldw, segments > 1 ? planes : C, segments > 1 ? N : ldc, (long)M * N, M, N, K, segments, 0, best, 0, 0, rows, 0, error_word};
   const int slices = (K + SLICE - 1) / SLICE;
   p.slices_per_segment = (slices + segments - 1) / segments;
   p.token_tiles = (M + best - 1) / best;
   p.items = tiles * segments * p.token_tiles;
-  CUtensorMap map;
+  CUtensorMap map, wmap;
   Q3EncodeTiledFn encode = q3_encode_tiled();
   if (!encode) return Q3_ERR_LAUNCH;
   const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)M, 3};
@@ -455,8 +534,20 @@ Q3_EXPORT int q3_gemm_f32_split(const float* A, int lda, const float* W, int ldw
   if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, parts, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return Q3_ERR_LAUNCH;
+  const cuuint64_t wdims[2] = {(cuuint64_t)K, (cuuint64_t)N}, wstrides[1] = {(cuuint64_t)ldw * 4};
+  const cuuint32_t wbox[2] = {SLICE, (cuuint32_t)rows};
+  if (encode(&wmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(W), wdims, wstrides, wbox, es,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return Q3_ERR_LAUNCH;
   const int grid = p.items < sms ? p.items : sms;
-  gemm_f32_split_kernel<<<grid, THREADS, smem_bytes(best), stream>>>(map, p);
+  if (best <= FEW_TOKENS) {
+    p.raw = (MOST_SMEM - smem_bytes(rows, best, 0)) / (rows * SLICE * 4);
+    if (p.raw > MOST_RAW) p.raw = MOST_RAW;
+    gemm_f32_split_kernel<FEW_TOKENS><<<grid, threads(FEW_TOKENS), smem_bytes(rows, best, p.raw), stream>>>(map, wmap, p);
+  } else {
+    gemm_f32_split_kernel<MOST_TOKENS><<<grid, threads(MOST_TOKENS), smem_bytes(rows, best, 0), stream>>>(map, wmap, p);
+  }
   if (segments > 1)
     add_segments<<<(unsigned)(((long)M * N / 4 + 255) / 256), 256, 0, stream>>>(planes, (long)M * N, segments, C, ldc, M, N);
   return q3_launch_status();

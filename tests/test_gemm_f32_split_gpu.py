@@ -111,3 +111,30 @@ def test_values_that_are_no_numbers_cost_little_and_stay_with_their_row(ops):
     assert got[:, 3].isnan().all() and torch.equal(got[:, 4:], want[:, 4:]) and torch.equal(got[:, :3], want[:, :3])
     assert ops.linear(y, w).isnan().all()
     ops.raise_if_kernel_error()
+
+
+@pytest.mark.parametrize("N,K", [(19456, 2560), (24576, 4096), (8192, 2560), (151936, 2560)])
+def test_few_rows_are_no_slower_than_on_the_fma_pipes(ops, N, K):
+    x, w = _matrices(32, N, K)
+
+    def fma(rows):
+        ops.f32_split = False
+        try:
+            ops.linear(x[:rows], w)
+        finally:
+            ops.f32_split = True
+
+    for rows in (1, 16, 32):
+        split, chain = _times(ops, [lambda: ops.linear(x[:rows], w), lambda: fma(rows)])
+        assert split <= 1.03 * chain, (rows, split, chain)
+
+
+@pytest.mark.parametrize("N,K", [(19456, 1032), (20480, 1024), (12288, 2048), (2308, 9728)])
+def test_few_rows_have_the_bits_of_many(ops, N, K):
+    """Items one after another on an SM, whose two halves of warps store unlike numbers of tokens: every number of rows, often."""
+    x, w = _matrices(40, N, K)
+    want = ops.linear(x, w)
+    for rows in range(1, 33):
+        for first in (0, 3, 8):
+            assert torch.equal(ops.linear(x[first:first + rows], w), want[first:first + rows]), (rows, first)
+    ops.raise_if_kernel_error()
