@@ -281,12 +281,15 @@ struct ScanArgs {
   int ones_col;
   const float* bonus;
   int seg;          // tokens per segment
+  int lo, hi;       // the tokens that this launch runs: the others' sequences are empty or shorter
   float* ends;      // [segments, H, D, Dv]: what a segment leaves behind, then the segments' first states
   float* products;  // [segments, H, D]
 };
 
+// the first token of sequence b among this launch's (of num_seqs: their end)
+__device__ __forceinline__ int first_token(const ScanArgs& a, int b) { return min(max(a.cu_seqlens[b], a.lo), a.hi); }
 __device__ __forceinline__ int segments_of(const ScanArgs& a, int b) {
-  return (a.cu_seqlens[b + 1] - a.cu_seqlens[b] + a.seg - 1) / a.seg;
+  return (first_token(a, b + 1) - first_token(a, b) + a.seg - 1) / a.seg;
 }
 
 // Channel i < D of a token's key (turned, scaled), decay and query (turned, scaled) of a head, from its raw values.
@@ -385,8 +388,8 @@ segment_join_kernel(const __grid_constant__ ScanArgs a) {
 //
 // scan_chunk_rows, a block per (chunk, head): a record of SC_REC words, namely B, G q and the keys decayed to the chunk's end as
 // parts in the order of the scan's fragments, [3][32 lanes][4] for every 16 channels, G_last [DP], whether values are not finite;
-// behind it the values in that order, 128 words for 16 columns.  Chunks of sequence b start at place cu_seqlens[b] / 16 + b; tokens
-// beyond a portion's end are k = q = v = 0, a = 1.  Bound by instructions (2.5 a cycle; the decays' exponentials, the pairs'
+// behind it the values in that order, 128 words for 16 columns.  Chunks of sequence b start at place first_token / 16 + b (tokens
+// counted from this launch's first); tokens beyond a portion's end are k = q = v = 0, a = 1.  Bound by instructions (2.5 a cycle; the decays' exponentials, the pairs'
 // sums): 38 us for 2048 tokens of 16 heads of 64 x 128, 30 with the loads' addresses worked out once and 8 blocks an SM.
 // scan_chunk_states, a block per (segment, 32 value columns, head): the state transposed in registers as in delta_state.cu, a
 // warp 16 channels; the warps' parts of (G q) S meet in shared memory, one barrier a chunk, and are added a chunk later.  The same
@@ -419,8 +422,8 @@ scan_chunk_rows_kernel(const __grid_constant__ ScanArgs a, uint32_t* __restrict_
     int first = 0, left = 0;
     bool found = false;
     if (b < a.num_seqs) {
-      const int c0 = a.cu_seqlens[b], c1 = a.cu_seqlens[b + 1], base = c0 / SC_C + b;
-      found = place >= base && place < c1 / SC_C + b + 1;
+      const int c0 = first_token(a, b), c1 = first_token(a, b + 1), base = (c0 - a.lo) / SC_C + b;
+      found = place >= base && place < (c1 - a.lo) / SC_C + b + 1;
       first = c0 + (place - base) * SC_C;
       left = min(c1 - first, SC_C);
     }
@@ -622,10 +625,10 @@ scan_chunk_states_kernel(const __grid_constant__ ScanArgs a, const uint32_t* __r
   const int mine = blockIdx.x - first;  // the segment's number in its sequence
   const bool last = mine == count - 1;
   if (!OUT && last) return;
-  const int seq0 = a.cu_seqlens[b], t0 = seq0 + mine * a.seg, t1 = min(a.cu_seqlens[b + 1], t0 + a.seg);
+  const int seq0 = first_token(a, b), t0 = seq0 + mine * a.seg, t1 = min(first_token(a, b + 1), t0 + a.seg);
   const int chunks = (t1 - t0 + SC_C - 1) / SC_C;
   const long rec_size = SC_REC(DP) + SC_VALUES(Dv);
-  const uint32_t* rec0 = records + ((long)(seq0 / SC_C + b + mine * (a.seg / SC_C)) * H + h) * rec_size;
+  const uint32_t* rec0 = records + ((long)((seq0 - a.lo) / SC_C + b + mine * (a.seg / SC_C)) * H + h) * rec_size;
   auto load = [&](int c) {
     if (c < chunks) {
       const uint32_t* src = rec0 + (long)c * H * rec_size;
@@ -772,8 +775,7 @@ scan_chunk_states_kernel(const __grid_constant__ ScanArgs a, const uint32_t* __r
 }
 
 template <int DP>
-static cudaError_t launch_segments(const ScanArgs& a, int num_tokens, int segments, bool cut, uint32_t* records,
-                                   cudaStream_t stream) {
+static cudaError_t launch_segments(const ScanArgs& a, int segments, bool cut, uint32_t* records, cudaStream_t stream) {
   constexpr size_t ends_smem = sizeof(uint32_t) * SC_STAGES * (25 * DP + 32 + SC_TILES * 128);
   constexpr size_t smem = sizeof(uint32_t) * (SC_STAGES * (SC_REC(DP) + SC_TILES * 128) + 2 * DP / 16 * SC_C * (16 * SC_TILES + 4));
   auto ends = scan_chunk_states_kernel<DP, false>, scan = scan_chunk_states_kernel<DP, true>;
@@ -786,7 +788,7 @@ static cudaError_t launch_segments(const ScanArgs& a, int num_tokens, int segmen
     configured = true;
   }
   const dim3 grid((unsigned)segments, (unsigned)((a.Dv + 16 * SC_TILES - 1) / (16 * SC_TILES)), (unsigned)a.H), block(2 * DP);
-  cudaError_t e = launch_pdl(scan_chunk_rows_kernel<DP>, dim3((unsigned)(num_tokens / SC_C + a.num_seqs), (unsigned)a.H),
+  cudaError_t e = launch_pdl(scan_chunk_rows_kernel<DP>, dim3((unsigned)((a.hi - a.lo) / SC_C + a.num_seqs), (unsigned)a.H),
                              dim3(2 * DP), 0, stream, a, records);
   if (e != cudaSuccess) return e;
   // Neither pass is a dependent launch: its blocks would start between those of the kernel before and crowd some SMs while others
@@ -803,10 +805,12 @@ static cudaError_t launch_segments(const ScanArgs& a, int num_tokens, int segmen
   return cudaGetLastError();
 }
 
-// The same arguments as q3_decayed_state_scan, bfloat16, key sizes up to 128: in segments of `seg` tokens, a multiple of 16.
-// segments: the number of them, sum over the sequences of ceil(tokens / seg), or more; cut: whether a sequence may have more than
-// one; scratch: 32-bit words, 16-byte aligned, (num_tokens / 16 + num_seqs) * H * (416 + 49 * DP + 256 * ceil(Dv / 32)) with
-// DP = 64 (D <= 64) or 128, and if cut segments * H * D * (Dv + 1) more.
+// The same arguments as q3_decayed_state_scan, bfloat16, key sizes up to 128: tokens lo .. hi - 1 of the step in segments of `seg`
+// tokens, a multiple of 16.  (A step whose records are too many runs in several calls over tokens one after another; a sequence's
+// state carries over.  cu_seqlens and state_slots may start at the first sequence that has tokens in the call.)  segments: the number
+// of them, sum over the sequences of ceil(tokens / seg), or more; cut: whether a sequence may have more than one; scratch: 32-bit
+// words, 16-byte aligned, ((hi - lo) / 16 + num_seqs) * H * (416 + 49 * DP + 256 * ceil(Dv / 32)) with DP = 64 (D <= 64) or 128, and
+// if cut segments * H * D * (Dv + 1) more.
 Q3_EXPORT int q3_decayed_segment_scan(int dtype, const void* q, long q_stride, const void* k, long k_stride, const void* v,
                                       long v_stride, const void* z, long z_stride, const float* z_bias, float inv_tau,
                                       const float* head_decay, const float* inv_freq, int rot_pairs, const int* positions,
@@ -814,24 +818,24 @@ Q3_EXPORT int q3_decayed_segment_scan(int dtype, const void* q, long q_stride, c
                                       const int* state_slots, float* out, int num_seqs, int H, int D, int Dv,
                                       int decay_mode, const float* tok_decay, const float* tok_kscale, int ones_col,
                                       const float* bonus, int seg, int segments, int cut, float* scratch,
-                                      int num_tokens, cudaStream_t stream) {
+                                      int lo, int hi, cudaStream_t stream) {
   if (!q || !k || !v || !state || !cu_seqlens || !state_slots || !out || !scratch || seg < 1 || seg % SC_C || segments < 1 ||
-      num_tokens < 0 || ((uintptr_t)scratch & 15))
+      lo < 0 || hi < lo || ((uintptr_t)scratch & 15))
     return Q3_ERR_ARGUMENT;
   if (!z && !head_decay && !tok_decay) return Q3_ERR_ARGUMENT;
   if (decay_mode < 0 || decay_mode > 1 || ones_col < 0 || ones_col > 1 || Dv - ones_col < 1) return Q3_ERR_ARGUMENT;
   if (rot_pairs < 0 || 2 * rot_pairs > D || (rot_pairs && (!inv_freq || !positions))) return Q3_ERR_ARGUMENT;
   if (H < 1 || D < 1 || Dv < 1 || H > 65535 || num_seqs > 65535) return Q3_ERR_ARGUMENT;
   if (D > 128 || dtype != Q3_DTYPE_BF16) return Q3_ERR_UNSUPPORTED;
-  if (num_seqs == 0 || num_tokens == 0) return Q3_OK;
+  if (num_seqs == 0 || hi == lo) return Q3_OK;
   const int DP = D <= 64 ? 64 : 128;
-  float* ends = scratch + ((long)num_tokens / SC_C + num_seqs) * H * (SC_REC(DP) + SC_VALUES(Dv));
+  float* ends = scratch + ((long)(hi - lo) / SC_C + num_seqs) * H * (SC_REC(DP) + SC_VALUES(Dv));
   uint32_t* records = reinterpret_cast<uint32_t*>(scratch);
   const ScanArgs a = {q, k, v, z, q_stride, k_stride, v_stride, z_stride, z_bias, inv_tau, head_decay, inv_freq, rot_pairs,
                       positions, q_scale, k_scale, state, cu_seqlens, state_slots, out, num_seqs, H, D, Dv, decay_mode,
-                      tok_decay, tok_kscale, ones_col, bonus, seg, ends, ends + (long)segments * H * D * Dv};
-  const cudaError_t e = DP == 64 ? launch_segments<64>(a, num_tokens, segments, cut, records, stream)
-                                 : launch_segments<128>(a, num_tokens, segments, cut, records, stream);
+                      tok_decay, tok_kscale, ones_col, bonus, seg, lo, hi, ends, ends + (long)segments * H * D * Dv};
+  const cudaError_t e = DP == 64 ? launch_segments<64>(a, segments, cut, records, stream)
+                                 : launch_segments<128>(a, segments, cut, records, stream);
   return e == cudaSuccess ? Q3_OK : Q3_ERR_LAUNCH;
 }
 

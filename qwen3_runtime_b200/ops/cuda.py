@@ -174,8 +174,7 @@ _SIGNATURES = {
         "q3_decayed_segment_scan": [c_int, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long,
                                   c_void_p, c_float, c_void_p, c_void_p, c_int, c_void_p, c_float, c_float, c_void_p,
                                   c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                                  c_int, c_void_p, c_int, c_int, c_int, c_void_p,
-                                    c_int, c_void_p],
+                                  c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p],
         "q3_head_norm_gate": [c_int, c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p, c_long, c_void_p, c_long,
                               c_float, c_int, c_int, c_int, c_int, c_void_p],
         "q3_stabilised_gates": [c_int, c_void_p, c_void_p, c_long, c_void_p, c_void_p, c_float, c_void_p, c_void_p,
@@ -288,7 +287,7 @@ class _Span:
 
 
 # ---- decayed state scans of bfloat16 steps: token by token or in segments -------------------------
-SCAN_SCRATCH = 1 << 28  # floats a segment scan may ask for (1 GiB)
+SCAN_SCRATCH = 1 << 28  # floats a segment scan may ask for (1 GiB): a step that needs more runs in several launches
 
 # Times in us of the scan token by token and of segments run token by token, by the padded key size: what cutting has to win by.
 # (Segments are run in chunks now, which takes 0.55 to 0.75 of these times, see CHUNK_COSTS.)  Least squares over 48 compositions of
@@ -333,6 +332,56 @@ def _segments(cu, seg):
     return sum(-(-n // seg) for n in lens), max(lens)
 
 
+def _scan_fits(T, H, D, Dv, segments, cut):
+    """Whether a step is small enough to be cut at all: its q, k and decays, and the segments' states, as float32 within 1 GiB.
+    (How far cutting has been measured.  Below it windows cost little: one sequence of 8192 / 10500 tokens, 64 heads of 128 x
+    128, in one launch and in two 1.67 / 1.82 ms, token by token 9.0 / 12.5.)"""
+    return T * H * 3 * (64 if D <= 64 else 128) + (segments * H * D * (Dv + 1) if cut else 0) <= 1 << 28
+
+
+def _scan_windows(cu, H, D, Dv, seg):
+    """``(seg, windows)``: the step's tokens as runs ``(first token, end, first sequence, end, segments, cut)``, one launch after
+    another, whose scratch is at most SCAN_SCRATCH each.  They end where a segment of ``seg`` tokens ends; a segment that
+    would not fit gets shorter (0: not even 16 tokens fit)."""
+    segments, longest = _segments(cu, seg)
+    if _scan_scratch(cu[-1], len(cu) - 1, H, D, Dv, segments, longest > seg) <= SCAN_SCRATCH:
+        return seg, [(cu[0], cu[-1], 0, len(cu) - 1, segments, longest > seg)]
+    record, state = _scan_scratch(0, 1, H, D, Dv, 0, False), H * D * (Dv + 1)
+    seg = min(seg, (SCAN_SCRATCH - state - record) // record * 16)
+    if seg < 16:
+        return 0, []
+    windows, lo, first, used, segments, cut = [], cu[0], 0, 0, 0, False
+    for b, (t, end) in enumerate(zip(cu, cu[1:])):
+        if used + record > SCAN_SCRATCH:
+            if segments:
+                windows.append((lo, t, first, b, segments, cut))
+            lo, first, used, segments, cut = t, b, 0, 0, False
+        used += record  # (a sequence's last chunk need not be full)
+        pieces = 0
+        while t < end:
+            n = min(seg, end - t)
+            need = -(-n // 16) * record + state
+            if used + need > SCAN_SCRATCH:
+                if segments:
+                    windows.append((lo, t, first, b + 1, segments, cut))
+                lo, first, used, segments, cut, pieces = t, b, record, 0, False, 0
+            used, t, segments, pieces = used + need, t + n, segments + 1, pieces + 1
+            cut |= pieces > 1
+    if segments:
+        windows.append((lo, cu[-1], first, len(cu) - 1, segments, cut))
+    return seg, windows
+
+
+def _scan_runs(T, num_seqs, H, D, Dv, seg):
+    """The same without the sequences' lengths: every launch then has room for all sequences."""
+    record, state = _scan_scratch(0, 1, H, D, Dv, 0, False), H * D * (Dv + 1)
+    most = (SCAN_SCRATCH - num_seqs * (record + state)) // (seg // 16 * record + state) * seg
+    if most < seg:
+        return 0, []
+    return seg, [(lo, min(T, lo + most), 0, num_seqs, min(T - lo, most) // seg + num_seqs, min(T - lo, most) > seg)
+                 for lo in range(0, T, most)]
+
+
 def _one_wave(lens, most):
     """The shortest segments, of 32 tokens and more, of which sequences of these lengths have ``most`` at most (0: there are
     more sequences than that)."""
@@ -373,7 +422,7 @@ def decayed_scan_segment(cu, H, D, Dv, sms) -> int:
             break
         count = sum(-(-n // seg) for n in lens)
         more = sum(-(-n // seg) - 1 for n in lens if n)
-        if _scan_scratch(T, len(lens), H, D, Dv, count, more > 0) > SCAN_SCRATCH:
+        if not _scan_fits(T, H, D, Dv, count, more > 0):
             continue
         cost = c["row"] * T * H * (64 if D <= 64 else 128) + one_pass(T, count, min(seg, longest), *c["out"])
         cost += c["join"] + one_pass(more * seg, more, seg, *c["ends"]) if more else -c["whole"]
@@ -856,28 +905,32 @@ class CudaOps:
             e = q.element_size()
             self._costs(2 * num_seqs * H * D * Dv * 4 + T * H * ((3 if z is not None else 2) * D + Dv) * e
                         + T * H * Dv * 4, 6.0 * T * H * D * Dv)
-        args = (_dtype_code(q.dtype), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(z),
-                z.stride(0) if z is not None else 0, _ptr(decay_bias), 1.0 / float(tau), _ptr(head_decay), _ptr(inv_freq),
-                pairs, _ptr(positions), float(q_scale), float(k_scale), _ptr(state), _ptr(cu_seqlens), _ptr(state_slots),
-                _ptr(out), int(num_seqs), H, D, Dv, modes[decay_mode], _ptr(token_decay), _ptr(token_k_scale),
-                int(bool(ones_column)), _ptr(bonus))
+        before = (_dtype_code(q.dtype), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(z),
+                  z.stride(0) if z is not None else 0, _ptr(decay_bias), 1.0 / float(tau), _ptr(head_decay), _ptr(inv_freq),
+                  pairs, _ptr(positions), float(q_scale), float(k_scale), _ptr(state))
+        after = (H, D, Dv, modes[decay_mode], _ptr(token_decay), _ptr(token_k_scale), int(bool(ones_column)), _ptr(bonus))
         # (float32 stays token by token: the same bits however a prompt is cut)
         cu = tuple(host_cu_seqlens) if host_cu_seqlens else None
         seg = self._scan_segment(T, int(num_seqs), H, D, Dv, cu) if q.dtype == torch.bfloat16 else 0
+        windows = []
         if seg:
             seg = -(-seg // 16) * 16  # whole chunks
-            segments, longest = _segments(cu, seg) if cu else (T // seg + int(num_seqs), T)
+            seg, windows = _scan_windows(cu, H, D, Dv, seg) if cu else _scan_runs(T, int(num_seqs), H, D, Dv, seg)
+        if windows:
             try:
-                scratch = torch.empty(_scan_scratch(T, int(num_seqs), H, D, Dv, segments, longest > seg), dtype=torch.float32,
-                                      device=q.device)
+                scratch = torch.empty(max(_scan_scratch(hi - lo, last - first, H, D, Dv, segments, cut)
+                                          for lo, hi, first, last, segments, cut in windows),
+                                      dtype=torch.float32, device=q.device)
             except torch.OutOfMemoryError:
-                seg = 0  # token by token needs none
-        if seg:
-            self.launches += 1 + 2 * int(longest > seg)
-            self._call("linear_state", "q3_decayed_segment_scan", "decayed_state_scan", *args, seg, segments, int(longest > seg),
-                       _ptr(scratch), T)
-        else:
-            self._call("linear_state", "q3_decayed_state_scan", "decayed_state_scan", *args)
+                windows = []  # token by token needs none
+        for lo, hi, first, last, segments, cut in windows:
+            self.launches += 1 + 2 * int(cut)
+            self._call("linear_state", "q3_decayed_segment_scan", "decayed_state_scan", *before,
+                       _ptr(cu_seqlens[first:]), _ptr(state_slots[first:]), _ptr(out), last - first, *after, seg, segments,
+                       int(cut), _ptr(scratch), lo, hi)
+        if not windows:
+            self._call("linear_state", "q3_decayed_state_scan", "decayed_state_scan", *before, _ptr(cu_seqlens),
+                       _ptr(state_slots), _ptr(out), int(num_seqs), *after)
         return out
 
     def _scan_segment(self, T, num_seqs, H, D, Dv, cu=None) -> int:
@@ -890,7 +943,7 @@ class CudaOps:
             seg = decayed_scan_segment(cu, H, D, Dv, self.SM_COUNT)
             return chunk_segment(cu, H, D, Dv, self.SM_COUNT, seg) if seg else 0
         seg = max(32, -(-T // max(1, 2 * self.SM_COUNT // _scan_blocks(H, D, Dv))))
-        if T < max(64, 8 * num_seqs) or _scan_scratch(T, num_seqs, H, D, Dv, T // seg + num_seqs, True) > SCAN_SCRATCH:
+        if T < max(64, 8 * num_seqs) or not _scan_fits(T, H, D, Dv, T // seg + num_seqs, True):
             return 0
         return seg
 

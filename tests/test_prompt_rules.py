@@ -180,3 +180,49 @@ def test_segments_are_whole_chunks_of_a_measured_length():
     # many blocks need no cut, few heads short segments
     assert chunk_segment(_cu([256] * 8), 16, 64, 128, 148, 128) == 256 and chunk_segment(_cu([64] * 32), 16, 64, 128, 148, 64) == 64
     assert chunk_segment(_cu([2048]), 4, 64, 128, 148, 32) < chunk_segment(_cu([2048]), 16, 64, 128, 148, 114) <= 512
+
+
+def test_large_steps_are_cut_whatever_their_records_take():
+    from qwen3_runtime_b200.ops.cuda import SCAN_SCRATCH, _scan_scratch, _scan_windows, decayed_scan_segment
+
+    for tokens, heads, dim, vdim in ((10500, 64, 128, 128), (10000, 64, 128, 256), (20000, 32, 128, 512), (80000, 16, 64, 128)):
+        cu = _cu([tokens])
+        seg = -(-decayed_scan_segment(cu, heads, dim, vdim, 148) // 16) * 16
+        assert seg > 0 and _scan_scratch(tokens, 1, heads, dim, vdim, -(-tokens // seg), seg < tokens) > SCAN_SCRATCH
+        assert len(_scan_windows(cu, heads, dim, vdim, seg)[1]) > 1
+    ops = _table()
+    assert ops._scan_segment(10000, 1, 64, 128, 128) > 0  # the lengths unknown
+
+
+def test_windows_cover_a_step_and_fit_their_scratch(monkeypatch):
+    import random
+
+    from qwen3_runtime_b200.ops import cuda
+
+    rnd = random.Random(0)
+    some = [0, 0]
+    for _ in range(400):
+        heads, dim, vdim = rnd.choice([1, 4, 16]), rnd.choice([64, 128]), rnd.choice([16, 128, 200])
+        lens = [rnd.choice([0, 1, 1, rnd.randint(2, 40), rnd.randint(1, 900)]) for _ in range(rnd.randint(1, 40))]
+        cu, T, seg = _cu(lens), sum(lens), 16 * rnd.randint(1, 20)
+        record, state = cuda._scan_scratch(0, 1, heads, dim, vdim, 0, False), heads * dim * (vdim + 1)
+        monkeypatch.setattr(cuda, "SCAN_SCRATCH", rnd.randint(2 * record + state, 60 * (record + state)))
+        got, windows = cuda._scan_windows(cu, heads, dim, vdim, seg)
+        assert 16 <= got <= seg and got % 16 == 0
+        if T == 0:
+            continue
+        some[len(windows) > 1] += 1
+        assert windows[0][0] == 0 and windows[-1][1] == T
+        assert all(a[1] == b[0] for a, b in zip(windows, windows[1:]))
+        for lo, hi, first, last, segments, cut in windows:
+            inside = [min(max(b, lo), hi) - min(max(a, lo), hi) for a, b in zip(cu, cu[1:])]
+            assert sum(inside) == sum(inside[first:last]) == hi - lo > 0
+            assert segments == sum(-(-n // got) for n in inside) and cut == any(n > got for n in inside)
+            assert cuda._scan_scratch(hi - lo, last - first, heads, dim, vdim, segments, cut) <= cuda.SCAN_SCRATCH
+        got, windows = cuda._scan_runs(T, len(lens), heads, dim, vdim, seg)
+        assert (got == 0) == (not windows)
+        for lo, hi, first, last, segments, cut in windows:
+            assert (first, last) == (0, len(lens)) and segments >= sum(
+                -(-(min(max(b, lo), hi) - min(max(a, lo), hi)) // got) for a, b in zip(cu, cu[1:]))
+            assert cuda._scan_scratch(hi - lo, last, heads, dim, vdim, segments, cut) <= cuda.SCAN_SCRATCH
+    assert min(some) > 50

@@ -74,3 +74,34 @@ def test_values_that_are_not_finite_stay_with_their_column_and_later_tokens(ops,
     assert not torch.isfinite(state[0, 1, :, 35]).any()
     state[0, 1, :, 35] = clean_state[0, 1, :, 35]
     assert torch.equal(state, clean_state)
+
+
+@pytest.mark.parametrize("host", [True, False])
+@pytest.mark.parametrize("D,Dv,windows", [(64, 33, 3), (128, 130, 6)])
+def test_steps_whose_scratch_is_too_large_run_in_windows(ops, monkeypatch, D, Dv, windows, host):
+    """Several launches over tokens one after another, whose boundaries fall into sequences, against one launch over all."""
+    from qwen3_runtime_b200.ops import cuda
+
+    lens, H, seg = [1, 15, 300, 0, 17, 1, 1, 640, 33, 0, 96], 3, 48
+    q, k, v, kw, start = _step(lens, H, D, Dv)
+    if not host:
+        kw["host_cu_seqlens"] = None
+    monkeypatch.setattr(ops, "_scan_segment", lambda *args: seg)
+    launched, call = [], ops._call
+
+    def spy(group, name, what, *args):
+        launched.append(name)
+        return call(group, name, what, *args)
+
+    monkeypatch.setattr(ops, "_call", spy)
+    out, states = [], []
+    for whole in (True, False):
+        if not whole:
+            most = cuda._scan_scratch(sum(lens), len(lens), H, D, Dv, -(-sum(lens) // seg) + len(lens), True)
+            monkeypatch.setattr(cuda, "SCAN_SCRATCH", most // windows + (0 if host else most // 3))
+        states.append(start.clone())
+        out.append(ops.decayed_state_scan(q, k, v, state=states[-1], **kw))
+    assert launched[0] == launched[-1] == "q3_decayed_segment_scan" and len(launched) > 2
+    # the sums over a sequence's segments in another order
+    assert float((out[0] - out[1]).abs().max()) <= 3e-5 * float(out[0].abs().max())
+    assert float((states[0] - states[1]).abs().max()) <= 3e-5 * float(states[0].abs().max())
