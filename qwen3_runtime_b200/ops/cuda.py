@@ -2090,10 +2090,7 @@ class CudaOps:
                 out = torch.empty((M, N), dtype=torch.float32, device=x.device)
             segments = self._f32_segments(x, weight)
             if segments and M:
-                # (in portions of rows, which bounds the scratch: a row's bits do not depend on its neighbours)
-                most = min(M, self.F32_SPLIT_ROWS)
-                parts = torch.empty(3 * most * K, dtype=torch.bfloat16, device=x.device)
-                planes = torch.empty((segments, most, N), dtype=torch.float32, device=x.device) if segments > 1 else None
+                most, parts, planes = self._f32_scratch(M, N, K, segments, x.device)
                 for m in range(0, M, most):
                     rows = min(most, M - m)
                     self.launches += 1 + (segments > 1)
@@ -2117,7 +2114,24 @@ class CudaOps:
                 return self._library_mm(x, weight, out, out_dtype)
         return self._library_mm(x, weight, out, out_dtype)
 
-    F32_SPLIT_ROWS = 4096
+    F32_SPLIT_ROWS, F32_SPLIT_BYTES = 4096, 1 << 28
+
+    def _f32_scratch(self, M, N, K, segments, device):
+        """``(rows, parts, planes)``: how many of M rows a float32 product on the tensor cores takes at a time, with its scratch
+        (the rows' parts, and the segments' sums where there are several): at most 256 MB, and less where the device has no
+        room.  A row's bits do not depend on its neighbours, so any portions give the same result."""
+        per_row = 6 * K + (4 * N * segments if segments > 1 else 0)
+        most = max(1, min(M, self.F32_SPLIT_ROWS, self.F32_SPLIT_BYTES // per_row))
+        if 160 < most < M:
+            most -= most % 160  # whole token tiles
+        while True:
+            try:
+                parts = torch.empty(3 * most * K, dtype=torch.bfloat16, device=device)
+                return most, parts, torch.empty((segments, most, N), dtype=torch.float32, device=device) if segments > 1 else None
+            except torch.OutOfMemoryError:
+                if most == 1:
+                    raise
+                most = -(-most // 2)
 
     def _f32_segments(self, x, weight) -> int:
         """Segments of K in the float32 product on the tensor cores (csrc/gemm_f32_split.cuh); 0: the FMA kernel computes it.

@@ -138,3 +138,25 @@ def test_few_rows_have_the_bits_of_many(ops, N, K):
         for first in (0, 3, 8):
             assert torch.equal(ops.linear(x[first:first + rows], w), want[first:first + rows]), (rows, first)
     ops.raise_if_kernel_error()
+
+
+def test_scratch_is_bounded_and_gets_smaller_where_there_is_no_room(ops, monkeypatch):
+    x, w = _matrices(1000, 24576, 4096)
+    want = ops.linear(x[:700], w)
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    got = ops.linear(x, w)
+    assert torch.cuda.max_memory_allocated() - before - got.nbytes <= ops.F32_SPLIT_BYTES + (1 << 20)
+    assert torch.equal(got[:700], want)
+    empty, asked = torch.empty, []
+
+    def little_room(*size, **options):
+        sizes = size[0] if isinstance(size[0], tuple) else size
+        if torch.Size(sizes).numel() > 2_000_000 and sizes != (700, 24576):
+            asked.append(sizes)
+            raise torch.OutOfMemoryError("no room")
+        return empty(*size, **options)
+
+    monkeypatch.setattr(torch, "empty", little_room)
+    assert torch.equal(ops.linear(x[:700], w), want) and len(asked) > 2
+    ops.raise_if_kernel_error()
