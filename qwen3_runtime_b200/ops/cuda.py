@@ -1079,12 +1079,16 @@ class CudaOps:
             self._costs(2 * num_seqs * H * D * Dv * 4 + T * (8 * G * D + H * Dv * (e + 4) + 4 * H * D),
                         7.0 * T * H * D * Dv)
         longest = 0x7fffffff  # of the sequences that go token by token
+        records = None
         if self.delta_chunks and D <= 128 and T >= max(32, 4 * num_seqs):
+            try:
+                records = torch.empty((T // 16 + num_seqs) * H * 73 * (64 if D <= 64 else 128), dtype=torch.float32, device=dev)
+                u0 = torch.empty_like(out)
+            except torch.OutOfMemoryError:
+                records = None  # token by token needs none
+        if records is not None:
             # prompts: chunks of 16 tokens (csrc/delta_state.cu); what does not depend on the state first
             num_long = self._delta_long(host_cu_seqlens, int(num_seqs), H, Dv)
-            padded = 64 if D <= 64 else 128
-            records = torch.empty((T // 16 + num_seqs) * H * 73 * padded, dtype=torch.float32, device=dev)
-            u0 = torch.empty_like(out)
             self.launches += 1
             self._call("delta_state", "q3_delta_chunk_scan", "delta_chunk_scan", _dtype_code(x.dtype), _ptr(qn), _ptr(kn),
                        _ptr(vc), _ptr(g), _ptr(beta), _ptr(records), _ptr(u0), _ptr(state), _ptr(cu_seqlens),
