@@ -792,15 +792,22 @@ static cudaError_t launch_segments(const ScanArgs& a, int segments, bool cut, ui
                              dim3(2 * DP), 0, stream, a, records);
   if (e != cudaSuccess) return e;
   // Neither pass is a dependent launch: its blocks would start between those of the kernel before and crowd some SMs while others
-  // stay empty (a prompt of 2048 tokens, 16 heads of 64 x 128, segments of 1024: the second pass 101 us).
+  // stay empty (a prompt of 2048 tokens, 16 heads of 64 x 128, segments of 1024: the second pass 101 us).  Unless they are few and
+  // short (16 prompts of 16 tokens, 4 heads of 32 x 32, lengths unknown: 20.4 us instead of 23.5).
+  const bool dependent = cut && a.seg <= 64 && (long)grid.x * grid.y * grid.z <= 512;
   if (cut) {
-    ends<<<grid, block, ends_smem, stream>>>(a, records);
-    e = cudaGetLastError();
+    if (dependent) {
+      e = launch_pdl(ends, grid, block, ends_smem, stream, a, (const uint32_t*)records);
+    } else {
+      ends<<<grid, block, ends_smem, stream>>>(a, records);
+      e = cudaGetLastError();
+    }
     if (e == cudaSuccess)
       e = launch_pdl(segment_join_kernel, dim3((unsigned)((a.D * a.Dv + 255) / 256), (unsigned)a.H, (unsigned)a.num_seqs),
                      dim3(256), 0, stream, a);
     if (e != cudaSuccess) return e;
   }
+  if (dependent) return launch_pdl(scan, grid, block, smem, stream, a, (const uint32_t*)records);
   scan<<<grid, block, smem, stream>>>(a, records);
   return cudaGetLastError();
 }
