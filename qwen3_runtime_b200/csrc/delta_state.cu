@@ -405,6 +405,52 @@ __device__ __forceinline__ void ds_copy16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
 }
 
+// Element (i, its column) of a product with a lower triangular matrix of tokens, whose parts lie at `left` in the order of a left
+// operand, from rows 0 .. i of the right operand only (at(j): row j's element of the column).
+template <typename F>
+__device__ __forceinline__ float ds_own_rows(const uint32_t* left, int i, F at) {
+  float sum = 0.f;
+  for (int j = 0; j <= i; ++j) {
+    const int place = ((i & 7) * 4 + ((j & 7) >> 1)) * 4 + (i >> 3) + 2 * (j >> 3), shift = j & 1 ? 0 : 16;
+    float w = 0.f;
+    for (int m = 2; m >= 0; --m) w += __uint_as_float((left[m * 128 + place] << shift) & 0xffff0000u);
+    sum = fmaf(w, at(j), sum);
+  }
+  return sum;
+}
+// A warp's share of a record once more where keys or values are not finite: W and B W hold zeros behind a row's own token, which in
+// the products make a NaN of an earlier token's row.  Behind everything else, so that the products' registers are free.
+template <typename T, int DP>
+__device__ __forceinline__ void delta_own_rows(uint32_t* rec, const uint32_t* w, const uint32_t* bw, const float* gk, const float* gq,
+                                            int pitch, const T* v, float* u0, float* out, long row, int n, int Dv) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, t4 = lane & 3;
+  for (int x = 0; x < 2; ++x)
+    for (int i = 0; i < 2; ++i) {
+      const int c = gr + 8 * i;
+      if (warp < DP / 16) {
+        const int d = warp * 16 + 8 * x + 2 * t4, at = warp * 384 + lane * 4 + 2 * i + x;
+        float p[2], q[2];
+        for (int e = 0; e < 2; ++e) {
+          p[e] = ds_own_rows(w, c, [&](int j) { return gk[j * pitch + d + e]; });
+          q[e] = gq[c * pitch + d + e] - ds_own_rows(bw, c, [&](int j) { return gk[j * pitch + d + e]; });
+        }
+        uint32_t p3[3], q3[3];
+        ds_split(p[0], p[1], p3);
+        ds_split(q[0], q[1], q3);
+        for (int m = 0; m < 3; ++m) {
+          rec[m * 128 + at] = p3[m];
+          rec[24 * DP + m * 128 + at] = q3[m];
+        }
+      }
+      for (int col = warp * 16 + 8 * x + 2 * t4; col < Dv; col += 128)
+        for (int e = 0; e < 2 && c < n && col + e < Dv; ++e) {
+          const T* column = v + col + e;
+          u0[c * row + col + e] = ds_own_rows(w, c, [&](int j) { return to_f32(column[j * row]); });
+          out[c * row + col + e] = ds_own_rows(bw, c, [&](int j) { return to_f32(column[j * row]); });
+        }
+    }
+}
+
 // A block makes one record.  Loads; the pairs' sums A and B; then, side by side, the decayed keys and queries (warps 4 up, in
 // place) and the 16 x 16 matrices W = (I + diag(beta) A)^(-1) diag(beta) and B W by substitution, a lane per column (warps 0
 // and 1); then a warp makes 16 channels of P = W (G k) and Q = G q - (B W) (G k) and 16 value columns of U0 = W V and O0 =
@@ -604,6 +650,11 @@ delta_chunk_rows_kernel(const float* __restrict__ qn, const float* __restrict__ 
   uint32_t w3[3][4], bw3[3][4];
   ds_parts(w3, tp[0], lane);
   ds_parts(bw3, tp[1], lane);
+  // becomes NaN where a right operand of this warp's is not finite (its first part tells)
+  __nv_bfloat162 none = __floats2bfloat162_rn(0.f, 0.f);
+  auto watch = [&](uint32_t first) {
+    none = __hfma2(*reinterpret_cast<__nv_bfloat162*>(&first), __floats2bfloat162_rn(0.f, 0.f), none);
+  };
   // tokens 2 t4, 2 t4 + 1, 2 t4 + 8, 2 t4 + 9 of channels 16 warp + gr (+ 8), in parts
   auto right = [&](const float(*from)[PITCH], uint32_t(&to)[3][4]) {
 #pragma unroll
@@ -638,6 +689,8 @@ delta_chunk_rows_kernel(const float* __restrict__ qn, const float* __restrict__ 
       store(to + warp * 384, r);
     };
     right(gs, gk);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) watch(gk[0][x]);
     ds_products(acc, w3, gk);
     record(rec);
     ds_products(acc, bw3, gk);
@@ -660,6 +713,7 @@ delta_chunk_rows_kernel(const float* __restrict__ qn, const float* __restrict__ 
     for (int x = 0; x < 4; ++x) {
       uint32_t p[3];
       ds_split(to_f32(vr[x >> 1][2 * (x & 1)]), to_f32(vr[x >> 1][2 * (x & 1) + 1]), p);
+      watch(p[0]);
 #pragma unroll
       for (int m = 0; m < 3; ++m) v3[m][x] = p[m];
     }
@@ -677,6 +731,9 @@ delta_chunk_rows_kernel(const float* __restrict__ qn, const float* __restrict__ 
     rows_out(u0, w3);
     rows_out(out, bw3);
   }
+  if (__any_sync(0xffffffffu, __hisnan(none.x) || __hisnan(none.y)))
+    delta_own_rows<T, DP>(rec, tp[0], tp[1], gs[0], qs[0], PITCH, vc + (t0 * H + h) * Dv, u0 + (t0 * H + h) * Dv,
+                          out + (t0 * H + h) * Dv, (long)H * Dv, n, Dv);
 }
 
 // The state is held transposed, as the accumulators of its update (rows: the 16 value columns; columns: a warp's 16

@@ -69,3 +69,32 @@ def test_a_step_without_room_for_its_records_runs_token_by_token(monkeypatch):
     # float32 sums of a few hundred addends in another order
     for a, c in zip(*got):
         assert float((a - c).abs().max()) <= 3e-5 * float(c.abs().max())
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("what", ["value", "key", "query", "step"])
+@pytest.mark.parametrize("D,Dv", [(64, 48), (128, 136), (40, 20)])
+def test_what_is_not_finite_leaves_earlier_tokens_alone(what, bad, D, Dv):
+    """One input that is no finite number, in the middle of a chunk: the tokens before it, of its chunk too, are as without it, and a
+    value's column is the only one that it reaches; as token by token."""
+    from qwen3_runtime_b200.ops.cuda import CudaOps
+
+    ops, G, H, at = CudaOps(), 2, 4, 200 + 7
+    x, z, b, kw, rings, states = _delta_step([200, 100], H=H, G=G, D=D, Dv=Dv)
+    clean = ops.delta_rule(x, z, b, ring=rings(), state=states(), **kw)
+    column = {"query": D + 3, "key": G * D + D + 3, "value": 2 * G * D + 3 * Dv + 5}  # of (q | k | v) heads 1, 1 and 3
+    if what == "step":
+        b[at, 3] = float("nan")
+    else:
+        x[at, column[what]] = bad
+    out = {}
+    for chunks in (True, False):
+        ops.delta_chunks = chunks
+        out[chunks] = ops.delta_rule(x, z, b, ring=rings(), state=states(), **kw)
+    heads = [2, 3] if what in ("query", "key") else [3]
+    touched = torch.zeros_like(clean, dtype=torch.bool)
+    touched[at:, heads, 5 if what == "value" else slice(None)] = True
+    for got in out.values():
+        # (sums of another order where an infinity stands beside them)
+        assert float((got - clean)[~touched].abs().max()) <= 3e-5 * float(clean.abs().max())
+        assert not torch.isfinite(got[at][heads][:, 5] if what == "value" else got[at][heads]).any()
