@@ -28,15 +28,15 @@
 //   warps 14, 15     : MMA issuers of PV for block A and B: PV_j when P_j is written.
 // Tensor memory: all 512 columns, per block S [0,64), P_0 and P_1 [64,128), O [128,256).
 // What bounds it: the softmax warps, and behind them the products (S with 64 columns is bound by its reads of shared memory,
-// 45 cycles per 16 k-values) and the keys' and values' way from L2 (32 KB a step and SM).  A step of both blocks takes 1520
+// 47 cycles per 16 k-values) and the keys' and values' way from L2 (32 KB a step and SM).  A step of both blocks takes 1520
 // cycles where the exp2 unit alone needs 1024.  What counted was code, not arithmetic: 32 heads over 8, 8192 tokens, one layer,
-// us (2048 tokens: 48 -> 43):
+// us (2048 tokens: 48 -> 43; forms of this code that differ only in what stands beside the loops lie 4 % apart, so time both sizes):
 //   554  one issuer per block (PV_j before S_(j+2): its waits, commits and products took longer than the softmax of a tile), one
 //        producer, S twice and P over S
 //   550  S issued before PV by warps of their own, four producers
 //   512  tiles that all rows see as a whole without the masks' branches; waits with their slow part out of line
 //   457  the reference point moved without a branch, the rescaling out of line
-//   440  the issuers' lane chosen by elect.sync (an MMA of 64 columns every 47 cycles instead of 60 to 78)
+//   451  the issuers' lane chosen by elect.sync (an MMA of 64 columns every 47 cycles instead of 60 to 78)
 // Not kept: 128 keys a step (830: the chain of a block twice as long), turns of the two blocks at the exponentials (482),
 // S_(j+1) loaded beside the exponentials of tile j with 192 registers a thread (585), waits that try again without looking at
 // the clock (512 -> 562).  Forms: differential attention, 16 heads over 4, 2333 + 419 tokens 60 -> 54 us (mma.sync: 247);
@@ -262,9 +262,9 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
         return in ? bt[pi] : -1;
       };
       int next = MODE == DENSE ? 0 : page_of(0);
-      int st = 0, issued = 0;
+      int st = 0, j = 0;
       uint32_t phase = 1;
-      for (int j = 0; j < num_tiles; ++j) {
+      for (; j < num_tiles; ++j) {
         const int page = next;
         const uint32_t dst = dst0 + st * stage_bytes;
         uint32_t bytes = HALF_KV + (MODE == DENSE && part == 1 ? HALF_KV : 0);
@@ -290,13 +290,12 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
           }
         }
         if (++st == KV_STAGES) st = 0, phase ^= 1;
-        ++issued;
       }
       // The last boxes may still be in flight when the others have given up.  (Then a stage that the other producer did not come to
       // any more is waited for until the limit.)
       if (lane == 0) {
         if (part == 3) mbar_wait_drain(bar(BAR_Q), 0);
-        for (int j = max(0, issued - KV_STAGES); j < issued; ++j) mbar_wait_drain(full + 8 * (j % KV_STAGES), (j / KV_STAGES) & 1);
+        for (int i = max(0, j - KV_STAGES); i < j; ++i) mbar_wait_drain(full + 8 * (i % KV_STAGES), (i / KV_STAGES) & 1);
       }
     } else if (warp > 11) {
       // ---- MMA issuers: warps 12 and 13 for S of block A and B, warps 14 and 15 for PV ---------
@@ -330,8 +329,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
                 umma_bf16(tmem_x, umma_desc(q_addr + half * HALF_Q) + sub,
                      umma_desc(k_addr + (MODE == MAPS ? x : half) * HALF_KV) + sub, idesc, k > 0 ? 1u : 0u);
               }
-              umma_commit(bar(BAR_K_EMPTY + st));  // this block is done with the key tile
               umma_commit(bar(BAR_S_FULL + x));    // S_j is in TMEM
+              umma_commit(bar(BAR_K_EMPTY + st));  // this block is done with the key tile
             } else {
               mbar_arrive(bar(BAR_K_EMPTY + st));
             }
@@ -353,8 +352,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
               for (int k = 0; k < BLOCK_N / 16; ++k)  // 16 keys: 8 columns of P, 2 KB down V's rows
                 umma_bf16_tmem(tmem_x + TMEM_O, tmem_x + TMEM_P + (j & 1) * (BLOCK_N / 2) + 8 * k,
                      umma_desc_mn_major(v_addr + k * 2048, HALF_KV), idesc, (j > 0 || k > 0) ? 1u : 0u);
-              umma_commit(bar(BAR_V_EMPTY + st));
               umma_commit(bar(BAR_PV_FULL + x));
+              umma_commit(bar(BAR_V_EMPTY + st));
             } else {
               mbar_arrive(bar(BAR_V_EMPTY + st));
             }
@@ -363,7 +362,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
           if (++st == KV_STAGES) st = 0, phase ^= 1;
         }
       }
-      if (leader) {  // nothing of this issuer's is in flight any more when the tensor memory is freed
+      if (elect_one()) {  // (the same lane again) nothing of this issuer's is in flight any more when the tensor memory is freed
         umma_commit(bar(BAR_END + role - 12));
         mbar_wait_drain(bar(BAR_END + role - 12), 0);
       }
@@ -492,9 +491,12 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
       const int pos_first = base_pos + row_first / G, pos_last = base_pos + row_last / G;
       const int lo_last = chunk > 0 ? pos_last / chunk * chunk : (window > 0 ? max(0, pos_last - window + 1) : 0);
       // (What rows that are none see in a last block has no say: nothing of theirs is stored.  A last block that goes through tiles with
-      // masks only is the longest of its sequence: 32 heads over 8, 500 tokens behind 3000, 76 us; so 64.)
-      const int whole0 = max(1, (max(lo_last, k_lo) + BLOCK_N - 1) / BLOCK_N - tile0);
-      const int whole1 = min(my_tiles, (pos_first + 1) / BLOCK_N - tile0);  // such tiles behind the first one
+      // masks only is the longest of its sequence: 32 heads over 8, 500 tokens behind 3000, 78 us; so 64.)
+      int whole0 = 1, whole1 = 0;  // such tiles behind the first one
+      if (row0[x] < rows) {
+        whole0 = max(1, (max(lo_last, k_lo) + BLOCK_N - 1) / BLOCK_N - tile0);
+        whole1 = min(my_tiles, (pos_first + 1) / BLOCK_N - tile0);
+      }
       bool ok = true;
       for (int j = 0; j < my_tiles && ok; ++j) {
         if (j < whole0 || j >= whole1) {
