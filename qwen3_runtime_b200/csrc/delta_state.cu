@@ -381,9 +381,9 @@ Q3_EXPORT int q3_delta_scan(int dtype, const float* qn, const float* kn, const v
 //   U = U0 - P S      O = O0 + Q S      S <- G_last S + sum_j (prod_(m > j) g_m k_j) u_j^T
 // P, Q, U0 and O0 do not depend on the state, so only two products are left in the chain from chunk to chunk.  A row of P
 // is beta_i k_i times a product of contractions and no longer than beta_i |k_i|.  Only products of decays occur, never
-// quotients, so strong decays lose nothing.  All of it is fp32 FMA.
+// quotients, so strong decays lose nothing.
 //
-// Products of matrices run on mma.sync with every operand as the sum of three bfloat16 (24 bits: nothing is lost) and the six
+// Products of matrices run on mma.sync with every operand as the sum of three bfloat16 (split_mma.cuh) and the six
 // products of parts that matter, the largest alone and added last; what a product adds to the state is summed from zero and
 // added to it in fp32, once per chunk.  Everything else is fp32 FMA.  Against float64 (700 + 300 tokens, 16 heads of 128,
 // mean decays of 0.95 / 0.9997 a token): outputs 1.2e-7 / 2.2e-7, state 1.0e-7 / 2.2e-7; with FMA throughout 1.3e-7 / 3.4e-7
@@ -400,10 +400,6 @@ Q3_EXPORT int q3_delta_scan(int dtype, const float* qn, const float* kn, const v
 // parts made in the scan instead of stored 125; the rows with substitutions for every column on FMA 68.)
 #define DC_C 16
 #define DC_REC(DP) ((DP) * 73)
-
-__device__ __forceinline__ void ds_copy16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
-}
 
 // Element (i, its column) of a product with a lower triangular matrix of tokens, whose parts lie at `left` in the order of a left
 // operand, from rows 0 .. i of the right operand only (at(j): row j's element of the column).

@@ -1,12 +1,14 @@
 // C[M, N] = A[M, K] * W[N, K]^T of float32 matrices on the tensor cores, every operand as the sum of three bfloat16 (8 + 8 + 8
-// bits: nothing is lost) and the six products of parts that matter; the other three are below 2^-26 of a product.
+// bits: nothing is lost, see split_mma.cuh) and the six products of parts that matter; the other three are below 2^-24 of a
+// product together (2^-25 each for the larger two).
 //
 // The accumulators of tcgen05.mma round towards zero at every step (products of 2560 values: 2.7e-6 off, 7e-6 if all are
-// positive; one chain of fp32 FMA 4.5e-7), so a chain is never longer than a slice of 64 k-values: its 20 small products first,
-// which cost no digits of the sum, then the 4 large ones; the slice's result is added to fp32 registers, rounded to nearest, in
-// ascending k.  K may be cut into segments, whose sums are added in order by a second kernel; how many depends on N and K
-// only.  So a row of C does not depend on M, on the tile chosen for M, or on where the row sits in the batch, and lies nearer to
-// the exact product than the FMA chain (split_matrix and the kernel below; K from 1024: see the dispatch).
+// positive; one chain of fp32 FMA 9e-7 and 7e-7, this kernel 1.2e-7 and 1.0e-7), so a chain is never longer than a slice of 64
+// k-values: its 20 small products first, which cost no digits of the sum, then the 4 large ones; the slice's result is added to
+// fp32 registers, rounded to nearest, in ascending k.  K may be cut into segments, whose sums are added in order by a second
+// kernel; how many depends on N and K only.  So a row of C does not depend on M, on the tile chosen for M, or on where the row
+// sits in the batch, and lies nearer to the exact product than the FMA chain (split_matrix and the kernel below; K from 1024:
+// see the dispatch).
 //
 // Weights are the 128 rows of an MMA, tokens its 16 to 160 columns.  Roles of a block (one per SM, persistent over items of
 // (128 weight rows, segment, token tile), token tiles of the same weights side by side):
@@ -24,6 +26,7 @@
 // pipes / here: 300 tokens 19456 x 2560 701 / 218, 2560 x 9728 412 / 112; one token 19456 x 2560 82 / 73 (105 without that kernel),
 // 24576 x 4096 129 / 105 (145), 151936 x 2560 383 / 345 (495), 4096 x 12288 111 / 64 (82).
 #include "async_tiles.cuh"
+#include "split_mma.cuh"
 
 namespace split {
 
@@ -36,16 +39,6 @@ constexpr int smem_bytes(int rows, int tokens, int raw) { return 768 * (rows + t
 constexpr int MOST_SMEM = 231936;
 enum { BAR_W_FULL = 0, BAR_X_FULL = 2, BAR_EMPTY = 4, BAR_D_FULL = 6, BAR_D_EMPTY = 8, BAR_END = 10, BAR_RAW_FULL = 11,
        BAR_RAW_EMPTY = BAR_RAW_FULL + MOST_RAW, NUM_BARS = BAR_RAW_EMPTY + MOST_RAW };
-
-// (x, y) as the sum of three pairs of bfloat16
-__device__ __forceinline__ void parts_of(float x, float y, uint32_t (&p)[3]) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p[i]) : "f"(y), "f"(x));
-    x -= __uint_as_float(p[i] << 16);
-    y -= __uint_as_float(p[i] & 0xffff0000u);
-  }
-}
 
 // x [M, K], rows ldx apart, as three dense bfloat16 matrices one behind the other; K a multiple of 8
 template <bool VEC>
@@ -64,7 +57,7 @@ split_matrix(const float* __restrict__ x, long ldx, uint4* __restrict__ to, int 
   }
   uint32_t p[4][3];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) parts_of(v[2 * i], v[2 * i + 1], p[i]);
+  for (int i = 0; i < 4; ++i) ds_split(v[2 * i], v[2 * i + 1], p[i]);
 #pragma unroll
   for (int i = 0; i < 3; ++i) to[i * M * per_row + at] = make_uint4(p[0][i], p[1][i], p[2][i], p[3][i]);
 }
@@ -370,8 +363,8 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_con
         for (int i = 0; i < 8; ++i) {
           if (FEW && i * 16 >= p.rows) break;  // (rows beyond stay as they are: a result depends on its own row only)
           uint32_t lo[3], hi[3];
-          parts_of(v[i].x, v[i].y, lo);
-          parts_of(v[i].z, v[i].w, hi);
+          ds_split(v[i].x, v[i].y, lo);
+          ds_split(v[i].z, v[i].w, hi);
           const int at = i * STEP * 128 + ((((lane & 15) >> 1) ^ ((r0 + STEP * i) & 7)) * 16);
 #pragma unroll
           for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(dst + q * w_part + at) = make_uint2(lo[q], hi[q]);

@@ -401,10 +401,6 @@ segment_join_kernel(const __grid_constant__ ScanArgs a) {
 #define SC_REC(DP) (416 + (DP) * 49)  // a record before its values, whole lines of 128 bytes
 #define SC_VALUES(Dv) (((Dv) + 16 * SC_TILES - 1) / (16 * SC_TILES) * SC_TILES * 128)
 
-__device__ __forceinline__ void sc_copy16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
-}
-
 template <int DP>
 __global__ void __launch_bounds__(2 * DP, 512 / DP)
 scan_chunk_rows_kernel(const __grid_constant__ ScanArgs a, uint32_t* __restrict__ records) {
@@ -636,7 +632,7 @@ scan_chunk_states_kernel(const __grid_constant__ ScanArgs a, const uint32_t* __r
 #pragma unroll
       for (int x = 0; x < (REC / 4 + NT - 1) / NT; ++x) {
         const int at = (tid + x * NT) * 4;
-        if (at < REC) sc_copy16(dst + at, src + (at < HEAD ? SKIP + at : SC_REC(DP) + blockIdx.y * NC * 128 + at - HEAD));
+        if (at < REC) ds_copy16(dst + at, src + (at < HEAD ? SKIP + at : SC_REC(DP) + blockIdx.y * NC * 128 + at - HEAD));
       }
     }
     asm volatile("cp.async.commit_group;\n" ::);  // also when empty: one group per call

@@ -1,7 +1,16 @@
-// fp32 products of small matrices on mma.sync with every operand as the sum of three bfloat16 (24 bits: nothing is lost) and the
-// six products of parts that matter; shared by the chunked scans of delta_state.cu and linear_state.cu.
+// fp32 products of small matrices on mma.sync with every operand as the sum of three bfloat16 and the six products of parts that
+// matter (the other three are below 2^-24 of a product together); shared by the chunked scans of delta_state.cu and
+// linear_state.cu.  The split also by gemm_f32_split.cuh.
+//
+// Three bfloat16 hold 24 bits, so nothing of a value is lost as long as its third part is one: from about 2^-110 on.  Below, the parts
+// end at the smallest bfloat16, 2^-133, and the value is off by 2^-134 at most (2^-118: 9e-6 of it, 2^-126: 2e-3).  Infinities,
+// and what rounds up to one in bfloat16 (from 3.396e38 on), have no parts: their sum is NaN.
 #pragma once
 #include "mma_tiles.cuh"
+
+__device__ __forceinline__ void ds_copy16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(dst)), "l"(src));
+}
 
 // (x, y) as the sum of three bfloat16 pairs
 __device__ __forceinline__ void ds_split(float x, float y, uint32_t (&p)[3]) {

@@ -160,3 +160,41 @@ def test_scratch_is_bounded_and_gets_smaller_where_there_is_no_room(ops, monkeyp
     monkeypatch.setattr(torch, "empty", little_room)
     assert torch.equal(ops.linear(x[:700], w), want) and len(asked) > 2
     ops.raise_if_kernel_error()
+
+
+@pytest.mark.parametrize("sx,sw", [(2.0 ** -100, 1.0), (2.0 ** -118, 1.0), (2.0 ** -126, 1.0), (1.0, 2.0 ** -118), (2.0 ** -64, 2.0 ** -60)])
+def test_small_operands_are_off_by_the_smallest_bfloat16_at_most(ops, sx, sw):
+    x, w = _matrices(20, 19456, 1088)
+    x, w = x * sx, w * sw
+    want = x.double() @ w.double().t()
+    got = ops.linear(x, w).double()
+    ops.raise_if_kernel_error()
+    # an operand's parts end at 2^-133: half of that each, times the other operands, beside the error of ordinary operands; results
+    # below the normal floats lose up to 2^-149 at every step
+    lost = 2.0 ** -134 * (x.double().abs().sum(1)[:, None] + w.double().abs().sum(1)[None, :])
+    usual = 2.0 ** -24 * 32 * (x.double().square().sum(1).sqrt()[:, None] * w.double().square().sum(1).sqrt()[None, :])
+    assert bool(((got - want).abs() <= lost + usual + 1088 * 2.0 ** -149).all())
+
+
+def test_products_that_are_left_out_are_below_half_a_digit(ops):
+    """Operands just above 1, all alike: their parts' remainders, and so the three products that are left out, have one sign."""
+    value = 1.0038987  # parts 1, 2^-8 - ..., with remainders near the largest
+    x, w = torch.full((17, 1088), value, device="cuda"), torch.full((19456, 1088), value, device="cuda")
+    want = x.double() @ w.double().t()
+    error = float(((ops.linear(x, w).double() - want).abs() / want).max())
+    # the products left out 2^-24, four large steps of a slice towards zero 2^-23 each, the slices' sums 2^-24 each
+    assert error <= 2.0 ** -24 * (1 + 8 + 1088 / 64)
+
+
+def test_products_that_overflow(ops):
+    x, w = torch.zeros((3, 1088), device="cuda"), torch.zeros((19456, 1088), device="cuda")
+    w[:, 5], w[:, 70] = 3.0, 3.0
+    w[7] = -w[7]
+    x[:, 5] = 2e38
+    x[1, 70], x[2, 5] = 1e38, 1e38
+    got, want = ops.linear(x, w), x.double() @ w.double().t()
+    ops.raise_if_kernel_error()
+    assert torch.equal(got.isinf(), want.float().isinf()) and not got.isnan().any()
+    assert torch.equal(got[got.isinf()], want.float()[got.isinf()])
+    finite = ~got.isinf()
+    assert torch.allclose(got[finite].double(), want[finite], rtol=1e-6)
