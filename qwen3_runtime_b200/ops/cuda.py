@@ -289,8 +289,10 @@ class _Span:
 # ---- decayed state scans of bfloat16 steps: token by token or in segments -------------------------
 SCAN_SCRATCH = 1 << 28  # floats a segment scan may ask for (1 GiB): a step that needs more runs in several launches
 
-# Times in us of the scan token by token and of segments run token by token, by the padded key size: what cutting has to win by.
-# (Segments are run in chunks now, which takes 0.55 to 0.75 of these times, see CHUNK_COSTS.)  Least squares over 48 compositions of
+# Times in us of the scan token by token and of segments run token by token, by the padded key size: by these it is decided whether
+# a step is cut.  Segments are run in chunks now, which takes 0.55 to 0.75 of their times here (CHUNK_COSTS): what is cut wins with room
+# to spare, and some short steps that are left would win too (16 heads of 64 x 128, us token by token / in chunks: 128 tokens 36 /
+# 28, beside 8 single ones 47 / 30, four prompts of 64 46 / 26).  Least squares over 48 compositions of
 # sequences (one token to 8,000, alone, in equal numbers and mixed, up to 128 of them) x 6 head counts and sizes x up to 10
 # segment lengths; 8 % off on average.  A pass of the segments takes the longer of one block's chain (`alone` per token)
 # and all blocks at two per SM (`shared` per token, `block` per block); rows and joining cost `row` and `join` more, and
@@ -315,7 +317,7 @@ CHUNK_COSTS = {
 
 
 def _scan_blocks(H, D, Dv):
-    """Blocks of one segment: (head, tile of value columns)."""
+    """Blocks of one segment as SCAN_COSTS counts them: (head, tile of 128 or 64 value columns).  (In chunks a tile is 32 columns.)"""
     return H * -(-Dv // (128 if D <= 64 else 64))
 
 
@@ -334,8 +336,8 @@ def _segments(cu, seg):
 
 def _scan_fits(T, H, D, Dv, segments, cut):
     """Whether a step is small enough to be cut at all: its q, k and decays, and the segments' states, as float32 within 1 GiB.
-    (How far cutting has been measured.  Below it windows cost little: one sequence of 8192 / 10500 tokens, 64 heads of 128 x
-    128, in one launch and in two 1.67 / 1.82 ms, token by token 9.0 / 12.5.)"""
+    (How far cutting has been measured; one sequence of 10500 tokens, 64 heads of 128 x 128, in two launches 1.8 ms, token by token
+    12.5.)"""
     return T * H * 3 * (64 if D <= 64 else 128) + (segments * H * D * (Dv + 1) if cut else 0) <= 1 << 28
 
 
@@ -398,10 +400,10 @@ def decayed_scan_segment(cu, H, D, Dv, sms) -> int:
     """Tokens per segment of a bfloat16 step's decayed state scan, or 0 for the scan token by token, whichever the measured
     costs make the fastest (segments where they win by 5 % at least).  A segment's length follows from the whole step: a few
     prompts are cut so that their blocks fill the SMs once at two each, many short prompts fill them as they are.  16 heads
-    of 64 x 128, us token by token / so: 64 tokens 22 / 22; 512 118 / 65; 2040 446 / 134; 2040 beside 31 single tokens 760 / 190,
-    beside 127 817 / 341; 8 prompts of 256 244 / 155; 32 of 64 246 / 114; over 150 compositions nothing was slower than token by
-    token.  A step of one short prompt and single tokens is never cut where its blocks leave most SMs idle (16 heads of
-    128 x 128, 128 tokens beside 8: 75 / 83)."""
+    of 64 x 128, us token by token / as this and :func:`chunk_segment` choose: 64 tokens 22 / 22; 512 117 / 42; 2048 438 / 87; 2040
+    beside 31 single tokens 573 / 120, beside 127 655 / 241; 8 prompts of 256 237 / 67; 32 of 64 238 / 70; over 88 compositions x 10
+    head counts and sizes nothing was slower than token by token.  A step of one short prompt and single tokens is not cut where
+    its blocks leave most SMs idle, which was the faster way when segments ran token by token."""
     lens = [b - a for a, b in zip(cu, cu[1:])]
     T, longest = sum(lens), max(lens)
     c = SCAN_COSTS[64 if D <= 64 else 128]

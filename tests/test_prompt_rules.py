@@ -226,3 +226,26 @@ def test_windows_cover_a_step_and_fit_their_scratch(monkeypatch):
                 -(-(min(max(b, lo), hi) - min(max(a, lo), hi)) // got) for a, b in zip(cu, cu[1:]))
             assert cuda._scan_scratch(hi - lo, last, heads, dim, vdim, segments, cut) <= cuda.SCAN_SCRATCH
     assert min(some) > 50
+
+
+def test_the_length_that_was_handed_in_stays_only_where_no_other_fits():
+    from qwen3_runtime_b200.ops.cuda import SCAN_SCRATCH, _scan_scratch, _segments, chunk_segment
+
+    kept = chosen = 0
+    for lens in ([2048], [2040] + [1] * 31, [256] * 8, [64] * 32, [17] * 100, [1000, 33, 0, 700], [4000] * 4):
+        cu = _cu(lens)
+        for heads, dim, vdim in ((4, 64, 128), (16, 64, 128), (16, 128, 128), (64, 128, 128)):
+            def fits(seg):
+                count, longest = _segments(cu, seg)
+                return _scan_scratch(sum(lens), len(lens), heads, dim, vdim, count, longest > seg) <= SCAN_SCRATCH
+
+            for seg in (33, 114, 2001):  # none is a multiple of 16
+                lengths = {-(-n // 16) * 16 for n in (32, 64, 96, 128, 192, 256, 512, 1024, seg, max(lens)) if n <= max(lens)}
+                got = chunk_segment(cu, heads, dim, vdim, 148, seg)
+                if any(fits(n) for n in lengths):
+                    chosen += 1
+                    assert got in lengths and fits(got), (lens, heads, dim, seg, got)
+                else:
+                    kept += 1
+                    assert got == seg
+    assert chosen > 60 and kept > 0
