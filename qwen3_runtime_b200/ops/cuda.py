@@ -342,12 +342,9 @@ def _scan_fits(T, H, D, Dv, segments, cut):
 
 
 def _scan_windows(cu, H, D, Dv, seg):
-    """``(seg, windows)``: the step's tokens as runs ``(first token, end, first sequence, end, segments, cut)``, one launch after
-    another, whose scratch is at most SCAN_SCRATCH each.  They end where a segment of ``seg`` tokens ends; a segment that
-    would not fit gets shorter (0: not even 16 tokens fit)."""
-    segments, longest = _segments(cu, seg)
-    if _scan_scratch(cu[-1], len(cu) - 1, H, D, Dv, segments, longest > seg) <= SCAN_SCRATCH:
-        return seg, [(cu[0], cu[-1], 0, len(cu) - 1, segments, longest > seg)]
+    """``(seg, windows)``: a step that is too large as runs of tokens ``(first, end, first sequence, end, segments, cut)``, one
+    launch after another, whose scratch is at most SCAN_SCRATCH each.  They end where a segment of ``seg`` tokens ends; a segment
+    that would not fit gets shorter (0: not even 16 tokens fit)."""
     record, state = _scan_scratch(0, 1, H, D, Dv, 0, False), H * D * (Dv + 1)
     seg = min(seg, (SCAN_SCRATCH - state - record) // record * 16)
     if seg < 16:
@@ -917,19 +914,22 @@ class CudaOps:
         windows = []
         if seg:
             seg = -(-seg // 16) * 16  # whole chunks
-            seg, windows = _scan_windows(cu, H, D, Dv, seg) if cu else _scan_runs(T, int(num_seqs), H, D, Dv, seg)
+            segments, longest = _segments(cu, seg) if cu else (T // seg + int(num_seqs), T)
+            words = _scan_scratch(T, int(num_seqs), H, D, Dv, segments, longest > seg)
+            windows = [(0, T, 0, int(num_seqs), segments, longest > seg)]
+            if words > SCAN_SCRATCH:
+                seg, windows = _scan_windows(cu, H, D, Dv, seg) if cu else _scan_runs(T, int(num_seqs), H, D, Dv, seg)
+                words = SCAN_SCRATCH
         if windows:
             try:
-                scratch = torch.empty(max(_scan_scratch(hi - lo, last - first, H, D, Dv, segments, cut)
-                                          for lo, hi, first, last, segments, cut in windows),
-                                      dtype=torch.float32, device=q.device)
+                scratch = torch.empty(words, dtype=torch.float32, device=q.device)
             except torch.OutOfMemoryError:
                 windows = []  # token by token needs none
         for lo, hi, first, last, segments, cut in windows:
             self.launches += 1 + 2 * int(cut)
             self._call("linear_state", "q3_decayed_segment_scan", "decayed_state_scan", *before,
-                       _ptr(cu_seqlens[first:]), _ptr(state_slots[first:]), _ptr(out), last - first, *after, seg, segments,
-                       int(cut), _ptr(scratch), lo, hi)
+                       _ptr(cu_seqlens) + 4 * first, _ptr(state_slots) + 4 * first, _ptr(out), last - first, *after, seg,
+                       segments, int(cut), _ptr(scratch), lo, hi)
         if not windows:
             self._call("linear_state", "q3_decayed_state_scan", "decayed_state_scan", *before, _ptr(cu_seqlens),
                        _ptr(state_slots), _ptr(out), int(num_seqs), *after)

@@ -105,3 +105,23 @@ def test_steps_whose_scratch_is_too_large_run_in_windows(ops, monkeypatch, D, Dv
     # the sums over a sequence's segments in another order
     assert float((out[0] - out[1]).abs().max()) <= 3e-5 * float(out[0].abs().max())
     assert float((states[0] - states[1]).abs().max()) <= 3e-5 * float(states[0].abs().max())
+
+
+def test_a_scan_that_is_refused_its_scratch_runs_token_by_token(ops, monkeypatch):
+    from qwen3_runtime_b200.ops import cuda
+
+    q, k, v, kw, start = _step([300, 40], 2, 64, 64)
+    launched, call = [], ops._call
+
+    def spy(group, name, what, *args):
+        launched.append(name)
+        return call(group, name, what, *args)
+
+    monkeypatch.setattr(ops, "_call", spy)
+    monkeypatch.setattr(ops, "_scan_segment", lambda *args: 64)
+    want = ops.decayed_state_scan(q, k, v, state=start.clone(), **kw)
+    monkeypatch.setattr(cuda, "SCAN_SCRATCH", 1 << 50)
+    monkeypatch.setattr(cuda, "_scan_scratch", lambda *args: 1 << 45)  # floats: more than any device has
+    got = ops.decayed_state_scan(q, k, v, state=start.clone(), **kw)
+    assert launched == ["q3_decayed_segment_scan", "q3_decayed_state_scan"]
+    assert float((got - want).abs().max()) <= 3e-5 * float(want.abs().max())
