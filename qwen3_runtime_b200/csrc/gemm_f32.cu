@@ -1,7 +1,8 @@
 // C[M, N] = A[M, K] * W[N, K]^T in true fp32 on the FMA pipes: no tensor cores, no
-// TF32 (large weights: gemm_f32_split.cuh, on the tensor cores in three bfloat16 parts).  Every output element is one accumulator that takes its K products in
-// ascending k order, so a row of C does not depend on M, on the tile shape chosen
-// for M, or on where the row sits in the batch.  This is the matrix product of the
+// TF32 (large weights: gemm_f32_split.cuh, on the tensor cores in three bfloat16 parts).
+// Every output element is one accumulator that takes its K products in ascending k
+// order, so a row of C does not depend on M, on the tile shape chosen for M, or on
+// where the row sits in the batch.  This is the matrix product of the
 // engine's 32-bit path (the reference's fp32 path is torch on the CPU,
 // qwen3_runtime/engine/factory.py:136-137).
 //

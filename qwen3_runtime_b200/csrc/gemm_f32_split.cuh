@@ -513,7 +513,8 @@ Q3_EXPORT int q3_gemm_f32_split(const float* A, int lda, const float* W, int ldw
     const double cost = (double)((items + sms - 1) / sms) * (slice < 180000 ? 180000 : slice);
     if (!best || cost < best_cost) best = t, best_cost = cost;
   }
-  Args p = {A, W, lda, ldw, segments > 1 ? planes : C, segments > 1 ? N : ldc, (long)M * N, M, N, K, segments, 0, best, 0, 0, rows, 0, error_word};
+  Args p = {A, W, lda, ldw, segments > 1 ? planes : C, segments > 1 ? N : ldc, (long)M * N, M, N, K, segments, 0, best, 0, 0, rows, 0,
+            error_word};
   const int slices = (K + SLICE - 1) / SLICE;
   p.slices_per_segment = (slices + segments - 1) / segments;
   p.token_tiles = (M + best - 1) / best;
@@ -529,10 +530,11 @@ Q3_EXPORT int q3_gemm_f32_split(const float* A, int lda, const float* W, int ldw
     return Q3_ERR_LAUNCH;
   const cuuint64_t wdims[2] = {(cuuint64_t)K, (cuuint64_t)N}, wstrides[1] = {(cuuint64_t)ldw * 4};
   const cuuint32_t wbox[2] = {SLICE, (cuuint32_t)rows};
-  if (encode(&wmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(W), wdims, wstrides, wbox, es,
+  if (best <= FEW_TOKENS &&
+      encode(&wmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(W), wdims, wstrides, wbox, es,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return Q3_ERR_LAUNCH;
+    return Q3_ERR_LAUNCH;  // (many tokens: not used)
   const int grid = p.items < sms ? p.items : sms;
   if (best <= FEW_TOKENS) {
     p.raw = (MOST_SMEM - smem_bytes(rows, best, 0)) / (rows * SLICE * 4);
