@@ -198,3 +198,18 @@ def test_products_that_overflow(ops):
     assert torch.equal(got[got.isinf()], want.float()[got.isinf()])
     finite = ~got.isinf()
     assert torch.allclose(got[finite].double(), want[finite], rtol=1e-6)
+
+
+@pytest.mark.parametrize("N,K", [(8192, 2560), (20004, 1088), (2564, 8008)])
+def test_edges_of_token_tiles_and_of_the_rows_of_a_pair(ops, N, K):
+    """Token tiles from one 16 to 160, with four, three and two slices of weights' parts in tensor memory; pairs whose second block
+    has few rows or none."""
+    x, w = _matrices(481, N, K, 4)
+    want = x.double() @ w.double().t()
+    whole = ops.linear(x, w)
+    for rows in (1, 16, 17, 31, 32, 48, 49, 63, 64, 65, 80, 111, 112, 113, 127, 128, 129, 144, 160, 161, 176, 319, 320, 321, 480):
+        got = ops.linear(x[:rows], w)
+        ops.raise_if_kernel_error()
+        assert torch.equal(got, whole[:rows]), rows
+    error = float((whole.double() - want).norm() / want.norm())
+    assert error <= 2.0 ** -24 * (6 + (K / 64) ** 0.5)  # (as above)
