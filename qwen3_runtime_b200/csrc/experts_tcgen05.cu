@@ -16,9 +16,13 @@
 // For the gated unit each CTA's 128 rows are 64 gate rows and the 64 up rows of the same features, so that both
 // halves of a feature meet in one CTA's epilogue.
 //
-// Persistent, one CTA per SM, three roles as in gemm_tcgen05.cu: warp 0 one lane TMA producer (6 stages of 16 KB
-// weights + 16 KB slots), warp 1 one lane MMA issuer (leader only), warps 2..5 epilogue (accumulators double-buffered in
-// tensor memory; 32 slots at a time through shared memory, so that a slot's features are stored side by side).
+// Persistent, one CTA per SM, three roles as in gemm_tcgen05.cu: warp 0 TMA producer (6 stages of 16 KB weights + at most 16 KB
+// slots), warp 1 MMA issuer (leader only), warps 2..9 epilogue in two groups (accumulators double-buffered in tensor memory; 32
+// slots at a time through shared memory as bfloat16, so that a slot's features are stored side by side).
+// What held it back beside the bytes: the issue of up to six boxes a k-slice by one lane (60 to 80 cycles each; two boxes now,
+// their lane chosen by elect.sync) and the gated unit in four warps (26,000 cycles a tile of 192 slots, its MMAs 12,300).  2048
+// tokens, us, gate_up / down: 64 experts of 2 x 1408 x 2048, top 6: 180 / 94, two boxes 170 / 92, two groups 158 / 90; 32 of 2 x
+// 2048 x 4096, top 4: 330 / 168, 268 / 137, 262 / 136.  512 tokens of the first: 146 / 84 -> 139 / 82 (5.3 TB/s of weights).
 // Feature tiles of a chunk are neighbours in the tile order: the pairs share its slots' rows in L2.
 //
 // Every wait is bounded; on expiry the waiter raises the block's abort flag and the error word, every role leaves its
@@ -30,15 +34,14 @@ namespace {
 enum { UNIT_NONE = 0, UNIT_RELU2 = 1, UNIT_GLU = 2 };
 constexpr int BK = 64;
 constexpr int STAGES = 6;
-constexpr int THREADS = 192;
+constexpr int THREADS = 64 + 2 * 128;     // two groups of four epilogue warps
 constexpr int A_BYTES = 128 * BK * 2;     // this CTA's 128 weight rows
-constexpr int B_BOX_ROWS = 32;            // slots per TMA box
-constexpr int B_BOX_BYTES = B_BOX_ROWS * BK * 2;
+constexpr int B_ROWS = 32, B_MAPS = 4;    // slots per TMA box: 32, 64, 96 or 128, a tensor map for each
 constexpr int B_BYTES = 128 * BK * 2;     // at most 128 slots per CTA
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int MAX_SLOTS = 256;            // slots per tile
 constexpr int ACC_COLS = 256, TMEM_COLS = 512;
-constexpr int OUT_STRIDE = 144;           // floats per slot in the epilogue's buffer: 128 rows, skewed by 16 banks
+constexpr int OUT_STRIDE = 160;           // bfloat16 per slot in a group's buffer: 128 rows; two slots cover all banks
 
 struct Tile {
   int expert, row0, rows, n, f;  // slots row0 .. row0 + rows of the grouped order; n: rows rounded up to 32; f: feature tile
@@ -64,31 +67,24 @@ __device__ __forceinline__ Tile tile_at(int tile, int ftiles, const int* __restr
   return t;
 }
 
-// First rows of a CTA's two boxes of 64 weight rows of a tile.
-template <int UNIT>
-__device__ __forceinline__ void weight_rows(const Tile& t, int N, int rank, int& w0, int& w1) {
-  if (UNIT == UNIT_GLU) {
-    w0 = t.expert * 2 * N + t.f * 128 + 64 * rank;
-    w1 = w0 + N;
-  } else {
-    w0 = t.expert * N + t.f * 256 + 128 * rank;
-    w1 = w0 + 64;
-  }
-}
+// The tensor maps of a product: weights as [2E][N][K] (gated: a box is 64 rows of a gate and the 64 of its up matrix) or
+// [E * N][K], and the slots' rows with every height of a box.
+struct Maps {
+  CUtensorMap w, x[B_MAPS];
+};
 
 template <int UNIT>
 __global__ void __launch_bounds__(THREADS, 1)
-expert_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
-                      bf16* __restrict__ out, int N, int K, int E, const int* __restrict__ offsets,
-                      const int* __restrict__ tile_offsets, float limit, float alpha, float up_offset,
-                      int* __restrict__ error_word) {
+expert_tcgen05_kernel(const __grid_constant__ Maps maps, bf16* __restrict__ out, int N, int K, int E,
+                      const int* __restrict__ offsets, const int* __restrict__ tile_offsets, float limit, float alpha,
+                      float up_offset, int* __restrict__ error_word) {
   constexpr int TILE_F = UNIT == UNIT_GLU ? 128 : 256;  // features per tile; half of them in each CTA
   extern __shared__ unsigned char smem_raw[];
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  float* stage_out = reinterpret_cast<float*>(tiles + (size_t)STAGES * STAGE_BYTES);  // [32 slots][OUT_STRIDE]
+  bf16* stage_out = reinterpret_cast<bf16*>(tiles + (size_t)STAGES * STAGE_BYTES);  // [2 groups][32 slots][OUT_STRIDE]
   __shared__ __align__(8) unsigned long long bars[2 * STAGES + 5];
   __shared__ uint32_t tmem_base_s;
-  __shared__ volatile int abort_flag, epilogue_gave_up;
+  __shared__ volatile int abort_flag, gave_up[2];
   int issued = 0;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -102,14 +98,14 @@ expert_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
   const uint32_t drained = smem_addr(&bars[2 * STAGES + 4]);
 
   if (threadIdx.x == 0) {
-    abort_flag = epilogue_gave_up = 0;
+    abort_flag = gave_up[0] = gave_up[1] = 0;
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(full0 + 8 * s, 1);
       mbar_init(empty0 + 8 * s, 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(acc_full0 + 8 * b, 1);
-      mbar_init(acc_empty0 + 8 * b, 8);  // one arrival per epilogue warp of both CTAs (used in the leader)
+      mbar_init(acc_empty0 + 8 * b, 16);  // one arrival per epilogue warp of both CTAs (used in the leader)
     }
     mbar_init(drained, 1);
     mbar_init_fence();
@@ -129,63 +125,74 @@ expert_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
   pdl_launch_dependents();
   const int num_tiles = tile_offsets[E] * ftiles;
 
-  if (warp == 0) {
-    if (lane == 0) {  // ---- TMA producer ---------------------------------------------------------------
-      const uint32_t leader_full0 = map_to_cta(full0, 0);
-      int g = 0;
-      bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-        const Tile t = tile_at(tile, ftiles, offsets, tile_offsets, E);
-        int w0, w1;
-        weight_rows<UNIT>(t, N, rank, w0, w1);
-        const int half = t.n / 2, boxes = (half + B_BOX_ROWS - 1) / B_BOX_ROWS;
-        const int x0 = t.row0 + (int)rank * half;
-        const uint32_t bytes = A_BYTES + boxes * B_BOX_BYTES;
-        for (int kb = 0; kb < num_kb; ++kb, ++g) {
-          const int s = g % STAGES;
-          ok = mbar_wait(empty0 + 8 * s, ((g / STAGES) & 1) ^ 1, &abort_flag);
-          if (!ok) break;
-          const uint32_t dst = smem_addr(tiles + (size_t)s * STAGE_BYTES);
+  if (warp == 0) {  // ---- TMA producer: one lane chosen by elect.sync, two boxes a k-slice ---------------------------
+    const bool chosen = elect_one();
+    const uint32_t leader_full0 = __shfl_sync(0xffffffffu, map_to_cta(full0, 0), 0), tiles0 = smem_addr(tiles);
+    int s = 0;
+    uint32_t phase = 1;
+    bool ok = true;
+    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+      const Tile t = tile_at(tile, ftiles, offsets, tile_offsets, E);
+      const int w_row = (UNIT == UNIT_GLU ? 0 : t.expert * N) + t.f * TILE_F + (TILE_F / 2) * (int)rank;
+      const int w_mat = UNIT == UNIT_GLU ? 2 * t.expert : 0;
+      const int half = t.n / 2, box = (half + B_ROWS - 1) / B_ROWS;
+      const int x0 = t.row0 + (int)rank * half;
+      const uint32_t bytes = A_BYTES + box * (B_ROWS * BK * 2);
+      const CUtensorMap* xmap = &maps.x[box - 1];
+      for (int kb = 0; kb < num_kb; ++kb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, phase, &abort_flag));
+        if (!ok) break;
+        const uint32_t dst = tiles0 + (uint32_t)s * STAGE_BYTES;
+        if (chosen) {
           if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * bytes);  // this CTA's boxes and the peer's
-          tma_load_2d_pair(dst, &tmap_w, leader_full0 + 8 * s, kb * BK, w0);
-          tma_load_2d_pair(dst + A_BYTES / 2, &tmap_w, leader_full0 + 8 * s, kb * BK, w1);
-          for (int b = 0; b < boxes; ++b)
-            tma_load_2d_pair(dst + A_BYTES + b * B_BOX_BYTES, &tmap_x, leader_full0 + 8 * s, kb * BK, x0 + b * B_BOX_ROWS);
-          issued = g + 1;
+          tma_load_3d_pair(dst, &maps.w, leader_full0 + 8 * s, kb * BK, w_row, w_mat);
+          tma_load_2d_pair(dst + A_BYTES, xmap, leader_full0 + 8 * s, kb * BK, x0);
         }
+        ++issued;
+        if (++s == STAGES) s = 0, phase ^= 1;
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {  // ---- MMA issuer of the pair -------------------------------------------
-      int g = 0, i = 0;
+    if (rank == 0) {  // ---- MMA issuer of the pair, one lane chosen by elect.sync ------------------------------------
+      const bool chosen = elect_one();
+      const uint32_t acc0 = __shfl_sync(0xffffffffu, tmem_base, 0), tiles0 = smem_addr(tiles);
+      int s = 0, i = 0;
+      uint32_t phase = 0;
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++i) {
         const Tile t = tile_at(tile, ftiles, offsets, tile_offsets, E);
         const uint32_t idesc = umma_idesc(256, t.n);
         const int buf = i & 1;
-        ok = mbar_wait(acc_empty0 + 8 * buf, ((i >> 1) & 1) ^ 1, &abort_flag);  // both epilogues have drained it
+        // both epilogues have drained it
+        ok = __all_sync(0xffffffffu, mbar_wait(acc_empty0 + 8 * buf, ((i >> 1) & 1) ^ 1, &abort_flag));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t acc = tmem_base + buf * ACC_COLS;
-        for (int kb = 0; kb < num_kb; ++kb, ++g) {
-          const int s = g % STAGES;
-          ok = mbar_wait(full0 + 8 * s, (g / STAGES) & 1, &abort_flag);
+        const uint32_t acc = acc0 + buf * ACC_COLS;
+        for (int kb = 0; kb < num_kb; ++kb) {
+          ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, phase, &abort_flag));
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a_addr = smem_addr(tiles + (size_t)s * STAGE_BYTES);
+          const uint32_t a_addr = tiles0 + (uint32_t)s * STAGE_BYTES;
           const uint64_t a_desc = umma_desc(a_addr), b_desc = umma_desc(a_addr + A_BYTES);
+          if (chosen) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k)
-            umma_pair(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          umma_commit_pair(empty0 + 8 * s);
+            for (int k = 0; k < BK / 16; ++k)
+              umma_pair(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            umma_commit_pair(empty0 + 8 * s);
+          }
+          __syncwarp();
+          if (++s == STAGES) s = 0, phase ^= 1;
         }
-        if (ok) umma_commit_pair(acc_full0 + 8 * buf);
+        if (ok && chosen) umma_commit_pair(acc_full0 + 8 * buf);
+        __syncwarp();
       }
     }
-  } else {  // ---- epilogue: warp w reads TMEM lanes 32 * (w % 4) .. + 31 of this CTA -------------------------
-    const int quarter = warp & 3, et = threadIdx.x - 64;
+  } else {  // ---- epilogue: warp w reads TMEM lanes 32 * (w % 4) .. + 31 of this CTA, a group every other 32 slots -------
+    const int group = (warp - 2) >> 2, quarter = warp & 3, et = (threadIdx.x - 64) & 127;
     const int slot_in = et >> 2, part = et & 3;  // second half: four threads per slot
     const uint32_t leader_acc_empty0 = map_to_cta(acc_empty0, 0);
+    bf16* const staged = stage_out + group * 32 * OUT_STRIDE;
+    auto meet = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(group + 1) : "memory"); };
     int i = 0;
     bool ok = true;
     for (int tile = pair; tile < num_tiles; tile += num_pairs, ++i) {
@@ -193,60 +200,57 @@ expert_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
       const int buf = i & 1;
       const int f0 = t.f * TILE_F + (int)rank * (TILE_F / 2);
       ok = mbar_wait(acc_full0 + 8 * buf, (i >> 1) & 1, &abort_flag);
-      if (!ok) epilogue_gave_up = 1;  // one warp may give up where another saw the barrier complete: the four agree
+      if (!ok) gave_up[group] = 1;  // one warp may give up where another saw the barrier complete: the four agree
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (epilogue_gave_up) break;
+      meet();
+      if (gave_up[group]) break;
       const uint32_t lane_addr = tmem_base + buf * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
+      if (group * 32 >= t.n && lane == 0) remote_arrive_only(leader_acc_empty0 + 8 * buf);  // nothing here for this group
 #pragma unroll 1
-      for (int c0 = 0; c0 < t.n; c0 += 32) {
+      for (int c0 = group * 32; c0 < t.n; c0 += 64) {
         uint32_t acc[32];
         tmem_load32(lane_addr + c0, acc);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (c0 + 32 >= t.n) {  // everything of this buffer is in registers: hand it back to the MMA issuer
+        if (c0 + 64 >= t.n) {  // the last of this buffer for this group is in registers: hand it back to the MMA issuer
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          if (lane == 0) remote_arrive(leader_acc_empty0 + 8 * buf);
+          if (lane == 0) remote_arrive_only(leader_acc_empty0 + 8 * buf);
         }
+        // (whatever follows takes the products rounded to bfloat16, as separate kernels would)
 #pragma unroll
-        for (int c = 0; c < 32; ++c) stage_out[c * OUT_STRIDE + quarter * 32 + lane] = __uint_as_float(acc[c]);
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        for (int c = 0; c < 32; ++c) staged[c * OUT_STRIDE + quarter * 32 + lane] = from_f32<bf16>(__uint_as_float(acc[c]));
+        meet();
         if (c0 + slot_in < t.rows) {
           bf16* row = out + (long)(t.row0 + c0 + slot_in) * N;
-          const float* src = stage_out + slot_in * OUT_STRIDE;
+          const bf16* src = staged + slot_in * OUT_STRIDE;
 #pragma unroll
-          for (int j = 0; j < TILE_F / 32; ++j) {
-            const int f = 4 * (part + 4 * j);
+          for (int j = 0; j < TILE_F / 64; ++j) {
+            const int f = 8 * (part + 4 * j);
             if (f0 + f >= N) continue;  // N is a multiple of 8
-            float v[4];
-            const float4 a = *reinterpret_cast<const float4*>(src + f);
-            const float av[4] = {a.x, a.y, a.z, a.w};
-            if (UNIT == UNIT_GLU) {
-              // both products are rounded to bfloat16 before the gated unit, as two separate products followed by
-              // an activation kernel would
-              const float4 b = *reinterpret_cast<const float4*>(src + 64 + f);
-              const float bv[4] = {b.x, b.y, b.z, b.w};
+            if (UNIT != UNIT_NONE) {
+              float a[8], v[8];
+              load8(src + f, a);
+              if (UNIT == UNIT_GLU) {
+                float b[8];
+                load8(src + 64 + f, b);
 #pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float gt = fminf(to_f32(from_f32<bf16>(av[e])), limit);
-                const float up = fminf(fmaxf(to_f32(from_f32<bf16>(bv[e])), -limit), limit);
-                v[e] = (gt / (1.f + expf(-alpha * gt))) * (up + up_offset);
-              }
-            } else if (UNIT == UNIT_RELU2) {
+                for (int e = 0; e < 8; ++e) {
+                  const float gt = fminf(a[e], limit), up = fminf(fmaxf(b[e], -limit), limit);
+                  v[e] = (gt / (1.f + expf(-alpha * gt))) * (up + up_offset);
+                }
+              } else {
 #pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float r = fmaxf(to_f32(from_f32<bf16>(av[e])), 0.f);
-                v[e] = r * r;
+                for (int e = 0; e < 8; ++e) {
+                  const float r = fmaxf(a[e], 0.f);
+                  v[e] = r * r;
+                }
               }
+              store8(row + f0 + f, v);
             } else {
-#pragma unroll
-              for (int e = 0; e < 4; ++e) v[e] = av[e];
+              *reinterpret_cast<uint4*>(row + f0 + f) = *reinterpret_cast<const uint4*>(src + f);
             }
-            __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
-            *reinterpret_cast<uint2*>(row + f0 + f) =
-                make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
           }
         }
-        asm volatile("bar.sync 1, 128;" ::: "memory");  // the buffer is free again
+        meet();  // the buffer is free again
       }
     }
   }
@@ -306,13 +310,24 @@ __global__ void gather_slots_kernel(const bf16* __restrict__ h, long h_stride, c
   }
 }
 
-constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + 32 * OUT_STRIDE * sizeof(float) + 1024;
+constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + 2 * 32 * OUT_STRIDE * sizeof(bf16) + 1024;
 
 template <int UNIT>
 int launch(const void* w, long w_rows, const void* x, void* out, int S, int E, int N, int K, const int* offsets,
            const int* tile_offsets, float limit, float alpha, float up_offset, int* error_word, cudaStream_t stream) {
-  CUtensorMap tw, tx;
-  if (!q3_bf16_map(&tw, w, w_rows, K, K, 64) || !q3_bf16_map(&tx, x, S, K, K, B_BOX_ROWS)) return Q3_ERR_LAUNCH;
+  Maps maps;
+  const bool glu = UNIT == UNIT_GLU;
+  const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)(glu ? N : w_rows), (cuuint64_t)(glu ? 2 * E : 1)};
+  const cuuint64_t strides[2] = {(cuuint64_t)K * 2, (cuuint64_t)K * 2 * dims[1]};
+  const cuuint32_t box[3] = {BK, glu ? 64u : 128u, glu ? 2u : 1u}, es[3] = {1, 1, 1};
+  Q3EncodeTiledFn encode = q3_encode_tiled();
+  if (!encode ||
+      encode(&maps.w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(w), dims, strides, box, es,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return Q3_ERR_LAUNCH;
+  for (int i = 0; i < B_MAPS; ++i)
+    if (!q3_bf16_map(&maps.x[i], x, S, K, K, B_ROWS * (i + 1))) return Q3_ERR_LAUNCH;
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(THREADS);
   cfg.dynamicSmemBytes = SMEM;
@@ -345,7 +360,7 @@ int launch(const void* w, long w_rows, const void* x, void* out, int S, int E, i
   constexpr int TILE_F = UNIT == UNIT_GLU ? 128 : 256;
   const long most = ((long)S / MAX_SLOTS + (E < S ? E : S)) * ((N + TILE_F - 1) / TILE_F);
   cfg.gridDim = dim3((unsigned)(2 * (most < pairs ? most : pairs)));
-  return cudaLaunchKernelEx(&cfg, expert_tcgen05_kernel<UNIT>, tw, tx, (bf16*)out, N, K, E, offsets, tile_offsets, limit,
+  return cudaLaunchKernelEx(&cfg, expert_tcgen05_kernel<UNIT>, maps, (bf16*)out, N, K, E, offsets, tile_offsets, limit,
                             alpha, up_offset, error_word) == cudaSuccess
              ? Q3_OK
              : Q3_ERR_LAUNCH;

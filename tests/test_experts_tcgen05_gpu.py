@@ -107,3 +107,11 @@ def test_router_in_every_batch(ops, tokens, experts, mode):
     for rows in (slice(0, 1), slice(tokens // 2, tokens)):
         c, w = ops.route_top(h[rows], router, 5, score=mode)
         assert torch.equal(c, chosen[rows]) and torch.equal(w, weights[rows])
+
+
+@pytest.mark.parametrize("counts", [[33, 64, 65, 96, 97, 128], [129, 160, 161, 192, 193, 224], [225, 256, 300, 20, 384, 500]])
+@pytest.mark.parametrize("unit", ["clamped_glu", "relu2"])
+def test_every_height_of_a_box_of_slots(ops, monkeypatch, counts, unit):
+    """Boxes of 32 to 128 rows, an odd and an even number of 32 slots for the two groups of the epilogue."""
+    monkeypatch.setitem(globals(), "COUNTS", counts)
+    test_products_against_their_statement(ops, 128, 392, unit, "input" if unit == "clamped_glu" else "output", 0)
