@@ -20,18 +20,22 @@
 // token's result does not depend on which other tokens chose the same expert.  Nothing here reads
 // a count back on the host: grids are sized for the worst case and surplus blocks leave at once.
 #include "common.cuh"
+#include "split_mma.cuh"
 
 constexpr int EXPERT_BM = 32;  // slots per row tile of the FMA products
 
 // ---- router ------------------------------------------------------------------------------------
-// Logits, then the choice.  Two kernels compute logits, with the same order of additions (a token's logits are the same bits
-// in every batch): lane l adds the products of k = 4 l .. 4 l + 3, then of those + 128, and so on; the lanes' sums are added by
-// halving.
-//   few tokens (route_logits): a block stages 2 tokens' rows in shared memory as fp32, each of its eight warps streams one
-//   expert's router row for them, so that a decode step's router runs on tens of SMs;
-//   many tokens (route_logits_tile): a warp keeps 8 tokens x 8 experts in registers and reads operands straight from L1.  With
-//   fewer experts a warp the reads of the tokens' values, not the FMAs, set the time: 2048 tokens x 64 experts x 2048 27 us,
-//   with four experts per warp 47 (FMAs alone: 7).
+// Logits, then the choice.  A token's logits are the same bits in every batch.
+//   bfloat16 tokens (route_logits_mma): mma.sync with the router's float32 as the sum of three bfloat16 (split_mma.cuh).  A block's
+//   eight warps share the width in equal runs of 32-value slices; a slice's six products are one chain, smallest first, its result
+//   is added to float32 sums; the warps' sums are added in order.  Blocks of 32 tokens x 32 experts where there are enough of
+//   them, else 16 x 8: the bits do not depend on it.  What is NaN is worked out once more with FMAs, as parts of infinities have
+//   no sum.  With the choice, us, FMAs (the float32 form) / here: 2048 tokens x 64 experts x 2048 31.2 / 14.3, 8 tokens 8.3 / 5.5,
+//   2048 x 32 x 4096 29.8 / 21.0, 2048 x 256 x 2048 80 / 42; relative error against float64 1.6e-7 .. 2.1e-7 / 1.0e-7 .. 1.1e-7.
+//   float32 tokens: lane l adds the products of k = 4 l .. 4 l + 3, then of those + 128, and so on; the lanes' sums are added by
+//   halving.  Few tokens (route_logits): a block stages 2 tokens' rows in shared memory, each of its eight warps streams one
+//   expert's router row for them.  Many tokens (route_logits_tile): a warp keeps 8 tokens x 8 experts in registers and reads
+//   operands straight from L1.
 // Three kernels choose, one warp per token: the `top` largest logits -- the choice is made on the logits, which order the
 // experts as their sigmoids do but do not collapse into ties where the sigmoid saturates; lowest index on an exact tie, NaN
 // after every number -- with logits in registers (route_pick_regs, up to 256 outputs) or in memory (route_pick), and the choice
@@ -148,9 +152,156 @@ route_logits_tile_kernel(const T* __restrict__ h, long h_stride, const float* __
     }
 }
 
+// MT x 16 tokens and NT x 8 experts a block.  Lane (g, t4) = (lane / 4, lane % 4) of a fragment holds rows g (and g + 8) and, of a
+// slice, k = 8 t4 .. 8 t4 + 7, half of them for each of two MMAs: the order of k within a slice is the same for both operands.
+// VEC: rows of both start at 16-byte boundaries and the width is a multiple of 8.
+constexpr int ROUTE_SLICE = 32, ROUTE_WARPS = 8;
+template <int MT, int NT, bool VEC>
+__global__ void __launch_bounds__(32 * ROUTE_WARPS)
+route_logits_mma_kernel(const bf16* __restrict__ h, long h_stride, const float* __restrict__ router, int num_tokens, int E,
+                        int W, float* __restrict__ logits) {
+  __shared__ float parts[ROUTE_WARPS][MT * 16][NT * 8 + 1];
+  pdl_wait();
+  pdl_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  const int t0 = blockIdx.x * (16 * MT), e0 = blockIdx.y * (8 * NT);
+  const bf16* x[MT][2];  // (what lies beyond the last token or expert is read as that one, and not stored)
+  const float* w[NT];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) x[m][r] = h + (long)min(t0 + m * 16 + r * 8 + g, num_tokens - 1) * h_stride;
+#pragma unroll
+  for (int n = 0; n < NT; ++n) w[n] = router + (long)min(e0 + n * 8 + g, E - 1) * W;
+  uint4 a[MT][2];
+  float b[NT][8];
+  auto load = [&](int slice) {
+    const int k = slice * ROUTE_SLICE + 8 * t4;
+    if (VEC) {
+      const bool in = k < W;
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+          a[m][r] = in ? __ldg(reinterpret_cast<const uint4*>(x[m][r] + k)) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int i = 0; i < 8; i += 4) {
+          const float4 v = in ? __ldg(reinterpret_cast<const float4*>(w[n] + k + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          b[n][i] = v.x, b[n][i + 1] = v.y, b[n][i + 2] = v.z, b[n][i + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          uint32_t p[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const bf16 lo = k + 2 * i < W ? x[m][r][k + 2 * i] : from_f32<bf16>(0.f);
+            const bf16 hi = k + 2 * i + 1 < W ? x[m][r][k + 2 * i + 1] : from_f32<bf16>(0.f);
+            p[i] = (uint32_t)__bfloat16_as_ushort(lo) | (uint32_t)__bfloat16_as_ushort(hi) << 16;
+          }
+          a[m][r] = make_uint4(p[0], p[1], p[2], p[3]);
+        }
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) b[n][i] = k + i < W ? w[n][k + i] : 0.f;
+    }
+  };
+  float sum[MT][NT][4];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sum[m][n][j] = 0.f;
+  const int slices = (W + ROUTE_SLICE - 1) / ROUTE_SLICE, per = (slices + ROUTE_WARPS - 1) / ROUTE_WARPS;
+  const int last = min(slices, (warp + 1) * per);
+  int slice = warp * per;
+  if (slice < last) load(slice);
+  for (; slice < last; ++slice) {
+    uint32_t left[MT][2][4], right[NT][2][2][3];  // by MMA; right: pairs of k, parts
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      const uint32_t lo[4] = {a[m][0].x, a[m][0].y, a[m][0].z, a[m][0].w}, hi[4] = {a[m][1].x, a[m][1].y, a[m][1].z, a[m][1].w};
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        left[m][i][0] = lo[2 * i];
+        left[m][i][1] = hi[2 * i];
+        left[m][i][2] = lo[2 * i + 1];
+        left[m][i][3] = hi[2 * i + 1];
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ds_split(b[n][2 * i], b[n][2 * i + 1], right[n][i >> 1][i & 1]);
+    if (slice + 1 < last) load(slice + 1);  // on its way while this one is multiplied
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        float acc[4];
+        ds_mma_zero(acc, left[m][0], right[n][0][0][2], right[n][0][1][2]);
+        mma_bf16(acc, left[m][1], right[n][1][0][2], right[n][1][1][2]);
+#pragma unroll
+        for (int part = 1; part >= 0; --part)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) mma_bf16(acc, left[m][i], right[n][i][0][part], right[n][i][1][part]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sum[m][n][j] += acc[j];
+      }
+  }
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) parts[warp][m * 16 + g + 4 * (j & 2)][n * 8 + 2 * t4 + (j & 1)] = sum[m][n][j];
+  __syncthreads();
+  constexpr int OUT = MT * 16 * NT * 8;
+#pragma unroll 1
+  for (int i = threadIdx.x; i - lane < OUT; i += 32 * ROUTE_WARPS) {  // (whole warps)
+    const int t = i / (NT * 8), e = i - t * (NT * 8);
+    const bool live = i < OUT && t0 + t < num_tokens && e0 + e < E;
+    float v = 0.f;
+    if (live) {
+      v = parts[0][t][e];
+#pragma unroll
+      for (int p = 1; p < ROUTE_WARPS; ++p) v += parts[p][t][e];
+    }
+    for (uint32_t none = __ballot_sync(0xffffffffu, v != v); none; none &= none - 1) {
+      const int from = i - lane + __ffs(none) - 1, ft = from / (NT * 8), fe = from - ft * (NT * 8);
+      const bf16* xr = h + (long)(t0 + ft) * h_stride;
+      const float* wr = router + (long)(e0 + fe) * W;
+      float again = 0.f;
+      for (int k = lane; k < W; k += 32) again = fmaf(to_f32(xr[k]), wr[k], again);
+      again = warp_sum(again);
+      if (lane == __ffs(none) - 1) v = again;
+    }
+    if (live) logits[(long)(t0 + t) * E + e0 + e] = v;
+  }
+}
+
 // The same choice as route_pick_kernel for up to 32 * PICK_REGS outputs: a token's logits are read once, all loads in
-// flight together, and wait in registers (one warp per token; lane l holds outputs l, l + 32, ...).
+// flight together, and wait in registers (one warp per token; lane l holds outputs l, l + 32, ...) as whole numbers of their order,
+// so that a choice is two reductions over the warp.  (2048 tokens, 6 of 64: with ten shuffles a choice 8.3 us; logits and choice
+// 18.7 -> 14.3.)
 constexpr int PICK_REGS = 8;
+
+// 0 for NaN; else larger for a larger number, the same for both zeros
+__device__ __forceinline__ uint32_t order_of(float x) {
+  const uint32_t b = __float_as_uint(x + 0.f);
+  return x != x ? 0u : b & 0x80000000u ? ~b : b | 0x80000000u;
+}
+__device__ __forceinline__ float number_of(uint32_t order) {
+  return order ? __uint_as_float(order & 0x80000000u ? order & 0x7fffffffu : ~order) : -INFINITY;
+}
+
+template <int REGS>
 __global__ void route_pick_regs_kernel(const float* __restrict__ logits, int num_tokens, int E, int top, int mode,
                                        float scale, int* __restrict__ chosen, float* __restrict__ weights) {
   pdl_wait();
@@ -158,53 +309,51 @@ __global__ void route_pick_regs_kernel(const float* __restrict__ logits, int num
   const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= num_tokens) return;
   const float* z = logits + (long)t * E;
-  float v[PICK_REGS];
+  float v[REGS];
+  uint32_t order[REGS], open = 0;  // open: outputs of this lane that exist and have not been taken
 #pragma unroll
-  for (int r = 0; r < PICK_REGS; ++r) v[r] = lane + 32 * r < E ? z[lane + 32 * r] : -INFINITY;
-  uint32_t open = 0;  // outputs of this lane that exist and have not been taken
+  for (int r = 0; r < REGS; ++r) v[r] = lane + 32 * r < E ? z[lane + 32 * r] : 0.f;
 #pragma unroll
-  for (int r = 0; r < PICK_REGS; ++r) open |= (lane + 32 * r < E ? 1u : 0u) << r;
-  float total = 0.f, first = 0.f;
-  float mine[PICK_REGS];  // lane k % 32 keeps the score of choice k
+  for (int r = 0; r < REGS; ++r) {
+    order[r] = order_of(v[r]);
+    open |= (lane + 32 * r < E ? 1u : 0u) << r;
+  }
+  float mine[REGS];  // lane k % 32 keeps the logit of choice k, then its score
+  int index[REGS];
 #pragma unroll
-  for (int r = 0; r < PICK_REGS; ++r) mine[r] = 0.f;
+  for (int r = 0; r < REGS; ++r) mine[r] = 0.f, index[r] = 0;
+  float first = 0.f;
   for (int k = 0; k < top; ++k) {
-    float best = -INFINITY;
-    int at = 0x7fffffff;
+    uint32_t best = 0;
+    int at = 0x7fffffff;  // (where nothing but NaN is left: the lowest open output)
 #pragma unroll
-    for (int r = 0; r < PICK_REGS; ++r)
-      if ((open >> r & 1u) && (v[r] > best || (v[r] == best && lane + 32 * r < at))) {
-        best = v[r];
+    for (int r = REGS - 1; r >= 0; --r)
+      if ((open >> r & 1u) && order[r] >= best) {
+        best = order[r];
         at = lane + 32 * r;
       }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oa = __shfl_xor_sync(0xffffffffu, at, o);
-      if (ob > best || (ob == best && oa < at)) {
-        best = ob;
-        at = oa;
-      }
-    }
-    if (at >= E) {  // nothing but NaN is left: the lowest open output
-      int low = open ? lane + 32 * (__ffs(open) - 1) : 0x7fffffff;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) low = min(low, __shfl_xor_sync(0xffffffffu, low, o));
-      at = low;
-    }
-    if (k == 0) first = best;  // the largest logit: the softmax's reference point
-    const float score = mode == 2 ? expf(best - first) : 1.f / (1.f + expf(-best));
-    if (lane == 0) chosen[(long)t * top + k] = at;
+    const uint32_t most = __reduce_max_sync(0xffffffffu, best);
+    at = (int)__reduce_min_sync(0xffffffffu, best == most ? (uint32_t)at : 0x7fffffffu);
     if ((at & 31) == lane) open &= ~(1u << (at >> 5));
+    if (k == 0) first = number_of(most);  // the largest logit: the softmax's reference point
 #pragma unroll
-    for (int r = 0; r < PICK_REGS; ++r)
-      if (k == lane + 32 * r) mine[r] = score;
-    total += score;
+    for (int r = 0; r < REGS; ++r)
+      if (k == lane + 32 * r) mine[r] = number_of(most), index[r] = at;
   }
 #pragma unroll
-  for (int r = 0; r < PICK_REGS; ++r) {
+  for (int r = 0; r < REGS; ++r) mine[r] = mode == 2 ? expf(mine[r] - first) : 1.f / (1.f + expf(-mine[r]));
+  float total = 0.f;
+  if (mode)
+#pragma unroll
+    for (int r = 0; r < REGS; ++r)
+      for (int k = 32 * r; k < min(top, 32 * r + 32); ++k) total += __shfl_sync(0xffffffffu, mine[r], k & 31);
+#pragma unroll
+  for (int r = 0; r < REGS; ++r) {
     const int k = lane + 32 * r;
-    if (k < top) weights[(long)t * top + k] = (mode ? mine[r] / total : mine[r]) * scale;
+    if (k < top) {
+      chosen[(long)t * top + k] = index[r];
+      weights[(long)t * top + k] = (mode ? mine[r] / total : mine[r]) * scale;
+    }
   }
 }
 
@@ -356,40 +505,44 @@ Q3_EXPORT int q3_route_top(int dtype, const void* h, long h_stride, const float*
   if (num_tokens == 0) return Q3_OK;
   if (reinterpret_cast<uintptr_t>(router) & 15) return Q3_ERR_UNSUPPORTED;
   if (dtype != Q3_DTYPE_F32 && dtype != Q3_DTYPE_BF16) return Q3_ERR_ARGUMENT;
-  const size_t elem = dtype == Q3_DTYPE_F32 ? 4 : 2;
-  // both kernels give the same bits; the tile kernel needs about 64 tokens to fill the SMs
-  const bool tile = num_tokens > 64 && E >= ROUTE_EPW && W % 4 == 0 && h_stride % 4 == 0 &&
-                    (reinterpret_cast<uintptr_t>(h) & (4 * elem - 1)) == 0;
-  // a block's four warps all have experts: 8 experts x 1024, 4096 tokens 23 us, with three idle warps a block 30
-  const int we = E > 2 * ROUTE_EPW ? 4 : E > ROUTE_EPW ? 2 : 1;
-  const int te = we * ROUTE_EPW, tokens = 4 / we * ROUTE_TT;
   cudaError_t e;
-  if (tile && (E + te - 1) / te <= 65535) {
-    const dim3 grid((num_tokens + tokens - 1) / tokens, (E + te - 1) / te);
-#define Q3_ROUTE_TILE(T_, WT_, WE_)                                                                                      \
-  e = launch_pdl(route_logits_tile_kernel<T_, WT_, WE_>, grid, dim3(32 * WT_ * WE_), 0, stream, (const T_*)h, h_stride, \
+  if (dtype == Q3_DTYPE_BF16) {
+    const bool vec = W % 8 == 0 && h_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0;
+    const dim3 large((num_tokens + 31) / 32, (E + 31) / 32), small((num_tokens + 15) / 16, (E + 7) / 8);
+    if (small.y > 65535) return Q3_ERR_UNSUPPORTED;
+#define Q3_ROUTE_MMA(MT_, NT_, VEC_, grid_)                                                                              \
+  e = launch_pdl(route_logits_mma_kernel<MT_, NT_, VEC_>, grid_, dim3(32 * ROUTE_WARPS), 0, stream, (const bf16*)h, h_stride, \
                  router, num_tokens, E, W, logits)
-#define Q3_ROUTE_TILES(T_)                                                                                               \
-  do { if (we == 4) Q3_ROUTE_TILE(T_, 1, 4); else if (we == 2) Q3_ROUTE_TILE(T_, 2, 2); else Q3_ROUTE_TILE(T_, 4, 1); } while (0)
-    if (dtype == Q3_DTYPE_F32) Q3_ROUTE_TILES(float); else Q3_ROUTE_TILES(bf16);
-#undef Q3_ROUTE_TILES
-#undef Q3_ROUTE_TILE
+    // large blocks from where they fill half of the SMs, and where 32 experts are not mostly none (8 x 512, 4096 tokens: 13.7 us
+    // with the choice, 6.1 with small blocks)
+    if (vec && E > 16 && (long)large.x * large.y >= 74) Q3_ROUTE_MMA(2, 4, true, large);
+    else if (vec) Q3_ROUTE_MMA(1, 1, true, small);
+    else Q3_ROUTE_MMA(1, 1, false, small);
+#undef Q3_ROUTE_MMA
   } else {
-    int tt = num_tokens > 64 ? ROUTE_TT : 2;
-    while (tt > 1 && (size_t)tt * W * sizeof(float) > 128 * 1024) tt >>= 1;  // fewer where their rows would not fit
-    const size_t smem = (size_t)tt * W * sizeof(float);
-    if (smem > 200 * 1024 || (E + 7) / 8 > 65535) return Q3_ERR_UNSUPPORTED;
-    const dim3 grid((num_tokens + tt - 1) / tt, (E + 7) / 8);
-    const int vec = W % 8 == 0 && h_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0;
-    if (dtype == Q3_DTYPE_F32) {
+    // both kernels give the same bits; the tile kernel needs about 64 tokens to fill the SMs
+    const bool tile = num_tokens > 64 && E >= ROUTE_EPW && W % 4 == 0 && h_stride % 4 == 0 &&
+                      (reinterpret_cast<uintptr_t>(h) & 15) == 0;
+    // a block's four warps all have experts: 8 experts x 1024, 4096 tokens 23 us, with three idle warps a block 30
+    const int we = E > 2 * ROUTE_EPW ? 4 : E > ROUTE_EPW ? 2 : 1;
+    const int te = we * ROUTE_EPW, tokens = 4 / we * ROUTE_TT;
+    if (tile && (E + te - 1) / te <= 65535) {
+      const dim3 grid((num_tokens + tokens - 1) / tokens, (E + te - 1) / te);
+#define Q3_ROUTE_TILE(WT_, WE_)                                                                                          \
+  e = launch_pdl(route_logits_tile_kernel<float, WT_, WE_>, grid, dim3(32 * WT_ * WE_), 0, stream, (const float*)h, h_stride, \
+                 router, num_tokens, E, W, logits)
+      if (we == 4) Q3_ROUTE_TILE(1, 4); else if (we == 2) Q3_ROUTE_TILE(2, 2); else Q3_ROUTE_TILE(4, 1);
+#undef Q3_ROUTE_TILE
+    } else {
+      int tt = num_tokens > 64 ? ROUTE_TT : 2;
+      while (tt > 1 && (size_t)tt * W * sizeof(float) > 128 * 1024) tt >>= 1;  // fewer where their rows would not fit
+      const size_t smem = (size_t)tt * W * sizeof(float);
+      if (smem > 200 * 1024 || (E + 7) / 8 > 65535) return Q3_ERR_UNSUPPORTED;
+      const dim3 grid((num_tokens + tt - 1) / tt, (E + 7) / 8);
+      const int vec = W % 8 == 0 && h_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0;
       if (smem > 48 * 1024)
         cudaFuncSetAttribute(route_logits_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       e = launch_pdl(route_logits_kernel<float>, grid, dim3(256), smem, stream, (const float*)h, h_stride, router,
-                     num_tokens, E, W, tt, vec, logits);
-    } else {
-      if (smem > 48 * 1024)
-        cudaFuncSetAttribute(route_logits_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      e = launch_pdl(route_logits_kernel<bf16>, grid, dim3(256), smem, stream, (const bf16*)h, h_stride, router,
                      num_tokens, E, W, tt, vec, logits);
     }
   }
@@ -401,9 +554,12 @@ Q3_EXPORT int q3_route_top(int dtype, const void* h, long h_stride, const float*
                    (const float*)logits, num_tokens, E, top, correction, count, keep, renorm, scale, chosen, weights);
     return e == cudaSuccess ? Q3_OK : Q3_ERR_LAUNCH;
   }
-  if (E <= 32 * PICK_REGS)
-    e = launch_pdl(route_pick_regs_kernel, dim3((num_tokens + 3) / 4), dim3(128), 0, stream, (const float*)logits,
-                   num_tokens, E, top, mode, scale, chosen, weights);
+#define Q3_PICK(REGS_)                                                                                                  \
+  e = launch_pdl(route_pick_regs_kernel<REGS_>, dim3((num_tokens + 3) / 4), dim3(128), 0, stream, (const float*)logits,  \
+                 num_tokens, E, top, mode, scale, chosen, weights)
+  if (E <= 64) Q3_PICK(2);
+  else if (E <= 32 * PICK_REGS) Q3_PICK(PICK_REGS);
+#undef Q3_PICK
   else
     e = launch_pdl(route_pick_kernel, dim3((num_tokens + 3) / 4), dim3(128), 0, stream, logits, num_tokens, E, top,
                    mode, scale, chosen, weights);

@@ -115,3 +115,37 @@ def test_every_height_of_a_box_of_slots(ops, monkeypatch, counts, unit):
     """Boxes of 32 to 128 rows, an odd and an even number of 32 slots for the two groups of the epilogue."""
     monkeypatch.setitem(globals(), "COUNTS", counts)
     test_products_against_their_statement(ops, 128, 392, unit, "input" if unit == "clamped_glu" else "output", 0)
+
+
+def _logits(ops, h, router):
+    T, E = h.shape[0], router.shape[0]
+    logits = torch.empty((T, E), device="cuda")
+    chosen, weights = torch.empty((T, 1), dtype=torch.int32, device="cuda"), torch.empty((T, 1), device="cuda")
+    ops._call("experts", "q3_route_top", "route_top", 1, h.data_ptr(), h.stride(0), router.data_ptr(), T, E, h.shape[1], 1, 0,
+              logits.data_ptr(), chosen.data_ptr(), weights.data_ptr(), None, 0, 0, 0, 1.0)
+    return logits
+
+
+@pytest.mark.parametrize("tokens,experts,width", [(1200, 64, 520), (2400, 33, 136), (400, 200, 72), (40, 20, 100), (33, 20, 37),
+                                                  (2500, 17, 2048), (1, 1, 8)])
+def test_router_logits_of_every_block(ops, tokens, experts, width):
+    """Large and small blocks, rows at odd places and widths that end inside a slice: the same bits, near to float64; infinities and
+    NaN as float32 products give them, in their own row and column only."""
+    g = torch.Generator().manual_seed(tokens + width)
+    h = torch.randn((tokens, width), generator=g).to(torch.bfloat16).cuda()
+    router = (0.02 * torch.randn((experts, width), generator=g)).cuda()
+    got, want = _logits(ops, h, router), h.double() @ router.double().t()
+    # a slice's chain of six products rounds six times, then the slices' and the warps' sums, each to 2^-24 of a partial sum
+    assert float((got - want).norm() / want.norm()) <= 2.0 ** -24 * (6 + (width / 32) ** 0.5)
+    for rows in (slice(0, 1), slice(tokens // 2, tokens)):
+        assert torch.equal(_logits(ops, h[rows], router), got[rows])
+    odd = torch.zeros((tokens, width + 3), dtype=torch.bfloat16, device="cuda")
+    odd[:, 1: 1 + width] = h
+    assert torch.equal(_logits(ops, odd[:, 1: 1 + width], router), got)
+    if tokens > 3 and experts > 2:
+        h[1, width // 2], h[2, 0], router[1, 3] = float("inf"), float("nan"), float("-inf")
+        again, want = _logits(ops, h, router), h.double() @ router.double().t()
+        assert torch.equal(again.isnan(), want.isnan()) and torch.equal(again.isinf(), want.isinf())
+        assert torch.equal(again[again.isinf()], want[want.isinf()].float())
+        fine = want.isfinite()
+        assert torch.equal(again[fine], got[fine])
