@@ -85,11 +85,9 @@ __device__ __forceinline__ void merge_row(const float* __restrict__ mid_o, const
                                           int num_splits, bf16* __restrict__ out_row, int first, int step,
                                           float sink, const bf16* __restrict__ gate_row) {
   float mx = -INFINITY;
-  for (int s = 0; s < num_splits; ++s) mx = fmaxf(mx, __ldcg(lse + s));
-  const float sink_w = exp2f(sink - mx);  // no sink: 2^(-inf) = 0
   for (int d = 4 * first; d < D; d += 4 * step) {
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    float wsum = sink_w;
+    float wsum = 0.f;
     for (int s0 = 0; s0 < num_splits; s0 += 8) {
       float4 v[8];
       float ls[8];
@@ -99,6 +97,14 @@ __device__ __forceinline__ void merge_row(const float* __restrict__ mid_o, const
           ls[j] = __ldcg(lse + s0 + j);
           v[j] = __ldcg(reinterpret_cast<const float4*>(mid_o + (long)(s0 + j) * D + d));
         }
+      if (s0 == 0) {  // the largest lse, from what is on its way anyway
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (j < num_splits) mx = fmaxf(mx, ls[j]);
+#pragma unroll 8
+        for (int s = 8; s < num_splits; ++s) mx = fmaxf(mx, __ldcg(lse + s));
+        wsum = exp2f(sink - mx);  // no sink: 2^(-inf) = 0
+      }
 #pragma unroll
       for (int j = 0; j < 8; ++j)
         if (s0 + j < num_splits && ls[j] != -INFINITY) {
@@ -128,14 +134,16 @@ __device__ __forceinline__ void merge_row(const float* __restrict__ mid_o, const
 // block puts the ticket word back to zero for the next launch.
 __device__ __forceinline__ bool drew_last_ticket(int* ticket, int num_splits) {
   __shared__ int last;
-  __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0) {  // (its fences stand for the block's, which the barriers order)
+    __threadfence();
     last = atomicAdd(ticket, 1) == num_splits - 1;
-    if (last) *ticket = 0;
+    if (last) {
+      *ticket = 0;
+      __threadfence();
+    }
   }
   __syncthreads();
-  if (last) __threadfence();
   return last;
 }
 
@@ -313,11 +321,11 @@ decode_attention_kernel(const bf16* __restrict__ q, int q_stride, const bf16* kp
     cp_async_commit();
   }
   if (FUSED) {
-    pdl_wait();  // the q/k/v projection of this step
     // D/16 threads per head; a thread owns elements [8c, 8c+8) and their rotation partners
     // [8c + D/2, 8c + D/2 + 8).  Items: the group's q heads, then (owner only) the k and v head.
+    // What does not come from the projection is loaded before it is waited for.
     constexpr int TPH = D / 16, HALF = D / 2, PER_PASS = THREADS / TPH;
-    const int items = G + (owner ? 2 : 0);
+    const int items = G + (owner ? 2 : 0), c = tid % TPH;
     const bf16* row = q + (long)tok * q_stride;
     long cache_row = -1;
     if (owner && p / ps < max_pages) {
@@ -326,9 +334,21 @@ decode_attention_kernel(const bf16* __restrict__ q, int q_stride, const bf16* kp
     }
     // a position beyond the tables is reported, not rotated with another position's angles
     const bool rotate = nt.cos_t && p < nt.max_pos;
+    float wa[8], wb[8];  // of the first pass's head
+    Angles angles;
+    if (rotate) angles = load_angles(nt.cos_t + (long)p * HALF, nt.sin_t + (long)p * HALF, c, HALF, nt.pairing);
+    auto load_weights = [&](int item) {
+      const float* w = item < G ? nt.q_w : nt.k_w;
+      if (w && item <= G) {
+        load8(w + 8 * c, wa);
+        load8(w + HALF + 8 * c, wb);
+      }
+    };
+    load_weights(tid / TPH);
+    pdl_wait();  // the q/k/v projection of this step
     if (nt.cos_t && !rotate && tid == 0 && error_word) atomicExch(error_word, Q3_ERR_POSITION);
     for (int base = 0; base < items; base += PER_PASS) {
-      const int item = base + tid / TPH, c = tid % TPH;
+      const int item = base + tid / TPH;
       const bool live = item < items;
       const bool is_q = item < G, is_v = item == G + 1;
       const bf16* x = row + (is_q ? (long)(kvh * G + item) * D
@@ -348,20 +368,16 @@ decode_attention_kernel(const bf16* __restrict__ q, int q_stride, const bf16* kp
       for (int o = TPH >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
       if (!live) continue;
       if (!is_v) {
-        const float* w = is_q ? nt.q_w : nt.k_w;
-        if (w) {
+        if (base > 0) load_weights(item);
+        if (is_q ? nt.q_w : nt.k_w) {
           const float rstd = rsqrtf(ss / (float)D + nt.eps);
-          float wa[8], wb[8];
-          load8(w + 8 * c, wa);
-          load8(w + HALF + 8 * c, wb);
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
             a[e] = (a[e] * rstd) * wa[e];
             b[e] = (b[e] * rstd) * wb[e];
           }
         }
-        if (rotate)
-          rotate_chunks(a, b, nt.cos_t + (long)p * HALF, nt.sin_t + (long)p * HALF, c, HALF, nt.pairing);
+        if (rotate) rotate_by(a, b, angles, nt.pairing);
         if (is_q && nt.q_scale) {
           const float f = nt.q_scale[tok];
 #pragma unroll
