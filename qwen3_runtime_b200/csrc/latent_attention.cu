@@ -180,17 +180,45 @@ Q3_EXPORT int q3_rotate_heads(int dtype, const void* x, long xs_t, long xs_h, vo
   return q3_launch_status();
 }
 
-// ---- the cached rows of a step's sequences, side by side ------------------------------------------
-// Sequence s keeps its rows from key first_s on, first_s = the multiple of 64 at or before the first key that its first
-// new token sees; row kv_base[s] + j of `rows` is key j.  One warp per row, 16 bytes a lane and turn.
+// ---- what a prompt's attention on expanded keys and values starts from -----------------------------
+// The step's queries' turned parts (64 columns), dense [T, H, 64], and the cached rows of its sequences side by side, in one
+// launch.  A block of the first num_tokens turns a token's heads: the angles' cosines and sines once for all of them (a thread
+// per pair and head computing its own: 9.0 us at 2048 tokens of 16 heads, with the rows' own launch 12.4 and a gap; now
+// 6.5).  The others copy rows: sequence s keeps its rows from key first_s on, first_s = the multiple of 64 at or before
+// the first key that its first new token sees; row kv_base[s] + j of `rows` is key j.  One warp per row, 16 bytes a lane and turn.
+constexpr int TURN = 64;
 __global__ void __launch_bounds__(256)
 latent_gather_kernel(const uint4* __restrict__ pages, int chunks, const int* __restrict__ block_table, int max_pages,
                      const int* __restrict__ kv_lens, const int* __restrict__ cu_seqlens, int num_seqs, int ps, int window,
-                     uint4* __restrict__ rows, int* __restrict__ kv_base, int num_rows) {
+                     uint4* __restrict__ rows, int* __restrict__ kv_base, int num_rows, const bf16* __restrict__ q, long qs_t,
+                     long qs_h, bf16* __restrict__ turned, const int* __restrict__ positions, const float* __restrict__ inv_freq,
+                     int pairs, int H, int num_tokens, int pairing, float magnitude) {
   pdl_wait();
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int r = blockIdx.x * 8 + warp;
+  if ((int)blockIdx.x < num_tokens) {
+    __shared__ float2 angle[TURN / 2];
+    const int t = blockIdx.x;
+    if ((int)threadIdx.x < pairs) {
+      const float ang = (float)positions[t] * inv_freq[threadIdx.x];
+      angle[threadIdx.x] = make_float2(cosf(ang) * magnitude, sinf(ang) * magnitude);
+    }
+    __syncthreads();
+    const bool turns = lane < pairs;
+    const float2 y = turns ? angle[lane] : make_float2(0.f, 0.f);
+    for (int h = warp; h < H; h += 8) {
+      const bf16* src = q + t * qs_t + h * qs_h;
+      bf16* dst = turned + ((long)t * H + h) * TURN;
+      // pair i: columns 2 i, 2 i + 1, or i, i + pairs; what belongs to no pair, columns from 2 pairs on, is copied
+      const int i0 = pairing || !turns ? 2 * lane : lane, i1 = pairing || !turns ? 2 * lane + 1 : lane + pairs;
+      const bf16 u = src[i0], v = src[i1];
+      const float a = to_f32(u), b = to_f32(v);
+      dst[i0] = turns ? from_f32<bf16>(a * y.x - b * y.y) : u;
+      dst[i1] = turns ? from_f32<bf16>(b * y.x + a * y.y) : v;
+    }
+    return;
+  }
+  const int r = ((int)blockIdx.x - num_tokens) * 8 + warp;
   int at = 0, seq = -1, key = 0;
   for (int s = 0; s < num_seqs; ++s) {
     const int kv = kv_lens[s], n = cu_seqlens[s + 1] - cu_seqlens[s];
@@ -211,17 +239,21 @@ latent_gather_kernel(const uint4* __restrict__ pages, int chunks, const int* __r
 }
 
 // pages: [*, ps, width] bf16 of rows of a multiple of 16 bytes; rows: [num_rows, width]; num_rows = sum over the sequences
-// of kv_len - first (see above); kv_base: int32 [num_seqs].
+// of kv_len - first (see above); kv_base: int32 [num_seqs].  q: bf16, 64 columns of each token's heads, qs_t and qs_h apart;
+// turned: dense [num_tokens, H, 64]; pairs, pairing, magnitude as in q3_rotate_heads.
 Q3_EXPORT int q3_latent_gather(const void* pages, int width, const int* block_table, int max_pages, const int* kv_lens,
                                const int* cu_seqlens, int num_seqs, int ps, int window, void* rows, int* kv_base, int num_rows,
-                               cudaStream_t stream) {
+                               const void* q, long qs_t, long qs_h, void* turned, const int* positions, const float* inv_freq,
+                               int pairs, int H, int num_tokens, int pairing, float magnitude, cudaStream_t stream) {
   if (!pages || !block_table || !kv_lens || !cu_seqlens || !rows || !kv_base || ps < 1 || num_seqs < 1 || num_rows < 1 ||
-      window < 0)
+      window < 0 || !q || !turned || H < 1 || num_tokens < 0 || pairs < 0 || 2 * pairs > TURN ||
+      (pairs && (!positions || !inv_freq)) || pairing < 0 || pairing > 1)
     return Q3_ERR_ARGUMENT;
   if (width % 8 || (((uintptr_t)pages | (uintptr_t)rows) & 15)) return Q3_ERR_UNSUPPORTED;
-  return launch_pdl(latent_gather_kernel, dim3((num_rows + 7) / 8), dim3(256), 0, stream, (const uint4*)pages, width / 8,
-                    block_table, max_pages, kv_lens, cu_seqlens, num_seqs, ps, window, (uint4*)rows, kv_base,
-                    num_rows) == cudaSuccess
+  return launch_pdl(latent_gather_kernel, dim3(num_tokens + (num_rows + 7) / 8), dim3(256), 0, stream, (const uint4*)pages,
+                    width / 8, block_table, max_pages, kv_lens, cu_seqlens, num_seqs, ps, window, (uint4*)rows, kv_base, num_rows,
+                    (const bf16*)q, qs_t, qs_h, (bf16*)turned, positions, inv_freq, pairs, H, num_tokens, pairing,
+                    magnitude) == cudaSuccess
              ? Q3_OK
              : Q3_ERR_LAUNCH;
 }

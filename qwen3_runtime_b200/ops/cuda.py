@@ -81,7 +81,8 @@ _SIGNATURES = {
         "q3_rotate_heads": [c_int, c_void_p, c_long, c_long, c_void_p, c_long, c_long, c_void_p, c_void_p, c_int,
                             c_int, c_int, c_int, c_int, c_float, c_void_p],
         "q3_latent_gather": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p,
-                             c_int, c_void_p],
+                             c_int, c_void_p, c_long, c_long, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float,
+                             c_void_p],
         "q3_latent_attention": [c_int, c_void_p, c_long, c_long, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p,
                                 c_void_p, c_void_p, c_void_p, c_long, c_long, c_int, c_int, c_int, c_float, c_int,
                                 c_void_p],
@@ -1302,26 +1303,28 @@ class CudaOps:
             seen[key] = rows, pairs
         return seen[key]
 
-    def latent_attention_expanded(self, q, q_turned, expand, rows, *, pages, kv_rank, block_table, sink, out, page_size, scale,
-                                  window, step):
+    def latent_attention_expanded(self, q, expand, rows, *, pages, kv_rank, block_table, sink, out, page_size, scale, window, step,
+                                  positions, inv_freq, pairing="interleaved", magnitude=1.0):
         """Attention of a step's prompts over cached rows ``[latent (kv_rank) | turned key part (64)]`` with keys and
         values expanded: ``expand`` ``[2 * H * 128, kv_rank]`` makes the heads' key columns, then the heads' values, of the
-        ``rows`` rows the step's tokens see (:meth:`latent_expand_rows`); ``q`` ``[T, H, >= 128]`` (the first 128 columns of
-        a head), ``q_turned`` dense ``[T, H, 64]``, ``out`` dense ``[T, H, 128]``."""
-        T, H, _ = q.shape
+        ``rows`` rows the step's tokens see (:meth:`latent_expand_rows`); ``q`` ``[T, H, 192]``, a head's last 64 columns to be
+        turned as :meth:`rotate_heads` does, ``out`` dense ``[T, H, 128]``."""
+        T, H, n = q.shape
         width = pages.shape[-1]
         qs = self._head_strides(q, "latent_attention_expanded")
-        if not (pages.is_contiguous() and out.is_contiguous() and q_turned.is_contiguous()
-                and q_turned.shape == (T, H, 64) and out.shape == (T, H, 128)):
-            raise KernelError("latent_attention_expanded: dense pages, turned queries [T, H, 64] and output [T, H, 128]")
+        if not (pages.is_contiguous() and out.is_contiguous() and n == 192 and out.shape == (T, H, 128)):
+            raise KernelError("latent_attention_expanded: dense pages, queries [T, H, 192] and a dense output [T, H, 128]")
         dev = out.device
         seen = torch.empty((rows, width), dtype=out.dtype, device=dev)
+        q_turned = torch.empty((T, H, 64), dtype=out.dtype, device=dev)
         base = torch.empty(step.num_seqs, dtype=torch.int32, device=dev)
         if self.timing is not None:
-            self._costs(2 * rows * width * out.element_size())
+            self._costs((2 * rows * width + 2 * T * H * 64) * out.element_size())
         self._call("latent_attention", "q3_latent_gather", "latent_gather", _ptr(pages), width, _ptr(block_table),
                    block_table.shape[1], _ptr(step.kv_lens), _ptr(step.cu_seqlens), step.num_seqs, page_size,
-                   int(window or 0), _ptr(seen), _ptr(base), rows)
+                   int(window or 0), _ptr(seen), _ptr(base), rows, q.data_ptr() + 256, qs[0], qs[1], _ptr(q_turned),
+                   _ptr(positions), _ptr(inv_freq), inv_freq.numel() if inv_freq is not None else 0, H, T,
+                   self.PAIRINGS[pairing], float(magnitude))
         kv = self.linear(seen[:, :kv_rank], expand)
         cu = step.host_cu_seqlens
         work = sum(-(-(-(-(cu[b + 1] - cu[b]) // 128)) // 2) for b in range(step.num_seqs) if cu[b + 1] > cu[b])

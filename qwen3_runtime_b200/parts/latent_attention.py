@@ -163,13 +163,12 @@ class LatentAttention(Part):
                                           window=self.window, dtype=h.dtype)
         if seen:
             try:
-                q_turned = torch.empty((T, H, self.rot_dim), dtype=h.dtype, device=h.device)
-                ops.rotate_heads(q[:, :, self.dim:], q_turned, positions=step.positions, inv_freq=inv_freq, **turn)
                 ops.latent_attention_expanded(
-                    q, q_turned, self.expand, seen, pages=cache.latent_pages, kv_rank=self.kv_rank, block_table=block_table,
-                    sink=self.sink, out=ctx_out, page_size=cache.page_size, scale=self.scale, window=self.window, step=step)
+                    q, self.expand, seen, pages=cache.latent_pages, kv_rank=self.kv_rank, block_table=block_table,
+                    sink=self.sink, out=ctx_out, page_size=cache.page_size, scale=self.scale, window=self.window, step=step,
+                    positions=step.positions, inv_freq=inv_freq, **turn)
             except torch.OutOfMemoryError:  # no room for the expanded rows
-                seen, q_turned = 0, None
+                seen = 0
         if not seen:
             q_lat = torch.empty((T, H, self.row_width), dtype=h.dtype, device=h.device)
             ops.head_linear(q[:, :, : self.dim], self.uk_t, q_lat[:, :, : self.kv_rank])

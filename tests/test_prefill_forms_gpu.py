@@ -285,3 +285,27 @@ def test_a_step_without_room_for_expanded_rows_stays_in_the_latent_space(ops):
 
     got, want = _steps(ops, spec, 16, [[300, 64], [100, 0]], [no_room, _set(latent_expand=False)])
     assert asked == [16, 16] and all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("pairing,pairs", [("interleaved", 32), ("interleaved", 5), ("half", 32), ("half", 7), ("half", 0)])
+def test_queries_turned_beside_the_gathered_rows(ops, pairing, pairs):
+    """One launch turns the queries' last 64 columns as rotate_heads does and lays the sequences' cached rows side by side."""
+    T, H, width, page, seqs = 37, 3, 40, 8, 2
+    g = torch.Generator(device="cuda").manual_seed(pairs)
+    q = torch.randn((T, H, 192), generator=g, device="cuda").to(torch.bfloat16)
+    positions = torch.randint(0, 5000, (T,), generator=g, device="cuda", dtype=torch.int32)
+    freqs = torch.rand(pairs, generator=g, device="cuda") if pairs else None
+    pages = torch.randn((9, page, width), generator=g, device="cuda").to(torch.bfloat16)
+    table = torch.tensor([[3, 0, 8, -1], [5, 1, 2, 7]], dtype=torch.int32, device="cuda")
+    kv, cu = torch.tensor([20, 25], dtype=torch.int32, device="cuda"), torch.tensor([0, 12, 37], dtype=torch.int32, device="cuda")
+    rows, base = torch.zeros((45, width), dtype=torch.bfloat16, device="cuda"), torch.zeros(seqs, dtype=torch.int32, device="cuda")
+    got, want = torch.zeros((T, H, 64), dtype=torch.bfloat16, device="cuda"), torch.zeros((T, H, 64), dtype=torch.bfloat16, device="cuda")
+    ops._call("latent_attention", "q3_latent_gather", "latent_gather", pages.data_ptr(), width, table.data_ptr(), 4, kv.data_ptr(),
+              cu.data_ptr(), seqs, page, 0, rows.data_ptr(), base.data_ptr(), 45, q.data_ptr() + 256, q.stride(0), q.stride(1),
+              got.data_ptr(), positions.data_ptr(), freqs.data_ptr() if pairs else None, pairs, H, T, ops.PAIRINGS[pairing], 1.25)
+    ops.rotate_heads(q[:, :, 128:], want, positions=positions, inv_freq=freqs, pairing=pairing, magnitude=1.25)
+    # the same angles and products; a fused multiply-add may stand at another product, then one rounding to bfloat16 moves
+    assert float((got.float() - want.float()).abs().max()) <= 2.0 ** -8 * float(want.float().abs().max())
+    assert torch.equal(got[:, :, 2 * pairs:], want[:, :, 2 * pairs:])
+    at = torch.cat([pages[[3, 0, 8]].flatten(0, 1)[:20], pages[[5, 1, 2, 7]].flatten(0, 1)[:25]])
+    assert torch.equal(rows, at) and base.tolist() == [0, 20]
