@@ -17,6 +17,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -38,6 +39,7 @@ NVCC_FLAGS = [
 # extra link flags per group
 EXTRA_FLAGS: dict[str, list[str]] = {
     "gemm_tcgen05": ["-lcuda"],
+    "host_call": ["-I" + sysconfig.get_paths()["include"]],
 }
 
 
@@ -181,3 +183,27 @@ def load_group(group: str) -> ctypes.CDLL:
             lib = ctypes.CDLL(str(compile_group(group)))
             _loaded[group] = lib
         return lib
+
+
+_maker = None  # False: there is none
+_KINDS = {ctypes.c_int: "i", ctypes.c_long: "i", ctypes.c_void_p: "p", ctypes.c_float: "f"}
+
+
+def native_caller(fn):
+    """A function that calls the launcher ``fn`` (a ctypes function with its argument types) as ctypes does, at a fraction of
+    the cost (csrc/host_call.cu); ``fn`` itself where there is no such thing for its arguments or on this machine."""
+    global _maker
+    with _lock:
+        if _maker is None:
+            try:
+                _maker = getattr(ctypes.PyDLL(str(compile_group("host_call"))), "q3_make_caller", False)
+            except (KernelBuildError, OSError):
+                _maker = False
+            if _maker:
+                _maker.restype, _maker.argtypes = ctypes.py_object, [ctypes.c_void_p, ctypes.c_char_p]
+        if not _maker:
+            return fn
+    kinds = [_KINDS.get(t) for t in fn.argtypes]
+    if None in kinds or fn.restype is not ctypes.c_int:
+        return fn
+    return _maker(ctypes.cast(fn, ctypes.c_void_p), "".join(kinds).encode()) or fn

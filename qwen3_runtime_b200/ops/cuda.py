@@ -513,7 +513,7 @@ class CudaOps:
             )
         self._device_index = torch.cuda.current_device()
         self.SM_COUNT = torch.cuda.get_device_properties(self._device_index).multi_processor_count
-        self._fn: dict[str, ctypes._CFuncPtr] = {}
+        self._fn: dict = {}  # launchers by name, as they are called
         self.launches = 0  # kernels of this engine launched (or captured) through this table
         # Per-kernel timing, off by default: a list makes every launch through this table record
         # (kernel, start event, stop event, algorithmic bytes, flops) into it; see timed_kernels().
@@ -535,7 +535,7 @@ class CudaOps:
             fn = getattr(lib, name)
             fn.argtypes = _SIGNATURES[group][name]
             fn.restype = c_int
-            self._fn[name] = fn
+            fn = self._fn[name] = build.native_caller(fn)
         return fn
 
     def _stream(self) -> int:

@@ -29,7 +29,7 @@ from .base import Addend, BuildContext, ParamSpec, Part, StepContext, build_part
 
 def heads_view(rows: torch.Tensor, start: int, heads: int, size: int) -> torch.Tensor:
     """Columns ``start .. start + heads * size`` of ``rows`` ``[T, n]`` as ``[T, heads, size]`` (a view)."""
-    return rows[:, start:start + heads * size].unflatten(1, (heads, size))
+    return rows[:, start:start + heads * size].view(rows.shape[0], heads, size)
 
 
 class BranchMixer(Part):
