@@ -59,7 +59,10 @@ __global__ void fused_norm_kernel(const void* __restrict__ pending, int parts, l
 // registers between the two passes (no staging through shared memory).
 // PLANES: what is pending may be partial-sum planes (a variant of its own, so that the common one
 // keeps its registers).
-template <typename T, bool REGS, bool PLANES>
+// EARLY (REGS): the weight is loaded before the kernel before this one is waited for.  With few rows a row's way is what counts
+// (8 rows of 2560 2.08 -> 1.81 us; a step of one request, 17 of these kernels, 584 -> 576), with many the registers (2048 rows
+// 10.7 -> 11.1).
+template <typename T, bool REGS, bool PLANES, bool EARLY>
 __global__ void __launch_bounds__(512) fused_norm_vec_kernel(const void* __restrict__ pending, int parts, long part_stride,
                                       float* __restrict__ resid, const int* __restrict__ ids,
                                       const T* __restrict__ table, const int* __restrict__ rows,
@@ -67,6 +70,8 @@ __global__ void __launch_bounds__(512) fused_norm_vec_kernel(const void* __restr
                                       int write_resid, int vocab) {
   extern __shared__ float vals[];
   float* red = REGS ? vals : vals + H;
+  float wv[8];
+  if (EARLY && (int)threadIdx.x * 8 < H) load8(w + threadIdx.x * 8, wv);
   pdl_wait();
   pdl_launch_dependents();
   const int r = blockIdx.x;
@@ -122,14 +127,14 @@ __global__ void __launch_bounds__(512) fused_norm_vec_kernel(const void* __restr
   const float rstd = rsqrtf(total / (float)H + eps);
   T* orow = out + (long)r * H;
   for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
-    float v[8], wv[8];
+    float v[8];
     if (REGS) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) v[e] = mine[e];
     } else {
       load8(vals + i, v);
     }
-    load8(w + i, wv);
+    if (!EARLY) load8(w + i, wv);
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] = (v[e] * rstd) * wv[e];
     store8(orow + i, v);
@@ -156,10 +161,14 @@ static int launch_fused_norm(const void* pending, int parts, long part_stride, f
     const size_t vec_smem = regs ? 33 * sizeof(float) : smem;
     void (*kernel)(const void*, int, long, float*, const int*, const T*, const int*, const float*, T*, int, float, int,
                    int);
+    // (200 rows of 2560 / 4096 2.67 -> 2.48 / 3.37 -> 3.20 us with the weight first, 296 2.73 -> 2.55 / 3.47 -> 3.89, 400 3.2 -> 3.5)
+    const bool early = regs && num_rows <= 200;
     if (parts)
-      kernel = regs ? fused_norm_vec_kernel<T, true, true> : fused_norm_vec_kernel<T, false, true>;
+      kernel = early ? fused_norm_vec_kernel<T, true, true, true>
+                     : regs ? fused_norm_vec_kernel<T, true, true, false> : fused_norm_vec_kernel<T, false, true, false>;
     else
-      kernel = regs ? fused_norm_vec_kernel<T, true, false> : fused_norm_vec_kernel<T, false, false>;
+      kernel = early ? fused_norm_vec_kernel<T, true, false, true>
+                     : regs ? fused_norm_vec_kernel<T, true, false, false> : fused_norm_vec_kernel<T, false, false, false>;
     if (vec_smem > 48 * 1024)
       cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vec_smem);
     return launch_pdl(kernel, dim3(num_rows), dim3(threads), vec_smem, stream, pending, parts, part_stride, resid, ids,
