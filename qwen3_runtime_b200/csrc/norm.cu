@@ -59,9 +59,10 @@ __global__ void fused_norm_kernel(const void* __restrict__ pending, int parts, l
 // registers between the two passes (no staging through shared memory).
 // PLANES: what is pending may be partial-sum planes (a variant of its own, so that the common one
 // keeps its registers).
-// EARLY (REGS): the weight is loaded before the kernel before this one is waited for.  With few rows a row's way is what counts
-// (8 rows of 2560 2.08 -> 1.81 us; a step of one request, 17 of these kernels, 584 -> 576), with many the registers (2048 rows
-// 10.7 -> 11.1).
+// EARLY (REGS): the weight is on its way with the row, and on its way to L2 before the kernel before is waited for (which may be
+// the one that writes it, so nothing is loaded until then).  With few rows a row's way is what counts (8 rows of 2560 2.08 -> 1.82
+// us, as with the load itself ahead of the wait; a step of one request, 17 of these kernels, 584 -> 576), with many the registers
+// (2048 rows 10.7 -> 11.1).
 template <typename T, bool REGS, bool PLANES, bool EARLY>
 __global__ void __launch_bounds__(512) fused_norm_vec_kernel(const void* __restrict__ pending, int parts, long part_stride,
                                       float* __restrict__ resid, const int* __restrict__ ids,
@@ -71,9 +72,11 @@ __global__ void __launch_bounds__(512) fused_norm_vec_kernel(const void* __restr
   extern __shared__ float vals[];
   float* red = REGS ? vals : vals + H;
   float wv[8];
-  if (EARLY && (int)threadIdx.x * 8 < H) load8(w + threadIdx.x * 8, wv);
+  const bool has = (int)threadIdx.x * 8 < H;
+  if (EARLY && has) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + threadIdx.x * 8));
   pdl_wait();
   pdl_launch_dependents();
+  if (EARLY && has) load8(w + threadIdx.x * 8, wv);
   const int r = blockIdx.x;
   const long src = rows ? rows[r] : r;
   const T* trow = nullptr;

@@ -34,6 +34,27 @@ def close(got, want, dtype, what, f32_tol=2e-5, bf16_tol=2e-2):
     assert diff <= tol * scale, f"{what}: max |diff| {diff:.3g} > {tol * scale:.3g}"
 
 
+@pytest.mark.parametrize("H,T", [(8, 1), (2560, 200), (2560, 201), (4096, 8), (4104, 3)])
+def test_norm_whose_weight_the_kernel_before_writes(ops, H, T):
+    """Few rows ask for the weight early (up to 200, with a thread for every 8 values): what the launch before wrote is what
+    counts all the same."""
+    x = rand((T, H), torch.float32, 11)
+    sources = [rand((1, H), torch.float32, 12 + i) for i in range(8)]
+    ones = torch.ones(H, device="cuda")
+    weight = torch.zeros(H, device="cuda")
+    got = [torch.empty((T, H), dtype=torch.bfloat16, device="cuda") for _ in sources]
+    torch.cuda.synchronize()
+    for src, out in zip(sources, got):
+        ops.fused_norm(weight.view(1, H), ones, 1e-6, resid=src, write_resid=False)
+        ops.fused_norm(out, weight, 1e-6, resid=x, write_resid=False)
+    for src, out in zip(sources, got):
+        ops.fused_norm(weight.view(1, H), ones, 1e-6, resid=src, write_resid=False)
+        torch.cuda.synchronize()
+        want = torch.empty_like(out)
+        ops.fused_norm(want, weight, 1e-6, resid=x, write_resid=False)
+        assert torch.equal(out, want), "same arithmetic, same weight: same bits"
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("H,T", [(2560, 33), (333, 7), (4096, 2), (80, 130), (12288, 3)])
 def test_fused_norm_variants(ops, dtype, H, T):
