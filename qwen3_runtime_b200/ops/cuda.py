@@ -249,6 +249,11 @@ _SIGNATURES = {
         "q3_gemm_stream_partial": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int,
                                    c_void_p, c_void_p],
     },
+    "gemm_few_tokens": {
+        "q3_gemm_few_parts": [c_int, c_int, c_int, c_int],
+        "q3_gemm_few_tokens": [c_int, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_int, c_int, c_int, c_int,
+                               c_void_p, c_void_p],
+    },
     "gemm_tcgen05": {
         "q3_gemm_tcgen05": [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
                             c_void_p],
@@ -2068,7 +2073,8 @@ class CudaOps:
     def _product(self, x, weight, out=None, out_dtype=None, partial_sums=False):
         """``x[M, K] @ weight[N, K]^T``.  float32: on the tensor cores with operands in three bfloat16 parts, which is
         nearer to the exact product than a chain of fp32 FMA (:meth:`_f32_segments`), small sizes on the FMA pipes; no TF32.
-        bfloat16, at most 16 tokens: one of this engine's two weight-streaming kernels
+        bfloat16, at most 128 tokens: csrc/gemm_few_tokens.cu for output heads and large partial
+        sums (:attr:`FEW_TOKENS`).  bfloat16, at most 16 tokens otherwise: one of this engine's two weight-streaming kernels
         (:meth:`_small_product`).  bfloat16, more tokens: the library product with fp32
         accumulation, as the reference's ``nn.Linear`` (qwen3_runtime/models/qwen3.py:76-77,
         134-135), or this engine's tcgen05 kernel with ``large_gemm="tcgen05"``.
@@ -2085,6 +2091,13 @@ class CudaOps:
             e = x.element_size()
             oe = 4 if out_dtype == torch.float32 else e
             self._costs(N * K * e + M * K * e + M * N * oe, 2.0 * M * N * K, f" {M}x{K}->{N}")
+        few = M > 0 and self._few_tokens_ok(x, weight)
+        if few and partial_sums and self.partial_sums and out is None and out_dtype is None:
+            parts = self._few_parts(M, N, K)
+            if parts > 1:
+                planes = torch.empty((parts, M, N), dtype=torch.float32, device=x.device)
+                self._few_product(1, x, weight, planes, parts, M, N, K)
+                return planes
         if (partial_sums and self.partial_sums and out is None and out_dtype is None and M > 0
                 and self.small_gemm != "registers" and self._small_m_ok(x, weight)):
             parts = self._stream_parts(M, N, K)
@@ -2094,6 +2107,13 @@ class CudaOps:
                            _ptr(weight), weight.stride(0), _ptr(planes), parts, M, N, K,
                            _ptr(self._error_word(x.device)))
                 return planes
+        odt = out_dtype or x.dtype
+        if (few and odt in (torch.float32, torch.bfloat16) and self._few_finished(M, N, K, odt)
+                and (out is None or (out.dtype == odt and out.stride(1) == 1))):
+            if out is None:
+                out = torch.empty((M, N), dtype=odt, device=x.device)
+            self._few_product(int(odt == torch.float32), x, weight, out, 1, M, N, K)
+            return out
         if x.dtype == torch.float32:
             if out is None:
                 out = torch.empty((M, N), dtype=torch.float32, device=x.device)
@@ -2111,7 +2131,6 @@ class CudaOps:
                        weight.stride(0), _ptr(out), out.stride(0), M, N, K, self.f32_tile)
             return out
         if self._small_m_ok(x, weight):
-            odt = out_dtype or x.dtype
             if out is None:
                 out = torch.empty((M, N), dtype=odt, device=x.device)
             self._small_product(1 if odt == torch.float32 else 0, x, weight, out, M, N, K)
@@ -2257,6 +2276,62 @@ class CudaOps:
     TCGEN05_MIN_TOKEN_FILL = 0.9
     TCGEN05_MIN_SHARE = 0.65
 
+    # What csrc/gemm_few_tokens.cu takes from the other kernels (streams of at most 16 tokens, the library above), as measured at 1 ..
+    # 128 tokens with the sizes of eight models (hidden 896 .. 8192), each alone and up to 16 tokens in whole steps as well.
+    # Finished products of at least two rounds of 128 rows over the SMs: output heads of 32,000 rows and more 5 to 16 % less than the
+    # library at every token count (one round of 16,384 rows: level); 8 tokens 151,936 x 2560 126 -> 118, x 4096 244 -> 186.
+    # bfloat16 results up to 64 tokens (24576 x 4096 2 to 6 % less); up to 16 tokens from 10,240 rows and 52 M weights on (10240 x
+    # 5120, 8 tokens 22.7 -> 19.3, 16 28.2 -> 19.5; 19456 x 2560: level; 6144 x 4096 11.8 -> 12.7).
+    # Partial sums, 17 to 64 tokens, where K is cut into four ranges or more: hidden 896 .. 4096 5 to 30 % less; two or three
+    # ranges of 5120 rows 8 % less to 12 % more, 1024 x 2048 2 % more.  Up to 16 tokens of long rows: 4096 x 12288 23.8 -> 21.5, 5120
+    # x 25600 58 -> 47, 8192 x 28672 92 -> 76, 5120 x 17408 level, 2560 x 9728 12.2 -> 12.9, 8192 x 8192 27.5 -> 29.0.
+    # Gated: up to 32 tokens 3 to 15 % less from 20 M weights on (6 M: level), up to 64 with 16,384 features and more (48 tokens:
+    # 2 x 17408 6 % less, 2 x 25600 12, 2 x 12288 and 2 x 9728 level).  Up to 16 tokens from 80 M on: 2 x 12288 x 4096 40.8 -> 35.3 (16
+    # tokens 71 -> 37), 2 x 11008 x 4096 39 -> 31, 2 x 25600 x 5120 103 -> 79; 2 x 9728 x 2560 19.3 -> 18.8 alone, a step 1 % more.
+    FEW_TOKENS, FEW_MIN_ROWS, FEW_BF16_TOKENS = 128, 24576, 64
+    FEW_SMALL_ROWS, FEW_SMALL_ROWS_WEIGHTS = 10240, 52_000_000
+    FEW_PARTS_TOKENS, FEW_MIN_PARTS, FEW_PARTS_MIN_WEIGHTS, FEW_PARTS_ROWS = 64, 4, 3 << 20, 4096
+    FEW_SMALL_PARTS_WEIGHTS, FEW_SMALL_PARTS_VALUES = 45_000_000, 12288
+    FEW_GATED_TOKENS, FEW_GATED_MIN_WEIGHTS, FEW_GATED_TOKENS_WIDE, FEW_GATED_WIDE = 32, 20_000_000, 64, 16384
+    FEW_SMALL_GATED_WEIGHTS = 80_000_000
+
+    def _few_finished(self, M: int, N: int, K: int, dtype) -> bool:
+        if M <= self.SMALL_M and N >= self.FEW_SMALL_ROWS and N * K >= self.FEW_SMALL_ROWS_WEIGHTS:
+            return True
+        return N >= self.FEW_MIN_ROWS and (dtype == torch.float32 or M <= self.FEW_BF16_TOKENS)
+
+    def _few_tokens_ok(self, x, weight) -> bool:
+        M = x.shape[0]
+        return ((self.small_gemm if M <= self.SMALL_M else self.large_gemm) == "auto" and M <= self.FEW_TOKENS
+                and self._tcgen05_ok(x, weight) and weight.dtype == torch.bfloat16
+                and x.stride(0) >= x.shape[1] <= weight.stride(0))
+
+    def _few_parts(self, M: int, N: int, K: int) -> int:
+        """Ranges of K in this kernel's partial sums (1: it does not take the product)."""
+        if M <= self.SMALL_M:
+            least = 2 if K >= self.FEW_SMALL_PARTS_VALUES and N * K >= self.FEW_SMALL_PARTS_WEIGHTS else 0
+        else:
+            least = self.FEW_MIN_PARTS if (M <= self.FEW_PARTS_TOKENS and N <= self.FEW_PARTS_ROWS
+                                           and N * K >= self.FEW_PARTS_MIN_WEIGHTS) else 0
+        if not least:
+            return 1
+        key = ("few", least, -(-M // 32), N, K)
+        parts = self._parts_cache.get(key)
+        if parts is None:
+            parts = int(self._get("gemm_few_tokens", "q3_gemm_few_parts")(M, N, K, 8))
+            parts = self._parts_cache[key] = parts if parts >= least else 1
+        return parts
+
+    def _few_gated(self, M: int, I: int, K: int) -> bool:
+        if M <= self.SMALL_M:
+            return 2 * I * K >= self.FEW_SMALL_GATED_WEIGHTS
+        return (M <= self.FEW_GATED_TOKENS and 2 * I * K >= self.FEW_GATED_MIN_WEIGHTS
+                or M <= self.FEW_GATED_TOKENS_WIDE and I >= self.FEW_GATED_WIDE)
+
+    def _few_product(self, mode: int, x, weight, out, parts, M, N, K) -> None:
+        self._call("gemm_few_tokens", "q3_gemm_few_tokens", "gemm_few_tokens", mode, _ptr(x), x.stride(0), _ptr(weight),
+                   weight.stride(0), _ptr(out), out.stride(-2), parts, M, N, K, _ptr(self._error_word(x.device)))
+
     def _stream_parts(self, M: int, N: int, K: int) -> int:
         """Ranges of K in the streaming kernel's partial-sum mode (0: it does not take the product)."""
         key = (M > 8, N, K)
@@ -2302,6 +2377,9 @@ class CudaOps:
         if self.timing is not None:
             e = x.element_size()
             self._costs((2 * I * K + M * K + M * I) * e, 4.0 * M * I * K, f" {M}x{K}->2x{I} swiglu")
+        if M > 0 and self._few_tokens_ok(x, gate_up_weight) and out.stride(1) == 1 and self._few_gated(M, I, K):
+            self._few_product(2 + act, x, gate_up_weight, out, 1, M, I, K)
+            return out
         if self._small_m_ok(x, gate_up_weight):
             self._small_product(2 + act, x, gate_up_weight, out, M, I, K)
             return out

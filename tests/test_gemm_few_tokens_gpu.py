@@ -1,0 +1,116 @@
+"""Products of 17 to 128 tokens (csrc/gemm_few_tokens.cu) against float64, at the edges of its tiles and of its dispatch."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+BF16, F32 = torch.bfloat16, torch.float32
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from qwen3_runtime_b200.ops.cuda import CudaOps
+
+    return CudaOps()
+
+
+def draw(M, N, K, seed=1, x_pad=0, w_pad=0):
+    g = torch.Generator().manual_seed(seed)
+    x = torch.randn(M, K + x_pad, generator=g).to(BF16).cuda()[:, :K]
+    w = torch.randn(N, K + w_pad, generator=g).to(BF16).cuda()[:, :K]
+    return x, w
+
+
+def f32_bound(x, w):
+    """The products are exact in fp32 and added up in fp32, rounded towards zero at worst: 2^-23 of the sum of magnitudes for each
+    of the K / 16 instructions that add to an accumulator, and as much again for the 16 products within one."""
+    K = x.shape[1]
+    return (x.double().abs() @ w.double().abs().t()) * 2.0**-23 * (K / 16 + 16)
+
+
+def product(ops, mode, x, w, out, parts=1):
+    N = w.shape[0] // (2 if mode >= 2 else 1)
+    ops._few_product(mode, x, w, out, parts, x.shape[0], N, x.shape[1])
+    ops.raise_if_kernel_error()
+    return out
+
+
+# rows: less than one tile, one row more than a round of 128 rows and of 64, odd; values: one slice, a remainder of 8, odd slices
+@pytest.mark.parametrize("N,K", [(1, 8), (3, 64), (296, 72), (18944, 128), (18945, 136), (9473, 320), (2560, 4096)])
+@pytest.mark.parametrize("M", [1, 17, 32, 33, 64, 65, 128])
+def test_every_mode_against_float64(ops, M, N, K):
+    x, w = draw(M, N, K, seed=M + N, x_pad=8, w_pad=16)
+    want, bound = x.double() @ w.double().t(), f32_bound(x, w)
+    guard = torch.full((M + 1, N + 3), 7.0, device="cuda")
+    got = product(ops, 1, x, w, guard[:M, :N])
+    assert bool(((got.double() - want).abs() <= bound).all())
+    assert bool((guard[M] == 7).all()) and bool((guard[:, N:] == 7).all()), "nothing beyond the result is written"
+    rounded = product(ops, 0, x, w, torch.empty((M, N), dtype=BF16, device="cuda"))
+    assert torch.equal(rounded, got.to(BF16))
+    parts = ops._get("gemm_few_tokens", "q3_gemm_few_parts")(M, N, K, 8)
+    if parts > 1:
+        planes = product(ops, 1, x, w, torch.full((parts, M, N), 7.0, device="cuda"), parts)
+        assert bool(((planes.double().sum(0) - want).abs() <= bound).all())
+    if N > 1:
+        I = N // 2
+        for mode, act in ((2, "silu"), (3, "gelu")):
+            unit = product(ops, mode, x, w[: 2 * I], torch.empty((M, I), dtype=BF16, device="cuda"))
+            sums = product(ops, 1, x, w[: 2 * I].contiguous(), torch.empty((M, 2 * I), device="cuda"))
+            want_unit = ops.glu_mul(sums, torch.empty((M, I), device="cuda"), act).to(BF16)
+            assert torch.equal(unit, want_unit), "the unit takes the fp32 products"
+
+
+# what linear and gated_linear send here and what they do not
+@pytest.mark.parametrize("M", [16, 17, 32, 33, 64, 65, 128, 129])
+@pytest.mark.parametrize("pad", [0, 8, 4])
+def test_routes_agree(ops, M, pad):
+    x, w = draw(M, 24577, 512, seed=M, x_pad=pad, w_pad=pad)
+    want = x.double() @ w.double().t()
+    before = ops.launches
+    got = ops.linear(x, w, out_dtype=F32)
+    assert bool(((got.double() - want).abs() <= f32_bound(x, w)).all())
+    assert (ops.launches > before) == (M <= 128 and pad % 8 == 0)
+    out = torch.empty((M, 24577), device="cuda")
+    assert ops.linear(x, w, out=out, out_dtype=F32) is out and torch.equal(out, got)
+    x, w = draw(M, 1024, 3072, seed=M + 1, x_pad=pad, w_pad=pad)
+    want = x.double() @ w.double().t()
+    planes = ops.linear(x, w, partial_sums=True)
+    if planes.dim() == 3:  # (the library's product of rows off 16 bytes may add its own ranges up in bfloat16)
+        assert bool(((planes.double().sum(0) - want).abs() <= f32_bound(x, w)).all())
+    if 16 < M <= 128:
+        assert (planes.dim() == 3) == (M <= 64 and pad % 8 == 0)
+    x, w = draw(M, 2 * 5008, 2048, seed=M + 2, x_pad=pad, w_pad=pad)
+    w = w * 0.02
+    got = ops.gated_linear(x, w, torch.empty((M, 5008), dtype=BF16, device="cuda"))
+    sums = (x.double() @ w.double().t()).to(BF16).double()
+    gate, up = sums[:, :5008], sums[:, 5008:]
+    want = gate * torch.sigmoid(gate) * up
+    # gate and up are off by their fp32 sums and may be rounded to the neighbouring bfloat16 (2^-8 of them), the unit's slope in
+    # the gate is at most 1.1, and the result is rounded once more
+    off = f32_bound(x, w)
+    off_gate, off_up = off[:, :5008] + 2.0**-8 * gate.abs(), off[:, 5008:] + 2.0**-8 * up.abs()
+    bound = 1.1 * (off_gate * (up.abs() + off_up) + off_up * gate.abs()) + 2.0**-8 * want.abs() + 1e-12
+    if pad % 8 == 0 or M <= 16:
+        assert bool(((got.double() - want).abs() <= bound).all())
+
+
+def test_weights_the_kernel_before_writes_and_a_captured_step(ops):
+    M, N, K = 48, 24576, 256
+    x, w = draw(M, N, K)
+    sources = [draw(M, N, K, seed=2 + i)[1] for i in range(4)]
+    weight, got = torch.zeros_like(w), []
+    for src in sources:
+        weight.copy_(src)
+        got.append(ops.linear(x, weight, out_dtype=F32))
+    for src, y in zip(sources, got):
+        assert torch.equal(y, ops.linear(x, src, out_dtype=F32)), "same sums in the same order"
+    out = torch.empty((M, N), device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ops.linear(x, weight, out=out, out_dtype=F32)
+    for src, y in zip(sources, got):
+        weight.copy_(src)
+        graph.replay()
+        assert torch.equal(out, y)
+    ops.raise_if_kernel_error()
