@@ -53,7 +53,7 @@ few_tokens_kernel(const __grid_constant__ Maps maps, void* __restrict__ out, lon
   __shared__ __align__(8) unsigned long long bars[2 * MAX_STAGES + 5];
   __shared__ float staged[GATED ? 32 * OUT_STRIDE : 1];
   __shared__ uint32_t tmem_base_s;
-  __shared__ volatile int abort_flag, gave_up;
+  __shared__ volatile int abort_flag;
   int issued = 0;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -67,7 +67,7 @@ few_tokens_kernel(const __grid_constant__ Maps maps, void* __restrict__ out, lon
   const uint32_t drained = smem_addr(&bars[2 * MAX_STAGES + 4]);
 
   if (threadIdx.x == 0) {
-    abort_flag = gave_up = 0;
+    abort_flag = 0;
     for (int s = 0; s < stages; ++s) {
       mbar_init(full0 + 8 * s, 1);
       mbar_init(empty0 + 8 * s, 1);
@@ -124,6 +124,9 @@ few_tokens_kernel(const __grid_constant__ Maps maps, void* __restrict__ out, lon
           for (int j = 0; j < MAX_KS; ++j) {
             if (j >= slices) break;
             tma_load_3d_pair(dst + j * slice_bytes, &maps.w, leader_full0 + 8 * s, (kb + j) * BK, w_row, 0);
+#ifdef Q3_TEST_WITHHOLD_A_BOX  // (a test build leaves the tokens' boxes of a pair's last item out: its stages never fill)
+            if (item + num_pairs >= items) continue;
+#endif
             tma_load_2d_pair(dst + j * slice_bytes + a_bytes, &maps.x, leader_full0 + 8 * s, (kb + j) * BK, (int)rank * (n / 2));
           }
         }
@@ -176,10 +179,8 @@ few_tokens_kernel(const __grid_constant__ Maps maps, void* __restrict__ out, lon
     for (int item = pair; item < items; item += num_pairs, ++i) {
       const int part = item / plan.tiles, tile = item - part * plan.tiles, buf = i & 1;
       const int f0 = (2 * tile + (int)rank) * plan.rows;
-      if (!mbar_wait(acc_full0 + 8 * buf, (i >> 1) & 1, &abort_flag)) gave_up = 1;
+      if (any_gave_up(1, 128, !mbar_wait(acc_full0 + 8 * buf, (i >> 1) & 1, &abort_flag))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      asm volatile("bar.sync 1, 128;" ::: "memory");  // one warp may give up where another saw the barrier complete: they agree
-      if (gave_up) break;
       const uint32_t lane_addr = tmem_base + buf * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
       for (int c0 = 0; c0 < n; c0 += 32) {

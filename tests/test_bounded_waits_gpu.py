@@ -82,3 +82,21 @@ def test_float32_product(ops, rows):
     got, want = ops.linear(x, w).double(), x.double() @ w.double().t()
     ops.raise_if_kernel_error()
     assert float((got - want).norm() / want.norm()) < 1e-6
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("M,N,K", [(1, 1024, 512), (48, 24576, 512), (16, 77000, 192), (128, 40000, 256)])
+def test_product_of_few_tokens(ops, mode, M, N, K):
+    """What is left out is a pair's last item's: its only one, or one behind finished ones, whose epilogue has been through before."""
+    x = torch.randn((M, K), device="cuda").to(torch.bfloat16)
+    w = (K ** -0.5 * torch.randn(((2 if mode == 2 else 1) * N, K), device="cuda")).to(torch.bfloat16)
+    out = torch.zeros((M, N), dtype=torch.float32 if mode == 1 else torch.bfloat16, device="cuda")
+    assert _expires(_build("gemm_few_tokens", "q3_gemm_few_tokens"), mode, x.data_ptr(), K, w.data_ptr(), K, out.data_ptr(), N, 1,
+                    M, N, K) == 1
+    # the ordinary build of the same kernel gives the right result
+    ops._few_product(mode, x, w, out, 1, M, N, K)
+    ops.raise_if_kernel_error()
+    want = x.double() @ w.double().t()
+    if mode == 2:
+        want = torch.nn.functional.silu(want[:, :N]) * want[:, N:]
+    assert float((out.double() - want).norm() / want.norm()) < (1e-6 if mode == 1 else 2.0 ** -8)
