@@ -100,3 +100,26 @@ def test_product_of_few_tokens(ops, mode, M, N, K):
     if mode == 2:
         want = torch.nn.functional.silu(want[:, :N]) * want[:, N:]
     assert float((out.double() - want).norm() / want.norm()) < (1e-6 if mode == 1 else 2.0 ** -8)
+
+
+@pytest.mark.parametrize("unit", [0, 1, 2])
+@pytest.mark.parametrize("counts", [[1], [33, 0, 256], [8, 40] * 60, [500] * 30])
+def test_product_of_routed_experts(ops, unit, counts):
+    """As above, with tiles in which the second group of the epilogue has slots and tiles in which it has none."""
+    E, S, N, K = len(counts), sum(counts), 520, 136
+    chunks = [-(-n // 256) for n in counts]
+    offsets, tiles = (torch.tensor([0, *torch.tensor(n).cumsum(0)], dtype=torch.int32, device="cuda") for n in (counts, chunks))
+    x = torch.randn((S, K), device="cuda").to(torch.bfloat16)
+    w = (K ** -0.5 * torch.randn((E, (2 if unit == 2 else 1) * N, K), device="cuda")).to(torch.bfloat16)
+    out = torch.zeros((S, N), dtype=torch.bfloat16, device="cuda")
+    args = (unit, w.data_ptr(), x.data_ptr(), out.data_ptr(), S, E, N, K, offsets.data_ptr(), tiles.data_ptr(), 7.0, 1.0, 0.0)
+    assert _expires(_build("experts_tcgen05", "q3_expert_tcgen05"), *args) == 1
+    # the ordinary build of the same kernel gives the right result
+    ops._call("experts_tcgen05", "q3_expert_tcgen05", "expert_tc", *args, ops._error_word(x.device).data_ptr())
+    ops.raise_if_kernel_error()
+    want = torch.cat([r.double() @ v.double().t() for r, v in zip(x.split(counts), w)])
+    if unit == 1:
+        want = want.clamp(min=0) ** 2
+    if unit == 2:
+        want = torch.nn.functional.silu(want[:, :N].clamp(max=7)) * want[:, N:].clamp(-7, 7)
+    assert float((out.double() - want).norm() / want.norm()) < 2.0 ** -7
