@@ -102,13 +102,13 @@ __device__ __forceinline__ bool mbar_wait_drain(uint32_t bar, uint32_t parity) {
 // Where the warps of a role meet inside their loop, some may have given up and others seen the barrier complete: all of the
 // `threads` threads that meet at named barrier `id` learn whether any of them has given up.  Meeting and asking are one operation: a
 // flag in shared memory, read behind a barrier, could be raised for the next round by a warp that is ahead before a slower one
-// has read it for this round; the two would part, and one would wait at the barrier for good.
+// has read it for this round; the two would part, and one would wait at the barrier for good.  (Whole warps, of one mind each.)
 __device__ __forceinline__ bool any_gave_up(int id, int threads, bool gave_up) {
   uint32_t any;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 p, %3, 0;\n\t"
-      "barrier.cta.red.or.pred q, %1, %2, p;\n\t"
+      "bar.red.or.pred q, %1, %2, p;\n\t"
       "selp.u32 %0, 1, 0, q;\n\t}"
       : "=r"(any)
       : "r"(id), "r"(threads), "r"((uint32_t)gave_up)

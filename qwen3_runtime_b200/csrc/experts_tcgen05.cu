@@ -202,7 +202,8 @@ expert_tcgen05_kernel(const __grid_constant__ Maps maps, bf16* __restrict__ out,
       const int buf = i & 1;
       const int f0 = t.f * TILE_F + (int)rank * (TILE_F / 2);
       // (a group without slots in a tile meets nowhere else in it)
-      if (any_gave_up(group + 1, 128, !mbar_wait(acc_full0 + 8 * buf, (i >> 1) & 1, &abort_flag))) break;
+      const bool lost = !__all_sync(0xffffffffu, mbar_wait(acc_full0 + 8 * buf, (i >> 1) & 1, &abort_flag));
+      if (any_gave_up(group + 1, 128, lost)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t lane_addr = tmem_base + buf * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
       if (group * 32 >= t.n && lane == 0) remote_arrive_only(leader_acc_empty0 + 8 * buf);  // nothing here for this group

@@ -14,11 +14,18 @@
 // 48 tokens, us, the library / this (partial sums and gated: with the kernel that takes them): head of 151,936 x 2560 136 / 121
 // (6.4 TB/s), x 4096 211 / 193; 7 or fewer ranges of 2560 x 9728 16.9 / 13.6, 4096 x 12288 24.7 / 22.8; gated 2 x 25600 x 5120
 // 99.8 / 87.6.  Finished products of a few thousand rows stay the library's (6144 x 2560 8.3 / 9.9): one round, whose ends count.
+// Sums of up to 16 tokens: the accumulators round towards zero at every instruction, so one chain over 2560 values is 2.7e-6 off,
+// and the streaming kernels, which add 16 chains of a sixteenth, 1.6e-7.  Here half a k-slice (two instructions) has an accumulator
+// of its own, eight to a buffer; the epilogue adds eight, then those sums, rounded to nearest: 8.7e-8, and 5.0e-8 .. 1.3e-7 from 64 to
+// 25,600 values (those kernels 5.0e-8 .. 9.5e-6, and never less).  8 tokens, us, one chain / this: 151936 x 2560 115.6 / 115.6, x 4096
+// 188.3 / 189.2, gated 2 x 11008 x 4096 30.7 / 32.2, 2 x 25600 x 5120 77.9 / 79.3, 10240 x 5120 20.4 / 21.0, 4096 x 12288 in parts
+// 19.3 / 19.9.  (A buffer for every slice: 125, 201, 42, 85, 30, 22 us: its way to the epilogue and back takes some 600 cycles.)
+// From 17 tokens on one chain, as in the library's products.
 // Before the kernel ahead is waited for the first ring's worth of weights is asked for into L2 (not into shared memory: that
 // kernel may be the one that writes them).
 //
 // Persistent, one CTA per SM: warp 0 TMA producer, warp 1 MMA issuer (leader only; both with their lane chosen by elect.sync),
-// warps 2..5 epilogue; two accumulators in tensor memory.  Every wait is bounded; on expiry the waiter raises the block's abort
+// warps 2..5 epilogue; two buffers in tensor memory.  Every wait is bounded; on expiry the waiter raises the block's abort
 // flag and the error word, every role leaves its loop, and what is in flight is waited for (bounded again) before tensor memory
 // is freed.  No load uses cluster multicast.
 #include "async_tiles.cuh"
@@ -28,7 +35,8 @@ namespace {
 enum { OUT_BF16 = 0, OUT_F32 = 1, OUT_SILU = 2, OUT_GELU = 3 };
 constexpr int MAX_KS = 4;                            // k-slices of 64 values a stage, at most
 constexpr int BK = 64, THREADS = 192, MAX_STAGES = 24, MAX_ROWS = 128, MAX_TOKENS = 128;
-constexpr int ACC_COLS = 128, TMEM_COLS = 256;
+constexpr int ACC_COLS = 128;                        // columns of a buffer of one accumulator; two buffers
+constexpr int FEW = 16, SUMS = 8, SLICE_SUMS = 2;    // up to 16 tokens: SUMS accumulators of 32 columns, two for every k-slice
 constexpr int OUT_STRIDE = 132;                      // floats per token in the gated unit's buffer
 constexpr int RING_BYTES = 204 * 1024;
 constexpr int KS_BYTES = 14 * 1024;                 // slices up to this size go four a stage, larger ones two
@@ -43,7 +51,7 @@ struct Plan {
   int tiles;   // of 2 h rows
 };
 
-template <int MODE>
+template <int MODE, bool FEW_SUMS>
 __global__ void __launch_bounds__(THREADS, 1)
 few_tokens_kernel(const __grid_constant__ Maps maps, void* __restrict__ out, long out_ld, int M, int N, int num_kb, Plan plan,
                   int n, int ks, int stages, int* __restrict__ error_word) {
@@ -65,6 +73,8 @@ few_tokens_kernel(const __grid_constant__ Maps maps, void* __restrict__ out, lon
   const uint32_t full0 = smem_addr(&bars[0]), empty0 = smem_addr(&bars[MAX_STAGES]);
   const uint32_t acc_full0 = smem_addr(&bars[2 * MAX_STAGES]), acc_empty0 = smem_addr(&bars[2 * MAX_STAGES + 2]);
   const uint32_t drained = smem_addr(&bars[2 * MAX_STAGES + 4]);
+  const int group = FEW_SUMS ? SUMS / SLICE_SUMS : plan.per;  // k-slices of a buffer
+  constexpr int BUF_COLS = FEW_SUMS ? 32 * SUMS : ACC_COLS, TMEM_COLS = 2 * BUF_COLS;
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
@@ -139,61 +149,100 @@ few_tokens_kernel(const __grid_constant__ Maps maps, void* __restrict__ out, lon
       const bool chosen = elect_one();
       const uint32_t acc0 = __shfl_sync(0xffffffffu, tmem_base, 0), tiles0 = smem_addr(tiles);
       const uint32_t idesc = umma_idesc(256, n);
-      int s = 0, i = 0;
-      uint32_t phase = 0;
+      int s = 0, buf = 0;
+      uint32_t phase = 0, acc_phase = 1;
       bool ok = true;
-      for (int item = pair; item < items && ok; item += num_pairs, ++i) {
-        const int kb0 = item / plan.tiles * plan.per, kb1 = min(num_kb, kb0 + plan.per), buf = i & 1;
-        ok = __all_sync(0xffffffffu, mbar_wait(acc_empty0 + 8 * buf, ((i >> 1) & 1) ^ 1, &abort_flag));
-        if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t acc = acc0 + buf * ACC_COLS;
-        for (int kb = kb0; kb < kb1; kb += ks) {
-          ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, phase, &abort_flag));
+      for (int item = pair; item < items && ok; item += num_pairs) {
+        const int kb0 = item / plan.tiles * plan.per, kb1 = min(num_kb, kb0 + plan.per);
+        for (int g0 = kb0; g0 < kb1; g0 += group) {
+          const int g1 = min(kb1, g0 + group);
+          ok = __all_sync(0xffffffffu, mbar_wait(acc_empty0 + 8 * buf, acc_phase, &abort_flag));
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a_addr = tiles0 + (uint32_t)(s * ks) * slice_bytes;
-          const int slices = min(ks, kb1 - kb);
-          if (chosen) {
+          const uint32_t acc = acc0 + buf * BUF_COLS;
+          for (int kb = g0; kb < g1; kb += ks) {  // (ks divides the group)
+            ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, phase, &abort_flag));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t a_addr = tiles0 + (uint32_t)(s * ks) * slice_bytes;
+            const int slices = min(ks, g1 - kb);
+            if (chosen) {
 #pragma unroll
-            for (int j = 0; j < MAX_KS; ++j) {
-              if (j >= slices) break;
-              const uint64_t a_desc = umma_desc(a_addr + j * slice_bytes), b_desc = umma_desc(a_addr + j * slice_bytes + a_bytes);
+              for (int j = 0; j < MAX_KS; ++j) {
+                if (j >= slices) break;
+                const uint64_t a_desc = umma_desc(a_addr + j * slice_bytes), b_desc = umma_desc(a_addr + j * slice_bytes + a_bytes);
+                const uint32_t to = FEW_SUMS ? acc + 32 * SLICE_SUMS * (kb - g0 + j) : acc;
 #pragma unroll
-              for (int k = 0; k < BK / 16; ++k)
-                umma_pair(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb > kb0 || j > 0 || k > 0) ? 1u : 0u);
+                for (int k = 0; k < BK / 16; ++k)
+                  umma_pair(FEW_SUMS ? to + 32 * (k / 2) : to, a_desc + 2 * k, b_desc + 2 * k, idesc,
+                            (FEW_SUMS ? k % 2 > 0 : kb > g0 || j > 0 || k > 0) ? 1u : 0u);
+              }
+              umma_commit_pair(empty0 + 8 * s);
             }
-            umma_commit_pair(empty0 + 8 * s);
+            __syncwarp();
+            if (++s == stages) s = 0, phase ^= 1;
           }
+          if (!ok) break;
+          if (chosen) umma_commit_pair(acc_full0 + 8 * buf);
           __syncwarp();
-          if (++s == stages) s = 0, phase ^= 1;
+          buf ^= 1, acc_phase ^= buf ^ 1;
         }
-        if (ok && chosen) umma_commit_pair(acc_full0 + 8 * buf);
-        __syncwarp();
       }
     }
   } else {  // ---- epilogue: warp w reads TMEM lanes 32 * (w % 4) .. + 31 of this CTA ---------------------------------------
     const int quarter = warp & 3, row = quarter * 32 + lane, et = threadIdx.x - 64;
     const uint32_t leader_acc_empty0 = map_to_cta(acc_empty0, 0);
-    int i = 0;
-    for (int item = pair; item < items; item += num_pairs, ++i) {
-      const int part = item / plan.tiles, tile = item - part * plan.tiles, buf = i & 1;
+    int buf = 0;
+    uint32_t phase = 0;
+    for (int item = pair; item < items; item += num_pairs) {
+      const int part = item / plan.tiles, tile = item - part * plan.tiles;
       const int f0 = (2 * tile + (int)rank) * plan.rows;
-      if (any_gave_up(1, 128, !mbar_wait(acc_full0 + 8 * buf, (i >> 1) & 1, &abort_flag))) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t lane_addr = tmem_base + buf * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
-#pragma unroll 1
-      for (int c0 = 0; c0 < n; c0 += 32) {
-        uint32_t acc[32];
-        tmem_load32(lane_addr + c0, acc);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (c0 + 32 >= n) {  // the last of this buffer is in registers: hand it back to the MMA issuer
+      uint32_t lane_addr = 0;
+      float v[32] = {};  // of this row: all tokens' sums, or the next 32 tokens'
+      bool lost = false;
+      const int per = min(plan.per, num_kb - part * plan.per);
+      for (int done = 0; done < per; done += group) {
+        lost = !__all_sync(0xffffffffu, mbar_wait(acc_full0 + 8 * buf, phase, &abort_flag));
+        if (lost) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        lane_addr = tmem_base + buf * BUF_COLS + ((uint32_t)(quarter * 32) << 16);
+        if constexpr (!FEW_SUMS) {
+          break;
+        } else {
+          uint32_t r[SUMS][FEW];
+#pragma unroll
+          for (int g = 0; g < SUMS; ++g) tmem_load16(lane_addr + 32 * g, r[g]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           if (lane == 0) remote_arrive_only(leader_acc_empty0 + 8 * buf);
+          buf ^= 1, phase ^= buf ^ 1;
+#pragma unroll
+          for (int c = 0; c < FEW; ++c) {
+            float f[SUMS];
+#pragma unroll
+            for (int g = 0; g < SUMS; ++g) f[g] = done + g / SLICE_SUMS < per ? __uint_as_float(r[g][c]) : 0.f;
+            v[c] += ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
+          }
+        }
+      }
+      if (any_gave_up(1, 128, lost)) break;
+#pragma unroll 1
+      for (int c0 = 0; c0 < n; c0 += 32) {
+        if (!FEW_SUMS) {
+          uint32_t acc[32];
+          tmem_load32(lane_addr + c0, acc);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (c0 + 32 >= n) {  // the last of this buffer is in registers: hand it back to the MMA issuer
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            if (lane == 0) remote_arrive_only(leader_acc_empty0 + 8 * buf);
+            buf ^= 1, phase ^= buf ^ 1;
+          }
+#pragma unroll
+          for (int c = 0; c < 32; ++c) v[c] = __uint_as_float(acc[c]);
         }
         if (GATED) {  // (the products go to the unit in fp32)
 #pragma unroll
-          for (int c = 0; c < 32; ++c) staged[c * OUT_STRIDE + row] = __uint_as_float(acc[c]);
+          for (int c = 0; c < 32; ++c) staged[c * OUT_STRIDE + row] = v[c];
           asm volatile("bar.sync 1, 128;" ::: "memory");
           const int tokens = min(32, M - c0);
           for (int j = et; j < tokens * plan.rows; j += 128) {
@@ -209,9 +258,9 @@ few_tokens_kernel(const __grid_constant__ Maps maps, void* __restrict__ out, lon
           for (int c = 0; c < 32; ++c) {
             if (c0 + c >= M) break;
             if (MODE == OUT_F32)
-              static_cast<float*>(out)[(part * (long)M + c0 + c) * out_ld + f0 + row] = __uint_as_float(acc[c]);
+              static_cast<float*>(out)[(part * (long)M + c0 + c) * out_ld + f0 + row] = v[c];
             else
-              static_cast<bf16*>(out)[(c0 + c) * out_ld + f0 + row] = from_f32<bf16>(__uint_as_float(acc[c]));
+              static_cast<bf16*>(out)[(c0 + c) * out_ld + f0 + row] = from_f32<bf16>(v[c]);
           }
         }
       }
@@ -269,7 +318,7 @@ Plan plan_of(int n, int N, int K, bool gated, int most_parts, int pairs) {
   return best;
 }
 
-template <int MODE>
+template <int MODE, bool FEW_SUMS>
 int pairs_of() {  // pairs of SMs the device runs at once with this kernel
   static int pairs_on[Q3_MAX_DEVICES];
   int& pairs = pairs_on[q3_current_device()];
@@ -286,10 +335,10 @@ int pairs_of() {  // pairs of SMs the device runs at once with this kernel
     cfg.numAttrs = 1;
     if (cudaGetDevice(&device) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
-        cudaFuncSetAttribute(few_tokens_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES) != cudaSuccess)
+        cudaFuncSetAttribute(few_tokens_kernel<MODE, FEW_SUMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES) != cudaSuccess)
       return 0;
     cfg.gridDim = dim3(sms / 2 * 2);
-    if (cudaOccupancyMaxActiveClusters(&n, few_tokens_kernel<MODE>, &cfg) != cudaSuccess || n < 1) {
+    if (cudaOccupancyMaxActiveClusters(&n, few_tokens_kernel<MODE, FEW_SUMS>, &cfg) != cudaSuccess || n < 1) {
       cudaGetLastError();
       return 0;
     }
@@ -298,11 +347,11 @@ int pairs_of() {  // pairs of SMs the device runs at once with this kernel
   return pairs;
 }
 
-template <int MODE>
-int launch(const void* x, long x_ld, const void* w, long w_ld, void* out, long out_ld, int parts, int M, int N, int K,
+template <int MODE, bool FEW_SUMS>
+int launch_as(const void* x, long x_ld, const void* w, long w_ld, void* out, long out_ld, int parts, int M, int N, int K,
            int* error_word, cudaStream_t stream) {
   constexpr bool GATED = MODE >= OUT_SILU;
-  const int pairs = pairs_of<MODE>();
+  const int pairs = pairs_of<MODE, FEW_SUMS>();
   if (!pairs) return Q3_ERR_UNSUPPORTED;
   // (given parts: the caller's planes are of that many)
   const int n = tokens_padded(M);
@@ -339,10 +388,17 @@ int launch(const void* x, long x_ld, const void* w, long w_ld, void* out, long o
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = q3_pdl_enabled() ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, few_tokens_kernel<MODE>, maps, out, out_ld, M, N, (K + BK - 1) / BK, plan, n, ks, stages,
+  return cudaLaunchKernelEx(&cfg, few_tokens_kernel<MODE, FEW_SUMS>, maps, out, out_ld, M, N, (K + BK - 1) / BK, plan, n, ks, stages,
                             error_word) == cudaSuccess
              ? Q3_OK
              : Q3_ERR_LAUNCH;
+}
+
+template <int MODE>
+int launch(const void* x, long x_ld, const void* w, long w_ld, void* out, long out_ld, int parts, int M, int N, int K,
+           int* error_word, cudaStream_t stream) {
+  return M <= FEW ? launch_as<MODE, true>(x, x_ld, w, w_ld, out, out_ld, parts, M, N, K, error_word, stream)
+                  : launch_as<MODE, false>(x, x_ld, w, w_ld, out, out_ld, parts, M, N, K, error_word, stream);
 }
 
 }  // namespace
@@ -350,7 +406,7 @@ int launch(const void* x, long x_ld, const void* w, long w_ld, void* out, long o
 // How many planes of partial sums the product is best cut into, at most most_parts (1: none).
 Q3_EXPORT int q3_gemm_few_parts(int M, int N, int K, int most_parts) {
   if (M < 1 || M > MAX_TOKENS || N < 1 || K < 1 || most_parts < 1) return 1;
-  const int pairs = pairs_of<OUT_F32>();
+  const int pairs = pairs_of<OUT_F32, false>();
   if (!pairs) return 1;
   // (found again when it is asked for as the most there may be: the least of fewer is the same)
   return plan_of(tokens_padded(M), N, K, false, most_parts, pairs).parts;

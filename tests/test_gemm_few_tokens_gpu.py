@@ -61,6 +61,31 @@ def test_every_mode_against_float64(ops, M, N, K):
             assert torch.equal(unit, want_unit), "the unit takes the fp32 products"
 
 
+@pytest.mark.parametrize("N,K,parts", [(24576, 256, 1), (1024, 328, 1), (24576, 896, 1), (24576, 2560, 1), (10240, 5120, 1),
+                                       (4096, 12288, 8)])
+@pytest.mark.parametrize("M", [1, 9, 16])
+@pytest.mark.parametrize("positive", [False, True])
+def test_sums_of_up_to_16_tokens_are_as_near_as_the_streams(ops, monkeypatch, M, N, K, parts, positive):
+    """The streaming kernels add 16 chains of a sixteenth of K each; one chain over all of K would be an order of magnitude further
+    off, most of all where nothing cancels."""
+    x, w = draw(M, N, K, seed=K + M)
+    if positive:
+        x, w = x.abs(), w.abs()
+    want = x.double() @ w.double().t()
+    if parts > 1:
+        parts = ops._get("gemm_few_tokens", "q3_gemm_few_parts")(M, N, K, parts)
+        assert parts > 1
+    got = product(ops, 1, x, w, torch.empty((parts, M, N), device="cuda"), parts).sum(0)
+    monkeypatch.setattr(ops, "small_gemm", "stream")
+    other = ops.linear(x, w, partial_sums=True) if parts > 1 else ops.linear(x, w, out_dtype=F32)
+    off = lambda y: float((y.double() - want).norm() / want.norm())
+    assert off(got) <= off(other.sum(0) if parts > 1 else other)
+    # two instructions to an accumulator, rounded towards zero, and 16 products within one (as f32_bound); then roundings to nearest:
+    # three on the way of eight accumulators, one of each eight, one of each plane
+    bound = (x.double().abs() @ w.double().abs().t()) * 2.0**-24 * (2 * (2 + 16) + 3 + K / 256 + parts)
+    assert bool(((got.double() - want).abs() <= bound).all())
+
+
 # what linear and gated_linear send here and what they do not
 @pytest.mark.parametrize("M", [16, 17, 32, 33, 64, 65, 128, 129])
 @pytest.mark.parametrize("pad", [0, 8, 4])
