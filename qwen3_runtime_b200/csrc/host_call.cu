@@ -1,8 +1,8 @@
 // Calls of the exported launchers from Python without ctypes, whose conversion of 15 to 45 arguments takes 2 to 5 us a call, as
 // much as the launch itself (27 arguments: 3.2 us, here 0.23).  Host code only.
 //
-// q3_make_caller(function, kinds) returns a Python function that takes one argument per letter of kinds -- i: a whole number, p: an
-// address or None, f: a number that is passed as float -- and returns the launcher's int.
+// q3_make_caller(function, kinds) returns a Python function that takes one argument per letter of kinds -- i: a whole number
+// or what stands for one (__index__), p: an address or None, f: a number that is passed as float -- and returns the launcher's int.
 //
 // All launchers are called through one type.  The calling convention of x86-64 Linux hands whole numbers and addresses over in six
 // registers and then in 8-byte places on the stack, in their order, and up to eight floats in registers of their own, so a
@@ -44,14 +44,19 @@ PyObject* call(PyObject* self, PyObject* const* args, Py_ssize_t n) {
       f[floats++] = (float)x;
     } else {
       long x = 0;
-      if (c->kinds[i] == 'i' || a != Py_None) {
-        if (!PyLong_Check(a)) {
-          PyErr_Format(PyExc_TypeError, "argument %d: %s expected, not %s", i + 1,
-                       c->kinds[i] == 'p' ? "an address or None" : "an int", Py_TYPE(a)->tp_name);
-          return nullptr;
-        }
+      if (PyLong_Check(a)) {
         x = PyLong_AsLong(a);
         if (x == -1 && PyErr_Occurred()) return nullptr;
+      } else if (c->kinds[i] == 'i' && PyIndex_Check(a)) {  // numpy's and torch's whole numbers, as ctypes takes them
+        PyObject* whole_number = PyNumber_Index(a);
+        if (!whole_number) return nullptr;
+        x = PyLong_AsLong(whole_number);
+        Py_DECREF(whole_number);
+        if (x == -1 && PyErr_Occurred()) return nullptr;
+      } else if (c->kinds[i] == 'i' || a != Py_None) {
+        PyErr_Format(PyExc_TypeError, "argument %d: %s expected, not %s", i + 1,
+                     c->kinds[i] == 'p' ? "an address or None" : "an int", Py_TYPE(a)->tp_name);
+        return nullptr;
       }
       v[whole++] = x;
     }

@@ -88,6 +88,38 @@ def test_what_is_no_argument_is_refused(callees):
         _native(by_signature["p"])(1.5)
 
 
+def test_what_stands_for_a_whole_number_is_taken_as_ctypes_takes_it(callees):
+    numpy, torch = pytest.importorskip("numpy"), pytest.importorskip("torch")
+
+    class Stands:
+        def __index__(self):
+            return -7
+
+    class Refuses:
+        def __index__(self):
+            raise ValueError("none")
+
+    by_signature, seen = dict(callees[0]), callees[1]
+    fn = by_signature["iiiiiii"]
+    native = _native(fn)
+    values = (True, numpy.int64(5), numpy.uint8(200), torch.tensor(-3), torch.tensor([9]), Stands(), numpy.int32(-2 ** 31))
+    code = fn(*values)
+    want = ctypes.string_at(ctypes.addressof(seen))
+    assert native(*values) == code and ctypes.string_at(ctypes.addressof(seen)) == want
+    with pytest.raises(ValueError):
+        native(1, 2, 3, 4, 5, 6, Refuses())
+    for bad in (numpy.float64(2), torch.tensor(1.5), torch.tensor([1, 2])):
+        with pytest.raises(ctypes.ArgumentError):
+            fn(1, 2, 3, 4, 5, 6, bad)
+        with pytest.raises(TypeError):
+            native(1, 2, 3, 4, 5, 6, bad)
+    address = by_signature["p"]
+    with pytest.raises(ctypes.ArgumentError):
+        address(numpy.int64(8))
+    with pytest.raises(TypeError):
+        _native(address)(numpy.int64(8))
+
+
 def test_signatures_beyond_the_common_type_stay_with_ctypes(callees):
     from qwen3_runtime_b200.ops import build
 
