@@ -146,8 +146,8 @@ def compile_group(group: str, *, verbose: bool = True, variant: str = "", define
     return out
 
 
-def compile_groups(groups: list[str], *, verbose: bool = True) -> dict[str, Path]:
-    """Compile several groups in parallel (one nvcc each)."""
+def compile_groups(groups: list[str], *, verbose: bool = True, optional: tuple[str, ...] = ()) -> dict[str, Path]:
+    """Compile several groups in parallel (one nvcc each).  What fails of ``optional`` ones is left to whoever asks for them."""
     results: dict[str, Path] = {}
     errors: list[BaseException] = []
     build_dir()  # settle the folder before the threads start
@@ -156,9 +156,10 @@ def compile_groups(groups: list[str], *, verbose: bool = True) -> dict[str, Path
         try:
             results[g] = compile_group(g, verbose=verbose)
         except BaseException as exc:  # noqa: BLE001 - re-raised below
-            errors.append(exc)
+            if g not in optional:
+                errors.append(exc)
 
-    threads = [threading.Thread(target=work, args=(g,)) for g in groups]
+    threads = [threading.Thread(target=work, args=(g,)) for g in [*groups, *optional]]
     for t in threads:
         t.start()
     for t in threads:
@@ -187,6 +188,11 @@ def load_group(group: str) -> ctypes.CDLL:
 
 _maker = None  # False: there is none
 _KINDS = {ctypes.c_int: "i", ctypes.c_long: "i", ctypes.c_void_p: "p", ctypes.c_float: "f"}
+
+
+def callers_known() -> bool:
+    """Whether this process has looked for csrc/host_call.cu's library."""
+    return _maker is not None
 
 
 def native_caller(fn):

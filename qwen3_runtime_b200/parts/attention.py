@@ -14,7 +14,7 @@ import torch
 
 from ..cache.layout import KVLayerSpec
 from ..config.spec import PartSpec
-from .base import BuildContext, ParamSpec, Part, StepContext, build_part, register_part
+from .base import BuildContext, ParamSpec, Part, StepContext, build_part, product_groups, register_part
 
 
 class PagedAttention(Part):
@@ -78,9 +78,8 @@ class PagedAttention(Part):
         self.o_bias_vec = tensors.get("o_proj.bias")
 
     def kernel_groups(self):
-        groups = ["rope_kv", "attention_generic", *self.position.kernel_groups()]
+        groups = ["rope_kv", "attention_generic", *product_groups(self.ctx), *self.position.kernel_groups()]
         if self.ctx.dtype == torch.bfloat16:
-            groups += ["gemm_small_m", "gemm_stream"]
             # the specialised attention kernels that this head size can reach (ops.paged_attention)
             group = self.num_heads // self.num_kv_heads
             if self.head_dim in (64, 128, 256) and group <= 16:
@@ -89,8 +88,6 @@ class PagedAttention(Part):
                 groups.append("attention_prefill")
             if self.head_dim == 128 and not self.window and 128 % group == 0:
                 groups.append("attention_prefill_tc")
-        if self.ctx.dtype == torch.float32:
-            groups.append("gemm_f32")
         return groups
 
     def step_choosers(self):

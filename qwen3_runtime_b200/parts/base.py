@@ -121,6 +121,12 @@ class Part:
         return None
 
 
+def product_groups(ctx: BuildContext) -> list[str]:
+    """CUDA source groups of the products that ``ops.linear`` and ``ops.gated_linear`` choose from (without the gated product of a
+    whole prompt, ``gemm_tcgen05``)."""
+    return ["gemm_f32"] if ctx.dtype == torch.float32 else ["gemm_small_m", "gemm_stream", "gemm_few_tokens"]
+
+
 _REGISTRY: dict[tuple[str, str], Callable[[PartSpec, BuildContext], Part]] = {}
 
 

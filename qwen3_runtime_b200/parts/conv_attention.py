@@ -18,7 +18,7 @@ import torch
 
 from ..cache.layout import KVLayerSpec, StateLayerSpec
 from ..config.spec import PartSpec
-from .base import BuildContext, ParamSpec, StepContext, build_part, register_part
+from .base import BuildContext, ParamSpec, StepContext, build_part, product_groups, register_part
 from .linear_state import BranchMixer
 
 
@@ -76,8 +76,7 @@ class ConvWindowAttention(BranchMixer):
         return self.o_weight
 
     def kernel_groups(self):
-        groups = ["short_conv", "attention_generic"]
-        groups += ["gemm_f32"] if self.ctx.dtype == torch.float32 else ["gemm_small_m", "gemm_stream"]
+        groups = ["short_conv", "attention_generic", *product_groups(self.ctx)]
         if self._specialised():
             groups += ["attention_decode", "attention_prefill"]
         return groups

@@ -18,7 +18,7 @@ from __future__ import annotations
 import torch
 
 from ..cache.layout import StateLayerSpec
-from .base import BuildContext, ParamSpec, StepContext, register_part, scan_lengths
+from .base import BuildContext, ParamSpec, StepContext, product_groups, register_part, scan_lengths
 from .linear_state import BranchMixer, _pad_rows
 
 
@@ -83,9 +83,7 @@ class GatedDelta(BranchMixer):
         return self.o_weight
 
     def kernel_groups(self):
-        groups = ["delta_state", "linear_state"]
-        groups += ["gemm_f32"] if self.ctx.dtype == torch.float32 else ["gemm_small_m", "gemm_stream"]
-        return groups
+        return ["delta_state", "linear_state", *product_groups(self.ctx)]
 
     def cache_spec(self):
         ring = StateLayerSpec((self.taps, self.channels)) if self.taps > 1 else None

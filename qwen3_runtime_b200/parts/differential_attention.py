@@ -21,7 +21,7 @@ from __future__ import annotations
 import torch
 
 from ..cache.layout import KVLayerSpec
-from .base import BuildContext, ParamSpec, Part, StepContext, register_part
+from .base import BuildContext, ParamSpec, Part, StepContext, product_groups, register_part
 from .linear_state import _pad_rows
 
 
@@ -69,10 +69,8 @@ class DifferentialAttention(Part):
         self.lam = float(torch.exp(first) - torch.exp(second) + self.diff)
 
     def kernel_groups(self):
-        groups = ["rope_kv", "attention_generic"]
-        groups += ["gemm_f32"] if self.ctx.dtype == torch.float32 else ["gemm_small_m", "gemm_stream", "attention_diff",
-                                                                             "attention_prefill_tc"]
-        return groups
+        groups = ["rope_kv", "attention_generic", *product_groups(self.ctx)]
+        return groups + ([] if self.ctx.dtype == torch.float32 else ["attention_diff", "attention_prefill_tc"])
 
     def cache_spec(self):
         return KVLayerSpec(self.num_kv_heads, 2 * self.dim, self.window, value_dim=self.vdim, chunk=self.chunk)

@@ -34,7 +34,7 @@ from __future__ import annotations
 
 import torch
 
-from .base import BuildContext, ParamSpec, Part, StepContext, register_part
+from .base import BuildContext, ParamSpec, Part, StepContext, product_groups, register_part
 
 
 class RoutedExperts(Part):
@@ -126,12 +126,7 @@ class RoutedExperts(Part):
             self.shared_down = tensors["shared.down"].contiguous()
 
     def kernel_groups(self):
-        groups = ["experts", "norm"]
-        if self.ctx.dtype == torch.float32:
-            groups.append("gemm_f32")
-        else:
-            groups += ["gemm_small_m", "gemm_stream", "experts_tcgen05"]
-        return groups
+        return ["experts", "norm", *product_groups(self.ctx)] + ([] if self.ctx.dtype == torch.float32 else ["experts_tcgen05"])
 
     def forward(self, h: torch.Tensor, step: StepContext) -> torch.Tensor:
         ops = self.ops

@@ -6,7 +6,7 @@ from __future__ import annotations
 
 import torch
 
-from .base import BuildContext, ParamSpec, Part, StepContext, register_part
+from .base import BuildContext, ParamSpec, Part, StepContext, product_groups, register_part
 
 
 class GatedMLP(Part):
@@ -46,9 +46,7 @@ class GatedMLP(Part):
         self.down_bias_vec = tensors.get(n["down_bias"])
 
     def kernel_groups(self):
-        if self.ctx.dtype == torch.float32:
-            return ["norm", "gemm_f32"]
-        return ["norm", "gemm_small_m", "gemm_stream", "gemm_tcgen05"]
+        return ["norm", *product_groups(self.ctx)] + ([] if self.ctx.dtype == torch.float32 else ["gemm_tcgen05"])
 
     def forward(self, h: torch.Tensor, step: StepContext) -> torch.Tensor:
         mid = torch.empty((h.shape[0], self.intermediate_size), dtype=h.dtype, device=h.device)
@@ -84,7 +82,7 @@ class ClampedMLP(Part):
         self.down_weight = tensors["down"].contiguous()
 
     def kernel_groups(self):
-        return ["norm", "gemm_f32"] if self.ctx.dtype == torch.float32 else ["norm", "gemm_small_m", "gemm_stream"]
+        return ["norm", *product_groups(self.ctx)]
 
     def forward(self, h: torch.Tensor, step: StepContext) -> torch.Tensor:
         mid = torch.empty((h.shape[0], self.intermediate_size), dtype=h.dtype, device=h.device)

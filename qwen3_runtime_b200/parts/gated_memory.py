@@ -27,12 +27,8 @@ from __future__ import annotations
 import torch
 
 from ..cache.layout import StateLayerSpec
-from .base import BuildContext, ParamSpec, Part, StepContext, register_part, scan_lengths
+from .base import BuildContext, ParamSpec, Part, StepContext, product_groups, register_part, scan_lengths
 from .linear_state import _pad_rows, heads_view
-
-
-def _product_groups(ctx: BuildContext) -> list[str]:
-    return ["gemm_f32"] if ctx.dtype == torch.float32 else ["gemm_small_m", "gemm_stream"]
 
 
 class MatrixLstm(Part):
@@ -66,7 +62,7 @@ class MatrixLstm(Part):
         self.f_bias = tensors["f.b"].contiguous()
 
     def kernel_groups(self):
-        return ["linear_state", *_product_groups(self.ctx)]
+        return ["linear_state", *product_groups(self.ctx)]
 
     def cache_spec(self):
         # the memory with the normaliser as its last value column, and the running maximum
@@ -127,7 +123,7 @@ class ShiftedWkv(Part):
         self.norm_weight = tensors["norm"].contiguous()
 
     def kernel_groups(self):
-        return ["linear_state", "token_state", "norm", *_product_groups(self.ctx)]
+        return ["linear_state", "token_state", "norm", *product_groups(self.ctx)]
 
     def cache_spec(self):
         # the memory, and the previous token's input row

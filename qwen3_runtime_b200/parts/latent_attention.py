@@ -23,7 +23,7 @@ import torch
 
 from ..cache.layout import LatentLayerSpec
 from ..config.spec import PartSpec
-from .base import BuildContext, ParamSpec, Part, StepContext, build_part, register_part
+from .base import BuildContext, ParamSpec, Part, StepContext, build_part, product_groups, register_part
 from .linear_state import _pad_rows
 
 
@@ -113,11 +113,8 @@ class LatentAttention(Part):
                 and self.kv_rank % 8 == 0 and hasattr(self.ops, "latent_expand_rows"))
 
     def kernel_groups(self):
-        groups = ["latent_attention", "head_gemm", *self.position.kernel_groups()]
-        if self.ctx.dtype == torch.float32:
-            groups.append("gemm_f32")
-        else:
-            groups += ["gemm_small_m", "gemm_stream"]
+        groups = ["latent_attention", "head_gemm", *product_groups(self.ctx), *self.position.kernel_groups()]
+        if self.ctx.dtype != torch.float32:
             if self.row_width % 16 == 0 and self.kv_rank % 16 == 0 and self.kv_rank <= 512:
                 groups.append("latent_attention_tc")
             if self._expands():

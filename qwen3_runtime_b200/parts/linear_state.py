@@ -24,7 +24,8 @@ import torch
 
 from ..cache.layout import StateLayerSpec
 from ..config.spec import PartSpec
-from .base import Addend, BuildContext, ParamSpec, Part, StepContext, build_part, register_part, scan_lengths
+from .base import (Addend, BuildContext, ParamSpec, Part, StepContext, build_part, product_groups, register_part,
+                   scan_lengths)
 
 
 def heads_view(rows: torch.Tensor, start: int, heads: int, size: int) -> torch.Tensor:
@@ -120,9 +121,7 @@ class _DecayedStateMixer(BranchMixer):
         return self.o_weight
 
     def kernel_groups(self):
-        groups = ["linear_state"]
-        groups += ["gemm_f32"] if self.ctx.dtype == torch.float32 else ["gemm_small_m", "gemm_stream"]
-        return groups
+        return ["linear_state", *product_groups(self.ctx)]
 
     def cache_spec(self):
         return StateLayerSpec((self.num_heads, self.dim, self.vdim))

@@ -10,7 +10,7 @@ import torch
 
 from ..cache.layout import CacheLayout, kept_for_readers
 from ..config.spec import ModelSpec
-from .base import BuildContext, ParamSpec, ResidualStream, StepContext, build_part
+from .base import BuildContext, ParamSpec, ResidualStream, StepContext, build_part, product_groups
 from .norm import fold_stream
 
 EMBEDDING_CACHE = -1  # cache layer id of what the embedding part keeps per request
@@ -101,7 +101,7 @@ class DecoderModel:
         self.loaded = True
 
     def kernel_groups(self) -> list[str]:
-        groups = {"norm"}
+        groups = {"norm", *product_groups(self.ctx)}  # (products: the output head)
         for part in [*self.blocks, self.final_norm, *([self.embedding] if self.embedding is not None else [])]:
             groups.update(part.kernel_groups())
         return sorted(groups)

@@ -32,7 +32,7 @@ import torch
 
 from ..cache.layout import KVLayerSpec
 from ..config.spec import PartSpec
-from .base import BuildContext, ParamSpec, StepContext, build_part, register_part
+from .base import BuildContext, ParamSpec, StepContext, build_part, product_groups, register_part
 from .linear_state import BranchMixer, _pad_rows
 
 
@@ -163,8 +163,7 @@ class SinkWindowAttention(BranchMixer):
         return self.o_weight
 
     def kernel_groups(self):
-        groups = ["rope_kv", "attention_generic"]
-        groups += ["gemm_f32"] if self.ctx.dtype == torch.float32 else ["gemm_small_m", "gemm_stream"]
+        groups = ["rope_kv", "attention_generic", *product_groups(self.ctx)]
         if self.ctx.dtype == torch.bfloat16 and not self.window and not self.gate and not self.softcap:
             if self.turned or not self._specialised() or self.dim == 256:
                 groups.append("attention_chunk")

@@ -15,7 +15,7 @@ from __future__ import annotations
 
 import torch
 
-from .base import BuildContext, ParamSpec, Part, ResidualStream, StepContext, register_part
+from .base import BuildContext, ParamSpec, Part, ResidualStream, StepContext, product_groups, register_part
 
 
 class GatedTokenInput(Part):
@@ -40,7 +40,7 @@ class GatedTokenInput(Part):
         self.norm_weight = tensors["norm"].contiguous()
 
     def kernel_groups(self):
-        return ["norm"] + (["gemm_f32"] if self.ctx.dtype == torch.float32 else ["gemm_small_m", "gemm_stream"])
+        return ["norm", *product_groups(self.ctx)]
 
     def forward(self, stream: ResidualStream, step: StepContext, fold) -> None:
         """``fold(stream)`` adds what is pending to the residual sum and returns the sum in the
