@@ -73,7 +73,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
   return true;
 }
-// the same for a barrier on which other blocks of the cluster arrive behind what they wrote
+// the same for a barrier on which other blocks of the cluster arrive
 __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   if (mbar_try_wait_cluster(bar, parity)) return true;
   const long long start = clock64();
@@ -137,11 +137,12 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void remote_arrive(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// The same in the default form (released to this block only): for what the arrival itself orders -- tensor memory that has been
-// read, shared memory behind a proxy fence that an MMA of the pair's leader will read.  With the release to the cluster the warp
-// waits about 1000 cycles for it.
-__device__ __forceinline__ void remote_arrive_only(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+// The same without a release: for what the arrival has to order is tensor memory alone, read (tcgen05.wait::ld) or written
+// (tcgen05.wait::st) by this warp.  tcgen05.fence::before_thread_sync ahead of it and ::after_thread_sync behind the wait order that,
+// and nothing that the warp wrote to shared or global memory may be read by whoever waits.  (With the release to the cluster the
+// warp waits about 1000 cycles for it.)
+__device__ __forceinline__ void remote_arrive_relaxed(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");

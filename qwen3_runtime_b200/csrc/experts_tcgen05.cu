@@ -167,7 +167,7 @@ expert_tcgen05_kernel(const __grid_constant__ Maps maps, bf16* __restrict__ out,
         const uint32_t idesc = umma_idesc(256, t.n);
         const int buf = i & 1;
         // both epilogues have drained it
-        ok = __all_sync(0xffffffffu, mbar_wait(acc_empty0 + 8 * buf, ((i >> 1) & 1) ^ 1, &abort_flag));
+        ok = __all_sync(0xffffffffu, mbar_wait_cluster(acc_empty0 + 8 * buf, ((i >> 1) & 1) ^ 1, &abort_flag));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = acc0 + buf * ACC_COLS;
@@ -206,7 +206,7 @@ expert_tcgen05_kernel(const __grid_constant__ Maps maps, bf16* __restrict__ out,
       if (any_gave_up(group + 1, 128, lost)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t lane_addr = tmem_base + buf * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
-      if (group * 32 >= t.n && lane == 0) remote_arrive_only(leader_acc_empty0 + 8 * buf);  // nothing here for this group
+      if (group * 32 >= t.n && lane == 0) remote_arrive_relaxed(leader_acc_empty0 + 8 * buf);  // nothing here for this group
 #pragma unroll 1
       for (int c0 = group * 32; c0 < t.n; c0 += 64) {
         uint32_t acc[32];
@@ -214,7 +214,7 @@ expert_tcgen05_kernel(const __grid_constant__ Maps maps, bf16* __restrict__ out,
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (c0 + 64 >= t.n) {  // the last of this buffer for this group is in registers: hand it back to the MMA issuer
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          if (lane == 0) remote_arrive_only(leader_acc_empty0 + 8 * buf);
+          if (lane == 0) remote_arrive_relaxed(leader_acc_empty0 + 8 * buf);
         }
         // (whatever follows takes the products rounded to bfloat16, as separate kernels would)
 #pragma unroll

@@ -326,7 +326,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_con
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) {
-        remote_arrive_only(leader_w_full + 8 * ws);
+        remote_arrive_relaxed(leader_w_full + 8 * ws);
         // (given back behind the stores of what they became: an arrival does not wait for loads that are still on their way)
         mbar_arrive(bar(RAW_EMPTY + raw_st));
       }
@@ -368,7 +368,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_con
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        if (lane == 0) remote_arrive_only(leader_d_empty + 8 * st);
+        if (lane == 0) remote_arrive_relaxed(leader_d_empty + 8 * st);
       }
       if (!ok) break;
       const int row0 = it.row0 + quarter * 32, t0 = it.token0 + col0;

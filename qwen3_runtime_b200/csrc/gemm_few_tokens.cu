@@ -156,7 +156,7 @@ few_tokens_kernel(const __grid_constant__ Maps maps, void* __restrict__ out, lon
         const int kb0 = item / plan.tiles * plan.per, kb1 = min(num_kb, kb0 + plan.per);
         for (int g0 = kb0; g0 < kb1; g0 += group) {
           const int g1 = min(kb1, g0 + group);
-          ok = __all_sync(0xffffffffu, mbar_wait(acc_empty0 + 8 * buf, acc_phase, &abort_flag));
+          ok = __all_sync(0xffffffffu, mbar_wait_cluster(acc_empty0 + 8 * buf, acc_phase, &abort_flag));
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t acc = acc0 + buf * BUF_COLS;
@@ -214,7 +214,7 @@ few_tokens_kernel(const __grid_constant__ Maps maps, void* __restrict__ out, lon
           for (int g = 0; g < SUMS; ++g) tmem_load16(lane_addr + 32 * g, r[g]);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          if (lane == 0) remote_arrive_only(leader_acc_empty0 + 8 * buf);
+          if (lane == 0) remote_arrive_relaxed(leader_acc_empty0 + 8 * buf);
           buf ^= 1, phase ^= buf ^ 1;
 #pragma unroll
           for (int c = 0; c < FEW; ++c) {
@@ -234,7 +234,7 @@ few_tokens_kernel(const __grid_constant__ Maps maps, void* __restrict__ out, lon
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
           if (c0 + 32 >= n) {  // the last of this buffer is in registers: hand it back to the MMA issuer
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            if (lane == 0) remote_arrive_only(leader_acc_empty0 + 8 * buf);
+            if (lane == 0) remote_arrive_relaxed(leader_acc_empty0 + 8 * buf);
             buf ^= 1, phase ^= buf ^ 1;
           }
 #pragma unroll
