@@ -42,9 +42,8 @@ constexpr int EXPERT_BM = 32;  // slots per row tile of the FMA products
 // on a softmax over all outputs (route_pick_softmax_all).
 constexpr int ROUTE_TT = 8;
 
-template <typename T>
 __global__ void __launch_bounds__(256)
-route_logits_kernel(const T* __restrict__ h, long h_stride, const float* __restrict__ router, int num_tokens, int E,
+route_logits_kernel(const float* __restrict__ h, long h_stride, const float* __restrict__ router, int num_tokens, int E,
                     int W, int tt, int vec, float* __restrict__ logits) {
   extern __shared__ float route_rows[];  // [tt][W], tt <= ROUTE_TT tokens per block
   pdl_wait();
@@ -53,7 +52,7 @@ route_logits_kernel(const T* __restrict__ h, long h_stride, const float* __restr
   const int nt = min(tt, num_tokens - t0);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int t = 0; t < nt; ++t) {
-    const T* src = h + (long)(t0 + t) * h_stride;
+    const float* src = h + (long)(t0 + t) * h_stride;
     if (vec) {
       for (int i = threadIdx.x * 8; i < W; i += 256 * 8) {
         float v[8];
@@ -61,7 +60,7 @@ route_logits_kernel(const T* __restrict__ h, long h_stride, const float* __restr
         store8(route_rows + t * W + i, v);
       }
     } else {
-      for (int i = threadIdx.x; i < W; i += 256) route_rows[t * W + i] = to_f32(src[i]);
+      for (int i = threadIdx.x; i < W; i += 256) route_rows[t * W + i] = src[i];
     }
   }
   __syncthreads();
@@ -101,19 +100,13 @@ route_logits_kernel(const T* __restrict__ h, long h_stride, const float* __restr
 }
 
 __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 load4(const bf16* p) {
-  const uint2 raw = *reinterpret_cast<const uint2*>(p);
-  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
-  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-  return make_float4(a.x, a.y, b.x, b.y);
-}
 
 constexpr int ROUTE_EPW = 8;  // experts per warp
 
 // WT, WE: warps of a block along tokens and along experts
-template <typename T, int WT, int WE>
+template <int WT, int WE>
 __global__ void __launch_bounds__(32 * WT * WE, 3)
-route_logits_tile_kernel(const T* __restrict__ h, long h_stride, const float* __restrict__ router, int num_tokens, int E,
+route_logits_tile_kernel(const float* __restrict__ h, long h_stride, const float* __restrict__ router, int num_tokens, int E,
                          int W, float* __restrict__ logits) {
   pdl_wait();
   pdl_launch_dependents();
@@ -124,7 +117,7 @@ route_logits_tile_kernel(const T* __restrict__ h, long h_stride, const float* __
   // a last group that would pass the end starts earlier: its first logits are computed twice, with the same bits
   t0 = min(t0, num_tokens - ROUTE_TT);
   e0 = min(e0, E - ROUTE_EPW);
-  const T* x = h + (long)t0 * h_stride + lane * 4;
+  const float* x = h + (long)t0 * h_stride + lane * 4;
   const float* w = router + (long)e0 * W + lane * 4;
   float acc[ROUTE_TT][ROUTE_EPW];
 #pragma unroll
@@ -494,6 +487,16 @@ __global__ void route_pick_softmax_all_kernel(const float* __restrict__ logits, 
     }
 }
 
+static int sm_count() {
+  static int count_on[Q3_MAX_DEVICES];
+  int& count = count_on[q3_current_device()];
+  int device = 0;
+  if (!count && (cudaGetDevice(&device) != cudaSuccess ||
+                 cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess))
+    count = 0;
+  return count;
+}
+
 // logits: fp32 scratch [num_tokens, E].
 // scale: a factor on all weights.  mode 3 takes correction (fp32 [E] or null), count and keep (groups) and renorm; the other modes ignore them.
 Q3_EXPORT int q3_route_top(int dtype, const void* h, long h_stride, const float* router, int num_tokens, int E, int W,
@@ -509,13 +512,13 @@ Q3_EXPORT int q3_route_top(int dtype, const void* h, long h_stride, const float*
   if (dtype == Q3_DTYPE_BF16) {
     const bool vec = W % 8 == 0 && h_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0;
     const dim3 large((num_tokens + 31) / 32, (E + 31) / 32), small((num_tokens + 15) / 16, (E + 7) / 8);
-    if (small.y > 65535) return Q3_ERR_UNSUPPORTED;
 #define Q3_ROUTE_MMA(MT_, NT_, VEC_, grid_)                                                                              \
   e = launch_pdl(route_logits_mma_kernel<MT_, NT_, VEC_>, grid_, dim3(32 * ROUTE_WARPS), 0, stream, (const bf16*)h, h_stride, \
                  router, num_tokens, E, W, logits)
     // large blocks from where they fill half of the SMs, and where 32 experts are not mostly none (8 x 512, 4096 tokens: 13.7 us
     // with the choice, 6.1 with small blocks)
-    if (vec && E > 16 && (long)large.x * large.y >= 74) Q3_ROUTE_MMA(2, 4, true, large);
+    if (vec && E > 16 && 2l * large.x * large.y >= sm_count() && large.y <= 65535) Q3_ROUTE_MMA(2, 4, true, large);
+    else if (small.y > 65535) return Q3_ERR_UNSUPPORTED;
     else if (vec) Q3_ROUTE_MMA(1, 1, true, small);
     else Q3_ROUTE_MMA(1, 1, false, small);
 #undef Q3_ROUTE_MMA
@@ -529,7 +532,7 @@ Q3_EXPORT int q3_route_top(int dtype, const void* h, long h_stride, const float*
     if (tile && (E + te - 1) / te <= 65535) {
       const dim3 grid((num_tokens + tokens - 1) / tokens, (E + te - 1) / te);
 #define Q3_ROUTE_TILE(WT_, WE_)                                                                                          \
-  e = launch_pdl(route_logits_tile_kernel<float, WT_, WE_>, grid, dim3(32 * WT_ * WE_), 0, stream, (const float*)h, h_stride, \
+  e = launch_pdl(route_logits_tile_kernel<WT_, WE_>, grid, dim3(32 * WT_ * WE_), 0, stream, (const float*)h, h_stride, \
                  router, num_tokens, E, W, logits)
       if (we == 4) Q3_ROUTE_TILE(1, 4); else if (we == 2) Q3_ROUTE_TILE(2, 2); else Q3_ROUTE_TILE(4, 1);
 #undef Q3_ROUTE_TILE
@@ -541,8 +544,8 @@ Q3_EXPORT int q3_route_top(int dtype, const void* h, long h_stride, const float*
       const dim3 grid((num_tokens + tt - 1) / tt, (E + 7) / 8);
       const int vec = W % 8 == 0 && h_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0;
       if (smem > 48 * 1024)
-        cudaFuncSetAttribute(route_logits_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      e = launch_pdl(route_logits_kernel<float>, grid, dim3(256), smem, stream, (const float*)h, h_stride, router,
+        cudaFuncSetAttribute(route_logits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      e = launch_pdl(route_logits_kernel, grid, dim3(256), smem, stream, (const float*)h, h_stride, router,
                      num_tokens, E, W, tt, vec, logits);
     }
   }
