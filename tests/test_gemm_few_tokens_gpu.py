@@ -1,4 +1,4 @@
-"""Products of 17 to 128 tokens (csrc/gemm_few_tokens.cu) against float64, at the edges of its tiles and of its dispatch."""
+"""Products of up to 128 tokens (csrc/gemm_few_tokens.cu) against float64, at the edges of its tiles and of its dispatch."""
 
 import pytest
 import torch
@@ -118,6 +118,82 @@ def test_routes_agree(ops, M, pad):
     bound = 1.1 * (off_gate * (up.abs() + off_up) + off_up * gate.abs()) + 2.0**-8 * want.abs() + 1e-12
     if pad % 8 == 0 or M <= 16:
         assert bool(((got.double() - want).abs() <= bound).all())
+
+
+def large(M, N, K):
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x = torch.randn((M, K), generator=g, device="cuda").to(BF16)
+    return x, (0.02 * torch.randn((N, K), generator=g, device="cuda")).to(BF16)
+
+
+def launched(ops, monkeypatch, call):
+    """The result of ``call()`` and the modes in which it launched this file's kernel."""
+    modes, under = [], ops._call
+
+    def spy(group, name, what, *args):
+        modes.extend(args[:1] if name == "q3_gemm_few_tokens" else [])
+        return under(group, name, what, *args)
+
+    monkeypatch.setattr(ops, "_call", spy)
+    result = call()
+    monkeypatch.undo()
+    ops.raise_if_kernel_error()
+    return result, modes
+
+
+# both sides of every line of CudaOps.FEW_TOKENS: tokens, rows, values, result, whether it is this kernel's
+@pytest.mark.parametrize("M,N,K,dtype,taken", [
+    (1, 24576, 64, F32, True), (16, 24568, 64, F32, False), (16, 24576, 64, BF16, True), (17, 24576, 64, BF16, True),
+    (17, 24568, 64, F32, False), (64, 24576, 64, BF16, True), (65, 24576, 64, BF16, False), (128, 24576, 64, F32, True),
+    (129, 24576, 64, F32, False), (16, 10240, 5080, BF16, True), (16, 10240, 5072, BF16, False), (16, 10232, 5088, BF16, False),
+    (1, 10240, 5080, F32, True), (17, 10240, 5080, F32, False)])
+def test_which_finished_products_are_taken(ops, monkeypatch, M, N, K, dtype, taken):
+    x, w = large(M, N, K)
+    got, modes = launched(ops, monkeypatch, lambda: ops.linear(x, w, out_dtype=dtype))
+    assert modes == [int(dtype == F32)] * taken and got.dtype == dtype
+    want = x.double() @ w.double().t()
+    assert bool(((got.double() - want).abs() <= f32_bound(x, w) + (2.0**-8 * want.abs() if dtype == BF16 else 0)).all())
+
+
+@pytest.mark.parametrize("M,N,K,taken", [
+    (16, 3664, 12288, True), (16, 3656, 12288, False), (16, 3680, 12280, False), (1, 3664, 12288, True), (17, 1024, 3072, True),
+    (17, 1024, 3064, False), (17, 4096, 12288, True), (17, 4104, 12288, False), (64, 1024, 3072, True), (65, 1024, 3072, False)])
+def test_which_partial_sums_are_taken(ops, monkeypatch, M, N, K, taken):
+    x, w = large(M, N, K)
+    got, modes = launched(ops, monkeypatch, lambda: ops.linear(x, w, partial_sums=True))
+    assert modes == [1] * taken
+    want, bound = x.double() @ w.double().t(), f32_bound(x, w)
+    if got.dim() == 3:
+        got = got.double().sum(0)
+    else:
+        assert not taken
+        bound = bound + 2.0**-8 * want.abs()
+    assert bool(((got.double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("M,I,K,taken", [
+    (1, 9768, 4096, True), (16, 9768, 4096, True), (16, 9760, 4096, False), (17, 2448, 4096, True), (17, 2440, 4096, False),
+    (32, 2448, 4096, True), (33, 2448, 4096, False), (33, 16384, 64, True), (33, 16376, 64, False), (64, 16384, 64, True),
+    (65, 16384, 64, False)])
+@pytest.mark.parametrize("act", ["silu", "gelu"])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_which_gated_products_are_taken(ops, monkeypatch, M, I, K, taken, act, aligned):
+    x, w = large(M, 2 * I, K)
+    if not aligned:  # rows at odd multiples of 8 bytes: never this kernel's
+        x = torch.nn.functional.pad(x, (0, 4))[:, :K]
+    got, modes = launched(ops, monkeypatch, lambda: ops.gated_linear(x, w, torch.empty((M, I), dtype=BF16, device="cuda"), act))
+    assert (modes == [2 + (act == "gelu")]) == (taken and aligned) and (aligned or not modes)
+    sums = x.double() @ w.double().t()
+    gate, up = sums[:, :I], sums[:, I:]
+    unit = torch.nn.functional.silu(gate) if act == "silu" else torch.nn.functional.gelu(gate, approximate="tanh")
+    want = unit * up
+    # gate and up are off by their fp32 sums and may be rounded to the neighbouring bfloat16 (2^-8 of them); where the library takes
+    # rows off 16 bytes, it may cut K and round the ranges' sums and their additions, each at most the sum of magnitudes, as well (16
+    # ranges: 16 x 2^-8).  The unit's slope in the gate is at most 1.13, and the result is rounded once more.
+    magnitudes = x.double().abs() @ w.double().abs().t()
+    off = f32_bound(x, w) + 2.0**-8 * sums.abs() + (0 if aligned else 16 * 2.0**-8 * magnitudes)
+    bound = 1.13 * (off[:, :I] * (up.abs() + off[:, I:]) + off[:, I:] * gate.abs()) + 2.0**-8 * want.abs() + 1e-12
+    assert bool(((got.double() - want).abs() <= bound).all())
 
 
 def test_weights_the_kernel_before_writes_and_a_captured_step(ops):
