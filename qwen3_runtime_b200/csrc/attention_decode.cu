@@ -196,9 +196,9 @@ __device__ __forceinline__ int slices_of(const int* __restrict__ kv_lens, const 
 // FUSED: `q` is the raw q/k/v projection; the block norms and rotates its own queries, and the
 // block whose slice holds the newest position also makes that token's key and value, writes
 // them to their page and patches them into its tile (q/k/v math as in rope_kv.cu, same order of
-// operations, so both ways give the same bits).  Nothing the block reads before pdl_wait() is
-// written by a kernel of the same step, so the first key tiles are in flight while the
-// projection before this kernel is still finishing.
+// operations, so both ways give the same bits).  Ahead of pdl_wait() it reads lengths and works out
+// its slice only; the projection's values, the angles and norm weights, the block table and the first
+// tile are asked for together right behind it (see there).
 // Blocks an SM has to hold (the cost model of the slice count assumes them): without the bound an option more in the
 // newest token's part can cost a block, and with it a sixth of a long step.
 template <int D> constexpr int resident_blocks() { return D == 64 ? 4 : D == 128 ? 3 : 1; }

@@ -449,8 +449,9 @@ static inline int segments_of(int N, int K) {
 }  // namespace split
 
 // Segments the product's K is cut into; 0: not a product for this kernel.  The tokens must have no say in it, so the line is
-// where few tokens do not lose: weights of 20 M values (one token, us, here when this was chosen / FMA: 8192 x 2560 38 / 41,
-// 7680 x 2688 38 / 43, 12288 x 2048 44 / 43, 5120 x 5120 44 / 64, 2560 x 9728 42 / 88).
+// where few tokens do not lose: weights of 20 M values (one token, us, here, parts and sums included / FMA: 8192 x 2560 32 / 38,
+// 7680 x 2688 32 / 39, 12288 x 2048 36 / 41, 5120 x 5120 35 / 62, 2560 x 9728 34 / 84, 24576 x 4096 83 / 125; 33 tokens of the first 33
+// / 84).  (It was drawn for the single blocks, for which the first three were level; a line further down would change the bits.)
 Q3_EXPORT int q3_gemm_f32_split_segments(int N, int K) {
   return N < 256 || N % 4 || K < 1024 || K % 8 || (long)N * K < 20000000 ? 0 : split::segments_of(N, K);
 }

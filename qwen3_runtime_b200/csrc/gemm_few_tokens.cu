@@ -1,4 +1,4 @@
-// Products of 17 to 128 tokens on the 5th-generation tensor cores:  out[M, N] = x[M, K] W[N, K]^T, bfloat16 operands.
+// Products of up to 128 tokens on the 5th-generation tensor cores:  out[M, N] = x[M, K] W[N, K]^T, bfloat16 operands.
 //
 // What bounds them: the weights' stream from memory (100 MB of gate_up take 15 us at the copy rate; 48 tokens' products a
 // quarter of that), as long as every SM has the same share of it and the tokens' rows, which every SM reads from L2, stay a
@@ -289,7 +289,7 @@ few_tokens_kernel(const __grid_constant__ Maps maps, void* __restrict__ out, lon
   if (threadIdx.x == 0 && abort_flag && error_word) atomicExch(error_word, 1);
 }
 
-int tokens_padded(int M) { return (M + 31) / 32 * 32; }  // a pair of SMs takes tokens in steps of 32
+int tokens_padded(int M) { return (M + 31) / 32 * 32; }  // the epilogue takes 32 columns at a time
 
 // Rounds, rows and ranges that leave an SM with the fewest bytes to take in: weights, half as much for the tokens' rows (they come
 // from L2), what partial sums cost on their way out and back in, and 8 KB an item for its ends.

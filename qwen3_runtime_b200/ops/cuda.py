@@ -2074,16 +2074,17 @@ class CudaOps:
     def _product(self, x, weight, out=None, out_dtype=None, partial_sums=False):
         """``x[M, K] @ weight[N, K]^T``.  float32: on the tensor cores with operands in three bfloat16 parts, which is
         nearer to the exact product than a chain of fp32 FMA (:meth:`_f32_segments`), small sizes on the FMA pipes; no TF32.
-        bfloat16, at most 128 tokens: csrc/gemm_few_tokens.cu for output heads and large partial
-        sums (:attr:`FEW_TOKENS`).  bfloat16, at most 16 tokens otherwise: one of this engine's two weight-streaming kernels
-        (:meth:`_small_product`).  bfloat16, more tokens: the library product with fp32
+        bfloat16, at most 128 tokens: csrc/gemm_few_tokens.cu for output heads, other products of many rows, and
+        large partial sums (:attr:`FEW_TOKENS`).  bfloat16, at most 16 tokens otherwise: one of this engine's two weight-streaming
+        kernels (:meth:`_small_product`).  bfloat16, more tokens: the library product with fp32
         accumulation, as the reference's ``nn.Linear`` (qwen3_runtime/models/qwen3.py:76-77,
         134-135), or this engine's tcgen05 kernel with ``large_gemm="tcgen05"``.
 
         ``partial_sums``: the caller also takes float32 ``[parts, M, N]`` whose sum over the
         first axis is the product (what :meth:`fused_norm` accepts as ``pending``).  It gets
-        that when the streaming kernel would cut K into ranges: the blocks then need not
-        wait for one another to add their parts up."""
+        that when the kernel that takes the product would cut K into ranges (the streaming one,
+        or csrc/gemm_few_tokens.cu): the blocks then need not wait for one another to add their
+        parts up."""
         M, K = x.shape
         N = weight.shape[0]
         if weight.shape[1] != K:
