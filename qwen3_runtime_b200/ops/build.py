@@ -155,6 +155,7 @@ def compile_groups(groups: list[str], *, verbose: bool = True, optional: tuple[s
     def work(g: str) -> None:
         try:
             results[g] = compile_group(g, verbose=verbose)
+            _ready.add(g)
         except BaseException as exc:  # noqa: BLE001 - re-raised below
             if g not in optional:
                 errors.append(exc)
@@ -170,11 +171,12 @@ def compile_groups(groups: list[str], *, verbose: bool = True, optional: tuple[s
 
 
 _loaded: dict[str, ctypes.CDLL] = {}
+_ready: set[str] = set()  # whose library this process has found or made
 _lock = threading.Lock()
 
 
-def is_loaded(group: str) -> bool:
-    return group in _loaded
+def is_ready(group: str) -> bool:
+    return group in _loaded or group in _ready
 
 
 def load_group(group: str) -> ctypes.CDLL:

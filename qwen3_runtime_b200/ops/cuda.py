@@ -525,13 +525,14 @@ class CudaOps:
         self.timing: list | None = None
         self._cost = (0, 0, "")
         if groups:
-            build.compile_groups([g for g in groups if not build.is_loaded(g)])
+            build.compile_groups([g for g in groups if not build.is_ready(g)])
 
     def prepare(self, groups: list[str]) -> None:
         """Compile (in parallel) the kernel groups a model is going to use, and what calls them (:func:`build.native_caller`)."""
-        # (what this process has loaded stays loaded, so its sources need not be read and hashed for every table: 0.5 ms and more)
-        build.compile_groups([g for g in groups if g in _SIGNATURES and not build.is_loaded(g)],
-                             optional=() if build.callers_known() else ("host_call",))
+        # (what this process has loaded or compiled is there: its sources need not be read and hashed for every table, 0.5 ms and more
+        # a group; whoever loads a library looks once more)
+        build.compile_groups([g for g in groups if g in _SIGNATURES and not build.is_ready(g)],
+                             optional=() if build.is_ready("host_call") or build.callers_known() else ("host_call",))
 
     # ---- plumbing -------------------------------------------------------------------
     def _get(self, group: str, name: str):

@@ -45,11 +45,15 @@ def test_preparing_compiles_what_calls_the_launchers_too(monkeypatch):
     asked = []
     monkeypatch.setattr(build, "compile_group", lambda g, **kw: asked.append(g))
     monkeypatch.setattr(build, "_loaded", {"rope_kv": None})
+    monkeypatch.setattr(build, "_ready", set())
     monkeypatch.setattr(build, "_maker", None)
     ops = object.__new__(cuda.CudaOps)  # (no device here)
     ops.prepare(["norm", "rope_kv", "a group of other operations"])
     assert sorted(asked) == ["host_call", "norm"]
+    ops.prepare(["norm", "sampling"])  # only what this process has not seen compiled
+    assert sorted(asked) == ["host_call", "norm", "sampling"]
     asked.clear()
+    monkeypatch.setattr(build, "_ready", set())
     monkeypatch.setattr(build, "_maker", False)  # this process has looked for it: there is none
     ops.prepare(["norm"])
     assert asked == ["norm"]
@@ -62,6 +66,7 @@ def test_launchers_are_called_without_it_where_it_does_not_compile(monkeypatch):
 
     monkeypatch.setattr(build, "compile_group", compile_group)
     monkeypatch.setattr(build, "_loaded", {})
+    monkeypatch.setattr(build, "_ready", set())
     monkeypatch.setattr(build, "_maker", None)
     object.__new__(cuda.CudaOps).prepare(["norm"])
     fn = object()
