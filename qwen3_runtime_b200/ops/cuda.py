@@ -2280,26 +2280,36 @@ class CudaOps:
     TCGEN05_MIN_SHARE = 0.65
 
     # What csrc/gemm_few_tokens.cu takes from the other kernels (streams of at most 16 tokens, the library above), as measured at 1 ..
-    # 128 tokens with the sizes of eight models (hidden 896 .. 8192), each alone and up to 16 tokens in whole steps as well.
+    # 128 tokens with the sizes of eight models (hidden 896 .. 8192) and, up to 16 tokens, on a grid of rows and values around every
+    # line; each alone and up to 16 tokens in whole steps as well.
     # Finished products of at least two rounds of 128 rows over the SMs: output heads of 32,000 rows and more 5 to 16 % less than the
-    # library at every token count (one round of 16,384 rows: level); 8 tokens 151,936 x 2560 126 -> 118, x 4096 244 -> 186.
-    # bfloat16 results up to 64 tokens (24576 x 4096 2 to 6 % less); up to 16 tokens from 10,240 rows and 52 M weights on (10240 x
-    # 5120, 8 tokens 22.7 -> 19.3, 16 28.2 -> 19.5; 19456 x 2560: level; 6144 x 4096 11.8 -> 12.7).
+    # library at every token count (one round of 16,384 rows: level); 8 tokens, stream / here: 151,936 x 2560 125 / 116, x 4096 241 / 189.
+    # bfloat16 results up to 64 tokens (24576 x 4096 2 to 6 % less).
+    # Up to 16 tokens from 10,240 rows and 52 M weights on, of more than the 2560 values that the stream holds of a finished row (20480 x
+    # 2560 2 % more to 4 % less, x 2688 28.6 / 21.2 at 16 tokens): 9 to 16 tokens 15 to 35 % less (10240 x 5120 27.8 / 20.5); up to 8
+    # tokens 0 to 20 % less from 4096 values on (22.4 / 20.3; 14336 x 4096 level) or in two rounds (20480 x 3072 26.9 / 23.6), not in
+    # one round of shorter rows (16384 x 3584 20.6 / 22.2).
     # Partial sums, 17 to 64 tokens, where K is cut into four ranges or more: hidden 896 .. 4096 5 to 30 % less; two or three
-    # ranges of 5120 rows 8 % less to 12 % more, 1024 x 2048 2 % more.  Up to 16 tokens of long rows: 4096 x 12288 23.8 -> 21.5, 5120
-    # x 25600 58 -> 47, 8192 x 28672 92 -> 76, 5120 x 17408 level, 2560 x 9728 12.2 -> 12.9, 8192 x 8192 27.5 -> 29.0.
+    # ranges of 5120 rows 8 % less to 12 % more, 1024 x 2048 2 % more.  Up to 16 tokens of long rows: the stream cuts K into eight
+    # ranges and takes as long for 1536 values of each as for 1792, and for 2048 and more by their number.  4096 x 12288 20.2 / 19.0, x
+    # 13056 20.5 / 20.2, but x 14336 20.7 / 21.4, x 16384 24.2 / 24.3, and x 17408 26.0 / 24.9, 8192 x 20480 55.8 / 53.4; 3584 x 18432 24.0 /
+    # 23.8 and 2560 x 18432 17.9 / 18.3: left with the stream.  Beyond 20,480 values, which it cannot hold: 5120 x 24576 54 / 42, 16
+    # tokens 66 / 42.  Rows of fewer than 45 M weights: 2560 x 9728 12.2 / 12.9.
     # Gated: up to 32 tokens 3 to 15 % less from 20 M weights on (6 M: level), up to 64 with 16,384 features and more (48 tokens:
-    # 2 x 17408 6 % less, 2 x 25600 12, 2 x 12288 and 2 x 9728 level).  Up to 16 tokens from 80 M on: 2 x 12288 x 4096 40.8 -> 35.3 (16
-    # tokens 71 -> 37), 2 x 11008 x 4096 39 -> 31, 2 x 25600 x 5120 103 -> 79; 2 x 9728 x 2560 19.3 -> 18.8 alone, a step 1 % more.
+    # 2 x 17408 6 % less, 2 x 25600 12, 2 x 12288 and 2 x 9728 level).  Up to 16 tokens from 80 M on, 8 tokens: 2 x 9768 x 4096 34.6 /
+    # 31.1, 2 x 12288 x 4096 39.5 / 35.9 (16 tokens 68 / 37), 2 x 7816 x 5120 30.1 / 28.8, 2 x 25600 x 5120 101 / 79, 2 x 19456 x 2560
+    # 34.7 / 33.7; 2 x 9728 x 2560 level alone, a step 1 % more.
     FEW_TOKENS, FEW_MIN_ROWS, FEW_BF16_TOKENS = 128, 24576, 64
-    FEW_SMALL_ROWS, FEW_SMALL_ROWS_WEIGHTS = 10240, 52_000_000
+    FEW_SMALL_ROWS, FEW_SMALL_ROWS_WEIGHTS, FEW_SMALL_VALUES, FEW_8_VALUES = 10240, 52_000_000, 2560, 4096
     FEW_PARTS_TOKENS, FEW_MIN_PARTS, FEW_PARTS_MIN_WEIGHTS, FEW_PARTS_ROWS = 64, 4, 3 << 20, 4096
-    FEW_SMALL_PARTS_WEIGHTS, FEW_SMALL_PARTS_VALUES = 45_000_000, 12288
+    FEW_SMALL_PARTS_WEIGHTS, FEW_SMALL_PARTS_ROWS = 45_000_000, 4096
+    FEW_SMALL_PARTS_VALUES, FEW_SMALL_PARTS_LONG, STREAM_VALUES = (12288, 13056), 16896, 20480
     FEW_GATED_TOKENS, FEW_GATED_MIN_WEIGHTS, FEW_GATED_TOKENS_WIDE, FEW_GATED_WIDE = 32, 20_000_000, 64, 16384
     FEW_SMALL_GATED_WEIGHTS = 80_000_000
 
     def _few_finished(self, M: int, N: int, K: int, dtype) -> bool:
-        if M <= self.SMALL_M and N >= self.FEW_SMALL_ROWS and N * K >= self.FEW_SMALL_ROWS_WEIGHTS:
+        if (M <= self.SMALL_M and N >= self.FEW_SMALL_ROWS and N * K >= self.FEW_SMALL_ROWS_WEIGHTS and K > self.FEW_SMALL_VALUES
+                and (M > 8 or K >= self.FEW_8_VALUES or N > 128 * self.SM_COUNT)):
             return True
         return N >= self.FEW_MIN_ROWS and (dtype == torch.float32 or M <= self.FEW_BF16_TOKENS)
 
@@ -2312,7 +2322,10 @@ class CudaOps:
     def _few_parts(self, M: int, N: int, K: int) -> int:
         """Ranges of K in this kernel's partial sums (1: it does not take the product)."""
         if M <= self.SMALL_M:
-            least = 2 if K >= self.FEW_SMALL_PARTS_VALUES and N * K >= self.FEW_SMALL_PARTS_WEIGHTS else 0
+            low, high = self.FEW_SMALL_PARTS_VALUES
+            least = 2 if N * K >= self.FEW_SMALL_PARTS_WEIGHTS and (
+                low <= K <= high or K > self.STREAM_VALUES
+                or K >= self.FEW_SMALL_PARTS_LONG and N >= self.FEW_SMALL_PARTS_ROWS) else 0
         else:
             least = self.FEW_MIN_PARTS if (M <= self.FEW_PARTS_TOKENS and N <= self.FEW_PARTS_ROWS
                                            and N * K >= self.FEW_PARTS_MIN_WEIGHTS) else 0

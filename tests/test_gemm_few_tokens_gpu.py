@@ -146,7 +146,9 @@ def launched(ops, monkeypatch, call):
     (1, 24576, 64, F32, True), (16, 24568, 64, F32, False), (16, 24576, 64, BF16, True), (17, 24576, 64, BF16, True),
     (17, 24568, 64, F32, False), (64, 24576, 64, BF16, True), (65, 24576, 64, BF16, False), (128, 24576, 64, F32, True),
     (129, 24576, 64, F32, False), (16, 10240, 5080, BF16, True), (16, 10240, 5072, BF16, False), (16, 10232, 5088, BF16, False),
-    (1, 10240, 5080, F32, True), (17, 10240, 5080, F32, False)])
+    (1, 10240, 5080, F32, True), (17, 10240, 5080, F32, False), (16, 20480, 2560, BF16, False), (16, 20480, 2568, BF16, True),
+    (9, 16384, 4088, BF16, True), (8, 16384, 4088, BF16, False), (8, 16384, 4096, BF16, True), (8, 18944, 2752, BF16, False),
+    (8, 18952, 2752, BF16, True)])
 def test_which_finished_products_are_taken(ops, monkeypatch, M, N, K, dtype, taken):
     x, w = large(M, N, K)
     got, modes = launched(ops, monkeypatch, lambda: ops.linear(x, w, out_dtype=dtype))
@@ -156,7 +158,9 @@ def test_which_finished_products_are_taken(ops, monkeypatch, M, N, K, dtype, tak
 
 
 @pytest.mark.parametrize("M,N,K,taken", [
-    (16, 3664, 12288, True), (16, 3656, 12288, False), (16, 3680, 12280, False), (1, 3664, 12288, True), (17, 1024, 3072, True),
+    (16, 3664, 12288, True), (16, 3656, 12288, False), (16, 3680, 12280, False), (1, 3664, 12288, True), (16, 4096, 13056, True),
+    (16, 4096, 13064, False), (16, 4096, 16888, False), (16, 4096, 16896, True), (16, 4088, 16896, False), (9, 2200, 20480, False),
+    (9, 2200, 20488, True), (9, 2192, 20488, False), (17, 1024, 3072, True),
     (17, 1024, 3064, False), (17, 4096, 12288, True), (17, 4104, 12288, False), (64, 1024, 3072, True), (65, 1024, 3072, False)])
 def test_which_partial_sums_are_taken(ops, monkeypatch, M, N, K, taken):
     x, w = large(M, N, K)
