@@ -2094,10 +2094,10 @@ class CudaOps:
             e = x.element_size()
             oe = 4 if out_dtype == torch.float32 else e
             self._costs(N * K * e + M * K * e + M * N * oe, 2.0 * M * N * K, f" {M}x{K}->{N}")
-        few = M > 0 and self._few_tokens_ok(x, weight)
+        few = 0 < M <= self.FEW_TOKENS and x.dtype == torch.bfloat16  # (sizes first: they settle most calls)
         if few and partial_sums and self.partial_sums and out is None and out_dtype is None:
             parts = self._few_parts(M, N, K)
-            if parts > 1:
+            if parts > 1 and self._few_tokens_ok(x, weight):
                 planes = torch.empty((parts, M, N), dtype=torch.float32, device=x.device)
                 self._few_product(1, x, weight, planes, parts, M, N, K)
                 return planes
@@ -2112,7 +2112,7 @@ class CudaOps:
                 return planes
         odt = out_dtype or x.dtype
         if (few and odt in (torch.float32, torch.bfloat16) and self._few_finished(M, N, K, odt)
-                and (out is None or (out.dtype == odt and out.stride(1) == 1))):
+                and (out is None or (out.dtype == odt and out.stride(1) == 1)) and self._few_tokens_ok(x, weight)):
             if out is None:
                 out = torch.empty((M, N), dtype=odt, device=x.device)
             self._few_product(int(odt == torch.float32), x, weight, out, 1, M, N, K)
@@ -2393,7 +2393,8 @@ class CudaOps:
         if self.timing is not None:
             e = x.element_size()
             self._costs((2 * I * K + M * K + M * I) * e, 4.0 * M * I * K, f" {M}x{K}->2x{I} swiglu")
-        if M > 0 and self._few_tokens_ok(x, gate_up_weight) and out.stride(1) == 1 and self._few_gated(M, I, K):
+        if (0 < M <= self.FEW_GATED_TOKENS_WIDE and self._few_gated(M, I, K) and out.stride(1) == 1
+                and self._few_tokens_ok(x, gate_up_weight)):
             self._few_product(2 + act, x, gate_up_weight, out, 1, M, I, K)
             return out
         if self._small_m_ok(x, gate_up_weight):

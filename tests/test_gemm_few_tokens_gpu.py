@@ -200,6 +200,16 @@ def test_which_gated_products_are_taken(ops, monkeypatch, M, I, K, taken, act, a
     assert bool(((got.double() - want).abs() <= bound).all())
 
 
+def test_sizes_settle_most_calls(ops, monkeypatch):
+    """Strides, types and alignment are looked at only where the sizes are this kernel's: a call that is not pays for comparisons."""
+    monkeypatch.setattr(ops, "_few_tokens_ok", lambda x, weight: pytest.fail("asked for"))
+    for M in (1, 16, 17, 64, 128, 129, 300):
+        x, w = draw(M, 256, 264)
+        for kw in ({}, dict(partial_sums=True), dict(out_dtype=F32)):
+            ops.linear(x, w, **kw)
+        ops.gated_linear(x, w, torch.empty((M, 128), dtype=BF16, device="cuda"))
+
+
 def test_weights_the_kernel_before_writes_and_a_captured_step(ops):
     M, N, K = 48, 24576, 256
     x, w = draw(M, N, K)
