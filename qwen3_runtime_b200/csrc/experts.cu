@@ -147,9 +147,9 @@ route_logits_tile_kernel(const float* __restrict__ h, long h_stride, const float
 
 // MT x 16 tokens and NT x 8 experts a block.  Lane (g, t4) = (lane / 4, lane % 4) of a fragment holds rows g (and g + 8) and, of a
 // slice, k = 8 t4 .. 8 t4 + 7, half of them for each of two MMAs: the order of k within a slice is the same for both operands.
-// VEC: rows of both start at 16-byte boundaries and the width is a multiple of 8.
+// VEC: values that a load takes, as far as strides, addresses and the width allow: 8 (tokens 16 bytes, the router 2 x 16), 4 or 1.
 constexpr int ROUTE_SLICE = 32, ROUTE_WARPS = 8;
-template <int MT, int NT, bool VEC>
+template <int MT, int NT, int VEC>
 __global__ void __launch_bounds__(32 * ROUTE_WARPS)
 route_logits_mma_kernel(const bf16* __restrict__ h, long h_stride, const float* __restrict__ router, int num_tokens, int E,
                         int W, float* __restrict__ logits) {
@@ -170,18 +170,25 @@ route_logits_mma_kernel(const bf16* __restrict__ h, long h_stride, const float* 
   float b[NT][8];
   auto load = [&](int slice) {
     const int k = slice * ROUTE_SLICE + 8 * t4;
-    if (VEC) {
-      const bool in = k < W;
+    if (VEC > 1) {
+      const bool in = k < W, on = VEC == 8 ? in : k + 4 < W;  // (of 4 values a load, the second may be beyond the end)
 #pragma unroll
       for (int m = 0; m < MT; ++m)
 #pragma unroll
-        for (int r = 0; r < 2; ++r)
-          a[m][r] = in ? __ldg(reinterpret_cast<const uint4*>(x[m][r] + k)) : make_uint4(0, 0, 0, 0);
+        for (int r = 0; r < 2; ++r) {
+          if (VEC == 8) {
+            a[m][r] = in ? __ldg(reinterpret_cast<const uint4*>(x[m][r] + k)) : make_uint4(0, 0, 0, 0);
+          } else {
+            const uint2 lo = in ? __ldg(reinterpret_cast<const uint2*>(x[m][r] + k)) : make_uint2(0, 0);
+            const uint2 hi = on ? __ldg(reinterpret_cast<const uint2*>(x[m][r] + k + 4)) : make_uint2(0, 0);
+            a[m][r] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+          }
+        }
 #pragma unroll
       for (int n = 0; n < NT; ++n)
 #pragma unroll
         for (int i = 0; i < 8; i += 4) {
-          const float4 v = in ? __ldg(reinterpret_cast<const float4*>(w[n] + k + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          const float4 v = (i ? on : in) ? __ldg(reinterpret_cast<const float4*>(w[n] + k + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
           b[n][i] = v.x, b[n][i + 1] = v.y, b[n][i + 2] = v.z, b[n][i + 3] = v.w;
         }
     } else {
@@ -510,17 +517,22 @@ Q3_EXPORT int q3_route_top(int dtype, const void* h, long h_stride, const float*
   if (dtype != Q3_DTYPE_F32 && dtype != Q3_DTYPE_BF16) return Q3_ERR_ARGUMENT;
   cudaError_t e;
   if (dtype == Q3_DTYPE_BF16) {
-    const bool vec = W % 8 == 0 && h_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0;
+    const uintptr_t at = reinterpret_cast<uintptr_t>(h) | (uintptr_t)(2 * h_stride) | (uintptr_t)(2 * W);
+    const int vec = (at & 15) == 0 ? 8 : (at & 7) == 0 ? 4 : 1;
     const dim3 large((num_tokens + 31) / 32, (E + 31) / 32), small((num_tokens + 15) / 16, (E + 7) / 8);
 #define Q3_ROUTE_MMA(MT_, NT_, VEC_, grid_)                                                                              \
   e = launch_pdl(route_logits_mma_kernel<MT_, NT_, VEC_>, grid_, dim3(32 * ROUTE_WARPS), 0, stream, (const bf16*)h, h_stride, \
                  router, num_tokens, E, W, logits)
     // large blocks from where they fill half of the SMs, and where 32 experts are not mostly none (8 x 512, 4096 tokens: 13.7 us
-    // with the choice, 6.1 with small blocks)
-    if (vec && E > 16 && 2l * large.x * large.y >= sm_count() && large.y <= 65535) Q3_ROUTE_MMA(2, 4, true, large);
-    else if (small.y > 65535) return Q3_ERR_UNSUPPORTED;
-    else if (vec) Q3_ROUTE_MMA(1, 1, true, small);
-    else Q3_ROUTE_MMA(1, 1, false, small);
+    // with the choice, 6.1 with small blocks).  Rows at 8-byte places (2048 tokens x 64 experts x 2052 with
+    // the choice): single loads in small blocks 45.5, FMAs 35.7, loads of 4 in large ones 16.8.
+    const bool wide = vec > 1 && E > 16 && 2l * large.x * large.y >= sm_count() && large.y <= 65535;
+    if (!wide && small.y > 65535) return Q3_ERR_UNSUPPORTED;
+    if (wide && vec == 8) Q3_ROUTE_MMA(2, 4, 8, large);
+    else if (wide) Q3_ROUTE_MMA(2, 4, 4, large);
+    else if (vec == 8) Q3_ROUTE_MMA(1, 1, 8, small);
+    else if (vec == 4) Q3_ROUTE_MMA(1, 1, 4, small);
+    else Q3_ROUTE_MMA(1, 1, 1, small);
 #undef Q3_ROUTE_MMA
   } else {
     // both kernels give the same bits; the tile kernel needs about 64 tokens to fill the SMs

@@ -127,7 +127,7 @@ def _logits(ops, h, router):
 
 
 @pytest.mark.parametrize("tokens,experts,width", [(1200, 64, 520), (2400, 33, 136), (400, 200, 72), (40, 20, 100), (33, 20, 37),
-                                                  (2500, 17, 2048), (1, 1, 8)])
+                                                  (2500, 17, 2048), (1, 1, 8), (1200, 64, 516), (1200, 64, 36), (300, 33, 4)])
 def test_router_logits_of_every_block(ops, tokens, experts, width):
     """Large and small blocks, rows at odd places and widths that end inside a slice: the same bits, near to float64; infinities and
     NaN as float32 products give them, in their own row and column only."""
@@ -149,3 +149,20 @@ def test_router_logits_of_every_block(ops, tokens, experts, width):
         assert torch.equal(again[again.isinf()], want[want.isinf()].float())
         fine = want.isfinite()
         assert torch.equal(again[fine], got[fine])
+
+
+@pytest.mark.parametrize("tokens,experts,width", [(1200, 64, 512), (1200, 64, 516), (2400, 33, 40), (40, 20, 100), (1, 5, 8)])
+def test_router_logits_of_rows_at_every_place(ops, tokens, experts, width):
+    """Loads of 8, 4 and single values, in large and small blocks: the same bits."""
+    g = torch.Generator().manual_seed(width)
+    h = torch.randn((tokens, width), generator=g).to(torch.bfloat16).cuda()
+    router = (0.02 * torch.randn((experts, width), generator=g)).cuda()
+    wanted = None
+    for pad, first in ((8, 0), (8, 8), (4, 0), (8, 4), (4, 4), (2, 2), (1, 0), (8, 1)):
+        rows = torch.full((tokens, width + pad), float("nan"), dtype=torch.bfloat16, device="cuda")
+        rows[:, first: first + width] = h
+        got = _logits(ops, rows[:, first: first + width], router)
+        wanted = got if wanted is None else wanted
+        assert torch.equal(got, wanted), (pad, first)
+    want = h.double() @ router.double().t()
+    assert float((wanted - want).norm() / want.norm()) <= 2.0 ** -24 * (6 + (width / 32) ** 0.5)  # (as above)
