@@ -101,8 +101,8 @@ __device__ __forceinline__ bool mbar_wait_drain(uint32_t bar, uint32_t parity) {
 }
 // Where the warps of a role meet inside their loop, some may have given up and others seen the barrier complete: all of the
 // `threads` threads that meet at named barrier `id` learn whether any of them has given up.  Meeting and asking are one operation: a
-// flag in shared memory, read behind a barrier, could be raised for the next round by a warp that is ahead before a slower one
-// has read it for this round; the two would part, and one would wait at the barrier for good.  (Whole warps, of one mind each.)
+// flag in shared memory, read behind a barrier, could be raised for the next item by a warp that is ahead before a slower one
+// has read it for the present one; the two would part, and one would wait at the barrier for good.  (Whole warps, of one mind each.)
 __device__ __forceinline__ bool any_gave_up(int id, int threads, bool gave_up) {
   uint32_t any;
   asm volatile(
